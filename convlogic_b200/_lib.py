@@ -1,16 +1,20 @@
-"""ctypes binding of the C-ABI library ``csrc/libconvlogic_b200.so``.
+"""Loads the C-ABI library ``csrc/libconvlogic_b200.so`` (ctypes) and the torch extension module over it,
+``csrc/_clb_torch.so``, which the layers call.
 
 The library is the product: there is no CPU or PyTorch fallback.  If it has not been built,
-every operation raises (``python -m convlogic_b200.build`` builds it with nvcc).
+every operation raises (``python -m convlogic_b200.build`` builds it with nvcc and g++).
 """
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import os
 
 import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "csrc", "libconvlogic_b200.so")
+BIND_PATH = os.path.join(_HERE, "csrc", "_clb_torch.so")
 
 F32, F64 = 0, 1
 W_PROB, W_SOFTMAX, W_ARGMAX = 0, 1, 2
@@ -22,6 +26,7 @@ TUNE_SLAB_MUX = 3
 ERR_SHAPE, ERR_ODD_OUTPUT, ERR_TOO_LARGE = -2, -5, -6
 
 _lib = None
+_native = None
 
 _vp, _i, _i64, _sz = C.c_void_p, C.c_int, C.c_int64, C.c_size_t
 _conv = [_i] * 11  # N, Ci, H, W, C, sh, sw, ph, pw, kh, kw
@@ -108,6 +113,22 @@ def lib():
             fn.argtypes, fn.restype = args, res
         _lib = handle
     return _lib
+
+
+def native():
+    """The torch extension module; raises RuntimeError when it is missing (no fallback exists)."""
+    global _native
+    if _native is None:
+        lib()  # the extension links against it
+        if not os.path.exists(BIND_PATH):
+            raise RuntimeError(
+                f"convlogic_b200: torch extension not found at {BIND_PATH}. "
+                "Build it with `python -m convlogic_b200.build`; there is no CPU fallback.")
+        loader = importlib.machinery.ExtensionFileLoader("_clb_torch", BIND_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_clb_torch", BIND_PATH, loader=loader))
+        loader.exec_module(module)
+        _native = module
+    return _native
 
 
 def trace(on):

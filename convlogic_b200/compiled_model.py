@@ -11,13 +11,12 @@ the code is the library's ``clb_net_*`` runtime, which runs the whole stack on t
 ``forward(x)`` with ``x`` bool ``[B, F]`` (or ``[B, C, H, W]``) returning int32 counts ``[B, num_classes]``.
 """
 
-import ctypes as C
 import struct
 
 import numpy as np
 import torch
 
-from . import _lib
+from ._lib import native
 from .convlogic_layer import ConvLogicLayer
 from .difflogic import GroupSum, LogicLayer
 
@@ -140,8 +139,6 @@ class CompiledLogicNet(torch.nn.Module):
         self.model, self.device, self.num_bits, self.input_shape = model, torch.device(device), num_bits, input_shape
         self.blob = None
         self._net = None
-        self._params = None
-        self._workspace = None
         if model is not None:
             self.num_classes = model[-1].k
             self.blob = serialise(model, input_shape, fuse)
@@ -172,41 +169,14 @@ class CompiledLogicNet(torch.nn.Module):
         return self
 
     def _create(self):
-        lib = _lib.lib()
-        need = C.c_size_t()
-        _lib.check(lib.clb_net_device_bytes(self.blob, len(self.blob), C.byref(need)))
-        self._params = torch.empty(max(need.value, 16), dtype=torch.uint8, device=self.device)
-        handle = C.c_void_p()
-        with torch.cuda.device(self.device):
-            _lib.check(lib.clb_net_create(self.blob, len(self.blob), _lib.ptr(self._params), _lib.stream(), C.byref(handle)))
-            torch.cuda.current_stream().synchronize()  # the blob is pageable host memory: wait for the copy
-        self._net = handle
-        feats, classes, n = C.c_int64(), C.c_int(), C.c_int()
-        _lib.check(lib.clb_net_info(handle, C.byref(feats), C.byref(classes), C.byref(n)))
-        self.num_inputs, self.num_classes, self.num_layers = feats.value, classes.value, n.value
-
-    def __del__(self):
-        if getattr(self, "_net", None) is not None:
-            try:
-                _lib.lib().clb_net_destroy(self._net)
-            except Exception:
-                pass
-            self._net = None
+        self._net = native().Net(self.blob, str(self.device))
+        self.num_inputs, self.num_classes, self.num_layers = self._net.features, self._net.classes, self._net.layers
 
     # ---- inference
     def _run(self, kind, x, batch, thresholds=None):
         if self._net is None:
             raise RuntimeError("convlogic_b200: call compile() or load() first")
-        lib = _lib.lib()
-        need = lib.clb_net_workspace_bytes(self._net, batch)
-        if self._workspace is None or self._workspace.numel() < need:
-            self._workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
-        counts = torch.empty((batch, self.num_classes), dtype=torch.int32, device=self.device)
-        levels = 0 if thresholds is None else thresholds.numel()
-        with torch.cuda.device(self.device):
-            _lib.check(lib.clb_net_forward(self._net, kind, _lib.ptr(x), _lib.ptr(thresholds), levels, batch, _lib.ptr(counts),
-                                           _lib.ptr(self._workspace), self._workspace.numel(), _lib.stream()))
-        return counts
+        return self._net.run(kind, x, thresholds, batch)
 
     # ---- CUDA graph replay for a fixed batch size (the runtime allocates nothing and never synchronises)
     def capture(self, example, thresholds=None):

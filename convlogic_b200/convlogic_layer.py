@@ -10,8 +10,8 @@ import torch
 from torch import nn
 
 from . import ops
-from ._lib import W_ARGMAX, W_SOFTMAX
-from .functional import ConvLogicFunction, FullConvLogicFunction, GradFactor
+from ._lib import W_ARGMAX, W_SOFTMAX, native
+from .functional import ConvLogicFunction, GradFactor
 from .packbitstensor import PackBitsTensor
 
 
@@ -21,6 +21,8 @@ def _pair(v):
 
 class ConvLogicLayer(nn.Module):
     """8 taps per output channel -> 4 gates, and with ``complete=True`` -> 2 -> 1 gate -> 2x2 max pool."""
+
+    output_feature_major = False  # set on a block in front of flat layers, see fuse_logic_layers
 
     def __init__(self, in_channels, out_channels, stride=1, padding=1, kernel=3, groups=1, selection=None,
                  residual_init=False, implementation="cuda", grad_factor=1.0, complete=False,
@@ -51,7 +53,8 @@ class ConvLogicLayer(nn.Module):
     def forward(self, x):
         if isinstance(x, PackBitsTensor):
             return self.forward_cuda_eval(x)
-        x = x.contiguous()
+        if not x.is_contiguous():
+            x = x.contiguous()
         if self.grad_factor != 1.0:
             x = GradFactor.apply(x, self.grad_factor)
         return self.forward_cuda(x)
@@ -60,12 +63,15 @@ class ConvLogicLayer(nn.Module):
         if not x.is_cuda:
             raise RuntimeError("CUDA implementation requested, but the input is not a CUDA tensor.")
         wmode = W_SOFTMAX if self.training else W_ARGMAX
-        w = self.weights if self.weights.dtype == x.dtype else self.weights.to(x.dtype)
-        sel = self.selection.contiguous()
+        w, sel = self._parameters["weights"], self._buffers["selection"]
+        if w.dtype != x.dtype:
+            w = w.to(x.dtype)
+        if not sel.is_contiguous():
+            sel = sel.contiguous()
         geom = (*self.stride, *self.padding, *self.kernel)
         if self.complete:
-            return FullConvLogicFunction.apply(x, w, sel, *geom, self.return_intermediate, self.return_indices, wmode,
-                                               getattr(self, "output_feature_major", False) and self.training)
+            return native().block(x, w, sel, *geom, self.return_intermediate, self.return_indices, wmode,
+                                  self.output_feature_major and self.training)
         return ConvLogicFunction.apply(x, w, sel, *geom, wmode)
 
     def forward_cuda_eval(self, x: PackBitsTensor):

@@ -1,0 +1,931 @@
+// Torch binding of the C-ABI library: tensors in, tensors out, autograd nodes in C++.
+//
+// What bounds a small call is the host: through ctypes and Python autograd Functions a layer cost 50 to 100 us of host
+// time (measured on a three-layer flat stack, batch 100: 506 us forward + backward, of which the kernels take 91), the
+// launches themselves about 2.5 us each.  Here a layer is one call: checks, output allocation, launch and the autograd
+// node, and its backward runs on autograd's own thread without entering Python (except for the gradient-bucket callback
+// of a parameter that carries one).  No arithmetic happens here; every number comes from the kernels behind
+// include/convlogic_b200.h.
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/accumulate_grad.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/utils/pybind.h>
+
+#include <map>
+#include <memory>
+#include <mutex>
+#include <optional>
+#include <string>
+#include <tuple>
+#include <vector>
+
+#include "../../include/convlogic_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::edge_list;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+
+namespace {
+
+// ------------------------------------------------------------------------------------------------ helpers
+// the exception the reference raises for the same condition (the Python side's `check`)
+void check(int status)
+{
+    if (status == CLB_OK) return;
+    const std::string text = std::string("convlogic_b200: ") + clb_status_string(status);
+    if (status == CLB_ERR_LAUNCH) TORCH_CHECK(false, text, " (cudaError ", clb_last_cuda_error(), ")");
+    TORCH_CHECK_VALUE(status != CLB_ERR_SHAPE && status != CLB_ERR_TOO_LARGE, text);
+    TORCH_CHECK(false, text);
+}
+
+void need_input(const Tensor &t)
+{
+    TORCH_CHECK(t.is_cuda(), "convlogic_b200: tensor must be a CUDA tensor");
+    TORCH_CHECK(t.is_contiguous(), "convlogic_b200: tensor must be contiguous");
+}
+template <typename... Ts> void need_inputs(const Ts &...ts) { (need_input(ts), ...); }
+
+int dtype_code(const Tensor &t)
+{
+    if (t.scalar_type() == at::kFloat) return CLB_F32;
+    TORCH_CHECK(t.scalar_type() == at::kDouble, "convlogic_b200: expected a float32 or float64 tensor, got ", t.scalar_type());
+    return CLB_F64;
+}
+
+void *stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+template <typename T = void> T *ptr(const Tensor &t) { return t.defined() ? static_cast<T *>(t.data_ptr()) : nullptr; }
+Tensor scratch_bytes(size_t n, const Tensor &like) { return at::empty({(int64_t)(n < 16 ? 16 : n)}, like.options().dtype(at::kByte)); }
+
+// Raw calls run below autograd and view tracking: their results get a history from our own nodes only.
+struct Below {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    c10::cuda::CUDAGuard device;
+    explicit Below(const Tensor &t) : device(t.device()) {}
+};
+
+bool wants_grad(std::initializer_list<std::reference_wrapper<const Tensor>> ts)
+{
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor &t : ts)
+        if (t.defined() && t.requires_grad()) return true;
+    return false;
+}
+
+// SavedVariable of an input (never an output) of a node
+SavedVariable saved(const Tensor &t) { return SavedVariable(t, false); }
+
+// One node kind per operation: `Derived` has fields, run(grads) and clear().
+template <typename Derived> std::shared_ptr<Derived> new_node() { return std::shared_ptr<Derived>(new Derived(), torch::autograd::deleteNode); }
+
+// [rows, cols] fp32 -> contiguous [cols, rows]
+Tensor transpose2d(const Tensor &x)
+{
+    need_input(x);
+    TORCH_CHECK(x.dim() == 2 && x.scalar_type() == at::kFloat, "convlogic_b200: transpose2d expects a contiguous 2-D float32 tensor");
+    Below below(x);
+    Tensor out = at::empty({x.size(1), x.size(0)}, x.options());
+    check(clb_transpose_f32(ptr<float>(x), ptr<float>(out), x.size(0), x.size(1), stream()));
+    return out;
+}
+
+// contiguous copy of t's transpose (t 2-D), with the library's tiled kernel where it applies
+Tensor transposed_copy(const Tensor &t)
+{
+    if (t.is_cuda() && t.scalar_type() == at::kFloat && t.is_contiguous() && t.numel()) return transpose2d(t);
+    return t.t().contiguous();
+}
+
+// feature-major storage [F, B] of a [B, F] activation: its own storage when it is the transposed view a flat layer returns
+Tensor feature_major(const Tensor &x)
+{
+    Tensor xt = x.t();
+    return xt.is_contiguous() ? xt : transposed_copy(x);
+}
+
+// a [B, F] gradient whose storage is [F, B]; a leaf that stores [B, F] gets a plain contiguous tensor, anything else the view
+Tensor batch_major_grad(const Tensor &g_fm, bool contiguous) { return contiguous ? transposed_copy(g_fm) : g_fm.t(); }
+bool feeds_leaf(const Node &n, size_t i)
+{
+    const auto &e = n.next_edge(i);
+    return e.function && dynamic_cast<torch::autograd::AccumulateGrad *>(e.function.get()) != nullptr;
+}
+
+// ------------------------------------------------------------------------------------------------ gradient sinks
+// A parameter may carry `_clb_grad_sink` = (slice of a flat gradient buffer, ready callback, ranges callback, range): its
+// gradient is then written into the slice by the kernel and the callback told, and autograd gets no gradient for it.
+struct Sink {
+    Tensor slice;
+    py::object ready, ranges, range;
+};
+std::optional<Sink> sink_of(const Tensor &w) // GIL held
+{
+    py::object obj = py::reinterpret_steal<py::object>(THPVariable_Wrap(w));
+    PyObject *s = nullptr;
+    if (PyObject_HasAttrString(obj.ptr(), "_clb_grad_sink")) s = PyObject_GetAttrString(obj.ptr(), "_clb_grad_sink");
+    if (!s) return std::nullopt;
+    py::object held = py::reinterpret_steal<py::object>(s);
+    if (held.is_none()) return std::nullopt;
+    py::tuple t = held.cast<py::tuple>();
+    Sink out;
+    out.slice = t[0].cast<Tensor>();
+    out.ready = t[1];
+    if (t.size() > 3) out.ranges = t[2], out.range = t[3];
+    return out;
+}
+
+// The slices of one backward call's parameters: all of them or none (a kernel writes them together).
+class Sinks {
+public:
+    explicit Sinks(std::initializer_list<std::reference_wrapper<const Tensor>> ws)
+    {
+        py::gil_scoped_acquire gil;
+        for (const Tensor &w : ws) {
+            auto s = sink_of(w);
+            if (!s) {
+                list_.clear();
+                return;
+            }
+            list_.push_back(std::move(*s));
+        }
+    }
+    ~Sinks()
+    {
+        if (list_.empty()) return;
+        py::gil_scoped_acquire gil;
+        list_.clear();
+    }
+    bool any() const { return !list_.empty(); }
+    Tensor slice(size_t i) const { return any() ? list_[i].slice : Tensor(); }
+    // the kernels that write the slices are enqueued: neighbouring slices of one bucket are reported as one exchange
+    void ready()
+    {
+        if (list_.empty()) return;
+        py::gil_scoped_acquire gil;
+        bool one_bucket = list_.size() > 1;
+        for (const Sink &s : list_) one_bucket = one_bucket && s.ranges && s.ranges.equal(list_[0].ranges);
+        if (one_bucket) {
+            py::list ranges;
+            for (const Sink &s : list_) ranges.append(s.range);
+            list_[0].ranges(ranges);
+        } else {
+            for (const Sink &s : list_) s.ready();
+        }
+    }
+
+private:
+    std::vector<Sink> list_;
+};
+
+// ------------------------------------------------------------------------------------------------ fused block
+struct Geom {
+    int sh, sw, ph, pw, kh, kw;
+    bool operator==(const Geom &o) const { return sh == o.sh && sw == o.sw && ph == o.ph && pw == o.pw && kh == o.kh && kw == o.kw; }
+};
+
+// What the kernels need to know about a selection: checked and laid out once per (selection tensor and version, geometry,
+// input channels), kept on the selection tensor object as `_clb_plan` (nothing outlives the tensor).
+struct BlockPlan {
+    Geom g;
+    int C, ci;
+    int64_t version;
+    const void *data;
+    int flag;                        // CLB_SEL_UNBOUNDED when a tap lies outside the window
+    bool channels_ok;
+    std::vector<int32_t> sel;        // host copy
+    std::mutex mu;
+    int lists = -1;                  // channel lists: -1 not built, 0 the selection does not fit two planes, 1 built
+    Tensor start, entry;
+    struct Groups {
+        Tensor start, list;
+        int cg, nb;
+    };
+    std::map<std::tuple<int64_t, int64_t, int64_t, int>, Groups> groups; // (N, H, W, dtype), at most 16 kept
+    c10::Device device{c10::kCUDA};
+
+    Tensor to_device(const std::vector<int32_t> &v)
+    {
+        return at::tensor(at::ArrayRef<int32_t>(v.data(), v.size()), at::TensorOptions().dtype(at::kInt)).to(device);
+    }
+    bool channel_lists()
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (lists < 0) {
+            std::vector<int32_t> st((size_t)ci + 1, 0), en((size_t)(2 * C > 0 ? 2 * C : 1), 0);
+            const int n = clb_conv_channel_lists(sel.data(), C, ci, g.kh, g.kw, st.data(), en.data(), (int)en.size());
+            if (n < 0 && n != CLB_ERR_SHAPE) check(n);
+            if (n >= 0) {
+                en.resize((size_t)(n > 0 ? n : 1));
+                start = to_device(st), entry = to_device(en);
+            }
+            lists = n >= 0;
+        }
+        return lists == 1;
+    }
+    Groups group_tables(int64_t n, int64_t h, int64_t w, int dtype)
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        const auto key = std::make_tuple(n, h, w, dtype);
+        auto it = groups.find(key);
+        if (it != groups.end()) return it->second;
+        Groups out;
+        check(clb_conv_group_plan((int)n, ci, (int)h, (int)w, C, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, dtype, &out.cg, &out.nb));
+        const int count = (ci + out.cg - 1) / out.cg;
+        std::vector<int32_t> st((size_t)count + 1, 0), ls((size_t)std::max<long long>(1, (long long)C * std::min(count, 8)), 0);
+        const int got = clb_conv_build_groups(sel.data(), C, ci, out.cg, st.data(), ls.data(), (int)ls.size());
+        TORCH_CHECK(got != CLB_ERR_ARG, "convlogic_b200: selection refers to a channel the input does not have");
+        if (got < 0) check(got);
+        ls.resize((size_t)(got > 0 ? got : 1));
+        out.start = to_device(st), out.list = to_device(ls);
+        if (groups.size() >= 16) groups.clear();
+        groups.emplace(key, out);
+        return out;
+    }
+};
+using PlanPtr = std::shared_ptr<BlockPlan>;
+
+PlanPtr plan_for(const py::handle &sel_obj, const Tensor &sel, const Geom &g, int64_t ci) // GIL held
+{
+    const int64_t version = sel.is_inference() ? 0 : (int64_t)sel._version();
+    if (PyObject_HasAttrString(sel_obj.ptr(), "_clb_plan")) {
+        PlanPtr p = py::reinterpret_steal<py::object>(PyObject_GetAttrString(sel_obj.ptr(), "_clb_plan")).cast<PlanPtr>();
+        if (p && p->version == version && p->data == sel.data_ptr() && p->g == g && p->ci == ci) return p;
+    }
+    auto p = std::make_shared<BlockPlan>();
+    p->g = g, p->C = (int)sel.size(0), p->ci = (int)ci, p->version = version, p->data = sel.data_ptr(), p->device = sel.device();
+    const Tensor host = sel.detach().to(at::kCPU).contiguous();
+    p->sel.assign(host.data_ptr<int32_t>(), host.data_ptr<int32_t>() + host.numel());
+    bool inside = true, channels = true;
+    for (const int32_t word : p->sel) {
+        inside = inside && ((word >> 8) & 0xFF) < g.kh && (word & 0xFF) < g.kw;
+        channels = channels && word >= 0 && ((word >> 16) & 0xFFFF) < ci;
+    }
+    p->flag = inside ? 0 : CLB_SEL_UNBOUNDED, p->channels_ok = channels;
+    sel_obj.attr("_clb_plan") = p;
+    return p;
+}
+
+bool is_feature_major(const Tensor &t) // [N, C, h, w] on the contiguous storage [C, h, w, N]
+{
+    if (t.dim() != 4 || t.is_contiguous()) return false;
+    const int64_t n = t.size(0), c = t.size(1), h = t.size(2), w = t.size(3);
+    auto ok = [](int64_t size, int64_t stride, int64_t want) { return size == 1 || stride == want; };
+    return ok(n, t.stride(0), 1) && ok(w, t.stride(3), n) && ok(h, t.stride(2), n * w) && ok(c, t.stride(1), n * w * h);
+}
+
+struct BlockDims {
+    int n, ci, h, w, c, ho, wo;
+};
+BlockDims block_dims(const Tensor &x, const Tensor &w, const Tensor &sel, const Geom &g)
+{
+    TORCH_CHECK(x.dim() == 4, "convlogic_b200: x must be [N, C, H, W]");
+    const int64_t c = w.size(0);
+    TORCH_CHECK(w.dim() == 3 && w.size(1) == 7 && w.size(2) == 16 && w.scalar_type() == x.scalar_type(), "convlogic_b200: gate tensor must be [", c,
+                ", 7, 16] ", x.scalar_type());
+    TORCH_CHECK(sel.scalar_type() == at::kInt && sel.dim() == 2 && sel.size(0) == c && sel.size(1) == 8,
+                "convlogic_b200: selection must be int32 [", c, ", 8], got ", sel.scalar_type(), " ", sel.sizes());
+    BlockDims d{(int)x.size(0), (int)x.size(1), (int)x.size(2), (int)x.size(3), (int)c, 0, 0};
+    d.ho = (d.h + 2 * g.ph - g.kh) / g.sh + 1, d.wo = (d.w + 2 * g.pw - g.kw) / g.sw + 1;
+    return d;
+}
+
+struct BlockOut {
+    Tensor y, amax, x2, x3, idx;
+};
+
+BlockOut block_fwd(const Tensor &x, const Tensor &w, const Tensor &sel, const Geom &g, const std::function<PlanPtr()> &get_plan, int wmode,
+                   bool want_amax, bool want_inter, bool want_idx, bool y_fm)
+{
+    need_inputs(x, w, sel);
+    const BlockDims d = block_dims(x, w, sel, g);
+    TORCH_CHECK(d.ho > 0 && d.wo > 0, "Invalid output shape: H_out=", d.ho, ", W_out=", d.wo);
+    TORCH_CHECK(d.ho % 2 == 0 && d.wo % 2 == 0, "Output height and width after convolution must be divisible by 2 for 2x2 max pooling, but got H_out=",
+                d.ho, ", W_out=", d.wo);
+    const int hp = d.ho / 2, wp = d.wo / 2, dt = dtype_code(x);
+    Below below(x);
+    BlockOut o;
+    if (want_amax) o.amax = at::empty({d.n, d.c, hp, wp}, x.options().dtype(at::kByte));
+    if (want_inter) o.x2 = at::empty({d.n, d.c, d.ho, d.wo, 4}, x.options()), o.x3 = at::empty({d.n, d.c, d.ho, d.wo, 2}, x.options());
+    if (want_idx) o.idx = at::empty({d.n, d.c, (int64_t)hp * wp}, x.options().dtype(at::kInt));
+    if (d.n == 0 || d.c == 0) { // empty batch: nothing to launch
+        o.y = at::empty({d.n, d.c, hp, wp}, x.options());
+        return o;
+    }
+    const PlanPtr plan = get_plan();
+    TORCH_CHECK(plan->channels_ok, "convlogic_b200: selection refers to a channel the input does not have");
+    if (y_fm && dt == CLB_F32 && !want_inter && !want_idx && !plan->flag) {
+        // the flat layers' layout, storage [C, h, w, N]; only the plane kernels write it
+        o.y = at::empty_strided({d.n, d.c, hp, wp}, {1, (int64_t)hp * wp * d.n, (int64_t)wp * d.n, d.n}, x.options());
+        const int rc = clb_convtree_fwd(ptr(x), ptr(w), ptr<int32_t>(sel), ptr(o.y), ptr<uint8_t>(o.amax), nullptr, nullptr, nullptr, d.n, d.ci, d.h, d.w,
+                                        d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, wmode | CLB_Y_FEATURE_MAJOR, dt, stream());
+        if (rc != CLB_ERR_SHAPE) {
+            check(rc);
+            return o;
+        }
+    }
+    o.y = at::empty({d.n, d.c, hp, wp}, x.options());
+    check(clb_convtree_fwd(ptr(x), ptr(w), ptr<int32_t>(sel), ptr(o.y), ptr<uint8_t>(o.amax), ptr(o.x2), ptr(o.x3), ptr<int32_t>(o.idx), d.n, d.ci, d.h,
+                           d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, wmode | plan->flag, dt, stream()));
+    return o;
+}
+
+// (gx or undefined, gw or undefined); gw_out: where the gate gradient goes (a slice of a flat bucket)
+std::pair<Tensor, Tensor> block_bwd(Tensor gy, const Tensor &x, const Tensor &w, const Tensor &sel, const Tensor &amax, const Geom &g,
+                                    const std::function<PlanPtr()> &get_plan, int wmode, bool need_gx, bool need_gw, const Tensor &gw_out)
+{
+    const bool fm = gy.is_cuda() && is_feature_major(gy);
+    need_inputs(x, w, sel);
+    if (!fm) need_input(gy);
+    const BlockDims d = block_dims(x, w, sel, g);
+    const int64_t hp = d.ho / 2, wp = d.wo / 2;
+    const std::vector<int64_t> want{d.n, d.c, hp, wp};
+    TORCH_CHECK(gy.sizes() == at::IntArrayRef(want) && gy.scalar_type() == x.scalar_type(), "convlogic_b200: upstream gradient must be ",
+                at::IntArrayRef(want), " ", x.scalar_type(), ", got ", gy.sizes(), " ", gy.scalar_type());
+    TORCH_CHECK(!amax.defined() || (amax.sizes() == at::IntArrayRef(want) && amax.scalar_type() == at::kByte),
+                "convlogic_b200: arg-max tensor must be uint8 ", at::IntArrayRef(want));
+    const int dt = dtype_code(x);
+    Below below(x);
+    Tensor gx, gw;
+    if (need_gx) gx = at::empty(x.sizes(), x.options());
+    if (need_gw) {
+        gw = gw_out.defined() ? gw_out : at::empty(w.sizes(), w.options());
+        TORCH_CHECK(gw.sizes() == w.sizes() && gw.scalar_type() == w.scalar_type() && gw.is_contiguous(),
+                    "convlogic_b200: `gw_out` must be contiguous with the gate tensor's shape and dtype");
+    }
+    if (d.n == 0 || d.c == 0) { // empty batch: the gate gradient is an empty sum
+        if (gw.defined()) gw.zero_();
+        return {gx, gw};
+    }
+    const PlanPtr plan = get_plan();
+    TORCH_CHECK(plan->channels_ok, "convlogic_b200: selection refers to a channel the input does not have");
+    if (!plan->flag && dt == CLB_F32 && amax.defined()) {
+        // The plane kernels (two channel planes per output channel streamed through shared memory): both gradients of the
+        // many-channel layers (16x16 .. 4x4 images), the gate gradient alone of a 32x32 first block.
+        const size_t bytes = clb_convtree_bwd_plane_scratch_bytes(d.n, d.ci, d.h, d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, dt);
+        if (bytes && plan->channel_lists()) {
+            Tensor scratch = scratch_bytes(bytes, x);
+            const int rc = clb_convtree_bwd_plane(ptr(gy), ptr(x), ptr(w), ptr<int32_t>(sel), ptr<uint8_t>(amax), ptr(gx), ptr(gw), ptr<int32_t>(plan->start),
+                                                  ptr<int32_t>(plan->entry), ptr(scratch), bytes, d.n, d.ci, d.h, d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh,
+                                                  g.kw, wmode | (fm ? CLB_Y_FEATURE_MAJOR : 0), dt, stream());
+            if (rc != CLB_ERR_SHAPE) {
+                check(rc);
+                return {gx, gw};
+            }
+        }
+    }
+    if (fm) gy = transposed_copy(gy.permute({1, 2, 3, 0}).reshape({(int64_t)d.c * hp * wp, d.n})).view({d.n, d.c, hp, wp});
+    const size_t bytes = clb_convtree_bwd_scratch_bytes(d.n, d.ci, d.h, d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, need_gx, need_gw, dt);
+    Tensor scratch = scratch_bytes(bytes, x);
+    BlockPlan::Groups gr{Tensor(), Tensor(), 1, 1};
+    if (need_gx) gr = plan->group_tables(d.n, d.h, d.w, dt);
+    check(clb_convtree_bwd(ptr(gy), ptr(x), ptr(w), ptr<int32_t>(sel), ptr<uint8_t>(amax), ptr(gx), ptr(gw), ptr<int32_t>(gr.start),
+                           ptr<int32_t>(gr.list), gr.cg, gr.nb, ptr(scratch), bytes, d.n, d.ci, d.h, d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw,
+                           wmode | plan->flag, dt, stream()));
+    return {gx, gw};
+}
+
+struct BlockNode : public Node {
+    SavedVariable x, w, sel;
+    Tensor amax;
+    PlanPtr plan;
+    Geom g;
+    int wmode;
+    std::string name() const override { return "FullConvLogicFunctionBackward"; }
+    void release_variables() override { x.reset_data(), w.reset_data(), sel.reset_data(), amax.reset(); }
+    variable_list apply(variable_list &&grads) override
+    {
+        if (!grads[0].defined()) return {Tensor(), Tensor()};
+        const Tensor xx = x.unpack(), ww = w.unpack(), ss = sel.unpack();
+        const bool need_gx = task_should_compute_output(0), need_gw = task_should_compute_output(1) && wmode != CLB_W_ARGMAX;
+        if (!need_gx && !need_gw) return {Tensor(), Tensor()};
+        Tensor gy = grads[0];
+        if (!is_feature_major(gy)) gy = gy.contiguous(); // a feature-major gradient (from flat layers behind this block) is read as it is
+        if (!need_gw) return {block_bwd(gy, xx, ww, ss, amax, g, [&] { return plan; }, wmode, need_gx, false, Tensor()).first, Tensor()};
+        Sinks sinks({ww});
+        auto out = block_bwd(gy, xx, ww, ss, amax, g, [&] { return plan; }, wmode, need_gx, true, sinks.slice(0));
+        if (!sinks.any()) return {out.first, out.second};
+        sinks.ready();
+        return {out.first, Tensor()};
+    }
+};
+
+// y, or (y[, x2, x3][, idx]) when extras are asked for
+py::object block(Tensor x, Tensor w, py::object sel_obj, int sh, int sw, int ph, int pw, int kh, int kw, bool want_inter, bool want_idx, int wmode,
+                 bool y_fm)
+{
+    const Tensor sel = sel_obj.cast<Tensor>();
+    x = x.contiguous(), w = w.contiguous();
+    const Geom g{sh, sw, ph, pw, kh, kw};
+    const bool graph = wants_grad({x, w});
+    PlanPtr plan;
+    auto get_plan = [&] { return plan = plan_for(sel_obj, sel, g, x.size(1)); };
+    BlockOut o = block_fwd(x, w, sel, g, get_plan, wmode, graph, want_inter, want_idx, y_fm);
+    if (graph) {
+        auto node = new_node<BlockNode>();
+        node->set_next_edges(torch::autograd::collect_next_edges(x, w));
+        if (!plan) get_plan();
+        node->x = saved(x), node->w = saved(w), node->sel = saved(sel), node->amax = o.amax, node->plan = plan, node->g = g, node->wmode = wmode;
+        torch::autograd::set_history(o.y, node);
+    }
+    if (!want_inter && !want_idx) return py::cast(o.y);
+    py::list out;
+    out.append(o.y);
+    if (want_inter) out.append(o.x2), out.append(o.x3);
+    if (want_idx) out.append(o.idx);
+    return py::tuple(out);
+}
+
+// ------------------------------------------------------------------------------------------------ flat layer
+struct LogicDims {
+    int64_t in, out, batch;
+};
+LogicDims logic_dims(const Tensor &x_fm, const Tensor &a, const Tensor &b, const Tensor &w)
+{
+    TORCH_CHECK(x_fm.dim() == 2, "convlogic_b200: x must be [in_dim, batch], got ", x_fm.sizes());
+    const int64_t out = w.size(0);
+    TORCH_CHECK(w.dim() == 2 && w.size(1) == 16 && w.scalar_type() == x_fm.scalar_type(), "convlogic_b200: gate tensor must be [", out, ", 16] ",
+                x_fm.scalar_type());
+    TORCH_CHECK(a.scalar_type() == at::kLong && b.scalar_type() == at::kLong && a.dim() == 1 && b.dim() == 1 && a.size(0) == out && b.size(0) == out,
+                "convlogic_b200: connection indices must be int64 [out_dim]");
+    return {x_fm.size(0), out, x_fm.size(1)};
+}
+
+void logic_fwd(const Tensor &x_fm, const Tensor &a, const Tensor &b, const Tensor &w, int wmode, const Tensor &y_storage)
+{
+    need_inputs(x_fm, a, b, w);
+    const LogicDims d = logic_dims(x_fm, a, b, w);
+    if (d.batch == 0 || d.out == 0) return;
+    check(clb_logic_fwd(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(y_storage), d.in, d.out, d.batch, wmode, dtype_code(x_fm), stream()));
+}
+
+Tensor logic_bwd_w(const Tensor &x_fm, const Tensor &a, const Tensor &b, const Tensor &w, const Tensor &gy_fm, int wmode, const Tensor &gw_out)
+{
+    need_inputs(x_fm, a, b, w, gy_fm);
+    const LogicDims d = logic_dims(x_fm, a, b, w);
+    Below below(x_fm);
+    Tensor gw = gw_out.defined() ? gw_out : at::empty(w.sizes(), w.options());
+    if (d.batch == 0 || d.out == 0) return gw.zero_();
+    check(clb_logic_bwd_w(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(gy_fm), ptr(gw), d.in, d.out, d.batch, wmode, dtype_code(x_fm),
+                          stream()));
+    return gw;
+}
+
+Tensor logic_bwd_x(const Tensor &x_fm, const Tensor &a, const Tensor &b, const Tensor &w, const Tensor &gy_fm, const Tensor &start, const Tensor &cons,
+                   int wmode)
+{
+    need_inputs(x_fm, a, b, w, gy_fm, start, cons);
+    const LogicDims d = logic_dims(x_fm, a, b, w);
+    TORCH_CHECK(start.scalar_type() == at::kLong && cons.scalar_type() == at::kLong && start.numel() == d.in + 1 && cons.numel() == 2 * d.out,
+                "convlogic_b200: consumer lists must be int64 [in_dim + 1] and [2 * out_dim]");
+    Below below(x_fm);
+    Tensor gx = at::empty(x_fm.sizes(), x_fm.options());
+    if (d.batch == 0) return gx;
+    check(clb_logic_bwd_x(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(gy_fm), ptr(gx), ptr<int64_t>(start), ptr<int64_t>(cons), d.in, d.out,
+                          d.batch, wmode, dtype_code(x_fm), stream()));
+    return gx;
+}
+
+struct LogicNode : public Node {
+    SavedVariable x, a, b, w, start, cons; // x: the feature-major storage the forward read
+    int wmode;
+    bool fm; // the call's own tensors are feature-major ([in, B] -> [out, B])
+    std::string name() const override { return "LogicLayerCudaFunctionBackward"; }
+    void release_variables() override
+    {
+        x.reset_data(), a.reset_data(), b.reset_data(), w.reset_data(), start.reset_data(), cons.reset_data();
+    }
+    variable_list apply(variable_list &&grads) override
+    {
+        if (!grads[0].defined()) return {Tensor(), Tensor()};
+        const Tensor xx = x.unpack(), aa = a.unpack(), bb = b.unpack(), ww = w.unpack();
+        Tensor gx, gw;
+        Below below(xx);
+        const Tensor gy = fm ? grads[0].contiguous() : feature_major(grads[0]);
+        if (task_should_compute_output(0)) {
+            gx = logic_bwd_x(xx, aa, bb, ww, gy, start.unpack(), cons.unpack(), wmode);
+            if (!fm) gx = batch_major_grad(gx, feeds_leaf(*this, 0));
+        }
+        if (task_should_compute_output(1) && wmode != CLB_W_ARGMAX) {
+            Sinks sinks({ww});
+            gw = logic_bwd_w(xx, aa, bb, ww, gy, wmode, sinks.slice(0));
+            if (sinks.any()) {
+                sinks.ready();
+                gw = Tensor();
+            }
+        }
+        return {gx, gw};
+    }
+};
+
+// fm: x [in, B] -> y [out, B] (the reference's Function); else x [B, in] -> y [B, out] on the storage [out, B]
+Tensor logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w_in, const Tensor &start, const Tensor &cons, int wmode, bool fm)
+{
+    const bool graph = wants_grad({x, w_in});
+    Tensor y, x_fm, w;
+    {
+        TORCH_CHECK(x.is_cuda(), "convlogic_b200: tensor must be a CUDA tensor");
+        TORCH_CHECK(x.dim() == 2, "convlogic_b200: x must be 2-D, got ", x.sizes());
+        Below below(x);
+        w = w_in.contiguous();
+        x_fm = fm ? x.contiguous() : feature_major(x);
+        const int64_t out = w.size(0), batch = x_fm.size(1);
+        y = fm ? at::empty({out, batch}, x.options()) : at::empty_strided({batch, out}, {1, std::max<int64_t>(batch, 1)}, x.options());
+        logic_fwd(x_fm, a, b, w, wmode, y);
+    }
+    if (graph) {
+        auto node = new_node<LogicNode>();
+        node->set_next_edges(torch::autograd::collect_next_edges(x, w_in));
+        // the parameter itself is saved (it may carry a gradient sink); its contiguous copy only where it is not contiguous
+        node->x = saved(x_fm), node->a = saved(a), node->b = saved(b), node->w = saved(w_in.is_contiguous() ? w_in : w), node->start = saved(start),
+        node->cons = saved(cons), node->wmode = wmode, node->fm = fm;
+        torch::autograd::set_history(y, node);
+    }
+    return y;
+}
+
+// ------------------------------------------------------------------------------------------------ class sums
+Tensor group_sum_bwd(const Tensor &gout, int64_t f, int k, double tau, const Tensor &scale)
+{
+    need_input(gout);
+    if (scale.defined()) {
+        need_input(scale);
+        TORCH_CHECK(scale.numel() == 1 && scale.scalar_type() == gout.scalar_type(),
+                    "convlogic_b200: `scale` must be a one-element tensor of the gradient's dtype");
+    }
+    Below below(gout);
+    Tensor gy = at::empty({f, gout.size(0)}, gout.options());
+    check(clb_group_sum_bwd_scaled(ptr(gout), ptr(scale), ptr(gy), f, gout.size(0), k, tau, dtype_code(gout), stream()));
+    return gy;
+}
+
+Tensor group_sum_fwd(const Tensor &y_fm, int k, double tau)
+{
+    need_input(y_fm);
+    const int64_t f = y_fm.size(0), b = y_fm.size(1);
+    const int dt = dtype_code(y_fm);
+    Below below(y_fm);
+    Tensor out = at::empty({b, k}, y_fm.options());
+    const size_t bytes = clb_group_sum_scratch_bytes(f, b, k, dt);
+    Tensor scratch = scratch_bytes(bytes, y_fm);
+    check(clb_group_sum_fwd(ptr(y_fm), ptr(out), ptr(scratch), bytes, f, b, k, tau, dt, stream()));
+    return out;
+}
+
+struct GroupSumNode : public Node {
+    int64_t f;
+    int k;
+    double tau;
+    std::string name() const override { return "GroupSumFunctionBackward"; }
+    variable_list apply(variable_list &&grads) override
+    {
+        if (!grads[0].defined()) return {Tensor()};
+        Below below(grads[0]);
+        return {batch_major_grad(group_sum_bwd(grads[0].contiguous(), f, k, tau, Tensor()), feeds_leaf(*this, 0))};
+    }
+};
+
+// x [B, F] on feature-major storage -> [B, k]
+Tensor group_sum(const Tensor &x, int k, double tau)
+{
+    Tensor out;
+    {
+        Below below(x);
+        out = group_sum_fwd(x.t(), k, tau);
+    }
+    if (wants_grad({x})) {
+        auto node = new_node<GroupSumNode>();
+        node->set_next_edges(torch::autograd::collect_next_edges(x));
+        node->f = x.size(1), node->k = k, node->tau = tau;
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+// (loss [1], dscore [B, k], scores [B, k] or undefined)
+std::tuple<Tensor, Tensor, Tensor> group_sum_ce_raw(const Tensor &y_fm, const Tensor &labels, int k, double tau, bool want_scores)
+{
+    need_inputs(y_fm, labels);
+    TORCH_CHECK(y_fm.scalar_type() == at::kFloat && labels.scalar_type() == at::kLong && labels.dim() == 1 && labels.size(0) == y_fm.size(1),
+                "convlogic_b200: group_sum_ce expects float32 [F, B] activations and int64 [B] labels");
+    const int64_t f = y_fm.size(0), b = y_fm.size(1);
+    TORCH_CHECK_VALUE(f % k == 0, "in_dim (", f, ") has to be divisible by k (", k, ") but it is not");
+    Below below(y_fm);
+    Tensor loss = at::empty({1}, y_fm.options()), dscore = at::empty({b, k}, y_fm.options()), scores;
+    if (want_scores) scores = at::empty({b, k}, y_fm.options());
+    const size_t bytes = clb_group_sum_scratch_bytes(f, b, k, CLB_F32);
+    Tensor scratch = scratch_bytes(bytes, y_fm);
+    check(clb_group_sum_ce(ptr<float>(y_fm), ptr<int64_t>(labels), ptr<float>(scores), ptr<float>(dscore), ptr<float>(loss), ptr(scratch), bytes, f, b, k,
+                           tau, stream()));
+    return {loss, dscore, scores};
+}
+
+struct GroupSumCeNode : public Node {
+    Tensor dscore;
+    int64_t f;
+    int k;
+    double tau;
+    std::string name() const override { return "GroupSumCrossEntropyFunctionBackward"; }
+    void release_variables() override { dscore.reset(); }
+    variable_list apply(variable_list &&grads) override
+    {
+        if (!grads[0].defined()) return {Tensor()};
+        TORCH_CHECK(dscore.defined(), "Trying to backward through the graph a second time: specify retain_graph=True the first time");
+        Below below(dscore);
+        const Tensor scale = grads[0].reshape({1}).to(dscore.scalar_type()).contiguous();
+        return {batch_major_grad(group_sum_bwd(dscore, f, k, tau, scale), feeds_leaf(*this, 0))};
+    }
+};
+
+Tensor group_sum_ce(const Tensor &x, const Tensor &labels, int k, double tau)
+{
+    Tensor loss, dscore;
+    {
+        Below below(x);
+        std::tie(loss, dscore, std::ignore) = group_sum_ce_raw(x.t(), labels.contiguous(), k, tau, false);
+        loss = loss.reshape({});
+    }
+    if (wants_grad({x})) {
+        auto node = new_node<GroupSumCeNode>();
+        node->set_next_edges(torch::autograd::collect_next_edges(x));
+        node->dscore = dscore, node->f = x.size(1), node->k = k, node->tau = tau;
+        torch::autograd::set_history(loss, node);
+    }
+    return loss;
+}
+
+// ------------------------------------------------------------------------------------------------ fused flat layers
+struct TreeTables {
+    Tensor leaf, node, start, slots;
+    bool covers_all; // every neuron of the first two layers sits in some tree: gate-gradient buffers need no clearing
+};
+
+void tree_fwd(const Tensor &x_fm, const TreeTables &t, const Tensor &w0, const Tensor &w1, const Tensor &w2, int wmode, const Tensor &y)
+{
+    need_inputs(x_fm, t.leaf, t.node, w0, w1, w2);
+    check(clb_logic_tree_fwd(ptr<float>(x_fm), ptr<int32_t>(t.leaf), ptr<int32_t>(t.node), ptr<float>(w0), ptr<float>(w1), ptr<float>(w2), ptr<float>(y),
+                             t.leaf.size(0), x_fm.size(1), wmode, stream()));
+}
+
+// upstream gradient: gy [T, B], or the head (dscore [B, k], scale [1]) of GroupSum + cross-entropy
+std::array<Tensor, 4> tree_bwd(const Tensor &x_fm, const TreeTables &t, const Tensor &w0, const Tensor &w1, const Tensor &w2, const Tensor &gy,
+                               const Tensor &dscore, const Tensor &scale, int k, double tau, int wmode, bool need_gx, std::array<Tensor, 3> gw)
+{
+    need_inputs(x_fm, t.leaf, t.node, w0, w1, w2, t.start, t.slots);
+    const int64_t trees = t.leaf.size(0), b = x_fm.size(1), in = x_fm.size(0);
+    Below below(x_fm);
+    Tensor tapgrad = at::empty({std::max<int64_t>(trees * 8, 1), b}, x_fm.options());
+    const Tensor *ws[3] = {&w0, &w1, &w2};
+    for (int i = 0; i < 3; ++i) {
+        if (!gw[i].defined()) gw[i] = at::empty(ws[i]->sizes(), ws[i]->options());
+        if (!t.covers_all) gw[i].zero_();
+    }
+    Tensor gx;
+    if (need_gx) gx = at::empty({in, b}, x_fm.options());
+    if (gy.defined()) {
+        need_input(gy);
+        check(clb_logic_tree_bwd(ptr<float>(x_fm), ptr<int32_t>(t.leaf), ptr<int32_t>(t.node), ptr<float>(w0), ptr<float>(w1), ptr<float>(w2),
+                                 ptr<float>(gy), ptr<float>(tapgrad), ptr<float>(gw[0]), ptr<float>(gw[1]), ptr<float>(gw[2]), ptr<float>(gx),
+                                 ptr<int64_t>(t.start), ptr<int32_t>(t.slots), in, trees, b, wmode, stream()));
+    } else {
+        check(clb_logic_tree_bwd_scores(ptr<float>(x_fm), ptr<int32_t>(t.leaf), ptr<int32_t>(t.node), ptr<float>(w0), ptr<float>(w1), ptr<float>(w2),
+                                        ptr<float>(dscore), ptr<float>(scale), k, tau, ptr<float>(tapgrad), ptr<float>(gw[0]), ptr<float>(gw[1]),
+                                        ptr<float>(gw[2]), ptr<float>(gx), ptr<int64_t>(t.start), ptr<int32_t>(t.slots), in, trees, b, wmode, stream()));
+    }
+    return {gx, gw[0], gw[1], gw[2]};
+}
+
+struct TreeNode : public Node {
+    SavedVariable x, w0, w1, w2; // x: feature-major
+    TreeTables t;
+    int wmode;
+    Tensor dscore; // head: GroupSum + cross-entropy
+    int k = 0;
+    double tau = 1.0;
+    std::string name() const override { return k ? "LogicTreeCrossEntropyFunctionBackward" : "LogicTreeFunctionBackward"; }
+    void release_variables() override { x.reset_data(), w0.reset_data(), w1.reset_data(), w2.reset_data(), dscore.reset(); }
+    variable_list apply(variable_list &&grads) override
+    {
+        if (!grads[0].defined()) return variable_list(4);
+        const Tensor xx = x.unpack(), a = w0.unpack(), b = w1.unpack(), c = w2.unpack();
+        Below below(xx);
+        Tensor gy, scale;
+        if (k)
+            scale = grads[0].reshape({1}).to(at::kFloat).contiguous();
+        else
+            gy = feature_major(grads[0]);
+        Sinks sinks({a, b, c});
+        const bool direct = sinks.any() && wmode != CLB_W_ARGMAX;
+        auto out = tree_bwd(xx, t, a, b, c, gy, dscore, scale, k, tau, wmode, task_should_compute_output(0),
+                            direct ? std::array<Tensor, 3>{sinks.slice(0), sinks.slice(1), sinks.slice(2)} : std::array<Tensor, 3>{});
+        Tensor gx = out[0].defined() ? batch_major_grad(out[0], feeds_leaf(*this, 0)) : Tensor();
+        if (direct) sinks.ready();
+        if (direct || wmode == CLB_W_ARGMAX) return {gx, Tensor(), Tensor(), Tensor()};
+        return {gx, out[1], out[2], out[3]};
+    }
+};
+
+// x [B, in] -> [B, T] (k == 0), or with labels the mean cross-entropy of GroupSum(k, tau) over the trees
+Tensor trees(const Tensor &x, const Tensor &w0, const Tensor &w1, const Tensor &w2, const Tensor &leaf, const Tensor &node_t, const Tensor &start,
+             const Tensor &slots, int wmode, bool covers_all, const std::optional<Tensor> &labels_in, int k, double tau)
+{
+    const bool graph = wants_grad({x, w0, w1, w2});
+    const TreeTables t{leaf, node_t, start, slots, covers_all};
+    TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.scalar_type() == at::kFloat, "convlogic_b200: the fused flat layers take float32 [B, in] CUDA tensors");
+    need_inputs(leaf, node_t, w0, w1, w2, start, slots);
+    const int64_t T = leaf.size(0), B = x.size(0);
+    Tensor x_fm, out, dscore;
+    {
+        Below below(x);
+        x_fm = feature_major(x);
+        if (!k) {
+            out = at::empty_strided({B, T}, {1, std::max<int64_t>(B, 1)}, x.options());
+            tree_fwd(x_fm, t, w0, w1, w2, wmode, out);
+        } else {
+            const Tensor labels = labels_in->contiguous();
+            need_input(labels);
+            TORCH_CHECK(labels.scalar_type() == at::kLong && labels.dim() == 1 && labels.size(0) == B, "convlogic_b200: labels must be int64 [B]");
+            const size_t bytes = clb_logic_tree_fwd_ce_scratch_bytes(T, B, k);
+            int rc = CLB_ERR_SHAPE;
+            if (bytes && B % 4 == 0 && B <= 512 && k <= 32) { // class sums without the activation
+                out = at::empty({1}, x.options()), dscore = at::empty({B, k}, x.options());
+                Tensor scratch = scratch_bytes(bytes, x);
+                rc = clb_logic_tree_fwd_ce(ptr<float>(x_fm), ptr<int32_t>(leaf), ptr<int32_t>(node_t), ptr<float>(w0), ptr<float>(w1), ptr<float>(w2),
+                                           ptr<int64_t>(labels), ptr<float>(dscore), ptr<float>(out), ptr(scratch), bytes, T, B, k, tau, wmode, stream());
+                if (rc != CLB_ERR_SHAPE) check(rc);
+            }
+            if (rc == CLB_ERR_SHAPE) {
+                Tensor y = at::empty({T, B}, x.options());
+                tree_fwd(x_fm, t, w0, w1, w2, wmode, y);
+                std::tie(out, dscore, std::ignore) = group_sum_ce_raw(y, labels, k, tau, false);
+            }
+            out = out.reshape({});
+        }
+    }
+    if (graph) {
+        auto node = new_node<TreeNode>();
+        node->set_next_edges(torch::autograd::collect_next_edges(x, w0, w1, w2));
+        node->x = saved(x_fm), node->w0 = saved(w0), node->w1 = saved(w1), node->w2 = saved(w2), node->t = t, node->wmode = wmode;
+        node->dscore = dscore, node->k = k, node->tau = tau;
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+// ------------------------------------------------------------------------------------------------ optimiser
+void adam_step(const Tensor &p, const Tensor &g, const Tensor &m, const Tensor &v, double lr, double beta1, double beta2, double eps, double weight_decay,
+               int64_t step, bool decoupled)
+{
+    need_inputs(p, g, m, v);
+    const int64_t n = p.numel();
+    for (const Tensor *t : {&p, &g, &m, &v})
+        TORCH_CHECK(t->numel() == n && t->scalar_type() == at::kFloat, "convlogic_b200: adam_step expects four float32 buffers of equal size");
+    c10::cuda::CUDAGuard device(p.device());
+    check(clb_adam_step(ptr<float>(p), ptr<float>(g), ptr<float>(m), ptr<float>(v), n, lr, beta1, beta2, eps, weight_decay, step, decoupled, stream()));
+}
+
+// ------------------------------------------------------------------------------------------------ packed inference
+at::ScalarType word_type(int bits)
+{
+    TORCH_CHECK_VALUE(bits == 8 || bits == 16 || bits == 32 || bits == 64, "`bit_count` has to be in { 8, 16, 32, 64 }");
+    return bits == 8 ? at::kChar : bits == 16 ? at::kShort : bits == 32 ? at::kInt : at::kLong;
+}
+
+std::pair<Tensor, int64_t> pack_bits(const Tensor &t, int bits, bool sample_major)
+{
+    const at::ScalarType type = word_type(bits);
+    need_input(t);
+    TORCH_CHECK(t.dim() == 2 && (t.scalar_type() == at::kBool || t.scalar_type() == at::kByte), "convlogic_b200: pack_bits expects a bool or uint8 tensor");
+    const int64_t b = t.size(sample_major ? 0 : 1), f = t.size(sample_major ? 1 : 0);
+    Below below(t);
+    Tensor packed = at::empty({f, (b + bits - 1) / bits}, t.options().dtype(type));
+    check(sample_major ? clb_pack_bits_nmajor(ptr<uint8_t>(t), ptr(packed), b, f, bits, stream()) : clb_pack_bits(ptr<uint8_t>(t), ptr(packed), f, b, bits, stream()));
+    return {packed, (bits - b % bits) % bits};
+}
+
+Tensor packed_logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &ops)
+{
+    need_inputs(x, a, b, ops);
+    TORCH_CHECK(ops.scalar_type() == at::kByte, "convlogic_b200: gate ids must be uint8");
+    Below below(x);
+    Tensor y = at::empty({ops.size(0), x.size(1)}, x.options());
+    check(clb_packed_logic(ptr(x), ptr<int64_t>(a), ptr<int64_t>(b), ptr<uint8_t>(ops), ptr(y), x.size(0), ops.size(0), x.size(1), (int)x.element_size() * 8,
+                           stream()));
+    return y;
+}
+
+Tensor group_popcount(const Tensor &x, int64_t pad, int k)
+{
+    need_input(x);
+    const int64_t f = x.size(0), words = x.size(1), bits = x.element_size() * 8;
+    TORCH_CHECK_VALUE(f % k == 0, "in_dim (", f, ") has to be divisible by k (", k, ") but it is not");
+    Below below(x);
+    Tensor counts = at::empty({words * bits - pad, k}, x.options().dtype(at::kInt));
+    check(clb_group_popcount(ptr(x), ptr<int32_t>(counts), f, words, (int)bits, (int)pad, k, stream()));
+    return counts;
+}
+
+// A compiled network on one device: the handle and the device copy of its parameters.  The workspace of a call comes from
+// torch's caching allocator, so calls on several streams or threads do not share one.
+class Net {
+public:
+    Net(const py::bytes &blob, const c10::Device &device)
+        : device_(device.has_index() ? device : c10::Device(c10::kCUDA, c10::cuda::current_device()))
+    {
+        TORCH_CHECK(device.is_cuda(), "convlogic_b200: a compiled network runs on a CUDA device, got ", device.str());
+        const std::string_view data(blob);
+        size_t need = 0;
+        check(clb_net_device_bytes(data.data(), data.size(), &need));
+        c10::cuda::CUDAGuard guard(device_);
+        params_ = at::empty({(int64_t)(need < 16 ? 16 : need)}, at::TensorOptions().dtype(at::kByte).device(device_));
+        check(clb_net_create(data.data(), data.size(), ptr(params_), stream(), &net_));
+        c10::cuda::getCurrentCUDAStream().synchronize(); // the blob is pageable host memory: wait for the copy
+        check(clb_net_info(net_, &features, &classes, &layers));
+    }
+    Net(const Net &) = delete;
+    ~Net() { clb_net_destroy(net_); }
+    Tensor run(int kind, const Tensor &x, const std::optional<Tensor> &thresholds, int64_t batch) const
+    {
+        need_input(x);
+        Below below(params_);
+        const size_t bytes = clb_net_workspace_bytes(net_, batch);
+        Tensor workspace = scratch_bytes(bytes, params_);
+        Tensor counts = at::empty({batch, classes}, params_.options().dtype(at::kInt));
+        check(clb_net_forward(net_, kind, ptr(x), thresholds ? ptr<float>(*thresholds) : nullptr, thresholds ? (int)thresholds->numel() : 0, batch,
+                              ptr<int32_t>(counts), ptr(workspace), bytes, stream()));
+        return counts;
+    }
+    int64_t features = 0;
+    int classes = 0, layers = 0;
+
+private:
+    c10::Device device_;
+    Tensor params_;
+    clb_net *net_ = nullptr;
+};
+
+// raw forward / backward of the fused block for callers that handle autograd themselves
+py::tuple block_fwd_py(const Tensor &x, const Tensor &w, py::object sel_obj, const std::array<int, 6> &geom, int wmode, bool want_amax, bool want_inter,
+                       bool want_idx, bool y_fm)
+{
+    const Tensor sel = sel_obj.cast<Tensor>();
+    const Geom g{geom[0], geom[1], geom[2], geom[3], geom[4], geom[5]};
+    BlockOut o = block_fwd(x, w, sel, g, [&] { return plan_for(sel_obj, sel, g, x.size(1)); }, wmode, want_amax, want_inter, want_idx, y_fm);
+    auto opt = [](const Tensor &t) { return t.defined() ? py::cast(t) : py::object(py::none()); };
+    return py::make_tuple(o.y, opt(o.amax), opt(o.x2), opt(o.x3), opt(o.idx));
+}
+py::tuple block_bwd_py(const Tensor &gy, const Tensor &x, const Tensor &w, py::object sel_obj, const std::optional<Tensor> &amax,
+                       const std::array<int, 6> &geom, int wmode, bool need_gx, bool need_gw, const std::optional<Tensor> &gw_out)
+{
+    const Tensor sel = sel_obj.cast<Tensor>();
+    const Geom g{geom[0], geom[1], geom[2], geom[3], geom[4], geom[5]};
+    auto out = block_bwd(gy, x, w, sel, amax.value_or(Tensor()), g, [&] { return plan_for(sel_obj, sel, g, x.size(1)); }, wmode, need_gx, need_gw,
+                         gw_out.value_or(Tensor()));
+    auto opt = [](const Tensor &t) { return t.defined() ? py::cast(t) : py::object(py::none()); };
+    return py::make_tuple(opt(out.first), opt(out.second));
+}
+
+Tensor logic_fwd_py(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w, int wmode)
+{
+    Below below(x);
+    Tensor y = at::empty({w.size(0), x.size(1)}, x.options());
+    logic_fwd(x, a, b, w, wmode, y);
+    return y;
+}
+
+} // namespace
+
+PYBIND11_MODULE(_clb_torch, m)
+{
+    py::class_<BlockPlan, PlanPtr>(m, "BlockPlan");
+    m.def("block", &block);
+    m.def("block_fwd", &block_fwd_py);
+    m.def("block_bwd", &block_bwd_py);
+    m.def("is_feature_major", &is_feature_major);
+    m.def("logic", &logic);
+    m.def("logic_fwd", &logic_fwd_py);
+    m.def("logic_bwd_w", [](const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w, const Tensor &gy, int wmode, const std::optional<Tensor> &out) {
+        return logic_bwd_w(x, a, b, w, gy, wmode, out.value_or(Tensor()));
+    });
+    m.def("logic_bwd_x", &logic_bwd_x);
+    m.def("group_sum", &group_sum);
+    m.def("group_sum_ce", &group_sum_ce);
+    m.def("trees", &trees);
+    m.def("transpose2d", &transpose2d);
+    m.def("adam_step", &adam_step);
+    m.def("pack_bits", &pack_bits);
+    m.def("packed_logic", &packed_logic);
+    m.def("group_popcount", &group_popcount);
+    py::class_<Net>(m, "Net")
+        .def(py::init([](const py::bytes &blob, const std::string &device) { return std::make_unique<Net>(blob, c10::Device(device)); }))
+        .def("run", &Net::run)
+        .def_readonly("features", &Net::features)
+        .def_readonly("classes", &Net::classes)
+        .def_readonly("layers", &Net::layers);
+}

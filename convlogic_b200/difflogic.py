@@ -9,10 +9,8 @@ loop (same result, seconds instead of minutes for million-neuron layers).
 
 import torch
 
-from . import ops
-from ._lib import W_ARGMAX, W_SOFTMAX
-from .functional import (GradFactor, GroupSumCrossEntropyFunction, GroupSumFunction, LogicLayerCudaFunction,
-                         LogicTreeCrossEntropyFunction, LogicTreeFunction, to_feature_major)
+from ._lib import W_ARGMAX, W_SOFTMAX, native
+from .functional import GradFactor
 from .packbitstensor import PackBitsTensor
 
 
@@ -89,14 +87,16 @@ class LogicLayer(torch.nn.Module):
     def forward_cuda(self, x):
         assert x.is_cuda, f"x must be a CUDA tensor, got device: {x.device}"
         assert x.ndim == 2, x.ndim
-        x = to_feature_major(x)  # free when x came from another LogicLayer
-        assert x.shape[0] == self.in_dim, (x.shape, self.in_dim)
-        w = self.weights if self.weights.dtype == x.dtype else self.weights.to(x.dtype)
-        args = (x, self.indices_0, self.indices_1, w, self.given_x_indices_of_y_start, self.given_x_indices_of_y)
+        assert x.shape[1] == self.in_dim, (x.shape, self.in_dim)
+        w, buf = self._parameters["weights"], self._buffers
+        if w.dtype != x.dtype:
+            w = w.to(x.dtype)
+        # [B, in] -> [B, out]; the result is a view of feature-major storage, which the next flat layer reads without a copy
+        args = (buf["indices_0"], buf["indices_1"], w, buf["given_x_indices_of_y_start"], buf["given_x_indices_of_y"])
         if self.training:
-            return LogicLayerCudaFunction.apply(*args, W_SOFTMAX).transpose(0, 1)
+            return native().logic(x, *args, W_SOFTMAX, False)
         with torch.no_grad():
-            return LogicLayerCudaFunction.apply(*args, W_ARGMAX).transpose(0, 1)
+            return native().logic(x, *args, W_ARGMAX, False)
 
     def forward_cuda_eval(self, x: PackBitsTensor):
         """Packed inference; returns a new PackBitsTensor (the reference rebinds ``x.t``)."""
@@ -104,8 +104,7 @@ class LogicLayer(torch.nn.Module):
         t = x.rows()
         t = t.reshape(-1, t.shape[-1])
         assert t.shape[0] == self.in_dim, (tuple(t.shape), self.in_dim)
-        gate_ids = self._gate_ids()
-        y = ops.packed_logic(t, self.indices_0, self.indices_1, gate_ids)
+        y = native().packed_logic(t, self._buffers["indices_0"], self._buffers["indices_1"], self._gate_ids())
         return PackBitsTensor.from_packed(y, x.pad_len)
 
     def _gate_ids(self):
@@ -155,7 +154,7 @@ class GroupSum(torch.nn.Module):
         assert x.shape[-1] % self.k == 0, (x.shape, self.k)
         if x.is_cuda and x.dim() == 2 and x.dtype in (torch.float32, torch.float64) and x.numel() and x.t().is_contiguous():
             # the transposed view a LogicLayer returns: sum its feature-major storage directly
-            return GroupSumFunction.apply(x.t(), self.k, self.tau)
+            return native().group_sum(x, self.k, self.tau)
         return x.reshape(*x.shape[:-1], self.k, x.shape[-1] // self.k).sum(-1) / self.tau
 
     def extra_repr(self):
@@ -176,7 +175,7 @@ class GroupSumCrossEntropy(torch.nn.Module):
         assert x.shape[-1] % self.k == 0, (x.shape, self.k)
         if (x.is_cuda and x.dim() == 2 and x.dtype == torch.float32 and x.numel() and x.t().is_contiguous() and self.k <= 32
                 and labels.dtype == torch.int64):
-            return GroupSumCrossEntropyFunction.apply(x.t(), labels, self.k, self.tau)
+            return native().group_sum_ce(x, labels, self.k, self.tau)
         scores = x.reshape(*x.shape[:-1], self.k, x.shape[-1] // self.k).sum(-1) / self.tau
         return torch.nn.functional.cross_entropy(scores, labels)
 
@@ -234,14 +233,15 @@ class FusedLogicLayers(torch.nn.Module):
                 x = layer(x)
             return x
         assert x.shape[1] == first.in_dim, (x.shape, first.in_dim)
-        x_fm = to_feature_major(x)
-        w = [l.weights for l in self.layers]
         if self.training:
-            y = LogicTreeFunction.apply(x_fm, w[0], w[1], w[2], self.leaf, self.node, self.leaf_start, self.leaf_slots, W_SOFTMAX, self.covers_all)
-        else:
-            with torch.no_grad():
-                y = LogicTreeFunction.apply(x_fm, w[0], w[1], w[2], self.leaf, self.node, self.leaf_start, self.leaf_slots, W_ARGMAX, self.covers_all)
-        return y.transpose(0, 1)
+            return self._trees(x, W_SOFTMAX, None, 0, 1.0)
+        with torch.no_grad():
+            return self._trees(x, W_ARGMAX, None, 0, 1.0)
+
+    def _trees(self, x, wmode, labels, k, tau):
+        buf = self._buffers
+        w = [l._parameters["weights"].contiguous() for l in self.layers]
+        return native().trees(x, *w, buf["leaf"], buf["node"], buf["leaf_start"], buf["leaf_slots"], wmode, self.covers_all, labels, k, tau)
 
     def cross_entropy(self, x, labels, k, tau=1.0):
         """``cross_entropy(GroupSum(k, tau)(self(x)), labels)`` of a training step as one autograd node: same loss and
@@ -254,9 +254,7 @@ class FusedLogicLayers(torch.nn.Module):
         if not fused:
             return GroupSumCrossEntropy(k, tau)(self(x), labels)
         assert x.shape[1] == self.layers[0].in_dim, (x.shape, self.layers[0].in_dim)
-        w = [l.weights for l in self.layers]
-        return LogicTreeCrossEntropyFunction.apply(to_feature_major(x), w[0], w[1], w[2], self.leaf, self.node, self.leaf_start,
-                                                   self.leaf_slots, labels, k, float(tau), self.covers_all)
+        return self._trees(x, W_SOFTMAX, labels, k, float(tau))
 
     def extra_repr(self):
         return f"{self.in_dim} -> {' -> '.join(str(l.out_dim) for l in self.layers)}"

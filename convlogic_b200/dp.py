@@ -200,8 +200,9 @@ class FlatAdam:
     trains with: src/convlogic/model.py:179-180) to fp32 rounding."""
 
     def __init__(self, bucket, lr=1e-3, betas=(0.9, 0.999), eps=1e-8, weight_decay=0.0, decoupled=False):
-        from . import ops  # noqa: F401  (needs the CUDA library)
+        from ._lib import native
 
+        self._adam_step = native().adam_step
         self.bucket, self.lr, self.betas, self.eps, self.weight_decay, self.decoupled = bucket, lr, betas, eps, weight_decay, decoupled
         self.params = torch.empty_like(bucket.flat)
         for p, (lo, hi) in zip(bucket.params, bucket.ranges):
@@ -217,11 +218,9 @@ class FlatAdam:
         self.bucket.zero()
 
     def _update(self, lo, hi):
-        from . import ops
-
         if hi > lo:
-            ops.adam_step(self.params[lo:hi], self.bucket.flat[lo:hi], self.exp_avg[lo:hi], self.exp_avg_sq[lo:hi], self.lr, self.betas[0],
-                          self.betas[1], self.eps, self.weight_decay, self.steps, self.decoupled)
+            self._adam_step(self.params[lo:hi], self.bucket.flat[lo:hi], self.exp_avg[lo:hi], self.exp_avg_sq[lo:hi], self.lr,
+                            self.betas[0], self.betas[1], self.eps, self.weight_decay, self.steps, bool(self.decoupled))
 
     def step(self):
         if not self.bucket._direct:

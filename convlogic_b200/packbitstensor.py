@@ -14,6 +14,7 @@ import numpy as np
 import torch
 
 from . import ops
+from ._lib import native
 
 
 class PackBitsTensor:
@@ -64,7 +65,7 @@ class PackBitsTensor:
 
     def group_sum(self, k):
         t = self.rows()
-        return ops.group_popcount(t.reshape(-1, t.shape[-1]), self.pad_len, k)
+        return native().group_popcount(t.reshape(-1, t.shape[-1]), self.pad_len, k)
 
     def flatten(self, start_dim=0, end_dim=-1, **kwargs):
         """Returns the tensor itself viewed as [features, words]; arguments are ignored."""
