@@ -23,6 +23,7 @@ Y_FEATURE_MAJOR = 0x200   # wmode flag: the block's output / upstream gradient i
 TUNE_TAPGRAD_SLICE_BYTES = 1
 TUNE_PLANE_KERNELS = 2
 TUNE_SLAB_MUX = 3
+TUNE_NET_ONE_LAUNCH = 4
 ERR_SHAPE, ERR_ODD_OUTPUT, ERR_TOO_LARGE = -2, -5, -6
 
 _lib = None

@@ -173,10 +173,10 @@ class CompiledLogicNet(torch.nn.Module):
         self.num_inputs, self.num_classes, self.num_layers = self._net.features, self._net.classes, self._net.layers
 
     # ---- inference
-    def _run(self, kind, x, batch, thresholds=None):
+    def _handle(self):
         if self._net is None:
             raise RuntimeError("convlogic_b200: call compile() or load() first")
-        return self._net.run(kind, x, thresholds, batch)
+        return self._net
 
     # ---- CUDA graph replay for a fixed batch size (the runtime allocates nothing and never synchronises)
     def capture(self, example, thresholds=None):
@@ -185,8 +185,7 @@ class CompiledLogicNet(torch.nn.Module):
         static buffer, the graph is launched, and the static int32 ``[B, num_classes]`` result is returned (valid
         until the next replay).  Worth it for small networks, where a call is a dozen launches of a few
         microseconds each."""
-        if self._net is None:
-            raise RuntimeError("convlogic_b200: call compile() or load() first")
+        net = self._handle()
         pixels = thresholds is not None
         static_in = example.to(self.device).contiguous().clone()
         th = thresholds.to(self.device, torch.float32).contiguous() if pixels else None
@@ -198,11 +197,11 @@ class CompiledLogicNet(torch.nn.Module):
         side.wait_stream(torch.cuda.current_stream(self.device))
         with torch.cuda.stream(side):                      # warm-up outside the capture: shared-memory attributes, workspace
             for _ in range(2):
-                self._run(kind, static_in, batch, th)
+                net.run(kind, static_in, th, batch)
         torch.cuda.current_stream(self.device).wait_stream(side)
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
-            static_out = self._run(kind, static_in, batch, th)
+            static_out = net.run(kind, static_in, th, batch)
 
         def replay(x):
             x = x.to(self.device)
@@ -218,14 +217,7 @@ class CompiledLogicNet(torch.nn.Module):
         del verbose
         if isinstance(x, np.ndarray):
             x = torch.from_numpy(x)
-        x = x.to(self.device)
-        if x.dtype not in (torch.bool, torch.uint8):
-            raise RuntimeError("convlogic_b200: CompiledLogicNet.forward expects bool inputs")
-        batch = x.shape[0]
-        x = x.reshape(batch, -1).contiguous()
-        if x.shape[1] != self.num_inputs:
-            raise ValueError(f"expected {self.num_inputs} input bits per sample, got {x.shape[1]}")
-        return self._run(0, x.view(torch.uint8), batch)
+        return self._handle().forward(x)
 
     def forward_packed(self, rows, batch):
         """Bit-packed input rows ``[in_features, 2 * ceil(batch / 128)]`` int64 (64 samples per word, the batch padded
@@ -234,12 +226,8 @@ class CompiledLogicNet(torch.nn.Module):
         words = 2 * (-(-batch // 128))
         if rows.dtype != torch.int64 or rows.dim() != 2 or rows.shape[0] != self.num_inputs or rows.shape[1] != words:
             raise ValueError(f"expected int64 rows [{self.num_inputs}, {words}], got {tuple(rows.shape)} {rows.dtype}")
-        return self._run(3, rows, batch)
+        return self._handle().run(3, rows, None, batch)
 
     def forward_pixels(self, pixels, thresholds):
         """float32 / uint8 pixels ``[B, C, H, W]`` + thermometer thresholds -> counts (input stage fused on the GPU)."""
-        pixels = pixels.to(self.device).contiguous()
-        thresholds = thresholds.to(self.device, torch.float32).contiguous()
-        if pixels.dtype not in (torch.float32, torch.uint8):
-            raise RuntimeError("convlogic_b200: pixels must be float32 or uint8")
-        return self._run(2 if pixels.dtype == torch.uint8 else 1, pixels, pixels.shape[0], thresholds)
+        return self._handle().pixels(pixels, thresholds)

@@ -61,6 +61,7 @@ namespace {
 std::atomic<long long> g_tapgrad_slice_bytes{0};
 std::atomic<long long> g_plane_kernels{1};
 std::atomic<long long> g_slab_mux{0};
+std::atomic<long long> g_net_one_launch{1};
 std::atomic<int> g_sm_count[64];
 } // namespace
 
@@ -70,6 +71,7 @@ long long tune_get(int key)
     if (key == CLB_TUNE_TAPGRAD_SLICE_BYTES) return g_tapgrad_slice_bytes.load(std::memory_order_relaxed);
     if (key == CLB_TUNE_PLANE_KERNELS) return g_plane_kernels.load(std::memory_order_relaxed);
     if (key == CLB_TUNE_SLAB_MUX) return g_slab_mux.load(std::memory_order_relaxed);
+    if (key == CLB_TUNE_NET_ONE_LAUNCH) return g_net_one_launch.load(std::memory_order_relaxed);
     return -1;
 }
 int sm_count()
@@ -126,6 +128,10 @@ extern "C" int clb_tune(int key, long long value)
     }
     if (key == CLB_TUNE_SLAB_MUX && (value == 0 || value == 1)) {
         g_slab_mux.store(value, std::memory_order_relaxed);
+        return CLB_OK;
+    }
+    if (key == CLB_TUNE_NET_ONE_LAUNCH && value >= 0 && value <= 2) {
+        g_net_one_launch.store(value, std::memory_order_relaxed);
         return CLB_OK;
     }
     if (key == CLB_TUNE_PLANE_KERNELS && (value == 0 || value == 1)) {

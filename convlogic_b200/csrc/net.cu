@@ -16,6 +16,7 @@
 //   arrays
 // The last flat layer's outputs are summed per class (GroupSum): counts[b][k].
 #include "clb_common.cuh"
+#include "clb_net.cuh"
 
 #include <cstring>
 #include <new>
@@ -27,6 +28,11 @@ namespace {
 
 constexpr char kMagic[8] = {'C', 'L', 'B', 'N', 'E', 'T', '0', '1'};
 constexpr size_t kHeaderBytes = 64, kLayerBytes = 64;
+// The one-launch kernel (net_cluster.cu) against layer-by-layer launches, us per call on B200: mnist k=16 batch 1 15.5 / 74.5,
+// batch 4096 25.9 / 82.5; cifar k=32 batch 1000 44 / 84, batch 8192 132 / 217; cifar k=128 (cost 0.5 M) batch 1 68 / 101, batch
+// 8192 469 / 513; cifar k=256 (cost 1 M) batch 1 136 / 107, batch 8192 1104 / 912.  Beyond one slab per SM the clusters come in waves
+// and the layered kernels win from k=32 on (batch 20000: 507 / 468).
+constexpr long long kOneLaunchCost = 600000;
 
 struct Header {
     char magic[8];
@@ -59,7 +65,13 @@ struct clb_net {
     size_t param_bytes = 0;    // the blob is copied to the device as it is
     const unsigned char *dev = nullptr;
     size_t max_conv_channels = 0;
+    clb::NetPlan plan = {};     // for the one-launch kernel
+    bool one_launch = false;    // the stack has the form that kernel takes
+    long long slab_cost = 0;    // gate trees per 128-sample slab, a conv window counting as four
 };
+
+int clb_net_cluster_launch(const clb::NetPlan &net, const void *input, const float *thresholds, const unsigned char *params, void *work,
+                           int32_t *counts, int64_t batch, cudaStream_t st); // net_cluster.cu
 
 static bool parse(const void *blob, size_t bytes, clb_net &net)
 {
@@ -147,6 +159,63 @@ static bool parse(const void *blob, size_t bytes, clb_net &net)
     return feat % net.num_classes == 0;
 }
 
+// The layout of a slab for the one-launch kernel: conv blocks first, at least one flat layer last, sizes that 32-bit unit
+// indices cover.
+static void plan_one_launch(clb_net &net)
+{
+    const size_t n = net.layers.size();
+    if (n > (size_t)clb::kNetMaxLayers || net.layers.back().kind == 1) return;
+    clb::NetPlan &P = net.plan;
+    P.n_layers = (int)n, P.classes = net.num_classes, P.in_features = net.in_features;
+    long long units = 0;
+    auto store = [&](size_t i, long long channels, int rows, int W, int ph, int pw) {
+        clb::NetStorage &st = P.store[i];
+        const long long image = (long long)rows * W, pitch = W + 2 * pw, per = (rows + 2LL * ph) * pitch;
+        if (units + channels * per > (1 << 24)) return false;
+        st.base = (int)units, st.W = W, st.image = (int)image, st.pitch = (int)pitch, st.per_channel = (int)per, st.rows = rows, st.ph = ph, st.pw = pw;
+        st.halo_units = ph || pw ? (int)(channels * per) : 0;
+        if (channels > 1 && channels * per * per >= (1LL << 32)) return false; // the kernel's divisions
+        st.by_image = clb::FastDiv::of((unsigned)image), st.by_W = clb::FastDiv::of((unsigned)W);
+        st.by_pitch = clb::FastDiv::of((unsigned)pitch), st.by_channel = clb::FastDiv::of((unsigned)per);
+        units += (channels * per + 7) / 8 * 8;
+        return true;
+    };
+    auto flat_store = [&](size_t i, long long features) { return features <= (1 << 24) && store(i, 1, 1, (int)features, 0, 0); };
+    const Layer &first = net.layers.front();
+    if (!(net.in_channels > 0 ? store(0, net.in_channels, net.in_h, net.in_w, first.kind == 1 ? first.ph : 0, first.kind == 1 ? first.pw : 0)
+                              : flat_store(0, net.in_features)))
+        return;
+    for (size_t i = 0; i < n; ++i) {
+        const Layer &L = net.layers[i];
+        clb::NetLayer &o = P.layer[i];
+        o.kind = L.kind, o.C = L.C, o.stride = L.stride, o.Hp = L.Hp, o.Wp = L.Wp, o.levels = L.levels;
+        o.off_a = L.off_a, o.off_b = L.off_b, o.off_ops = L.off_ops;
+        if (L.kind == 1) {
+            const Layer &next = net.layers[i + 1];
+            const bool conv = next.kind == 1;
+            if (!store(i + 1, L.C, L.Hp, L.Wp, conv ? next.ph : 0, conv ? next.pw : 0)) return;
+            o.by_windows = clb::FastDiv::of((unsigned)(L.Hp * L.Wp)), o.by_Wp = clb::FastDiv::of((unsigned)L.Wp);
+            net.slab_cost += 4LL * L.C * L.Hp * L.Wp;
+        } else {
+            if (L.out_dim > (1 << 24)) return;
+            o.out_dim = (int)L.out_dim;
+            if (i + 1 < n && !flat_store(i + 1, L.out_dim)) return;
+            net.slab_cost += L.out_dim;
+        }
+    }
+    P.slab_units = units;
+    net.one_launch = true;
+}
+
+// When the one-launch kernel is used: small stacks (a slab is one cluster's work) and at most a slab per SM, see kOneLaunchCost.
+static bool use_one_launch(const clb_net *net, int input_kind, int64_t batch)
+{
+    if (!net->one_launch || input_kind == 3 || tune_get(CLB_TUNE_NET_ONE_LAUNCH) == 0) return false;
+    const long long slabs = (batch + 127) / 128;
+    if (slabs * net->plan.slab_units > (1LL << 27)) return false; // 2 GB of activations
+    return tune_get(CLB_TUNE_NET_ONE_LAUNCH) == 2 || (net->slab_cost <= kOneLaunchCost && slabs <= sm_count());
+}
+
 extern "C" int clb_net_device_bytes(const void *blob, size_t bytes, size_t *device_bytes)
 {
     clb_net tmp;
@@ -171,6 +240,7 @@ extern "C" int clb_net_create(const void *blob, size_t bytes, void *device_mem, 
         return check_launch(0);
     }
     net->dev = (const unsigned char *)device_mem;
+    plan_one_launch(*net);
     *out = net;
     return CLB_OK;
 }
@@ -205,7 +275,9 @@ extern "C" size_t clb_net_workspace_bytes(const clb_net *net, int64_t batch)
 {
     if (!net || batch <= 0) return 0;
     const size_t act = align256(widest(net) * row_bytes(batch));
-    return 2 * act + align256((size_t)clb_packed_convtree_slab_scratch_bytes((int)net->max_conv_channels)) + 256;
+    const size_t layers = 2 * act + align256((size_t)clb_packed_convtree_slab_scratch_bytes((int)net->max_conv_channels)) + 256;
+    const size_t slabs = use_one_launch(net, 0, batch) ? (size_t)((batch + 127) / 128) * (size_t)net->plan.slab_units * 16 : 0;
+    return slabs > layers ? slabs : layers;
 }
 
 // input_kind: 0 = bool / uint8 bits [batch][in_features]; 1 = float32 pixels, 2 = uint8 pixels [batch][pc][H*W] with
@@ -216,6 +288,12 @@ extern "C" int clb_net_forward(const clb_net *net, int input_kind, const void *i
     if (!net || !input || !counts || !workspace || batch <= 0 || input_kind < 0 || input_kind > 3) return CLB_ERR_ARG;
     if ((reinterpret_cast<uintptr_t>(workspace) & 255)) return CLB_ERR_ARG;
     if (workspace_bytes < clb_net_workspace_bytes(net, batch)) return CLB_ERR_SCRATCH;
+    if (use_one_launch(net, input_kind, batch) && levels <= clb::kNetMaxLevels) {
+        if (input_kind != 0 && (net->in_channels <= 0 || !thresholds || levels <= 0 || net->in_channels % levels)) return CLB_ERR_SHAPE;
+        clb::NetPlan plan = net->plan;
+        plan.input_kind = input_kind, plan.levels = levels;
+        return clb_net_cluster_launch(plan, input, thresholds, net->dev, workspace, counts, batch, (cudaStream_t)stream);
+    }
     const size_t rb = row_bytes(batch);
     const int64_t words = (int64_t)(rb / 8), U = (int64_t)(rb / 16);
     const size_t act = align256(widest(net) * rb);

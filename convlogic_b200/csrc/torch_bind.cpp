@@ -850,6 +850,21 @@ public:
     }
     Net(const Net &) = delete;
     ~Net() { clb_net_destroy(net_); }
+    // bool / uint8 bits [B, ...] -> counts
+    Tensor forward(const Tensor &x_in) const
+    {
+        TORCH_CHECK(x_in.scalar_type() == at::kBool || x_in.scalar_type() == at::kByte, "convlogic_b200: CompiledLogicNet.forward expects bool inputs");
+        const int64_t batch = x_in.size(0), bits = batch ? x_in.numel() / batch : features;
+        TORCH_CHECK_VALUE(bits == features, "expected ", features, " input bits per sample, got ", bits);
+        return run(0, x_in.device() == device_ ? x_in.contiguous() : x_in.to(device_).contiguous(), std::nullopt, batch);
+    }
+    // float32 / uint8 pixels [B, C, H, W] and thermometer thresholds -> counts
+    Tensor pixels(const Tensor &x_in, const Tensor &thresholds) const
+    {
+        const Tensor x = x_in.device() == device_ ? x_in.contiguous() : x_in.to(device_).contiguous();
+        TORCH_CHECK(x.scalar_type() == at::kFloat || x.scalar_type() == at::kByte, "convlogic_b200: pixels must be float32 or uint8");
+        return run(x.scalar_type() == at::kByte ? 2 : 1, x, thresholds.to(device_, at::kFloat).contiguous(), x.size(0));
+    }
     Tensor run(int kind, const Tensor &x, const std::optional<Tensor> &thresholds, int64_t batch) const
     {
         need_input(x);
@@ -925,6 +940,8 @@ PYBIND11_MODULE(_clb_torch, m)
     py::class_<Net>(m, "Net")
         .def(py::init([](const py::bytes &blob, const std::string &device) { return std::make_unique<Net>(blob, c10::Device(device)); }))
         .def("run", &Net::run)
+        .def("forward", &Net::forward)
+        .def("pixels", &Net::pixels)
         .def_readonly("features", &Net::features)
         .def_readonly("classes", &Net::classes)
         .def_readonly("layers", &Net::layers);

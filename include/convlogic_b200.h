@@ -90,6 +90,9 @@ long long clb_trace_report(char *buf, size_t cap);
 /*   CLB_TUNE_SLAB_MUX  how the packed ConvLogic block on the slab layout applies a gate to its words: 0 = a block-uniform
  *       16-way switch with one lop3 per word, 1 = a branch-free multiplexer over four masks, three lop3 per word. */
 #define CLB_TUNE_SLAB_MUX 3
+/*   CLB_TUNE_NET_ONE_LAUNCH  clb_net_forward runs a whole network in one launch, a thread-block cluster per 128 samples:
+ *       1 (default) for small networks and batches, where launches bind; 0 never; 2 whenever the network has that form. */
+#define CLB_TUNE_NET_ONE_LAUNCH 4
 int clb_tune(int key, long long value);
 long long clb_tune_get(int key);
 
