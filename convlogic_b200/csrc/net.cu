@@ -70,6 +70,7 @@ struct clb_net {
     long long slab_cost = 0;    // gate trees per 128-sample slab, a conv window counting as four
 };
 
+int clb_pack_bits_units(const uint8_t *t, void *packed, int64_t N, int64_t F, int64_t U, int64_t HW, cudaStream_t st); // packed.cu
 int clb_net_cluster_launch(const clb::NetPlan &net, const void *input, const float *thresholds, const unsigned char *params, void *work,
                            int32_t *counts, int64_t batch, cudaStream_t st); // net_cluster.cu
 
@@ -308,24 +309,8 @@ extern "C" int clb_net_forward(const clb_net *net, int input_kind, const void *i
 
     // ---- input stage
     if (input_kind == 0) {
-        if ((batch + 63) / 64 != words) { // pack_bits writes ceil(batch/64) words per row: clear the padding word first
-            if (cudaMemsetAsync(buf[0], 0, (size_t)net->in_features * rb, (cudaStream_t)stream) != cudaSuccess) return check_launch(0);
-            // rows of `words` words cannot be produced by a kernel that strides ceil(batch/64): pack into buf[1], then widen
-            st = clb_pack_bits_nmajor((const uint8_t *)input, buf[1], batch, net->in_features, 64, stream);
-            if (st != CLB_OK) return st;
-            const size_t narrow = (size_t)((batch + 63) / 64) * 8;
-            if (cudaMemcpy2DAsync(buf[0], rb, buf[1], narrow, narrow, (size_t)net->in_features, cudaMemcpyDeviceToDevice,
-                                  (cudaStream_t)stream) != cudaSuccess)
-                return check_launch(0);
-        } else {
-            st = clb_pack_bits_nmajor((const uint8_t *)input, buf[0], batch, net->in_features, 64, stream);
-            if (st != CLB_OK) return st;
-        }
-        if (slab) {
-            st = clb_packed_layout(buf[0], buf[1], net->in_channels, (int64_t)net->in_h * net->in_w, U, 1, stream);
-            if (st != CLB_OK) return st;
-            cur = 1;
-        }
+        st = clb_pack_bits_units((const uint8_t *)input, buf[0], batch, net->in_features, U, slab ? (int64_t)net->in_h * net->in_w : 0, (cudaStream_t)stream);
+        if (st != CLB_OK) return st;
     } else if (input_kind == 1 || input_kind == 2) {
         if (!image || !thresholds || levels <= 0 || net->in_channels % levels) return CLB_ERR_SHAPE;
         st = clb_thermometer_pack(input, input_kind == 2, thresholds, levels, buf[0], batch, net->in_channels / levels,

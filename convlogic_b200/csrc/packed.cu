@@ -4,13 +4,15 @@
 // little-endian machine that is the same as a row of ceil(B/bits)*bits/8 BYTES with sample s in bit
 // (s & 7) of byte (s >> 3), whatever `bits` is; bitwise gates do not care about the word width either.
 // The kernels therefore see rows of bytes and move them in the widest unit the row length and the
-// pointers allow (8 bytes when the row length is a multiple of 8 and the bases are 8-byte aligned,
-// single bytes otherwise); `bits` only fixes how many pad samples a row ends with.
+// pointers allow (16, 8 or 4 bytes; rows of any other length as 4-byte words shifted into place);
+// `bits` only fixes how many pad samples a row ends with.
 //
 // A 2-input gate with truth table (f00, f01, f10, f11), given as four all-ones/all-zero masks, is the
 // two-level multiplexer  y = a ? (b ? m11 : m10) : (b ? m01 : m00): three 3-input logic operations per
 // 32 bits, branch-free, with the masks uniform over the thread block.
 #include "clb_common.cuh"
+
+#include <type_traits>
 
 namespace clb {
 
@@ -50,34 +52,76 @@ __global__ void pack_bits_kernel(const uint8_t *__restrict__ t, uint8_t *__restr
     }
 }
 
-// sample-major source t [N,F]: thread <-> feature, loops over 8*BY samples and writes BY bytes of its row.
-template <int BY>
-__global__ void __launch_bounds__(256) pack_bits_nmajor_kernel(const uint8_t *__restrict__ t, uint8_t *__restrict__ out, long long N,
-                                                               long long F, long long rowbytes)
+// sample-major source t [N, F]: the transpose and the packing in one pass.  Block: 128 features x 256 samples, warp w the
+// samples 32w..32w+31, lane l the features 4l..4l+3 of the block: a load is four features of one sample (one 32-bit word when F
+// and t allow it), and eight samples' words, each byte 0 or 1, shifted by the sample's number and OR-ed are the eight-sample
+// bytes of four features at once.  The words leave through shared memory, so that every row receives 32 contiguous bytes
+// (rows layout, words beyond the row cut off) or every (channel, slab) 16 bytes per position (slab layout).
+// Bound by the bytes read (a feature per thread, one byte per load, took 68 us for 30.7 MB; this takes 9).
+__device__ __forceinline__ unsigned nonzero_bytes(unsigned v) { return ((((v & 0x7f7f7f7fu) + 0x7f7f7f7fu) | v) >> 7) & 0x01010101u; }
+
+template <bool QUAD>
+__global__ void __launch_bounds__(256) pack_bits_nmajor_kernel(const uint8_t *__restrict__ t, uint8_t *__restrict__ out, long long N, long long F,
+                                                               long long rowbytes, int word_stores, int HW, long long U)
 {
-    const long long f = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= F) return;
-    for (long long q0 = (long long)blockIdx.y * BY; q0 < rowbytes; q0 += (long long)gridDim.y * BY) {
-        uint8_t bytes[BY];
+    __shared__ unsigned sm[128 * 9];
+    const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
+    const long long f0 = (long long)blockIdx.x * 128, f = f0 + 4 * lane;
+    for (long long n0 = (long long)blockIdx.y * 256; n0 < rowbytes * 8; n0 += (long long)gridDim.y * 256) {
+        const long long nb = n0 + wv * 32;
+        const int live = (int)max(0LL, min(32LL, N - nb));
+        const uint8_t *src = t + nb * F + f;
+        unsigned g[4] = {0u, 0u, 0u, 0u}; // byte k of g[q]: samples 8q..8q+7 of feature f + k
+        if (f < F) {
 #pragma unroll
-        for (int q = 0; q < BY; ++q) {
-            unsigned v = 0;
+            for (int q = 0; q < 4; ++q) {
+                unsigned v[8];
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const long long n = (q0 + q) * 8 + k;
-                if (n < N) v |= (__ldg(t + n * F + f) != 0 ? 1u : 0u) << k;
+                for (int j = 0; j < 8; ++j) {
+                    v[j] = 0u;
+                    if (8 * q + j < live) {
+                        const uint8_t *p = src + (8 * q + j) * F;
+                        if (QUAD) {
+                            v[j] = __ldg(reinterpret_cast<const unsigned *>(p));
+                        } else {
+#pragma unroll
+                            for (int k = 0; k < 4; ++k)
+                                if (f + k < F) v[j] |= (unsigned)__ldg(p + k) << (8 * k);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 8; ++j) g[q] |= nonzero_bytes(v[j]) << j;
             }
-            bytes[q] = (uint8_t)v;
         }
-        uint8_t *dst = out + f * rowbytes + q0;
-        if (BY == 32 && q0 + BY <= rowbytes && ((reinterpret_cast<uintptr_t>(dst) & 15) == 0)) {
-            const uint4 *b4 = reinterpret_cast<const uint4 *>(bytes);
-            reinterpret_cast<uint4 *>(dst)[0] = b4[0];
-            reinterpret_cast<uint4 *>(dst)[1] = b4[1];
-        } else {
+        __syncthreads(); // the previous pass has been written out
 #pragma unroll
-            for (int q = 0; q < BY; ++q)
-                if (q0 + q < rowbytes) dst[q] = bytes[q];
+        for (int k = 0; k < 4; ++k) {
+            const unsigned lo = __byte_perm(g[0], g[1], 0x40 + 0x11 * k), hi = __byte_perm(g[2], g[3], 0x40 + 0x11 * k);
+            sm[(4 * lane + k) * 9 + wv] = (lo & 0xffffu) | (hi << 16);
+        }
+        __syncthreads();
+        if (HW > 0) { // slab layout [channel][U][HW] of 16-byte units
+            for (int e = threadIdx.x; e < 1024; e += 256) {
+                const int q = e & 3, i = (e >> 2) & 127, h = e >> 9;
+                const long long u = n0 / 128 + h, ff = f0 + i;
+                if (ff < F && u < U) {
+                    const long long c = ff / HW;
+                    reinterpret_cast<unsigned *>(out)[((c * U + u) * HW + (ff - c * HW)) * 4 + q] = sm[i * 9 + 4 * h + q];
+                }
+            }
+        } else if (word_stores) {
+            for (int e = threadIdx.x; e < 1024; e += 256) {
+                const int w = e & 7, i = e >> 3;
+                const long long at = n0 / 8 + 4 * w;
+                if (f0 + i < F && at < rowbytes) *reinterpret_cast<unsigned *>(out + (f0 + i) * rowbytes + at) = sm[i * 9 + w];
+            }
+        } else {
+            for (int e = threadIdx.x; e < 4096; e += 256) {
+                const int y = e & 31, i = e >> 5;
+                const long long at = n0 / 8 + y;
+                if (f0 + i < F && at < rowbytes) out[(f0 + i) * rowbytes + at] = (uint8_t)(sm[i * 9 + (y >> 2)] >> (8 * (y & 3)));
+            }
         }
     }
 }
@@ -200,44 +244,88 @@ __global__ void __launch_bounds__(256) thermometer_pack_kernel(const PIX *__rest
 }
 
 // ----------------------------------------------------------------------------------- flat layer
-// U = transfer unit; units = units per row.  thread <-> (neuron, unit), unit fastest.
-template <typename U>
-__global__ void __launch_bounds__(256) packed_logic_kernel(const U *__restrict__ x, const int64_t *__restrict__ ia,
-                                                           const int64_t *__restrict__ ib, const uint8_t *__restrict__ ops,
-                                                           U *__restrict__ y, long long out_dim, long long units)
+template <typename V> struct Words { // a transfer unit as 32-bit words
+    static constexpr int N = sizeof(V) / 4;
+    unsigned w[N];
+};
+template <typename V> __device__ __forceinline__ Words<V> load_words(const V *p)
 {
-    // (neuron, unit) of the thread's items by carried additions: one 64-bit division per thread, none per item
-    const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
-    const long long dj = stride / units, du = stride - dj * units;
-    long long j = i0 / units, u = i0 - j * units;
-    for (long long i = i0; j < out_dim; i += stride, j += dj, u += du) {
-        if (u >= units) u -= units, ++j;
-        if (j >= out_dim) break;
-        const OpMasks<U> m = op_masks<U>(ops[j]);
-        y[i] = op_apply<U>(m, x[ia[j] * units + u], x[ib[j] * units + u]);
+    const V v = __ldg(p);
+    Words<V> r;
+    const unsigned *q = reinterpret_cast<const unsigned *>(&v);
+#pragma unroll
+    for (int i = 0; i < Words<V>::N; ++i) r.w[i] = q[i];
+    return r;
+}
+
+// Rows of `units` units of type V (4, 8 or 16 bytes).  A group of 2^lg lanes (the power of two that covers a row, at most a
+// warp) owns a neuron at a time: its indices and gate are read once, the next neuron's one neuron ahead, and its row is walked
+// with R units per lane in flight.  Bound by L2: two gathered rows in, one out.
+template <typename V, int R>
+__global__ void __launch_bounds__(256) packed_logic_kernel(const V *__restrict__ x, const int64_t *__restrict__ ia, const int64_t *__restrict__ ib,
+                                                           const uint8_t *__restrict__ ops, V *__restrict__ y, long long out_dim, int units, int lg)
+{
+    const long long first = ((long long)blockIdx.x * 256 + threadIdx.x) >> lg, step = ((long long)gridDim.x * 256) >> lg;
+    const int g = 1 << lg, l = threadIdx.x & (g - 1);
+    long long a = 0, b = 0;
+    int op = 0;
+    if (first < out_dim) a = __ldg(ia + first), b = __ldg(ib + first), op = __ldg(ops + first);
+    for (long long j = first; j < out_dim; j += step) {
+        const V *xa = x + a * units, *xb = x + b * units;
+        V *yo = y + j * units;
+        const OpMasks<unsigned> m = op_masks<unsigned>(op);
+        const long long jn = j + step;
+        if (jn < out_dim) a = __ldg(ia + jn), b = __ldg(ib + jn), op = __ldg(ops + jn);
+        for (int u0 = l; u0 < units; u0 += g * R) {
+            Words<V> va[R], vb[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (u0 + r * g < units) va[r] = load_words(xa + u0 + r * g), vb[r] = load_words(xb + u0 + r * g);
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (u0 + r * g < units) {
+                    V o;
+                    unsigned *q = reinterpret_cast<unsigned *>(&o);
+#pragma unroll
+                    for (int i = 0; i < Words<V>::N; ++i) q[i] = op_apply<unsigned>(m, va[r].w[i], vb[r].w[i]);
+                    yo[u0 + r * g] = o;
+                }
+        }
     }
 }
 
-// 16-byte variant: one thread moves a uint4 (two 64-bit units) per operand.
-__global__ void __launch_bounds__(256) packed_logic_v4_kernel(const uint4 *__restrict__ x, const int64_t *__restrict__ ia,
-                                                              const int64_t *__restrict__ ib, const uint8_t *__restrict__ ops,
-                                                              uint4 *__restrict__ y, long long out_dim, long long units)
+// Rows whose length is no multiple of four bytes, so that a neuron's two input rows and its output row start anywhere: the
+// output is written in aligned 32-bit words, each input word put together from the two aligned words it straddles; up to three
+// bytes at either end of a row go one by one.  The same split as above.
+__global__ void __launch_bounds__(256) packed_logic_bytes_kernel(const uint8_t *__restrict__ x, const int64_t *__restrict__ ia, const int64_t *__restrict__ ib,
+                                                                 const uint8_t *__restrict__ ops, uint8_t *__restrict__ y, long long out_dim, int rowbytes,
+                                                                 int lg)
 {
-    // (neuron, unit) of the thread's items by carried additions: one 64-bit division per thread, none per item
-    const long long i0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
-    const long long dj = stride / units, du = stride - dj * units;
-    long long j = i0 / units, u = i0 - j * units;
-    for (long long i = i0; j < out_dim; i += stride, j += dj, u += du) {
-        if (u >= units) u -= units, ++j;
-        if (j >= out_dim) break;
-        const OpMasks<unsigned> m = op_masks<unsigned>(ops[j]);
-        const uint4 a = __ldg(x + ia[j] * units + u), b = __ldg(x + ib[j] * units + u);
-        uint4 r;
-        r.x = op_apply<unsigned>(m, a.x, b.x);
-        r.y = op_apply<unsigned>(m, a.y, b.y);
-        r.z = op_apply<unsigned>(m, a.z, b.z);
-        r.w = op_apply<unsigned>(m, a.w, b.w);
-        y[i] = r;
+    const long long first = ((long long)blockIdx.x * 256 + threadIdx.x) >> lg, step = ((long long)gridDim.x * 256) >> lg;
+    const int g = 1 << lg, l = threadIdx.x & (g - 1);
+    for (long long j = first; j < out_dim; j += step) {
+        const uint8_t *xa = x + __ldg(ia + j) * rowbytes, *xb = x + __ldg(ib + j) * rowbytes;
+        uint8_t *yo = y + j * rowbytes;
+        const OpMasks<unsigned> m = op_masks<unsigned>(__ldg(ops + j));
+        const int head = min(rowbytes, (int)(-reinterpret_cast<uintptr_t>(yo) & 3)), words = (rowbytes - head) >> 2, tail = rowbytes - head - 4 * words;
+        auto word_at = [](const uint8_t *p, int w) { // bytes 4w..4w+3 from p on
+            const unsigned *q = reinterpret_cast<const unsigned *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3) + w;
+            const unsigned sh = 8 * (unsigned)(reinterpret_cast<uintptr_t>(p) & 3), lo = __ldg(q);
+            return sh ? __funnelshift_r(lo, __ldg(q + 1), sh) : lo; // the second word holds bytes of the row whenever it is read
+        };
+        for (int w0 = l; w0 < words; w0 += 4 * g) {
+            unsigned va[4], vb[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (w0 + r * g < words) va[r] = word_at(xa + head, w0 + r * g), vb[r] = word_at(xb + head, w0 + r * g);
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (w0 + r * g < words) reinterpret_cast<unsigned *>(yo + head)[w0 + r * g] = op_apply<unsigned>(m, va[r], vb[r]);
+        }
+        for (int e = l; e < head + tail; e += g) {
+            const int at = e < head ? e : 4 * words + e;
+            yo[at] = (uint8_t)op_apply<unsigned>(m, __ldg(xa + at), __ldg(xb + at));
+        }
     }
 }
 
@@ -291,11 +379,12 @@ __global__ void __launch_bounds__(256) packed_tree_kernel(const V4 *__restrict__
 }
 
 // ----------------------------------------------------------------------------------- group sum
-// x rows as 32-bit units (32 samples each).  thread <-> (class, row split, unit).  Rows are added 16 at
-// a time into bit-sliced counters (carry-save adders: ones, twos, fours, eights + ripple counter for
-// the sixteens), so a row costs a handful of logic operations per 32 samples; the per-sample integers
-// are only extracted once at the end.  With more than one row split the partial counts are combined
-// with integer atomics (exact, order-independent) into a zeroed output.
+// x rows as 32-bit units (32 samples each).  Block (32 units, part of a class's rows, class): lane <-> unit, the eight warps
+// share the rows of the part.  Rows are added 16 at a time into bit-sliced counters (carry-save adders: ones, twos, fours,
+// eights + ripple counter for the sixteens), so a row costs a handful of logic operations per 32 samples; the eight warps' counters
+// are added in bit-sliced form through shared memory, and only then are the per-sample integers extracted, four of a unit's 32
+// by each warp.  With more than one part they are combined with integer atomics (exact, order-independent) into a zeroed
+// output: per part, not per thread (a thread's 32 atomics were most of the kernel: 50 us for 80 MB).
 __device__ __forceinline__ void csa(unsigned &hi, unsigned &lo, unsigned a, unsigned b, unsigned c)
 {
     const unsigned u = a ^ b;
@@ -303,25 +392,22 @@ __device__ __forceinline__ void csa(unsigned &hi, unsigned &lo, unsigned a, unsi
     lo = u ^ c;
 }
 
-// PLANES bit planes above the sixteens: a thread can count 16 * 2^PLANES rows (8 planes when its share of the rows
-// allows it: the ripple through the planes is most of the work per 16 rows)
+// PLANES bit planes above the sixteens: a warp can count 16 * 2^PLANES rows, and so can the sum of the eight warps
 template <int PLANES>
-__global__ void __launch_bounds__(128) group_popcount_kernel(const unsigned *__restrict__ x, int *__restrict__ counts, long long S,
-                                                             long long units, long long B, int k, int splits)
+__global__ void __launch_bounds__(256) group_popcount_kernel(const unsigned *__restrict__ x, int *__restrict__ counts, long long S, long long units, long long B,
+                                                             int k)
 {
-    const long long total = (long long)k * splits * units;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const long long u = i % units;
-        const int sp = (int)((i / units) % splits);
-        const int cls = (int)(i / (units * splits));
-        const long long per = ((S + splits - 1) / splits + 15) / 16 * 16;
-        const long long r_lo = per * sp, r_hi = min(S, r_lo + per);
-        const unsigned *base = x + ((long long)cls * S) * units + u;
-        unsigned ones = 0, twos = 0, fours = 0, eights = 0;
-        unsigned up[PLANES];
+    constexpr int P = PLANES + 4;
+    __shared__ unsigned sm[4][P][32];
+    const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
+    const long long u = (long long)blockIdx.x * 32 + lane;
+    const int cls = blockIdx.z, parts = gridDim.y, sp = blockIdx.y * 8 + wv;
+    const long long r_lo = S * sp / (8LL * parts), r_hi = S * (sp + 1) / (8LL * parts);
+    unsigned n[P]; // plane p: bit p of the counts
 #pragma unroll
-        for (int p = 0; p < PLANES; ++p) up[p] = 0;
-        const unsigned *pr = base + r_lo * units; // walks down the rows: one addition per load, no multiplication
+    for (int p = 0; p < P; ++p) n[p] = 0;
+    if (u < units) {
+        const unsigned *pr = x + ((long long)cls * S + r_lo) * units + u; // walks down the rows: one addition per load, no multiplication
         for (long long r = r_lo; r < r_hi; r += 16) {
             unsigned v[16];
             if (r + 16 <= r_hi) {
@@ -331,43 +417,65 @@ __global__ void __launch_bounds__(128) group_popcount_kernel(const unsigned *__r
 #pragma unroll
                 for (int q = 0; q < 16; ++q) v[q] = (r + q < r_hi) ? __ldg(pr + q * units) : 0u;
             }
-            unsigned t2a, t2b, t4a, t4b, t8a, t8b, t16;
-            csa(t2a, ones, ones, v[0], v[1]);
-            csa(t2b, ones, ones, v[2], v[3]);
-            csa(t4a, twos, twos, t2a, t2b);
-            csa(t2a, ones, ones, v[4], v[5]);
-            csa(t2b, ones, ones, v[6], v[7]);
-            csa(t4b, twos, twos, t2a, t2b);
-            csa(t8a, fours, fours, t4a, t4b);
-            csa(t2a, ones, ones, v[8], v[9]);
-            csa(t2b, ones, ones, v[10], v[11]);
-            csa(t4a, twos, twos, t2a, t2b);
-            csa(t2a, ones, ones, v[12], v[13]);
-            csa(t2b, ones, ones, v[14], v[15]);
-            csa(t4b, twos, twos, t2a, t2b);
-            csa(t8b, fours, fours, t4a, t4b);
-            csa(t16, eights, eights, t8a, t8b);
-            // ripple the sixteens into the upper counter
-            unsigned carry = t16;
+            unsigned t2a, t2b, t4a, t4b, t8a, t8b, carry;
+            csa(t2a, n[0], n[0], v[0], v[1]);
+            csa(t2b, n[0], n[0], v[2], v[3]);
+            csa(t4a, n[1], n[1], t2a, t2b);
+            csa(t2a, n[0], n[0], v[4], v[5]);
+            csa(t2b, n[0], n[0], v[6], v[7]);
+            csa(t4b, n[1], n[1], t2a, t2b);
+            csa(t8a, n[2], n[2], t4a, t4b);
+            csa(t2a, n[0], n[0], v[8], v[9]);
+            csa(t2b, n[0], n[0], v[10], v[11]);
+            csa(t4a, n[1], n[1], t2a, t2b);
+            csa(t2a, n[0], n[0], v[12], v[13]);
+            csa(t2b, n[0], n[0], v[14], v[15]);
+            csa(t4b, n[1], n[1], t2a, t2b);
+            csa(t8b, n[2], n[2], t4a, t4b);
+            csa(carry, n[3], n[3], t8a, t8b);
 #pragma unroll
-            for (int p = 0; p < PLANES; ++p) {
-                const unsigned nc = up[p] & carry;
-                up[p] ^= carry;
-                carry = nc;
+            for (int p = 4; p < P; ++p) { // ripple the sixteens into the upper planes
+                const unsigned c = n[p] & carry;
+                n[p] ^= carry;
+                carry = c;
             }
         }
-#pragma unroll 1
-        for (int bit = 0; bit < 32; ++bit) {
-            const long long s = u * 32 + bit;
-            if (s >= B) break;
-            int c = ((ones >> bit) & 1) + 2 * ((twos >> bit) & 1) + 4 * ((fours >> bit) & 1) + 8 * ((eights >> bit) & 1);
+    }
 #pragma unroll
-            for (int p = 0; p < PLANES; ++p) c += (int)((up[p] >> bit) & 1u) << (4 + p);
-            if (splits == 1)
-                counts[s * k + cls] = c;
-            else if (c)
-                atomicAdd(counts + s * k + cls, c);
+    for (int half = 4; half >= 1; half >>= 1) { // warps [half, 2 half) hand their counters to warps [0, half)
+        if (wv >= half && wv < 2 * half)
+#pragma unroll
+            for (int p = 0; p < P; ++p) sm[wv - half][p][lane] = n[p];
+        __syncthreads();
+        if (wv < half) {
+            unsigned carry = 0u;
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                unsigned c;
+                csa(c, n[p], n[p], sm[wv][p][lane], carry);
+                carry = c;
+            }
         }
+        __syncthreads();
+    }
+    if (wv == 0)
+#pragma unroll
+        for (int p = 0; p < P; ++p) sm[0][p][lane] = n[p];
+    __syncthreads();
+    if (u >= units) return;
+#pragma unroll
+    for (int p = 0; p < P; ++p) n[p] = sm[0][p][lane] >> (4 * wv);
+#pragma unroll
+    for (int bit = 0; bit < 4; ++bit) {
+        const long long s = u * 32 + 4 * wv + bit;
+        int c = 0;
+#pragma unroll
+        for (int p = 0; p < P; ++p) c += (int)((n[p] >> bit) & 1u) << p;
+        if (s >= B) continue;
+        if (parts == 1)
+            counts[s * k + cls] = c;
+        else if (c)
+            atomicAdd(counts + s * k + cls, c);
     }
 }
 
@@ -828,16 +936,32 @@ extern "C" int clb_pack_bits(const uint8_t *t, void *packed, int64_t F, int64_t 
     return check_launch();
 }
 
+// rows of `rowbytes` bytes (HW == 0) or the slab layout [F / HW][U][HW] of 16-byte units
+static int pack_nmajor(const uint8_t *t, void *packed, int64_t N, int64_t F, int64_t rowbytes, int64_t HW, int64_t U, cudaStream_t st)
+{
+    long long gy = (rowbytes + 31) / 32;
+    if (gy > 4096) gy = 4096;
+    const dim3 grid((unsigned)((F + 127) / 128), (unsigned)gy);
+    const int words = rowbytes % 4 == 0 && aligned_to(packed, 4);
+    if (F % 4 == 0 && aligned_to(t, 4))
+        CLB_TRACED("pack_bits_nmajor_kernel", st, pack_bits_nmajor_kernel<true><<<grid, 256, 0, st>>>(t, (uint8_t *)packed, N, F, rowbytes, words, (int)HW, U));
+    else
+        CLB_TRACED("pack_bits_nmajor_kernel", st, pack_bits_nmajor_kernel<false><<<grid, 256, 0, st>>>(t, (uint8_t *)packed, N, F, rowbytes, words, (int)HW, U));
+    return check_launch();
+}
+
 extern "C" int clb_pack_bits_nmajor(const uint8_t *t, void *packed, int64_t N, int64_t F, int bits, void *stream)
 {
     if (!t || !packed || F < 0 || N < 0 || !bits_ok(bits)) return CLB_ERR_ARG;
     const long long words = (N + bits - 1) / bits, rowbytes = words * (bits / 8);
     if (F == 0 || rowbytes == 0) return CLB_OK;
-    long long gy = (rowbytes + 31) / 32;
-    if (gy > 4096) gy = 4096;
-    dim3 grid((unsigned)((F + 255) / 256), (unsigned)gy);
-    CLB_TRACED("pack_bits_nmajor_kernel", (cudaStream_t)stream, pack_bits_nmajor_kernel<32><<<grid, 256, 0, (cudaStream_t)stream>>>(t, (uint8_t *)packed, N, F, rowbytes));
-    return check_launch();
+    return pack_nmajor(t, packed, N, F, rowbytes, 0, 0, (cudaStream_t)stream);
+}
+
+// The same with the batch padded to U units of 128 samples (zero bits): rows of U units, or with HW > 0 the slab layout.
+int clb_pack_bits_units(const uint8_t *t, void *packed, int64_t N, int64_t F, int64_t U, int64_t HW, cudaStream_t st)
+{
+    return pack_nmajor(t, packed, N, F, U * 16, HW, U, st);
 }
 
 extern "C" int clb_thermometer_pack(const void *pixels, int pixels_u8, const float *thresholds, int levels, void *packed, int64_t N,
@@ -872,17 +996,34 @@ extern "C" int clb_packed_logic(const void *x, const int64_t *a, const int64_t *
     if (!x || !a || !b || !ops || !y || in_dim <= 0 || out_dim < 0 || words < 0 || !bits_ok(bits)) return CLB_ERR_ARG;
     const long long rowbytes = words * (bits / 8);
     if (out_dim == 0 || rowbytes == 0) return CLB_OK;
+    if (rowbytes > 0x7fffffffLL) return CLB_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
+    auto group = [](long long units) { // log2 of the lanes per neuron
+        int lg = 0;
+        while (lg < 5 && (1LL << lg) < units) ++lg;
+        return lg;
+    };
+    auto blocks = [&](int lg) { // eight resident blocks per SM walk the neurons
+        const long long want = ((out_dim << lg) + 255) / 256, cap = (long long)sm_count() * 8;
+        return (unsigned)(want < cap ? want : cap);
+    };
+    auto go = [&](auto unit, auto rounds) {
+        using V = decltype(unit);
+        const long long units = rowbytes / (long long)sizeof(V);
+        const int lg = group(units);
+        CLB_TRACED("packed_logic_kernel", st,
+                   packed_logic_kernel<V, decltype(rounds)::value><<<blocks(lg), 256, 0, st>>>((const V *)x, a, b, ops, (V *)y, out_dim, (int)units, lg));
+    };
     if (rowbytes % 16 == 0 && aligned_to(x, 16) && aligned_to(y, 16)) {
-        const long long units = rowbytes / 16;
-        CLB_TRACED("packed_logic_v4_kernel", st, packed_logic_v4_kernel<<<flat_grid(out_dim * units, 256), 256, 0, st>>>((const uint4 *)x, a, b, ops, (uint4 *)y, out_dim, units));
+        go(uint4{}, std::integral_constant<int, 2>{});
     } else if (rowbytes % 8 == 0 && aligned_to(x, 8) && aligned_to(y, 8)) {
-        const long long units = rowbytes / 8;
-        CLB_TRACED("packed_logic_kernel", st, packed_logic_kernel<unsigned long long><<<flat_grid(out_dim * units, 256), 256, 0, st>>>(
-            (const unsigned long long *)x, a, b, ops, (unsigned long long *)y, out_dim, units));
+        go(uint2{}, std::integral_constant<int, 4>{});
+    } else if (rowbytes % 4 == 0 && aligned_to(x, 4) && aligned_to(y, 4)) {
+        go(0u, std::integral_constant<int, 5>{});
     } else {
-        CLB_TRACED("packed_logic_kernel", st, packed_logic_kernel<uint8_t><<<flat_grid(out_dim * rowbytes, 256), 256, 0, st>>>((const uint8_t *)x, a, b, ops, (uint8_t *)y,
-                                                                                        out_dim, rowbytes));
+        const int lg = group((rowbytes + 3) / 4);
+        CLB_TRACED("packed_logic_bytes_kernel", st,
+                   packed_logic_bytes_kernel<<<blocks(lg), 256, 0, st>>>((const uint8_t *)x, a, b, ops, (uint8_t *)y, out_dim, (int)rowbytes, lg));
     }
     return check_launch();
 }
@@ -942,19 +1083,24 @@ extern "C" int clb_group_popcount(const void *x, int32_t *counts, int64_t F, int
     const long long S = F / k;
     cudaStream_t st = (cudaStream_t)stream;
     if (rowbytes % 4 == 0 && aligned_to(x, 4)) {
-        const long long units = rowbytes / 4;
-        long long splits = 1;
-        while ((long long)k * splits * units < (long long)sm_count() * 128 * 16 && S / (splits * 2) >= 64) splits *= 2; // 16 resident blocks per SM: the row loop is latency-bound
-        if (splits > 1) {
-            if (cudaMemsetAsync(counts, 0, (size_t)B * k * sizeof(int32_t), st) != cudaSuccess) return check_launch();
-        }
-        const long long per = ((S + splits - 1) / splits + 15) / 16 * 16; // rows per thread, as the kernel computes it
-        if (per <= 16 * 256)
-            CLB_TRACED("group_popcount_kernel", st, group_popcount_kernel<8><<<flat_grid((long long)k * splits * units, 128), 128, 0, st>>>((const unsigned *)x, counts, S, units, B, k,
-                                                                                                    (int)splits));
+        const long long units = rowbytes / 4, ublocks = (units + 31) / 32;
+        // parts of a class: four blocks per SM in all, at least 16 rows per warp
+        long long parts = 1;
+        while (ublocks * k * parts < (long long)sm_count() * 4 && S / (parts * 2) >= 128) parts *= 2;
+        if (ublocks > 0x7fffffffLL || k > 65535) return CLB_ERR_SHAPE;
+        if (parts > 1 && cudaMemsetAsync(counts, 0, (size_t)B * k * sizeof(int32_t), st) != cudaSuccess) return check_launch(0);
+        const dim3 grid((unsigned)ublocks, (unsigned)parts, (unsigned)k);
+        const long long rows = S / parts + 1; // of a block: what its counters have to hold
+        auto go = [&](auto planes) {
+            CLB_TRACED("group_popcount_kernel", st,
+                       group_popcount_kernel<decltype(planes)::value><<<grid, 256, 0, st>>>((const unsigned *)x, counts, S, units, B, k));
+        };
+        if (rows < (1LL << 12))
+            go(std::integral_constant<int, 8>{});
+        else if (rows < (1LL << 20))
+            go(std::integral_constant<int, 16>{});
         else
-            CLB_TRACED("group_popcount_kernel", st, group_popcount_kernel<27><<<flat_grid((long long)k * splits * units, 128), 128, 0, st>>>((const unsigned *)x, counts, S, units, B,
-                                                                                                     k, (int)splits));
+            go(std::integral_constant<int, 27>{});
     } else {
         CLB_TRACED("group_popcount_bytes_kernel", st, group_popcount_bytes_kernel<<<flat_grid(B * k, 256), 256, 0, st>>>((const uint8_t *)x, counts, S, rowbytes, B, k));
     }

@@ -1,0 +1,53 @@
+"""Packing, flat layer and class counts on rows of every alignment, against the CPU oracle: batches around the 32-sample words,
+the 256-sample tiles and the widths at which the number of lanes per neuron changes; feature counts around the 128-feature tiles."""
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("bits", [8, 16, 32, 64])
+@pytest.mark.parametrize("batch,features", [(1, 1), (7, 131), (33, 4), (129, 127), (256, 128), (257, 132), (1000, 37), (4104, 12), (2056, 9)])
+def test_pack_logic_count_at_row_edges(bits, batch, features):
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    g = torch.Generator().manual_seed(batch * 7 + bits)
+    x = torch.rand(batch, features, generator=g) < 0.5
+    packed, pad = _lib.native().pack_bits(x.cuda(), bits, True)
+    want, want_pad = oracle.pack_bits(x.T.numpy(), bits)
+    assert pad == want_pad and np.array_equal(packed.cpu().numpy().view(want.dtype), want)
+    out = 530
+    a, b = torch.randint(0, features, (out,), generator=g), torch.randint(0, features, (out,), generator=g)
+    ops = torch.randint(0, 16, (out,), generator=g, dtype=torch.uint8)
+    y = _lib.native().packed_logic(packed, a.cuda(), b.cuda(), ops.cuda())
+    # truth-table bit of gate g for inputs (a, b): bit 3 - (2a + b)
+    av, bv = x[:, a].long(), x[:, b].long()
+    bit = (ops.long() >> (3 - (2 * av + bv))) & 1
+    assert np.array_equal(y.cpu().numpy().view(want.dtype)[:, : want.shape[1]], oracle.pack_bits(bit.bool().T.numpy(), bits)[0] | _pad_bits(ops, want, batch, bits))
+    counts = cb.PackBitsTensor.from_packed(y, pad).group_sum(10)
+    assert torch.equal(counts.cpu().long(), bit.reshape(batch, 10, out // 10).sum(-1))
+
+
+def _pad_bits(ops, like, batch, bits):
+    """What a gate makes of the zero pad samples: f(0, 0)."""
+    words = like.shape[1]
+    mask = np.zeros((1, words), dtype=np.uint64)
+    if batch % bits:
+        mask[0, -1] = ((1 << bits) - 1) & ~((1 << (batch % bits)) - 1)
+    on = ((ops.numpy() >> 3) & 1).astype(np.uint64)[:, None]
+    return (on * mask).astype(np.uint64).astype(f"uint{bits}").view(like.dtype)
+
+
+@pytest.mark.parametrize("rows_per_class", [1, 15, 128, 4096, 40000])
+def test_class_counts_over_many_rows(rows_per_class):
+    from convlogic_b200 import _lib
+
+    x = torch.randint(-2**31, 2**31 - 1, (3 * rows_per_class, 33), device="cuda", dtype=torch.int32)
+    want = torch.stack([(x.view(3, rows_per_class, 33).long() >> s) & 1 for s in range(32)], -1).sum(1)   # [3, 33, 32]
+    got = _lib.native().group_popcount(x, 5, 3)
+    assert torch.equal(got.long(), want.reshape(3, -1).t()[: 33 * 32 - 5])
