@@ -13,102 +13,18 @@
 // derivative (the reference kernel, src/difflogic/cuda/difflogic_kernel.cu:196-226, applies the
 // first-input derivative twice in that case; its CPU path gives the sum used here).
 #include "clb_common.cuh"
+#include "clb_logic.cuh"
 
 #include <cmath>
 
 namespace clb {
 
-// Each half-warp reduces the 16 values of one neuron: the lane handles value (lane & 15) of neuron
-// `j` (the same j in all 16 lanes of a half-warp; the two halves may name unrelated neurons).
-// Returns that neuron's gate in every lane of the half-warp, plus the lane's mixture value p.
-// Neurons outside [0, out_dim) give zeros.
-template <typename T>
-__device__ __forceinline__ Gate<T> half_warp_gate(const T *__restrict__ w, long long j, long long out_dim, int wmode, int lane, T &p)
-{
-    const int i = lane & 15;
-    T v = (j >= 0 && j < out_dim) ? w[j * 16 + i] : T(0);
-    if (wmode == CLB_W_SOFTMAX) {
-        T m = v;
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
-            const T u = __shfl_xor_sync(0xffffffffu, m, o);
-            m = u > m ? u : m;
-        }
-        v = exp(v - m);
-        T s = v;
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        v = v / s;
-    } else if (wmode == CLB_W_ARGMAX) {
-        // first maximum: compare (value, -index) pairs
-        T m = v;
-        int bi = i;
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) {
-            const T um = __shfl_xor_sync(0xffffffffu, m, o);
-            const int ui = __shfl_xor_sync(0xffffffffu, bi, o);
-            if (um > m || (um == m && ui < bi)) {
-                m = um;
-                bi = ui;
-            }
-        }
-        v = (i == bi) ? T(1) : T(0);
-    }
-    p = v;
-    Gate<T> g;
-    g.kab = T(kcoef(0, i)) * v;
-    g.ka = T(kcoef(1, i)) * v;
-    g.kb = T(kcoef(2, i)) * v;
-    g.k1 = T(kcoef(3, i)) * v;
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) {
-        g.kab += __shfl_xor_sync(0xffffffffu, g.kab, o);
-        g.ka += __shfl_xor_sync(0xffffffffu, g.ka, o);
-        g.kb += __shfl_xor_sync(0xffffffffu, g.kb, o);
-        g.k1 += __shfl_xor_sync(0xffffffffu, g.k1, o);
-    }
-    return g;
-}
-
-template <typename T> __device__ __forceinline__ Gate<T> gate_from_lane(const Gate<T> &g, int src)
-{
-    Gate<T> r;
-    r.kab = __shfl_sync(0xffffffffu, g.kab, src);
-    r.ka = __shfl_sync(0xffffffffu, g.ka, src);
-    r.kb = __shfl_sync(0xffffffffu, g.kb, src);
-    r.k1 = __shfl_sync(0xffffffffu, g.k1, src);
-    return r;
-}
-
-template <typename T, int V> struct Vec;
-template <> struct Vec<float, 4> { using type = float4; };
-template <> struct Vec<float, 1> { using type = float; };
-template <> struct Vec<double, 1> { using type = double; };
-template <> struct Vec<double, 2> { using type = double2; };
-
-template <typename T, int V> __device__ __forceinline__ void vload(const T *p, T (&r)[V])
-{
-    using VT = typename Vec<T, V>::type;
-    const VT v = __ldg(reinterpret_cast<const VT *>(p));
-    const T *e = reinterpret_cast<const T *>(&v);
-#pragma unroll
-    for (int k = 0; k < V; ++k) r[k] = e[k];
-}
-template <typename T, int V> __device__ __forceinline__ void vstore(T *p, const T (&r)[V])
-{
-    using VT = typename Vec<T, V>::type;
-    VT v;
-    T *e = reinterpret_cast<T *>(&v);
-#pragma unroll
-    for (int k = 0; k < V; ++k) e[k] = r[k];
-    *reinterpret_cast<VT *>(p) = v;
-}
-
 // ---------------------------------------------------------------------------------------- forward
 template <typename T, int V>
 __global__ void __launch_bounds__(256) logic_fwd_kernel(const T *__restrict__ x, const int64_t *__restrict__ ia,
                                                         const int64_t *__restrict__ ib, const T *__restrict__ w, T *__restrict__ y,
-                                                        long long out_dim, long long B, int wmode)
+                                                        T *__restrict__ coef /* [out][4] for the backward pass, or null */, long long out_dim,
+                                                        long long B, int wmode)
 {
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -116,6 +32,10 @@ __global__ void __launch_bounds__(256) logic_fwd_kernel(const T *__restrict__ x,
     for (long long j0 = warp * 2; j0 < out_dim; j0 += nwarps * 2) {
         T p;
         const Gate<T> gh = half_warp_gate<T>(w, j0 + (lane >> 4), out_dim, wmode, lane, p);
+        if (coef != nullptr && (lane & 15) == 0 && j0 + (lane >> 4) < out_dim) {
+            T *o = coef + 4 * (j0 + (lane >> 4));
+            o[0] = gh.k1, o[1] = gh.ka, o[2] = gh.kb, o[3] = gh.kab;
+        }
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const long long j = j0 + h;
@@ -306,29 +226,33 @@ __global__ void __launch_bounds__(256) logic_bwd_x_kernel(const T *__restrict__ 
 
 // ----------------------------------------------------------------------------------- group sum
 // GroupSum on the feature-major activations the flat layers produce ([F][B]; class c owns rows [c*S, (c+1)*S)):
-// out[b][c] = (sum of the class's rows at sample b) / tau.  Two stages with a fixed order: block (batch tile,
-// class, part) adds its share of the rows warp by warp and combines the eight warps in order; the finalize kernel
-// adds the parts in order.  No transposed copy of the activations, no atomics.
+// out[b][c] = (sum of the class's rows at sample b) / tau.  Block (batch tile, class, part): its W warps add the part's rows
+// round robin and are combined in warp order; with several parts the finalize kernel adds those in order.  One part of 32 warps,
+// and no second launch, while a class has few rows.  No transposed copy of the activations, no atomics.
 constexpr int kGroupSumParts = 16;
 
-template <typename T>
-__global__ void __launch_bounds__(256) group_sum_partial_kernel(const T *__restrict__ y, T *__restrict__ partial, long long S, long long B, int k)
+template <typename T, int W, bool FINAL>
+__global__ void __launch_bounds__(32 * W) group_sum_partial_kernel(const T *__restrict__ y, T *__restrict__ out, long long S, long long B, int k, T tau)
 {
-    __shared__ T red[8][32];
+    __shared__ T red[W][32];
     const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
     const long long b = (long long)blockIdx.x * 32 + lane;
     const int c = blockIdx.y, part = blockIdx.z;
     const long long r0 = S * part / gridDim.z, r1 = S * (part + 1) / gridDim.z;
     T acc = T(0);
     if (b < B)
-        for (long long r = r0 + wv; r < r1; r += 8) acc += y[((long long)c * S + r) * B + b];
+#pragma unroll 8
+        for (long long r = r0 + wv; r < r1; r += W) acc += y[((long long)c * S + r) * B + b];
     red[wv][lane] = acc;
     __syncthreads();
     if (wv == 0 && b < B) {
         T t = red[0][lane];
 #pragma unroll
-        for (int i = 1; i < 8; ++i) t += red[i][lane];
-        partial[((long long)part * k + c) * B + b] = t;
+        for (int i = 1; i < W; ++i) t += red[i][lane];
+        if (FINAL)
+            out[b * k + c] = t / tau;
+        else
+            out[((long long)part * k + c) * B + b] = t;
     }
 }
 
@@ -452,30 +376,24 @@ __global__ void __launch_bounds__(256) adam_step_kernel(float *__restrict__ p, c
     }
 }
 
-// gy[f][b] = gout[b][f / S] / tau.  grid (row chunks, k): a thread keeps the quotients of its batch positions
-// in registers and writes them to every row of its chunk (coalesced along the batch).
-template <typename T>
+// gy[f][b] = gout[b][f / S] / tau.  grid (row chunks, k): a thread keeps the quotients of its batch positions -- V neighbours at
+// a time -- in registers and writes them to every row of its chunk; a batch that needs fewer than 256 threads leaves the rest
+// to further rows.
+template <typename T, int V>
 __global__ void __launch_bounds__(256) group_sum_bwd_kernel(const T *__restrict__ gout, const T *__restrict__ scale, T *__restrict__ gy,
                                                             long long S, long long B, int k, T tau)
 {
     const int c = blockIdx.y;
     if (scale != nullptr) tau = tau / scale[0]; // an upstream scalar gradient, read on the device
     const long long r0 = S * blockIdx.x / gridDim.x, r1 = S * (blockIdx.x + 1) / gridDim.x;
-    for (long long b0 = 0; b0 < B; b0 += 4 * 256) {
-        T v[4];
+    const int per_row = (int)min(256LL, (B + V - 1) / V), rows = 256 / per_row; // threads per row, rows at a time
+    const int row = threadIdx.x / per_row, col = threadIdx.x - row * per_row;
+    if (row >= rows) return;
+    for (long long b0 = (long long)col * V; b0 < B; b0 += (long long)per_row * V) {
+        T v[V];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const long long b = b0 + q * 256 + threadIdx.x;
-            v[q] = b < B ? gout[b * k + c] / tau : T(0);
-        }
-        for (long long r = r0; r < r1; ++r) {
-            T *row = gy + ((long long)c * S + r) * B;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const long long b = b0 + q * 256 + threadIdx.x;
-                if (b < B) row[b] = v[q];
-            }
-        }
+        for (int q = 0; q < V; ++q) v[q] = gout[(b0 + q) * k + c] / tau;
+        for (long long r = r0 + row; r < r1; r += rows) vstore<T, V>(gy + ((long long)c * S + r) * B + b0, v);
     }
 }
 
@@ -854,20 +772,36 @@ static int logic_grid(long long units_of_warps)
     return (int)blocks;
 }
 
+int clb_logic_fwd_cols(const float *x, const int64_t *a, const int64_t *b, const float *w, float *y, float *coef, int64_t out_dim, int64_t B, int wmode,
+                       cudaStream_t st); // logic_bwd.cu
+
 extern "C" int clb_logic_fwd(const void *x, const int64_t *a, const int64_t *b, const void *w, void *y, int64_t in_dim,
                              int64_t out_dim, int64_t B, int wmode, int dtype, void *stream)
+{
+    return clb_logic_fwd_coef(x, a, b, w, y, nullptr, in_dim, out_dim, B, wmode, dtype, stream);
+}
+
+extern "C" int clb_logic_fwd_coef(const void *x, const int64_t *a, const int64_t *b, const void *w, void *y, void *coef, int64_t in_dim,
+                                  int64_t out_dim, int64_t B, int wmode, int dtype, void *stream)
 {
     if (!x || !a || !b || !w || !y || in_dim <= 0 || out_dim < 0 || B < 0 || wmode < 0 || wmode > 2) return CLB_ERR_ARG;
     if (out_dim == 0 || B == 0) return CLB_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const int grid = logic_grid((out_dim + 1) / 2);
     if (dtype == CLB_F32) {
-        if (B % 4 == 0 && aligned16(x) && aligned16(y))
-            CLB_TRACED("logic_fwd_kernel", st, logic_fwd_kernel<float, 4><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (float *)y, out_dim, B, wmode));
+        const bool vec = B % 4 == 0 && aligned16(x) && aligned16(y);
+        // an input beyond about half the L2 is walked in column stretches that fit it (0.44 -> 0.40 ms per 256000 x 1024 layer)
+        if (coef && vec && aligned16(coef) && aligned16(w) && B >= 256 && B <= 4000000 && in_dim * B * 4 > (64LL << 20) && in_dim <= 0x3fffffff && out_dim <= 0x3fffffff)
+            return clb_logic_fwd_cols((const float *)x, a, b, (const float *)w, (float *)y, (float *)coef, out_dim, B, wmode, st);
+        if (vec)
+            CLB_TRACED("logic_fwd_kernel", st,
+                       logic_fwd_kernel<float, 4><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (float *)y, (float *)coef, out_dim, B, wmode));
         else
-            CLB_TRACED("logic_fwd_kernel", st, logic_fwd_kernel<float, 1><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (float *)y, out_dim, B, wmode));
+            CLB_TRACED("logic_fwd_kernel", st,
+                       logic_fwd_kernel<float, 1><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (float *)y, (float *)coef, out_dim, B, wmode));
     } else if (dtype == CLB_F64) {
-        CLB_TRACED("logic_fwd_kernel", st, logic_fwd_kernel<double, 1><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (double *)y, out_dim, B, wmode));
+        CLB_TRACED("logic_fwd_kernel", st,
+                   logic_fwd_kernel<double, 1><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (double *)y, (double *)coef, out_dim, B, wmode));
     } else
         return CLB_ERR_ARG;
     return check_launch();
@@ -964,14 +898,18 @@ extern "C" int clb_group_sum_fwd(const void *y, void *out, void *scratch, size_t
     cudaStream_t st = (cudaStream_t)stream;
     dim3 grid((unsigned)((B + 31) / 32), (unsigned)k, (unsigned)parts);
     const int fb = (int)((B * k + 255) / 256);
-    if (dtype == CLB_F32) {
-        CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<float><<<grid, 256, 0, st>>>((const float *)y, (float *)scratch, S, B, k));
-        CLB_TRACED("group_sum_finalize_kernel", st, group_sum_finalize_kernel<float><<<fb, 256, 0, st>>>((const float *)scratch, (float *)out, B, k, parts, (float)tau));
-    } else {
-        CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<double><<<grid, 256, 0, st>>>((const double *)y, (double *)scratch, S, B, k));
-        CLB_TRACED("group_sum_finalize_kernel", st, group_sum_finalize_kernel<double><<<fb, 256, 0, st>>>((const double *)scratch, (double *)out, B, k, parts, tau));
-    }
-    return check_launch(2);
+    auto go = [&](auto t) {
+        using T = decltype(t);
+        if (S <= 4096) { // 128 rows per warp at most: about what a second launch costs
+            grid.z = 1;
+            CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<T, 32, true><<<grid, 1024, 0, st>>>((const T *)y, (T *)out, S, B, k, (T)tau));
+            return 1;
+        }
+        CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<T, 8, false><<<grid, 256, 0, st>>>((const T *)y, (T *)scratch, S, B, k, (T)tau));
+        CLB_TRACED("group_sum_finalize_kernel", st, group_sum_finalize_kernel<T><<<fb, 256, 0, st>>>((const T *)scratch, (T *)out, B, k, parts, (T)tau));
+        return 2;
+    };
+    return check_launch(dtype == CLB_F32 ? go(0.f) : go(0.0));
 }
 
 extern "C" int clb_group_sum_ce(const float *y, const int64_t *labels, float *scores, float *dscore, float *loss, void *scratch,
@@ -984,7 +922,7 @@ extern "C" int clb_group_sum_ce(const float *y, const int64_t *labels, float *sc
     const int parts = group_sum_parts(S);
     cudaStream_t st = (cudaStream_t)stream;
     dim3 grid((unsigned)((B + 31) / 32), (unsigned)k, (unsigned)parts);
-    CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<float><<<grid, 256, 0, st>>>(y, (float *)scratch, S, B, k));
+    CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<float, 8, false><<<grid, 256, 0, st>>>(y, (float *)scratch, S, B, k, 1.f));
     CLB_TRACED("group_sum_ce_sample_kernel", st,
                group_sum_ce_sample_kernel<<<(unsigned)((B + 7) / 8), 256, 0, st>>>((float *)scratch, labels, scores, dscore, B, k, parts, (float)tau));
     CLB_TRACED("group_sum_loss_mean_kernel", st, group_sum_loss_mean_kernel<<<1, 256, 0, st>>>((const float *)scratch, loss, B));
@@ -1037,13 +975,15 @@ extern "C" int clb_group_sum_bwd_scaled(const void *gout, const void *scale, voi
     cudaStream_t st = (cudaStream_t)stream;
     const long long S = F / k;
     if (k > 65535) return CLB_ERR_SHAPE;
-    long long chunks = ((long long)sm_count() * 16 + k - 1) / k; // about sixteen blocks per SM in all
-    if (chunks > S) chunks = S;
+    long long chunks = ((long long)sm_count() * 16 + k - 1) / k; // about sixteen blocks per SM in all, at least 16 rows each
+    if (chunks > (S + 15) / 16) chunks = (S + 15) / 16;
     dim3 grid((unsigned)chunks, (unsigned)k);
-    if (dtype == CLB_F32)
-        CLB_TRACED("group_sum_bwd_kernel", st, group_sum_bwd_kernel<float><<<grid, 256, 0, st>>>((const float *)gout, (const float *)scale, (float *)gy, S, B, k, (float)tau));
+    if (dtype == CLB_F32 && B % 4 == 0 && aligned16(gy))
+        CLB_TRACED("group_sum_bwd_kernel", st, group_sum_bwd_kernel<float, 4><<<grid, 256, 0, st>>>((const float *)gout, (const float *)scale, (float *)gy, S, B, k, (float)tau));
+    else if (dtype == CLB_F32)
+        CLB_TRACED("group_sum_bwd_kernel", st, group_sum_bwd_kernel<float, 1><<<grid, 256, 0, st>>>((const float *)gout, (const float *)scale, (float *)gy, S, B, k, (float)tau));
     else
-        CLB_TRACED("group_sum_bwd_kernel", st, group_sum_bwd_kernel<double><<<grid, 256, 0, st>>>((const double *)gout, (const double *)scale, (double *)gy, S, B, k, tau));
+        CLB_TRACED("group_sum_bwd_kernel", st, group_sum_bwd_kernel<double, 1><<<grid, 256, 0, st>>>((const double *)gout, (const double *)scale, (double *)gy, S, B, k, tau));
     return check_launch();
 }
 

@@ -7,6 +7,7 @@
 // of a parameter that carries one).  No arithmetic happens here; every number comes from the kernels behind
 // include/convlogic_b200.h.
 #include <ATen/ATen.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -16,6 +17,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/utils/pybind.h>
 
+#include <atomic>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -60,9 +62,16 @@ int dtype_code(const Tensor &t)
     return CLB_F64;
 }
 
-void *stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
+void *cur_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 template <typename T = void> T *ptr(const Tensor &t) { return t.defined() ? static_cast<T *>(t.data_ptr()) : nullptr; }
-Tensor scratch_bytes(size_t n, const Tensor &like) { return at::empty({(int64_t)(n < 16 ? 16 : n)}, like.options().dtype(at::kByte)); }
+// device memory from torch's caching allocator, without the dispatcher's detour (about half a microsecond each)
+Tensor alloc(at::IntArrayRef sizes, const Tensor &like, at::ScalarType type) { return at::detail::empty_cuda(sizes, type, like.device(), std::nullopt); }
+Tensor alloc(at::IntArrayRef sizes, const Tensor &like) { return alloc(sizes, like, like.scalar_type()); }
+Tensor alloc_strided(at::IntArrayRef sizes, at::IntArrayRef strides, const Tensor &like)
+{
+    return at::detail::empty_strided_cuda(sizes, strides, like.scalar_type(), like.device());
+}
+Tensor scratch_bytes(size_t n, const Tensor &like) { return alloc({(int64_t)(n < 16 ? 16 : n)}, like, at::kByte); }
 
 // Raw calls run below autograd and view tracking: their results get a history from our own nodes only.
 struct Below {
@@ -91,8 +100,8 @@ Tensor transpose2d(const Tensor &x)
     need_input(x);
     TORCH_CHECK(x.dim() == 2 && x.scalar_type() == at::kFloat, "convlogic_b200: transpose2d expects a contiguous 2-D float32 tensor");
     Below below(x);
-    Tensor out = at::empty({x.size(1), x.size(0)}, x.options());
-    check(clb_transpose_f32(ptr<float>(x), ptr<float>(out), x.size(0), x.size(1), stream()));
+    Tensor out = alloc({x.size(1), x.size(0)}, x);
+    check(clb_transpose_f32(ptr<float>(x), ptr<float>(out), x.size(0), x.size(1), cur_stream()));
     return out;
 }
 
@@ -103,15 +112,20 @@ Tensor transposed_copy(const Tensor &t)
     return t.t().contiguous();
 }
 
-// feature-major storage [F, B] of a [B, F] activation: its own storage when it is the transposed view a flat layer returns
-Tensor feature_major(const Tensor &x)
+// Is a [B, F] activation stored feature-major ([F, B], what a flat layer returns)?  Then its storage is read as it is.
+bool stored_feature_major(const Tensor &x)
 {
-    Tensor xt = x.t();
-    return xt.is_contiguous() ? xt : transposed_copy(x);
+    return x.dim() == 2 && (x.size(0) <= 1 || x.stride(0) == 1) && (x.size(1) <= 1 || x.stride(1) == x.size(0));
 }
+// a tensor whose storage is [F, B], from a [B, F] activation (x itself where possible; the shape of the result is not to be used)
+Tensor feature_major_storage(const Tensor &x) { return stored_feature_major(x) ? x : transposed_copy(x); }
 
-// a [B, F] gradient whose storage is [F, B]; a leaf that stores [B, F] gets a plain contiguous tensor, anything else the view
-Tensor batch_major_grad(const Tensor &g_fm, bool contiguous) { return contiguous ? transposed_copy(g_fm) : g_fm.t(); }
+// A [B, F] gradient of feature-major storage: made in that form, or, for a leaf that stores [B, F], turned round at the end.
+Tensor feature_major_grad(int64_t batch, int64_t features, const Tensor &like)
+{
+    return alloc_strided({batch, features}, {1, std::max<int64_t>(batch, 1)}, like);
+}
+Tensor finished_grad(const Tensor &g, bool leaf) { return leaf && !g.is_contiguous() ? transposed_copy(g.t()) : g; }
 bool feeds_leaf(const Node &n, size_t i)
 {
     const auto &e = n.next_edge(i);
@@ -141,11 +155,14 @@ std::optional<Sink> sink_of(const Tensor &w) // GIL held
     return out;
 }
 
+std::atomic<int64_t> g_sinks{0}; // parameters that carry one: while there are none, no backward pass needs to ask Python
+
 // The slices of one backward call's parameters: all of them or none (a kernel writes them together).
 class Sinks {
 public:
     explicit Sinks(std::initializer_list<std::reference_wrapper<const Tensor>> ws)
     {
+        if (g_sinks.load(std::memory_order_relaxed) <= 0) return;
         py::gil_scoped_acquire gil;
         for (const Tensor &w : ws) {
             auto s = sink_of(w);
@@ -311,28 +328,28 @@ BlockOut block_fwd(const Tensor &x, const Tensor &w, const Tensor &sel, const Ge
     const int hp = d.ho / 2, wp = d.wo / 2, dt = dtype_code(x);
     Below below(x);
     BlockOut o;
-    if (want_amax) o.amax = at::empty({d.n, d.c, hp, wp}, x.options().dtype(at::kByte));
-    if (want_inter) o.x2 = at::empty({d.n, d.c, d.ho, d.wo, 4}, x.options()), o.x3 = at::empty({d.n, d.c, d.ho, d.wo, 2}, x.options());
-    if (want_idx) o.idx = at::empty({d.n, d.c, (int64_t)hp * wp}, x.options().dtype(at::kInt));
+    if (want_amax) o.amax = alloc({d.n, d.c, hp, wp}, x, at::kByte);
+    if (want_inter) o.x2 = alloc({d.n, d.c, d.ho, d.wo, 4}, x), o.x3 = alloc({d.n, d.c, d.ho, d.wo, 2}, x);
+    if (want_idx) o.idx = alloc({d.n, d.c, (int64_t)hp * wp}, x, at::kInt);
     if (d.n == 0 || d.c == 0) { // empty batch: nothing to launch
-        o.y = at::empty({d.n, d.c, hp, wp}, x.options());
+        o.y = alloc({d.n, d.c, hp, wp}, x);
         return o;
     }
     const PlanPtr plan = get_plan();
     TORCH_CHECK(plan->channels_ok, "convlogic_b200: selection refers to a channel the input does not have");
     if (y_fm && dt == CLB_F32 && !want_inter && !want_idx && !plan->flag) {
         // the flat layers' layout, storage [C, h, w, N]; only the plane kernels write it
-        o.y = at::empty_strided({d.n, d.c, hp, wp}, {1, (int64_t)hp * wp * d.n, (int64_t)wp * d.n, d.n}, x.options());
+        o.y = alloc_strided({d.n, d.c, hp, wp}, {1, (int64_t)hp * wp * d.n, (int64_t)wp * d.n, d.n}, x);
         const int rc = clb_convtree_fwd(ptr(x), ptr(w), ptr<int32_t>(sel), ptr(o.y), ptr<uint8_t>(o.amax), nullptr, nullptr, nullptr, d.n, d.ci, d.h, d.w,
-                                        d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, wmode | CLB_Y_FEATURE_MAJOR, dt, stream());
+                                        d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, wmode | CLB_Y_FEATURE_MAJOR, dt, cur_stream());
         if (rc != CLB_ERR_SHAPE) {
             check(rc);
             return o;
         }
     }
-    o.y = at::empty({d.n, d.c, hp, wp}, x.options());
+    o.y = alloc({d.n, d.c, hp, wp}, x);
     check(clb_convtree_fwd(ptr(x), ptr(w), ptr<int32_t>(sel), ptr(o.y), ptr<uint8_t>(o.amax), ptr(o.x2), ptr(o.x3), ptr<int32_t>(o.idx), d.n, d.ci, d.h,
-                           d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, wmode | plan->flag, dt, stream()));
+                           d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, wmode | plan->flag, dt, cur_stream()));
     return o;
 }
 
@@ -353,9 +370,9 @@ std::pair<Tensor, Tensor> block_bwd(Tensor gy, const Tensor &x, const Tensor &w,
     const int dt = dtype_code(x);
     Below below(x);
     Tensor gx, gw;
-    if (need_gx) gx = at::empty(x.sizes(), x.options());
+    if (need_gx) gx = alloc(x.sizes(), x);
     if (need_gw) {
-        gw = gw_out.defined() ? gw_out : at::empty(w.sizes(), w.options());
+        gw = gw_out.defined() ? gw_out : alloc(w.sizes(), w);
         TORCH_CHECK(gw.sizes() == w.sizes() && gw.scalar_type() == w.scalar_type() && gw.is_contiguous(),
                     "convlogic_b200: `gw_out` must be contiguous with the gate tensor's shape and dtype");
     }
@@ -373,7 +390,7 @@ std::pair<Tensor, Tensor> block_bwd(Tensor gy, const Tensor &x, const Tensor &w,
             Tensor scratch = scratch_bytes(bytes, x);
             const int rc = clb_convtree_bwd_plane(ptr(gy), ptr(x), ptr(w), ptr<int32_t>(sel), ptr<uint8_t>(amax), ptr(gx), ptr(gw), ptr<int32_t>(plan->start),
                                                   ptr<int32_t>(plan->entry), ptr(scratch), bytes, d.n, d.ci, d.h, d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh,
-                                                  g.kw, wmode | (fm ? CLB_Y_FEATURE_MAJOR : 0), dt, stream());
+                                                  g.kw, wmode | (fm ? CLB_Y_FEATURE_MAJOR : 0), dt, cur_stream());
             if (rc != CLB_ERR_SHAPE) {
                 check(rc);
                 return {gx, gw};
@@ -387,22 +404,23 @@ std::pair<Tensor, Tensor> block_bwd(Tensor gy, const Tensor &x, const Tensor &w,
     if (need_gx) gr = plan->group_tables(d.n, d.h, d.w, dt);
     check(clb_convtree_bwd(ptr(gy), ptr(x), ptr(w), ptr<int32_t>(sel), ptr<uint8_t>(amax), ptr(gx), ptr(gw), ptr<int32_t>(gr.start),
                            ptr<int32_t>(gr.list), gr.cg, gr.nb, ptr(scratch), bytes, d.n, d.ci, d.h, d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw,
-                           wmode | plan->flag, dt, stream()));
+                           wmode | plan->flag, dt, cur_stream()));
     return {gx, gw};
 }
 
 struct BlockNode : public Node {
-    SavedVariable x, w, sel;
-    Tensor amax;
+    SavedVariable x, w;
+    Tensor sel, amax;
     PlanPtr plan;
     Geom g;
     int wmode;
     std::string name() const override { return "FullConvLogicFunctionBackward"; }
-    void release_variables() override { x.reset_data(), w.reset_data(), sel.reset_data(), amax.reset(); }
+    void release_variables() override { x.reset_data(), w.reset_data(), amax.reset(); }
     variable_list apply(variable_list &&grads) override
     {
         if (!grads[0].defined()) return {Tensor(), Tensor()};
-        const Tensor xx = x.unpack(), ww = w.unpack(), ss = sel.unpack();
+        const Tensor xx = x.unpack(), ww = w.unpack(), &ss = sel;
+        TORCH_CHECK(ss.is_inference() || plan->version == (int64_t)ss._version(), "convlogic_b200: the selection was modified between forward and backward");
         const bool need_gx = task_should_compute_output(0), need_gw = task_should_compute_output(1) && wmode != CLB_W_ARGMAX;
         if (!need_gx && !need_gw) return {Tensor(), Tensor()};
         Tensor gy = grads[0];
@@ -431,7 +449,7 @@ py::object block(Tensor x, Tensor w, py::object sel_obj, int sh, int sw, int ph,
         auto node = new_node<BlockNode>();
         node->set_next_edges(torch::autograd::collect_next_edges(x, w));
         if (!plan) get_plan();
-        node->x = saved(x), node->w = saved(w), node->sel = saved(sel), node->amax = o.amax, node->plan = plan, node->g = g, node->wmode = wmode;
+        node->x = saved(x), node->w = saved(w), node->sel = sel, node->amax = o.amax, node->plan = plan, node->g = g, node->wmode = wmode;
         torch::autograd::set_history(o.y, node);
     }
     if (!want_inter && !want_idx) return py::cast(o.y);
@@ -457,12 +475,51 @@ LogicDims logic_dims(const Tensor &x_fm, const Tensor &a, const Tensor &b, const
     return {x_fm.size(0), out, x_fm.size(1)};
 }
 
-void logic_fwd(const Tensor &x_fm, const Tensor &a, const Tensor &b, const Tensor &w, int wmode, const Tensor &y_storage)
+// The consumer lists as the combined backward reads them, laid out once per layer and kept on the list tensor object as
+// `_clb_plan` (checked by the tensors' addresses and versions).
+using LogicKey = std::array<std::pair<const void *, int64_t>, 4>; // a, b, start, consumers: address and version
+LogicKey logic_key(const Tensor &a, const Tensor &b, const Tensor &start, const Tensor &cons)
+{
+    auto id = [](const Tensor &t) { return std::make_pair((const void *)t.data_ptr(), t.is_inference() ? (int64_t)0 : (int64_t)t._version()); };
+    return {id(a), id(b), id(start), id(cons)};
+}
+struct LogicPlan {
+    LogicKey key;
+    int64_t in = 0, out = 0;
+    Tensor start32, entry;
+};
+using LogicPlanPtr = std::shared_ptr<LogicPlan>;
+
+LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const Tensor &b, const Tensor &start, const Tensor &cons, int64_t in, int64_t out)
+{
+    const LogicKey key = logic_key(a, b, start, cons);
+    if (PyObject_HasAttrString(start_obj.ptr(), "_clb_plan")) {
+        LogicPlanPtr p = py::reinterpret_steal<py::object>(PyObject_GetAttrString(start_obj.ptr(), "_clb_plan")).cast<LogicPlanPtr>();
+        if (p && p->key == key && p->in == in && p->out == out) return p;
+    }
+    need_inputs(a, b, start, cons);
+    TORCH_CHECK(start.scalar_type() == at::kLong && cons.scalar_type() == at::kLong && start.numel() == in + 1 && cons.numel() == 2 * out,
+                "convlogic_b200: consumer lists must be int64 [in_dim + 1] and [2 * out_dim]");
+    if (in > 0x3fffffff || out > 0x3fffffff) return nullptr;
+    auto p = std::make_shared<LogicPlan>();
+    p->key = key, p->in = in, p->out = out;
+    Below below(start);
+    p->start32 = alloc({in + 1}, start, at::kInt), p->entry = alloc({2 * out, 2}, start, at::kInt);
+    check(clb_logic_entries(ptr<int64_t>(a), ptr<int64_t>(b), ptr<int64_t>(start), ptr<int64_t>(cons), ptr<int32_t>(p->start32), ptr(p->entry), in, out,
+                            cur_stream()));
+    // the plan outlives this call: work of other streams may read it next
+    c10::cuda::getCurrentCUDAStream().synchronize();
+    start_obj.attr("_clb_plan") = p;
+    return p;
+}
+
+void logic_fwd(const Tensor &x_fm, const Tensor &a, const Tensor &b, const Tensor &w, int wmode, const Tensor &y_storage, const Tensor &coef = Tensor())
 {
     need_inputs(x_fm, a, b, w);
     const LogicDims d = logic_dims(x_fm, a, b, w);
     if (d.batch == 0 || d.out == 0) return;
-    check(clb_logic_fwd(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(y_storage), d.in, d.out, d.batch, wmode, dtype_code(x_fm), stream()));
+    check(clb_logic_fwd_coef(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(y_storage), ptr(coef), d.in, d.out, d.batch, wmode, dtype_code(x_fm),
+                             cur_stream()));
 }
 
 Tensor logic_bwd_w(const Tensor &x_fm, const Tensor &a, const Tensor &b, const Tensor &w, const Tensor &gy_fm, int wmode, const Tensor &gw_out)
@@ -470,10 +527,10 @@ Tensor logic_bwd_w(const Tensor &x_fm, const Tensor &a, const Tensor &b, const T
     need_inputs(x_fm, a, b, w, gy_fm);
     const LogicDims d = logic_dims(x_fm, a, b, w);
     Below below(x_fm);
-    Tensor gw = gw_out.defined() ? gw_out : at::empty(w.sizes(), w.options());
+    Tensor gw = gw_out.defined() ? gw_out : alloc(w.sizes(), w);
     if (d.batch == 0 || d.out == 0) return gw.zero_();
     check(clb_logic_bwd_w(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(gy_fm), ptr(gw), d.in, d.out, d.batch, wmode, dtype_code(x_fm),
-                          stream()));
+                          cur_stream()));
     return gw;
 }
 
@@ -485,72 +542,117 @@ Tensor logic_bwd_x(const Tensor &x_fm, const Tensor &a, const Tensor &b, const T
     TORCH_CHECK(start.scalar_type() == at::kLong && cons.scalar_type() == at::kLong && start.numel() == d.in + 1 && cons.numel() == 2 * d.out,
                 "convlogic_b200: consumer lists must be int64 [in_dim + 1] and [2 * out_dim]");
     Below below(x_fm);
-    Tensor gx = at::empty(x_fm.sizes(), x_fm.options());
+    Tensor gx = alloc(x_fm.sizes(), x_fm);
     if (d.batch == 0) return gx;
     check(clb_logic_bwd_x(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(gy_fm), ptr(gx), ptr<int64_t>(start), ptr<int64_t>(cons), d.in, d.out,
-                          d.batch, wmode, dtype_code(x_fm), stream()));
+                          d.batch, wmode, dtype_code(x_fm), cur_stream()));
     return gx;
 }
 
 struct LogicNode : public Node {
-    SavedVariable x, a, b, w, start, cons; // x: the feature-major storage the forward read
+    SavedVariable x, w;      // x: a tensor on the feature-major storage the forward read
+    Tensor a, b, start, cons; // connections, checked against `key`
+    LogicKey key;
+    Tensor coef;             // gate coefficients and the laid-out lists (fp32 with an input gradient)
+    LogicPlanPtr plan;
+    int64_t in, out, batch;
     int wmode;
     bool fm; // the call's own tensors are feature-major ([in, B] -> [out, B])
     std::string name() const override { return "LogicLayerCudaFunctionBackward"; }
-    void release_variables() override
-    {
-        x.reset_data(), a.reset_data(), b.reset_data(), w.reset_data(), start.reset_data(), cons.reset_data();
-    }
+    void release_variables() override { x.reset_data(), w.reset_data(), coef.reset(); }
     variable_list apply(variable_list &&grads) override
     {
         if (!grads[0].defined()) return {Tensor(), Tensor()};
-        const Tensor xx = x.unpack(), aa = a.unpack(), bb = b.unpack(), ww = w.unpack();
-        Tensor gx, gw;
+        const Tensor xx = x.unpack(), ww = w.unpack();
+        TORCH_CHECK(key == logic_key(a, b, start, cons), "convlogic_b200: the connections of a layer were modified between forward and backward");
+        const bool need_gx = task_should_compute_output(0), need_gw = task_should_compute_output(1) && wmode != CLB_W_ARGMAX;
         Below below(xx);
-        const Tensor gy = fm ? grads[0].contiguous() : feature_major(grads[0]);
-        if (task_should_compute_output(0)) {
-            gx = logic_bwd_x(xx, aa, bb, ww, gy, start.unpack(), cons.unpack(), wmode);
-            if (!fm) gx = batch_major_grad(gx, feeds_leaf(*this, 0));
+        const Tensor gy = fm ? grads[0].contiguous() : feature_major_storage(grads[0]);
+        TORCH_CHECK(gy.numel() == out * batch && gy.scalar_type() == xx.scalar_type(), "convlogic_b200: upstream gradient must be [", out, ", ", batch, "] ",
+                    xx.scalar_type());
+        const int dt = dtype_code(xx);
+        Tensor gx, gw;
+        Sinks sinks(need_gw ? std::initializer_list<std::reference_wrapper<const Tensor>>{ww} : std::initializer_list<std::reference_wrapper<const Tensor>>{});
+        if (need_gx) gx = fm ? alloc({in, batch}, xx) : feature_major_grad(batch, in, xx);
+        if (need_gw) {
+            gw = sinks.any() ? sinks.slice(0) : alloc(ww.sizes(), ww);
+            TORCH_CHECK(gw.sizes() == ww.sizes() && gw.is_contiguous() && gw.scalar_type() == ww.scalar_type(),
+                        "convlogic_b200: a gradient slice must be contiguous with the gate tensor's shape and dtype");
         }
-        if (task_should_compute_output(1) && wmode != CLB_W_ARGMAX) {
-            Sinks sinks({ww});
-            gw = logic_bwd_w(xx, aa, bb, ww, gy, wmode, sinks.slice(0));
-            if (sinks.any()) {
-                sinks.ready();
-                gw = Tensor();
+        if (batch == 0 || out == 0) {
+            if (gw.defined()) gw.zero_();
+            if (gx.defined()) gx.zero_();
+        } else {
+            int rc = CLB_ERR_SHAPE;
+            if (need_gx && coef.defined() && plan) { // both gradients in one pass
+                const size_t bytes = need_gw ? clb_logic_bwd_scratch_bytes(in, out, batch) : 0;
+                Tensor scratch;
+                if (need_gw) scratch = scratch_bytes(bytes, xx);
+                rc = clb_logic_bwd(ptr<float>(xx), ptr<float>(ww), ptr<float>(coef), ptr<float>(gy), ptr<float>(gx), ptr<float>(gw),
+                                   ptr<int32_t>(plan->start32), ptr(plan->entry), ptr(scratch), bytes, in, out, batch, wmode, cur_stream());
+                if (rc != CLB_ERR_SHAPE) check(rc);
             }
+            if (rc == CLB_ERR_SHAPE && need_gx)
+                check(clb_logic_bwd_x(ptr(xx), ptr<int64_t>(a), ptr<int64_t>(b), ptr(ww), ptr(gy), ptr(gx), ptr<int64_t>(start), ptr<int64_t>(cons), in, out, batch,
+                                      wmode, dt, cur_stream()));
+            if (rc == CLB_ERR_SHAPE && need_gw)
+                check(clb_logic_bwd_w(ptr(xx), ptr<int64_t>(a), ptr<int64_t>(b), ptr(ww), ptr(gy), ptr(gw), in, out, batch, wmode, dt, cur_stream()));
+        }
+        if (gx.defined() && !fm) gx = finished_grad(gx, feeds_leaf(*this, 0));
+        if (sinks.any()) {
+            sinks.ready();
+            gw = Tensor();
         }
         return {gx, gw};
     }
 };
 
 // fm: x [in, B] -> y [out, B] (the reference's Function); else x [B, in] -> y [B, out] on the storage [out, B]
-Tensor logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w_in, const Tensor &start, const Tensor &cons, int wmode, bool fm)
+Tensor logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w_in, py::object start_obj, const Tensor &cons, int wmode, bool fm)
 {
+    const Tensor start = start_obj.cast<Tensor>();
     const bool graph = wants_grad({x, w_in});
-    Tensor y, x_fm, w;
+    TORCH_CHECK(x.is_cuda(), "convlogic_b200: tensor must be a CUDA tensor");
+    TORCH_CHECK(x.dim() == 2, "convlogic_b200: x must be 2-D, got ", x.sizes());
+    const int64_t in = x.size(fm ? 0 : 1), batch = x.size(fm ? 1 : 0), out = w_in.size(0);
+    const int dt = dtype_code(x);
+    TORCH_CHECK(w_in.dim() == 2 && w_in.size(1) == 16 && w_in.scalar_type() == x.scalar_type(), "convlogic_b200: gate tensor must be [", out, ", 16] ",
+                x.scalar_type());
+    TORCH_CHECK(a.scalar_type() == at::kLong && b.scalar_type() == at::kLong && a.dim() == 1 && b.dim() == 1 && a.size(0) == out && b.size(0) == out,
+                "convlogic_b200: connection indices must be int64 [out_dim]");
+    need_inputs(a, b);
+    Tensor y, x_fm, w, coef;
+    LogicPlanPtr plan;
     {
-        TORCH_CHECK(x.is_cuda(), "convlogic_b200: tensor must be a CUDA tensor");
-        TORCH_CHECK(x.dim() == 2, "convlogic_b200: x must be 2-D, got ", x.sizes());
         Below below(x);
         w = w_in.contiguous();
-        x_fm = fm ? x.contiguous() : feature_major(x);
-        const int64_t out = w.size(0), batch = x_fm.size(1);
-        y = fm ? at::empty({out, batch}, x.options()) : at::empty_strided({batch, out}, {1, std::max<int64_t>(batch, 1)}, x.options());
-        logic_fwd(x_fm, a, b, w, wmode, y);
+        need_input(w);
+        x_fm = fm ? x.contiguous() : feature_major_storage(x);
+        y = fm ? alloc({out, batch}, x) : alloc_strided({batch, out}, {1, std::max<int64_t>(batch, 1)}, x);
+        if (graph && x.requires_grad() && dt == CLB_F32 && out) { // the backward takes both gradients in one pass
+            plan = logic_plan_for(start_obj, a, b, start, cons, in, out);
+            coef = alloc({out, 4}, x);
+        }
+        if (batch && out)
+            check(clb_logic_fwd_coef(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(y), ptr(coef), in, out, batch, wmode, dt, cur_stream()));
     }
     if (graph) {
         auto node = new_node<LogicNode>();
         node->set_next_edges(torch::autograd::collect_next_edges(x, w_in));
+        need_inputs(start, cons);
+        TORCH_CHECK(start.scalar_type() == at::kLong && cons.scalar_type() == at::kLong && start.numel() == in + 1 && cons.numel() == 2 * out,
+                    "convlogic_b200: consumer lists must be int64 [in_dim + 1] and [2 * out_dim]");
         // the parameter itself is saved (it may carry a gradient sink); its contiguous copy only where it is not contiguous
-        node->x = saved(x_fm), node->a = saved(a), node->b = saved(b), node->w = saved(w_in.is_contiguous() ? w_in : w), node->start = saved(start),
-        node->cons = saved(cons), node->wmode = wmode, node->fm = fm;
+        node->x = saved(x_fm), node->w = saved(w_in.is_contiguous() ? w_in : w);
+        node->a = a, node->b = b, node->start = start, node->cons = cons, node->key = plan ? plan->key : logic_key(a, b, start, cons);
+        node->coef = coef, node->plan = plan, node->in = in, node->out = out, node->batch = batch, node->wmode = wmode, node->fm = fm;
         torch::autograd::set_history(y, node);
     }
     return y;
 }
 
 // ------------------------------------------------------------------------------------------------ class sums
+// [B, k] -> the [B, F] gradient on feature-major storage
 Tensor group_sum_bwd(const Tensor &gout, int64_t f, int k, double tau, const Tensor &scale)
 {
     need_input(gout);
@@ -560,21 +662,22 @@ Tensor group_sum_bwd(const Tensor &gout, int64_t f, int k, double tau, const Ten
                     "convlogic_b200: `scale` must be a one-element tensor of the gradient's dtype");
     }
     Below below(gout);
-    Tensor gy = at::empty({f, gout.size(0)}, gout.options());
-    check(clb_group_sum_bwd_scaled(ptr(gout), ptr(scale), ptr(gy), f, gout.size(0), k, tau, dtype_code(gout), stream()));
+    Tensor gy = feature_major_grad(gout.size(0), f, gout);
+    check(clb_group_sum_bwd_scaled(ptr(gout), ptr(scale), ptr(gy), f, gout.size(0), k, tau, dtype_code(gout), cur_stream()));
     return gy;
 }
 
-Tensor group_sum_fwd(const Tensor &y_fm, int k, double tau)
+// y: [B, F] on feature-major storage
+Tensor group_sum_fwd(const Tensor &y, int k, double tau)
 {
-    need_input(y_fm);
-    const int64_t f = y_fm.size(0), b = y_fm.size(1);
-    const int dt = dtype_code(y_fm);
-    Below below(y_fm);
-    Tensor out = at::empty({b, k}, y_fm.options());
+    TORCH_CHECK(y.is_cuda() && stored_feature_major(y), "convlogic_b200: class sums are taken from a flat layer's output");
+    const int64_t f = y.size(1), b = y.size(0);
+    const int dt = dtype_code(y);
+    Below below(y);
+    Tensor out = alloc({b, k}, y);
     const size_t bytes = clb_group_sum_scratch_bytes(f, b, k, dt);
-    Tensor scratch = scratch_bytes(bytes, y_fm);
-    check(clb_group_sum_fwd(ptr(y_fm), ptr(out), ptr(scratch), bytes, f, b, k, tau, dt, stream()));
+    Tensor scratch = scratch_bytes(bytes, y);
+    check(clb_group_sum_fwd(ptr(y), ptr(out), ptr(scratch), bytes, f, b, k, tau, dt, cur_stream()));
     return out;
 }
 
@@ -587,7 +690,7 @@ struct GroupSumNode : public Node {
     {
         if (!grads[0].defined()) return {Tensor()};
         Below below(grads[0]);
-        return {batch_major_grad(group_sum_bwd(grads[0].contiguous(), f, k, tau, Tensor()), feeds_leaf(*this, 0))};
+        return {finished_grad(group_sum_bwd(grads[0].contiguous(), f, k, tau, Tensor()), feeds_leaf(*this, 0))};
     }
 };
 
@@ -597,7 +700,7 @@ Tensor group_sum(const Tensor &x, int k, double tau)
     Tensor out;
     {
         Below below(x);
-        out = group_sum_fwd(x.t(), k, tau);
+        out = group_sum_fwd(x, k, tau);
     }
     if (wants_grad({x})) {
         auto node = new_node<GroupSumNode>();
@@ -609,20 +712,20 @@ Tensor group_sum(const Tensor &x, int k, double tau)
 }
 
 // (loss [1], dscore [B, k], scores [B, k] or undefined)
-std::tuple<Tensor, Tensor, Tensor> group_sum_ce_raw(const Tensor &y_fm, const Tensor &labels, int k, double tau, bool want_scores)
+// y_fm: a tensor whose storage is [F, B]
+std::tuple<Tensor, Tensor, Tensor> group_sum_ce_raw(const Tensor &y_fm, int64_t f, int64_t b, const Tensor &labels, int k, double tau, bool want_scores)
 {
-    need_inputs(y_fm, labels);
-    TORCH_CHECK(y_fm.scalar_type() == at::kFloat && labels.scalar_type() == at::kLong && labels.dim() == 1 && labels.size(0) == y_fm.size(1),
+    need_input(labels);
+    TORCH_CHECK(y_fm.is_cuda() && y_fm.scalar_type() == at::kFloat && labels.scalar_type() == at::kLong && labels.dim() == 1 && labels.size(0) == b,
                 "convlogic_b200: group_sum_ce expects float32 [F, B] activations and int64 [B] labels");
-    const int64_t f = y_fm.size(0), b = y_fm.size(1);
     TORCH_CHECK_VALUE(f % k == 0, "in_dim (", f, ") has to be divisible by k (", k, ") but it is not");
     Below below(y_fm);
-    Tensor loss = at::empty({1}, y_fm.options()), dscore = at::empty({b, k}, y_fm.options()), scores;
-    if (want_scores) scores = at::empty({b, k}, y_fm.options());
+    Tensor loss = alloc({1}, y_fm), dscore = alloc({b, k}, y_fm), scores;
+    if (want_scores) scores = alloc({b, k}, y_fm);
     const size_t bytes = clb_group_sum_scratch_bytes(f, b, k, CLB_F32);
     Tensor scratch = scratch_bytes(bytes, y_fm);
     check(clb_group_sum_ce(ptr<float>(y_fm), ptr<int64_t>(labels), ptr<float>(scores), ptr<float>(dscore), ptr<float>(loss), ptr(scratch), bytes, f, b, k,
-                           tau, stream()));
+                           tau, cur_stream()));
     return {loss, dscore, scores};
 }
 
@@ -639,7 +742,7 @@ struct GroupSumCeNode : public Node {
         TORCH_CHECK(dscore.defined(), "Trying to backward through the graph a second time: specify retain_graph=True the first time");
         Below below(dscore);
         const Tensor scale = grads[0].reshape({1}).to(dscore.scalar_type()).contiguous();
-        return {batch_major_grad(group_sum_bwd(dscore, f, k, tau, scale), feeds_leaf(*this, 0))};
+        return {finished_grad(group_sum_bwd(dscore, f, k, tau, scale), feeds_leaf(*this, 0))};
     }
 };
 
@@ -648,7 +751,7 @@ Tensor group_sum_ce(const Tensor &x, const Tensor &labels, int k, double tau)
     Tensor loss, dscore;
     {
         Below below(x);
-        std::tie(loss, dscore, std::ignore) = group_sum_ce_raw(x.t(), labels.contiguous(), k, tau, false);
+        std::tie(loss, dscore, std::ignore) = group_sum_ce_raw(x, x.size(1), x.size(0), labels.contiguous(), k, tau, false);
         loss = loss.reshape({});
     }
     if (wants_grad({x})) {
@@ -666,44 +769,43 @@ struct TreeTables {
     bool covers_all; // every neuron of the first two layers sits in some tree: gate-gradient buffers need no clearing
 };
 
-void tree_fwd(const Tensor &x_fm, const TreeTables &t, const Tensor &w0, const Tensor &w1, const Tensor &w2, int wmode, const Tensor &y)
+// x_fm: a tensor whose storage is [in, B]
+void tree_fwd(const Tensor &x_fm, int64_t batch, const TreeTables &t, const Tensor &w0, const Tensor &w1, const Tensor &w2, int wmode, const Tensor &y)
 {
-    need_inputs(x_fm, t.leaf, t.node, w0, w1, w2);
     check(clb_logic_tree_fwd(ptr<float>(x_fm), ptr<int32_t>(t.leaf), ptr<int32_t>(t.node), ptr<float>(w0), ptr<float>(w1), ptr<float>(w2), ptr<float>(y),
-                             t.leaf.size(0), x_fm.size(1), wmode, stream()));
+                             t.leaf.size(0), batch, wmode, cur_stream()));
 }
 
-// upstream gradient: gy [T, B], or the head (dscore [B, k], scale [1]) of GroupSum + cross-entropy
-std::array<Tensor, 4> tree_bwd(const Tensor &x_fm, const TreeTables &t, const Tensor &w0, const Tensor &w1, const Tensor &w2, const Tensor &gy,
+// upstream gradient: gy on the storage [T, B], or the head (dscore [B, k], scale [1]) of GroupSum + cross-entropy
+std::array<Tensor, 4> tree_bwd(const Tensor &x_fm, int64_t in, int64_t b, const TreeTables &t, const Tensor &w0, const Tensor &w1, const Tensor &w2, const Tensor &gy,
                                const Tensor &dscore, const Tensor &scale, int k, double tau, int wmode, bool need_gx, std::array<Tensor, 3> gw)
 {
-    need_inputs(x_fm, t.leaf, t.node, w0, w1, w2, t.start, t.slots);
-    const int64_t trees = t.leaf.size(0), b = x_fm.size(1), in = x_fm.size(0);
+    const int64_t trees = t.leaf.size(0);
     Below below(x_fm);
-    Tensor tapgrad = at::empty({std::max<int64_t>(trees * 8, 1), b}, x_fm.options());
+    Tensor tapgrad = alloc({std::max<int64_t>(trees * 8, 1), b}, x_fm);
     const Tensor *ws[3] = {&w0, &w1, &w2};
     for (int i = 0; i < 3; ++i) {
-        if (!gw[i].defined()) gw[i] = at::empty(ws[i]->sizes(), ws[i]->options());
+        if (!gw[i].defined()) gw[i] = alloc(ws[i]->sizes(), *ws[i]);
         if (!t.covers_all) gw[i].zero_();
     }
     Tensor gx;
-    if (need_gx) gx = at::empty({in, b}, x_fm.options());
+    if (need_gx) gx = feature_major_grad(b, in, x_fm);
     if (gy.defined()) {
-        need_input(gy);
         check(clb_logic_tree_bwd(ptr<float>(x_fm), ptr<int32_t>(t.leaf), ptr<int32_t>(t.node), ptr<float>(w0), ptr<float>(w1), ptr<float>(w2),
                                  ptr<float>(gy), ptr<float>(tapgrad), ptr<float>(gw[0]), ptr<float>(gw[1]), ptr<float>(gw[2]), ptr<float>(gx),
-                                 ptr<int64_t>(t.start), ptr<int32_t>(t.slots), in, trees, b, wmode, stream()));
+                                 ptr<int64_t>(t.start), ptr<int32_t>(t.slots), in, trees, b, wmode, cur_stream()));
     } else {
         check(clb_logic_tree_bwd_scores(ptr<float>(x_fm), ptr<int32_t>(t.leaf), ptr<int32_t>(t.node), ptr<float>(w0), ptr<float>(w1), ptr<float>(w2),
                                         ptr<float>(dscore), ptr<float>(scale), k, tau, ptr<float>(tapgrad), ptr<float>(gw[0]), ptr<float>(gw[1]),
-                                        ptr<float>(gw[2]), ptr<float>(gx), ptr<int64_t>(t.start), ptr<int32_t>(t.slots), in, trees, b, wmode, stream()));
+                                        ptr<float>(gw[2]), ptr<float>(gx), ptr<int64_t>(t.start), ptr<int32_t>(t.slots), in, trees, b, wmode, cur_stream()));
     }
     return {gx, gw[0], gw[1], gw[2]};
 }
 
 struct TreeNode : public Node {
-    SavedVariable x, w0, w1, w2; // x: feature-major
+    SavedVariable x, w0, w1, w2; // x: a tensor on feature-major storage [in, batch]
     TreeTables t;
+    int64_t in, batch;
     int wmode;
     Tensor dscore; // head: GroupSum + cross-entropy
     int k = 0;
@@ -719,12 +821,12 @@ struct TreeNode : public Node {
         if (k)
             scale = grads[0].reshape({1}).to(at::kFloat).contiguous();
         else
-            gy = feature_major(grads[0]);
+            gy = feature_major_storage(grads[0]);
         Sinks sinks({a, b, c});
         const bool direct = sinks.any() && wmode != CLB_W_ARGMAX;
-        auto out = tree_bwd(xx, t, a, b, c, gy, dscore, scale, k, tau, wmode, task_should_compute_output(0),
+        auto out = tree_bwd(xx, in, batch, t, a, b, c, gy, dscore, scale, k, tau, wmode, task_should_compute_output(0),
                             direct ? std::array<Tensor, 3>{sinks.slice(0), sinks.slice(1), sinks.slice(2)} : std::array<Tensor, 3>{});
-        Tensor gx = out[0].defined() ? batch_major_grad(out[0], feeds_leaf(*this, 0)) : Tensor();
+        Tensor gx = out[0].defined() ? finished_grad(out[0], feeds_leaf(*this, 0)) : Tensor();
         if (direct) sinks.ready();
         if (direct || wmode == CLB_W_ARGMAX) return {gx, Tensor(), Tensor(), Tensor()};
         return {gx, out[1], out[2], out[3]};
@@ -743,10 +845,10 @@ Tensor trees(const Tensor &x, const Tensor &w0, const Tensor &w1, const Tensor &
     Tensor x_fm, out, dscore;
     {
         Below below(x);
-        x_fm = feature_major(x);
+        x_fm = feature_major_storage(x);
         if (!k) {
-            out = at::empty_strided({B, T}, {1, std::max<int64_t>(B, 1)}, x.options());
-            tree_fwd(x_fm, t, w0, w1, w2, wmode, out);
+            out = alloc_strided({B, T}, {1, std::max<int64_t>(B, 1)}, x);
+            tree_fwd(x_fm, B, t, w0, w1, w2, wmode, out);
         } else {
             const Tensor labels = labels_in->contiguous();
             need_input(labels);
@@ -754,16 +856,16 @@ Tensor trees(const Tensor &x, const Tensor &w0, const Tensor &w1, const Tensor &
             const size_t bytes = clb_logic_tree_fwd_ce_scratch_bytes(T, B, k);
             int rc = CLB_ERR_SHAPE;
             if (bytes && B % 4 == 0 && B <= 512 && k <= 32) { // class sums without the activation
-                out = at::empty({1}, x.options()), dscore = at::empty({B, k}, x.options());
+                out = alloc({1}, x), dscore = alloc({B, k}, x);
                 Tensor scratch = scratch_bytes(bytes, x);
                 rc = clb_logic_tree_fwd_ce(ptr<float>(x_fm), ptr<int32_t>(leaf), ptr<int32_t>(node_t), ptr<float>(w0), ptr<float>(w1), ptr<float>(w2),
-                                           ptr<int64_t>(labels), ptr<float>(dscore), ptr<float>(out), ptr(scratch), bytes, T, B, k, tau, wmode, stream());
+                                           ptr<int64_t>(labels), ptr<float>(dscore), ptr<float>(out), ptr(scratch), bytes, T, B, k, tau, wmode, cur_stream());
                 if (rc != CLB_ERR_SHAPE) check(rc);
             }
             if (rc == CLB_ERR_SHAPE) {
-                Tensor y = at::empty({T, B}, x.options());
-                tree_fwd(x_fm, t, w0, w1, w2, wmode, y);
-                std::tie(out, dscore, std::ignore) = group_sum_ce_raw(y, labels, k, tau, false);
+                Tensor y = alloc({T, B}, x);
+                tree_fwd(x_fm, B, t, w0, w1, w2, wmode, y);
+                std::tie(out, dscore, std::ignore) = group_sum_ce_raw(y, T, B, labels, k, tau, false);
             }
             out = out.reshape({});
         }
@@ -771,7 +873,8 @@ Tensor trees(const Tensor &x, const Tensor &w0, const Tensor &w1, const Tensor &
     if (graph) {
         auto node = new_node<TreeNode>();
         node->set_next_edges(torch::autograd::collect_next_edges(x, w0, w1, w2));
-        node->x = saved(x_fm), node->w0 = saved(w0), node->w1 = saved(w1), node->w2 = saved(w2), node->t = t, node->wmode = wmode;
+        node->x = saved(x_fm), node->w0 = saved(w0), node->w1 = saved(w1), node->w2 = saved(w2), node->t = t, node->in = x.size(1), node->batch = B,
+        node->wmode = wmode;
         node->dscore = dscore, node->k = k, node->tau = tau;
         torch::autograd::set_history(out, node);
     }
@@ -787,7 +890,7 @@ void adam_step(const Tensor &p, const Tensor &g, const Tensor &m, const Tensor &
     for (const Tensor *t : {&p, &g, &m, &v})
         TORCH_CHECK(t->numel() == n && t->scalar_type() == at::kFloat, "convlogic_b200: adam_step expects four float32 buffers of equal size");
     c10::cuda::CUDAGuard device(p.device());
-    check(clb_adam_step(ptr<float>(p), ptr<float>(g), ptr<float>(m), ptr<float>(v), n, lr, beta1, beta2, eps, weight_decay, step, decoupled, stream()));
+    check(clb_adam_step(ptr<float>(p), ptr<float>(g), ptr<float>(m), ptr<float>(v), n, lr, beta1, beta2, eps, weight_decay, step, decoupled, cur_stream()));
 }
 
 // ------------------------------------------------------------------------------------------------ packed inference
@@ -804,8 +907,8 @@ std::pair<Tensor, int64_t> pack_bits(const Tensor &t, int bits, bool sample_majo
     TORCH_CHECK(t.dim() == 2 && (t.scalar_type() == at::kBool || t.scalar_type() == at::kByte), "convlogic_b200: pack_bits expects a bool or uint8 tensor");
     const int64_t b = t.size(sample_major ? 0 : 1), f = t.size(sample_major ? 1 : 0);
     Below below(t);
-    Tensor packed = at::empty({f, (b + bits - 1) / bits}, t.options().dtype(type));
-    check(sample_major ? clb_pack_bits_nmajor(ptr<uint8_t>(t), ptr(packed), b, f, bits, stream()) : clb_pack_bits(ptr<uint8_t>(t), ptr(packed), f, b, bits, stream()));
+    Tensor packed = alloc({f, (b + bits - 1) / bits}, t, type);
+    check(sample_major ? clb_pack_bits_nmajor(ptr<uint8_t>(t), ptr(packed), b, f, bits, cur_stream()) : clb_pack_bits(ptr<uint8_t>(t), ptr(packed), f, b, bits, cur_stream()));
     return {packed, (bits - b % bits) % bits};
 }
 
@@ -814,9 +917,9 @@ Tensor packed_logic(const Tensor &x, const Tensor &a, const Tensor &b, const Ten
     need_inputs(x, a, b, ops);
     TORCH_CHECK(ops.scalar_type() == at::kByte, "convlogic_b200: gate ids must be uint8");
     Below below(x);
-    Tensor y = at::empty({ops.size(0), x.size(1)}, x.options());
+    Tensor y = alloc({ops.size(0), x.size(1)}, x);
     check(clb_packed_logic(ptr(x), ptr<int64_t>(a), ptr<int64_t>(b), ptr<uint8_t>(ops), ptr(y), x.size(0), ops.size(0), x.size(1), (int)x.element_size() * 8,
-                           stream()));
+                           cur_stream()));
     return y;
 }
 
@@ -826,8 +929,8 @@ Tensor group_popcount(const Tensor &x, int64_t pad, int k)
     const int64_t f = x.size(0), words = x.size(1), bits = x.element_size() * 8;
     TORCH_CHECK_VALUE(f % k == 0, "in_dim (", f, ") has to be divisible by k (", k, ") but it is not");
     Below below(x);
-    Tensor counts = at::empty({words * bits - pad, k}, x.options().dtype(at::kInt));
-    check(clb_group_popcount(ptr(x), ptr<int32_t>(counts), f, words, (int)bits, (int)pad, k, stream()));
+    Tensor counts = alloc({words * bits - pad, k}, x, at::kInt);
+    check(clb_group_popcount(ptr(x), ptr<int32_t>(counts), f, words, (int)bits, (int)pad, k, cur_stream()));
     return counts;
 }
 
@@ -844,7 +947,7 @@ public:
         check(clb_net_device_bytes(data.data(), data.size(), &need));
         c10::cuda::CUDAGuard guard(device_);
         params_ = at::empty({(int64_t)(need < 16 ? 16 : need)}, at::TensorOptions().dtype(at::kByte).device(device_));
-        check(clb_net_create(data.data(), data.size(), ptr(params_), stream(), &net_));
+        check(clb_net_create(data.data(), data.size(), ptr(params_), cur_stream(), &net_));
         c10::cuda::getCurrentCUDAStream().synchronize(); // the blob is pageable host memory: wait for the copy
         check(clb_net_info(net_, &features, &classes, &layers));
     }
@@ -871,9 +974,9 @@ public:
         Below below(params_);
         const size_t bytes = clb_net_workspace_bytes(net_, batch);
         Tensor workspace = scratch_bytes(bytes, params_);
-        Tensor counts = at::empty({batch, classes}, params_.options().dtype(at::kInt));
+        Tensor counts = alloc({batch, classes}, params_, at::kInt);
         check(clb_net_forward(net_, kind, ptr(x), thresholds ? ptr<float>(*thresholds) : nullptr, thresholds ? (int)thresholds->numel() : 0, batch,
-                              ptr<int32_t>(counts), ptr(workspace), bytes, stream()));
+                              ptr<int32_t>(counts), ptr(workspace), bytes, cur_stream()));
         return counts;
     }
     int64_t features = 0;
@@ -909,7 +1012,7 @@ py::tuple block_bwd_py(const Tensor &gy, const Tensor &x, const Tensor &w, py::o
 Tensor logic_fwd_py(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w, int wmode)
 {
     Below below(x);
-    Tensor y = at::empty({w.size(0), x.size(1)}, x.options());
+    Tensor y = alloc({w.size(0), x.size(1)}, x);
     logic_fwd(x, a, b, w, wmode, y);
     return y;
 }
@@ -919,6 +1022,7 @@ Tensor logic_fwd_py(const Tensor &x, const Tensor &a, const Tensor &b, const Ten
 PYBIND11_MODULE(_clb_torch, m)
 {
     py::class_<BlockPlan, PlanPtr>(m, "BlockPlan");
+    py::class_<LogicPlan, LogicPlanPtr>(m, "LogicPlan");
     m.def("block", &block);
     m.def("block_fwd", &block_fwd_py);
     m.def("block_bwd", &block_bwd_py);
@@ -934,6 +1038,7 @@ PYBIND11_MODULE(_clb_torch, m)
     m.def("trees", &trees);
     m.def("transpose2d", &transpose2d);
     m.def("adam_step", &adam_step);
+    m.def("count_sinks", [](int64_t change) { g_sinks += change; });
     m.def("pack_bits", &pack_bits);
     m.def("packed_logic", &packed_logic);
     m.def("group_popcount", &group_popcount);

@@ -10,6 +10,8 @@ nothing.  The reference gets the same effect implicitly from Lightning's DDP str
 import torch
 import torch.distributed as dist
 
+from ._lib import native
+
 
 def gate_parameters(model):
     """The ``weights`` parameters of every logic layer, in module order."""
@@ -115,6 +117,8 @@ class GradBucket:
         (its slice is overwritten, not added to) -- true of the layer stacks this library models.  With ``overlap()``
         active the slice is all-reduced the moment its kernel has been enqueued, as the hooks would do."""
         for p, (lo, hi) in zip(self.params, self.ranges):
+            if p.is_cuda and bool(on) != hasattr(p, "_clb_grad_sink"):
+                native().count_sinks(1 if on else -1)  # backward passes look for sinks while any parameter carries one
             if on:
                 p._clb_grad_sink = (self.flat[lo:hi].view_as(p), lambda lo=lo, hi=hi: self._slice_ready(lo, hi) if self._hooks else None,
                                     self._ranges_ready, (lo, hi))
@@ -200,8 +204,6 @@ class FlatAdam:
     trains with: src/convlogic/model.py:179-180) to fp32 rounding."""
 
     def __init__(self, bucket, lr=1e-3, betas=(0.9, 0.999), eps=1e-8, weight_decay=0.0, decoupled=False):
-        from ._lib import native
-
         self._adam_step = native().adam_step
         self.bucket, self.lr, self.betas, self.eps, self.weight_decay, self.decoupled = bucket, lr, betas, eps, weight_decay, decoupled
         self.params = torch.empty_like(bucket.flat)

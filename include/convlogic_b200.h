@@ -241,6 +241,21 @@ int clb_tree_bwd_w(const void *gy, const void *x, const void *w, void *gw, void 
  */
 int clb_logic_fwd(const void *x, const int64_t *a, const int64_t *b, const void *w, void *y, int64_t in_dim,
                   int64_t out_dim, int64_t B, int wmode, int dtype, void *stream);
+/* The same, also writing what the combined backward below reads: coef [out][4] = (k1, ka, kb, kab) of every neuron's gate,
+ * y = k1 + ka*a + kb*b + kab*a*b (16-byte aligned; NULL: not written). */
+int clb_logic_fwd_coef(const void *x, const int64_t *a, const int64_t *b, const void *w, void *y, void *coef, int64_t in_dim,
+                       int64_t out_dim, int64_t B, int wmode, int dtype, void *stream);
+/* Both gradients of a flat layer in one pass over the rows (fp32; stands in for the pair backward_w + backward_x that the
+ * reference's autograd Function calls, src/difflogic/difflogic.py:219-230).  clb_logic_entries lays the consumer lists out once
+ * per layer: start32 int32 [in+1], entry 8 bytes per list entry [2*out].  gx [in][B] required, gw [out][16] may be NULL;
+ * scratch: clb_logic_bwd_scratch_bytes(in, out, B), 16-byte aligned.  CLB_ERR_SHAPE for rows it does not take (B a multiple of
+ * 4 with unaligned pointers, sizes beyond 2^30): use clb_logic_bwd_w / clb_logic_bwd_x.  Fixed summation order. */
+int clb_logic_entries(const int64_t *a, const int64_t *b, const int64_t *start, const int64_t *consumers, int32_t *start32, void *entry,
+                      int64_t in_dim, int64_t out_dim, void *stream);
+size_t clb_logic_bwd_scratch_bytes(int64_t in_dim, int64_t out_dim, int64_t B);
+int clb_logic_bwd(const float *x, const float *w, const float *coef, const float *gy, float *gx, float *gw, const int32_t *start32,
+                  const void *entry, void *scratch, size_t scratch_bytes, int64_t in_dim, int64_t out_dim, int64_t B, int wmode,
+                  void *stream);
 int clb_logic_bwd_w(const void *x, const int64_t *a, const int64_t *b, const void *w, const void *gy, void *gw,
                     int64_t in_dim, int64_t out_dim, int64_t B, int wmode, int dtype, void *stream);
 int clb_logic_bwd_x(const void *x, const int64_t *a, const int64_t *b, const void *w, const void *gy, void *gx,
