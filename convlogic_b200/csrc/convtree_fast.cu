@@ -1248,12 +1248,16 @@ int clb_convtree_fwd_fast_f32(const float *x, const float *w, const int32_t *sel
 {
     FastShape s;
     if (sh != 1 || sw != 1) return CLB_ERR_SHAPE;
-    // many input channels: an image's channels do not fit shared memory (or barely one image does)
-    if ((size_t)Ci * (H + 2 * ph) * (W + 2 * pw) * 4 > 48 * 1024) {
+    // The plane kernels (images of 16, 8 or 4 pixels) stream two channel planes per output channel; the tiled ones below stage all
+    // channels of a few images.  With few channels and few windows the latter have less set-up (1 -> 64 channels, 16x16, batch 64: 6.1
+    // against 7.9 us); otherwise the former are faster whatever the channel count (9 -> 128, 16x16, batch 256: 24.8 against 32.3;
+    // 32 -> 128, batch 100: 13.3 against 35.6, batch 500: 41 against 70; 16 -> 1024, 4x4, batch 500: 38 against 85).
+    const bool many_channels = (size_t)Ci * (H + 2 * ph) * (W + 2 * pw) * 4 > 48 * 1024;
+    if (many_channels || Ci >= 16 || (long long)N * C * H * W >= (4LL << 20)) {
         const int rc = clb_convtree_fwd_plane_f32(x, w, sel, y, amax, N, Ci, H, W, C, sh, sw, ph, pw, kh, kw, wmode, st);
         if (rc != CLB_ERR_SHAPE) return rc;
-        return launch_fwd_chan(x, w, sel, y, amax, N, Ci, H, W, C, ph, pw, kh, kw, wmode, st);
     }
+    if (many_channels) return launch_fwd_chan(x, w, sel, y, amax, N, Ci, H, W, C, ph, pw, kh, kw, wmode, st);
     if (!make_fast_shape(s, N, Ci, H, W, C, sh, sw, ph, pw, kh, kw, wmode)) return CLB_ERR_SHAPE;
     const int I = (s.Ho / 2) * (s.Wo / 2);
     const size_t img_bytes = (size_t)s.IS * 4;
