@@ -17,6 +17,7 @@
 // The last flat layer's outputs are summed per class (GroupSum): counts[b][k].
 #include "clb_common.cuh"
 #include "clb_net.cuh"
+#include "clb_slab.cuh"
 
 #include <cstring>
 #include <new>
@@ -53,6 +54,8 @@ struct Layer {
     long long in_dim, out_dim;
     int levels;
     size_t off_a, off_b, off_ops;
+    bool slab3 = false;   // a 3x3 block of the stacks' geometry: its tap records are laid out when the network is created
+    size_t off_recs = 0;  // behind the blob in the parameter memory
 };
 
 } // namespace
@@ -62,15 +65,14 @@ struct clb_net {
     int num_classes = 0;
     int in_channels = 0, in_h = 0, in_w = 0;
     long long in_features = 0; // features of one sample at the input
-    size_t param_bytes = 0;    // the blob is copied to the device as it is
+    size_t param_bytes = 0;    // the blob, copied to the device as it is, and the tap records behind it
     const unsigned char *dev = nullptr;
     size_t max_conv_channels = 0;
     clb::NetPlan plan = {};     // for the one-launch kernel
     bool one_launch = false;    // the stack has the form that kernel takes
     long long slab_cost = 0;    // gate trees per 128-sample slab, a conv window counting as four
 };
-
-int clb_pack_bits_units(const uint8_t *t, void *packed, int64_t N, int64_t F, int64_t U, int64_t HW, cudaStream_t st); // packed.cu
+ // packed.cu
 int clb_net_cluster_launch(const clb::NetPlan &net, const void *input, const float *thresholds, const unsigned char *params, void *work,
                            int32_t *counts, int64_t batch, cudaStream_t st); // net_cluster.cu
 
@@ -155,6 +157,10 @@ static bool parse(const void *blob, size_t bytes, clb_net &net)
         } else {
             return false;
         }
+        if (L.kind == 1 && clb_slab3_covers(L.H, L.W, L.stride, L.stride, L.ph, L.pw, L.kh, L.kw)) {
+            L.slab3 = true, L.off_recs = (net.param_bytes + 255) / 256 * 256;
+            net.param_bytes = L.off_recs + clb_slab3_record_bytes(L.C);
+        }
         net.layers.push_back(L);
     }
     return feat % net.num_classes == 0;
@@ -222,7 +228,7 @@ extern "C" int clb_net_device_bytes(const void *blob, size_t bytes, size_t *devi
     clb_net tmp;
     if (!device_bytes) return CLB_ERR_ARG;
     if (!parse(blob, bytes, tmp)) return CLB_ERR_SHAPE;
-    *device_bytes = bytes;
+    *device_bytes = tmp.param_bytes;
     return CLB_OK;
 }
 
@@ -241,6 +247,15 @@ extern "C" int clb_net_create(const void *blob, size_t bytes, void *device_mem, 
         return check_launch(0);
     }
     net->dev = (const unsigned char *)device_mem;
+    for (const Layer &L : net->layers) {
+        if (!L.slab3) continue;
+        const int rc = clb_slab3_records(net->dev + L.off_ops, (const int32_t *)(net->dev + L.off_a), (unsigned char *)device_mem + L.off_recs, L.Ci, L.H, L.C,
+                                         (cudaStream_t)stream);
+        if (rc != CLB_OK) {
+            delete net;
+            return rc;
+        }
+    }
     plan_one_launch(*net);
     *out = net;
     return CLB_OK;
@@ -302,28 +317,31 @@ extern "C" int clb_net_forward(const clb_net *net, int input_kind, const void *i
     void *scratch = (unsigned char *)workspace + 2 * act;
     const bool image = net->in_channels > 0;
     const Layer &first = net->layers.front();
-    // conv blocks run on the slab layout where the kernel covers them (stride 1, <= 256 pooled outputs per image)
-    auto slab_ok = [](const Layer &L) { return L.kind == 1 && L.stride == 1 && L.Hp * L.Wp <= 256; };
-    bool slab = image && slab_ok(first);
+    // conv blocks run on slabs where a kernel covers them (stride 1, <= 256 pooled outputs per image), and the stacks' own geometry
+    // takes and gives them in split order; the order of the activations that a layer wants:
+    auto wanted = [&](size_t i) {
+        if (i >= net->layers.size() || net->layers[i].kind != 1) return clb::kRows;
+        const Layer &L = net->layers[i];
+        return L.slab3 ? clb::kSplitSlabs : L.stride == 1 && L.Hp * L.Wp <= 256 ? clb::kSlabs : clb::kRows;
+    };
+    clb::Order order = image ? wanted(0) : clb::kRows; // of the current activations
+    const int64_t in_hw = (int64_t)net->in_h * net->in_w;
+    cudaStream_t cs = (cudaStream_t)stream;
     int cur = 0, st;
 
     // ---- input stage
     if (input_kind == 0) {
-        st = clb_pack_bits_units((const uint8_t *)input, buf[0], batch, net->in_features, U, slab ? (int64_t)net->in_h * net->in_w : 0, (cudaStream_t)stream);
+        st = clb_pack_bits_units((const uint8_t *)input, buf[0], batch, net->in_features, U, in_hw, net->in_w, order, cs);
         if (st != CLB_OK) return st;
     } else if (input_kind == 1 || input_kind == 2) {
         if (!image || !thresholds || levels <= 0 || net->in_channels % levels) return CLB_ERR_SHAPE;
-        st = clb_thermometer_pack(input, input_kind == 2, thresholds, levels, buf[0], batch, net->in_channels / levels,
-                                  (int64_t)net->in_h * net->in_w, words, slab ? 1 : 0, stream);
+        st = clb_thermometer_pack_units(input, input_kind == 2, thresholds, levels, buf[0], batch, net->in_channels / levels, in_hw, words, net->in_w, order, cs);
+        if (st != CLB_OK) return st;
+    } else if (order != clb::kRows) {
+        st = clb_packed_rows_to_slabs(input, buf[0], net->in_channels, in_hw, U, net->in_w, order, cs);
         if (st != CLB_OK) return st;
     } else {
-        if (slab) {
-            st = clb_packed_layout(input, buf[0], net->in_channels, (int64_t)net->in_h * net->in_w, U, 1, stream);
-            if (st != CLB_OK) return st;
-        } else {
-            if (cudaMemcpyAsync(buf[0], input, (size_t)net->in_features * rb, cudaMemcpyDeviceToDevice, (cudaStream_t)stream) != cudaSuccess)
-                return check_launch(0);
-        }
+        if (cudaMemcpyAsync(buf[0], input, (size_t)net->in_features * rb, cudaMemcpyDeviceToDevice, cs) != cudaSuccess) return check_launch(0);
     }
 
     // ---- layers
@@ -332,32 +350,36 @@ extern "C" int clb_net_forward(const clb_net *net, int input_kind, const void *i
     for (size_t i = 0; i < net->layers.size(); ++i) {
         const Layer &L = net->layers[i];
         if (L.kind == 1) {
-            const bool want_slab = slab_ok(L);
-            if (slab != want_slab) { // change of layout between blocks
-                st = clb_packed_layout(buf[cur], buf[cur ^ 1], L.Ci, (int64_t)L.H * L.W, U, want_slab ? 1 : 0, stream);
+            const clb::Order want = wanted(i), next = wanted(i + 1);
+            if ((order == clb::kRows) != (want == clb::kRows)) { // change of layout between blocks
+                st = want == clb::kRows ? clb_packed_layout(buf[cur], buf[cur ^ 1], L.Ci, (int64_t)L.H * L.W, U, 0, stream)
+                                        : clb_packed_rows_to_slabs(buf[cur], buf[cur ^ 1], L.Ci, (int64_t)L.H * L.W, U, L.W, want, cs);
                 if (st != CLB_OK) return st;
-                cur ^= 1, slab = want_slab;
+                cur ^= 1, order = want;
             }
-            if (slab) {
+            if (L.slab3) { // takes either slab order and writes what the next layer reads
+                st = clb_slab3_block(buf[cur], P + L.off_recs, buf[cur ^ 1], L.Ci, L.H, L.C, U, order, next, cs);
+                order = next;
+            } else if (order != clb::kRows) {
                 st = clb_packed_convtree_slab(buf[cur], P + L.off_ops, (const int32_t *)(P + L.off_a), buf[cur ^ 1], scratch, L.Ci, L.H, L.W,
                                               L.C, 1, 1, L.ph, L.pw, L.kh, L.kw, U, stream);
                 if (st == CLB_ERR_SHAPE) { // a tile the slab kernel cannot hold: this block runs on the rows layout
                     st = clb_packed_layout(buf[cur], buf[cur ^ 1], L.Ci, (int64_t)L.H * L.W, U, 0, stream);
                     if (st != CLB_OK) return st;
-                    cur ^= 1, slab = false;
+                    cur ^= 1, order = clb::kRows;
                 }
             }
-            if (!slab)
+            if (!L.slab3 && order == clb::kRows)
                 st = clb_packed_convtree(buf[cur], P + L.off_ops, (const int32_t *)(P + L.off_a), buf[cur ^ 1], L.Ci, L.H, L.W, L.C,
                                          L.stride, L.stride, L.ph, L.pw, L.kh, L.kw, words, 64, stream);
             if (st != CLB_OK) return st;
             cur ^= 1;
             feat = (long long)L.C * L.Hp * L.Wp;
             const bool last_conv = i + 1 == net->layers.size() || net->layers[i + 1].kind != 1;
-            if (last_conv && slab) { // Flatten: back to feature rows
+            if (last_conv && order != clb::kRows) { // Flatten: back to feature rows
                 st = clb_packed_layout(buf[cur], buf[cur ^ 1], L.C, (int64_t)L.Hp * L.Wp, U, 0, stream);
                 if (st != CLB_OK) return st;
-                cur ^= 1, slab = false;
+                cur ^= 1, order = clb::kRows;
             }
         } else if (L.kind == 2) {
             st = clb_packed_logic(buf[cur], (const int64_t *)(P + L.off_a), (const int64_t *)(P + L.off_b), P + L.off_ops, buf[cur ^ 1],

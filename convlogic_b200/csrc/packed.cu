@@ -11,6 +11,7 @@
 // two-level multiplexer  y = a ? (b ? m11 : m10) : (b ? m01 : m00): three 3-input logic operations per
 // 32 bits, branch-free, with the masks uniform over the thread block.
 #include "clb_common.cuh"
+#include "clb_slab.cuh"
 
 #include <type_traits>
 
@@ -62,7 +63,7 @@ __device__ __forceinline__ unsigned nonzero_bytes(unsigned v) { return ((((v & 0
 
 template <bool QUAD>
 __global__ void __launch_bounds__(256) pack_bits_nmajor_kernel(const uint8_t *__restrict__ t, uint8_t *__restrict__ out, long long N, long long F,
-                                                               long long rowbytes, int word_stores, int HW, long long U)
+                                                               long long rowbytes, int word_stores, int HW, int side, long long U)
 {
     __shared__ unsigned sm[128 * 9];
     const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
@@ -101,13 +102,15 @@ __global__ void __launch_bounds__(256) pack_bits_nmajor_kernel(const uint8_t *__
             sm[(4 * lane + k) * 9 + wv] = (lo & 0xffffu) | (hi << 16);
         }
         __syncthreads();
-        if (HW > 0) { // slab layout [channel][U][HW] of 16-byte units
+        if (HW > 0) { // slab layout [channel][U][HW] of 16-byte units, in split order if a side is given
             for (int e = threadIdx.x; e < 1024; e += 256) {
                 const int q = e & 3, i = (e >> 2) & 127, h = e >> 9;
                 const long long u = n0 / 128 + h, ff = f0 + i;
                 if (ff < F && u < U) {
                     const long long c = ff / HW;
-                    reinterpret_cast<unsigned *>(out)[((c * U + u) * HW + (ff - c * HW)) * 4 + q] = sm[i * 9 + 4 * h + q];
+                    int yx = (int)(ff - c * HW);
+                    if (side) yx = split_position(yx, side);
+                    reinterpret_cast<unsigned *>(out)[((c * U + u) * HW + yx) * 4 + q] = sm[i * 9 + 4 * h + q];
                 }
             }
         } else if (word_stores) {
@@ -152,7 +155,7 @@ __device__ __forceinline__ float pixel_value<uint8_t>(const uint8_t *p)
 template <typename PIX>
 __global__ void __launch_bounds__(256) thermometer_pack_kernel(const PIX *__restrict__ pix, const float *__restrict__ thr, int L,
                                                                unsigned *__restrict__ out, long long N, int P, int HW,
-                                                               long long words32, int to_slab)
+                                                               long long words32, int to_slab, int side)
 {
     __shared__ unsigned sm[kThermoLevels * 32 * 9];
     __shared__ unsigned lut[256]; // uint8 pixels: level mask of every pixel value
@@ -233,7 +236,9 @@ __global__ void __launch_bounds__(256) thermometer_pack_kernel(const PIX *__rest
             const int pp = blockIdx.x * 32 + pos;
             const long long u = w0 / 4 + u2;
             if (pp < P && u < U) {
-                const int c = pp / HW, yx = pp - c * HW;
+                const int c = pp / HW;
+                int yx = pp - c * HW;
+                if (side) yx = split_position(yx, side);
                 unsigned *dst = out + ((((long long)l0 * (P / HW) + c) * U + u) * HW + yx) * 4 + q;
                 const unsigned *srcw = sm + pos * 9 + u2 * 4 + q;
                 const long long dstep = (long long)(P / HW) * U * HW * 4;
@@ -894,15 +899,16 @@ __global__ void __launch_bounds__(256, 2) packed_convtree_slab_kernel(const uint
 }
 
 // rows [F][2U] of 64-bit words  <->  slab [C][U][HW] of uint4, F = C*HW (pure data movement)
-__global__ void packed_rows_to_slab_kernel(const uint4 *__restrict__ rows, uint4 *__restrict__ slab, int C, int HW, int U, int to_slab)
+__global__ void packed_rows_to_slab_kernel(const uint4 *__restrict__ rows, uint4 *__restrict__ slab, int C, int HW, int U, int to_slab, int side)
 {
     const long long total = (long long)C * HW * U;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         // i enumerates the rows layout: ((c*HW + p)*U + u)
         const int u = (int)(i % U);
         const long long cp = i / U;
-        const int p = (int)(cp % HW);
+        int p = (int)(cp % HW);
         const long long c = cp / HW;
+        if (side) p = split_position(p, side);
         const long long j = (c * U + u) * HW + p;
         if (to_slab)
             slab[j] = rows[i];
@@ -937,16 +943,16 @@ extern "C" int clb_pack_bits(const uint8_t *t, void *packed, int64_t F, int64_t 
 }
 
 // rows of `rowbytes` bytes (HW == 0) or the slab layout [F / HW][U][HW] of 16-byte units
-static int pack_nmajor(const uint8_t *t, void *packed, int64_t N, int64_t F, int64_t rowbytes, int64_t HW, int64_t U, cudaStream_t st)
+static int pack_nmajor(const uint8_t *t, void *packed, int64_t N, int64_t F, int64_t rowbytes, int64_t HW, int side, int64_t U, cudaStream_t st)
 {
     long long gy = (rowbytes + 31) / 32;
     if (gy > 4096) gy = 4096;
     const dim3 grid((unsigned)((F + 127) / 128), (unsigned)gy);
     const int words = rowbytes % 4 == 0 && aligned_to(packed, 4);
     if (F % 4 == 0 && aligned_to(t, 4))
-        CLB_TRACED("pack_bits_nmajor_kernel", st, pack_bits_nmajor_kernel<true><<<grid, 256, 0, st>>>(t, (uint8_t *)packed, N, F, rowbytes, words, (int)HW, U));
+        CLB_TRACED("pack_bits_nmajor_kernel", st, pack_bits_nmajor_kernel<true><<<grid, 256, 0, st>>>(t, (uint8_t *)packed, N, F, rowbytes, words, (int)HW, side, U));
     else
-        CLB_TRACED("pack_bits_nmajor_kernel", st, pack_bits_nmajor_kernel<false><<<grid, 256, 0, st>>>(t, (uint8_t *)packed, N, F, rowbytes, words, (int)HW, U));
+        CLB_TRACED("pack_bits_nmajor_kernel", st, pack_bits_nmajor_kernel<false><<<grid, 256, 0, st>>>(t, (uint8_t *)packed, N, F, rowbytes, words, (int)HW, side, U));
     return check_launch();
 }
 
@@ -955,17 +961,16 @@ extern "C" int clb_pack_bits_nmajor(const uint8_t *t, void *packed, int64_t N, i
     if (!t || !packed || F < 0 || N < 0 || !bits_ok(bits)) return CLB_ERR_ARG;
     const long long words = (N + bits - 1) / bits, rowbytes = words * (bits / 8);
     if (F == 0 || rowbytes == 0) return CLB_OK;
-    return pack_nmajor(t, packed, N, F, rowbytes, 0, 0, (cudaStream_t)stream);
+    return pack_nmajor(t, packed, N, F, rowbytes, 0, 0, 0, (cudaStream_t)stream);
 }
 
-// The same with the batch padded to U units of 128 samples (zero bits): rows of U units, or with HW > 0 the slab layout.
-int clb_pack_bits_units(const uint8_t *t, void *packed, int64_t N, int64_t F, int64_t U, int64_t HW, cudaStream_t st)
+int clb_pack_bits_units(const uint8_t *t, void *packed, int64_t N, int64_t F, int64_t U, int64_t HW, int side, Order order, cudaStream_t st)
 {
-    return pack_nmajor(t, packed, N, F, U * 16, HW, U, st);
+    return pack_nmajor(t, packed, N, F, U * 16, order == kRows ? 0 : HW, order == kSplitSlabs ? side : 0, U, st);
 }
 
-extern "C" int clb_thermometer_pack(const void *pixels, int pixels_u8, const float *thresholds, int levels, void *packed, int64_t N,
-                                    int64_t channels, int64_t HW, int64_t words, int to_slab, void *stream)
+int clb_thermometer_pack_units(const void *pixels, int pixels_u8, const float *thresholds, int levels, void *packed, int64_t N, int64_t channels, int64_t HW,
+                               int64_t words, int side, Order order, cudaStream_t st)
 {
     if (!pixels || !thresholds || !packed || levels <= 0 || N < 0 || channels <= 0 || HW <= 0 || words < 0) return CLB_ERR_ARG;
     const long long P = channels * HW;
@@ -975,19 +980,26 @@ extern "C" int clb_thermometer_pack(const void *pixels, int pixels_u8, const flo
     if (words < need || words > need + 1) return CLB_ERR_SHAPE; // rows of ceil(N/64) words, or one more to reach an even count
     if (words == 0) return CLB_OK;
     const long long words32 = words * 2;
+    const int to_slab = order != kRows;
     if (to_slab && (words32 % 4)) return CLB_ERR_SHAPE; // a slab unit is 128 samples
+    if (order != kSplitSlabs) side = 0;
     if (!aligned_to(packed, 16)) return CLB_ERR_ARG;
     const long long gy = (words32 + 7) / 8; // a block writes 8 half-words of every row: all of them are written, bits beyond N as zeros
     if (gy > 65535) return CLB_ERR_SHAPE;
     dim3 grid((unsigned)((P + 31) / 32), (unsigned)gy);
-    cudaStream_t st = (cudaStream_t)stream;
     if (pixels_u8)
         CLB_TRACED("thermometer_pack_kernel", st, thermometer_pack_kernel<uint8_t><<<grid, 256, 0, st>>>((const uint8_t *)pixels, thresholds, levels, (unsigned *)packed, N, (int)P,
-                                                                (int)HW, words32, to_slab));
+                                                                (int)HW, words32, to_slab, side));
     else
         CLB_TRACED("thermometer_pack_kernel", st, thermometer_pack_kernel<float><<<grid, 256, 0, st>>>((const float *)pixels, thresholds, levels, (unsigned *)packed, N, (int)P, (int)HW,
-                                                              words32, to_slab));
+                                                              words32, to_slab, side));
     return check_launch();
+}
+
+extern "C" int clb_thermometer_pack(const void *pixels, int pixels_u8, const float *thresholds, int levels, void *packed, int64_t N,
+                                    int64_t channels, int64_t HW, int64_t words, int to_slab, void *stream)
+{
+    return clb_thermometer_pack_units(pixels, pixels_u8, thresholds, levels, packed, N, channels, HW, words, 0, to_slab ? kSlabs : kRows, (cudaStream_t)stream);
 }
 
 extern "C" int clb_packed_logic(const void *x, const int64_t *a, const int64_t *b, const uint8_t *ops, void *y, int64_t in_dim,
@@ -1146,19 +1158,32 @@ extern "C" int clb_packed_convtree(const void *x, const uint8_t *ops, const int3
     return check_launch();
 }
 
-extern "C" int clb_packed_layout(const void *src, void *dst, int64_t C, int64_t HW, int64_t U, int to_slab, void *stream)
+static int packed_layout(const void *src, void *dst, int64_t C, int64_t HW, int64_t U, int to_slab, int side, cudaStream_t st)
 {
     if (!src || !dst || C < 0 || HW < 0 || U < 0) return CLB_ERR_ARG;
     if (!aligned_to(src, 16) || !aligned_to(dst, 16)) return CLB_ERR_ARG;
     if (C > 0x7fffffff || HW > 0x7fffffff || U > 0x7fffffff) return CLB_ERR_SHAPE;
     const long long total = C * HW * U;
     if (total == 0) return CLB_OK;
-    CLB_TRACED("packed_rows_to_slab_kernel", (cudaStream_t)stream, packed_rows_to_slab_kernel<<<flat_grid(total, 256), 256, 0, (cudaStream_t)stream>>>((const uint4 *)src, (uint4 *)dst, (int)C, (int)HW,
-                                                                                        (int)U, to_slab));
+    CLB_TRACED("packed_rows_to_slab_kernel", st, packed_rows_to_slab_kernel<<<flat_grid(total, 256), 256, 0, st>>>((const uint4 *)src, (uint4 *)dst, (int)C, (int)HW,
+                                                                                        (int)U, to_slab, side));
     return check_launch();
 }
+extern "C" int clb_packed_layout(const void *src, void *dst, int64_t C, int64_t HW, int64_t U, int to_slab, void *stream)
+{
+    return packed_layout(src, dst, C, HW, U, to_slab, 0, (cudaStream_t)stream);
+}
+int clb_packed_rows_to_slabs(const void *rows, void *slabs, int64_t C, int64_t HW, int64_t U, int side, Order order, cudaStream_t st)
+{
+    return packed_layout(rows, slabs, C, HW, U, 1, order == kSplitSlabs ? side : 0, st);
+}
 
-extern "C" int64_t clb_packed_convtree_slab_scratch_bytes(int C) { return C < 0 ? 0 : (int64_t)C * (int64_t)sizeof(SlabRec); }
+extern "C" int64_t clb_packed_convtree_slab_scratch_bytes(int C)
+{
+    if (C < 0) return 0;
+    const int64_t a = (int64_t)C * (int64_t)sizeof(SlabRec), b = (int64_t)clb_slab3_record_bytes(C);
+    return a > b ? a : b;
+}
 
 extern "C" int clb_packed_convtree_slab(const void *x, const uint8_t *ops, const int32_t *sel, void *y, void *scratch, int Ci, int H,
                                         int W, int C, int sh, int sw, int ph, int pw, int kh, int kw, int64_t U, void *stream)
@@ -1175,6 +1200,10 @@ extern "C" int clb_packed_convtree_slab(const void *x, const uint8_t *ops, const
     if (C > 65535 || I > 256 || U > 0x7fffffff) return CLB_ERR_SHAPE;
     if ((long long)Ci * U * H * W >= (1LL << 31) || (long long)C * U * I >= (1LL << 31)) return CLB_ERR_SHAPE;
     if (C == 0 || U == 0) return CLB_OK;
+    if (clb_slab3_covers(H, W, sh, sw, ph, pw, kh, kw)) { // the stacks' own geometry
+        const int rc = clb_slab3_records(ops, sel, scratch, Ci, H, C, (cudaStream_t)stream);
+        return rc != CLB_OK ? rc : clb_slab3_block(x, scratch, y, Ci, H, C, U, kSlabs, kSlabs, (cudaStream_t)stream);
+    }
     s.U = (int)U;
     s.UB = 256 / I;
     if (s.UB > s.U) s.UB = s.U;
