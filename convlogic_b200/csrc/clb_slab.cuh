@@ -39,3 +39,5 @@ int clb_pack_bits_units(const uint8_t *t, void *packed, int64_t N, int64_t F, in
 int clb_thermometer_pack_units(const void *pixels, int pixels_u8, const float *thresholds, int levels, void *packed, int64_t N, int64_t channels, int64_t HW,
                                int64_t words, int side, clb::Order order, cudaStream_t st);
 int clb_packed_rows_to_slabs(const void *rows, void *slabs, int64_t C, int64_t HW, int64_t U, int side, clb::Order order, cudaStream_t st);
+// class sums over rows of U units, of whose samples the first B count
+int clb_group_popcount_units(const void *x, int32_t *counts, int64_t F, int64_t U, int64_t B, int k, cudaStream_t st);

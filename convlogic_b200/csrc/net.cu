@@ -395,16 +395,6 @@ extern "C" int clb_net_forward(const clb_net *net, int input_kind, const void *i
             feat = L.out_dim;
         }
     }
-    // ---- GroupSum: pad bits are the zero samples of the input, but gates such as NOT turn them on: exclude them
-    const int pad = (int)(words * 64 - batch);
-    if (pad >= 64) { // the kernel takes a pad below one word: count on the narrower view is not possible, so mask by size
-        // rows are [feat][words]; a pad of 64..127 samples means the last word of every row is padding only
-        // -> run the count on words-1 words per row through a strided copy
-        const size_t narrow = (size_t)(words - 1) * 8;
-        if (cudaMemcpy2DAsync(buf[cur ^ 1], narrow, buf[cur], rb, narrow, (size_t)feat, cudaMemcpyDeviceToDevice, (cudaStream_t)stream) !=
-            cudaSuccess)
-            return check_launch(0);
-        return clb_group_popcount(buf[cur ^ 1], counts, feat, words - 1, 64, pad - 64, net->num_classes, stream);
-    }
-    return clb_group_popcount(buf[cur], counts, feat, words, 64, pad, net->num_classes, stream);
+    // ---- GroupSum over the samples of the batch: gates such as NOT turn the zero samples behind them on
+    return clb_group_popcount_units(buf[cur], counts, feat, U, batch, net->num_classes, cs);
 }

@@ -399,7 +399,7 @@ __device__ __forceinline__ void csa(unsigned &hi, unsigned &lo, unsigned a, unsi
 
 // PLANES bit planes above the sixteens: a warp can count 16 * 2^PLANES rows, and so can the sum of the eight warps
 template <int PLANES>
-__global__ void __launch_bounds__(256) group_popcount_kernel(const unsigned *__restrict__ x, int *__restrict__ counts, long long S, long long units, long long B,
+__global__ void __launch_bounds__(256, 3) group_popcount_kernel(const unsigned *__restrict__ x, int *__restrict__ counts, long long S, long long units, long long B,
                                                              int k)
 {
     constexpr int P = PLANES + 4;
@@ -413,15 +413,22 @@ __global__ void __launch_bounds__(256) group_popcount_kernel(const unsigned *__r
     for (int p = 0; p < P; ++p) n[p] = 0;
     if (u < units) {
         const unsigned *pr = x + ((long long)cls * S + r_lo) * units + u; // walks down the rows: one addition per load, no multiplication
-        for (long long r = r_lo; r < r_hi; r += 16) {
-            unsigned v[16];
+        unsigned next[16]; // sixteen rows ahead
+        auto load = [&](long long r) {
             if (r + 16 <= r_hi) {
 #pragma unroll
-                for (int q = 0; q < 16; ++q) v[q] = __ldg(pr), pr += units;
+                for (int q = 0; q < 16; ++q) next[q] = __ldg(pr), pr += units;
             } else {
 #pragma unroll
-                for (int q = 0; q < 16; ++q) v[q] = (r + q < r_hi) ? __ldg(pr + q * units) : 0u;
+                for (int q = 0; q < 16; ++q) next[q] = (r + q < r_hi) ? __ldg(pr + q * units) : 0u;
             }
+        };
+        load(r_lo);
+        for (long long r = r_lo; r < r_hi; r += 16) {
+            unsigned v[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = next[q];
+            load(r + 16);
             unsigned t2a, t2b, t4a, t4b, t8a, t8b, carry;
             csa(t2a, n[0], n[0], v[0], v[1]);
             csa(t2b, n[0], n[0], v[2], v[3]);
@@ -1084,21 +1091,18 @@ extern "C" int clb_packed_tree(const void *x, const int32_t *leaf, const uint8_t
     return check_launch();
 }
 
-extern "C" int clb_group_popcount(const void *x, int32_t *counts, int64_t F, int64_t words, int bits, int pad_len, int k,
-                                  void *stream)
+// Rows of rowbytes bytes of which B samples count (whatever the bits behind them).
+static int group_popcount(const void *x, int32_t *counts, int64_t F, long long rowbytes, long long B, int k, cudaStream_t st)
 {
-    if (!x || !counts || F < 0 || words < 0 || !bits_ok(bits) || k <= 0 || pad_len < 0 || pad_len >= bits) return CLB_ERR_ARG;
-    if (F % k) return CLB_ERR_SHAPE;
-    const long long rowbytes = words * (bits / 8);
-    const long long B = words * bits - pad_len;
     if (B <= 0) return CLB_OK;
     const long long S = F / k;
-    cudaStream_t st = (cudaStream_t)stream;
     if (rowbytes % 4 == 0 && aligned_to(x, 4)) {
         const long long units = rowbytes / 4, ublocks = (units + 31) / 32;
-        // parts of a class: four blocks per SM in all, at least 16 rows per warp
-        long long parts = 1;
-        while (ublocks * k * parts < (long long)sm_count() * 4 && S / (parts * 2) >= 128) parts *= 2;
+        // parts of a class: three blocks per SM in all, at least 16 rows per warp.  All of them run at once (a second, short wave
+        // cost 30 of 150 us for 335 MB), and no more parts than that, as each adds its counts with atomics.
+        long long parts = 3LL * sm_count() / (ublocks * k);
+        if (parts > S / 128) parts = S / 128;
+        if (parts < 1) parts = 1;
         if (ublocks > 0x7fffffffLL || k > 65535) return CLB_ERR_SHAPE;
         if (parts > 1 && cudaMemsetAsync(counts, 0, (size_t)B * k * sizeof(int32_t), st) != cudaSuccess) return check_launch(0);
         const dim3 grid((unsigned)ublocks, (unsigned)parts, (unsigned)k);
@@ -1107,8 +1111,8 @@ extern "C" int clb_group_popcount(const void *x, int32_t *counts, int64_t F, int
             CLB_TRACED("group_popcount_kernel", st,
                        group_popcount_kernel<decltype(planes)::value><<<grid, 256, 0, st>>>((const unsigned *)x, counts, S, units, B, k));
         };
-        if (rows < (1LL << 12))
-            go(std::integral_constant<int, 8>{});
+        if (rows < (1LL << 14))
+            go(std::integral_constant<int, 10>{});
         else if (rows < (1LL << 20))
             go(std::integral_constant<int, 16>{});
         else
@@ -1117,6 +1121,17 @@ extern "C" int clb_group_popcount(const void *x, int32_t *counts, int64_t F, int
         CLB_TRACED("group_popcount_bytes_kernel", st, group_popcount_bytes_kernel<<<flat_grid(B * k, 256), 256, 0, st>>>((const uint8_t *)x, counts, S, rowbytes, B, k));
     }
     return check_launch();
+}
+
+extern "C" int clb_group_popcount(const void *x, int32_t *counts, int64_t F, int64_t words, int bits, int pad_len, int k, void *stream)
+{
+    if (!x || !counts || F < 0 || words < 0 || !bits_ok(bits) || k <= 0 || pad_len < 0 || pad_len >= bits) return CLB_ERR_ARG;
+    if (F % k) return CLB_ERR_SHAPE;
+    return group_popcount(x, counts, F, words * (bits / 8), words * bits - pad_len, k, (cudaStream_t)stream);
+}
+int clb_group_popcount_units(const void *x, int32_t *counts, int64_t F, int64_t U, int64_t B, int k, cudaStream_t st)
+{
+    return group_popcount(x, counts, F, U * 16, B, k, st);
 }
 
 extern "C" int clb_packed_convtree(const void *x, const uint8_t *ops, const int32_t *sel, void *y, int Ci, int H, int W, int C,

@@ -26,9 +26,10 @@
 namespace clb {
 namespace slab {
 
-template <int S> struct Geo {
+// Blocks come in two sizes: the large one, and (but for 32x32 images) one for few slabs, where most of a large block's threads had none.
+template <int S, bool SMALL> struct Geo {
     static constexpr int H2 = S / 2, I = H2 * H2;                // pooled side, outputs (threads) per slab
-    static constexpr int THREADS = S == 4 ? 128 : 256;
+    static constexpr int THREADS = SMALL ? (S == 16 ? 64 : 32) : S == 4 ? 128 : 256;
     static constexpr int UB = THREADS / I;                       // slabs of a block
     static constexpr int PITCH = S == 8 ? 10 : S + 1;            // units of a padded row
     static constexpr int SLAB = S == 4 ? 28 : (S + 1) * PITCH;   // units from one slab to the next
@@ -39,9 +40,9 @@ template <int S> struct Geo {
 template <int S> __host__ __device__ constexpr int column(int c) { return (c & 1) ? (c - 1) / 2 : S / 2 + c / 2; } // unit of padded column c
 
 // tile bytes from unit p of the first slab to unit p + i * THREADS of the group
-template <int S> __host__ __device__ constexpr int unit_step(int i)
+template <int S, typename G> __host__ __device__ constexpr int unit_step(int i)
 {
-    return 16 * (i * Geo<S>::THREADS / Geo<S>::HW * Geo<S>::SLAB + i * Geo<S>::THREADS % Geo<S>::HW / S * Geo<S>::PITCH);
+    return 16 * (i * G::THREADS / G::HW * G::SLAB + i * G::THREADS % G::HW / S * G::PITCH);
 }
 
 __device__ __forceinline__ void cp_async16(unsigned dst, const void *src)
@@ -117,11 +118,11 @@ template <int S> __device__ __noinline__ uint4 window_global(const uint4 *__rest
     return acc;
 }
 
-template <int S>
-__global__ void __launch_bounds__(Geo<S>::THREADS, 1024 / Geo<S>::THREADS)
+template <int S, bool SMALL>
+__global__ void __launch_bounds__(Geo<S, SMALL>::THREADS, 1024 / Geo<S, SMALL>::THREADS)
     packed_convtree_slab3_kernel(const uint4 *__restrict__ x, const Rec *__restrict__ recs, uint4 *__restrict__ y, Shape s)
 {
-    using G = Geo<S>;
+    using G = Geo<S, SMALL>;
     constexpr int NT = G::THREADS;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(16) Rec rec[3];
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(Geo<S>::THREADS, 1024 / Geo<S>::THREADS)
         for (int slot = 0; slot < R.nst; ++slot) {
             const uint4 *src = x + ((size_t)R.ch[slot] * s.U + u0) * G::HW + tid;
             const unsigned d = sdst + slot * G::PLANE_BYTES;
-            constexpr int D1 = unit_step<S>(1), D2 = unit_step<S>(2), D3 = unit_step<S>(3);
+            constexpr int D1 = unit_step<S, G>(1), D2 = unit_step<S, G>(2), D3 = unit_step<S, G>(3);
             if (n > 3 * NT) {
                 cp_async16_at<0, 0>(d, src), cp_async16_at<D1, NT * 16>(d, src);
                 cp_async16_at<D2, 2 * NT * 16>(d, src), cp_async16_at<D3, 3 * NT * 16>(d, src);
@@ -224,10 +225,10 @@ __global__ void __launch_bounds__(Geo<S>::THREADS, 1024 / Geo<S>::THREADS)
 }
 
 // One record per output channel; offsets are bytes from a window's unit of the first plane.
-template <int S>
+template <int S, bool SMALL>
 __global__ void packed_slab3_records_kernel(const uint8_t *__restrict__ ops, const int32_t *__restrict__ sel, Rec *__restrict__ recs, int C, int Ci)
 {
-    using G = Geo<S>;
+    using G = Geo<S, SMALL>;
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= C) return;
     Rec R;
@@ -251,19 +252,30 @@ __global__ void packed_slab3_records_kernel(const uint8_t *__restrict__ ops, con
     recs[c] = R;
 }
 
-template <int S> static int launch(const void *x, const void *recs, void *y, int Ci, int C, int64_t U, Order in, Order out, cudaStream_t st)
+template <int S, bool SMALL> static int launch(const void *x, const void *recs, void *y, int Ci, int C, int64_t U, Order in, Order out, cudaStream_t st)
 {
-    using G = Geo<S>;
+    using G = Geo<S, SMALL>;
     using namespace clb_host;
     Shape s{Ci, C, (int)U, (int)((U + G::UB - 1) / G::UB), in, out};
     constexpr int bytes = 2 * G::PLANE_BYTES;
-    auto k = packed_convtree_slab3_kernel<S>;
+    auto k = packed_convtree_slab3_kernel<S, SMALL>;
     if (ensure_dynamic_smem(k, bytes) != cudaSuccess) return check_launch(0);
     constexpr int by_smem = 227 * 1024 / (bytes + 2048), by_threads = 1024 / G::THREADS; // 64 registers a thread
     const long long items = (long long)C * s.n_ug, all = (long long)sm_count() * (by_smem < by_threads ? by_smem : by_threads);
     CLB_TRACED("packed_convtree_slab3_kernel", st,
-               k<<<(unsigned)(items < all ? items : all), G::THREADS, bytes, st>>>((const uint4 *)x, (const Rec *)recs, (uint4 *)y, s));
+               k<<<(unsigned)(items < all ? items : all), G::THREADS, bytes, st>>>((const uint4 *)x, (const Rec *)recs + (SMALL ? C : 0), (uint4 *)y, s));
     return check_launch();
+}
+// Small blocks where a large one would be at most half full (k = 1024, 100 samples: 8x8 images 52 -> 16 us, 4x4 61 -> 28).
+template <int S> static int launch_by_slabs(const void *x, const void *recs, void *y, int Ci, int C, int64_t U, Order in, Order out, cudaStream_t st)
+{
+    return 2 * U <= Geo<S, false>::UB ? launch<S, true>(x, recs, y, Ci, C, U, in, out, st) : launch<S, false>(x, recs, y, Ci, C, U, in, out, st);
+}
+template <int S> static int records(const uint8_t *ops, const int32_t *sel, Rec *recs, int Ci, int C, cudaStream_t st)
+{
+    packed_slab3_records_kernel<S, false><<<(C + 127) / 128, 128, 0, st>>>(ops, sel, recs, C, Ci);
+    if constexpr (S < 32) packed_slab3_records_kernel<S, true><<<(C + 127) / 128, 128, 0, st>>>(ops, sel, recs + C, C, Ci);
+    return clb_host::check_launch(S < 32 ? 2 : 1);
 }
 
 } // namespace slab
@@ -276,23 +288,21 @@ bool clb_slab3_covers(int H, int W, int sh, int sw, int ph, int pw, int kh, int 
 {
     return H == W && (H == 32 || H == 16 || H == 8 || H == 4) && sh == 1 && sw == 1 && ph == 1 && pw == 1 && kh == 3 && kw == 3;
 }
-size_t clb_slab3_record_bytes(int C) { return (size_t)C * sizeof(slab::Rec); }
+size_t clb_slab3_record_bytes(int C) { return 2 * (size_t)C * sizeof(slab::Rec); } // of the large and of the small blocks
 
 int clb_slab3_records(const uint8_t *ops, const int32_t *sel, void *recs, int Ci, int side, int C, cudaStream_t st)
 {
-    const int grid = (C + 127) / 128;
     slab::Rec *r = (slab::Rec *)recs;
-    if (side == 32) slab::packed_slab3_records_kernel<32><<<grid, 128, 0, st>>>(ops, sel, r, C, Ci);
-    else if (side == 16) slab::packed_slab3_records_kernel<16><<<grid, 128, 0, st>>>(ops, sel, r, C, Ci);
-    else if (side == 8) slab::packed_slab3_records_kernel<8><<<grid, 128, 0, st>>>(ops, sel, r, C, Ci);
-    else slab::packed_slab3_records_kernel<4><<<grid, 128, 0, st>>>(ops, sel, r, C, Ci);
-    return check_launch();
+    if (side == 32) return slab::records<32>(ops, sel, r, Ci, C, st);
+    if (side == 16) return slab::records<16>(ops, sel, r, Ci, C, st);
+    if (side == 8) return slab::records<8>(ops, sel, r, Ci, C, st);
+    return slab::records<4>(ops, sel, r, Ci, C, st);
 }
 
 int clb_slab3_block(const void *x, const void *recs, void *y, int Ci, int side, int C, int64_t U, Order in, Order out, cudaStream_t st)
 {
-    if (side == 32) return slab::launch<32>(x, recs, y, Ci, C, U, in, out, st);
-    if (side == 16) return slab::launch<16>(x, recs, y, Ci, C, U, in, out, st);
-    if (side == 8) return slab::launch<8>(x, recs, y, Ci, C, U, in, out, st);
-    return slab::launch<4>(x, recs, y, Ci, C, U, in, out, st);
+    if (side == 32) return slab::launch<32, false>(x, recs, y, Ci, C, U, in, out, st);
+    if (side == 16) return slab::launch_by_slabs<16>(x, recs, y, Ci, C, U, in, out, st);
+    if (side == 8) return slab::launch_by_slabs<8>(x, recs, y, Ci, C, U, in, out, st);
+    return slab::launch_by_slabs<4>(x, recs, y, Ci, C, U, in, out, st);
 }
