@@ -18,19 +18,18 @@
 // (fma.rn.f32x2: two independent IEEE FMAs, so the values are the scalar kernels' bit for bit).  The 2x2 pool is
 // finished with a shuffle between the lanes ox and ox^1.
 //
-// Backward, pass 1: a thread owns pooled windows, a warp whole images.  The gate chain is recomputed at the saved
-// arg-max position from the staged planes; the 28 gate-gradient basis sums stay in registers until the end; the
-// gradient w.r.t. the 8 taps is ADDED INTO a shared-memory copy of the two planes (one tap after the other, __syncwarp
-// between them: within one tap the map window -> pixel is injective), and the two gradient planes of (image, output
-// channel) are written out with 128-bit stores.  Pass 2 (plane_sum_kernel) adds, for every input channel, the planes of
+// Backward, pass 1 (8x8 and 4x4 images here, larger ones in convtree_tile.cu): a thread owns a pooled window, a warp whole images.
+// The gate chain is recomputed at the saved arg-max position from the staged planes; the 28 gate-gradient basis sums stay in
+// registers until the end; the gradient w.r.t. the 8 taps is ADDED INTO a shared-memory copy of the two planes (one tap after the
+// other, __syncwarp between them: within one tap the map window -> pixel is injective), and the two gradient planes of (image,
+// output channel) are written out with 128-bit stores.  Pass 2 (plane_sum_kernel) adds, for every input channel, the planes of
 // the output channels that read it, in a fixed order: a pure streaming kernel.  Deterministic, no float atomics.
-#include "clb_common.cuh"
+#include "clb_plane.cuh"
 #include "clb_tma.cuh"
 
 namespace clb {
 namespace plane {
 
-constexpr int kThreads = 128;
 constexpr int kLead = 4; // columns in front of the image in a staged row: 16 bytes, so that the box starts aligned
 
 // Geometry of a square S x S layer (3x3 window, padding 1): staged pitch P, rows R, images per box.
@@ -42,7 +41,7 @@ template <int S> struct Geo;
 // the always-zero lead cell of the next one), pairs 68 apart (banks 0, 4, 8, 12), a pair being images p and p + 4 of the
 // warp's eight.
 template <> struct Geo<16> {
-    static constexpr int P = 24, R = 18, FWD_NIMG = 2, BWD_NIMG = 1, BWD_WPT = 2, FWD_P = 24, FWD_IMG = 18 * 24;
+    static constexpr int P = 24, R = 18, FWD_NIMG = 2, FWD_P = 24, FWD_IMG = 18 * 24;
 };
 template <> struct Geo<8> {
     static constexpr int P = 20, R = 10, FWD_NIMG = 2, BWD_NIMG = 2, BWD_WPT = 1, FWD_P = 20, FWD_IMG = 10 * 20;
@@ -56,38 +55,10 @@ struct Args {
     int parts; // the batch is split into this many contiguous parts; a (channel, part) pair is one task
     int y_fm;  // the block's output (forward) / upstream gradient (backward) is feature-major: [C][windows][N] instead of
                // [N][C][windows] -- the layout the flat layers behind the last block work in; the arg-max bytes keep [N][C][windows]
+    int n_stride; // images of the whole batch (backward: N may be a slice of it): the pitch of a feature-major gy
 };
 
 __device__ int g_plane_error; // set when a bounded wait gave up (never expected); read by clb_plane_error()
-
-struct SlotInfo {
-    int slot[8];
-    int ch[2];
-    int nslot; // 3 = the selection does not fit two staged planes (more channels, or taps outside the 3x3 window)
-};
-
-// channel -> slot map of output channel c's taps (one thread fills it)
-__device__ __forceinline__ void fill_slots(SlotInfo &si, const int32_t *__restrict__ sel, int c, int Ci)
-{
-    int n = 0, chs[8];
-    bool inside = true;
-    for (int k = 0; k < 8; ++k) {
-        const int word = sel[c * 8 + k];
-        const int ch = (word >> 16) & 0xFFFF;
-        inside = inside && word >= 0 && ch < Ci && ((word >> 8) & 0xFF) < 3 && (word & 0xFF) < 3;
-        int slot = -1;
-        for (int j = 0; j < n; ++j)
-            if (chs[j] == ch) slot = j;
-        if (slot < 0) {
-            slot = n;
-            chs[n++] = ch;
-        }
-        si.slot[k] = slot;
-    }
-    si.ch[0] = min(chs[0], Ci - 1);
-    si.ch[1] = min(chs[n > 1 ? 1 : 0], Ci - 1);
-    si.nslot = (inside && n <= 2) ? n : 3;
-}
 
 typedef unsigned long long f32x2; // two floats in one 64-bit register
 __device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
@@ -180,6 +151,7 @@ template <int S> struct FwdCfg {
     static_assert(IMG >= R * P && IMG % 4 == 0 && P % 4 == 0 && (!TMA || IMG == R * P), "tile geometry");
     static constexpr int STAGES = TMA ? 4 : 3;
     static constexpr int SMEM = GROUPS * STAGES * STAGE_BYTES;
+    static constexpr int BLOCKS = S == 16 ? 7 : S == 8 ? 5 : 4; // resident per SM: by registers, by shared memory, by shared memory
     static constexpr int GSIZE = WIDE ? kThreads : 32;
     static constexpr int CPQ = NIMG * 2 * S * (S / 4) / GSIZE;   // 16-byte copies per thread and iteration (cp.async staging)
     static_assert(WIDE ? (TPI == kThreads && NIMG == 2) : (32 % TPI == 0 && NIMG == 2 * (32 / TPI)), "thread mapping");
@@ -475,26 +447,7 @@ __device__ __forceinline__ void bwd_windows(const uint32_t (&base)[WPT], const u
             cell[j][k] = base[j] + toff[k];
             a[k] = lds_f32<B>(cell[j][k]);
         }
-        const float d = dz[j];
-        const float g0 = gate_eval<float>(g[0], a[0], a[1]), g1 = gate_eval<float>(g[1], a[2], a[3]);
-        const float g2 = gate_eval<float>(g[2], a[4], a[5]), g3 = gate_eval<float>(g[3], a[6], a[7]);
-        const float t0 = gate_eval<float>(g[4], g0, g1), t1 = gate_eval<float>(g[5], g2, g3);
-        const float dt0 = d * gate_da<float>(g[6], t1), dt1 = d * gate_db<float>(g[6], t0);
-        float dg[4];
-        dg[0] = dt0 * gate_da<float>(g[4], g1), dg[1] = dt0 * gate_db<float>(g[4], g0);
-        dg[2] = dt1 * gate_da<float>(g[5], g3), dg[3] = dt1 * gate_db<float>(g[5], g2);
-        acc[24] = fmaf(d, t0 * t1, acc[24]), acc[25] = fmaf(d, t0, acc[25]), acc[26] = fmaf(d, t1, acc[26]), acc[27] += d;
-        acc[16] = fmaf(dt0, g0 * g1, acc[16]), acc[17] = fmaf(dt0, g0, acc[17]), acc[18] = fmaf(dt0, g1, acc[18]), acc[19] += dt0;
-        acc[20] = fmaf(dt1, g2 * g3, acc[20]), acc[21] = fmaf(dt1, g2, acc[21]), acc[22] = fmaf(dt1, g3, acc[22]), acc[23] += dt1;
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-            acc[4 * p] = fmaf(dg[p], a[2 * p] * a[2 * p + 1], acc[4 * p]);
-            acc[4 * p + 1] = fmaf(dg[p], a[2 * p], acc[4 * p + 1]);
-            acc[4 * p + 2] = fmaf(dg[p], a[2 * p + 1], acc[4 * p + 2]);
-            acc[4 * p + 3] += dg[p];
-            tg[j][2 * p] = dg[p] * gate_da<float>(g[p], a[2 * p + 1]);
-            tg[j][2 * p + 1] = dg[p] * gate_db<float>(g[p], a[2 * p]);
-        }
+        window_bwd(a, g, dz[j], acc, tg[j]);
     }
     // (Skipping the accesses of taps that repeat an earlier tap's cell -- about one tap in six with 8 taps over 18 cells --
     // was measured slower in both forms tried: warp-uniform branches around each access break the batching of the loads,
@@ -634,7 +587,7 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const __gr
             const bool live = it < iters && n < n_hi;
             const size_t o = ((size_t)n * s.C + c) * I + win[j];
             if constexpr (FM) // gy is [C][windows][N] (compile-time: the flag in the index arithmetic cost the 8x8 kernel 7 %)
-                dz_next[j] = live ? __ldg(gy + ((size_t)c * I + win[j]) * s.N + n) : 0.f;
+                dz_next[j] = live ? __ldg(gy + ((size_t)c * I + win[j]) * s.n_stride + n) : 0.f;
             else
                 dz_next[j] = live ? __ldg(gy + o) : 0.f;
             bd_next[j] = live ? (int)__ldg(amax + o) : 0;
@@ -710,20 +663,8 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const __gr
     if (!usable && lane == 0) g_plane_error = 2;
 
     // the warp's 28 basis sums: lane i ends up with sum i (a transposed butterfly over the 32 lanes)
-    float v[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = i < 28 ? acc[i] : 0.f;
-#pragma unroll
-    for (int half = 16; half >= 1; half >>= 1) {
-        const bool upper = (lane & half) != 0;
-#pragma unroll
-        for (int i = 0; i < half; ++i) {
-            const float keep = upper ? v[i + half] : v[i];
-            const float send = upper ? v[i] : v[i + half];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
-        }
-    }
-    if (lane < 28) partial[((size_t)part * s.C + c) * 28 + lane] = v[0];
+    const float sum = warp_sums28(acc, lane);
+    if (lane < 28) partial[((size_t)part * s.C + c) * 28 + lane] = sum;
 }
 
 // ======================================================================= gate gradient alone, 32x32 images
@@ -868,20 +809,8 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_w_plane32_kernel(const 
     }
     if (!usable && tid == 0) g_plane_error = 2;
 
-    float v[32];
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = i < 28 ? acc[i] : 0.f;
-#pragma unroll
-    for (int half = 16; half >= 1; half >>= 1) {
-        const bool upper = (lane & half) != 0;
-#pragma unroll
-        for (int i = 0; i < half; ++i) {
-            const float keep = upper ? v[i + half] : v[i];
-            const float send = upper ? v[i] : v[i + half];
-            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, half);
-        }
-    }
-    if (lane < 28) red[warp][lane] = v[0];
+    const float sum = warp_sums28(acc, lane);
+    if (lane < 28) red[warp][lane] = sum;
     __syncthreads();
     if (tid < 28) partial[((size_t)part * s.C + c) * 28 + tid] = (red[0][tid] + red[1][tid]) + (red[2][tid] + red[3][tid]);
 }
@@ -978,17 +907,6 @@ int plane_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int p
     return (H == 32 || H == 16 || H == 8 || H == 4) ? H : 0; // 32: the gate gradient alone (clb_convtree_bwd_plane without gx)
 }
 
-// Parts of the batch per output channel: enough (channel, part) tasks for about three waves of resident groups, but
-// at least eight iterations per task so that a task's set-up (soft-max of 7 gates, tap table) stays a small share.
-int plane_parts(int N, int C, int images_per_iteration, int resident_groups_per_sm)
-{
-    long long parts = ((long long)sm_count() * resident_groups_per_sm * 3 + C - 1) / C;
-    const long long most = N / (8LL * images_per_iteration);
-    if (parts > most) parts = most;
-    if (parts < 1) parts = 1;
-    return (int)parts;
-}
-
 template <int S>
 int launch_fwd(const float *x, const float *w, const int32_t *sel, float *y, uint8_t *amax, int N, int Ci, int C, int wmode, cudaStream_t st)
 {
@@ -997,40 +915,72 @@ int launch_fwd(const float *x, const float *w, const int32_t *sel, float *y, uin
     if (!clb_tma::make_plane_map(&map, x, N, Ci, S, S, Cf::P, Cf::R, Cf::NIMG)) return CLB_ERR_SHAPE;
     auto k = convtree_fwd_plane_kernel<S>;
     if (clb_host::ensure_dynamic_smem(k, Cf::SMEM) != cudaSuccess) return check_launch(0);
-    const int parts = plane_parts(N, C, Cf::NIMG, Cf::WIDE ? 6 : 12);
-    const Args a{N, Ci, C, wmode & 0xff, parts, (wmode & CLB_Y_FEATURE_MAJOR) ? 1 : 0};
+    const int parts = clb_plane_parts(N, C, Cf::NIMG, Cf::GROUPS, Cf::BLOCKS);
+    const Args a{N, Ci, C, wmode & 0xff, parts, (wmode & CLB_Y_FEATURE_MAJOR) ? 1 : 0, N};
     const long long tasks = (long long)C * parts;
     CLB_TRACED("convtree_fwd_plane_kernel", st,
                k<<<(unsigned)((tasks + Cf::GROUPS - 1) / Cf::GROUPS), kThreads, Cf::SMEM, st>>>(map, x, w, sel, y, amax, a));
     return check_launch();
 }
 
-template <int S> int bwd_parts(int N, int C) { return plane_parts(N, C, BwdCfg<S>::NIMG, 12); }
-
-template <int S>
-int launch_bwd(const float *gy, const float *x, const float *w, const int32_t *sel, const uint8_t *amax, float *partial, float *planes, int N,
-               int Ci, int C, int wmode, cudaStream_t st)
+template <int S> int launch_bwd(const ClbTileBwd &a, cudaStream_t st)
 {
     using Cf = BwdCfg<S>;
     CUtensorMap map;
-    if (!clb_tma::make_plane_map(&map, x, N, Ci, S, S, Cf::P, Cf::R, Cf::NIMG)) return CLB_ERR_SHAPE;
-    const bool fm = (wmode & CLB_Y_FEATURE_MAJOR) != 0;
-    auto k = fm ? convtree_bwd_plane_kernel<S, true> : convtree_bwd_plane_kernel<S, false>;
+    if (!clb_tma::make_plane_map(&map, a.x, a.N, a.Ci, S, S, Cf::P, Cf::R, Cf::NIMG)) return CLB_ERR_SHAPE;
+    auto k = a.fm ? convtree_bwd_plane_kernel<S, true> : convtree_bwd_plane_kernel<S, false>;
     if (clb_host::ensure_dynamic_smem(k, Cf::SMEM) != cudaSuccess) return check_launch(0);
-    const int parts = bwd_parts<S>(N, C);
-    const Args a{N, Ci, C, wmode & 0xff, parts, fm ? 1 : 0};
-    const long long tasks = (long long)C * parts;
-    CLB_TRACED("convtree_bwd_plane_kernel", st, k<<<(unsigned)((tasks + 3) / 4), kThreads, Cf::SMEM, st>>>(map, gy, x, w, sel, amax, partial, planes, a));
+    const Args s{a.N, a.Ci, a.C, a.wmode, a.parts, a.fm, a.n_stride};
+    const long long tasks = (long long)a.C * a.parts;
+    CLB_TRACED("convtree_bwd_plane_kernel", st,
+               k<<<(unsigned)((tasks + 3) / 4), kThreads, Cf::SMEM, st>>>(map, a.gy, a.x, a.w, a.sel, a.amax, a.partial, a.planes, s));
     return CLB_OK;
 }
 
-int bwd_parts_for(int side, int N, int C)
+// The sides of the two backward passes.  16, 8 and 4: always, as in the forward.  32, 28 and 12: from 4, 8 and 12 channels on.  With
+// fewer the kernel that keeps all channels of a few images in shared memory, and needs no second pass over the planes, is
+// as good or better (us with it / with the planes; 128 images, 128 channels out: 32x32 with 4 channels in 98 / 93, with 16
+// 211 / 99; 28x28 with 4 95 / 104, with 8 111 / 105, with 32 242 / 112; 256 images of 12x12, 256 out: with 8 71 / 87, with 32 271 / 88).
+int bwd_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw, int kh, int kw)
 {
-    if (side == 32) return plane_parts(N, C, 1, 5);
-    return side == 16 ? bwd_parts<16>(N, C) : side == 8 ? bwd_parts<8>(N, C) : bwd_parts<4>(N, C);
+    if (sh != 1 || sw != 1 || ph != 1 || pw != 1 || kh != 3 || kw != 3 || H != W || N <= 0 || C <= 0 || C > 65535 || Ci > 65535) return 0;
+    if (tune_get(CLB_TUNE_PLANE_KERNELS) == 0) return 0;
+    const int least = H == 32 ? 4 : H == 28 ? 8 : H == 12 ? 12 : H == 16 || H == 8 || H == 4 ? 1 : Ci + 1;
+    return Ci >= least ? H : 0;
 }
+// Images of a slice of the batch: the gradient planes, eight bytes per pixel and output channel, of a slice stay below 1 GB.
+int bwd_slice(int N, int C, int HW)
+{
+    const long long most = (1LL << 30) / ((long long)C * HW * 8);
+    return most >= N ? N : most < 16 ? 16 : (int)most;
+}
+int bwd_parts(int side, int N, int C)
+{
+    return side == 8 ? clb_plane_parts(N, C, BwdCfg<8>::NIMG, 4, 4) : side == 4 ? clb_plane_parts(N, C, BwdCfg<4>::NIMG, 4, 4) : clb_tile_bwd_parts(side, N, C);
+}
+size_t bwd_partial_bytes(int side, int N, int C)
+{
+    const int slice = bwd_slice(N, C, side * side);
+    return ((size_t)((N + slice - 1) / slice) * bwd_parts(side, slice, C) * C * 28 * sizeof(float) + 255) / 256 * 256;
+}
+int w32_parts(int N, int C) { return clb_plane_parts(N, C, 1, 1, 5); }
 
 } // namespace
+
+int clb_plane_parts(int N, int C, int images_per_iteration, int groups, int resident)
+{
+    const long long setup = 2 * images_per_iteration;
+    const long long sms = sm_count();
+    long long best = -1;
+    int parts = 1;
+    for (int p = 1; p <= 64 && (long long)(p - 1) * images_per_iteration < N; ++p) {
+        const long long iters = ((N + p - 1) / p + images_per_iteration - 1) / images_per_iteration + setup;
+        const long long blocks = ((long long)C * p + groups - 1) / groups, per_sm = (blocks + sms - 1) / sms;
+        const long long cost = iters * (per_sm + (per_sm + resident - 1) / resident * resident);
+        if (best < 0 || cost < best) best = cost, parts = p;
+    }
+    return parts;
+}
 
 // Forward of a many-channel layer through the plane kernels; CLB_ERR_SHAPE when they do not cover the shape.
 int clb_convtree_fwd_plane_f32(const float *x, const float *w, const int32_t *sel, float *y, uint8_t *amax, int N, int Ci, int H, int W, int C,
@@ -1089,11 +1039,14 @@ extern "C" int clb_conv_channel_lists(const int32_t *sel_host, int C, int Ci, in
 extern "C" size_t clb_convtree_bwd_plane_scratch_bytes(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw, int kh, int kw, int dtype)
 {
     if (dtype != CLB_F32 || !conv_args_ok(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw)) return 0;
-    const int side = plane_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw);
-    if (!side) return 0;
-    const size_t partial = ((size_t)bwd_parts_for(side, N, C) * C * 28 * sizeof(float) + 255) / 256 * 256;
-    if (side == 32) return partial; // gate gradient alone: no gradient planes
-    return partial + (size_t)N * C * 2 * H * W * sizeof(float);
+    size_t bytes = 0;
+    if (const int side = bwd_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw))
+        bytes = bwd_partial_bytes(side, N, C) + (size_t)bwd_slice(N, C, H * W) * C * 2 * H * W * sizeof(float);
+    if (plane_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw) == 32) { // the gate gradient alone
+        const size_t alone = (size_t)w32_parts(N, C) * C * 28 * sizeof(float);
+        if (alone > bytes) bytes = alone;
+    }
+    return bytes;
 }
 
 extern "C" int clb_convtree_bwd_plane(const void *gy, const void *x, const void *w, const int32_t *sel, const uint8_t *amax, void *gx, void *gw,
@@ -1105,18 +1058,15 @@ extern "C" int clb_convtree_bwd_plane(const void *gy, const void *x, const void 
     if (!gy || !x || !w || !sel || !amax || (!gx && !gw) || !scratch || wmode < 0 || wmode > 2) return CLB_ERR_ARG;
     if (gx && (!ch_start || !ch_entry)) return CLB_ERR_ARG;
     if (dtype != CLB_F32 || !conv_args_ok(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw)) return CLB_ERR_SHAPE;
-    const int side = plane_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw);
-    if (!side || (side == 32) != (gx == nullptr)) return CLB_ERR_SHAPE; // 32x32: gate gradient alone; smaller: both gradients
-    if (side == 32 && wmode_in != wmode) return CLB_ERR_SHAPE;          // the 32x32 kernel reads gy as [N][C][windows] only
-    if (side == 32) {
-        const int parts32 = bwd_parts_for(32, N, C);
+    if (!gx && plane_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw) == 32 && wmode_in == wmode) { // gy as [N][C][windows] only
+        const int parts32 = w32_parts(N, C);
         if (scratch_bytes < (size_t)parts32 * C * 28 * sizeof(float) || (reinterpret_cast<uintptr_t>(scratch) & 15)) return CLB_ERR_SCRATCH;
         CUtensorMap map32;
         if (!clb_tma::make_plane_map(&map32, (const float *)x, N, Ci, 32, 32, BwdW32::P, BwdW32::R, 1)) return CLB_ERR_SHAPE;
         auto k32 = convtree_bwd_w_plane32_kernel;
         if (clb_host::ensure_dynamic_smem(k32, BwdW32::SMEM) != cudaSuccess) return check_launch(0);
         cudaStream_t st32 = (cudaStream_t)stream;
-        const Args a32{N, Ci, C, wmode, parts32, 0};
+        const Args a32{N, Ci, C, wmode, parts32, 0, N};
         CLB_TRACED("convtree_bwd_w_plane32_kernel", st32,
                    k32<<<(unsigned)((long long)C * parts32), kThreads, BwdW32::SMEM, st32>>>(map32, (const float *)gy, (const float *)w, sel, amax,
                                                                                            (float *)scratch, a32));
@@ -1126,33 +1076,39 @@ extern "C" int clb_convtree_bwd_plane(const void *gy, const void *x, const void 
                                                                                               parts32, ngates32, wmode));
         return check_launch(2);
     }
-    const size_t need = clb_convtree_bwd_plane_scratch_bytes(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw, dtype);
-    if (scratch_bytes < need || (reinterpret_cast<uintptr_t>(scratch) & 15) || (reinterpret_cast<uintptr_t>(gx) & 15)) return CLB_ERR_SCRATCH;
+    const int side = bwd_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw);
+    if (!side || !gx || (reinterpret_cast<uintptr_t>(x) & 15)) return CLB_ERR_SHAPE;
+    const int slice = bwd_slice(N, C, H * W), slices = (N + slice - 1) / slice, parts = bwd_parts(side, slice, C);
+    const size_t partial_bytes = bwd_partial_bytes(side, N, C);
+    if (scratch_bytes < partial_bytes + (size_t)slice * C * 2 * H * W * sizeof(float) || (reinterpret_cast<uintptr_t>(scratch) & 15) ||
+        (reinterpret_cast<uintptr_t>(gx) & 15))
+        return CLB_ERR_SCRATCH;
     cudaStream_t st = (cudaStream_t)stream;
-    const int parts = bwd_parts_for(side, N, C);
-    float *partial = (float *)scratch;
-    float *planes = (float *)((unsigned char *)scratch + ((size_t)parts * C * 28 * sizeof(float) + 255) / 256 * 256);
-    const float *gyf = (const float *)gy, *xf = (const float *)x, *wf = (const float *)w;
-    const int rc = side == 16  ? launch_bwd<16>(gyf, xf, wf, sel, amax, partial, planes, N, Ci, C, wmode_in, st)
-                   : side == 8 ? launch_bwd<8>(gyf, xf, wf, sel, amax, partial, planes, N, Ci, C, wmode_in, st)
-                               : launch_bwd<4>(gyf, xf, wf, sel, amax, partial, planes, N, Ci, C, wmode_in, st);
-    if (rc != CLB_OK) return rc;
-    int launched = 1;
-    const int HW4 = H * W / 4;
-    const long long total = (long long)N * Ci * HW4;
-    long long blocks = (total + 255) / 256;
-    const long long cap = (long long)sm_count() * 32;
-    if (blocks > cap) blocks = cap;
-    GateFinish fin{partial, wf, (float *)gw, parts, wmode, 0, (long long)C * 7};
-    if (gw) fin.blocks = (int)((fin.ngates + 255) / 256);
-    if (total + (blocks + fin.blocks) * 256 < 0x7fffffffLL)
-        CLB_TRACED("plane_sum_kernel", st,
-                   plane_sum_kernel<unsigned><<<(unsigned)(blocks + fin.blocks), 256, 0, st>>>(planes, ch_start, ch_entry, (float *)gx, N, Ci, C, HW4, fin));
-    else
-        CLB_TRACED("plane_sum_kernel", st,
-                   plane_sum_kernel<long long><<<(unsigned)(blocks + fin.blocks), 256, 0, st>>>(planes, ch_start, ch_entry, (float *)gx, N, Ci, C, HW4, fin));
-    ++launched;
-    return check_launch(launched);
+    float *partial = (float *)scratch, *planes = (float *)((unsigned char *)scratch + partial_bytes);
+    const int HW4 = H * W / 4, fm = wmode_in != wmode; // HW4: also the windows of an image
+    for (int i = 0; i < slices; ++i) {
+        const int n0 = i * slice, n = N - n0 < slice ? N - n0 : slice;
+        const size_t windows = (size_t)n0 * C * HW4, pixels = (size_t)n0 * Ci * H * W;
+        const ClbTileBwd a{(const float *)gy + (fm ? (size_t)n0 : windows), (const float *)x + pixels, (const float *)w, sel, amax + windows,
+                           partial + (size_t)i * parts * C * 28, planes, n, Ci, C, wmode, parts, fm, N};
+        const int rc = side == 8 ? launch_bwd<8>(a, st) : side == 4 ? launch_bwd<4>(a, st) : clb_tile_bwd(side, a, st);
+        if (rc != CLB_OK) return rc;
+        const long long total = (long long)n * Ci * HW4;
+        long long blocks = (total + 255) / 256;
+        const long long cap = (long long)sm_count() * 32;
+        if (blocks > cap) blocks = cap;
+        GateFinish fin{partial, (const float *)w, (float *)gw, slices * parts, wmode, 0, (long long)C * 7};
+        if (gw && i + 1 == slices) fin.blocks = (int)((fin.ngates + 255) / 256);
+        auto sum = [&](auto kernel) {
+            CLB_TRACED("plane_sum_kernel", st,
+                       kernel<<<(unsigned)(blocks + fin.blocks), 256, 0, st>>>(planes, ch_start, ch_entry, (float *)gx + pixels, n, Ci, C, HW4, fin));
+        };
+        if (total + (blocks + fin.blocks) * 256 < 0x7fffffffLL)
+            sum(plane_sum_kernel<unsigned>);
+        else
+            sum(plane_sum_kernel<long long>);
+    }
+    return check_launch(2 * slices);
 }
 
 // Diagnostic: the device-side flag a plane kernel sets when one of its bounded waits ran out (0 = never).  Synchronises.

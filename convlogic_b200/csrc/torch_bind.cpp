@@ -383,8 +383,8 @@ std::pair<Tensor, Tensor> block_bwd(Tensor gy, const Tensor &x, const Tensor &w,
     const PlanPtr plan = get_plan();
     TORCH_CHECK(plan->channels_ok, "convlogic_b200: selection refers to a channel the input does not have");
     if (!plan->flag && dt == CLB_F32 && amax.defined()) {
-        // The plane kernels (two channel planes per output channel streamed through shared memory): both gradients of the
-        // many-channel layers (16x16 .. 4x4 images), the gate gradient alone of a 32x32 first block.
+        // The plane kernels (two channel planes per output channel in shared memory): both gradients of 3x3 blocks on images of 32 to 4
+        // pixels, the gate gradient alone of a 32x32 first block.
         const size_t bytes = clb_convtree_bwd_plane_scratch_bytes(d.n, d.ci, d.h, d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, dt);
         if (bytes && plan->channel_lists()) {
             Tensor scratch = scratch_bytes(bytes, x);
