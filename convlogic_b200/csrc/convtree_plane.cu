@@ -1,6 +1,5 @@
-// Fused ConvLogic block for layers with many input channels (blocks 2-4 of the CIFAR stacks): fp32, stride 1,
-// 3x3 window, padding 1, square images of 16, 8 or 4 pixels (other shapes take the kernels of convtree_fast.cu /
-// convtree.cu).
+// Fused ConvLogic block on channel planes: fp32, stride 1, 3x3 window, padding 1, square images of 32, 28, 16, 12, 8 or 4 pixels (other
+// shapes take the kernels of convtree_fast.cu / convtree.cu).
 //
 // An output channel reads only the (normally two) input channels its 8 taps name, so a block owns ONE output
 // channel and streams, image by image, just those two channel planes through shared memory.  The planes are
@@ -11,12 +10,13 @@
 // instruction on staging, and the loads of the next images are in flight while one is evaluated.  The geometry is
 // a template parameter, so every shared-memory access is  [per-thread register + immediate].
 //
-// Forward: a thread owns one COLUMN position ox of one pooled row py of an image PAIR, i.e. the conv positions
-// (2py, ox) and (2py+1, ox) of two images.  The lanes of a warp are consecutive ox (then py), so a tap is a
-// row-major, stride-1, conflict-free shared load (the row pitch P keeps the pooled rows of a warp in disjoint banks);
-// the two images of a pair are packed into one 64-bit register and the gate polynomials run as packed two-float FMAs
-// (fma.rn.f32x2: two independent IEEE FMAs, so the values are the scalar kernels' bit for bit).  The 2x2 pool is
-// finished with a shuffle between the lanes ox and ox^1.
+// Forward: a thread owns one COLUMN position ox of one pooled row py of an image PAIR, i.e. the conv positions (2py, ox) and
+// (2py+1, ox) of two images (from 28 pixels on, of the two halves of one image).  The lanes of a warp are consecutive ox (then py),
+// so a tap is a row-major, stride-1, conflict-free shared load (the row pitch P keeps the pooled rows of a warp in disjoint banks);
+// the two members of a pair are packed into one 64-bit register and the gate polynomials run as packed two-float FMAs
+// (fma.rn.f32x2: two independent IEEE FMAs, so the values are the scalar kernels' bit for bit).  The 2x2 pool is finished with a
+// shuffle between the lanes ox and ox^1.  256 images, 9 -> 256 channels of 32x32: 102 us, where a tile of all nine channels took 132;
+// 128 images, 64 -> 128 channels of 28x28: 35, where a tile of a few channels at a time took 106.
 //
 // Backward, pass 1 (8x8 and 4x4 images here, larger ones in convtree_tile.cu): a thread owns a pooled window, a warp whole images.
 // The gate chain is recomputed at the saved arg-max position from the staged planes; the 28 gate-gradient basis sums stay in
@@ -40,6 +40,16 @@ template <int S> struct Geo;
 // rows 40 apart (banks 0, 8, 16, 24).  4x4: 4 pairs x 2 rows x 4 columns; rows 16 apart (pitch 8: the right halo of a row is
 // the always-zero lead cell of the next one), pairs 68 apart (banks 0, 4, 8, 12), a pair being images p and p + 4 of the
 // warp's eight.
+// 32x32 and 28x28: one row of (up to) 32 columns.  12x12: 2 rows x 12 columns, rows 48 floats apart.
+template <> struct Geo<32> {
+    static constexpr int R = 34, FWD_NIMG = 1, FWD_P = 40, FWD_IMG = 34 * 40;
+};
+template <> struct Geo<28> {
+    static constexpr int R = 30, FWD_NIMG = 1, FWD_P = 36, FWD_IMG = 30 * 36;
+};
+template <> struct Geo<12> {
+    static constexpr int R = 14, FWD_NIMG = 2, FWD_P = 24, FWD_IMG = 14 * 24;
+};
 template <> struct Geo<16> {
     static constexpr int P = 24, R = 18, FWD_NIMG = 2, FWD_P = 24, FWD_IMG = 18 * 24;
 };
@@ -124,8 +134,8 @@ template <int OFF> __device__ __forceinline__ void cp_async16_off(uint32_t dst, 
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int PENDING> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
-// How the planes reach shared memory.  16x16 images: TMA box loads (one elected thread, halo zero-filled by the copy
-// engine).  8x8 and 4x4 images: the copy engine handles a box row by row at a few cycles per row, and rows of 32 or 16
+// How the planes reach shared memory.  16x16 images and larger: TMA box loads (one elected thread, halo zero-filled by the copy
+// engine).  Smaller images: the copy engine handles a box row by row at a few cycles per row, and rows of 32 or 16
 // useful bytes make it the bottleneck (measured: 290-300 us per layer against 230-240 us for register staging); there
 // every thread of the group issues two 16-byte cp.async copies per iteration into the interior of a tile whose halo was
 // zeroed once.
@@ -138,31 +148,32 @@ template <int S> struct FwdCfg {
     using G = Geo<S>;
     static constexpr int P = G::FWD_P, R = G::R, NIMG = G::FWD_NIMG;
     static constexpr int WO = S, HP = S / 2, WP = S / 2, I = HP * WP;
-    static constexpr int TPI = HP * WO;                          // threads per image pair
-    static constexpr bool WIDE = TPI >= kThreads;                // one group of 128 threads, else four warps on their own
-    static constexpr int GROUPS = WIDE ? 1 : kThreads / 32;
+    static constexpr bool WIDE = S >= 16;                        // one group of 128 threads, else four warps on their own
+    static constexpr int GROUPS = WIDE ? 1 : kThreads / 32, GSIZE = WIDE ? kThreads : 32;
     static constexpr int IMG = G::FWD_IMG;                       // floats of one staged plane (R * P + padding)
     static constexpr int SLOT = (NIMG * IMG + 31) / 32 * 32;     // floats of one slot (NIMG planes of one channel)
     static constexpr int STAGE_BYTES = 2 * SLOT * 4;
     static constexpr bool TMA = UseTma<S>::value;
-    // pair p of a group = images (2p, 2p + 1) of its batch, or (p, p + NIMG / 2) when several pairs share a warp
-    static constexpr bool SPLIT_PAIRS = NIMG > 2;
-    static constexpr int PAIR_STRIDE = SPLIT_PAIRS ? IMG : 2 * IMG, SECOND = SPLIT_PAIRS ? (NIMG / 2) * IMG : IMG;
-    static_assert(IMG >= R * P && IMG % 4 == 0 && P % 4 == 0 && (!TMA || IMG == R * P), "tile geometry");
-    static constexpr int STAGES = TMA ? 4 : 3;
-    static constexpr int SMEM = GROUPS * STAGES * STAGE_BYTES;
-    static constexpr int BLOCKS = S == 16 ? 7 : S == 8 ? 5 : 4; // resident per SM: by registers, by shared memory, by shared memory
-    static constexpr int GSIZE = WIDE ? kThreads : 32;
-    static constexpr int CPQ = NIMG * 2 * S * (S / 4) / GSIZE;   // 16-byte copies per thread and iteration (cp.async staging)
-    static_assert(WIDE ? (TPI == kThreads && NIMG == 2) : (32 % TPI == 0 && NIMG == 2 * (32 / TPI)), "thread mapping");
-    static_assert(NIMG * 2 * S * (S / 4) % GSIZE == 0, "copies per thread");
+    // What a thread evaluates as a pair: the same position of images (2p, 2p + 1) of its batch, of (p, p + NIMG / 2) when several
+    // pairs share a warp, or of pooled rows (r, r + HP / 2) of the one image when a stage holds no more.
+    static constexpr bool SPLIT_PAIRS = NIMG > 2, ROW_PAIRS = NIMG == 1;
+    static constexpr int PAIR_STRIDE = SPLIT_PAIRS ? IMG : 2 * IMG, SECOND = ROW_PAIRS ? HP * P : SPLIT_PAIRS ? (NIMG / 2) * IMG : IMG;
+    // A row of a pair takes LANES lanes, RPG rows are evaluated at a time, and the ROWS of an iteration take SUB turns.
+    static constexpr int LANES = S == 28 ? 32 : S, RPG = GSIZE / 32 * (32 / LANES), ROWS = ROW_PAIRS ? HP / 2 : NIMG / 2 * HP, SUB = (ROWS + RPG - 1) / RPG;
+    static constexpr bool FULL = 32 % S == 0 && ROWS % RPG == 0;  // else some threads have no position, or none in the last turn
+    static_assert(IMG >= R * P && IMG % 4 == 0 && P % 4 == 0 && (!TMA || IMG == R * P) && (SUB == 1 || NIMG <= 2), "tile geometry");
+    static constexpr int STAGES = S == 16 ? 4 : 3;
+    static constexpr int SMEM = GROUPS * STAGES * STAGE_BYTES + (FULL ? 0 : 2 * 2 * P * 4); // rows that a last turn reads in vain
+    // resident per SM: by registers (16), else by shared memory
+    static constexpr int BLOCKS = S == 16 ? 7 : S >= 28 ? 6 : S == 8 ? 5 : S == 4 ? 4 : 3;
+    static constexpr int UNITS = NIMG * 2 * S * (S / 4), CPQ = (UNITS + GSIZE - 1) / GSIZE; // 16-byte copies per iteration, and per thread (cp.async staging)
 };
 
-// One stage of the ring: both conv rows of both images of the thread's pair.
-template <int S, int ST> __device__ __forceinline__ void fwd_stage(const uint32_t (&toff)[8], const Gate2 (&g)[7], f32x2 (&z)[2])
+// Turn J of one stage of the ring: both conv rows of both members of the thread's pair.
+template <int S, int ST, int J> __device__ __forceinline__ void fwd_stage(const uint32_t (&toff)[8], const Gate2 (&g)[7], f32x2 (&z)[2])
 {
     using Cf = FwdCfg<S>;
-    constexpr int B = ST * Cf::STAGE_BYTES, ROWB = Cf::P * 4, IMGB = Cf::SECOND * 4;
+    constexpr int B = ST * Cf::STAGE_BYTES + J * Cf::RPG * 2 * Cf::P * 4, ROWB = Cf::P * 4, IMGB = Cf::SECOND * 4;
     {
         f32x2 v[8];
 #pragma unroll
@@ -265,10 +276,10 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
 #pragma unroll
     for (int i = 0; i < 7; ++i) g[i].k1 = dup2(sg[i].k1), g[i].ka = dup2(sg[i].ka), g[i].kb = dup2(sg[i].kb), g[i].kab = dup2(sg[i].kab);
 
-    // this thread's place: pair `pair_local` of the group's batch, pooled row py, column position ox
-    const int pair_local = gt / Cf::TPI;
-    const int t = gt - pair_local * Cf::TPI;
-    const int py = t / Cf::WO, ox = t - py * Cf::WO;
+    // this thread's place: pair `pair_local` of the group's batch, pooled row py (of its first turn), column position ox
+    const int row_at = min(gt / Cf::LANES, Cf::RPG - 1), pair_local = Cf::SUB > 1 ? 0 : row_at / Cf::HP, py = row_at - pair_local * Cf::HP;
+    const int ox = min(gt % Cf::LANES, S - 1);
+    const bool placed = Cf::FULL || (gt / Cf::LANES < Cf::RPG && gt % Cf::LANES < S);
     unsigned char *gbase = smem_raw + (size_t)gid * Cf::STAGES * Cf::STAGE_BYTES;
     const uint32_t thr = clb_tma::smem_addr(gbase) + 4u * (uint32_t)(pair_local * Cf::PAIR_STRIDE + 2 * py * Cf::P + ox);
     uint32_t toff[8];
@@ -300,7 +311,7 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
         constexpr int W4 = S / 4;
         const int col4 = u % W4, row = (u / W4) % S, slot = (u / (W4 * S)) & 1, img = u / (W4 * S * 2);
         csrc[q] = x + ((size_t)(n_lo + img) * s.Ci + (slot ? ch_b : ch_a)) * HW + row * S + col4 * 4;
-        cp_iters[q] = (n_hi - n_lo - img + Cf::NIMG - 1) / Cf::NIMG;
+        cp_iters[q] = u < Cf::UNITS ? (n_hi - n_lo - img + Cf::NIMG - 1) / Cf::NIMG : 0;
         cdst[q] = clb_tma::smem_addr(gbase) + 4u * (uint32_t)(slot * Cf::SLOT + img * Cf::IMG + (row + 1) * Cf::P + kLead + col4 * 4);
     }
     const size_t cstep = (size_t)Cf::NIMG * s.Ci * HW;
@@ -329,23 +340,25 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
         static_assert(Cf::TMA || Cf::STAGES == 3, "prologue of the cp.async ring");
     }
 
-    // 2x2 pool: lanes ox and ox^1 hold the two columns of a window, each for both images of the pair.  The even lane
-    // pools and stores the pair's first image, the odd lane the second; each hands the other the half it does not need.
-    const bool odd = ox & 1;
-    const int my_img = Cf::SPLIT_PAIRS ? pair_local + (odd ? Cf::NIMG / 2 : 0) : 2 * pair_local + (odd ? 1 : 0);
-    const int my_iters = (n_hi - n_lo - my_img + Cf::NIMG - 1) / Cf::NIMG;   // iterations in which that image exists
-    const size_t o0 = ((size_t)(n_lo + my_img) * s.C + c) * I + py * Cf::WP + (ox >> 1);
+    // 2x2 pool: lanes ox and ox^1 hold the two columns of a window, each for both members of the pair.  The even lane
+    // pools and stores the first member, the odd lane the second; each hands the other the half it does not need.
+    const bool odd = gt & 1;
+    const int my_img = Cf::ROW_PAIRS ? 0 : Cf::SPLIT_PAIRS ? pair_local + (odd ? Cf::NIMG / 2 : 0) : 2 * pair_local + (odd ? 1 : 0);
+    const int my_iters = placed ? (n_hi - n_lo - my_img + Cf::NIMG - 1) / Cf::NIMG : 0; // iterations in which that image exists
+    const int my_win = (py + (Cf::ROW_PAIRS && odd ? Cf::HP / 2 : 0)) * Cf::WP + (ox >> 1);
+    const size_t o0 = ((size_t)(n_lo + my_img) * s.C + c) * I + my_win;
     const size_t ostep = (size_t)Cf::NIMG * s.C * I;
     const bool want_amax = amax != nullptr;
-    float *yp = y + (s.y_fm ? ((size_t)c * I + py * Cf::WP + (ox >> 1)) * s.N + (n_lo + my_img) : o0); // run along with the iterations
+    float *yp = y + (s.y_fm ? ((size_t)c * I + my_win) * s.N + (n_lo + my_img) : o0); // run along with the iterations
     const size_t ystep = s.y_fm ? (size_t)Cf::NIMG : ostep;
+    const size_t yturn = (size_t)Cf::RPG * Cf::WP * (s.y_fm ? s.N : 1);
     uint8_t *ap = want_amax ? amax + o0 : nullptr;
     bool failed = false;
     int it = 0;
-    auto pool_store = [&](const f32x2(&z)[2]) {
-        const float m0 = odd ? hi_of(z[0]) : lo_of(z[0]), m1 = odd ? hi_of(z[1]) : lo_of(z[1]);   // my image, my column
-        const float t0 = odd ? lo_of(z[0]) : hi_of(z[0]), t1 = odd ? lo_of(z[1]) : hi_of(z[1]);   // the other lane's image
-        const float r0 = __shfl_xor_sync(0xffffffffu, t0, 1), r1 = __shfl_xor_sync(0xffffffffu, t1, 1); // my image, other column
+    auto pool_store = [&](const f32x2(&z)[2], int turn) {
+        const float m0 = odd ? hi_of(z[0]) : lo_of(z[0]), m1 = odd ? hi_of(z[1]) : lo_of(z[1]);   // my member, my column
+        const float t0 = odd ? lo_of(z[0]) : hi_of(z[0]), t1 = odd ? lo_of(z[1]) : hi_of(z[1]);   // the other lane's member
+        const float r0 = __shfl_xor_sync(0xffffffffu, t0, 1), r1 = __shfl_xor_sync(0xffffffffu, t1, 1); // my member, other column
         // candidates in scan order (0,0),(0,1),(1,0),(1,1); the even lane holds the even column
         const float c0 = odd ? r0 : m0, c1 = odd ? m0 : r0, c2 = odd ? r1 : m1, c3 = odd ? m1 : r1;
         float best = c0;
@@ -353,12 +366,10 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
         if (c1 > best) best = c1, bd = 1; // strict '>' in scan order keeps the first maximum
         if (c2 > best) best = c2, bd = 2;
         if (c3 > best) best = c3, bd = 3;
-        if (it < my_iters) {
-            *yp = best;
-            if (want_amax) *ap = (uint8_t)bd;
+        if (it < my_iters && (Cf::ROWS % Cf::RPG == 0 || py + turn * Cf::RPG < Cf::ROWS)) {
+            yp[turn * yturn] = best;
+            if (want_amax) ap[turn * Cf::RPG * Cf::WP] = (uint8_t)bd;
         }
-        yp += ystep;
-        if (want_amax) ap += ostep;
     };
     // the ring is walked with the stage index as a compile-time constant: every load is [register + immediate]
     while (it < iters && !failed) {
@@ -372,8 +383,10 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
             cp_async_wait<Cf::STAGES - 1>();                                                                              \
             group_sync(); /* the other threads' pieces of this stage are visible */                                      \
         }                                                                                                                 \
-        f32x2 z[2];                                                                                                       \
-        fwd_stage<S, ST>(toff, g, z);                                                                                     \
+        f32x2 z[Cf::SUB][2];                                                                                              \
+        fwd_stage<S, ST, 0>(toff, g, z[0]);                                                                               \
+        if constexpr (Cf::SUB > 1) fwd_stage<S, ST, 1>(toff, g, z[1]);                                                    \
+        if constexpr (Cf::SUB > 2) fwd_stage<S, ST, 2>(toff, g, z[2]);                                                    \
         /* The tile has been read by the whole group: refill this stage.  With TMA the same vote tells every thread    */ \
         /* whether anyone's wait ran out (never expected): then nothing of this iteration is stored.                   */ \
         if constexpr (Cf::TMA) {                                                                                          \
@@ -387,7 +400,9 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
             CLB_FWD_ISSUE_CP(ST, it + Cf::STAGES)                                                                         \
         }                                                                                                                 \
         if (!failed) {                                                                                                    \
-            pool_store(z);                                                                                                \
+            _Pragma("unroll") for (int j = 0; j < Cf::SUB; ++j) pool_store(z[j], j);                                      \
+            yp += ystep;                                                                                                  \
+            if (want_amax) ap += ostep;                                                                                   \
             ++it;                                                                                                         \
         }                                                                                                                 \
     }
@@ -899,12 +914,23 @@ using namespace clb::plane;
 
 namespace {
 
-// The plane kernels cover: fp32, stride 1, 3x3 window, padding 1, square images of 16, 8 or 4 pixels.
-int plane_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw, int kh, int kw)
+// The plane kernels cover: fp32, stride 1, 3x3 window, padding 1, square images of certain sides, which this returns (0: not covered).
+int square_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw, int kh, int kw)
 {
     if (sh != 1 || sw != 1 || ph != 1 || pw != 1 || kh != 3 || kw != 3 || H != W || N <= 0 || C <= 0 || C > 65535 || Ci > 65535) return 0;
-    if (tune_get(CLB_TUNE_PLANE_KERNELS) == 0 || clb_tma::encode_tiled_fn() == nullptr) return 0;
-    return (H == 32 || H == 16 || H == 8 || H == 4) ? H : 0; // 32: the gate gradient alone (clb_convtree_bwd_plane without gx)
+    return tune_get(CLB_TUNE_PLANE_KERNELS) == 0 ? 0 : H;
+}
+// (when the forward is worth it: the caller)
+int fwd_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw, int kh, int kw)
+{
+    const int side = square_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw);
+    if (clb_tma::encode_tiled_fn() == nullptr) return 0;
+    return side == 32 || side == 28 || side == 16 || side == 12 || side == 8 || side == 4 ? side : 0;
+}
+// the gate gradient alone of a 32x32 block
+bool w32_covers(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw, int kh, int kw)
+{
+    return square_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw) == 32 && clb_tma::encode_tiled_fn() != nullptr;
 }
 
 template <int S>
@@ -943,10 +969,9 @@ template <int S> int launch_bwd(const ClbTileBwd &a, cudaStream_t st)
 // 211 / 99; 28x28 with 4 95 / 104, with 8 111 / 105, with 32 242 / 112; 256 images of 12x12, 256 out: with 8 71 / 87, with 32 271 / 88).
 int bwd_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw, int kh, int kw)
 {
-    if (sh != 1 || sw != 1 || ph != 1 || pw != 1 || kh != 3 || kw != 3 || H != W || N <= 0 || C <= 0 || C > 65535 || Ci > 65535) return 0;
-    if (tune_get(CLB_TUNE_PLANE_KERNELS) == 0) return 0;
-    const int least = H == 32 ? 4 : H == 28 ? 8 : H == 12 ? 12 : H == 16 || H == 8 || H == 4 ? 1 : Ci + 1;
-    return Ci >= least ? H : 0;
+    const int side = square_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw);
+    const int least = side == 32 ? 4 : side == 28 ? 8 : side == 12 ? 12 : side == 16 || side == 8 || side == 4 ? 1 : Ci + 1;
+    return Ci >= least ? side : 0;
 }
 // Images of a slice of the batch: the gradient planes, eight bytes per pixel and output channel, of a slice stay below 1 GB.
 int bwd_slice(int N, int C, int HW)
@@ -986,7 +1011,10 @@ int clb_plane_parts(int N, int C, int images_per_iteration, int groups, int resi
 int clb_convtree_fwd_plane_f32(const float *x, const float *w, const int32_t *sel, float *y, uint8_t *amax, int N, int Ci, int H, int W, int C,
                                int sh, int sw, int ph, int pw, int kh, int kw, int wmode, cudaStream_t st)
 {
-    const int side = plane_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw);
+    const int side = fwd_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw);
+    if (side == 32) return launch_fwd<32>(x, w, sel, y, amax, N, Ci, C, wmode, st);
+    if (side == 28) return launch_fwd<28>(x, w, sel, y, amax, N, Ci, C, wmode, st);
+    if (side == 12) return launch_fwd<12>(x, w, sel, y, amax, N, Ci, C, wmode, st);
     if (side == 16) return launch_fwd<16>(x, w, sel, y, amax, N, Ci, C, wmode, st);
     if (side == 8) return launch_fwd<8>(x, w, sel, y, amax, N, Ci, C, wmode, st);
     if (side == 4) return launch_fwd<4>(x, w, sel, y, amax, N, Ci, C, wmode, st);
@@ -1042,7 +1070,7 @@ extern "C" size_t clb_convtree_bwd_plane_scratch_bytes(int N, int Ci, int H, int
     size_t bytes = 0;
     if (const int side = bwd_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw))
         bytes = bwd_partial_bytes(side, N, C) + (size_t)bwd_slice(N, C, H * W) * C * 2 * H * W * sizeof(float);
-    if (plane_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw) == 32) { // the gate gradient alone
+    if (w32_covers(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw)) { // the gate gradient alone
         const size_t alone = (size_t)w32_parts(N, C) * C * 28 * sizeof(float);
         if (alone > bytes) bytes = alone;
     }
@@ -1058,7 +1086,7 @@ extern "C" int clb_convtree_bwd_plane(const void *gy, const void *x, const void 
     if (!gy || !x || !w || !sel || !amax || (!gx && !gw) || !scratch || wmode < 0 || wmode > 2) return CLB_ERR_ARG;
     if (gx && (!ch_start || !ch_entry)) return CLB_ERR_ARG;
     if (dtype != CLB_F32 || !conv_args_ok(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw)) return CLB_ERR_SHAPE;
-    if (!gx && plane_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw) == 32 && wmode_in == wmode) { // gy as [N][C][windows] only
+    if (!gx && w32_covers(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw) && wmode_in == wmode) { // gy as [N][C][windows] only
         const int parts32 = w32_parts(N, C);
         if (scratch_bytes < (size_t)parts32 * C * 28 * sizeof(float) || (reinterpret_cast<uintptr_t>(scratch) & 15)) return CLB_ERR_SCRATCH;
         CUtensorMap map32;

@@ -1,0 +1,35 @@
+"""The plane forward at 32, 28 and 12 pixels (pairs of pooled rows of one image; rows of 28 or 24 of 32 lanes; a last turn that is
+half empty) against the general kernel, bit for bit: ragged batches, one image, feature-major output, selections on three channels."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+GEOM = (1, 1, 1, 1, 3, 3)
+
+
+@pytest.mark.parametrize("n,ci,c,side", [(1, 16, 5, 32), (9, 20, 3, 32), (300, 16, 2, 32), (7, 16, 4, 28), (1, 30, 2, 28), (1, 16, 7, 12), (35, 16, 3, 12),
+                                         (130, 40, 9, 12)])
+@pytest.mark.parametrize("spread", [False, True])
+def test_plane_forward_sides(n, ci, c, side, spread):
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib, ops
+    from convlogic_b200._lib import W_SOFTMAX
+
+    torch.manual_seed(n + side)
+    sel = cb.ConvLogicLayer(ci, c, padding=1, complete=True).selection.clone().cuda()
+    if spread:
+        sel[0, 3] = (sel[0, 3] & 0xFFFF) | ((ci - 1) << 16)
+        sel[0, 5] = (sel[0, 5] & 0xFFFF) | ((ci // 2) << 16)
+    x, w = torch.rand(n, ci, side, side, device="cuda"), torch.randn(c, 7, 16, device="cuda")
+    x = (x * 4).round() / 4  # ties between pooled positions
+    want, amax_want, _, _, _ = ops.convtree_fwd(x, w, sel, GEOM, W_SOFTMAX, want_indices=True)
+    _lib.trace(True)
+    y, amax, _, _, _ = ops.convtree_fwd(x, w, sel, GEOM, W_SOFTMAX)
+    torch.cuda.synchronize()
+    rep = _lib.trace_report()
+    _lib.trace(False)
+    assert "convtree_fwd_plane_kernel" in rep, rep
+    assert torch.equal(y, want) and torch.equal(amax, amax_want)
+    fm = ops.convtree_fwd(x, w, sel, GEOM, W_SOFTMAX, y_feature_major=True)[0]
+    assert torch.equal(fm, want)
