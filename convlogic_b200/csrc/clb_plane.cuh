@@ -90,8 +90,7 @@ __device__ __forceinline__ void window_bwd(const float (&a)[8], const Gate<float
 // times the iterations of one (256 images, 1024 channels of 16x16: 1 to 12 parts took 288, 279, 275, 246, 255, 256, 259, 247, ..
 // 253, 253 us, in proportion); but where the last few blocks leave an SM half empty it also goes with the rounds (28x28, 128
 // channels: 3 parts 80 us, 4 parts 99).  The sum of both decides; a task's set-up (soft-max of 7 gates, tap table, first
-// copies) counts as two iterations per image of one.  (4x4, eight images an iteration, 8192 channels: 205, 222, 237, 259 us with 1 to
-// 4 parts.)
+// copies) counts as a few iterations (4x4, eight images an iteration, 8192 channels: 189, 212, 230, 255 us with 1 to 4 parts).
 int clb_plane_parts(int N, int C, int images_per_iteration, int groups, int resident);
 
 // Pass 1 of the backward of a block of square images of 32, 28, 16 or 12 pixels (convtree_tile.cu): partial [parts][C][28] basis

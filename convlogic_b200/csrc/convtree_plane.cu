@@ -981,7 +981,7 @@ int bwd_slice(int N, int C, int HW)
 }
 int bwd_parts(int side, int N, int C)
 {
-    return side == 8 ? clb_plane_parts(N, C, BwdCfg<8>::NIMG, 4, 4) : side == 4 ? clb_plane_parts(N, C, BwdCfg<4>::NIMG, 4, 4) : clb_tile_bwd_parts(side, N, C);
+    return side == 8 ? clb_plane_parts(N, C, BwdCfg<8>::NIMG, 4, 4) : side == 4 ? clb_plane_parts(N, C, BwdCfg<4>::NIMG, 4, 3) : clb_tile_bwd_parts(side, N, C);
 }
 size_t bwd_partial_bytes(int side, int N, int C)
 {
@@ -994,7 +994,7 @@ int w32_parts(int N, int C) { return clb_plane_parts(N, C, 1, 1, 5); }
 
 int clb_plane_parts(int N, int C, int images_per_iteration, int groups, int resident)
 {
-    const long long setup = 2 * images_per_iteration;
+    const long long setup = images_per_iteration == 1 ? 2 : 4;
     const long long sms = sm_count();
     long long best = -1;
     int parts = 1;
