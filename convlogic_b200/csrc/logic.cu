@@ -422,14 +422,10 @@ __device__ __forceinline__ float quad_sum(float v)
 }
 
 // the lane's four entries of the mixture over the 16 gates (zeros on an idle lane); every lane of the warp calls this
-__device__ __forceinline__ void quad_load(const float *__restrict__ w16, int q, bool active, float (&p)[4])
+__device__ __forceinline__ void quad_mixture(const float *__restrict__ w16, int wmode, int q, bool active, float (&p)[4])
 {
 #pragma unroll
     for (int i = 0; i < 4; ++i) p[i] = active ? __ldg(w16 + 4 * q + i) : 0.f;
-}
-// the quad's four-entry pieces of a row of 16 values -> of the gate mixture
-__device__ __forceinline__ void quad_mixture(int wmode, int q, float (&p)[4])
-{
     if (wmode == CLB_W_SOFTMAX) {
         float m = fmaxf(fmaxf(p[0], p[1]), fmaxf(p[2], p[3]));
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
@@ -483,8 +479,7 @@ __device__ __forceinline__ void tree_gates(const TreeTables &tt, long long t, in
     const bool active = lane < 28;
     const long long n = active ? tree_node(tt, t, lane) : 0;
     float p[4];
-    quad_load(tree_row(tt, active ? lane : 0, n), lane & 3, active, p);
-    quad_mixture(wmode, lane & 3, p);
+    quad_mixture(tree_row(tt, active ? lane : 0, n), wmode, lane & 3, active, p);
     const Gate<float> mine = quad_gate(p, lane & 3);
 #pragma unroll
     for (int i = 0; i < 7; ++i) {
@@ -492,10 +487,11 @@ __device__ __forceinline__ void tree_gates(const TreeTables &tt, long long t, in
         g[i].kb = __shfl_sync(0xffffffffu, mine.kb, 4 * i), g[i].kab = __shfl_sync(0xffffffffu, mine.kab, 4 * i);
     }
 }
-// the same with the lane's piece of its neuron's row already loaded; p becomes the lane's four mixture entries
-__device__ __forceinline__ void tree_gates_of(int lane, int wmode, Gate<float> (&g)[7], float (&p)[4])
+// the same with the lane's neuron already known (lanes >= 28: any value); p = the lane's four mixture entries
+__device__ __forceinline__ void tree_gates_of(const TreeTables &tt, long long n, int lane, int wmode, Gate<float> (&g)[7], float (&p)[4])
 {
-    quad_mixture(wmode, lane & 3, p);
+    const bool active = lane < 28;
+    quad_mixture(tree_row(tt, active ? lane : 0, n), wmode, lane & 3, active, p);
     const Gate<float> mine = quad_gate(p, lane & 3);
 #pragma unroll
     for (int i = 0; i < 7; ++i) {
@@ -510,29 +506,21 @@ __global__ void __launch_bounds__(256, 3) logic_tree_fwd_kernel(const float *__r
 {
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    // The tables of a tree (leaf rows on lanes 0..7, the gates' neurons on lanes 0..27) are fetched two trees ahead and its gate rows
-    // one, so that a tree's own chain of dependent loads is one hop (the leaf rows).  (The backward kernel has no registers for
-    // that: gate rows and leaf rows fetched ahead took it from 269 to 357 us, half chunks in two buffers to 339.)
-    const bool active = lane < 28;
-    auto leaf_of = [&](long long t) { return t < T && lane < 8 ? __ldg(tt.leaf + t * 8 + lane) : 0; };
-    auto node_of = [&](long long t) { return t < T && active ? __ldg(tt.node + t * 7 + (lane >> 2)) : 0; };
-    int my_leaf = leaf_of(warp), nx_leaf = leaf_of(warp + nwarps), nx_node = node_of(warp + nwarps);
-    float w_next[4];
-    quad_load(tree_row(tt, active ? lane : 0, node_of(warp)), lane & 3, active && warp < T, w_next);
+    // The tables of a tree (leaf rows on lanes 0..7, the gates' neurons on lanes 0..27) are fetched one tree ahead, so that
+    // a tree's own chain of dependent loads is one hop (the rows, the logits) instead of two (index, then data).
+    int my_leaf = (warp < T && lane < 8) ? __ldg(tt.leaf + warp * 8 + lane) : 0;
+    int my_node = (warp < T && lane < 28) ? __ldg(tt.node + warp * 7 + (lane >> 2)) : 0;
     for (long long t = warp; t < T; t += nwarps) {
         const long long tn = t + nwarps;
+        const int nx_leaf = (tn < T && lane < 8) ? __ldg(tt.leaf + tn * 8 + lane) : 0;
+        const int nx_node = (tn < T && lane < 28) ? __ldg(tt.node + tn * 7 + (lane >> 2)) : 0;
         Gate<float> g[7];
         float pq[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) pq[i] = w_next[i];
-        quad_load(tree_row(tt, active ? lane : 0, nx_node), lane & 3, active && tn < T, w_next);
-        const int nn_leaf = leaf_of(tn + nwarps);
-        nx_node = node_of(tn + nwarps);
-        tree_gates_of(lane, wmode, g, pq);
+        tree_gates_of(tt, my_node, lane, wmode, g, pq);
         const float *row[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) row[k] = x + (long long)__shfl_sync(0xffffffffu, my_leaf, k) * B;
-        my_leaf = nx_leaf, nx_leaf = nn_leaf;
+        my_leaf = nx_leaf, my_node = nx_node;
         for (long long b0 = (long long)lane * V; b0 < B; b0 += 32 * V) {
             float a[8][V], r[V];
 #pragma unroll
@@ -567,25 +555,19 @@ __global__ void __launch_bounds__(256, TR <= 2 ? 3 : 2) logic_tree_fwd_sum_kerne
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[tr][e] = 0.f;
     const long long t0 = t_lo + wv;
-    const bool active = lane < 28; // tables two trees ahead, gate rows one, as in logic_tree_fwd_kernel
-    auto leaf_of = [&](long long t) { return t < t_hi && lane < 8 ? __ldg(tt.leaf + t * 8 + lane) : 0; };
-    auto node_of = [&](long long t) { return t < t_hi && active ? __ldg(tt.node + t * 7 + (lane >> 2)) : 0; };
-    int my_leaf = leaf_of(t0), nx_leaf = leaf_of(t0 + 8), nx_node = node_of(t0 + 8);
-    float w_next[4];
-    quad_load(tree_row(tt, active ? lane : 0, node_of(t0)), lane & 3, active && t0 < t_hi, w_next);
+    int my_leaf = (t0 < t_hi && lane < 8) ? __ldg(tt.leaf + t0 * 8 + lane) : 0;   // index tables one tree ahead
+    int my_node = (t0 < t_hi && lane < 28) ? __ldg(tt.node + t0 * 7 + (lane >> 2)) : 0;
     for (long long t = t0; t < t_hi; t += 8) {
+        const long long tn = t + 8;
+        const int nx_leaf = (tn < t_hi && lane < 8) ? __ldg(tt.leaf + tn * 8 + lane) : 0;
+        const int nx_node = (tn < t_hi && lane < 28) ? __ldg(tt.node + tn * 7 + (lane >> 2)) : 0;
         Gate<float> g[7];
         float pq[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) pq[i] = w_next[i];
-        quad_load(tree_row(tt, active ? lane : 0, nx_node), lane & 3, active && t + 8 < t_hi, w_next);
-        const int nn_leaf = leaf_of(t + 16);
-        nx_node = node_of(t + 16);
-        tree_gates_of(lane, wmode, g, pq);
+        tree_gates_of(tt, my_node, lane, wmode, g, pq);
         const float *row[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) row[q] = x + (long long)__shfl_sync(0xffffffffu, my_leaf, q) * B;
-        my_leaf = nx_leaf, nx_leaf = nn_leaf;
+        my_leaf = nx_leaf, my_node = nx_node;
 #pragma unroll
         for (int tr = 0; tr < TR; ++tr) {
             const long long b0 = ((long long)tr * 32 + lane) * 4;
@@ -644,8 +626,7 @@ __global__ void __launch_bounds__(128, 3) logic_tree_bwd_kernel(const float *__r
         const int nx_node = (tn < T && lane < 28) ? __ldg(tt.node + tn * 7 + (lane >> 2)) : 0;
         Gate<float> g[7];
         float pq[4]; // the lane's four mixture entries, kept for the soft-max Jacobian at the end
-        quad_load(tree_row(tt, lane < 28 ? lane : 0, my_node), lane & 3, lane < 28, pq);
-        tree_gates_of(lane, wmode, g, pq);
+        tree_gates_of(tt, my_node, lane, wmode, g, pq);
         const float *row[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) row[k] = x + (long long)__shfl_sync(0xffffffffu, my_leaf, k) * B;
@@ -1030,11 +1011,10 @@ extern "C" int clb_logic_tree_fwd(const float *x, const int32_t *leaf, const int
 
 // tapgrad: scratch of T*8*B floats.  gw0/gw1/gw2 must be zeroed by the caller: neurons no tree uses keep zero.
 // start int64 [in_dim + 1], list int32 [T*8]: the leaf slots (t*8 + k) grouped by the input feature they read.
-// parts of a class for the fused forward + class sums: one wave of blocks, which are three to an SM (two beyond 256 samples); four to
-// an SM, the rule before, left a second wave a third full (81920 trees, 256 samples: 108 us, now 85)
-static int tree_sum_parts(int64_t T, int64_t B, int k)
+// parts of a class for the fused forward + class sums: enough blocks to fill the GPU a few times over
+static int tree_sum_parts(int64_t T, int k)
 {
-    long long parts = (long long)sm_count() * (B <= 256 ? 3 : 2) / k;
+    long long parts = ((long long)sm_count() * 4 + k - 1) / k;
     const long long most = T / k / 8; // at least eight trees (one per warp) per part
     if (parts > most) parts = most;
     return (int)(parts < 1 ? 1 : parts);
@@ -1043,7 +1023,7 @@ static int tree_sum_parts(int64_t T, int64_t B, int k)
 extern "C" size_t clb_logic_tree_fwd_ce_scratch_bytes(int64_t T, int64_t B, int k)
 {
     if (T <= 0 || B <= 0 || k <= 0 || T % k) return 0;
-    return (size_t)tree_sum_parts(T, B, k) * (size_t)k * (size_t)B * sizeof(float);
+    return (size_t)tree_sum_parts(T, k) * (size_t)k * (size_t)B * sizeof(float);
 }
 
 extern "C" int clb_logic_tree_fwd_ce(const float *x, const int32_t *leaf, const int32_t *node, const float *w0, const float *w1,
@@ -1055,7 +1035,7 @@ extern "C" int clb_logic_tree_fwd_ce(const float *x, const int32_t *leaf, const 
     if (!scratch || scratch_bytes < clb_logic_tree_fwd_ce_scratch_bytes(T, B, k)) return CLB_ERR_SCRATCH;
     TreeTables tt{leaf, node, {w0, w1, w2}};
     cudaStream_t st = (cudaStream_t)stream;
-    const int parts = tree_sum_parts(T, B, k);
+    const int parts = tree_sum_parts(T, k);
     const dim3 grid((unsigned)parts, (unsigned)k);
     float *partial = (float *)scratch;
     if (B <= 128)
