@@ -226,15 +226,15 @@ __global__ void __launch_bounds__(256) logic_bwd_x_kernel(const T *__restrict__ 
 
 // ----------------------------------------------------------------------------------- group sum
 // GroupSum on the feature-major activations the flat layers produce ([F][B]; class c owns rows [c*S, (c+1)*S)):
-// out[b][c] = (sum of the class's rows at sample b) / tau.  Block (batch tile, class, part): its W warps add the part's rows
-// round robin and are combined in warp order; with several parts the finalize kernel adds those in order.  One part of 32 warps,
-// and no second launch, while a class has few rows.  No transposed copy of the activations, no atomics.
+// out[b][c] = (sum of the class's rows at sample b) / tau.  The rows of a class are 16 parts (one when there are few) of eight
+// chains, row by row in turn; chains are added in order, then parts.  No transposed copy of the activations, no atomics.
 constexpr int kGroupSumParts = 16;
 
-template <typename T, int W, bool FINAL>
-__global__ void __launch_bounds__(32 * W) group_sum_partial_kernel(const T *__restrict__ y, T *__restrict__ out, long long S, long long B, int k, T tau)
+// Block (batch tile, class, part): a warp per chain.
+template <typename T>
+__global__ void __launch_bounds__(256) group_sum_partial_kernel(const T *__restrict__ y, T *__restrict__ partial, long long S, long long B, int k)
 {
-    __shared__ T red[W][32];
+    __shared__ T red[8][32];
     const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
     const long long b = (long long)blockIdx.x * 32 + lane;
     const int c = blockIdx.y, part = blockIdx.z;
@@ -242,17 +242,49 @@ __global__ void __launch_bounds__(32 * W) group_sum_partial_kernel(const T *__re
     T acc = T(0);
     if (b < B)
 #pragma unroll 8
-        for (long long r = r0 + wv; r < r1; r += W) acc += y[((long long)c * S + r) * B + b];
+        for (long long r = r0 + wv; r < r1; r += 8) acc += y[((long long)c * S + r) * B + b];
     red[wv][lane] = acc;
     __syncthreads();
     if (wv == 0 && b < B) {
         T t = red[0][lane];
 #pragma unroll
-        for (int i = 1; i < W; ++i) t += red[i][lane];
-        if (FINAL)
-            out[b * k + c] = t / tau;
-        else
-            out[((long long)part * k + c) * B + b] = t;
+        for (int i = 1; i < 8; ++i) t += red[i][lane];
+        partial[((long long)part * k + c) * B + b] = t;
+    }
+}
+
+// Few rows: block (batch tile, class), two warps to a part and four chains to a warp, and no second launch.
+template <typename T>
+__global__ void __launch_bounds__(1024) group_sum_one_kernel(const T *__restrict__ y, T *__restrict__ out, long long S, long long B, int k, int parts, T tau)
+{
+    __shared__ T red[kGroupSumParts][8][32];
+    const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5, part = wv >> 1, w0 = (wv & 1) * 4;
+    const long long b = (long long)blockIdx.x * 32 + lane;
+    const int c = blockIdx.y;
+    if (part < parts && b < B) {
+        const long long r0 = S * part / parts, r1 = S * (part + 1) / parts;
+        const T *col = y + (long long)c * S * B + b;
+        T acc[4] = {T(0), T(0), T(0), T(0)};
+#pragma unroll 4
+        for (long long r = r0 + w0; r < r1; r += 8)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (r + j < r1) acc[j] += col[(r + j) * B];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) red[part][w0 + j][lane] = acc[j];
+    }
+    __syncthreads();
+    if (wv < parts) {
+        T t = red[wv][0][lane];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) t += red[wv][i][lane];
+        red[wv][0][lane] = t;
+    }
+    __syncthreads();
+    if (wv == 0 && b < B) {
+        T t = T(0);
+        for (int p = 0; p < parts; ++p) t += red[p][0][lane];
+        out[b * k + c] = t / tau;
     }
 }
 
@@ -902,10 +934,10 @@ extern "C" int clb_group_sum_fwd(const void *y, void *out, void *scratch, size_t
         using T = decltype(t);
         if (S <= 4096) { // 128 rows per warp at most: about what a second launch costs
             grid.z = 1;
-            CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<T, 32, true><<<grid, 1024, 0, st>>>((const T *)y, (T *)out, S, B, k, (T)tau));
+            CLB_TRACED("group_sum_one_kernel", st, group_sum_one_kernel<T><<<grid, 1024, 0, st>>>((const T *)y, (T *)out, S, B, k, parts, (T)tau));
             return 1;
         }
-        CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<T, 8, false><<<grid, 256, 0, st>>>((const T *)y, (T *)scratch, S, B, k, (T)tau));
+        CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<T><<<grid, 256, 0, st>>>((const T *)y, (T *)scratch, S, B, k));
         CLB_TRACED("group_sum_finalize_kernel", st, group_sum_finalize_kernel<T><<<fb, 256, 0, st>>>((const T *)scratch, (T *)out, B, k, parts, (T)tau));
         return 2;
     };
@@ -922,7 +954,7 @@ extern "C" int clb_group_sum_ce(const float *y, const int64_t *labels, float *sc
     const int parts = group_sum_parts(S);
     cudaStream_t st = (cudaStream_t)stream;
     dim3 grid((unsigned)((B + 31) / 32), (unsigned)k, (unsigned)parts);
-    CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<float, 8, false><<<grid, 256, 0, st>>>(y, (float *)scratch, S, B, k, 1.f));
+    CLB_TRACED("group_sum_partial_kernel", st, group_sum_partial_kernel<float><<<grid, 256, 0, st>>>(y, (float *)scratch, S, B, k));
     CLB_TRACED("group_sum_ce_sample_kernel", st,
                group_sum_ce_sample_kernel<<<(unsigned)((B + 7) / 8), 256, 0, st>>>((float *)scratch, labels, scores, dscore, B, k, parts, (float)tau));
     CLB_TRACED("group_sum_loss_mean_kernel", st, group_sum_loss_mean_kernel<<<1, 256, 0, st>>>((const float *)scratch, loss, B));
