@@ -1248,14 +1248,15 @@ int clb_convtree_fwd_fast_f32(const float *x, const float *w, const int32_t *sel
 {
     FastShape s;
     if (sh != 1 || sw != 1) return CLB_ERR_SHAPE;
-    // The plane kernels (images of 32, 28, 16, 12, 8 or 4 pixels) stream two channel planes per output channel; the tiled ones below
+    // The plane kernels (images of 32, 28, 16, 12, 8, 6 or 4 pixels) stream two channel planes per output channel; the tiled ones below
     // stage all channels of a few images.  With few channels and few windows the latter have less set-up (1 -> 64 channels, 16x16,
     // batch 64: 6.1 against 7.9 us); otherwise the former are faster whatever the channel count (9 -> 128, 16x16, batch 256:
     // 24.8 against 32.3; 32 -> 128, batch 100: 13.3 against 35.6; 16 -> 1024, 4x4, batch 500: 38 against 85).  Images of 28 and 32
-    // pixels have enough windows always (9 -> 256, 32x32, batch 256: 102 against 132; 1 -> 16, 28x28, batch 8: 4.9 and 4.9); of 12 from
-    // eight channels on (512 out, batch 400: with 16 channels 88 against 105, with 5 94 against 83).
+    // pixels have enough windows always (9 -> 256, 32x32, batch 256: 102 against 132; 1 -> 16, 28x28, batch 8: 4.9 and 4.9); 6x6
+    // suits the tiled kernels badly (24 -> 72, batch 200: 7.6 against 70); images of 12 from eight channels on (512 out, batch 400:
+    // with 16 channels 88 against 105, with 5 94 against 83).
     const bool many_channels = (size_t)Ci * (H + 2 * ph) * (W + 2 * pw) * 4 > 48 * 1024;
-    if (many_channels || Ci >= 16 || H >= 28 || (H == 12 && Ci >= 8) || (H != 12 && (long long)N * C * H * W >= (4LL << 20))) {
+    if (many_channels || Ci >= 16 || H >= 28 || H == 6 || (H == 12 && Ci >= 8) || (H != 12 && (long long)N * C * H * W >= (4LL << 20))) {
         const int rc = clb_convtree_fwd_plane_f32(x, w, sel, y, amax, N, Ci, H, W, C, sh, sw, ph, pw, kh, kw, wmode, st);
         if (rc != CLB_ERR_SHAPE) return rc;
     }

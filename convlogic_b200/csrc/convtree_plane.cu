@@ -1,4 +1,4 @@
-// Fused ConvLogic block on channel planes: fp32, stride 1, 3x3 window, padding 1, square images of 32, 28, 16, 12, 8 or 4 pixels (other
+// Fused ConvLogic block on channel planes: fp32, stride 1, 3x3 window, padding 1, square images of 32, 28, 16, 12, 8, 6 or 4 pixels (other
 // shapes take the kernels of convtree_fast.cu / convtree.cu).
 //
 // An output channel reads only the (normally two) input channels its 8 taps name, so a block owns ONE output
@@ -49,6 +49,10 @@ template <> struct Geo<28> {
 };
 template <> struct Geo<12> {
     static constexpr int R = 14, FWD_NIMG = 2, FWD_P = 24, FWD_IMG = 14 * 24;
+};
+// 6x6: rows of 6 columns over the whole block; every placement of a warp's 32 lanes has some banks twice (rows 24 apart, images 104).
+template <> struct Geo<6> {
+    static constexpr int R = 8, FWD_NIMG = 14, FWD_P = 12, FWD_IMG = 104;
 };
 template <> struct Geo<16> {
     static constexpr int P = 24, R = 18, FWD_NIMG = 2, FWD_P = 24, FWD_IMG = 18 * 24;
@@ -131,6 +135,13 @@ template <int OFF> __device__ __forceinline__ void cp_async16_off(uint32_t dst, 
 {
     asm volatile("cp.async.cg.shared.global [%0+%2], [%1], 16;" ::"r"(dst), "l"(src), "n"(OFF) : "memory");
 }
+template <int OFF, int BYTES> __device__ __forceinline__ void cp_async_off(uint32_t dst, const void *src)
+{
+    if constexpr (BYTES == 16)
+        cp_async16_off<OFF>(dst, src);
+    else
+        asm volatile("cp.async.ca.shared.global [%0+%2], [%1], %3;" ::"r"(dst), "l"(src), "n"(OFF), "n"(BYTES) : "memory");
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int PENDING> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
@@ -148,7 +159,7 @@ template <int S> struct FwdCfg {
     using G = Geo<S>;
     static constexpr int P = G::FWD_P, R = G::R, NIMG = G::FWD_NIMG;
     static constexpr int WO = S, HP = S / 2, WP = S / 2, I = HP * WP;
-    static constexpr bool WIDE = S >= 16;                        // one group of 128 threads, else four warps on their own
+    static constexpr bool WIDE = S >= 16 || S == 6;                      // one group of 128 threads, else four warps on their own
     static constexpr int GROUPS = WIDE ? 1 : kThreads / 32, GSIZE = WIDE ? kThreads : 32;
     static constexpr int IMG = G::FWD_IMG;                       // floats of one staged plane (R * P + padding)
     static constexpr int SLOT = (NIMG * IMG + 31) / 32 * 32;     // floats of one slot (NIMG planes of one channel)
@@ -159,14 +170,15 @@ template <int S> struct FwdCfg {
     static constexpr bool SPLIT_PAIRS = NIMG > 2, ROW_PAIRS = NIMG == 1;
     static constexpr int PAIR_STRIDE = SPLIT_PAIRS ? IMG : 2 * IMG, SECOND = ROW_PAIRS ? HP * P : SPLIT_PAIRS ? (NIMG / 2) * IMG : IMG;
     // A row of a pair takes LANES lanes, RPG rows are evaluated at a time, and the ROWS of an iteration take SUB turns.
-    static constexpr int LANES = S == 28 ? 32 : S, RPG = GSIZE / 32 * (32 / LANES), ROWS = ROW_PAIRS ? HP / 2 : NIMG / 2 * HP, SUB = (ROWS + RPG - 1) / RPG;
+    static constexpr int LANES = S == 28 ? 32 : S, RPG = S == 6 ? GSIZE / LANES : GSIZE / 32 * (32 / LANES), ROWS = ROW_PAIRS ? HP / 2 : NIMG / 2 * HP, SUB = (ROWS + RPG - 1) / RPG;
     static constexpr bool FULL = 32 % S == 0 && ROWS % RPG == 0;  // else some threads have no position, or none in the last turn
     static_assert(IMG >= R * P && IMG % 4 == 0 && P % 4 == 0 && (!TMA || IMG == R * P) && (SUB == 1 || NIMG <= 2), "tile geometry");
     static constexpr int STAGES = S == 16 ? 4 : 3;
     static constexpr int SMEM = GROUPS * STAGES * STAGE_BYTES + (FULL ? 0 : 2 * 2 * P * 4); // rows that a last turn reads in vain
-    // resident per SM: by registers (16), else by shared memory
-    static constexpr int BLOCKS = S == 16 ? 7 : S >= 28 ? 6 : S == 8 ? 5 : S == 4 ? 4 : 3;
-    static constexpr int UNITS = NIMG * 2 * S * (S / 4), CPQ = (UNITS + GSIZE - 1) / GSIZE; // 16-byte copies per iteration, and per thread (cp.async staging)
+    // resident per SM: by registers (16 and 6), else by shared memory
+    static constexpr int BLOCKS = S == 16 ? 7 : S >= 28 ? 6 : S == 8 || S == 6 ? 5 : S == 4 ? 4 : 3;
+    // asynchronous copies of PIECE floats: per iteration, and per thread
+    static constexpr int PIECE = S % 4 == 0 ? 4 : 2, UNITS = NIMG * 2 * S * (S / PIECE), CPQ = (UNITS + GSIZE - 1) / GSIZE;
 };
 
 // Turn J of one stage of the ring: both conv rows of both members of the thread's pair.
@@ -308,11 +320,11 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
 #pragma unroll
     for (int q = 0; q < Cf::CPQ; ++q) {
         const int u = gt + q * Cf::GSIZE;
-        constexpr int W4 = S / 4;
+        constexpr int W4 = S / Cf::PIECE;
         const int col4 = u % W4, row = (u / W4) % S, slot = (u / (W4 * S)) & 1, img = u / (W4 * S * 2);
-        csrc[q] = x + ((size_t)(n_lo + img) * s.Ci + (slot ? ch_b : ch_a)) * HW + row * S + col4 * 4;
+        csrc[q] = x + ((size_t)(n_lo + img) * s.Ci + (slot ? ch_b : ch_a)) * HW + row * S + col4 * Cf::PIECE;
         cp_iters[q] = u < Cf::UNITS ? (n_hi - n_lo - img + Cf::NIMG - 1) / Cf::NIMG : 0;
-        cdst[q] = clb_tma::smem_addr(gbase) + 4u * (uint32_t)(slot * Cf::SLOT + img * Cf::IMG + (row + 1) * Cf::P + kLead + col4 * 4);
+        cdst[q] = clb_tma::smem_addr(gbase) + 4u * (uint32_t)(slot * Cf::SLOT + img * Cf::IMG + (row + 1) * Cf::P + kLead + col4 * Cf::PIECE);
     }
     const size_t cstep = (size_t)Cf::NIMG * s.Ci * HW;
     // Called once per iteration in rising order (the pointers advance); always commits, so that the group counts stay
@@ -321,7 +333,7 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
     {                                                                                                                     \
         _Pragma("unroll") for (int q = 0; q < Cf::CPQ; ++q)                                                               \
         {                                                                                                                 \
-            if ((IT) < cp_iters[q]) cp_async16_off<(ST) * Cf::STAGE_BYTES>(cdst[q], csrc[q]);                             \
+            if ((IT) < cp_iters[q]) cp_async_off<(ST) * Cf::STAGE_BYTES, 4 * Cf::PIECE>(cdst[q], csrc[q]);                             \
             csrc[q] += cstep;                                                                                             \
         }                                                                                                                 \
         cp_async_commit();                                                                                                \
@@ -925,7 +937,7 @@ int fwd_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw,
 {
     const int side = square_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw);
     if (clb_tma::encode_tiled_fn() == nullptr) return 0;
-    return side == 32 || side == 28 || side == 16 || side == 12 || side == 8 || side == 4 ? side : 0;
+    return side == 32 || side == 28 || side == 16 || side == 12 || side == 8 || side == 6 || side == 4 ? side : 0;
 }
 // the gate gradient alone of a 32x32 block
 bool w32_covers(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw, int kh, int kw)
@@ -937,8 +949,9 @@ template <int S>
 int launch_fwd(const float *x, const float *w, const int32_t *sel, float *y, uint8_t *amax, int N, int Ci, int C, int wmode, cudaStream_t st)
 {
     using Cf = FwdCfg<S>;
-    CUtensorMap map;
-    if (!clb_tma::make_plane_map(&map, x, N, Ci, S, S, Cf::P, Cf::R, Cf::NIMG)) return CLB_ERR_SHAPE;
+    CUtensorMap map{};
+    if (reinterpret_cast<uintptr_t>(x) & 15) return CLB_ERR_SHAPE;
+    if (Cf::TMA && !clb_tma::make_plane_map(&map, x, N, Ci, S, S, Cf::P, Cf::R, Cf::NIMG)) return CLB_ERR_SHAPE;
     auto k = convtree_fwd_plane_kernel<S>;
     if (clb_host::ensure_dynamic_smem(k, Cf::SMEM) != cudaSuccess) return check_launch(0);
     const int parts = clb_plane_parts(N, C, Cf::NIMG, Cf::GROUPS, Cf::BLOCKS);
@@ -963,14 +976,14 @@ template <int S> int launch_bwd(const ClbTileBwd &a, cudaStream_t st)
     return CLB_OK;
 }
 
-// The sides of the two backward passes.  16, 8 and 4: always, as in the forward.  32, 28 and 12: from 4, 8 and 12 channels on.  With
+// The sides of the two backward passes.  16, 8, 6 and 4: always, as in the forward.  32, 28 and 12: from 4, 8 and 12 channels on.  With
 // fewer the kernel that keeps all channels of a few images in shared memory, and needs no second pass over the planes, is
 // as good or better (us with it / with the planes; 128 images, 128 channels out: 32x32 with 4 channels in 98 / 93, with 16
 // 211 / 99; 28x28 with 4 95 / 104, with 8 111 / 105, with 32 242 / 112; 256 images of 12x12, 256 out: with 8 71 / 87, with 32 271 / 88).
 int bwd_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw, int kh, int kw)
 {
     const int side = square_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw);
-    const int least = side == 32 ? 4 : side == 28 ? 8 : side == 12 ? 12 : side == 16 || side == 8 || side == 4 ? 1 : Ci + 1;
+    const int least = side == 32 ? 4 : side == 28 ? 8 : side == 12 ? 12 : side == 16 || side == 8 || side == 6 || side == 4 ? 1 : Ci + 1;
     return Ci >= least ? side : 0;
 }
 // Images of a slice of the batch: the gradient planes, eight bytes per pixel and output channel, of a slice stay below 1 GB.
@@ -1015,6 +1028,7 @@ int clb_convtree_fwd_plane_f32(const float *x, const float *w, const int32_t *se
     if (side == 32) return launch_fwd<32>(x, w, sel, y, amax, N, Ci, C, wmode, st);
     if (side == 28) return launch_fwd<28>(x, w, sel, y, amax, N, Ci, C, wmode, st);
     if (side == 12) return launch_fwd<12>(x, w, sel, y, amax, N, Ci, C, wmode, st);
+    if (side == 6) return launch_fwd<6>(x, w, sel, y, amax, N, Ci, C, wmode, st);
     if (side == 16) return launch_fwd<16>(x, w, sel, y, amax, N, Ci, C, wmode, st);
     if (side == 8) return launch_fwd<8>(x, w, sel, y, amax, N, Ci, C, wmode, st);
     if (side == 4) return launch_fwd<4>(x, w, sel, y, amax, N, Ci, C, wmode, st);

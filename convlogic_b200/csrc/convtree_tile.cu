@@ -1,5 +1,5 @@
 // Backward, pass 1, of a fused ConvLogic block whose output channels each read (at most) two input channels: fp32, stride 1, 3x3
-// window, padding 1, square images of 32, 28, 16 or 12 pixels.
+// window, padding 1, square images of 32, 28, 16, 12 or 6 pixels.
 //
 // A group of threads (a warp; four warps for 32 and 28 pixels) owns one output channel and a part of the batch.  It keeps the two
 // channel planes of NIMG images in shared memory, recomputes the gate chain of every pooled window at its saved arg-max, keeps the
@@ -28,20 +28,20 @@ template <int S> struct Tile {
     static constexpr int H2 = S / 2, I = H2 * H2;
     static constexpr int WARPS = S >= 28 ? 4 : 1, GROUPS = 4 / WARPS, GSIZE = 32 * WARPS;
     static constexpr int BLOCKS = S == 28 || S == 12 ? 3 : 4; // resident per SM: 128 registers a thread where the kernel fits them, else 168
-    static constexpr int NIMG = S == 12 ? 2 : 1;              // images per iteration
+    static constexpr int NIMG = S == 6 ? 3 : S == 12 ? 2 : 1;  // images per iteration
     // a warp's 32 lanes are RW window rows, PASSES apart, of H2 windows; a thread has its place in WPT of the PASSES such sets
-    static constexpr int RW = S == 12 ? 4 : 32 / H2, PASSES = NIMG * H2 / RW, WPT = (PASSES + WARPS - 1) / WARPS;
+    static constexpr int RW = S == 6 ? 9 : S == 12 ? 4 : 32 / H2, PASSES = NIMG * H2 / RW, WPT = (PASSES + WARPS - 1) / WARPS;
     static constexpr bool FULL = RW * H2 == 32;
     // floats: pitch of a parity plane's rows, distance of images in it, size of a plane, of a channel slot, of the tile
-    static constexpr int P = S == 32 ? 22 : S == 28 ? 16 : S == 16 ? 12 : 8;
-    static constexpr int IMG = S == 12 ? 80 : 0;
+    static constexpr int P = S == 32 ? 22 : S == 28 ? 16 : S == 16 ? 12 : S == 6 ? 4 : 8;
+    static constexpr int IMG = S == 12 ? 80 : S == 6 ? 21 : 0;
     static constexpr int PL = ((NIMG - 1) * IMG + H2 * P + H2 + 2 + 31) / 32 * 32, SLOT = 4 * PL, LEAD = 2;
     static constexpr int BYTES = (LEAD + 2 * SLOT + 2) * 4, GRAD = (BYTES + 15) / 16 * 16; // the gradient tile, GRAD bytes behind
     static constexpr int SMEM = GROUPS * 2 * GRAD;
-    // four neighbouring pixels of a row: unit u = (channel slot, row parity, image, row of that parity, column / 4), column fastest
-    static constexpr int W4 = S / 4, UNITS = 2 * NIMG * S * W4, UPT = (UNITS + GSIZE - 1) / GSIZE;
+    // a unit is QUAD neighbouring pixels of a row: u = (channel slot, row parity, image, row of that parity, column / QUAD), column fastest
+    static constexpr int QUAD = S % 4 == 0 ? 4 : 2, W4 = S / QUAD, UNITS = 2 * NIMG * S * W4, UPT = (UNITS + GSIZE - 1) / GSIZE;
     static constexpr bool REGULAR = NIMG * H2 * W4 == GSIZE; // then unit q of a thread is its pixel quad in row parity q & 1 of channel slot q >> 1
-    static_assert(NIMG * H2 == RW * PASSES && (NIMG == 1 || IMG >= H2 * P + H2 + 2) && P > H2 && P % 2 == 0, "tile geometry");
+    static_assert(NIMG * H2 == RW * PASSES && (NIMG == 1 || IMG >= H2 * P + H2 + 2) && P > H2 && (QUAD == 2 || P % 2 == 0), "tile geometry");
 };
 
 template <int OFF> __device__ __forceinline__ float lds1(uint32_t a)
@@ -79,7 +79,7 @@ template <int S, bool FM>
 __global__ void __launch_bounds__(kThreads, Tile<S>::BLOCKS) convtree_bwd_plane_kernel(ClbTileBwd s)
 {
     using T = Tile<S>;
-    constexpr int WPT = T::WPT, UPT = T::UPT, I = T::I, H2 = T::H2, HW = S * S, NIMG = T::NIMG, GT = T::GRAD;
+    constexpr int WPT = T::WPT, UPT = T::UPT, I = T::I, H2 = T::H2, HW = S * S, NIMG = T::NIMG, GT = T::GRAD, QUAD = T::QUAD;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ __align__(16) Gate<float> sgs[T::GROUPS][7];
     __shared__ SlotInfo sis[T::GROUPS];
@@ -146,9 +146,9 @@ __global__ void __launch_bounds__(kThreads, Tile<S>::BLOCKS) convtree_bwd_plane_
         const int col4 = u % T::W4, k = u / T::W4 % H2, img = u / (T::W4 * H2) % NIMG, even = u / (T::W4 * H2 * NIMG) & 1, slot = u / (T::W4 * H2 * NIMG * 2);
         const int r = S == 16 ? (k % 4) * 2 + k / 4 : S == 32 ? (k % 2) * 8 + k / 2 : k; // rows of a half-warp's pairs in different banks
         const int y = 2 * r + even;                                                      // padded row y + 1
-        xoff[q] = (img * s.Ci + (slot ? si.ch[1] : si.ch[0])) * HW + y * S + 4 * col4;
-        poff[q] = (img * s.C * 2 + slot) * HW + y * S + 4 * col4;
-        ucell[q] = tile + 4u * (uint32_t)(T::LEAD + slot * T::SLOT + (even ? 0 : 2 * T::PL) + img * T::IMG + (r + even) * T::P + 2 * col4);
+        xoff[q] = (img * s.Ci + (slot ? si.ch[1] : si.ch[0])) * HW + y * S + QUAD * col4;
+        poff[q] = (img * s.C * 2 + slot) * HW + y * S + QUAD * col4;
+        ucell[q] = tile + 4u * (uint32_t)(T::LEAD + slot * T::SLOT + (even ? 0 : 2 * T::PL) + img * T::IMG + (r + even) * T::P + QUAD / 2 * col4);
         uimg[q] = u < T::UNITS ? img : 1 << 20;
     }
     const int second = T::REGULAR ? (si.ch[1] - si.ch[0]) * HW : 0;
@@ -157,18 +157,28 @@ __global__ void __launch_bounds__(kThreads, Tile<S>::BLOCKS) convtree_bwd_plane_
     auto cell_at = [&](int q) { return T::REGULAR ? ucell[0] + 4u * (uint32_t)((q & 1) * (T::P - 2 * T::PL) + (q >> 1) * T::SLOT) : ucell[q]; };
     auto img_at = [&](int q) { return uimg[T::REGULAR ? 0 : q]; };
 
-    float4 xv[UPT];
+    float xv[UPT][QUAD];
     float dz[WPT];
     int bd[WPT];
 #pragma unroll
-    for (int q = 0; q < UPT; ++q) xv[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int q = 0; q < UPT; ++q)
+#pragma unroll
+        for (int i = 0; i < QUAD; ++i) xv[q][i] = 0.f;
     const float *gb = FM ? s.gy + (size_t)c * I * s.n_stride + n_lo : s.gy + ((size_t)n_lo * s.C + c) * I;
     const uint8_t *ab = s.amax + ((size_t)n_lo * s.C + c) * I;
     int left = n_hi - n_lo; // images from the next to be fetched on
     auto fetch = [&] {
 #pragma unroll
         for (int q = 0; q < UPT; ++q)
-            if (img_at(q) < left) xv[q] = __ldg(reinterpret_cast<const float4 *>(xb + x_at(q)));
+            if (img_at(q) < left) {
+                if constexpr (QUAD == 4) {
+                    const float4 v = __ldg(reinterpret_cast<const float4 *>(xb + x_at(q)));
+                    xv[q][0] = v.x, xv[q][1] = v.y, xv[q][2] = v.z, xv[q][3] = v.w;
+                } else {
+                    const float2 v = __ldg(reinterpret_cast<const float2 *>(xb + x_at(q)));
+                    xv[q][0] = v.x, xv[q][1] = v.y;
+                }
+            }
 #pragma unroll
         for (int j = 0; j < WPT; ++j) {
             const bool live = img_of[j] >= 0 && img_of[j] < left;
@@ -182,10 +192,15 @@ __global__ void __launch_bounds__(kThreads, Tile<S>::BLOCKS) convtree_bwd_plane_
     fetch();
 #pragma unroll 1
     for (int it = 0; it < iters; ++it) {
-        // pixels 4q .. 4q + 3 are padded columns 4q + 1 .. 4q + 4: two of the odd plane, two of the even one
+        // pixels 4q .. 4q + 3 are padded columns 4q + 1 .. 4q + 4: two of the odd plane, two of the even one (of a pair one each)
 #pragma unroll
         for (int q = 0; q < UPT; ++q)
-            if (T::UNITS % T::GSIZE == 0 || img_at(q) < NIMG) sts2<4 * T::PL>(cell_at(q), xv[q].x, xv[q].z), sts2<0>(cell_at(q), xv[q].y, xv[q].w);
+            if (T::UNITS % T::GSIZE == 0 || img_at(q) < NIMG) {
+                if constexpr (QUAD == 4)
+                    sts2<4 * T::PL>(cell_at(q), xv[q][0], xv[q][2]), sts2<0>(cell_at(q), xv[q][1], xv[q][3]);
+                else
+                    sts1<4 * T::PL>(cell_at(q), xv[q][0]), sts1<0>(cell_at(q), xv[q][1]);
+            }
         float d[WPT];
         uint32_t pos[WPT];
 #pragma unroll
@@ -225,9 +240,15 @@ __global__ void __launch_bounds__(kThreads, Tile<S>::BLOCKS) convtree_bwd_plane_
         for (int q = 0; q < UPT; ++q) {
             if (T::UNITS % T::GSIZE != 0 && img_at(q) >= NIMG) continue;
             const uint32_t at = cell_at(q);
-            const float2 odd = lds2<GT + 4 * T::PL>(at), even = lds2<GT>(at);
-            sts2<GT + 4 * T::PL>(at, 0.f, 0.f), sts2<GT>(at, 0.f, 0.f);
-            if (img_at(q) < have) *reinterpret_cast<float4 *>(pb + p_at(q)) = make_float4(odd.x, even.x, odd.y, even.y);
+            if constexpr (QUAD == 4) {
+                const float2 odd = lds2<GT + 4 * T::PL>(at), even = lds2<GT>(at);
+                sts2<GT + 4 * T::PL>(at, 0.f, 0.f), sts2<GT>(at, 0.f, 0.f);
+                if (img_at(q) < have) *reinterpret_cast<float4 *>(pb + p_at(q)) = make_float4(odd.x, even.x, odd.y, even.y);
+            } else {
+                const float odd = lds1<GT + 4 * T::PL>(at), even = lds1<GT>(at);
+                sts1<GT + 4 * T::PL>(at, 0.f), sts1<GT>(at, 0.f);
+                if (img_at(q) < have) *reinterpret_cast<float2 *>(pb + p_at(q)) = make_float2(odd, even);
+            }
         }
         pb += (size_t)NIMG * s.C * 2 * HW;
     }
@@ -262,10 +283,12 @@ using namespace clb::plane;
 
 int clb_tile_bwd_parts(int side, int N, int C)
 {
-    return side == 32 ? parts_for<32>(N, C) : side == 28 ? parts_for<28>(N, C) : side == 16 ? parts_for<16>(N, C) : parts_for<12>(N, C);
+    return side == 32 ? parts_for<32>(N, C) : side == 28 ? parts_for<28>(N, C) : side == 16 ? parts_for<16>(N, C) : side == 12 ? parts_for<12>(N, C)
+           : parts_for<6>(N, C);
 }
 
 int clb_tile_bwd(int side, const ClbTileBwd &a, cudaStream_t st)
 {
-    return side == 32 ? launch<32>(a, st) : side == 28 ? launch<28>(a, st) : side == 16 ? launch<16>(a, st) : launch<12>(a, st);
+    return side == 32 ? launch<32>(a, st) : side == 28 ? launch<28>(a, st) : side == 16 ? launch<16>(a, st) : side == 12 ? launch<12>(a, st)
+           : launch<6>(a, st);
 }

@@ -1,4 +1,4 @@
-"""The plane backward at every side it takes (32 and 28: four warps per image; 12: two images per warp, eight idle lanes), against
+"""The plane backward at every side it takes (32 and 28: four warps per image; 12 and 6: two and three images per warp, idle lanes), against
 the CPU oracle at the kernels' own pooled positions: ragged batches, one image, parts of the batch, channels whose taps all name
 one plane, an upstream gradient in the flat layers' layout (the same bits as for the ordinary one)."""
 
@@ -13,7 +13,8 @@ GEOM = (1, 1, 1, 1, 3, 3)
 
 
 @pytest.mark.parametrize("n,ci,c,side", [(1, 16, 5, 32), (9, 20, 3, 32), (5, 4, 2, 32), (40, 16, 4, 28), (1, 17, 2, 28), (1, 16, 7, 12), (35, 16, 3, 12),
-                                         (130, 40, 2, 12), (3, 4, 6, 16), (17, 4, 3, 8), (9, 4, 5, 4)])
+                                         (130, 40, 2, 12), (1, 12, 3, 6), (38, 48, 10, 6), (300, 20, 4, 6),
+                                         (3, 4, 6, 16), (17, 4, 3, 8), (9, 4, 5, 4)])
 def test_plane_backward_sides(n, ci, c, side):
     import convlogic_b200 as cb
     from convlogic_b200 import _lib, ops

@@ -1,4 +1,4 @@
-"""The plane forward at 32, 28 and 12 pixels (pairs of pooled rows of one image; rows of 28 or 24 of 32 lanes; a last turn that is
+"""The plane forward at 32, 28, 12 and 6 pixels (pairs of pooled rows of one image; rows of 28 or 24 of 32 lanes; a last turn that is
 half empty) against the general kernel, bit for bit: ragged batches, one image, feature-major output, selections on three channels."""
 
 import pytest
@@ -9,7 +9,7 @@ GEOM = (1, 1, 1, 1, 3, 3)
 
 
 @pytest.mark.parametrize("n,ci,c,side", [(1, 16, 5, 32), (9, 20, 3, 32), (300, 16, 2, 32), (7, 16, 4, 28), (1, 30, 2, 28), (1, 16, 7, 12), (35, 16, 3, 12),
-                                         (130, 40, 9, 12)])
+                                         (130, 40, 9, 12), (1, 16, 3, 6), (37, 48, 10, 6), (300, 20, 4, 6)])
 @pytest.mark.parametrize("spread", [False, True])
 def test_plane_forward_sides(n, ci, c, side, spread):
     import convlogic_b200 as cb
