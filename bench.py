@@ -190,19 +190,14 @@ def traced(fn, steps):
     return {k: (n / steps, ms / steps) for k, (n, ms) in rep.items()}
 
 
-# DRAM bytes (read + write) ncu counted for each kernel, summed over the kernel's launches in ONE step (c3, c2, c5) or
-# one 8192-image chunk (c4) of the default workload sizes: dram__bytes.sum over one capture of the same bench command
-# per workload (c5: the 64 000-neuron case of the same kernels, scaled by 4 to 256 000 neurons; its traffic grows with
-# the neuron count).  Other sizes report null.
+# DRAM bytes (read + write) ncu counted for each kernel, summed over the kernel's launches in ONE step (c3) or one 8192-image
+# chunk (c4) of the default workload sizes: dram__bytes.sum over one capture of the same bench command.  Other sizes, and
+# kernels without an entry, report null.
 NCU_TRAFFIC = {
     "c3": {"convtree_bwd_plane_kernel": 1930.7e6, "plane_sum_kernel": 1526.9e6, "logic_tree_bwd_kernel": 954.8e6,
-           "row_segment_sum_kernel": 706.5e6, "convtree_fwd_plane_kernel": 383.1e6, "adam_step_kernel": 245.7e6,
-           "logic_tree_fwd_sum_kernel": 92.1e6, "convtree_bwd_w_plane32_kernel": 97.8e6, "convtree_fwd_pair_kernel": 37.7e6},
-    "c4": {"packed_convtree_slab_kernel": 2317.2e6, "packed_tree_kernel": 1639.4e6, "group_popcount_kernel": 676.1e6,
-           "packed_rows_to_slab_kernel": 223.9e6, "thermometer_pack_kernel": 65.1e6},
-    "c2": {"convtree_fwd_pair_kernel": 37.3e6, "convtree_bwd_cls_kernel": 105.4e6, "convtree_bwd_post_kernel": 33.1e6},
-    "c5": {"logic_bwd_x_kernel": 7 * 4 * 1254.0e6, "logic_bwd_w_kernel": 7 * 4 * 741.0e6 + 4 * 288.5e6,
-           "logic_fwd_kernel": 7 * 4 * 707.5e6 + 4 * 227.0e6},
+           "row_segment_sum_kernel": 706.5e6, "convtree_fwd_plane_kernel": 420.8e6, "adam_step_kernel": 245.7e6,
+           "logic_tree_fwd_sum_kernel": 92.1e6, "convtree_bwd_w_plane32_kernel": 97.8e6},
+    "c4": {"packed_tree_kernel": 1639.4e6, "thermometer_pack_kernel": 65.1e6},
 }
 
 
@@ -246,7 +241,7 @@ def c3_algorithmic_bytes(batch):
         "convtree_fwd_chan_kernel": (y1 + y2) + (y2 + y3) + (y3 + y4),
         "convtree_bwd_cls_kernel": y1 + x1,
         "convtree_bwd_w_plane32_kernel": y1 + x1,
-        "convtree_fwd_plane_kernel": (y1 + y2) + (y2 + y3) + (y3 + y4),
+        "convtree_fwd_plane_kernel": (x1 + y1) + (y1 + y2) + (y2 + y3) + (y3 + y4),
         "convtree_bwd_plane_kernel": (y2 + y1) + (y3 + y2) + (y4 + y3),            # upstream gradient + input
         "plane_sum_kernel": y1 + y2 + y3,                                           # the input gradients
         "convtree_bwd_w_win_kernel<tapgrad>": (y2 + y1) + (y3 + y2) + (y4 + y3),   # upstream gradient + input
@@ -477,7 +472,7 @@ def run_c4(ctx, args):
     ms_e2e = ctx.timed(step_e2e, 1, 1)
     clocks = sampler.stop()
     peak, kind = measured_peaks()
-    per_image = {"packed_convtree_slab_kernel": 44672 + 65536 + 65536 + 49152, "packed_tree_kernel": 16384 + 81920,
+    per_image = {"packed_convtree_slab3_kernel": 44672 + 65536 + 65536 + 49152, "packed_tree_kernel": 16384 + 81920,
                  "group_popcount_kernel": 81920 + 40, "thermometer_pack_kernel": 3072 + 11904}
     kernels = kernel_table(trace, {k: v * chunk for k, v in per_image.items()}, peak, traffic=NCU_TRAFFIC["c4"] if chunk == 8192 else None)
     top = kernels[0] if kernels else {}
@@ -596,8 +591,9 @@ def run_c2(ctx, args):
     clocks = sampler.stop()
     peak, kind = measured_peaks()
     alg = c2_algorithmic_bytes()
-    names = {"convtree_fwd_pair_kernel": alg["fwd"], "convtree_fwd_tile_kernel": alg["fwd"], "convtree_bwd_cls_kernel": alg["bwd"]}
-    kernels = kernel_table(trace, names, peak, traffic=NCU_TRAFFIC["c2"])
+    names = {"convtree_fwd_pair_kernel": alg["fwd"], "convtree_fwd_tile_kernel": alg["fwd"], "convtree_bwd_cls_kernel": alg["bwd"],
+             "convtree_fwd_plane_kernel": alg["fwd"], "convtree_bwd_plane_kernel": alg["bwd"]}
+    kernels = kernel_table(trace, names, peak, traffic=None)
     top = kernels[0] if kernels else {}
     imgs = b * world * steps
     rec = {
@@ -691,9 +687,11 @@ def run_c5(ctx, args):
         "logic_fwd_kernel": (xin + row) + (depth - 1) * 2 * row,    # layer 1: x + y; the others: x + y
         "logic_bwd_w_kernel": (xin + row) + (depth - 1) * 2 * row,  # gy + x per layer
         "logic_bwd_x_kernel": (depth - 1) * 3 * row,                # all but the first layer: gy + x + gx
+        "logic_fwd_cols_kernel": (depth - 1) * 2 * row,             # the layers that walk the batch in stretches: x + y
+        "logic_bwd_kernel": (depth - 1) * 3 * row,                  # both gradients of all but the first layer: gy + x + gx
         "group_sum_partial_kernel": row, "group_sum_bwd_kernel": row,
     }
-    kernels = kernel_table(trace, names, peak, traffic=NCU_TRAFFIC["c5"] if (width, depth, batch) == (256000, 8, 1024) else None)
+    kernels = kernel_table(trace, names, peak, traffic=None)
     top = kernels[0] if kernels else {}
     # forward: layer 1 in + out, the others 2 rows each, GroupSum read; backward: 3 rows per layer, the first gy + x
     # (the GroupSum gradient counted as fused into the last layer): 39.9 GB at 256000 x 8
