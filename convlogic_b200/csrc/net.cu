@@ -29,11 +29,11 @@ namespace {
 
 constexpr char kMagic[8] = {'C', 'L', 'B', 'N', 'E', 'T', '0', '1'};
 constexpr size_t kHeaderBytes = 64, kLayerBytes = 64;
-// The one-launch kernel (net_cluster.cu) against layer-by-layer launches, us per call on B200: mnist k=16 batch 1 15.5 / 74.5,
-// batch 4096 25.9 / 82.5; cifar k=32 batch 1000 44 / 84, batch 8192 132 / 217; cifar k=128 (cost 0.5 M) batch 1 68 / 101, batch
-// 8192 469 / 513; cifar k=256 (cost 1 M) batch 1 136 / 107, batch 8192 1104 / 912.  Beyond one slab per SM the clusters come in waves
-// and the layered kernels win from k=32 on (batch 20000: 507 / 468).
-constexpr long long kOneLaunchCost = 600000;
+// The one-launch kernel (net_cluster.cu) against layer-by-layer launches, us per call on B200: mnist k=64 (cost 0.1 M) batch 1 25 / 52,
+// batch 8192 103 / 148; cifar k=32 (0.13 M) batch 1 31 / 39, batch 2000 57 / 62, batch 8192 131 / 127; cifar k=64 (0.25 M) batch 1
+// 43 / 39, batch 500 43 / 49, batch 1000 66 / 59, batch 8192 233 / 190; cifar k=128 batch 1 66 / 45.  Beyond one slab per SM the
+// clusters come in waves and the layered kernels win from k=32 on.
+constexpr long long kOneLaunchCost = 200000;
 
 struct Header {
     char magic[8];

@@ -133,117 +133,165 @@ __global__ void __launch_bounds__(256) pack_bits_nmajor_kernel(const uint8_t *__
 // Fused input stage of packed inference: pixels [N][P] (P = channels * H * W, fp32 in [0,1] or uint8 that is
 // divided by 255 as torchvision's ToTensor does) -> the L*P thermometer features "pixel > threshold[i]",
 // threshold-major (feature i*P + p), bit-packed along the batch, without the [N, L*P] byte tensor in between.
-// Block: 32 pixel positions (lanes: coalesced 128-byte reads of one sample) x 256 samples (8 warps x 32);
-// a thread builds, for its position, the 32-sample word of every level in registers; the words go through
-// shared memory so that each feature row receives 32 contiguous bytes (rows layout) or each (feature, slab)
-// 512 contiguous bytes (slab layout, one 16-byte unit per position).
-constexpr int kThermoLevels = 32; // levels handled per pass over the pixels
+// A block has 256 samples, 32 to a warp, and 32 pixel positions at a time, one to a lane: a thread builds, for its position, the 32-sample
+// word of every level in registers; the words go through shared memory so that each feature row receives 32 contiguous bytes
+// (rows layout) or each (feature, slab) 512 contiguous bytes (slab layout, one 16-byte unit per position).  Levels are taken 8 G at a
+// time, G = 1 .. 4 by their number.
+struct ThermoOut {
+    unsigned *out;
+    int P, HW;
+    long long words32;
+    int to_slab, side; // side: split column order
+};
 
-template <typename PIX>
-__device__ __forceinline__ float pixel_value(const PIX *p);
-template <>
-__device__ __forceinline__ float pixel_value<float>(const float *p)
+// nl levels from l0 of positions p0 .. p0 + 31: thread = (position, word), so only the level walks -- one shared load, one store and
+// two additions per level
+__device__ __forceinline__ void thermo_write(const unsigned *sm, const ThermoOut &o, int l0, int nl, int p0, long long n0)
 {
-    return __ldg(p);
-}
-template <>
-__device__ __forceinline__ float pixel_value<uint8_t>(const uint8_t *p)
-{
-    return __fdiv_rn((float)__ldg(p), 255.0f);
+    const long long w0 = n0 / 32; // first 32-bit word of this block in a row
+    if (!o.to_slab) {
+        // (level, position, word): 8 consecutive lanes write the 32 bytes of one row
+        const int w = threadIdx.x & 7, pos = (threadIdx.x >> 3) & 31;
+        const int pp = p0 + pos;
+        if (pp < o.P && w0 + w < o.words32) {
+            unsigned *dst = o.out + ((long long)l0 * o.P + pp) * o.words32 + w0 + w;
+            const unsigned *srcw = sm + pos * 9 + w;
+            const long long dstep = (long long)o.P * o.words32;
+            for (int i = 0; i < nl; ++i) dst[i * dstep] = srcw[i * 32 * 9];
+        }
+    } else {
+        // slab layout [feature channel][U][HW] of 16-byte units: 4 consecutive lanes write one unit
+        const long long U = o.words32 / 4;
+        const int q = threadIdx.x & 3, pos = (threadIdx.x >> 2) & 31, u2 = (threadIdx.x >> 7) & 1;
+        const int pp = p0 + pos;
+        const long long u = w0 / 4 + u2;
+        if (pp < o.P && u < U) {
+            const int c = pp / o.HW;
+            int yx = pp - c * o.HW;
+            if (o.side) yx = split_position(yx, o.side);
+            unsigned *dst = o.out + ((((long long)l0 * (o.P / o.HW) + c) * U + u) * o.HW + yx) * 4 + q;
+            const unsigned *srcw = sm + pos * 9 + u2 * 4 + q;
+            const long long dstep = (long long)(o.P / o.HW) * U * o.HW * 4;
+            for (int i = 0; i < nl; ++i) dst[i * dstep] = srcw[i * 32 * 9];
+        }
+    }
 }
 
-template <typename PIX>
-__global__ void __launch_bounds__(256) thermometer_pack_kernel(const PIX *__restrict__ pix, const float *__restrict__ thr, int L,
-                                                               unsigned *__restrict__ out, long long N, int P, int HW,
-                                                               long long words32, int to_slab, int side)
+// word |= bit where v > t: a comparison and a predicated OR (the compiler makes five instructions of the expression)
+__device__ __forceinline__ void set_if_above(unsigned &word, float v, float t, unsigned bit)
 {
-    __shared__ unsigned sm[kThermoLevels * 32 * 9];
-    __shared__ unsigned lut[256]; // uint8 pixels: level mask of every pixel value
+    asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %1, %2;\n\t@p or.b32 %0, %0, %3;\n\t}" : "+r"(word) : "f"(v), "f"(t), "r"(bit));
+}
+
+// Bound by the comparisons, two instructions per level and sample.
+template <int G>
+__global__ void __launch_bounds__(256) thermometer_pack_kernel(const float *__restrict__ pix, const float *__restrict__ thr, int L, long long N, ThermoOut o)
+{
+    constexpr int NL = 8 * G;
+    __shared__ unsigned sm[NL * 32 * 9];
     const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
     const int p = blockIdx.x * 32 + lane;
-    const long long n0 = (long long)blockIdx.y * 256;
-    for (int l0 = 0; l0 < L; l0 += kThermoLevels) {
-        const int nl = min(kThermoLevels, L - l0);
-        float th[kThermoLevels];
+    const long long n0 = (long long)blockIdx.y * 256, nb = n0 + wv * 32;
+    const int live = p < o.P ? (int)max(0LL, min(32LL, N - nb)) : 0;
+    for (int l0 = 0; l0 < L; l0 += NL) {
+        const int nl = min(NL, L - l0);
+        float th[NL];
+        unsigned word[NL];
 #pragma unroll
-        for (int i = 0; i < kThermoLevels; ++i) th[i] = i < nl ? __ldg(thr + l0 + i) : 0.f;
-        unsigned word[kThermoLevels];
-        if constexpr (sizeof(PIX) == 1) {
-            // uint8 pixels take 256 values: thread t builds the level mask of value t once per block (the same float
-            // expression as below, so the bits are the same), a sample is then one byte load and one table look-up,
-            // and a 32x32 bit transpose in registers turns the 32 samples' level masks into the 32 levels' sample words.
-            __syncthreads(); // the previous pass no longer reads the table
-            {
-                const float v = __fdiv_rn((float)threadIdx.x, 255.0f);
-                unsigned m = 0u;
+        for (int i = 0; i < NL; ++i) th[i] = i < nl ? __ldg(thr + l0 + i) : 0.f, word[i] = 0u;
+        const float *src = pix + nb * o.P + p;
 #pragma unroll
-                for (int i = 0; i < kThermoLevels; ++i) m |= ((i < nl && v > th[i]) ? 1u : 0u) << i;
-                lut[threadIdx.x] = m;
-            }
-            __syncthreads();
-            {
-                const long long nb = n0 + wv * 32;                  // first of the warp's 32 samples
-                const int live = p < P ? (int)min((long long)32, N - nb) : 0; // how many of them exist (<= 0: none)
-                const uint8_t *src = reinterpret_cast<const uint8_t *>(pix) + nb * P + p;
+        for (int j0 = 0; j0 < 32; j0 += 16) { // sixteen samples in flight
+            float v[16];
 #pragma unroll
-                for (int j = 0; j < 32; ++j) word[j] = j < live ? lut[__ldg(src + (long long)j * P)] : 0u;
-            }
-            unsigned m = 0x0000FFFFu;
+            for (int j = 0; j < 16; ++j) v[j] = j0 + j < live ? __ldg(src + (long long)(j0 + j) * o.P) : __int_as_float(0x7fc00000); // a NaN is above nothing
 #pragma unroll
-            for (int j = 16; j != 0; j >>= 1) {
+            for (int j = 0; j < 16; ++j)
 #pragma unroll
-                for (int k = 0; k < 32; k = (k + j + 1) & ~j) {
-                    const unsigned t = ((word[k] >> j) ^ word[k + j]) & m;
-                    word[k + j] ^= t;
-                    word[k] ^= t << j;
-                }
-                m ^= m << (j >> 1);
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < kThermoLevels; ++i) word[i] = 0u;
-#pragma unroll 4
-            for (int j = 0; j < 32; ++j) {
-                const long long n = n0 + wv * 32 + j;
-                if (n < N && p < P) {
-                    const float v = pixel_value<PIX>(pix + n * P + p);
-#pragma unroll
-                    for (int i = 0; i < kThermoLevels; ++i) word[i] |= (v > th[i] ? 1u : 0u) << j;
-                }
-            }
+                for (int i = 0; i < NL; ++i) set_if_above(word[i], v[j], th[i], 1u << (j0 + j));
         }
         __syncthreads(); // the previous pass has been written out
 #pragma unroll
-        for (int i = 0; i < kThermoLevels; ++i) sm[(i * 32 + lane) * 9 + wv] = word[i];
+        for (int i = 0; i < NL; ++i) sm[(i * 32 + lane) * 9 + wv] = word[i];
         __syncthreads();
-        const long long w0 = n0 / 32; // first 32-bit word of this block in a row
-        // Write-out: element e = thread + 256 * level, so a thread's (position, word) never changes and only the level
-        // walks: one shared load, one store and two additions per level.
-        if (!to_slab) {
-            // (level, position, word): 8 consecutive lanes write the 32 bytes of one row
-            const int w = threadIdx.x & 7, pos = (threadIdx.x >> 3) & 31;
-            const int pp = blockIdx.x * 32 + pos;
-            if (pp < P && w0 + w < words32) {
-                unsigned *dst = out + ((long long)l0 * P + pp) * words32 + w0 + w;
-                const unsigned *srcw = sm + pos * 9 + w;
-                const long long dstep = (long long)P * words32;
-                for (int i = 0; i < nl; ++i) dst[i * dstep] = srcw[i * 32 * 9];
+        thermo_write(sm, o, l0, nl, blockIdx.x * 32, n0);
+    }
+}
+
+// uint8 pixels take 256 values: thread t builds the level mask of value t once per block (the float expression of the other kernel,
+// so the bits are the same), a sample is then one byte and one table look-up, and 8x8 bit transposes in registers turn the
+// masks of 32 samples into sample words, eight levels at a time.  The bytes come through a tile of 256 samples x 128 positions, read in
+// 16-byte pieces where the rows allow it: read position by position, a warp fetched 32 bytes from each of 32 rows at a time, and
+// 20000 images of 3 levels took 132 us, now 59.
+// CH: positions of a block / 32, fewer where the larger blocks would not fill the GPU twice.
+template <int G, int CH>
+__global__ void __launch_bounds__(256) thermometer_pack_bytes_kernel(const uint8_t *__restrict__ pix, const float *__restrict__ thr, int L, long long N, int vec, ThermoOut o)
+{
+    constexpr int NL = 8 * G;
+    using Mask = std::conditional_t<G == 1, uint8_t, std::conditional_t<G == 2, uint16_t, unsigned>>;
+    constexpr int W = 32 * CH;
+    __shared__ __align__(16) uint8_t tile[256 * W];
+    __shared__ Mask lut[256];
+    extern __shared__ unsigned sm[]; // [NL][32][9]
+    const int tid = threadIdx.x, lane = tid & 31, wv = tid >> 5;
+    const int p0 = blockIdx.x * W;
+    const long long n0 = (long long)blockIdx.y * 256;
+    if (vec) {
+#pragma unroll
+        for (int i = 0; i < 2 * CH; ++i) {
+            const int u = tid + 256 * i, row = u / (2 * CH), q = u % (2 * CH) * 16;
+            uint4 v = make_uint4(0u, 0u, 0u, 0u);
+            if (n0 + row < N && p0 + q < o.P) v = __ldg(reinterpret_cast<const uint4 *>(pix + (n0 + row) * o.P + p0 + q));
+            *reinterpret_cast<uint4 *>(tile + row * W + q) = v;
+        }
+    } else {
+        for (int i = tid; i < 256 * W; i += 256) {
+            const int row = i / W, q = i % W;
+            tile[i] = n0 + row < N && p0 + q < o.P ? __ldg(pix + (n0 + row) * o.P + p0 + q) : 0;
+        }
+    }
+    const int live = (int)max(0LL, min(32LL, N - (n0 + wv * 32)));
+    for (int l0 = 0; l0 < L; l0 += NL) {
+        const int nl = min(NL, L - l0);
+        __syncthreads(); // the previous pass no longer reads the table
+        {
+            const float v = __fdiv_rn((float)tid, 255.0f);
+            unsigned m = 0u;
+#pragma unroll
+            for (int i = 0; i < NL; ++i) m |= ((i < nl && v > __ldg(thr + l0 + min(i, nl - 1))) ? 1u : 0u) << i;
+            lut[tid] = (Mask)m;
+        }
+        __syncthreads();
+#pragma unroll 1
+        for (int chunk = 0; chunk < CH && p0 + chunk * 32 < o.P; ++chunk) {
+            unsigned m[32];
+            const uint8_t *src = tile + wv * 32 * W + chunk * 32 + lane;
+#pragma unroll
+            for (int j = 0; j < 32; ++j) m[j] = j < live ? (unsigned)lut[src[j * W]] : 0u;
+            if (chunk) __syncthreads(); // the previous chunk has been written out
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                unsigned w[8]; // byte b of w[q]: sample 8 b + q
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const unsigned lo = __byte_perm(m[q], m[8 + q], 0x0040 + 0x0011 * g), hi = __byte_perm(m[16 + q], m[24 + q], 0x0040 + 0x0011 * g);
+                    w[q] = __byte_perm(lo, hi, 0x5410);
+                }
+#pragma unroll
+                for (int s = 4; s >= 1; s >>= 1) {
+                    const unsigned keep = s == 4 ? 0x0f0f0f0fu : s == 2 ? 0x33333333u : 0x55555555u;
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (!(q & s)) {
+                            const unsigned t = ((w[q] >> s) ^ w[q + s]) & keep;
+                            w[q + s] ^= t, w[q] ^= t << s;
+                        }
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) sm[((8 * g + i) * 32 + lane) * 9 + wv] = w[i];
             }
-        } else {
-            // slab layout [feature channel][U][HW] of 16-byte units: 4 consecutive lanes write one unit
-            const long long U = words32 / 4;
-            const int q = threadIdx.x & 3, pos = (threadIdx.x >> 2) & 31, u2 = (threadIdx.x >> 7) & 1;
-            const int pp = blockIdx.x * 32 + pos;
-            const long long u = w0 / 4 + u2;
-            if (pp < P && u < U) {
-                const int c = pp / HW;
-                int yx = pp - c * HW;
-                if (side) yx = split_position(yx, side);
-                unsigned *dst = out + ((((long long)l0 * (P / HW) + c) * U + u) * HW + yx) * 4 + q;
-                const unsigned *srcw = sm + pos * 9 + u2 * 4 + q;
-                const long long dstep = (long long)(P / HW) * U * HW * 4;
-                for (int i = 0; i < nl; ++i) dst[i * dstep] = srcw[i * 32 * 9];
-            }
+            __syncthreads();
+            thermo_write(sm, o, l0, nl, p0 + chunk * 32, n0);
         }
     }
 }
@@ -993,13 +1041,34 @@ int clb_thermometer_pack_units(const void *pixels, int pixels_u8, const float *t
     if (!aligned_to(packed, 16)) return CLB_ERR_ARG;
     const long long gy = (words32 + 7) / 8; // a block writes 8 half-words of every row: all of them are written, bits beyond N as zeros
     if (gy > 65535) return CLB_ERR_SHAPE;
-    dim3 grid((unsigned)((P + 31) / 32), (unsigned)gy);
-    if (pixels_u8)
-        CLB_TRACED("thermometer_pack_kernel", st, thermometer_pack_kernel<uint8_t><<<grid, 256, 0, st>>>((const uint8_t *)pixels, thresholds, levels, (unsigned *)packed, N, (int)P,
-                                                                (int)HW, words32, to_slab, side));
+    const ThermoOut o{(unsigned *)packed, (int)P, (int)HW, words32, to_slab, side};
+    const int groups = levels > 24 ? 4 : (levels + 7) / 8;
+    auto go = [&](auto G) {
+        constexpr int g = decltype(G)::value;
+        if (pixels_u8) {
+            const int vec = P % 16 == 0 && aligned_to(pixels, 16), bytes = 8 * g * 32 * 9 * 4;
+            auto launch = [&](auto k, int width) {
+                if (ensure_dynamic_smem(k, bytes) != cudaSuccess) return;
+                CLB_TRACED("thermometer_pack_kernel", st,
+                           k<<<dim3((unsigned)((P + width - 1) / width), (unsigned)gy), 256, bytes, st>>>((const uint8_t *)pixels, thresholds, levels, N, vec, o));
+            };
+            if ((P + 127) / 128 * gy >= 2LL * sm_count())
+                launch(thermometer_pack_bytes_kernel<g, 4>, 128);
+            else
+                launch(thermometer_pack_bytes_kernel<g, 1>, 32);
+        } else {
+            CLB_TRACED("thermometer_pack_kernel", st,
+                       thermometer_pack_kernel<g><<<dim3((unsigned)((P + 31) / 32), (unsigned)gy), 256, 0, st>>>((const float *)pixels, thresholds, levels, N, o));
+        }
+    };
+    if (groups == 1)
+        go(std::integral_constant<int, 1>{});
+    else if (groups == 2)
+        go(std::integral_constant<int, 2>{});
+    else if (groups == 3)
+        go(std::integral_constant<int, 3>{});
     else
-        CLB_TRACED("thermometer_pack_kernel", st, thermometer_pack_kernel<float><<<grid, 256, 0, st>>>((const float *)pixels, thresholds, levels, (unsigned *)packed, N, (int)P, (int)HW,
-                                                              words32, to_slab, side));
+        go(std::integral_constant<int, 4>{});
     return check_launch();
 }
 
