@@ -69,6 +69,7 @@ template <typename T> __device__ __forceinline__ Gate<T> gate_from_lane(const Ga
 
 template <typename T, int V> struct Vec;
 template <> struct Vec<float, 4> { using type = float4; };
+template <> struct Vec<float, 2> { using type = float2; };
 template <> struct Vec<float, 1> { using type = float; };
 template <> struct Vec<double, 1> { using type = double; };
 template <> struct Vec<double, 2> { using type = double2; };

@@ -20,7 +20,9 @@
 namespace clb {
 
 // ---------------------------------------------------------------------------------------- forward
-template <typename T, int V>
+// V: elements per access, by the alignment that a row of B elements has; R: accesses of a row in flight per lane, more where they
+// are narrow (349 samples, one by one: 196140 neurons in 155 us with one in flight).
+template <typename T, int V, int R>
 __global__ void __launch_bounds__(256) logic_fwd_kernel(const T *__restrict__ x, const int64_t *__restrict__ ia,
                                                         const int64_t *__restrict__ ib, const T *__restrict__ w, T *__restrict__ y,
                                                         T *__restrict__ coef /* [out][4] for the backward pass, or null */, long long out_dim,
@@ -43,20 +45,26 @@ __global__ void __launch_bounds__(256) logic_fwd_kernel(const T *__restrict__ x,
             const Gate<T> g = gate_from_lane<T>(gh, h * 16);
             const T *xa = x + ia[j] * B, *xb = x + ib[j] * B;
             T *yo = y + j * B;
-            for (long long b0 = (long long)lane * V; b0 < B; b0 += 32 * V) {
-                T a[V], b[V], r[V];
-                vload<T, V>(xa + b0, a);
-                vload<T, V>(xb + b0, b);
+            for (long long b0 = (long long)lane * V; b0 < B; b0 += 32 * V * R) {
+                T a[R][V], b[R][V];
 #pragma unroll
-                for (int k = 0; k < V; ++k) r[k] = gate_eval<T>(g, a[k], b[k]);
-                vstore<T, V>(yo + b0, r);
+                for (int i = 0; i < R; ++i)
+                    if (b0 + 32 * V * i < B) vload<T, V>(xa + b0 + 32 * V * i, a[i]), vload<T, V>(xb + b0 + 32 * V * i, b[i]);
+#pragma unroll
+                for (int i = 0; i < R; ++i)
+                    if (b0 + 32 * V * i < B) {
+                        T r[V];
+#pragma unroll
+                        for (int k = 0; k < V; ++k) r[k] = gate_eval<T>(g, a[i][k], b[i][k]);
+                        vstore<T, V>(yo + b0 + 32 * V * i, r);
+                    }
             }
         }
     }
 }
 
 // ------------------------------------------------------------------------------------ gate grads
-template <typename T, int V>
+template <typename T, int V, int R>
 __global__ void __launch_bounds__(256) logic_bwd_w_kernel(const T *__restrict__ x, const int64_t *__restrict__ ia,
                                                           const int64_t *__restrict__ ib, const T *__restrict__ w,
                                                           const T *__restrict__ gy, T *__restrict__ gw, long long out_dim, long long B,
@@ -73,18 +81,25 @@ __global__ void __launch_bounds__(256) logic_bwd_w_kernel(const T *__restrict__ 
             T acc[4] = {T(0), T(0), T(0), T(0)};
             if (j < out_dim) {
                 const T *xa = x + ia[j] * B, *xb = x + ib[j] * B, *g = gy + j * B;
-                for (long long b0 = (long long)lane * V; b0 < B; b0 += 32 * V) {
-                    T a[V], b[V], d[V];
-                    vload<T, V>(xa + b0, a);
-                    vload<T, V>(xb + b0, b);
-                    vload<T, V>(g + b0, d);
+                for (long long b0 = (long long)lane * V; b0 < B; b0 += 32 * V * R) {
+                    T a[R][V], b[R][V], d[R][V];
 #pragma unroll
-                    for (int k = 0; k < V; ++k) {
-                        acc[0] = fma_t<T>(d[k], a[k] * b[k], acc[0]);
-                        acc[1] = fma_t<T>(d[k], a[k], acc[1]);
-                        acc[2] = fma_t<T>(d[k], b[k], acc[2]);
-                        acc[3] += d[k];
-                    }
+                    for (int i = 0; i < R; ++i)
+                        if (b0 + 32 * V * i < B) {
+                            vload<T, V>(xa + b0 + 32 * V * i, a[i]);
+                            vload<T, V>(xb + b0 + 32 * V * i, b[i]);
+                            vload<T, V>(g + b0 + 32 * V * i, d[i]);
+                        }
+#pragma unroll
+                    for (int i = 0; i < R; ++i)
+                        if (b0 + 32 * V * i < B)
+#pragma unroll
+                            for (int k = 0; k < V; ++k) {
+                                acc[0] = fma_t<T>(d[i][k], a[i][k] * b[i][k], acc[0]);
+                                acc[1] = fma_t<T>(d[i][k], a[i][k], acc[1]);
+                                acc[2] = fma_t<T>(d[i][k], b[i][k], acc[2]);
+                                acc[3] += d[i][k];
+                            }
                 }
             }
 #pragma unroll
@@ -793,6 +808,7 @@ __global__ void __launch_bounds__(256) row_segment_sum_kernel(const float *__res
 using namespace clb;
 using namespace clb_host;
 
+static bool aligned8(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; }
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 static int logic_grid(long long units_of_warps)
@@ -827,13 +843,16 @@ extern "C" int clb_logic_fwd_coef(const void *x, const int64_t *a, const int64_t
             return clb_logic_fwd_cols((const float *)x, a, b, (const float *)w, (float *)y, (float *)coef, out_dim, B, wmode, st);
         if (vec)
             CLB_TRACED("logic_fwd_kernel", st,
-                       logic_fwd_kernel<float, 4><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (float *)y, (float *)coef, out_dim, B, wmode));
+                       logic_fwd_kernel<float, 4, 1><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (float *)y, (float *)coef, out_dim, B, wmode));
+        else if (B % 2 == 0 && aligned8(x) && aligned8(y))
+            CLB_TRACED("logic_fwd_kernel", st,
+                       logic_fwd_kernel<float, 2, 2><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (float *)y, (float *)coef, out_dim, B, wmode));
         else
             CLB_TRACED("logic_fwd_kernel", st,
-                       logic_fwd_kernel<float, 1><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (float *)y, (float *)coef, out_dim, B, wmode));
+                       logic_fwd_kernel<float, 1, 4><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (float *)y, (float *)coef, out_dim, B, wmode));
     } else if (dtype == CLB_F64) {
         CLB_TRACED("logic_fwd_kernel", st,
-                   logic_fwd_kernel<double, 1><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (double *)y, (double *)coef, out_dim, B, wmode));
+                   logic_fwd_kernel<double, 1, 1><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (double *)y, (double *)coef, out_dim, B, wmode));
     } else
         return CLB_ERR_ARG;
     return check_launch();
@@ -848,11 +867,13 @@ extern "C" int clb_logic_bwd_w(const void *x, const int64_t *a, const int64_t *b
     const int grid = logic_grid((out_dim + 1) / 2);
     if (dtype == CLB_F32) {
         if (B % 4 == 0 && aligned16(x) && aligned16(gy))
-            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 4><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
+            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 4, 1><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
+        else if (B % 2 == 0 && aligned8(x) && aligned8(gy))
+            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 2, 2><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
         else
-            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 1><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
+            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 1, 4><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
     } else if (dtype == CLB_F64) {
-        CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<double, 1><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (const double *)gy, (double *)gw, out_dim, B, wmode));
+        CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<double, 1, 1><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (const double *)gy, (double *)gw, out_dim, B, wmode));
     } else
         return CLB_ERR_ARG;
     return check_launch();

@@ -138,6 +138,9 @@ template <int LPR, int V, int R> struct Row {
                 if (r * LPR * 4 < left) q = __ldg(reinterpret_cast<const ulonglong2 *>(row + r * LPR * 4));
                 p[2 * r] = q.x, p[2 * r + 1] = q.y;
             }
+        } else if constexpr (V == 2) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) p[r] = r * LPR * 2 < left ? __ldg(reinterpret_cast<const f32x2 *>(row + r * LPR * 2)) : 0ull;
         } else {
             float t[R];
 #pragma unroll
@@ -152,6 +155,10 @@ template <int LPR, int V, int R> struct Row {
 #pragma unroll
             for (int r = 0; r < R; ++r)
                 if (r * LPR * 4 < left) __stcs(reinterpret_cast<float4 *>(row + r * LPR * 4), *reinterpret_cast<const float4 *>(&p[2 * r]));
+        } else if constexpr (V == 2) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (r * LPR * 2 < left) __stcs(reinterpret_cast<float2 *>(row + r * LPR * 2), *reinterpret_cast<const float2 *>(&p[r]));
         } else {
 #pragma unroll
             for (int r = 0; r < R; ++r)
@@ -312,6 +319,7 @@ extern "C" int clb_logic_bwd(const float *x, const float *w, const float *coef, 
     cudaStream_t st = (cudaStream_t)stream;
     const BwdCut cut = bwd_cut(in_dim, out_dim, B);
     if (cut.cols > 65535) return CLB_ERR_SHAPE;
+    const bool pairs = B % 2 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(gy) | reinterpret_cast<uintptr_t>(gx)) & 7) == 0;
     auto go = [&](auto kern, int lanes) {
         long long blocks = (in_dim * cut.cols * lanes + 255) / 256;
         const long long wave = (long long)sm_count() * 3; // resident at once; a second wave would walk all stretches again
@@ -323,8 +331,12 @@ extern "C" int clb_logic_bwd(const float *x, const float *w, const float *coef, 
         gw ? go(logic_bwd_kernel<8, 4, 2, 2, true>, 8) : go(logic_bwd_kernel<8, 4, 2, 2, false>, 8);
     else if (vec)
         gw ? go(logic_bwd_kernel<8, 4, 1, 4, true>, 8) : go(logic_bwd_kernel<8, 4, 1, 4, false>, 8);
+    else if (pairs && cut.wide)
+        gw ? go(logic_bwd_kernel<8, 2, 4, 2, true>, 8) : go(logic_bwd_kernel<8, 2, 4, 2, false>, 8);
+    else if (pairs)
+        gw ? go(logic_bwd_kernel<8, 2, 2, 4, true>, 8) : go(logic_bwd_kernel<8, 2, 2, 4, false>, 8);
     else if (cut.wide)
-        gw ? go(logic_bwd_kernel<16, 1, 4, 2, true>, 16) : go(logic_bwd_kernel<16, 1, 4, 2, false>, 16);
+        gw ? go(logic_bwd_kernel<8, 1, 8, 2, true>, 8) : go(logic_bwd_kernel<8, 1, 8, 2, false>, 8);
     else
         gw ? go(logic_bwd_kernel<8, 1, 4, 4, true>, 8) : go(logic_bwd_kernel<8, 1, 4, 4, false>, 8);
     if (!gw || out_dim == 0) return check_launch(1);

@@ -347,6 +347,14 @@ __global__ void __launch_bounds__(256) packed_logic_kernel(const V *__restrict__
     }
 }
 
+// bytes 4 w .. 4 w + 3 from p on, of which `valid` (more than 4: all) belong to the row: only words that hold one of those are read
+__device__ __forceinline__ unsigned word_at(const uint8_t *p, long long w, long long valid = 4)
+{
+    const unsigned *q = reinterpret_cast<const unsigned *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3) + w;
+    const unsigned at = (unsigned)(reinterpret_cast<uintptr_t>(p) & 3), lo = __ldg(q);
+    return at ? __funnelshift_r(lo, at + min(4LL, valid) > 4 ? __ldg(q + 1) : 0u, 8 * at) : lo;
+}
+
 // Rows whose length is no multiple of four bytes, so that a neuron's two input rows and its output row start anywhere: the
 // output is written in aligned 32-bit words, each input word put together from the two aligned words it straddles; up to three
 // bytes at either end of a row go one by one.  The same split as above.
@@ -361,11 +369,6 @@ __global__ void __launch_bounds__(256) packed_logic_bytes_kernel(const uint8_t *
         uint8_t *yo = y + j * rowbytes;
         const OpMasks<unsigned> m = op_masks<unsigned>(__ldg(ops + j));
         const int head = min(rowbytes, (int)(-reinterpret_cast<uintptr_t>(yo) & 3)), words = (rowbytes - head) >> 2, tail = rowbytes - head - 4 * words;
-        auto word_at = [](const uint8_t *p, int w) { // bytes 4w..4w+3 from p on
-            const unsigned *q = reinterpret_cast<const unsigned *>(reinterpret_cast<uintptr_t>(p) & ~(uintptr_t)3) + w;
-            const unsigned sh = 8 * (unsigned)(reinterpret_cast<uintptr_t>(p) & 3), lo = __ldg(q);
-            return sh ? __funnelshift_r(lo, __ldg(q + 1), sh) : lo; // the second word holds bytes of the row whenever it is read
-        };
         for (int w0 = l; w0 < words; w0 += 4 * g) {
             unsigned va[4], vb[4];
 #pragma unroll
@@ -445,14 +448,16 @@ __device__ __forceinline__ void csa(unsigned &hi, unsigned &lo, unsigned a, unsi
     lo = u ^ c;
 }
 
-// PLANES bit planes above the sixteens: a warp can count 16 * 2^PLANES rows, and so can the sum of the eight warps
-template <int PLANES>
-__global__ void __launch_bounds__(256, 3) group_popcount_kernel(const unsigned *__restrict__ x, int *__restrict__ counts, long long S, long long units, long long B,
+// PLANES bit planes above the sixteens: a warp can count 16 * 2^PLANES rows, and so can the sum of the eight warps.
+// ANY: rows of any number of bytes, whose words are put together from the two aligned ones that they straddle.
+template <int PLANES, bool ANY>
+__global__ void __launch_bounds__(256, 3) group_popcount_kernel(const uint8_t *__restrict__ xb, int *__restrict__ counts, long long S, long long rowbytes, long long B,
                                                              int k)
 {
     constexpr int P = PLANES + 4;
     __shared__ unsigned sm[4][P][32];
     const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
+    const long long units = ANY ? (rowbytes + 3) / 4 : rowbytes / 4;
     const long long u = (long long)blockIdx.x * 32 + lane;
     const int cls = blockIdx.z, parts = gridDim.y, sp = blockIdx.y * 8 + wv;
     const long long r_lo = S * sp / (8LL * parts), r_hi = S * (sp + 1) / (8LL * parts);
@@ -460,15 +465,24 @@ __global__ void __launch_bounds__(256, 3) group_popcount_kernel(const unsigned *
 #pragma unroll
     for (int p = 0; p < P; ++p) n[p] = 0;
     if (u < units) {
-        const unsigned *pr = x + ((long long)cls * S + r_lo) * units + u; // walks down the rows: one addition per load, no multiplication
+        const uint8_t *row = xb + ((long long)cls * S + r_lo) * rowbytes; // walks down the rows: one addition per load, no multiplication
+        const unsigned *pr = ANY ? nullptr : reinterpret_cast<const unsigned *>(row) + u;
         unsigned next[16]; // sixteen rows ahead
+        auto one = [&] {
+            unsigned v;
+            if constexpr (ANY)
+                v = word_at(row, u, rowbytes - 4 * u), row += rowbytes;
+            else
+                v = __ldg(pr), pr += units;
+            return v;
+        };
         auto load = [&](long long r) {
             if (r + 16 <= r_hi) {
 #pragma unroll
-                for (int q = 0; q < 16; ++q) next[q] = __ldg(pr), pr += units;
+                for (int q = 0; q < 16; ++q) next[q] = one();
             } else {
 #pragma unroll
-                for (int q = 0; q < 16; ++q) next[q] = (r + q < r_hi) ? __ldg(pr + q * units) : 0u;
+                for (int q = 0; q < 16; ++q) next[q] = r + q < r_hi ? one() : 0u;
             }
         };
         load(r_lo);
@@ -536,21 +550,6 @@ __global__ void __launch_bounds__(256, 3) group_popcount_kernel(const unsigned *
             counts[s * k + cls] = c;
         else if (c)
             atomicAdd(counts + s * k + cls, c);
-    }
-}
-
-// byte-unit fallback for rows whose length is not a multiple of 4 bytes: thread <-> (sample, class)
-__global__ void group_popcount_bytes_kernel(const uint8_t *__restrict__ x, int *__restrict__ counts, long long S, long long rowbytes,
-                                            long long B, int k)
-{
-    const long long total = B * k;
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const long long s = i / k;
-        const int cls = (int)(i % k);
-        const uint8_t *base = x + (long long)cls * S * rowbytes + (s >> 3);
-        int c = 0;
-        for (long long r = 0; r < S; ++r) c += (base[r * rowbytes] >> (s & 7)) & 1;
-        counts[i] = c;
     }
 }
 
@@ -1165,30 +1164,30 @@ static int group_popcount(const void *x, int32_t *counts, int64_t F, long long r
 {
     if (B <= 0) return CLB_OK;
     const long long S = F / k;
-    if (rowbytes % 4 == 0 && aligned_to(x, 4)) {
-        const long long units = rowbytes / 4, ublocks = (units + 31) / 32;
-        // parts of a class: three blocks per SM in all, at least 16 rows per warp.  All of them run at once (a second, short wave
-        // cost 30 of 150 us for 335 MB), and no more parts than that, as each adds its counts with atomics.
-        long long parts = 3LL * sm_count() / (ublocks * k);
-        if (parts > S / 128) parts = S / 128;
-        if (parts < 1) parts = 1;
-        if (ublocks > 0x7fffffffLL || k > 65535) return CLB_ERR_SHAPE;
-        if (parts > 1 && cudaMemsetAsync(counts, 0, (size_t)B * k * sizeof(int32_t), st) != cudaSuccess) return check_launch(0);
-        const dim3 grid((unsigned)ublocks, (unsigned)parts, (unsigned)k);
-        const long long rows = S / parts + 1; // of a block: what its counters have to hold
-        auto go = [&](auto planes) {
-            CLB_TRACED("group_popcount_kernel", st,
-                       group_popcount_kernel<decltype(planes)::value><<<grid, 256, 0, st>>>((const unsigned *)x, counts, S, units, B, k));
-        };
-        if (rows < (1LL << 14))
-            go(std::integral_constant<int, 10>{});
-        else if (rows < (1LL << 20))
-            go(std::integral_constant<int, 16>{});
-        else
-            go(std::integral_constant<int, 27>{});
-    } else {
-        CLB_TRACED("group_popcount_bytes_kernel", st, group_popcount_bytes_kernel<<<flat_grid(B * k, 256), 256, 0, st>>>((const uint8_t *)x, counts, S, rowbytes, B, k));
-    }
+    const bool any = rowbytes % 4 != 0 || !aligned_to(x, 4);
+    const long long ublocks = (rowbytes + 127) / 128;
+    // parts of a class: three blocks per SM in all, at least 16 rows per warp.  All of them run at once (a second, short wave
+    // cost 30 of 150 us for 335 MB), and no more parts than that, as each adds its counts with atomics.
+    long long parts = 3LL * sm_count() / (ublocks * k);
+    if (parts > S / 128) parts = S / 128;
+    if (parts < 1) parts = 1;
+    if (ublocks > 0x7fffffffLL || k > 65535) return CLB_ERR_SHAPE;
+    if (parts > 1 && cudaMemsetAsync(counts, 0, (size_t)B * k * sizeof(int32_t), st) != cudaSuccess) return check_launch(0);
+    const dim3 grid((unsigned)ublocks, (unsigned)parts, (unsigned)k);
+    const long long rows = S / parts + 1; // of a block: what its counters have to hold
+    auto launch = [&](auto kernel) {
+        CLB_TRACED("group_popcount_kernel", st, kernel<<<grid, 256, 0, st>>>((const uint8_t *)x, counts, S, rowbytes, B, k));
+    };
+    auto go = [&](auto planes) {
+        constexpr int P = decltype(planes)::value;
+        any ? launch(group_popcount_kernel<P, true>) : launch(group_popcount_kernel<P, false>);
+    };
+    if (rows < (1LL << 14))
+        go(std::integral_constant<int, 10>{});
+    else if (rows < (1LL << 20))
+        go(std::integral_constant<int, 16>{});
+    else
+        go(std::integral_constant<int, 27>{});
     return check_launch();
 }
 

@@ -1,0 +1,42 @@
+"""Flat layers on rows whose length leaves them 16-, 8- or 4-byte aligned, around the accesses that a lane has in flight, against a
+double-precision restatement (outputs and both gradients, fp32)."""
+
+import pytest
+import torch
+
+from tests.util import assert_close
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("batch", [1, 2, 31, 62, 63, 65, 66, 127, 128, 129, 130, 257, 258])
+@pytest.mark.parametrize("in_dim,out_dim", [(40, 70), (3000, 5000)])
+def test_flat_layer_rows_of_any_alignment(batch, in_dim, out_dim):
+    import convlogic_b200 as cb
+
+    torch.manual_seed(batch)
+    first, layer = cb.LogicLayer(in_dim, out_dim).cuda(), cb.LogicLayer(out_dim, out_dim).cuda()
+    x = torch.rand(batch, in_dim, device="cuda", requires_grad=True)
+    gy = torch.randn(batch, out_dim, device="cuda")
+    y = layer(first(x))
+    gx, g1, g2 = torch.autograd.grad(y, (x, first.weights, layer.weights), gy)
+    xo = x.detach().double().cpu().requires_grad_(True)
+    h, ws = xo, []
+    for m in (first, layer):
+        w = m.weights.detach().double().cpu().requires_grad_(True)
+        ws.append(w)
+        a, b = h[:, m.indices_0.cpu()], h[:, m.indices_1.cpu()]
+        h = sum(p * f for p, f in zip(torch.softmax(w, -1).unbind(-1), oracle_gates(a, b)))
+    gxo, g1o, g2o = torch.autograd.grad(h, (xo, *ws), gy.double().cpu())
+    assert_close(y, h, 1e-5, "y")
+    assert_close(gx, gxo, 1e-5, "gx")
+    assert_close(g1, g1o, 1e-5, "first gates")
+    assert_close(g2, g2o, 1e-5, "second gates")
+
+
+def oracle_gates(a, b):
+    """The sixteen gates as real-valued functions, in the order of their truth tables."""
+    one, ab = torch.ones_like(a), a * b
+    terms = [(0, 0, 0, 0), (0, 0, 0, 1), (0, 1, 0, -1), (0, 1, 0, 0), (0, 0, 1, -1), (0, 0, 1, 0), (0, 1, 1, -2), (0, 1, 1, -1)]
+    half = [k * one + p * a + q * b + r * ab for k, p, q, r in terms]
+    return half + [one - g for g in reversed(half)]

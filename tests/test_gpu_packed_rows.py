@@ -51,3 +51,13 @@ def test_class_counts_over_many_rows(rows_per_class):
     want = torch.stack([(x.view(3, rows_per_class, 33).long() >> s) & 1 for s in range(32)], -1).sum(1)   # [3, 33, 32]
     got = _lib.native().group_popcount(x, 5, 3)
     assert torch.equal(got.long(), want.reshape(3, -1).t()[: 33 * 32 - 5])
+
+
+@pytest.mark.parametrize("rows_per_class,row_bytes", [(1, 1), (15, 3), (127, 62), (128, 131), (2600, 257)])
+def test_class_counts_over_rows_of_any_bytes(rows_per_class, row_bytes):
+    from convlogic_b200 import _lib
+
+    x = torch.randint(0, 256, (3 * rows_per_class, row_bytes), device="cuda", dtype=torch.uint8)
+    want = torch.stack([(x.view(3, rows_per_class, row_bytes).long() >> s) & 1 for s in range(8)], -1).sum(1)   # [3, row_bytes, 8]
+    got = _lib.native().group_popcount(x, 3, 3)
+    assert torch.equal(got.long(), want.reshape(3, -1).t()[: 8 * row_bytes - 3])
