@@ -9,11 +9,9 @@ namespace clb {
 // `j` (the same j in all 16 lanes of a half-warp; the two halves may name unrelated neurons).
 // Returns that neuron's gate in every lane of the half-warp, plus the lane's mixture value p.
 // Neurons outside [0, out_dim) give zeros.
-template <typename T>
-__device__ __forceinline__ Gate<T> half_warp_gate(const T *__restrict__ w, long long j, long long out_dim, int wmode, int lane, T &p)
+template <typename T> __device__ __forceinline__ Gate<T> half_warp_gate_of(T v, int wmode, int lane, T &p) // v: the lane's value
 {
     const int i = lane & 15;
-    T v = (j >= 0 && j < out_dim) ? w[j * 16 + i] : T(0);
     if (wmode == CLB_W_SOFTMAX) {
         T m = v;
 #pragma unroll
@@ -55,6 +53,12 @@ __device__ __forceinline__ Gate<T> half_warp_gate(const T *__restrict__ w, long 
         g.k1 += __shfl_xor_sync(0xffffffffu, g.k1, o);
     }
     return g;
+}
+
+template <typename T>
+__device__ __forceinline__ Gate<T> half_warp_gate(const T *__restrict__ w, long long j, long long out_dim, int wmode, int lane, T &p)
+{
+    return half_warp_gate_of<T>((j >= 0 && j < out_dim) ? w[j * 16 + (lane & 15)] : T(0), wmode, lane, p);
 }
 
 template <typename T> __device__ __forceinline__ Gate<T> gate_from_lane(const Gate<T> &g, int src)
