@@ -92,6 +92,8 @@ _SIGNATURES = {
     "clb_group_sum_bwd": ([_vp, _vp, _i64, _i64, _i, C.c_double, _i, _vp], _i),
     "clb_net_device_bytes": ([_vp, _sz, _vp], _i),
     "clb_net_create": ([_vp, _sz, _vp, _vp, _vp], _i),
+    "clb_net_record_bytes": ([_vp], _sz),
+    "clb_net_records": ([_vp, _vp, _vp], _i),
     "clb_net_destroy": ([_vp], None),
     "clb_net_info": ([_vp, _vp, _vp, _vp], _i),
     "clb_net_workspace_bytes": ([_vp, _i64], _sz),

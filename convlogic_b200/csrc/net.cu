@@ -54,8 +54,8 @@ struct Layer {
     long long in_dim, out_dim;
     int levels;
     size_t off_a, off_b, off_ops;
-    bool slab3 = false;   // a 3x3 block of the stacks' geometry: its tap records are laid out when the network is created
-    size_t off_recs = 0;  // behind the blob in the parameter memory
+    bool slab3 = false;   // a 3x3 block of the stacks' geometry, which works from tap records ...
+    size_t off_recs = 0;  // ... in the records memory, where the caller gave some
 };
 
 } // namespace
@@ -65,7 +65,9 @@ struct clb_net {
     int num_classes = 0;
     int in_channels = 0, in_h = 0, in_w = 0;
     long long in_features = 0; // features of one sample at the input
-    size_t param_bytes = 0;    // the blob, copied to the device as it is, and the tap records behind it
+    size_t param_bytes = 0;    // the blob is copied to the device as it is
+    size_t record_bytes = 0;   // tap records of all 3x3 blocks
+    const unsigned char *records = nullptr; // device memory that holds them, or null: laid out in the workspace on every call
     const unsigned char *dev = nullptr;
     size_t max_conv_channels = 0;
     clb::NetPlan plan = {};     // for the one-launch kernel
@@ -158,8 +160,8 @@ static bool parse(const void *blob, size_t bytes, clb_net &net)
             return false;
         }
         if (L.kind == 1 && clb_slab3_covers(L.H, L.W, L.stride, L.stride, L.ph, L.pw, L.kh, L.kw)) {
-            L.slab3 = true, L.off_recs = (net.param_bytes + 255) / 256 * 256;
-            net.param_bytes = L.off_recs + clb_slab3_record_bytes(L.C);
+            L.slab3 = true, L.off_recs = net.record_bytes;
+            net.record_bytes += (clb_slab3_record_bytes(L.C) + 255) / 256 * 256;
         }
         net.layers.push_back(L);
     }
@@ -247,17 +249,23 @@ extern "C" int clb_net_create(const void *blob, size_t bytes, void *device_mem, 
         return check_launch(0);
     }
     net->dev = (const unsigned char *)device_mem;
-    for (const Layer &L : net->layers) {
-        if (!L.slab3) continue;
-        const int rc = clb_slab3_records(net->dev + L.off_ops, (const int32_t *)(net->dev + L.off_a), (unsigned char *)device_mem + L.off_recs, L.Ci, L.H, L.C,
-                                         (cudaStream_t)stream);
-        if (rc != CLB_OK) {
-            delete net;
-            return rc;
-        }
-    }
     plan_one_launch(*net);
     *out = net;
+    return CLB_OK;
+}
+
+extern "C" size_t clb_net_record_bytes(const clb_net *net) { return net ? net->record_bytes : 0; }
+
+extern "C" int clb_net_records(clb_net *net, void *records, void *stream)
+{
+    if (!net || (net->record_bytes && (!records || (reinterpret_cast<uintptr_t>(records) & 15)))) return CLB_ERR_ARG;
+    for (const Layer &L : net->layers) {
+        if (!L.slab3) continue;
+        const int rc = clb_slab3_records(net->dev + L.off_ops, (const int32_t *)(net->dev + L.off_a), (unsigned char *)records + L.off_recs, L.Ci, L.H, L.C,
+                                         (cudaStream_t)stream);
+        if (rc != CLB_OK) return rc;
+    }
+    net->records = (const unsigned char *)records;
     return CLB_OK;
 }
 
@@ -358,7 +366,12 @@ extern "C" int clb_net_forward(const clb_net *net, int input_kind, const void *i
                 cur ^= 1, order = want;
             }
             if (L.slab3) { // takes either slab order and writes what the next layer reads
-                st = clb_slab3_block(buf[cur], P + L.off_recs, buf[cur ^ 1], L.Ci, L.H, L.C, U, order, next, cs);
+                const void *recs = net->records ? (const void *)(net->records + L.off_recs) : scratch;
+                if (!net->records) {
+                    st = clb_slab3_records(P + L.off_ops, (const int32_t *)(P + L.off_a), scratch, L.Ci, L.H, L.C, cs);
+                    if (st != CLB_OK) return st;
+                }
+                st = clb_slab3_block(buf[cur], recs, buf[cur ^ 1], L.Ci, L.H, L.C, U, order, next, cs);
                 order = next;
             } else if (order != clb::kRows) {
                 st = clb_packed_convtree_slab(buf[cur], P + L.off_ops, (const int32_t *)(P + L.off_a), buf[cur ^ 1], scratch, L.Ci, L.H, L.W,

@@ -948,6 +948,10 @@ public:
         c10::cuda::CUDAGuard guard(device_);
         params_ = at::empty({(int64_t)(need < 16 ? 16 : need)}, at::TensorOptions().dtype(at::kByte).device(device_));
         check(clb_net_create(data.data(), data.size(), ptr(params_), cur_stream(), &net_));
+        if (const size_t bytes = clb_net_record_bytes(net_)) {
+            records_ = at::empty({(int64_t)bytes}, params_.options());
+            check(clb_net_records(net_, ptr(records_), cur_stream()));
+        }
         c10::cuda::getCurrentCUDAStream().synchronize(); // the blob is pageable host memory: wait for the copy
         check(clb_net_info(net_, &features, &classes, &layers));
     }
@@ -984,7 +988,7 @@ public:
 
 private:
     c10::Device device_;
-    Tensor params_;
+    Tensor params_, records_;
     clb_net *net_ = nullptr;
 };
 

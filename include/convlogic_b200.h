@@ -411,6 +411,11 @@ int clb_adam_step(float *p, const float *g, float *m, float *v, int64_t n, doubl
 typedef struct clb_net clb_net;
 int clb_net_device_bytes(const void *blob, size_t bytes, size_t *device_bytes);
 int clb_net_create(const void *blob, size_t bytes, void *device_mem, void *stream, clb_net **net);
+/* Optional: lay the tap records of the 3x3 blocks out once, in caller-provided device memory (16-byte aligned, lives as long as the
+ * net, clb_net_record_bytes of it; 0: nothing to lay out), behind clb_net_create on the same stream.  Without it every
+ * clb_net_forward lays them out in its workspace. */
+size_t clb_net_record_bytes(const clb_net *net);
+int clb_net_records(clb_net *net, void *records, void *stream);
 void clb_net_destroy(clb_net *net);
 int clb_net_info(const clb_net *net, int64_t *in_features, int *num_classes, int *n_layers);
 size_t clb_net_workspace_bytes(const clb_net *net, int64_t batch);

@@ -41,3 +41,37 @@ def test_slab_blocks_equal_the_float_model(side, ci, slabs):
             assert torch.equal(got.long(), want)
     finally:
         _lib.check(_lib.lib().clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 1))
+
+
+def test_records_laid_out_on_every_call_equal_those_laid_out_once():
+    """A caller of the C functions who gives no records memory."""
+    import ctypes as C
+
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+    from convlogic_b200.compiled_model import serialise
+
+    torch.manual_seed(3)
+    net = cb.ConvLogicCifarModel(k_param=4, input_channels=6).network.cuda()
+    for p in net.parameters():
+        p.data.normal_()
+    x = torch.rand(300, 6, 32, 32, device="cuda") < 0.5
+    lib = _lib.lib()
+    _lib.check(lib.clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 0))
+    try:
+        want = cb.CompiledLogicNet(net.eval(), input_shape=(6, 32, 32)).compile()(x)
+        blob = serialise(net, input_shape=(6, 32, 32))
+        params, handle = torch.empty(len(blob), dtype=torch.uint8, device="cuda"), C.c_void_p()
+        stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        _lib.check(lib.clb_net_create(blob, len(blob), C.c_void_p(params.data_ptr()), stream, C.byref(handle)))
+        try:
+            ws = torch.empty(lib.clb_net_workspace_bytes(handle, 300), dtype=torch.uint8, device="cuda")
+            got = torch.empty_like(want)
+            _lib.check(lib.clb_net_forward(handle, 0, C.c_void_p(x.data_ptr()), None, 0, 300, C.c_void_p(got.data_ptr()), C.c_void_p(ws.data_ptr()),
+                                           ws.numel(), stream))
+            torch.cuda.synchronize()
+        finally:
+            lib.clb_net_destroy(handle)
+    finally:
+        _lib.check(lib.clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 1))
+    assert torch.equal(got, want)
