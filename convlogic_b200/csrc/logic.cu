@@ -23,7 +23,7 @@ namespace clb {
 // A half-warp per neuron.  V: elements per access, by the alignment that a row of B elements has; R: accesses of a row in flight per
 // lane.  What bounds a neuron is its chain of dependent loads: its first rows are under way while the soft-max of its 16 values is
 // taken, and the values and indices of the half-warp's next neuron are loaded a neuron ahead.  (A warp for two neurons in turn, rows
-// behind the soft-max: 109660 neurons x 6 layers, 112 samples 228 us; 519000 neurons, 20 samples 128.)
+// behind the soft-max: 109660 neurons x 6 layers, 112 samples 228 us, now 124; 519000 neurons, 20 samples 128, now 80.)
 template <typename T, int V, int R>
 __global__ void __launch_bounds__(256) logic_fwd_kernel(const T *__restrict__ x, const int64_t *__restrict__ ia,
                                                         const int64_t *__restrict__ ib, const T *__restrict__ w, T *__restrict__ y,
@@ -819,10 +819,11 @@ using namespace clb_host;
 static bool aligned8(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; }
 static bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-static int logic_grid(long long units_of_warps)
+// per: blocks of an SM at most.  The resident ones (4 at 64 registers) where a warp loads ahead for its next unit.
+static int logic_grid(long long units_of_warps, int per = 32)
 {
     long long blocks = (units_of_warps + 7) / 8; // 8 warps per block
-    const long long cap = (long long)sm_count() * 8 * 4;
+    const long long cap = (long long)sm_count() * per;
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     return (int)blocks;
@@ -843,7 +844,7 @@ extern "C" int clb_logic_fwd_coef(const void *x, const int64_t *a, const int64_t
     if (!x || !a || !b || !w || !y || in_dim <= 0 || out_dim < 0 || B < 0 || wmode < 0 || wmode > 2) return CLB_ERR_ARG;
     if (out_dim == 0 || B == 0) return CLB_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    const int grid = logic_grid((out_dim + 1) / 2);
+    const int grid = logic_grid((out_dim + 1) / 2, 4);
     if (dtype == CLB_F32) {
         const bool vec = B % 4 == 0 && aligned16(x) && aligned16(y);
         // an input beyond about half the L2 is walked in column stretches that fit it (0.44 -> 0.40 ms per 256000 x 1024 layer)
@@ -872,7 +873,7 @@ extern "C" int clb_logic_bwd_w(const void *x, const int64_t *a, const int64_t *b
     if (!x || !a || !b || !w || !gy || !gw || in_dim <= 0 || out_dim < 0 || B < 0 || wmode < 0 || wmode > 2) return CLB_ERR_ARG;
     if (out_dim == 0) return CLB_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    const int grid = logic_grid((out_dim + 1) / 2);
+    const int grid = logic_grid((out_dim + 1) / 2, 4);
     if (dtype == CLB_F32) {
         if (B % 4 == 0 && aligned16(x) && aligned16(gy))
             CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 4, 1><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
