@@ -72,63 +72,67 @@ __global__ void __launch_bounds__(256) logic_fwd_kernel(const T *__restrict__ x,
 }
 
 // ------------------------------------------------------------------------------------ gate grads
+// A half-warp per neuron, as in the forward pass and for its reason: the values and indices come a neuron ahead and the first rows
+// are under way while the soft-max is taken.  (A warp for two neurons in turn, first layer of 125090 neurons, 472 samples 114 us, now
+// 67; 109660 x 112 44, now 28; 256000 x 1024 269, now 228.  64 registers, so that four blocks are resident: at 74 and three 76, 29, 255.)
 template <typename T, int V, int R>
-__global__ void __launch_bounds__(256) logic_bwd_w_kernel(const T *__restrict__ x, const int64_t *__restrict__ ia,
-                                                          const int64_t *__restrict__ ib, const T *__restrict__ w,
-                                                          const T *__restrict__ gy, T *__restrict__ gw, long long out_dim, long long B,
-                                                          int wmode)
+__global__ void __launch_bounds__(256, 4) logic_bwd_w_kernel(const T *__restrict__ x, const int64_t *__restrict__ ia,
+                                                             const int64_t *__restrict__ ib, const T *__restrict__ w,
+                                                             const T *__restrict__ gy, T *__restrict__ gw, long long out_dim, long long B,
+                                                             int wmode)
 {
-    const int lane = threadIdx.x & 31;
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    for (long long j0 = warp * 2; j0 < out_dim; j0 += nwarps * 2) {
-        T s[2][4];
+    const int lane = threadIdx.x & 31, l = lane & 15;
+    const long long step = ((long long)gridDim.x * blockDim.x) >> 4;
+    long long j = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4, ja = 0, jb = 0;
+    T v = T(0);
+    auto fetch = [&](long long n) {
+        if (n < out_dim) v = w[n * 16 + l], ja = ia[n], jb = ib[n];
+    };
+    fetch(j);
+    for (; j - (lane >> 4) < out_dim; j += step) { // uniform over the warp
+        const bool mine = j < out_dim;
+        const T *xa = x + ja * B, *xb = x + jb * B, *g = gy + j * B;
+        T a[R][V], b[R][V], d[R][V], p = T(0);
+        auto load = [&](long long b0) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const long long j = j0 + h;
-            T acc[4] = {T(0), T(0), T(0), T(0)};
-            if (j < out_dim) {
-                const T *xa = x + ia[j] * B, *xb = x + ib[j] * B, *g = gy + j * B;
-                for (long long b0 = (long long)lane * V; b0 < B; b0 += 32 * V * R) {
-                    T a[R][V], b[R][V], d[R][V];
-#pragma unroll
-                    for (int i = 0; i < R; ++i)
-                        if (b0 + 32 * V * i < B) {
-                            vload<T, V>(xa + b0 + 32 * V * i, a[i]);
-                            vload<T, V>(xb + b0 + 32 * V * i, b[i]);
-                            vload<T, V>(g + b0 + 32 * V * i, d[i]);
-                        }
-#pragma unroll
-                    for (int i = 0; i < R; ++i)
-                        if (b0 + 32 * V * i < B)
-#pragma unroll
-                            for (int k = 0; k < V; ++k) {
-                                acc[0] = fma_t<T>(d[i][k], a[i][k] * b[i][k], acc[0]);
-                                acc[1] = fma_t<T>(d[i][k], a[i][k], acc[1]);
-                                acc[2] = fma_t<T>(d[i][k], b[i][k], acc[2]);
-                                acc[3] += d[i][k];
-                            }
+            for (int i = 0; i < R; ++i)
+                if (b0 + 16 * V * i < B) {
+                    vload<T, V>(g + b0 + 16 * V * i, d[i]);
+                    vload<T, V>(xa + b0 + 16 * V * i, a[i]);
+                    vload<T, V>(xb + b0 + 16 * V * i, b[i]);
                 }
+        };
+        if (mine) load(l * V);
+        const T mine_v = v;
+        fetch(j + step);
+        if (wmode == CLB_W_SOFTMAX) (void)half_warp_gate_of<T>(mine_v, CLB_W_SOFTMAX, lane, p);
+        T s[4] = {T(0), T(0), T(0), T(0)};
+        if (mine)
+            for (long long b0 = l * V; b0 < B; b0 += 16 * V * R) {
+                if (b0 != l * V) load(b0);
+#pragma unroll
+                for (int i = 0; i < R; ++i)
+                    if (b0 + 16 * V * i < B)
+#pragma unroll
+                        for (int k = 0; k < V; ++k) {
+                            s[0] = fma_t<T>(d[i][k], a[i][k] * b[i][k], s[0]);
+                            s[1] = fma_t<T>(d[i][k], a[i][k], s[1]);
+                            s[2] = fma_t<T>(d[i][k], b[i][k], s[2]);
+                            s[3] += d[i][k];
+                        }
             }
 #pragma unroll
-            for (int k = 0; k < 4; ++k) s[h][k] = warp_sum<T>(acc[k]);
-        }
-        // lane l writes gradient (l & 15) of neuron j0 + (l >> 4)
-        const int h = lane >> 4, i = lane & 15;
-        const long long j = j0 + h;
-        T sh4[4];
+        for (int k = 0; k < 4; ++k)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) sh4[k] = h ? s[1][k] : s[0][k];
-        T gi = T(kcoef(0, i)) * sh4[0] + T(kcoef(1, i)) * sh4[1] + T(kcoef(2, i)) * sh4[2] + T(kcoef(3, i)) * sh4[3];
+            for (int o = 8; o > 0; o >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], o);
+        T gi = T(kcoef(0, l)) * s[0] + T(kcoef(1, l)) * s[1] + T(kcoef(2, l)) * s[2] + T(kcoef(3, l)) * s[3];
         if (wmode == CLB_W_SOFTMAX) {
-            T p;
-            (void)half_warp_gate<T>(w, j, out_dim, CLB_W_SOFTMAX, lane, p);
             T dot = p * gi;
 #pragma unroll
             for (int o = 8; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
             gi = p * (gi - dot);
         }
-        if (j < out_dim) gw[j * 16 + i] = gi;
+        if (mine) gw[j * 16 + l] = gi;
     }
 }
 
@@ -876,13 +880,13 @@ extern "C" int clb_logic_bwd_w(const void *x, const int64_t *a, const int64_t *b
     const int grid = logic_grid((out_dim + 1) / 2, 4);
     if (dtype == CLB_F32) {
         if (B % 4 == 0 && aligned16(x) && aligned16(gy))
-            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 4, 1><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
+            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 4, 2><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
         else if (B % 2 == 0 && aligned8(x) && aligned8(gy))
-            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 2, 2><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
+            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 2, 4><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
         else
-            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 1, 4><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
+            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 1, 8><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
     } else if (dtype == CLB_F64) {
-        CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<double, 1, 1><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (const double *)gy, (double *)gw, out_dim, B, wmode));
+        CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<double, 1, 2><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (const double *)gy, (double *)gw, out_dim, B, wmode));
     } else
         return CLB_ERR_ARG;
     return check_launch();

@@ -34,6 +34,22 @@ def test_flat_layer_rows_of_any_alignment(batch, in_dim, out_dim):
     assert_close(g2, g2o, 1e-5, "second gates")
 
 
+@pytest.mark.parametrize("batch", [1, 14, 68, 131])
+@pytest.mark.parametrize("dtype,tol", [(torch.float32, 1e-5), (torch.float64, 1e-12)])
+def test_gate_gradient_of_more_neurons_than_half_warps(batch, dtype, tol):
+    """The first layer of a network (no input gradient); a half-warp takes two or three neurons in turn, the last ones none."""
+    import convlogic_b200 as cb
+
+    torch.manual_seed(batch)
+    layer = cb.LogicLayer(50, 21001).to("cuda", dtype)
+    x, gy = torch.rand(batch, 50, device="cuda", dtype=dtype), torch.randn(batch, 21001, device="cuda", dtype=dtype)
+    (gw,) = torch.autograd.grad(layer(x), layer.weights, gy)
+    w, xo = layer.weights.detach().double().cpu().requires_grad_(True), x.double().cpu()
+    gates = oracle_gates(xo[:, layer.indices_0.cpu()], xo[:, layer.indices_1.cpu()])
+    (gwo,) = torch.autograd.grad(sum(p * f for p, f in zip(torch.softmax(w, -1).unbind(-1), gates)), w, gy.double().cpu())
+    assert_close(gw, gwo, tol, "gates")
+
+
 def oracle_gates(a, b):
     """The sixteen gates as real-valued functions, in the order of their truth tables."""
     one, ab = torch.ones_like(a), a * b
