@@ -456,6 +456,36 @@ __global__ void __launch_bounds__(256) group_sum_bwd_kernel(const T *__restrict_
     }
 }
 
+// The same where rows of B floats are not whole 16-byte words: a chunk is one contiguous stretch of gy, written in aligned words of
+// four from the class's B quotients in shared memory, so that the L2 gets whole sectors.  Bound by the writes (one float per store: 125090 x 473 65 us,
+// now 40; 256000 x 1022 380, now 186: 86 % of the copy rate).  At most kGroupSumFlatMax quotients.
+constexpr int kGroupSumFlatMax = 4096;
+__global__ void __launch_bounds__(256) group_sum_bwd_flat_kernel(const float *__restrict__ gout, const float *__restrict__ scale, float *__restrict__ gy,
+                                                                 long long S, int B, int k, float tau)
+{
+    extern __shared__ float quot[];
+    const int c = blockIdx.y, tid = threadIdx.x;
+    if (scale != nullptr) tau = tau / scale[0];
+    for (int b = tid; b < B; b += 256) quot[b] = gout[(long long)b * k + c] / tau;
+    __syncthreads();
+    const long long r0 = S * blockIdx.x / gridDim.x, r1 = S * (blockIdx.x + 1) / gridDim.x;
+    const long long first = (c * S + r0) * B, n = (r1 - r0) * B;
+    const int lead = (int)min(n, (4 - (first & 3)) & 3);
+    const long long words = (n - lead) >> 2;
+    gy += first;
+    if (tid < lead) gy[tid] = quot[tid % B];
+    const int step = 1024 % B;
+    int b = (lead + 4 * tid) % B;
+    for (long long i = tid; i < words; i += 256) {
+        const int b1 = b + 1 < B ? b + 1 : 0, b2 = b1 + 1 < B ? b1 + 1 : 0, b3 = b2 + 1 < B ? b2 + 1 : 0;
+        reinterpret_cast<float4 *>(gy + lead)[i] = make_float4(quot[b], quot[b1], quot[b2], quot[b3]);
+        b += step;
+        if (b >= B) b -= B;
+    }
+    const long long done = lead + 4 * words;
+    if (tid < n - done) gy[done + tid] = quot[(done + tid) % B];
+}
+
 // ----------------------------------------------------------------------------------- fused flat layers (training)
 // Three consecutive flat layers whose outputs are each read at most once by the next one, as ONE differentiable
 // gate tree per neuron of the last layer: leaf [T][8] are rows of the first layer's input (gate p of the first
@@ -1046,6 +1076,8 @@ extern "C" int clb_group_sum_bwd_scaled(const void *gout, const void *scale, voi
     dim3 grid((unsigned)chunks, (unsigned)k);
     if (dtype == CLB_F32 && B % 4 == 0 && aligned16(gy))
         CLB_TRACED("group_sum_bwd_kernel", st, group_sum_bwd_kernel<float, 4><<<grid, 256, 0, st>>>((const float *)gout, (const float *)scale, (float *)gy, S, B, k, (float)tau));
+    else if (dtype == CLB_F32 && B <= kGroupSumFlatMax && aligned16(gy))
+        CLB_TRACED("group_sum_bwd_kernel", st, group_sum_bwd_flat_kernel<<<grid, 256, (size_t)B * 4, st>>>((const float *)gout, (const float *)scale, (float *)gy, S, (int)B, k, (float)tau));
     else if (dtype == CLB_F32)
         CLB_TRACED("group_sum_bwd_kernel", st, group_sum_bwd_kernel<float, 1><<<grid, 256, 0, st>>>((const float *)gout, (const float *)scale, (float *)gy, S, B, k, (float)tau));
     else

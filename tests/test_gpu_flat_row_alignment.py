@@ -50,6 +50,19 @@ def test_gate_gradient_of_more_neurons_than_half_warps(batch, dtype, tol):
     assert_close(gw, gwo, tol, "gates")
 
 
+@pytest.mark.parametrize("batch", [1, 2, 3, 5, 255, 1022, 1025, 4095, 4097])
+@pytest.mark.parametrize("per_class", [1, 3, 5003])
+def test_class_sum_gradient_rows_of_any_alignment(batch, per_class):
+    """Rows that are not whole 16-byte words: every chunk's first words, its last ones and the wrap from a row to the next."""
+    import convlogic_b200 as cb
+
+    k = 3
+    x = torch.zeros(k * per_class, batch, device="cuda").t().requires_grad_(True)
+    g = torch.randn(batch, k, device="cuda")
+    (gx,) = torch.autograd.grad(cb.GroupSum(k, tau=3.5)(x), x, g)
+    assert torch.equal(gx, (g / torch.tensor(3.5, device="cuda")).repeat_interleave(per_class, 1))
+
+
 def oracle_gates(a, b):
     """The sixteen gates as real-valued functions, in the order of their truth tables."""
     one, ab = torch.ones_like(a), a * b
