@@ -457,8 +457,8 @@ __global__ void __launch_bounds__(256) group_sum_bwd_kernel(const T *__restrict_
 }
 
 // The same where rows of B floats are not whole 16-byte words: a chunk is one contiguous stretch of gy, written in aligned words of
-// four from the class's B quotients in shared memory, so that the L2 gets whole sectors.  Bound by the writes (one float per store: 125090 x 473 65 us,
-// now 40; 256000 x 1022 380, now 186: 86 % of the copy rate).  At most kGroupSumFlatMax quotients.
+// four from the class's B quotients in shared memory, so that the L2 gets whole sectors.  Bound by the writes (a float per store:
+// 125090 x 473 65 us, now 40; 256000 x 1022 380, now 186: 86 % of the copy rate).  At most kGroupSumFlatMax quotients.
 constexpr int kGroupSumFlatMax = 4096;
 __global__ void __launch_bounds__(256) group_sum_bwd_flat_kernel(const float *__restrict__ gout, const float *__restrict__ scale, float *__restrict__ gy,
                                                                  long long S, int B, int k, float tau)
