@@ -1,11 +1,10 @@
 // Flat LogicLayer kernels on feature-major activations: x [in,B], y [out,B], batch contiguous.
 //
 // The work is HBM-bound (two gathered input rows and one output row per neuron, three FMAs per
-// element), so the layout of the loop is chosen for memory: one warp owns one neuron (forward, gate
-// gradient) or one input feature (input gradient) and sweeps the batch with 128-bit accesses, every
-// row access being a fully coalesced 512-byte segment per warp.  The 16 gate values of a neuron are
-// read once per warp: 16 lanes load one value each and the soft-max / 4-coefficient reduction runs on
-// shuffles inside the half-warp, two neurons at a time.
+// element), so the layout of the loop is chosen for memory: a half-warp owns a neuron (forward, gate
+// gradient), a warp a stretch of input features (input gradient), and sweeps the batch with the widest
+// accesses that the rows allow.  The 16 gate values of a neuron are read once: each lane of the half-warp
+// loads one value and the soft-max / 4-coefficient reduction runs on shuffles.
 //
 // Input gradient: segmented reduction over the consumer lists (CSR), no atomics, fixed order.
 // A neuron whose two inputs are the same feature is listed twice in a row; the first entry takes the
