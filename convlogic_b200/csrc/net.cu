@@ -178,15 +178,8 @@ static void plan_one_launch(clb_net &net)
     P.n_layers = (int)n, P.classes = net.num_classes, P.in_features = net.in_features;
     long long units = 0;
     auto store = [&](size_t i, long long channels, int rows, int W, int ph, int pw) {
-        clb::NetStorage &st = P.store[i];
-        const long long image = (long long)rows * W, pitch = W + 2 * pw, per = (rows + 2LL * ph) * pitch;
-        if (units + channels * per > (1 << 24)) return false;
-        st.base = (int)units, st.W = W, st.image = (int)image, st.pitch = (int)pitch, st.per_channel = (int)per, st.rows = rows, st.ph = ph, st.pw = pw;
-        st.halo_units = ph || pw ? (int)(channels * per) : 0;
-        if (channels > 1 && channels * per * per >= (1LL << 32)) return false; // the kernel's divisions
-        st.by_image = clb::FastDiv::of((unsigned)image), st.by_W = clb::FastDiv::of((unsigned)W);
-        st.by_pitch = clb::FastDiv::of((unsigned)pitch), st.by_channel = clb::FastDiv::of((unsigned)per);
-        units += (channels * per + 7) / 8 * 8;
+        if (!P.store[i].lay_out(units, channels, rows, W, ph, pw)) return false;
+        units += (channels * P.store[i].per_channel + 7) / 8 * 8;
         return true;
     };
     auto flat_store = [&](size_t i, long long features) { return features <= (1 << 24) && store(i, 1, 1, (int)features, 0, 0); };
@@ -203,6 +196,8 @@ static void plan_one_launch(clb_net &net)
             const Layer &next = net.layers[i + 1];
             const bool conv = next.kind == 1;
             if (!store(i + 1, L.C, L.Hp, L.Wp, conv ? next.ph : 0, conv ? next.pw : 0)) return;
+            const long long windows = (long long)L.Hp * L.Wp;
+            if (!clb::FastDiv::exact(L.C * windows, windows) || !clb::FastDiv::exact(windows, L.Wp)) return;
             o.by_windows = clb::FastDiv::of((unsigned)(L.Hp * L.Wp)), o.by_Wp = clb::FastDiv::of((unsigned)L.Wp);
             net.slab_cost += 4LL * L.C * L.Hp * L.Wp;
         } else {

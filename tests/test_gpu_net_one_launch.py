@@ -54,3 +54,17 @@ def test_one_launch_equals_layer_launches(one_launch, batch):
                 want = compiled.forward_pixels(pixels, th)
                 one_launch(2)
                 assert torch.equal(compiled.forward_pixels(pixels, th), want), (name, batch, pixels.dtype)
+
+
+def test_one_channel_image_of_more_than_65536_pixels():
+    """The smallest square whose pixel count does not divide exactly by the kernel's multiplication runs layer by layer, whatever the switch."""
+    import convlogic_b200 as cb
+
+    torch.manual_seed(5)
+    net = torch.nn.Sequential(cb.ConvLogicLayer(1, 3, stride=2, complete=True), torch.nn.Flatten(), cb.LogicLayer(3 * 65 * 65, 6400), cb.GroupSum(10))
+    for p in net.parameters():
+        p.data.normal_()
+    x = torch.rand(40, 1, 260, 260, device="cuda") < 0.4
+    got = cb.CompiledLogicNet(net.eval(), input_shape=(1, 260, 260)).compile()(x)
+    with torch.no_grad():
+        assert torch.equal(got, net.cuda()(cb.PackBitsTensor(x, 64)))
