@@ -268,13 +268,25 @@ struct BlockPlan {
 };
 using PlanPtr = std::shared_ptr<BlockPlan>;
 
+// What a plan is on a copied or unpickled tensor (Tensor.__deepcopy__ and __reduce_ex__ take a tensor's attributes along): nothing
+// that `kept` accepts, so that the copy's first use lays its own out.  An empty OrderedDict is what torch.load reads without
+// this extension and under weights_only.
+template <typename Plan> void copies_as_nothing(py::class_<Plan, std::shared_ptr<Plan>> c)
+{
+    c.def("__deepcopy__", [](const Plan &, const py::object &) { return py::none(); });
+    c.def("__reduce__", [](const Plan &) { return py::make_tuple(py::module_::import("collections").attr("OrderedDict"), py::tuple()); });
+}
+template <typename Plan> std::shared_ptr<Plan> kept(const py::handle &tensor) // GIL held
+{
+    if (!PyObject_HasAttrString(tensor.ptr(), "_clb_plan")) return nullptr;
+    const py::object o = py::reinterpret_steal<py::object>(PyObject_GetAttrString(tensor.ptr(), "_clb_plan"));
+    return py::isinstance<Plan>(o) ? o.cast<std::shared_ptr<Plan>>() : nullptr;
+}
+
 PlanPtr plan_for(const py::handle &sel_obj, const Tensor &sel, const Geom &g, int64_t ci) // GIL held
 {
     const int64_t version = sel.is_inference() ? 0 : (int64_t)sel._version();
-    if (PyObject_HasAttrString(sel_obj.ptr(), "_clb_plan")) {
-        PlanPtr p = py::reinterpret_steal<py::object>(PyObject_GetAttrString(sel_obj.ptr(), "_clb_plan")).cast<PlanPtr>();
-        if (p && p->version == version && p->data == sel.data_ptr() && p->g == g && p->ci == ci) return p;
-    }
+    if (PlanPtr p = kept<BlockPlan>(sel_obj); p && p->version == version && p->data == sel.data_ptr() && p->g == g && p->ci == ci) return p;
     auto p = std::make_shared<BlockPlan>();
     p->g = g, p->C = (int)sel.size(0), p->ci = (int)ci, p->version = version, p->data = sel.data_ptr(), p->device = sel.device();
     const Tensor host = sel.detach().to(at::kCPU).contiguous();
@@ -493,10 +505,7 @@ using LogicPlanPtr = std::shared_ptr<LogicPlan>;
 LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const Tensor &b, const Tensor &start, const Tensor &cons, int64_t in, int64_t out)
 {
     const LogicKey key = logic_key(a, b, start, cons);
-    if (PyObject_HasAttrString(start_obj.ptr(), "_clb_plan")) {
-        LogicPlanPtr p = py::reinterpret_steal<py::object>(PyObject_GetAttrString(start_obj.ptr(), "_clb_plan")).cast<LogicPlanPtr>();
-        if (p && p->key == key && p->in == in && p->out == out) return p;
-    }
+    if (LogicPlanPtr p = kept<LogicPlan>(start_obj); p && p->key == key && p->in == in && p->out == out) return p;
     need_inputs(a, b, start, cons);
     TORCH_CHECK(start.scalar_type() == at::kLong && cons.scalar_type() == at::kLong && start.numel() == in + 1 && cons.numel() == 2 * out,
                 "convlogic_b200: consumer lists must be int64 [in_dim + 1] and [2 * out_dim]");
@@ -1025,8 +1034,8 @@ Tensor logic_fwd_py(const Tensor &x, const Tensor &a, const Tensor &b, const Ten
 
 PYBIND11_MODULE(_clb_torch, m)
 {
-    py::class_<BlockPlan, PlanPtr>(m, "BlockPlan");
-    py::class_<LogicPlan, LogicPlanPtr>(m, "LogicPlan");
+    copies_as_nothing(py::class_<BlockPlan, PlanPtr>(m, "BlockPlan").def(py::init<>()));
+    copies_as_nothing(py::class_<LogicPlan, LogicPlanPtr>(m, "LogicPlan").def(py::init<>()));
     m.def("block", &block);
     m.def("block_fwd", &block_fwd_py);
     m.def("block_bwd", &block_bwd_py);
