@@ -63,7 +63,7 @@ class ConvLogicLayer(nn.Module):
         if not x.is_cuda:
             raise RuntimeError("CUDA implementation requested, but the input is not a CUDA tensor.")
         wmode = W_SOFTMAX if self.training else W_ARGMAX
-        w, sel = self._parameters["weights"], self._buffers["selection"]
+        w, sel = self.weights, self.selection
         if w.dtype != x.dtype:
             w = w.to(x.dtype)
         if not sel.is_contiguous():

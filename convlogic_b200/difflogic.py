@@ -88,7 +88,7 @@ class LogicLayer(torch.nn.Module):
         assert x.is_cuda, f"x must be a CUDA tensor, got device: {x.device}"
         assert x.ndim == 2, x.ndim
         assert x.shape[1] == self.in_dim, (x.shape, self.in_dim)
-        w, buf = self._parameters["weights"], self._buffers
+        w, buf = self.weights, self._buffers   # the attribute: a parametrization or pruning puts something else there than the parameter
         if w.dtype != x.dtype:
             w = w.to(x.dtype)
         # [B, in] -> [B, out]; the result is a view of feature-major storage, which the next flat layer reads without a copy
@@ -240,7 +240,7 @@ class FusedLogicLayers(torch.nn.Module):
 
     def _trees(self, x, wmode, labels, k, tau):
         buf = self._buffers
-        w = [l._parameters["weights"].contiguous() for l in self.layers]
+        w = [l.weights.contiguous() for l in self.layers]
         return native().trees(x, *w, buf["leaf"], buf["node"], buf["leaf_start"], buf["leaf_slots"], wmode, self.covers_all, labels, k, tau)
 
     def cross_entropy(self, x, labels, k, tau=1.0):
