@@ -95,6 +95,29 @@ def conv_groups(sel, x_shape, geom, dtype):
     return out
 
 
+def plane_lists(sel, ci, geom):
+    """Per input channel, the (output channel, slot) gradient planes that belong to it -- the tables of
+    ``clb_convtree_bwd_plane`` -- or None when the selection does not fit those kernels (an output channel with more
+    than two input channels, or taps outside the window).  Cached on the selection tensor like ``conv_groups``."""
+    key = (sel._version, ci, geom[4], geom[5])
+    cache = getattr(sel, "_clb_planes", None)
+    if cache is not None and cache[0] == key:
+        return cache[1]
+    c = sel.shape[0]
+    sel_host = np.ascontiguousarray(sel.detach().cpu().numpy(), dtype=np.int32)
+    start = np.zeros(ci + 1, dtype=np.int32)
+    entry = np.zeros(max(2 * c, 1), dtype=np.int32)
+    cnt = lib().clb_conv_channel_lists(sel_host.ctypes.data_as(C.c_void_p), c, ci, geom[4], geom[5],
+                                       start.ctypes.data_as(C.c_void_p), entry.ctypes.data_as(C.c_void_p), entry.size)
+    out = None
+    if cnt >= 0:
+        out = (torch.from_numpy(start).to(sel.device), torch.from_numpy(entry[:max(cnt, 1)].copy()).to(sel.device))
+    elif cnt != _lib.ERR_SHAPE:
+        check(cnt)
+    sel._clb_planes = (key, out)
+    return out
+
+
 def _bwd_args_ok(gy, x, w, sel, amax, geom):
     """Shapes and dtypes of the fused block's backward inputs (the C ABI receives bare pointers)."""
     n, ci, h, wd = x.shape
@@ -272,6 +295,14 @@ def pack_bits(t, bit_count, sample_major=False):
     return native().pack_bits(t, bit_count, sample_major)
 
 
+def packed_logic(x, a, b, ops):
+    return native().packed_logic(x, a, b, ops)
+
+
+def group_popcount(x, pad_len, k):
+    return native().group_popcount(x, pad_len, k)
+
+
 def packed_convtree(x, ops, sel, geom):
     check_input(x, ops, sel)
     ci, h, w, words = x.shape
@@ -355,6 +386,114 @@ def thermometer_pack(pixels, thresholds, slab=False):
     return out, (64 - n % 64) % 64
 
 
+# ------------------------------------------------------------------- class sums, fused flat layers, optimiser
+def group_sum_fwd(y_fm, k, tau):
+    """Feature-major activations [F, B] -> [B, k] class sums / tau."""
+    check_input(y_fm)
+    f, b = y_fm.shape
+    out = torch.empty((b, k), dtype=y_fm.dtype, device=y_fm.device)
+    nbytes = lib().clb_group_sum_scratch_bytes(f, b, k, dtype_code(y_fm))
+    scratch = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=y_fm.device)
+    check(lib().clb_group_sum_fwd(ptr(y_fm), ptr(out), ptr(scratch), nbytes, f, b, k, float(tau), dtype_code(y_fm), stream()))
+    return out
+
+
+def group_sum_bwd(gout, f, k, tau, scale=None):
+    """Gradient of group_sum_fwd: [B, k] -> feature-major [F, B]; ``scale``: a one-element device tensor every value is
+    multiplied by (the upstream gradient of a scalar loss), read by the kernel."""
+    check_input(gout)
+    b = gout.shape[0]
+    gy = torch.empty((f, b), dtype=gout.dtype, device=gout.device)
+    if scale is not None:
+        check_input(scale)
+        if scale.numel() != 1 or scale.dtype != gout.dtype:
+            raise RuntimeError("convlogic_b200: `scale` must be a one-element tensor of the gradient's dtype")
+    check(lib().clb_group_sum_bwd_scaled(ptr(gout), ptr(scale), ptr(gy), f, b, k, float(tau), dtype_code(gout), stream()))
+    return gy
+
+
+def logic_tree_fwd(x_fm, leaf, node, w0, w1, w2, wmode):
+    """Three fused flat layers, forward: x [in, B] -> y [T, B] (see ``clb_logic_tree_fwd``)."""
+    check_input(x_fm, leaf, node, w0, w1, w2)
+    t, b = leaf.shape[0], x_fm.shape[1]
+    y = torch.empty((t, b), dtype=torch.float32, device=x_fm.device)
+    check(lib().clb_logic_tree_fwd(ptr(x_fm), ptr(leaf), ptr(node), ptr(w0), ptr(w1), ptr(w2), ptr(y), t, b, wmode, stream()))
+    return y
+
+
+def logic_tree_bwd(x_fm, leaf, node, w0, w1, w2, gy, start, slots, wmode, need_gx=True, gw_out=None, clear_gw=True, head=None):
+    """Gradients of ``logic_tree_fwd``: (gx [in, B] or None, gw0, gw1, gw2).  ``gw_out``: three contiguous tensors to
+    receive the gate gradients (cleared first: a neuron no tree reads keeps a zero gradient; ``clear_gw=False`` when the
+    caller knows that every neuron sits in a tree).  ``head = (dscore [B, k], scale [1], k, tau)`` instead of ``gy``: the
+    trees feed GroupSum + cross-entropy, and the upstream gradient is derived from that head's score gradient inside
+    the kernel."""
+    if head is None:
+        check_input(x_fm, leaf, node, w0, w1, w2, gy, start, slots)
+    else:
+        check_input(x_fm, leaf, node, w0, w1, w2, head[0], head[1], start, slots)
+        if head[0].dtype != torch.float32 or head[1].dtype != torch.float32 or tuple(head[0].shape) != (x_fm.shape[1], head[2]) \
+                or head[1].numel() != 1 or leaf.shape[0] % head[2]:
+            raise RuntimeError("convlogic_b200: the head of logic_tree_bwd is (dscore float32 [B, k], scale float32 [1], k, tau)")
+    t, b, in_dim = leaf.shape[0], x_fm.shape[1], x_fm.shape[0]
+    tapgrad = torch.empty((max(t * 8, 1), b), dtype=torch.float32, device=x_fm.device)
+    if gw_out is None:
+        gws = [torch.zeros_like(w) if clear_gw else torch.empty_like(w) for w in (w0, w1, w2)]
+    else:
+        gws = [g.zero_() if clear_gw else g for g in gw_out]
+    gx = torch.empty_like(x_fm) if need_gx else None
+    if head is None:
+        check(lib().clb_logic_tree_bwd(ptr(x_fm), ptr(leaf), ptr(node), ptr(w0), ptr(w1), ptr(w2), ptr(gy), ptr(tapgrad), ptr(gws[0]),
+                                       ptr(gws[1]), ptr(gws[2]), ptr(gx), ptr(start), ptr(slots), in_dim, t, b, wmode, stream()))
+    else:
+        check(lib().clb_logic_tree_bwd_scores(ptr(x_fm), ptr(leaf), ptr(node), ptr(w0), ptr(w1), ptr(w2), ptr(head[0]), ptr(head[1]),
+                                              int(head[2]), float(head[3]), ptr(tapgrad), ptr(gws[0]), ptr(gws[1]), ptr(gws[2]), ptr(gx),
+                                              ptr(start), ptr(slots), in_dim, t, b, wmode, stream()))
+    return gx, gws[0], gws[1], gws[2]
+
+
+def logic_tree_fwd_ce(x_fm, leaf, node, w0, w1, w2, labels, k, tau, wmode):
+    """Fused flat layers + GroupSum + mean cross-entropy without the activation in between: (loss [1], dscore [B, k]),
+    or None for a shape that path does not take (the caller then runs ``logic_tree_fwd`` and ``group_sum_ce``)."""
+    check_input(x_fm, leaf, node, w0, w1, w2, labels)
+    t, b = leaf.shape[0], x_fm.shape[1]
+    if x_fm.dtype != torch.float32 or labels.dtype != torch.int64 or labels.shape != (b,):
+        raise RuntimeError("convlogic_b200: logic_tree_fwd_ce expects float32 [in, B] activations and int64 [B] labels")
+    nbytes = lib().clb_logic_tree_fwd_ce_scratch_bytes(t, b, k)
+    if nbytes == 0 or b % 4 or b > 512 or k > 32:
+        return None
+    loss = torch.empty(1, dtype=torch.float32, device=x_fm.device)
+    dscore = torch.empty((b, k), dtype=torch.float32, device=x_fm.device)
+    scratch = torch.empty(nbytes, dtype=torch.uint8, device=x_fm.device)
+    rc = lib().clb_logic_tree_fwd_ce(ptr(x_fm), ptr(leaf), ptr(node), ptr(w0), ptr(w1), ptr(w2), ptr(labels), ptr(dscore), ptr(loss),
+                                     ptr(scratch), nbytes, t, b, k, float(tau), wmode, stream())
+    if rc == _lib.ERR_SHAPE:
+        return None
+    check(rc)
+    return loss, dscore
+
+
+def group_sum_ce(y_fm, labels, k, tau, want_scores=False):
+    """GroupSum + mean cross-entropy on feature-major activations [F, B]: (loss [1], dscore [B, k], scores or None)."""
+    check_input(y_fm, labels)
+    if y_fm.dtype != torch.float32 or labels.dtype != torch.int64 or labels.shape != (y_fm.shape[1],):
+        raise RuntimeError("convlogic_b200: group_sum_ce expects float32 [F, B] activations and int64 [B] labels")
+    f, b = y_fm.shape
+    if f % k:
+        raise ValueError(f"in_dim ({f}) has to be divisible by k ({k}) but it is not")
+    loss = torch.empty(1, dtype=torch.float32, device=y_fm.device)
+    dscore = torch.empty((b, k), dtype=torch.float32, device=y_fm.device)
+    scores = torch.empty((b, k), dtype=torch.float32, device=y_fm.device) if want_scores else None
+    nbytes = lib().clb_group_sum_scratch_bytes(f, b, k, dtype_code(y_fm))
+    scratch = torch.empty(max(nbytes, 16), dtype=torch.uint8, device=y_fm.device)
+    check(lib().clb_group_sum_ce(ptr(y_fm), ptr(labels), ptr(scores), ptr(dscore), ptr(loss), ptr(scratch), nbytes, f, b, k, float(tau), stream()))
+    return loss, dscore, scores
+
+
 def transpose2d(x):
     """Contiguous [cols, rows] copy of a contiguous float32 [rows, cols] tensor (one tiled kernel)."""
     return native().transpose2d(x)
+
+
+def adam_step(p, g, m, v, lr, beta1, beta2, eps, weight_decay, step, decoupled):
+    """One Adam / AdamW step over flat fp32 buffers, in place."""
+    native().adam_step(p, g, m, v, float(lr), float(beta1), float(beta2), float(eps), float(weight_decay), int(step), bool(decoupled))
