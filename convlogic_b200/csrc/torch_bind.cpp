@@ -15,6 +15,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/pybind.h>
 
 #include <atomic>
@@ -64,11 +65,17 @@ int dtype_code(const Tensor &t)
 
 void *cur_stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 template <typename T = void> T *ptr(const Tensor &t) { return t.defined() ? static_cast<T *>(t.data_ptr()) : nullptr; }
-// device memory from torch's caching allocator, without the dispatcher's detour (about half a microsecond each)
-Tensor alloc(at::IntArrayRef sizes, const Tensor &like, at::ScalarType type) { return at::detail::empty_cuda(sizes, type, like.device(), std::nullopt); }
+// device memory from torch's caching allocator, without the dispatcher's detour (about half a microsecond each) unless a trace
+// has to see where an operation's result comes from
+Tensor alloc(at::IntArrayRef sizes, const Tensor &like, at::ScalarType type)
+{
+    if (torch::jit::tracer::isTracing()) return at::empty(sizes, at::TensorOptions().dtype(type).device(like.device()));
+    return at::detail::empty_cuda(sizes, type, like.device(), std::nullopt);
+}
 Tensor alloc(at::IntArrayRef sizes, const Tensor &like) { return alloc(sizes, like, like.scalar_type()); }
 Tensor alloc_strided(at::IntArrayRef sizes, at::IntArrayRef strides, const Tensor &like)
 {
+    if (torch::jit::tracer::isTracing()) return at::empty_strided(sizes, strides, like.options());
     return at::detail::empty_strided_cuda(sizes, strides, like.scalar_type(), like.device());
 }
 Tensor scratch_bytes(size_t n, const Tensor &like) { return alloc({(int64_t)(n < 16 ? 16 : n)}, like, at::kByte); }
@@ -86,6 +93,20 @@ bool wants_grad(std::initializer_list<std::reference_wrapper<const Tensor>> ts)
     for (const Tensor &t : ts)
         if (t.defined() && t.requires_grad()) return true;
     return false;
+}
+
+// Does torch follow this call by something that knows Python Functions only: torch.jit.trace, which would take a result made here for
+// a constant, or forward-mode AD, whose tangents would be dropped?  Then it is handed to convlogic_b200.functional.
+bool followed(std::initializer_list<std::reference_wrapper<const Tensor>> ts)
+{
+    if (torch::jit::tracer::isTracing()) return true;
+    for (const Tensor &t : ts)
+        if (t.defined() && t._fw_grad(0).defined()) return true;
+    return false;
+}
+template <typename... Args> py::object in_python(const char *name, Args &&...args)
+{
+    return py::module_::import("convlogic_b200.functional").attr(name)(std::forward<Args>(args)...);
 }
 
 // SavedVariable of an input (never an output) of a node
@@ -450,6 +471,7 @@ struct BlockNode : public Node {
 py::object block(Tensor x, Tensor w, py::object sel_obj, int sh, int sw, int ph, int pw, int kh, int kw, bool want_inter, bool want_idx, int wmode,
                  bool y_fm)
 {
+    if (followed({x, w})) return in_python("followed_block", x, w, sel_obj, sh, sw, ph, pw, kh, kw, want_inter, want_idx, wmode, y_fm);
     const Tensor sel = sel_obj.cast<Tensor>();
     x = x.contiguous(), w = w.contiguous();
     const Geom g{sh, sw, ph, pw, kh, kw};
@@ -619,6 +641,7 @@ struct LogicNode : public Node {
 // fm: x [in, B] -> y [out, B] (the reference's Function); else x [B, in] -> y [B, out] on the storage [out, B]
 Tensor logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w_in, py::object start_obj, const Tensor &cons, int wmode, bool fm)
 {
+    if (followed({x, w_in})) return in_python("followed_logic", x, a, b, w_in, start_obj, cons, wmode, fm).cast<Tensor>();
     const Tensor start = start_obj.cast<Tensor>();
     const bool graph = wants_grad({x, w_in});
     TORCH_CHECK(x.is_cuda(), "convlogic_b200: tensor must be a CUDA tensor");
@@ -706,6 +729,7 @@ struct GroupSumNode : public Node {
 // x [B, F] on feature-major storage -> [B, k]
 Tensor group_sum(const Tensor &x, int k, double tau)
 {
+    if (followed({x})) return in_python("followed_group_sum", x, k, tau).cast<Tensor>();
     Tensor out;
     {
         Below below(x);
@@ -757,6 +781,7 @@ struct GroupSumCeNode : public Node {
 
 Tensor group_sum_ce(const Tensor &x, const Tensor &labels, int k, double tau)
 {
+    if (followed({x})) return in_python("followed_group_sum_ce", x, labels, k, tau).cast<Tensor>();
     Tensor loss, dscore;
     {
         Below below(x);
@@ -846,6 +871,8 @@ struct TreeNode : public Node {
 Tensor trees(const Tensor &x, const Tensor &w0, const Tensor &w1, const Tensor &w2, const Tensor &leaf, const Tensor &node_t, const Tensor &start,
              const Tensor &slots, int wmode, bool covers_all, const std::optional<Tensor> &labels_in, int k, double tau)
 {
+    if (followed({x, w0, w1, w2}))
+        return in_python("followed_trees", x, w0, w1, w2, leaf, node_t, start, slots, wmode, covers_all, labels_in, k, tau).cast<Tensor>();
     const bool graph = wants_grad({x, w0, w1, w2});
     const TreeTables t{leaf, node_t, start, slots, covers_all};
     TORCH_CHECK(x.is_cuda() && x.dim() == 2 && x.scalar_type() == at::kFloat, "convlogic_b200: the fused flat layers take float32 [B, in] CUDA tensors");

@@ -63,3 +63,60 @@ def test_parametrized_weights(kind):
     assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
     for a, b in zip(got[2:], want[2:]):
         assert torch.equal(a, 2 * b)
+
+
+class _Loss(torch.nn.Module):
+    def __init__(self, trees):
+        super().__init__()
+        self.trees = trees
+
+    def forward(self, x):
+        return self.trees.cross_entropy(x, torch.arange(x.shape[0], device="cuda") % 4, 4, 2.0)
+
+
+def _followed_cases():
+    import convlogic_b200 as cb
+
+    for kind in MADE:
+        m, x = MADE[kind]()
+        yield kind, m, x
+    m, x = _flat()
+    yield "class sums", torch.nn.Sequential(m, cb.GroupSum(4, 2.0)), x
+    m, x = _trees()
+    yield "loss", _Loss(m), x
+
+
+@pytest.mark.parametrize("train", [True, False])
+def test_traces_follow_the_input(train):
+    for name, m, x in _followed_cases():
+        m.train(train)
+        traced = torch.jit.trace(m, (x,), check_trace=False)
+        other = 1 - x
+        assert torch.equal(traced(other), m(other)), name
+        assert not torch.equal(m(other), m(x)), name
+        if train:
+            a, b = (torch.autograd.grad(f(other).sum(), _weights(m)) for f in (traced, m))
+            assert all(torch.allclose(p, q, rtol=1e-5, atol=1e-7) for p, q in zip(a, b)), name  # the general kernels' order of additions
+
+
+def test_a_tangent_is_refused_and_not_dropped():
+    import torch.autograd.forward_ad as fwad
+
+    for name, m, x in _followed_cases():
+        with fwad.dual_level(), pytest.raises(NotImplementedError, match="jvp"):
+            m(fwad.make_dual(x, torch.ones_like(x)))
+    m, x = _flat()
+    w = m.weights.detach()
+    del m.weights
+    with fwad.dual_level(), pytest.raises(NotImplementedError, match="jvp"):
+        m.weights = fwad.make_dual(w, torch.ones_like(w))
+        m(x)
+
+
+@pytest.mark.parametrize("kind", MADE)
+def test_functorch_transforms_are_refused(kind):
+    m, x = MADE[kind]()
+    with pytest.raises(RuntimeError):
+        torch.func.vmap(m)(torch.stack([x, x]))
+    with pytest.raises(RuntimeError):
+        torch.func.grad(lambda t: m(t).sum())(x)
