@@ -115,6 +115,10 @@ SavedVariable saved(const Tensor &t) { return SavedVariable(t, false); }
 // One node kind per operation: `Derived` has fields, run(grads) and clear().
 template <typename Derived> std::shared_ptr<Derived> new_node() { return std::shared_ptr<Derived>(new Derived(), torch::autograd::deleteNode); }
 
+// A node's upstream gradient.  Where nothing comes in (a consumer whose backward gives no gradient) it is zeros, as for a Python Function: the
+// parameters' gradients are then zeros too, and a gradient slice is overwritten and not left with the last step's values.
+Tensor upstream(const Node &n, const variable_list &grads) { return grads[0].defined() ? grads[0] : n.input_metadata(0).zeros_like(); }
+
 // [rows, cols] fp32 -> contiguous [cols, rows]
 Tensor transpose2d(const Tensor &x)
 {
@@ -451,12 +455,11 @@ struct BlockNode : public Node {
     void release_variables() override { x.reset_data(), w.reset_data(), amax.reset(); }
     variable_list apply(variable_list &&grads) override
     {
-        if (!grads[0].defined()) return {Tensor(), Tensor()};
         const Tensor xx = x.unpack(), ww = w.unpack(), &ss = sel;
         TORCH_CHECK(ss.is_inference() || plan->version == (int64_t)ss._version(), "convlogic_b200: the selection was modified between forward and backward");
         const bool need_gx = task_should_compute_output(0), need_gw = task_should_compute_output(1) && wmode != CLB_W_ARGMAX;
         if (!need_gx && !need_gw) return {Tensor(), Tensor()};
-        Tensor gy = grads[0];
+        Tensor gy = upstream(*this, grads);
         if (!is_feature_major(gy)) gy = gy.contiguous(); // a feature-major gradient (from flat layers behind this block) is read as it is
         if (!need_gw) return {block_bwd(gy, xx, ww, ss, amax, g, [&] { return plan; }, wmode, need_gx, false, Tensor()).first, Tensor()};
         Sinks sinks({ww});
@@ -593,12 +596,11 @@ struct LogicNode : public Node {
     void release_variables() override { x.reset_data(), w.reset_data(), coef.reset(); }
     variable_list apply(variable_list &&grads) override
     {
-        if (!grads[0].defined()) return {Tensor(), Tensor()};
         const Tensor xx = x.unpack(), ww = w.unpack();
         TORCH_CHECK(key == logic_key(a, b, start, cons), "convlogic_b200: the connections of a layer were modified between forward and backward");
         const bool need_gx = task_should_compute_output(0), need_gw = task_should_compute_output(1) && wmode != CLB_W_ARGMAX;
         Below below(xx);
-        const Tensor gy = fm ? grads[0].contiguous() : feature_major_storage(grads[0]);
+        const Tensor up = upstream(*this, grads), gy = fm ? up.contiguous() : feature_major_storage(up);
         TORCH_CHECK(gy.numel() == out * batch && gy.scalar_type() == xx.scalar_type(), "convlogic_b200: upstream gradient must be [", out, ", ", batch, "] ",
                     xx.scalar_type());
         const int dt = dtype_code(xx);
@@ -720,9 +722,9 @@ struct GroupSumNode : public Node {
     std::string name() const override { return "GroupSumFunctionBackward"; }
     variable_list apply(variable_list &&grads) override
     {
-        if (!grads[0].defined()) return {Tensor()};
-        Below below(grads[0]);
-        return {finished_grad(group_sum_bwd(grads[0].contiguous(), f, k, tau, Tensor()), feeds_leaf(*this, 0))};
+        const Tensor gout = upstream(*this, grads);
+        Below below(gout);
+        return {finished_grad(group_sum_bwd(gout.contiguous(), f, k, tau, Tensor()), feeds_leaf(*this, 0))};
     }
 };
 
@@ -771,10 +773,9 @@ struct GroupSumCeNode : public Node {
     void release_variables() override { dscore.reset(); }
     variable_list apply(variable_list &&grads) override
     {
-        if (!grads[0].defined()) return {Tensor()};
         TORCH_CHECK(dscore.defined(), "Trying to backward through the graph a second time: specify retain_graph=True the first time");
         Below below(dscore);
-        const Tensor scale = grads[0].reshape({1}).to(dscore.scalar_type()).contiguous();
+        const Tensor scale = upstream(*this, grads).reshape({1}).to(dscore.scalar_type()).contiguous();
         return {finished_grad(group_sum_bwd(dscore, f, k, tau, scale), feeds_leaf(*this, 0))};
     }
 };
@@ -848,14 +849,14 @@ struct TreeNode : public Node {
     void release_variables() override { x.reset_data(), w0.reset_data(), w1.reset_data(), w2.reset_data(), dscore.reset(); }
     variable_list apply(variable_list &&grads) override
     {
-        if (!grads[0].defined()) return variable_list(4);
         const Tensor xx = x.unpack(), a = w0.unpack(), b = w1.unpack(), c = w2.unpack();
         Below below(xx);
+        const Tensor up = upstream(*this, grads);
         Tensor gy, scale;
         if (k)
-            scale = grads[0].reshape({1}).to(at::kFloat).contiguous();
+            scale = up.reshape({1}).to(at::kFloat).contiguous();
         else
-            gy = feature_major_storage(grads[0]);
+            gy = feature_major_storage(up);
         Sinks sinks({a, b, c});
         const bool direct = sinks.any() && wmode != CLB_W_ARGMAX;
         auto out = tree_bwd(xx, in, batch, t, a, b, c, gy, dscore, scale, k, tau, wmode, task_should_compute_output(0),

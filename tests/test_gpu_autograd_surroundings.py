@@ -120,3 +120,29 @@ def test_functorch_transforms_are_refused(kind):
         torch.func.vmap(m)(torch.stack([x, x]))
     with pytest.raises(RuntimeError):
         torch.func.grad(lambda t: m(t).sum())(x)
+
+
+class _NoGradient(torch.autograd.Function):
+    @staticmethod
+    def forward(ctx, y):
+        return y.sum()
+
+    @staticmethod
+    def backward(ctx, g):
+        return None
+
+
+def test_no_upstream_gradient_is_a_gradient_of_zeros():
+    import convlogic_b200 as cb
+
+    for name, m, x in _followed_cases():
+        x.requires_grad_(True)
+        _NoGradient.apply(m(x)).backward()
+        for t in [x] + _weights(m):
+            assert t.grad is not None and not t.grad.any(), name
+        bucket = cb.GradBucket(m).direct()
+        m(x).sum().backward()
+        assert bucket.flat.any(), name
+        _NoGradient.apply(m(x)).backward()
+        assert not bucket.flat.any(), name   # not the step before's
+        bucket.direct(False)
