@@ -446,24 +446,24 @@ std::pair<Tensor, Tensor> block_bwd(Tensor gy, const Tensor &x, const Tensor &w,
 }
 
 struct BlockNode : public Node {
-    SavedVariable x, w;
-    Tensor sel, amax;
+    SavedVariable x, w, amax; // what the call made or was given goes through saved-tensor hooks; `sel` belongs to the module
+    Tensor sel;
     PlanPtr plan;
     Geom g;
     int wmode;
     std::string name() const override { return "FullConvLogicFunctionBackward"; }
-    void release_variables() override { x.reset_data(), w.reset_data(), amax.reset(); }
+    void release_variables() override { x.reset_data(), w.reset_data(), amax.reset_data(); }
     variable_list apply(variable_list &&grads) override
     {
-        const Tensor xx = x.unpack(), ww = w.unpack(), &ss = sel;
+        const Tensor xx = x.unpack(), ww = w.unpack(), best = amax.unpack(), &ss = sel;
         TORCH_CHECK(ss.is_inference() || plan->version == (int64_t)ss._version(), "convlogic_b200: the selection was modified between forward and backward");
         const bool need_gx = task_should_compute_output(0), need_gw = task_should_compute_output(1) && wmode != CLB_W_ARGMAX;
         if (!need_gx && !need_gw) return {Tensor(), Tensor()};
         Tensor gy = upstream(*this, grads);
         if (!is_feature_major(gy)) gy = gy.contiguous(); // a feature-major gradient (from flat layers behind this block) is read as it is
-        if (!need_gw) return {block_bwd(gy, xx, ww, ss, amax, g, [&] { return plan; }, wmode, need_gx, false, Tensor()).first, Tensor()};
+        if (!need_gw) return {block_bwd(gy, xx, ww, ss, best, g, [&] { return plan; }, wmode, need_gx, false, Tensor()).first, Tensor()};
         Sinks sinks({ww});
-        auto out = block_bwd(gy, xx, ww, ss, amax, g, [&] { return plan; }, wmode, need_gx, true, sinks.slice(0));
+        auto out = block_bwd(gy, xx, ww, ss, best, g, [&] { return plan; }, wmode, need_gx, true, sinks.slice(0));
         if (!sinks.any()) return {out.first, out.second};
         sinks.ready();
         return {out.first, Tensor()};
@@ -486,7 +486,7 @@ py::object block(Tensor x, Tensor w, py::object sel_obj, int sh, int sw, int ph,
         auto node = new_node<BlockNode>();
         node->set_next_edges(torch::autograd::collect_next_edges(x, w));
         if (!plan) get_plan();
-        node->x = saved(x), node->w = saved(w), node->sel = sel, node->amax = o.amax, node->plan = plan, node->g = g, node->wmode = wmode;
+        node->x = saved(x), node->w = saved(w), node->sel = sel, node->amax = saved(o.amax), node->plan = plan, node->g = g, node->wmode = wmode;
         torch::autograd::set_history(o.y, node);
     }
     if (!want_inter && !want_idx) return py::cast(o.y);
@@ -587,13 +587,13 @@ struct LogicNode : public Node {
     SavedVariable x, w;      // x: a tensor on the feature-major storage the forward read
     Tensor a, b, start, cons; // connections, checked against `key`
     LogicKey key;
-    Tensor coef;             // gate coefficients and the laid-out lists (fp32 with an input gradient)
+    SavedVariable coef;      // gate coefficients and the laid-out lists (fp32 with an input gradient)
     LogicPlanPtr plan;
     int64_t in, out, batch;
     int wmode;
     bool fm; // the call's own tensors are feature-major ([in, B] -> [out, B])
     std::string name() const override { return "LogicLayerCudaFunctionBackward"; }
-    void release_variables() override { x.reset_data(), w.reset_data(), coef.reset(); }
+    void release_variables() override { x.reset_data(), w.reset_data(), coef.reset_data(); }
     variable_list apply(variable_list &&grads) override
     {
         const Tensor xx = x.unpack(), ww = w.unpack();
@@ -617,11 +617,12 @@ struct LogicNode : public Node {
             if (gx.defined()) gx.zero_();
         } else {
             int rc = CLB_ERR_SHAPE;
-            if (need_gx && coef.defined() && plan) { // both gradients in one pass
+            if (need_gx && plan) { // both gradients in one pass
+                const Tensor cc = coef.unpack();
                 const size_t bytes = need_gw ? clb_logic_bwd_scratch_bytes(in, out, batch) : 0;
                 Tensor scratch;
                 if (need_gw) scratch = scratch_bytes(bytes, xx);
-                rc = clb_logic_bwd(ptr<float>(xx), ptr<float>(ww), ptr<float>(coef), ptr<float>(gy), ptr<float>(gx), ptr<float>(gw),
+                rc = clb_logic_bwd(ptr<float>(xx), ptr<float>(ww), ptr<float>(cc), ptr<float>(gy), ptr<float>(gx), ptr<float>(gw),
                                    ptr<int32_t>(plan->start32), ptr(plan->entry), ptr(scratch), bytes, in, out, batch, wmode, cur_stream());
                 if (rc != CLB_ERR_SHAPE) check(rc);
             }
@@ -679,7 +680,8 @@ Tensor logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w_
         // the parameter itself is saved (it may carry a gradient sink); its contiguous copy only where it is not contiguous
         node->x = saved(x_fm), node->w = saved(w_in.is_contiguous() ? w_in : w);
         node->a = a, node->b = b, node->start = start, node->cons = cons, node->key = plan ? plan->key : logic_key(a, b, start, cons);
-        node->coef = coef, node->plan = plan, node->in = in, node->out = out, node->batch = batch, node->wmode = wmode, node->fm = fm;
+        if (plan) node->coef = saved(coef);
+        node->plan = plan, node->in = in, node->out = out, node->batch = batch, node->wmode = wmode, node->fm = fm;
         torch::autograd::set_history(y, node);
     }
     return y;
@@ -765,18 +767,18 @@ std::tuple<Tensor, Tensor, Tensor> group_sum_ce_raw(const Tensor &y_fm, int64_t 
 }
 
 struct GroupSumCeNode : public Node {
-    Tensor dscore;
+    SavedVariable dscore;
     int64_t f;
     int k;
     double tau;
     std::string name() const override { return "GroupSumCrossEntropyFunctionBackward"; }
-    void release_variables() override { dscore.reset(); }
+    void release_variables() override { dscore.reset_data(); }
     variable_list apply(variable_list &&grads) override
     {
-        TORCH_CHECK(dscore.defined(), "Trying to backward through the graph a second time: specify retain_graph=True the first time");
-        Below below(dscore);
-        const Tensor scale = upstream(*this, grads).reshape({1}).to(dscore.scalar_type()).contiguous();
-        return {finished_grad(group_sum_bwd(dscore, f, k, tau, scale), feeds_leaf(*this, 0))};
+        const Tensor ds = dscore.unpack();
+        Below below(ds);
+        const Tensor scale = upstream(*this, grads).reshape({1}).to(ds.scalar_type()).contiguous();
+        return {finished_grad(group_sum_bwd(ds, f, k, tau, scale), feeds_leaf(*this, 0))};
     }
 };
 
@@ -792,7 +794,7 @@ Tensor group_sum_ce(const Tensor &x, const Tensor &labels, int k, double tau)
     if (wants_grad({x})) {
         auto node = new_node<GroupSumCeNode>();
         node->set_next_edges(torch::autograd::collect_next_edges(x));
-        node->dscore = dscore, node->f = x.size(1), node->k = k, node->tau = tau;
+        node->dscore = saved(dscore), node->f = x.size(1), node->k = k, node->tau = tau;
         torch::autograd::set_history(loss, node);
     }
     return loss;
@@ -842,11 +844,11 @@ struct TreeNode : public Node {
     TreeTables t;
     int64_t in, batch;
     int wmode;
-    Tensor dscore; // head: GroupSum + cross-entropy
+    SavedVariable dscore; // head: GroupSum + cross-entropy
     int k = 0;
     double tau = 1.0;
     std::string name() const override { return k ? "LogicTreeCrossEntropyFunctionBackward" : "LogicTreeFunctionBackward"; }
-    void release_variables() override { x.reset_data(), w0.reset_data(), w1.reset_data(), w2.reset_data(), dscore.reset(); }
+    void release_variables() override { x.reset_data(), w0.reset_data(), w1.reset_data(), w2.reset_data(), dscore.reset_data(); }
     variable_list apply(variable_list &&grads) override
     {
         const Tensor xx = x.unpack(), a = w0.unpack(), b = w1.unpack(), c = w2.unpack();
@@ -859,7 +861,7 @@ struct TreeNode : public Node {
             gy = feature_major_storage(up);
         Sinks sinks({a, b, c});
         const bool direct = sinks.any() && wmode != CLB_W_ARGMAX;
-        auto out = tree_bwd(xx, in, batch, t, a, b, c, gy, dscore, scale, k, tau, wmode, task_should_compute_output(0),
+        auto out = tree_bwd(xx, in, batch, t, a, b, c, gy, k ? dscore.unpack() : Tensor(), scale, k, tau, wmode, task_should_compute_output(0),
                             direct ? std::array<Tensor, 3>{sinks.slice(0), sinks.slice(1), sinks.slice(2)} : std::array<Tensor, 3>{});
         Tensor gx = out[0].defined() ? finished_grad(out[0], feeds_leaf(*this, 0)) : Tensor();
         if (direct) sinks.ready();
@@ -912,7 +914,8 @@ Tensor trees(const Tensor &x, const Tensor &w0, const Tensor &w1, const Tensor &
         node->set_next_edges(torch::autograd::collect_next_edges(x, w0, w1, w2));
         node->x = saved(x_fm), node->w0 = saved(w0), node->w1 = saved(w1), node->w2 = saved(w2), node->t = t, node->in = x.size(1), node->batch = B,
         node->wmode = wmode;
-        node->dscore = dscore, node->k = k, node->tau = tau;
+        if (k) node->dscore = saved(dscore);
+        node->k = k, node->tau = tau;
         torch::autograd::set_history(out, node);
     }
     return out;

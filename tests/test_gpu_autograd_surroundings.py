@@ -146,3 +146,23 @@ def test_no_upstream_gradient_is_a_gradient_of_zeros():
         _NoGradient.apply(m(x)).backward()
         assert not bucket.flat.any(), name   # not the step before's
         bucket.direct(False)
+
+
+def test_saved_tensor_hooks_see_what_a_call_keeps():
+    for name, m, x in _followed_cases():
+        want = _step(m, x)
+        kept = []
+
+        def pack(t):
+            kept.append((t.dtype, tuple(t.shape)))
+            return t.cpu()
+
+        with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+            xr = x.detach().requires_grad_(True)
+            y = m(xr)
+        got = [y.detach(), *torch.autograd.grad(y.sum(), [xr] + _weights(m))]
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), name
+        extra = {"block": (torch.uint8, (8, 16, 8, 8)), "loss": (torch.float32, (36, 4))}.get(name)   # arg-max bytes, score gradient
+        assert extra is None or extra in kept, (name, kept)
+        with pytest.raises(RuntimeError, match="second time"):
+            torch.autograd.grad(y.sum(), _weights(m))
