@@ -8,6 +8,7 @@
 // include/convlogic_b200.h.
 #include <ATen/ATen.h>
 #include <ATen/cuda/EmptyTensor.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -535,6 +536,8 @@ LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const 
     TORCH_CHECK(start.scalar_type() == at::kLong && cons.scalar_type() == at::kLong && start.numel() == in + 1 && cons.numel() == 2 * out,
                 "convlogic_b200: consumer lists must be int64 [in_dim + 1] and [2 * out_dim]");
     if (in > 0x3fffffff || out > 0x3fffffff) return nullptr;
+    // inside a stream capture nothing would be laid out before the replay: this call runs the two separate gradient kernels
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return nullptr;
     auto p = std::make_shared<LogicPlan>();
     p->key = key, p->in = in, p->out = out;
     Below below(start);
@@ -666,7 +669,7 @@ Tensor logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w_
         y = fm ? alloc({out, batch}, x) : alloc_strided({batch, out}, {1, std::max<int64_t>(batch, 1)}, x);
         if (graph && x.requires_grad() && dt == CLB_F32 && out) { // the backward takes both gradients in one pass
             plan = logic_plan_for(start_obj, a, b, start, cons, in, out);
-            coef = alloc({out, 4}, x);
+            if (plan) coef = alloc({out, 4}, x);
         }
         if (batch && out)
             check(clb_logic_fwd_coef(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(y), ptr(coef), in, out, batch, wmode, dt, cur_stream()));

@@ -166,3 +166,24 @@ def test_saved_tensor_hooks_see_what_a_call_keeps():
         assert extra is None or extra in kept, (name, kept)
         with pytest.raises(RuntimeError, match="second time"):
             torch.autograd.grad(y.sum(), _weights(m))
+
+
+def test_the_first_step_of_a_flat_layer_may_be_captured():
+    m, x = _flat()
+    want = _step(_flat()[0], x)
+    x.requires_grad_(True)
+    go = torch.ones(33, 96, device="cuda")
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = m(x)
+        g = torch.autograd.grad(y, [x, m.weights], go)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want[0])
+    # The separate kernels add in another order.  A basis sum has 33 terms of at most 1: any two orders agree to 2 * 32 * 33 * 2^-24 = 1.3e-4,
+    # and a gate gradient, p (g - sum p g) with g of up to four basis sums, to 8 times that; in practice 2e-6.
+    for a, b in zip(g, want[1:]):
+        assert (a - b).abs().max() < 1e-3 and (a - b).norm() < 1e-5 * b.norm()
+    again = _step(m, x)                                  # and the layer lays its lists out afterwards
+    assert all(torch.equal(a, b) for a, b in zip(again, want))
