@@ -709,6 +709,7 @@ Tensor group_sum_bwd(const Tensor &gout, int64_t f, int k, double tau, const Ten
 // y: [B, F] on feature-major storage
 Tensor group_sum_fwd(const Tensor &y, int k, double tau)
 {
+    TORCH_CHECK_VALUE(k > 0, "the number of classes has to be positive, got ", k);
     TORCH_CHECK(y.is_cuda() && stored_feature_major(y), "convlogic_b200: class sums are taken from a flat layer's output");
     const int64_t f = y.size(1), b = y.size(0);
     const int dt = dtype_code(y);
@@ -787,6 +788,7 @@ struct GroupSumCeNode : public Node {
 
 Tensor group_sum_ce(const Tensor &x, const Tensor &labels, int k, double tau)
 {
+    TORCH_CHECK_VALUE(k > 0, "the number of classes has to be positive, got ", k);
     if (followed({x})) return in_python("followed_group_sum_ce", x, labels, k, tau).cast<Tensor>();
     Tensor loss, dscore;
     {
@@ -968,6 +970,7 @@ Tensor packed_logic(const Tensor &x, const Tensor &a, const Tensor &b, const Ten
 
 Tensor group_popcount(const Tensor &x, int64_t pad, int k)
 {
+    TORCH_CHECK_VALUE(k > 0, "the number of classes has to be positive, got ", k);
     need_input(x);
     const int64_t f = x.size(0), words = x.size(1), bits = x.element_size() * 8;
     TORCH_CHECK_VALUE(f % k == 0, "in_dim (", f, ") has to be divisible by k (", k, ") but it is not");

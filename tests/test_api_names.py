@@ -1,5 +1,6 @@
-"""The function-level interface: names that callers of ``ops`` and ``functional`` use, and the Functions as torch Functions."""
+"""The function-level interface on the host: names that callers of ``ops`` and ``functional`` use, and the Functions as torch Functions."""
 
+import pytest
 import torch
 
 
@@ -15,3 +16,17 @@ def test_functions_and_ops():
                  "pack_bits", "packed_logic", "group_popcount", "packed_convtree", "packed_convtree_slab", "thermometer_pack", "group_sum_fwd",
                  "group_sum_bwd", "group_sum_ce", "logic_tree_fwd", "logic_tree_bwd", "logic_tree_fwd_ce", "transpose2d", "adam_step"):
         assert callable(getattr(ops, name)), name
+
+
+@pytest.mark.parametrize("k", [0, -4])
+def test_class_counts_that_are_not_positive_raise(k):
+    """k = 0 was an integer division by zero in C++, which ends the process."""
+    from convlogic_b200 import _lib, ops
+
+    with pytest.raises(ValueError, match="positive"):
+        ops.group_popcount(torch.zeros(4, 2, dtype=torch.int32), 0, k)
+    with pytest.raises(ValueError, match="positive"):
+        _lib.native().group_sum_ce(torch.zeros(3, 8), torch.zeros(3, dtype=torch.int64), k, 1.0)
+    lib = _lib.lib()
+    assert lib.clb_group_sum_scratch_bytes(8, 4, k, 0) == 0   # the C interface takes no such count either
+    assert lib.clb_group_popcount(1 << 20, 1 << 20, 8, 2, 32, 0, k, None) == -1   # before any pointer is looked at
