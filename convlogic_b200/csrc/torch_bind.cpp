@@ -311,7 +311,7 @@ template <typename Plan> std::shared_ptr<Plan> kept(const py::handle &tensor) //
 
 PlanPtr plan_for(const py::handle &sel_obj, const Tensor &sel, const Geom &g, int64_t ci) // GIL held
 {
-    const int64_t version = sel.is_inference() ? 0 : (int64_t)sel._version();
+    const int64_t version = (int64_t)sel._version(); // raises for a tensor made in inference mode: nothing would tell that it has changed
     if (PlanPtr p = kept<BlockPlan>(sel_obj); p && p->version == version && p->data == sel.data_ptr() && p->g == g && p->ci == ci) return p;
     auto p = std::make_shared<BlockPlan>();
     p->g = g, p->C = (int)sel.size(0), p->ci = (int)ci, p->version = version, p->data = sel.data_ptr(), p->device = sel.device();
@@ -457,7 +457,7 @@ struct BlockNode : public Node {
     variable_list apply(variable_list &&grads) override
     {
         const Tensor xx = x.unpack(), ww = w.unpack(), best = amax.unpack(), &ss = sel;
-        TORCH_CHECK(ss.is_inference() || plan->version == (int64_t)ss._version(), "convlogic_b200: the selection was modified between forward and backward");
+        TORCH_CHECK(plan->version == (int64_t)ss._version(), "convlogic_b200: the selection was modified between forward and backward");
         const bool need_gx = task_should_compute_output(0), need_gw = task_should_compute_output(1) && wmode != CLB_W_ARGMAX;
         if (!need_gx && !need_gw) return {Tensor(), Tensor()};
         Tensor gy = upstream(*this, grads);
@@ -518,7 +518,7 @@ LogicDims logic_dims(const Tensor &x_fm, const Tensor &a, const Tensor &b, const
 using LogicKey = std::array<std::pair<const void *, int64_t>, 4>; // a, b, start, consumers: address and version
 LogicKey logic_key(const Tensor &a, const Tensor &b, const Tensor &start, const Tensor &cons)
 {
-    auto id = [](const Tensor &t) { return std::make_pair((const void *)t.data_ptr(), t.is_inference() ? (int64_t)0 : (int64_t)t._version()); };
+    auto id = [](const Tensor &t) { return std::make_pair((const void *)t.data_ptr(), (int64_t)t._version()); };
     return {id(a), id(b), id(start), id(cons)};
 }
 struct LogicPlan {

@@ -187,3 +187,17 @@ def test_the_first_step_of_a_flat_layer_may_be_captured():
         assert (a - b).abs().max() < 1e-3 and (a - b).norm() < 1e-5 * b.norm()
     again = _step(m, x)                                  # and the layer lays its lists out afterwards
     assert all(torch.equal(a, b) for a, b in zip(again, want))
+
+
+def test_connections_made_in_inference_mode_get_no_plan():
+    """Such a tensor has no version, so a plan of it could not be told from an outdated one."""
+    with torch.inference_mode():
+        flat, x = _flat()
+        assert flat(x).shape == (33, 96)      # no plan needed
+        block, img = _block()
+        with pytest.raises(RuntimeError, match="[Ii]nference"):
+            block(img)
+    flat.weights = torch.nn.Parameter(flat.weights.clone())
+    x = x.clone().requires_grad_(True)
+    with pytest.raises(RuntimeError, match="[Ii]nference"):
+        flat(x)
