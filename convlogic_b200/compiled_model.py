@@ -188,7 +188,7 @@ class CompiledLogicNet(torch.nn.Module):
         net = self._handle()
         pixels = thresholds is not None
         static_in = example.to(self.device).contiguous().clone()
-        th = thresholds.to(self.device, torch.float32).contiguous() if pixels else None
+        th = thresholds.to(self.device, torch.float32).contiguous().clone() if pixels else None
         if not pixels:
             static_in = static_in.reshape(static_in.shape[0], -1).contiguous().view(torch.uint8)
         batch = static_in.shape[0]
@@ -209,6 +209,7 @@ class CompiledLogicNet(torch.nn.Module):
             graph.replay()
             return static_out
 
+        replay.reads = (net, th)  # the graph knows only the addresses of the parameters and thresholds: they live as long as it does
         return replay
 
     def forward(self, x, verbose=False):

@@ -174,3 +174,22 @@ def test_packed_rows_input(batch):
     assert torch.equal(net.forward_packed(torch.from_numpy(padded), batch), net(x))
     with pytest.raises(ValueError):
         net.forward_packed(torch.from_numpy(padded[:, :1].copy()), batch)
+
+
+@pytest.mark.parametrize("pixels", [False, True])
+def test_replay_keeps_what_the_graph_reads(pixels):
+    import convlogic_b200 as cb
+
+    torch.manual_seed(0)
+    model = cb.ConvLogicCifarModel(k_param=2, input_channels=6, input_size=32, tau=8.0).cuda().eval()
+    _randomise(model, 1)
+    net = cb.CompiledLogicNet(model.network, input_shape=(6, 32, 32)).compile()
+    th = torch.tensor([0.3, 0.6], dtype=torch.float64)   # capture() makes the device copy
+    x = torch.rand(40, 3, 32, 32, device="cuda") if pixels else torch.rand(40, 6, 32, 32, device="cuda") < 0.5
+    replay = net.capture(x, th if pixels else None)
+    want = net.forward_pixels(x, th) if pixels else net(x)
+    net.compile()                                        # another handle; the captured one belongs to the graph now
+    fill = [torch.full((n,), 0.99, device="cuda") for n in (2, 2, 64, 64, 4096, 4096, 1 << 20) for _ in range(8)]
+    torch.cuda.synchronize()
+    assert torch.equal(replay(x), want)
+    del fill
