@@ -146,16 +146,17 @@ bool stored_feature_major(const Tensor &x)
 // a tensor whose storage is [F, B], from a [B, F] activation (x itself where possible; the shape of the result is not to be used)
 Tensor feature_major_storage(const Tensor &x) { return stored_feature_major(x) ? x : transposed_copy(x); }
 
-// A [B, F] gradient of feature-major storage: made in that form, or, for a leaf that stores [B, F], turned round at the end.
+// A [B, F] gradient of feature-major storage: made in that form, and turned round at the end for a leaf that stores [B, F] itself (`.grad`
+// takes the leaf's strides).
 Tensor feature_major_grad(int64_t batch, int64_t features, const Tensor &like)
 {
     return alloc_strided({batch, features}, {1, std::max<int64_t>(batch, 1)}, like);
 }
-Tensor finished_grad(const Tensor &g, bool leaf) { return leaf && !g.is_contiguous() ? transposed_copy(g.t()) : g; }
-bool feeds_leaf(const Node &n, size_t i)
+Tensor finished_grad(const Tensor &g, const Node &n) // of the node's first input
 {
-    const auto &e = n.next_edge(i);
-    return e.function && dynamic_cast<torch::autograd::AccumulateGrad *>(e.function.get()) != nullptr;
+    if (g.is_contiguous()) return g;
+    const auto *leaf = dynamic_cast<const torch::autograd::AccumulateGrad *>(n.next_edge(0).function.get());
+    return leaf && !stored_feature_major(leaf->variable) ? transposed_copy(g.t()) : g;
 }
 
 // ------------------------------------------------------------------------------------------------ gradient sinks
@@ -635,7 +636,7 @@ struct LogicNode : public Node {
             if (rc == CLB_ERR_SHAPE && need_gw)
                 check(clb_logic_bwd_w(ptr(xx), ptr<int64_t>(a), ptr<int64_t>(b), ptr(ww), ptr(gy), ptr(gw), in, out, batch, wmode, dt, cur_stream()));
         }
-        if (gx.defined() && !fm) gx = finished_grad(gx, feeds_leaf(*this, 0));
+        if (gx.defined() && !fm) gx = finished_grad(gx, *this);
         if (sinks.any()) {
             sinks.ready();
             gw = Tensor();
@@ -730,7 +731,7 @@ struct GroupSumNode : public Node {
     {
         const Tensor gout = upstream(*this, grads);
         Below below(gout);
-        return {finished_grad(group_sum_bwd(gout.contiguous(), f, k, tau, Tensor()), feeds_leaf(*this, 0))};
+        return {finished_grad(group_sum_bwd(gout.contiguous(), f, k, tau, Tensor()), *this)};
     }
 };
 
@@ -782,7 +783,7 @@ struct GroupSumCeNode : public Node {
         const Tensor ds = dscore.unpack();
         Below below(ds);
         const Tensor scale = upstream(*this, grads).reshape({1}).to(ds.scalar_type()).contiguous();
-        return {finished_grad(group_sum_bwd(ds, f, k, tau, scale), feeds_leaf(*this, 0))};
+        return {finished_grad(group_sum_bwd(ds, f, k, tau, scale), *this)};
     }
 };
 
@@ -868,7 +869,7 @@ struct TreeNode : public Node {
         const bool direct = sinks.any() && wmode != CLB_W_ARGMAX;
         auto out = tree_bwd(xx, in, batch, t, a, b, c, gy, k ? dscore.unpack() : Tensor(), scale, k, tau, wmode, task_should_compute_output(0),
                             direct ? std::array<Tensor, 3>{sinks.slice(0), sinks.slice(1), sinks.slice(2)} : std::array<Tensor, 3>{});
-        Tensor gx = out[0].defined() ? finished_grad(out[0], feeds_leaf(*this, 0)) : Tensor();
+        Tensor gx = out[0].defined() ? finished_grad(out[0], *this) : Tensor();
         if (direct) sinks.ready();
         if (direct || wmode == CLB_W_ARGMAX) return {gx, Tensor(), Tensor(), Tensor()};
         return {gx, out[1], out[2], out[3]};

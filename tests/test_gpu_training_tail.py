@@ -199,3 +199,25 @@ def test_fused_layers_with_the_loss_head_equal_the_separate_modules(dims, batch)
         assert abs(float(a[0]) - float(b[0])) <= 1e-6 * abs(float(a[0]))
         for i, (u, v) in enumerate(zip(a[1:], b[1:])):
             assert_close(v, u, 1e-5, f"gradient {i}")
+
+
+@pytest.mark.parametrize("feature_major", [True, False])
+def test_gradient_of_a_leaf_comes_in_its_own_layout(feature_major):
+    """A transposed copy only for a leaf that is stored sample by sample."""
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    torch.manual_seed(0)
+    layer = cb.LogicLayer(96, 120).cuda().train()
+    values, go = torch.rand(37, 96, device="cuda"), torch.rand(37, 120, device="cuda")
+    modules = [(layer, go)] + ([(cb.GroupSum(4, 2.0), go[:, :4].contiguous())] if feature_major else [])
+    for module, upstream in modules:
+        leaf = (values.t().contiguous().t() if feature_major else values.clone()).requires_grad_(True)
+        y = module(leaf)
+        _lib.trace(True)
+        y.backward(upstream.t().contiguous().t() if module is layer else upstream)
+        torch.cuda.synchronize()
+        names = _lib.trace_report()
+        _lib.trace(False)
+        assert leaf.grad.stride() == leaf.stride()
+        assert ("transpose_f32_kernel" in names) == (not feature_major), names
