@@ -866,7 +866,8 @@ extern "C" int clb_convtree_fwd(const void *x, const void *w, const int32_t *sel
 {
     const bool sel_unbounded = (wmode & CLB_SEL_UNBOUNDED) != 0;
     const bool y_fm = (wmode & CLB_Y_FEATURE_MAJOR) != 0;
-    wmode &= ~(CLB_SEL_UNBOUNDED | CLB_Y_FEATURE_MAJOR);
+    const int sel_many = wmode & CLB_SEL_MANY;
+    wmode &= ~(CLB_SEL_UNBOUNDED | CLB_Y_FEATURE_MAJOR | CLB_SEL_MANY);
     ConvShape s;
     int rc = make_shape(s, N, Ci, H, W, C, sh, sw, ph, pw, kh, kw, true);
     if (rc) return rc;
@@ -875,13 +876,13 @@ extern "C" int clb_convtree_fwd(const void *x, const void *w, const int32_t *sel
     if (C > 65535) return CLB_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
     if (y_fm) { // feature-major output: the plane kernels or nothing
-        if (dtype != CLB_F32 || x2 || idx || sel_unbounded) return CLB_ERR_SHAPE;
+        if (dtype != CLB_F32 || x2 || idx || sel_unbounded || (sel_many && Ci < 16)) return CLB_ERR_SHAPE;
         return clb_convtree_fwd_plane_f32((const float *)x, (const float *)w, sel, (float *)y, amax, N, Ci, H, W, C, sh, sw, ph, pw, kh, kw,
                                           wmode | CLB_Y_FEATURE_MAJOR, st);
     }
     if (dtype == CLB_F32 && !x2 && !idx && !sel_unbounded) {
         rc = clb_convtree_fwd_fast_f32((const float *)x, (const float *)w, sel, (float *)y, amax, N, Ci, H, W, C, sh, sw, ph, pw,
-                                       kh, kw, wmode, st);
+                                       kh, kw, wmode | sel_many, st);
         if (rc != CLB_ERR_SHAPE) return rc;
     }
     const long long total = (long long)N * (s.Ho / 2) * (s.Wo / 2);

@@ -1254,9 +1254,14 @@ int clb_convtree_fwd_fast_f32(const float *x, const float *w, const int32_t *sel
     // 24.8 against 32.3; 32 -> 128, batch 100: 13.3 against 35.6; 16 -> 1024, 4x4, batch 500: 38 against 85).  Images of 28 and 32
     // pixels have enough windows always (9 -> 256, 32x32, batch 256: 102 against 132; 1 -> 16, 28x28, batch 8: 4.9 and 4.9); 6x6
     // suits the tiled kernels badly (24 -> 72, batch 200: 7.6 against 70); images of 12 from eight channels on (512 out, batch 400:
-    // with 16 channels 88 against 105, with 5 94 against 83).
+    // with 16 channels 88 against 105, with 5 94 against 83).  An output channel that reads more than two channels takes every tap from
+    // global memory in the plane kernels: with few input channels the tiled ones then win (eight channels a selection: 9 -> 256, 32x32,
+    // batch 64: 46 against 164; 4 -> 64, 16x16, batch 256: 19 against 36; but 24 -> 64, 28x28, batch 32: 35 against 21, 24 -> 72, 6x6: 39
+    // against 10).
+    const bool sel_many = (wmode & CLB_SEL_MANY) != 0;
+    wmode &= ~CLB_SEL_MANY;
     const bool many_channels = (size_t)Ci * (H + 2 * ph) * (W + 2 * pw) * 4 > 48 * 1024;
-    if (many_channels || Ci >= 16 || H >= 28 || H == 6 || (H == 12 && Ci >= 8) || (H != 12 && (long long)N * C * H * W >= (4LL << 20))) {
+    if (many_channels || Ci >= 16 || H == 6 || (!sel_many && (H >= 28 || (H == 12 && Ci >= 8) || (H != 12 && (long long)N * C * H * W >= (4LL << 20))))) {
         const int rc = clb_convtree_fwd_plane_f32(x, w, sel, y, amax, N, Ci, H, W, C, sh, sw, ph, pw, kh, kw, wmode, st);
         if (rc != CLB_ERR_SHAPE) return rc;
     }

@@ -242,6 +242,7 @@ struct BlockPlan {
     int64_t version;
     const void *data;
     int flag;                        // CLB_SEL_UNBOUNDED when a tap lies outside the window
+    int many;                        // CLB_SEL_MANY when an output channel reads more than two input channels
     bool channels_ok;
     std::vector<int32_t> sel;        // host copy
     std::mutex mu;
@@ -318,12 +319,20 @@ PlanPtr plan_for(const py::handle &sel_obj, const Tensor &sel, const Geom &g, in
     p->g = g, p->C = (int)sel.size(0), p->ci = (int)ci, p->version = version, p->data = sel.data_ptr(), p->device = sel.device();
     const Tensor host = sel.detach().to(at::kCPU).contiguous();
     p->sel.assign(host.data_ptr<int32_t>(), host.data_ptr<int32_t>() + host.numel());
-    bool inside = true, channels = true;
-    for (const int32_t word : p->sel) {
-        inside = inside && ((word >> 8) & 0xFF) < g.kh && (word & 0xFF) < g.kw;
-        channels = channels && word >= 0 && ((word >> 16) & 0xFFFF) < ci;
+    bool inside = true, channels = true, two = true;
+    for (size_t c = 0; c < p->sel.size(); c += 8) {
+        int first = -1, second = -1;
+        for (size_t k = c; k < c + 8; ++k) {
+            const int32_t word = p->sel[k];
+            const int ch = (word >> 16) & 0xFFFF;
+            inside = inside && ((word >> 8) & 0xFF) < g.kh && (word & 0xFF) < g.kw;
+            channels = channels && word >= 0 && ch < ci;
+            if (first < 0) first = ch;
+            else if (ch != first && second < 0) second = ch;
+            two = two && (ch == first || ch == second);
+        }
     }
-    p->flag = inside ? 0 : CLB_SEL_UNBOUNDED, p->channels_ok = channels;
+    p->flag = inside ? 0 : CLB_SEL_UNBOUNDED, p->many = two ? 0 : CLB_SEL_MANY, p->channels_ok = channels;
     sel_obj.attr("_clb_plan") = p;
     return p;
 }
@@ -380,7 +389,7 @@ BlockOut block_fwd(const Tensor &x, const Tensor &w, const Tensor &sel, const Ge
         // the flat layers' layout, storage [C, h, w, N]; only the plane kernels write it
         o.y = alloc_strided({d.n, d.c, hp, wp}, {1, (int64_t)hp * wp * d.n, (int64_t)wp * d.n, d.n}, x);
         const int rc = clb_convtree_fwd(ptr(x), ptr(w), ptr<int32_t>(sel), ptr(o.y), ptr<uint8_t>(o.amax), nullptr, nullptr, nullptr, d.n, d.ci, d.h, d.w,
-                                        d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, wmode | CLB_Y_FEATURE_MAJOR, dt, cur_stream());
+                                        d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, wmode | CLB_Y_FEATURE_MAJOR | plan->many, dt, cur_stream());
         if (rc != CLB_ERR_SHAPE) {
             check(rc);
             return o;
@@ -388,7 +397,7 @@ BlockOut block_fwd(const Tensor &x, const Tensor &w, const Tensor &sel, const Ge
     }
     o.y = alloc({d.n, d.c, hp, wp}, x);
     check(clb_convtree_fwd(ptr(x), ptr(w), ptr<int32_t>(sel), ptr(o.y), ptr<uint8_t>(o.amax), ptr(o.x2), ptr(o.x3), ptr<int32_t>(o.idx), d.n, d.ci, d.h,
-                           d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, wmode | plan->flag, dt, cur_stream()));
+                           d.w, d.c, g.sh, g.sw, g.ph, g.pw, g.kh, g.kw, wmode | plan->flag | plan->many, dt, cur_stream()));
     return o;
 }
 

@@ -33,3 +33,25 @@ def test_plane_forward_sides(n, ci, c, side, spread):
     assert torch.equal(y, want) and torch.equal(amax, amax_want)
     fm = ops.convtree_fwd(x, w, sel, GEOM, W_SOFTMAX, y_feature_major=True)[0]
     assert torch.equal(fm, want)
+
+
+@pytest.mark.parametrize("n,ci,c,side,plane", [(9, 9, 12, 32, False), (17, 5, 8, 28, False), (300, 8, 70, 12, False), (300, 4, 64, 16, False),
+                                               (9, 18, 12, 32, True), (40, 8, 9, 6, True), (9, 15, 5, 28, True)])
+def test_selections_on_many_channels_take_the_tiled_kernels_while_there_are_few(n, ci, c, side, plane):
+    from convlogic_b200 import _lib, ops
+    from convlogic_b200._lib import W_SOFTMAX
+
+    torch.manual_seed(n + side)
+    ch = torch.randint(0, ci, (c, 8))
+    ch[:, :3] = torch.tensor([0, 1, 2])
+    sel = ((ch << 16) | (torch.randint(0, 3, (c, 8)) << 8) | torch.randint(0, 3, (c, 8))).int().cuda()
+    x, w = torch.rand(n, ci, side, side, device="cuda"), torch.randn(c, 7, 16, device="cuda")
+    want, amax_want, _, _, _ = ops.convtree_fwd(x, w, sel, GEOM, W_SOFTMAX, want_indices=True)
+    _lib.trace(True)
+    y, amax, _, _, _ = ops.convtree_fwd(x, w, sel, GEOM, W_SOFTMAX)
+    torch.cuda.synchronize()
+    rep = _lib.trace_report()
+    _lib.trace(False)
+    assert ("convtree_fwd_plane_kernel" in rep) == plane, rep
+    assert torch.equal(y, want) and torch.equal(amax, amax_want)
+    assert torch.equal(ops.convtree_fwd(x, w, sel, GEOM, W_SOFTMAX, y_feature_major=True)[0], want)
