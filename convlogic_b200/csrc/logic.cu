@@ -267,7 +267,6 @@ __global__ void __launch_bounds__(256) group_sum_partial_kernel(const T *__restr
     const long long r0 = S * part / gridDim.z, r1 = S * (part + 1) / gridDim.z;
     T acc = T(0);
     if (b < B)
-#pragma unroll 8
         for (long long r = r0 + wv; r < r1; r += 8) acc += y[((long long)c * S + r) * B + b];
     red[wv][lane] = acc;
     __syncthreads();
@@ -279,7 +278,7 @@ __global__ void __launch_bounds__(256) group_sum_partial_kernel(const T *__restr
     }
 }
 
-// Few rows: block (batch tile, class), two warps to a part and four chains to a warp, and no second launch.
+// Few rows and blocks (clb_group_sum_fwd): block (batch tile, class), two warps to a part and four chains to a warp, and no second launch.
 template <typename T>
 __global__ void __launch_bounds__(1024) group_sum_one_kernel(const T *__restrict__ y, T *__restrict__ out, long long S, long long B, int k, int parts, T tau)
 {
@@ -993,9 +992,15 @@ extern "C" int clb_group_sum_fwd(const void *y, void *out, void *scratch, size_t
     cudaStream_t st = (cudaStream_t)stream;
     dim3 grid((unsigned)((B + 31) / 32), (unsigned)k, (unsigned)parts);
     const int fb = (int)((B * k + 255) / 256);
+    // One launch while a block is short and there are few of them.  Sixteen parts: up to 1024 rows in at most two blocks per SM, else up to
+    // 448 (us with one launch / two; 500 rows, 2000 samples, 2 classes 4.3 / 8.6; 2000 rows, 512 x 10 11.8 / 11.1; 400 rows, 4096 x 10 28
+    // / 37; 512 rows, 2000 x 80 154 / 134).  One part, which two of the 32 warps add up: below 64 rows in at most a block per SM
+    // (40 rows, 100 x 10 3.1 / 3.8, 944 x 10 6.8 / 4.4; 100 rows, 20001 x 10 201 / 20; 2 rows, 512 x 1000 133 / 24).
+    const long long blocks = (B + 31) / 32 * k;
+    const bool one = parts > 1 ? S <= (blocks <= 2LL * sm_count() ? 1024 : 448) : S < 64 && blocks <= sm_count();
     auto go = [&](auto t) {
         using T = decltype(t);
-        if (S <= 4096) { // 128 rows per warp at most: about what a second launch costs
+        if (one) {
             grid.z = 1;
             CLB_TRACED("group_sum_one_kernel", st, group_sum_one_kernel<T><<<grid, 1024, 0, st>>>((const T *)y, (T *)out, S, B, k, parts, (T)tau));
             return 1;

@@ -221,3 +221,21 @@ def test_gradient_of_a_leaf_comes_in_its_own_layout(feature_major):
         _lib.trace(False)
         assert leaf.grad.stride() == leaf.stride()
         assert ("transpose_f32_kernel" in names) == (not feature_major), names
+
+
+@pytest.mark.parametrize("rows,batch,k,launches", [(63, 33, 10, 1), (64, 33, 10, 2), (20, 2000, 10, 2), (128, 2000, 10, 1), (448, 2000, 10, 1), (449, 2000, 10, 2),
+                                                   (1024, 100, 10, 1), (1025, 100, 10, 2), (2, 33, 100, 2)])
+def test_group_sum_on_both_sides_of_its_lines(rows, batch, k, launches):
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    y = torch.rand(rows * k, batch, device="cuda").t()
+    with torch.no_grad():
+        _lib.trace(True)
+        got = cb.GroupSum(k, 3.0)(y)
+        torch.cuda.synchronize()
+        names = _lib.trace_report()
+        _lib.trace(False)
+    assert len(names) == launches, names
+    want = y.double().reshape(batch, k, rows).sum(-1) / 3.0
+    assert (got - want).abs().max() <= rows / 3.0 * 2.0 ** -24 * (rows / 8 + 24)   # chains of an eighth of the rows at most, 24 further additions
