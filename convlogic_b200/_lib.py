@@ -66,6 +66,7 @@ _SIGNATURES = {
     "clb_tree_bwd_w": ([_vp] * 5 + [_sz] + [_i] * 6 + [_vp], _i),
     "clb_logic_fwd": ([_vp] * 5 + [_i64] * 3 + [_i, _i, _vp], _i),
     "clb_logic_fwd_coef": ([_vp] * 6 + [_i64] * 3 + [_i, _i, _vp], _i),
+    "clb_logic_fwd_scratch_bytes": ([_i64] * 3 + [_i], _sz),
     "clb_logic_entries": ([_vp] * 6 + [_i64] * 2 + [_vp], _i),
     "clb_logic_bwd_scratch_bytes": ([_i64] * 3, _sz),
     "clb_logic_bwd": ([_vp] * 9 + [_sz] + [_i64] * 3 + [_i, _vp], _i),

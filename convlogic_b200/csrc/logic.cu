@@ -864,6 +864,25 @@ static int logic_grid(long long units_of_warps, int per = 32)
 int clb_logic_fwd_cols(const float *x, const int64_t *a, const int64_t *b, const float *w, float *y, float *coef, int64_t out_dim, int64_t B, int wmode,
                        cudaStream_t st); // logic_bwd.cu
 
+// When the forward of a layer walks its rows in stretches of 64 samples (logic_fwd_cols_kernel).  The input has to be beyond half the L2
+// (us without / with; 48 MB 18.4 / 18.5, 80 MB 36 / 32, 262144 x 1024 480 / 451, 65536 x 4096 480 / 422), a stretch worth the walk
+// (196608 x 64 29 / 30, 131072 x 256 59 / 58, 87381 x 384 58 / 51) and nearly all of them whole (264 samples 129 / 175, 520 127 / 138, 1032
+// 126 / 107), and its rows made of whole sectors unless they are long (500 samples 123 / 150, 1020 123 / 115, 2052 128 / 107).  A layer with
+// fewer outputs than inputs reads a row once at most and gains nothing (200000 -> 100000, 512 samples 96 / 106); just above half the
+// L2 the two are level there (66000 -> 33001, 260 samples 17 / 15, 57671 -> 28835, 300 15 / 16, 16962 -> 8481, 1020 14 / 16).
+static bool cols_pay(int64_t in_dim, int64_t out_dim, int64_t B)
+{
+    const int64_t bytes = in_dim * B * 4;
+    if (B < 256 || B > 4000000 || B % 4 || in_dim > 0x3fffffff || out_dim > 0x3fffffff || bytes <= (64LL << 20)) return false;
+    if (out_dim < in_dim) return bytes <= (72LL << 20);
+    return (B % 8 == 0 || B >= 1000) && 12 * ((B + 63) / 64 * 64) <= 13 * B;
+}
+
+extern "C" size_t clb_logic_fwd_scratch_bytes(int64_t in_dim, int64_t out_dim, int64_t B, int dtype)
+{
+    return dtype == CLB_F32 && in_dim > 0 && out_dim > 0 && B > 0 && cols_pay(in_dim, out_dim, B) ? (size_t)out_dim * 16 : 0;
+}
+
 extern "C" int clb_logic_fwd(const void *x, const int64_t *a, const int64_t *b, const void *w, void *y, int64_t in_dim,
                              int64_t out_dim, int64_t B, int wmode, int dtype, void *stream)
 {
@@ -876,11 +895,14 @@ extern "C" int clb_logic_fwd_coef(const void *x, const int64_t *a, const int64_t
     if (!x || !a || !b || !w || !y || in_dim <= 0 || out_dim < 0 || B < 0 || wmode < 0 || wmode > 2) return CLB_ERR_ARG;
     if (out_dim == 0 || B == 0) return CLB_OK;
     cudaStream_t st = (cudaStream_t)stream;
-    const int grid = logic_grid((out_dim + 1) / 2, 4);
+    // The resident blocks alone while the input is in the L2, or where the last accesses of a row leave more than a quarter of the lanes idle; for
+    // larger inputs more of them, which the SMs take up as they come (us with 4 / 32 blocks per SM: 65536 x 128 12.4 / 14.3, 109660 x 112
+    // 20.7 / 25.5; 131072 x 512 128 / 117, 262144 x 1024 525 / 480; but 258111 x 260 131 / 137).
+    const bool beyond_l2 = in_dim * B * (dtype == CLB_F64 ? 8 : 4) > (96LL << 20) && 4 * B >= 3 * ((B + 127) / 128 * 128);
+    const int grid = logic_grid((out_dim + 1) / 2, beyond_l2 ? 32 : 4);
     if (dtype == CLB_F32) {
         const bool vec = B % 4 == 0 && aligned16(x) && aligned16(y);
-        // an input beyond about half the L2 is walked in column stretches that fit it (0.44 -> 0.40 ms per 256000 x 1024 layer)
-        if (coef && vec && aligned16(coef) && aligned16(w) && B >= 256 && B <= 4000000 && in_dim * B * 4 > (64LL << 20) && in_dim <= 0x3fffffff && out_dim <= 0x3fffffff)
+        if (coef && vec && aligned16(coef) && aligned16(w) && cols_pay(in_dim, out_dim, B))
             return clb_logic_fwd_cols((const float *)x, a, b, (const float *)w, (float *)y, (float *)coef, out_dim, B, wmode, st);
         if (vec)
             CLB_TRACED("logic_fwd_kernel", st,

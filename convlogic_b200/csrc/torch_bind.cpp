@@ -560,11 +560,12 @@ LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const 
     return p;
 }
 
-void logic_fwd(const Tensor &x_fm, const Tensor &a, const Tensor &b, const Tensor &w, int wmode, const Tensor &y_storage, const Tensor &coef = Tensor())
+void logic_fwd(const Tensor &x_fm, const Tensor &a, const Tensor &b, const Tensor &w, int wmode, const Tensor &y_storage)
 {
     need_inputs(x_fm, a, b, w);
     const LogicDims d = logic_dims(x_fm, a, b, w);
     if (d.batch == 0 || d.out == 0) return;
+    const Tensor coef = clb_logic_fwd_scratch_bytes(d.in, d.out, d.batch, dtype_code(x_fm)) ? alloc({d.out, 4}, x_fm) : Tensor();
     check(clb_logic_fwd_coef(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(y_storage), ptr(coef), d.in, d.out, d.batch, wmode, dtype_code(x_fm),
                              cur_stream()));
 }
@@ -681,6 +682,7 @@ Tensor logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w_
             plan = logic_plan_for(start_obj, a, b, start, cons, in, out);
             if (plan) coef = alloc({out, 4}, x);
         }
+        if (!coef.defined() && clb_logic_fwd_scratch_bytes(in, out, batch, dt)) coef = alloc({out, 4}, x); // (then not kept)
         if (batch && out)
             check(clb_logic_fwd_coef(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(y), ptr(coef), in, out, batch, wmode, dt, cur_stream()));
     }

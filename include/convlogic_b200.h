@@ -245,7 +245,9 @@ int clb_tree_bwd_w(const void *gy, const void *x, const void *w, void *gw, void 
 int clb_logic_fwd(const void *x, const int64_t *a, const int64_t *b, const void *w, void *y, int64_t in_dim,
                   int64_t out_dim, int64_t B, int wmode, int dtype, void *stream);
 /* The same, also writing what the combined backward below reads: coef [out][4] = (k1, ka, kb, kab) of every neuron's gate,
- * y = k1 + ka*a + kb*b + kab*a*b (16-byte aligned; NULL: not written). */
+ * y = k1 + ka*a + kb*b + kab*a*b (16-byte aligned; NULL: not written).  A caller that has no backward pass to come gains by
+ * giving the memory where clb_logic_fwd_scratch_bytes (16 * out_dim, or 0) says so: large inputs are then walked in stretches. */
+size_t clb_logic_fwd_scratch_bytes(int64_t in_dim, int64_t out_dim, int64_t B, int dtype);
 int clb_logic_fwd_coef(const void *x, const int64_t *a, const int64_t *b, const void *w, void *y, void *coef, int64_t in_dim,
                        int64_t out_dim, int64_t B, int wmode, int dtype, void *stream);
 /* Both gradients of a flat layer in one pass over the rows (fp32; stands in for the pair backward_w + backward_x that the

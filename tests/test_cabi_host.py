@@ -173,3 +173,18 @@ def test_network_blob_with_an_index_out_of_range_is_rejected():
         damaged = bytearray(tb)
         struct.pack_into(fmt, damaged, off, bad)
         assert status(damaged) == _lib.ERR_SHAPE, (off, fmt, bad)
+
+
+def test_when_a_flat_forward_asks_for_memory(lib):
+    """The lines of the walk in stretches (16 bytes per neuron): half the L2, 256 samples, whole stretches, whole sectors, rows read twice."""
+    def asks(n_in, n_out, batch, dtype=0):
+        got = lib.clb_logic_fwd_scratch_bytes(n_in, n_out, batch, dtype)
+        assert got in (0, 16 * n_out)
+        return got > 0
+
+    assert asks(65537, 65537, 256) and not asks(65536, 65536, 256)
+    assert not asks(1 << 18, 1 << 18, 128) and not asks(1 << 18, 1 << 18, 252)
+    assert asks(1 << 17, 1 << 17, 512) and not asks(1 << 17, 1 << 17, 520) and not asks(1 << 17, 1 << 17, 264)
+    assert not asks(1 << 17, 1 << 17, 500) and asks(1 << 16, 1 << 16, 1020) and not asks(1 << 16, 1 << 16, 1022)
+    assert not asks(200000, 199999, 512) and asks(66000, 33001, 260) and not asks(80000, 40000, 260) and asks(200000, 200000, 512)
+    assert not asks(1 << 17, 1 << 17, 512, 1) and not asks(0, 5, 512) and not asks(5, 0, 512)

@@ -69,3 +69,34 @@ def oracle_gates(a, b):
     terms = [(0, 0, 0, 0), (0, 0, 0, 1), (0, 1, 0, -1), (0, 1, 0, 0), (0, 0, 1, -1), (0, 0, 1, 0), (0, 1, 1, -2), (0, 1, 1, -1)]
     half = [k * one + p * a + q * b + r * ab for k, p, q, r in terms]
     return half + [one - g for g in reversed(half)]
+
+
+@pytest.mark.parametrize("n_in,n_out,batch,walk", [(66000, 66002, 256, True), (33000, 33300, 520, False), (75000, 65000, 256, False), (17000, 17008, 1004, True),
+                                                   (35000, 35007, 500, False)])
+@pytest.mark.parametrize("train", [False, True])
+def test_large_forwards_without_a_gradient(n_in, n_out, batch, walk, train):
+    """The walk in stretches is chosen by the layer's size, not by whether a gradient follows; both against the gate polynomial in 64 bits."""
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    torch.manual_seed(batch)
+    layer = cb.LogicLayer(n_in, n_out).cuda().train(train)
+    layer.weights.data.normal_()
+    x = torch.rand(n_in, batch, device="cuda").t()
+    assert (_lib.lib().clb_logic_fwd_scratch_bytes(n_in, n_out, batch, 0) > 0) == walk
+    with torch.no_grad():
+        _lib.trace(True)
+        y = layer(x)
+        torch.cuda.synchronize()
+        names = _lib.trace_report()
+        _lib.trace(False)
+    assert ("logic_fwd_cols_kernel" in names) == walk, names
+    pick = torch.randint(0, n_out, (500,), device="cuda")
+    p = layer.weights[pick].detach().double()
+    p = p.softmax(-1) if train else torch.nn.functional.one_hot(p.argmax(-1), 16).double()
+    a, b = (x[:, i[pick]].double() for i in (layer.indices_0, layer.indices_1))
+    want = torch.zeros(batch, 500, device="cuda", dtype=torch.float64)
+    for g in range(16):
+        f00, f01, f10, f11 = ((g >> s) & 1 for s in (3, 2, 1, 0))
+        want += p[:, g] * (f00 * (1 - a) * (1 - b) + f01 * (1 - a) * b + f10 * a * (1 - b) + f11 * a * b)
+    assert (y[:, pick] - want).abs().max() <= 64 * 2.0 ** -24   # 16 weights, four coefficients of up to 16 of them, three multiply-adds
