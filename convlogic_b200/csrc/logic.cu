@@ -936,7 +936,11 @@ extern "C" int clb_logic_bwd_w(const void *x, const int64_t *a, const int64_t *b
         else
             CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<float, 1, 8><<<grid, 256, 0, st>>>((const float *)x, a, b, (const float *)w, (const float *)gy, (float *)gw, out_dim, B, wmode));
     } else if (dtype == CLB_F64) {
-        CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<double, 1, 2><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (const double *)gy, (double *)gw, out_dim, B, wmode));
+        // four accesses in flight once a row fills them (us with two / four: 64000 x 512 144 / 117, 64000 x 128 41 / 32, 64000 x 32 18 / 21)
+        if (B >= 64)
+            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<double, 1, 4><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (const double *)gy, (double *)gw, out_dim, B, wmode));
+        else
+            CLB_TRACED("logic_bwd_w_kernel", st, logic_bwd_w_kernel<double, 1, 2><<<grid, 256, 0, st>>>((const double *)x, a, b, (const double *)w, (const double *)gy, (double *)gw, out_dim, B, wmode));
     } else
         return CLB_ERR_ARG;
     return check_launch();
