@@ -289,6 +289,29 @@ static BwdCut bwd_cut(int64_t in_dim, int64_t out_dim, int64_t B)
     return c;
 }
 
+// Is the combined pass the faster way?  us with it / with the two separate kernels, fp32.
+// Both gradients: yes (64000 x 1024 199 / 329, 8000 x 100 10 / 29, 64000 -> 512000 x 256 377 / 523), but for inputs of a few MB in 32-sample
+// stretches, where the separate kernels' second reading costs nothing and the stretches' sums do (1000 x 1024 15 / 11, 1000 -> 256000
+// x 512 473 / 419, 2000 x 512 12 / 10; 4000 x 512 24 / 27, 300 -> 76800 x 1024 249 / 364), and for neurons that read a feature once
+// each, far beyond the L2, in rows that are not whole stretches (200000 -> 100000, 1000 samples 677 / 605, 300 228 / 218; 1024 544 / 580,
+// 64000 -> 32000 x 1000 173 / 203).
+// The input gradient alone (no rows are saved by combining): while the input is in the L2 or little beyond and lists are short, where the soft-max of
+// every consumer that it saves is most of the work (64000 x 128 17 / 72, 8000 -> 64000 x 256 32 / 39; 8000 -> 256000 x 512 253 / 227, 64000
+// -> 256000 x 1024 870 / 636); beyond, where features have one to four readers and rows are whole sectors (200000 x 512 314 / 334, 64000
+// x 1024 167 / 214; 200000 x 1000 781 / 683, 200000 -> 100000 x 512 236 / 202); unaligned rows, which the separate kernel reads a float at
+// a time (64000 x 511 121 / 172; 200000 -> 100000 368 / 321).
+static bool combined_pays(int64_t in_dim, int64_t out_dim, int64_t B, bool gates)
+{
+    const int64_t bytes = in_dim * B * 4, reads = 2 * out_dim;
+    const bool wide = bwd_cut(in_dim, out_dim, B).wide, few = 4 * out_dim < 3 * in_dim && in_dim >= 131072;
+    if (B % 4 == 0 && !wide && B >= 512 && bytes > (3LL << 19) && bytes <= (4LL << 20)) return false;
+    if (gates) return !(few && B >= 256 && B % 32 && bytes > (192LL << 20));
+    if (B % 4) return !few;
+    if (!wide) return reads < 64 * in_dim ? bytes <= (100LL << 20) : B <= 128 || bytes <= (3LL << 19);
+    if (4 * out_dim < 3 * in_dim && bytes > (160LL << 20) && B > 128) return false;
+    return in_dim < 131072 || B % 32 == 0 || B <= 128;
+}
+
 extern "C" int clb_logic_entries(const int64_t *a, const int64_t *b, const int64_t *start, const int64_t *consumers, int32_t *start32, void *entry,
                                  int64_t in_dim, int64_t out_dim, void *stream)
 {
@@ -302,7 +325,7 @@ extern "C" int clb_logic_entries(const int64_t *a, const int64_t *b, const int64
 
 extern "C" size_t clb_logic_bwd_scratch_bytes(int64_t in_dim, int64_t out_dim, int64_t B)
 {
-    if (in_dim <= 0 || out_dim <= 0 || B <= 0) return 0;
+    if (in_dim <= 0 || out_dim <= 0 || B <= 0 || !combined_pays(in_dim, out_dim, B, true)) return 0;
     return (size_t)bwd_cut(in_dim, out_dim, B).cols * (size_t)out_dim * 16;
 }
 
@@ -314,7 +337,7 @@ extern "C" int clb_logic_bwd(const float *x, const float *w, const float *coef, 
     if (in_dim > 0x3fffffff || out_dim > 0x3fffffff || B > 0x3fffffff || !aligned16(coef)) return CLB_ERR_SHAPE;
     const bool vec = B % 4 == 0;
     if ((vec && !(aligned16(x) && aligned16(gy) && aligned16(gx))) || !aligned16(w) || (gw && !aligned16(gw))) return CLB_ERR_SHAPE;
-    if (in_dim * 16 > 0x7fffffffLL * 256) return CLB_ERR_SHAPE;
+    if (in_dim * 16 > 0x7fffffffLL * 256 || !combined_pays(in_dim, out_dim, B, gw != nullptr)) return CLB_ERR_SHAPE;
     if (gw && (!scratch || !aligned16(scratch) || scratch_bytes < clb_logic_bwd_scratch_bytes(in_dim, out_dim, B))) return CLB_ERR_SCRATCH;
     cudaStream_t st = (cudaStream_t)stream;
     const BwdCut cut = bwd_cut(in_dim, out_dim, B);

@@ -631,9 +631,9 @@ struct LogicNode : public Node {
             if (gx.defined()) gx.zero_();
         } else {
             int rc = CLB_ERR_SHAPE;
-            if (need_gx && plan) { // both gradients in one pass
+            const size_t bytes = need_gx && need_gw && plan ? clb_logic_bwd_scratch_bytes(in, out, batch) : 0;
+            if (need_gx && plan && (bytes || !need_gw)) { // both gradients in one pass, where that is the faster way
                 const Tensor cc = coef.unpack();
-                const size_t bytes = need_gw ? clb_logic_bwd_scratch_bytes(in, out, batch) : 0;
                 Tensor scratch;
                 if (need_gw) scratch = scratch_bytes(bytes, xx);
                 rc = clb_logic_bwd(ptr<float>(xx), ptr<float>(ww), ptr<float>(cc), ptr<float>(gy), ptr<float>(gx), ptr<float>(gw),

@@ -254,7 +254,8 @@ int clb_logic_fwd_coef(const void *x, const int64_t *a, const int64_t *b, const 
  * reference's autograd Function calls, src/difflogic/difflogic.py:219-230).  clb_logic_entries lays the consumer lists out once
  * per layer: start32 int32 [in+1], entry 8 bytes per list entry [2*out].  gx [in][B] required, gw [out][16] may be NULL;
  * scratch: clb_logic_bwd_scratch_bytes(in, out, B), 16-byte aligned.  CLB_ERR_SHAPE for rows it does not take (B a multiple of
- * 4 with unaligned pointers, sizes beyond 2^30): use clb_logic_bwd_w / clb_logic_bwd_x.  Fixed summation order. */
+ * 4 with unaligned pointers, sizes beyond 2^30) and for sizes at which the two are faster (with gw the scratch size is then 0):
+ * use clb_logic_bwd_w / clb_logic_bwd_x.  Fixed summation order. */
 int clb_logic_entries(const int64_t *a, const int64_t *b, const int64_t *start, const int64_t *consumers, int32_t *start32, void *entry,
                       int64_t in_dim, int64_t out_dim, void *stream);
 size_t clb_logic_bwd_scratch_bytes(int64_t in_dim, int64_t out_dim, int64_t B);

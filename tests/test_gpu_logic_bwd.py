@@ -61,3 +61,36 @@ def test_large_activation_forward_walks_in_stretches():
     _lib.trace(False)
     small = layer(x[:128].contiguous())
     assert float((y[:128] - small).abs().max()) <= 1e-6
+
+
+@pytest.mark.parametrize("fin,fout,batch,both,alone", [(1000, 1500, 512, False, False), (1000, 1500, 508, True, True), (500, 600, 512, True, True),
+                                                       (1000, 1500, 514, True, True), (200, 6500, 128, True, True), (900, 30000, 512, False, False),
+                                                       (3000, 97000, 256, True, False), (140000, 90000, 380, False, False), (140000, 90000, 384, True, False),
+                                                       (140000, 140000, 300, True, False), (140000, 90000, 381, False, False)])
+def test_combined_or_separate_backward_by_size(fin, fout, batch, both, alone):
+    """Both sides of the lines of the choice, with and without a gate gradient, against the separate kernels."""
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib, ops
+    from convlogic_b200._lib import W_SOFTMAX
+
+    torch.manual_seed(batch)
+    layer = cb.LogicLayer(fin, fout).cuda().train()
+    layer.weights.data.normal_()
+    x, gy = torch.rand(fin, batch, device="cuda"), torch.randn(fout, batch, device="cuda")
+    tables = (layer.indices_0, layer.indices_1, layer.weights.detach())
+    want_x = ops.logic_bwd_x(x, *tables, gy, layer.given_x_indices_of_y_start, layer.given_x_indices_of_y, W_SOFTMAX)
+    want_w = ops.logic_bwd_w(x, *tables, gy, W_SOFTMAX)
+    for gates, combined in ((True, both), (False, alone)):
+        layer.weights.requires_grad_(gates)
+        xd = x.t().detach().requires_grad_(True)
+        y = layer(xd)
+        _lib.trace(True)
+        got = torch.autograd.grad(y, [xd] + ([layer.weights] if gates else []), gy.t())
+        torch.cuda.synchronize()
+        names = _lib.trace_report()
+        _lib.trace(False)
+        assert ("logic_bwd_kernel" in names) == combined and ("logic_bwd_x_kernel" in names) == (not combined), names
+        # the same terms in another order: sums over a feature's readers, over the samples and of four basis sums
+        assert (got[0].t() - want_x).norm() <= 1e-5 * want_x.norm()
+        if gates:
+            assert (got[1] - want_w).norm() <= 1e-5 * want_w.norm()
