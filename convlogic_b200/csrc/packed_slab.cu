@@ -224,13 +224,10 @@ __global__ void __launch_bounds__(Geo<S, SMALL>::THREADS, 1024 / Geo<S, SMALL>::
     cp_async_wait_all();
 }
 
-// One record per output channel; offsets are bytes from a window's unit of the first plane.
-template <int S, bool SMALL>
-__global__ void packed_slab3_records_kernel(const uint8_t *__restrict__ ops, const int32_t *__restrict__ sel, Rec *__restrict__ recs, int C, int Ci)
+// The record of output channel c; offsets are bytes from a window's unit of the first plane.
+template <int S, bool SMALL> __device__ __forceinline__ void lay_out_record(const uint8_t *__restrict__ ops, const int32_t *__restrict__ sel, Rec *__restrict__ recs, int c, int Ci)
 {
     using G = Geo<S, SMALL>;
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= C) return;
     Rec R;
     int ch0 = 0, ch1 = -1;
     bool all = true;
@@ -250,6 +247,18 @@ __global__ void packed_slab3_records_kernel(const uint8_t *__restrict__ ops, con
     }
     R.ch[0] = ch0, R.ch[1] = ch1 < 0 ? ch0 : ch1, R.nst = ch1 < 0 ? 1 : 2, R.all_in_tile = all;
     recs[c] = R;
+}
+
+// Those of the large blocks and behind them those of the small ones (but for 32x32 images), in one launch: a module's call lays them
+// out every time (two launches: 64 -> 256 channels of 16x16, 1000 samples 39 us, before 37).
+template <int S> __global__ void packed_slab3_records_kernel(const uint8_t *__restrict__ ops, const int32_t *__restrict__ sel, Rec *__restrict__ recs, int C, int Ci)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < C) {
+        lay_out_record<S, false>(ops, sel, recs, i, Ci);
+    } else if constexpr (S < 32) {
+        if (i < 2 * C) lay_out_record<S, true>(ops, sel, recs + C, i - C, Ci);
+    }
 }
 
 template <int S, bool SMALL> static int launch(const void *x, const void *recs, void *y, int Ci, int C, int64_t U, Order in, Order out, cudaStream_t st)
@@ -273,9 +282,9 @@ template <int S> static int launch_by_slabs(const void *x, const void *recs, voi
 }
 template <int S> static int records(const uint8_t *ops, const int32_t *sel, Rec *recs, int Ci, int C, cudaStream_t st)
 {
-    packed_slab3_records_kernel<S, false><<<(C + 127) / 128, 128, 0, st>>>(ops, sel, recs, C, Ci);
-    if constexpr (S < 32) packed_slab3_records_kernel<S, true><<<(C + 127) / 128, 128, 0, st>>>(ops, sel, recs + C, C, Ci);
-    return clb_host::check_launch(S < 32 ? 2 : 1);
+    const int n = S < 32 ? 2 * C : C;
+    packed_slab3_records_kernel<S><<<(n + 127) / 128, 128, 0, st>>>(ops, sel, recs, C, Ci);
+    return clb_host::check_launch();
 }
 
 } // namespace slab
