@@ -61,3 +61,18 @@ def test_class_counts_over_rows_of_any_bytes(rows_per_class, row_bytes):
     want = torch.stack([(x.view(3, rows_per_class, row_bytes).long() >> s) & 1 for s in range(8)], -1).sum(1)   # [3, row_bytes, 8]
     got = _lib.native().group_popcount(x, 3, 3)
     assert torch.equal(got.long(), want.reshape(3, -1).t()[: 8 * row_bytes - 3])
+
+
+@pytest.mark.parametrize("n,side,levels", [(1, 32, 64), (70, 9, 33), (300, 16, 100), (2000, 32, 40)])
+@pytest.mark.parametrize("bytes_", [False, True])
+def test_more_thermometer_levels_than_a_pass(n, side, levels, bytes_):
+    """Passes over 32 levels at a time, each its own blocks where the grid is small (the last shape: in turn)."""
+    from convlogic_b200 import ops
+
+    torch.manual_seed(levels)
+    px = torch.randint(0, 256, (n, 2, side, side), device="cuda", dtype=torch.uint8)
+    th = torch.rand(levels, device="cuda")
+    got, _ = ops.thermometer_pack(px if bytes_ else px.float() / 255, th)
+    bits = torch.cat([px.float() / 255 > t for t in th], dim=1)
+    want, _ = ops.pack_bits(bits.reshape(n, -1), 64, sample_major=True)
+    assert torch.equal(got.reshape(want.shape), want)
