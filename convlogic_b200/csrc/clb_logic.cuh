@@ -5,11 +5,9 @@
 
 namespace clb {
 
-// Each half-warp reduces the 16 values of one neuron: the lane handles value (lane & 15) of neuron
-// `j` (the same j in all 16 lanes of a half-warp; the two halves may name unrelated neurons).
+// Each half-warp reduces the 16 values of one neuron (the two halves' neurons are unrelated): v is value (lane & 15) of the lane's.
 // Returns that neuron's gate in every lane of the half-warp, plus the lane's mixture value p.
-// Neurons outside [0, out_dim) give zeros.
-template <typename T> __device__ __forceinline__ Gate<T> half_warp_gate_of(T v, int wmode, int lane, T &p) // v: the lane's value
+template <typename T> __device__ __forceinline__ Gate<T> half_warp_gate_of(T v, int wmode, int lane, T &p)
 {
     const int i = lane & 15;
     if (wmode == CLB_W_SOFTMAX) {
@@ -55,28 +53,11 @@ template <typename T> __device__ __forceinline__ Gate<T> half_warp_gate_of(T v, 
     return g;
 }
 
-template <typename T>
-__device__ __forceinline__ Gate<T> half_warp_gate(const T *__restrict__ w, long long j, long long out_dim, int wmode, int lane, T &p)
-{
-    return half_warp_gate_of<T>((j >= 0 && j < out_dim) ? w[j * 16 + (lane & 15)] : T(0), wmode, lane, p);
-}
-
-template <typename T> __device__ __forceinline__ Gate<T> gate_from_lane(const Gate<T> &g, int src)
-{
-    Gate<T> r;
-    r.kab = __shfl_sync(0xffffffffu, g.kab, src);
-    r.ka = __shfl_sync(0xffffffffu, g.ka, src);
-    r.kb = __shfl_sync(0xffffffffu, g.kb, src);
-    r.k1 = __shfl_sync(0xffffffffu, g.k1, src);
-    return r;
-}
-
 template <typename T, int V> struct Vec;
 template <> struct Vec<float, 4> { using type = float4; };
 template <> struct Vec<float, 2> { using type = float2; };
 template <> struct Vec<float, 1> { using type = float; };
 template <> struct Vec<double, 1> { using type = double; };
-template <> struct Vec<double, 2> { using type = double2; };
 
 template <typename T, int V> __device__ __forceinline__ void vload(const T *p, T (&r)[V])
 {

@@ -27,7 +27,7 @@ __host__ __device__ __forceinline__ int split_position(int pixel, int side) // s
 }
 } // namespace clb
 
-// does the kernel take this block?  (U > 0 slabs, units below 2^31 are checked by the caller)
+// does the kernel take this block?  (U > 0 slabs of side * side units below 2^31 in all: 268 million samples of 32x32)
 bool clb_slab3_covers(int H, int W, int sh, int sw, int ph, int pw, int kh, int kw);
 size_t clb_slab3_record_bytes(int C);
 int clb_slab3_records(const uint8_t *ops, const int32_t *sel, void *recs, int Ci, int side, int C, cudaStream_t st);

@@ -145,14 +145,10 @@ template <int OFF, int BYTES> __device__ __forceinline__ void cp_async_off(uint3
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int PENDING> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(PENDING) : "memory"); }
 
-// How the planes reach shared memory.  16x16 images and larger: TMA box loads (one elected thread, halo zero-filled by the copy
-// engine).  Smaller images: the copy engine handles a box row by row at a few cycles per row, and rows of 32 or 16
-// useful bytes make it the bottleneck (measured: 290-300 us per layer against 230-240 us for register staging); there
-// every thread of the group issues two 16-byte cp.async copies per iteration into the interior of a tile whose halo was
-// zeroed once.
-template <int S> struct UseTma {
-    static constexpr bool value = S >= 16;
-};
+// How the forward's planes reach shared memory.  16x16 images and larger: TMA box loads (one elected thread, halo zero-filled by the
+// copy engine).  Smaller images, and the backward here: the copy engine handles a box row by row at a few cycles per row, and rows of
+// 32 or 16 useful bytes make it the bottleneck (measured: 290-300 us per layer against 230-240 us for register staging); there
+// every thread of the group issues cp.async copies into the interior of a tile whose halo was zeroed once.
 
 // =========================================================================================== forward
 template <int S> struct FwdCfg {
@@ -164,7 +160,7 @@ template <int S> struct FwdCfg {
     static constexpr int IMG = G::FWD_IMG;                       // floats of one staged plane (R * P + padding)
     static constexpr int SLOT = (NIMG * IMG + 31) / 32 * 32;     // floats of one slot (NIMG planes of one channel)
     static constexpr int STAGE_BYTES = 2 * SLOT * 4;
-    static constexpr bool TMA = UseTma<S>::value;
+    static constexpr bool TMA = S >= 16;
     // What a thread evaluates as a pair: the same position of images (2p, 2p + 1) of its batch, of (p, p + NIMG / 2) when several
     // pairs share a warp, or of pooled rows (r, r + HP / 2) of the one image when a stage holds no more.
     static constexpr bool SPLIT_PAIRS = NIMG > 2, ROW_PAIRS = NIMG == 1;
@@ -452,7 +448,6 @@ template <int S> struct BwdCfg {
     static constexpr int WARP_BYTES = (XST + 1) * STAGE_BYTES;
     static constexpr int SMEM = (kThreads / 32) * WARP_BYTES;
     static constexpr int UNITS = NIMG * 2 * S * (S / 4); // float4 units of the interior of the gradient tile (and of a stage)
-    static constexpr bool TMA = UseTma<S>::value;
     static_assert(I >= 32 ? (NIMG == 1 && WPT * 32 == I) : (WPT == 1 && NIMG * I == 32), "thread mapping");
     static_assert(UNITS % 32 == 0, "write-out units per lane");
 };
@@ -494,18 +489,16 @@ __device__ __forceinline__ void bwd_windows(const uint32_t (&base)[WPT], const u
 }
 
 template <int S, bool FM>
-__global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const __grid_constant__ CUtensorMap xmap, const float *__restrict__ gy,
-                                                                      const float *__restrict__ x, const float *__restrict__ w,
-                                                                      const int32_t *__restrict__ sel, const uint8_t *__restrict__ amax,
-                                                                      float *__restrict__ partial, float *__restrict__ planes, Args s)
+__global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const float *__restrict__ gy, const float *__restrict__ x,
+                                                                      const float *__restrict__ w, const int32_t *__restrict__ sel,
+                                                                      const uint8_t *__restrict__ amax, float *__restrict__ partial,
+                                                                      float *__restrict__ planes, Args s)
 {
     using Cf = BwdCfg<S>;
     constexpr int XST = Cf::XST, WPT = Cf::WPT, I = Cf::I, HW = S * S;
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t full[4][XST];
     __shared__ Gate<float> sgs[4][7];
     __shared__ SlotInfo sis[4];
-    __shared__ int saborts[4];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const long long task = (long long)blockIdx.x * 4 + warp;
@@ -515,13 +508,7 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const __gr
     SlotInfo &si = sis[warp];
     if (lane < 7) sg[lane] = gate_load<float>(w + ((size_t)c * 7 + lane) * 16, s.wmode);
     if (lane == 8) fill_slots(si, sel, c, s.Ci);
-    if (lane == 9) {
-        for (int st = 0; st < XST; ++st) clb_tma::mbar_init(&full[warp][st], 1);
-        clb_tma::mbar_init_fence();
-        saborts[warp] = *reinterpret_cast<volatile int *>(&g_plane_error);
-    }
     __syncwarp();
-    if (saborts[warp]) return;
     Gate<float> g[7];
 #pragma unroll
     for (int i = 0; i < 7; ++i) g[i] = sg[i];
@@ -555,16 +542,7 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const __gr
     const bool usable = si.nslot <= 2; // the host only routes selections here that fit two planes
 
     const int iters = usable ? (n_hi - n_lo + Cf::NIMG - 1) / Cf::NIMG : 0;
-    constexpr uint32_t tx_bytes = 2u * (uint32_t)(Cf::NIMG * Cf::IMG * 4);
-    auto issue = [&](int it) {
-        const int st = it % XST;
-        const int n0 = n_lo + it * Cf::NIMG;
-        unsigned char *dst = wbase + (size_t)st * Cf::STAGE_BYTES;
-        clb_tma::mbar_expect_tx(&full[warp][st], tx_bytes);
-        clb_tma::load_box_4d(dst, &xmap, -kLead, -1, ch_a, n0, &full[warp][st]);
-        clb_tma::load_box_4d(dst + Cf::SLOT * 4, &xmap, -kLead, -1, ch_b, n0, &full[warp][st]);
-    };
-    // cp.async staging (small images): the 16-byte pieces this lane moves, the same for every iteration; the source
+    // cp.async staging: the 16-byte pieces this lane moves, the same for every iteration; the source
     // pointers run along with the iterations, cp_iters = iterations in which the piece's image exists
     constexpr int CPQ = Cf::UNITS / 32;
     const float *csrc[CPQ];
@@ -591,18 +569,13 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const __gr
         }                                                                                                                 \
         cp_async_commit();                                                                                                \
     }
-    if (Cf::TMA) {
-        if (lane == 0)
-            for (int it = 0; it < XST && it < iters; ++it) issue(it);
-    } else {
-        for (int i = lane * 4; i < XST * Cf::STAGE_FLOATS; i += 128)   // the halo is zeroed once; copies write the interior
-            *reinterpret_cast<float4 *>(reinterpret_cast<float *>(wbase) + i) = make_float4(0.f, 0.f, 0.f, 0.f);
-        __syncwarp();
-        CLB_BWD_ISSUE_CP(0, 0)
-        CLB_BWD_ISSUE_CP(1, 1)
-        CLB_BWD_ISSUE_CP(2, 2)
-        static_assert(XST == 3, "prologue of the cp.async ring");
-    }
+    for (int i = lane * 4; i < XST * Cf::STAGE_FLOATS; i += 128)   // the halo is zeroed once; copies write the interior
+        *reinterpret_cast<float4 *>(reinterpret_cast<float *>(wbase) + i) = make_float4(0.f, 0.f, 0.f, 0.f);
+    __syncwarp();
+    CLB_BWD_ISSUE_CP(0, 0)
+    CLB_BWD_ISSUE_CP(1, 1)
+    CLB_BWD_ISSUE_CP(2, 2)
+    static_assert(XST == 3, "prologue of the cp.async ring");
 
     // upstream gradient and arg-max: fetched one iteration ahead
     float dz_next[WPT];
@@ -622,7 +595,6 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const __gr
     };
     fetch(0);
 
-    bool failed = false;
     int it = 0;
     __syncwarp();
     // write-out: the lane's float4 units of the gradient tile are the cells its cp.async pieces have in a stage
@@ -646,46 +618,28 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const __gr
         }
         __syncwarp();
     };
-    while (it < iters && !failed) {
-        const uint32_t parity = (it / XST) & 1;
+    while (it < iters) {
 #define CLB_BWD_STAGE(ST)                                                                                                 \
-    if (it < iters && !failed) {                                                                                          \
+    if (it < iters) {                                                                                                     \
         float dz[WPT];                                                                                                    \
         int bd[WPT];                                                                                                      \
         _Pragma("unroll") for (int j = 0; j < WPT; ++j) dz[j] = dz_next[j], bd[j] = bd_next[j];                            \
         fetch(it + 1);                                                                                                    \
-        bool ok = true;                                                                                                   \
-        if (Cf::TMA) {                                                                                                    \
-            ok = clb_tma::mbar_wait(&full[warp][ST], parity);                                                             \
-        } else {                                                                                                          \
-            cp_async_wait<XST - 1>();                                                                                     \
-        }                                                                                                                 \
-        ok = __all_sync(0xffffffffu, ok ? 1 : 0) != 0; /* also: the other lanes' pieces of this stage are visible */     \
-        if (!ok) {                                                                                                        \
-            failed = true;                                                                                                \
-        } else {                                                                                                          \
-            uint32_t base[WPT];                                                                                           \
-            _Pragma("unroll") for (int j = 0; j < WPT; ++j) base[j] = woff[j] + 4u * (uint32_t)(((bd[j] >> 1) ? Cf::P : 0) + (bd[j] & 1)); \
-            bwd_windows<S, ST, WPT>(base, toff, g, dz, acc);                                                              \
-            /* the input planes of this stage have been read by every lane (the taps' __syncwarp): refill it */           \
-            if (Cf::TMA) {                                                                                                \
-                if (lane == 0 && it + XST < iters) issue(it + XST);                                                       \
-            } else {                                                                                                      \
-                CLB_BWD_ISSUE_CP(ST, it + XST)                                                                            \
-            }                                                                                                             \
-            finish();                                                                                                     \
-            ++it;                                                                                                         \
-        }                                                                                                                 \
+        cp_async_wait<XST - 1>();                                                                                         \
+        __syncwarp(); /* the other lanes' pieces of this stage are visible */                                            \
+        uint32_t base[WPT];                                                                                               \
+        _Pragma("unroll") for (int j = 0; j < WPT; ++j) base[j] = woff[j] + 4u * (uint32_t)(((bd[j] >> 1) ? Cf::P : 0) + (bd[j] & 1)); \
+        bwd_windows<S, ST, WPT>(base, toff, g, dz, acc);                                                                  \
+        /* the input planes of this stage have been read by every lane (the taps' __syncwarp): refill it */               \
+        CLB_BWD_ISSUE_CP(ST, it + XST)                                                                                    \
+        finish();                                                                                                         \
+        ++it;                                                                                                             \
     }
         CLB_BWD_STAGE(0)
         CLB_BWD_STAGE(1)
         CLB_BWD_STAGE(2)
 #undef CLB_BWD_STAGE
 #undef CLB_BWD_ISSUE_CP
-    }
-    if (failed && lane == 0) {
-        g_plane_error = 1;
-        for (int j = it + 1; j < iters && j < it + XST; ++j) clb_tma::mbar_wait(&full[warp][j % XST], (j / XST) & 1);
     }
     if (!usable && lane == 0) g_plane_error = 2;
 
@@ -936,7 +890,7 @@ int square_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int 
 int fwd_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw, int kh, int kw)
 {
     const int side = square_side(N, Ci, H, W, C, sh, sw, ph, pw, kh, kw);
-    if (clb_tma::encode_tiled_fn() == nullptr) return 0;
+    if (side >= 16 && clb_tma::encode_tiled_fn() == nullptr) return 0;
     return side == 32 || side == 28 || side == 16 || side == 12 || side == 8 || side == 6 || side == 4 ? side : 0;
 }
 // the gate gradient alone of a 32x32 block
@@ -965,14 +919,12 @@ int launch_fwd(const float *x, const float *w, const int32_t *sel, float *y, uin
 template <int S> int launch_bwd(const ClbTileBwd &a, cudaStream_t st)
 {
     using Cf = BwdCfg<S>;
-    CUtensorMap map;
-    if (!clb_tma::make_plane_map(&map, a.x, a.N, a.Ci, S, S, Cf::P, Cf::R, Cf::NIMG)) return CLB_ERR_SHAPE;
     auto k = a.fm ? convtree_bwd_plane_kernel<S, true> : convtree_bwd_plane_kernel<S, false>;
     if (clb_host::ensure_dynamic_smem(k, Cf::SMEM) != cudaSuccess) return check_launch(0);
     const Args s{a.N, a.Ci, a.C, a.wmode, a.parts, a.fm, a.n_stride};
     const long long tasks = (long long)a.C * a.parts;
     CLB_TRACED("convtree_bwd_plane_kernel", st,
-               k<<<(unsigned)((tasks + 3) / 4), kThreads, Cf::SMEM, st>>>(map, a.gy, a.x, a.w, a.sel, a.amax, a.partial, a.planes, s));
+               k<<<(unsigned)((tasks + 3) / 4), kThreads, Cf::SMEM, st>>>(a.gy, a.x, a.w, a.sel, a.amax, a.partial, a.planes, s));
     return CLB_OK;
 }
 
@@ -986,7 +938,8 @@ int bwd_side(int N, int Ci, int H, int W, int C, int sh, int sw, int ph, int pw,
     const int least = side == 32 ? 4 : side == 28 ? 8 : side == 12 ? 12 : side == 16 || side == 8 || side == 6 || side == 4 ? 1 : Ci + 1;
     return Ci >= least ? side : 0;
 }
-// Images of a slice of the batch: the gradient planes, eight bytes per pixel and output channel, of a slice stay below 1 GB.
+// Images of a slice of the batch: the gradient planes, eight bytes per pixel and output channel, of a slice stay below 1 GB, or are those of
+// 16 images (beyond 64 MB of planes an image: 8192 channels of 32x32).
 int bwd_slice(int N, int C, int HW)
 {
     const long long most = (1LL << 30) / ((long long)C * HW * 8);

@@ -552,29 +552,14 @@ __device__ __forceinline__ Gate<float> quad_gate(const float (&p)[4], int q)
     return g;
 }
 
-// neuron behind the lane's gate (lane < 28) and that neuron's row of 16 values
-__device__ __forceinline__ long long tree_node(const TreeTables &tt, long long t, int lane) { return __ldg(tt.node + t * 7 + (lane >> 2)); }
+// the row of 16 values of neuron n behind the lane's gate (lane < 28)
 __device__ __forceinline__ const float *tree_row(const TreeTables &tt, int lane, long long n)
 {
     const int g = lane >> 2;
     return tt.w[g < 4 ? 0 : (g < 6 ? 1 : 2)] + n * 16;
 }
 
-// every lane gets all seven gates
-__device__ __forceinline__ void tree_gates(const TreeTables &tt, long long t, int lane, int wmode, Gate<float> (&g)[7])
-{
-    const bool active = lane < 28;
-    const long long n = active ? tree_node(tt, t, lane) : 0;
-    float p[4];
-    quad_mixture(tree_row(tt, active ? lane : 0, n), wmode, lane & 3, active, p);
-    const Gate<float> mine = quad_gate(p, lane & 3);
-#pragma unroll
-    for (int i = 0; i < 7; ++i) {
-        g[i].k1 = __shfl_sync(0xffffffffu, mine.k1, 4 * i), g[i].ka = __shfl_sync(0xffffffffu, mine.ka, 4 * i);
-        g[i].kb = __shfl_sync(0xffffffffu, mine.kb, 4 * i), g[i].kab = __shfl_sync(0xffffffffu, mine.kab, 4 * i);
-    }
-}
-// the same with the lane's neuron already known (lanes >= 28: any value); p = the lane's four mixture entries
+// every lane gets all seven gates; n: the lane's neuron (lanes >= 28: any value), p: the lane's four mixture entries
 __device__ __forceinline__ void tree_gates_of(const TreeTables &tt, long long n, int lane, int wmode, Gate<float> (&g)[7], float (&p)[4])
 {
     const bool active = lane < 28;

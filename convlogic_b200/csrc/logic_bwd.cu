@@ -174,15 +174,14 @@ __global__ void __launch_bounds__(256, 3) logic_bwd_kernel(const float *__restri
 {
     using RowT = Row<LPR, V, R>;
     constexpr int GPW = 32 / LPR; // features a warp works on at a time
-    static_assert(U % 2 == 0 && (LPR == 8 || LPR == 16), "sums are reduced two entries at a time");
+    static_assert(U % 2 == 0 && LPR == 8, "eight lanes reduce the sums of two entries at a time");
     const int l = threadIdx.x & (LPR - 1), grp = (threadIdx.x & 31) / LPR;
     const int warps = (in_dim + GPW - 1) / GPW, step = (int)gridDim.x * 8; // warps' worth of features; all of a warp stays in one stretch
     int wf = (int)((blockIdx.x * 256u + threadIdx.x) >> 5), left = B - l * V;
     x += l * V, gy += l * V, gx += l * V;
-    // reduction of an entry pair: lane (i * LPR / 8) ends up with sum i & 3 of entry i >> 2
-    const int my = l / (LPR / 8);
-    const bool up4 = my & 4, up2 = my & 2, up1 = my & 1;
-    partial += my & 3;
+    // reduction of an entry pair: lane i ends up with sum i & 3 of entry i >> 2
+    const bool up4 = l & 4, up2 = l & 2, up1 = l & 1;
+    partial += l & 3;
     for (;; wf += step) {
         while (wf >= warps) { // the next stretch
             wf -= warps, left -= LPR * V * R;
@@ -235,13 +234,12 @@ __global__ void __launch_bounds__(256, 3) logic_bwd_kernel(const float *__restri
                 if (GW) {
                     float a4[4], a2[2], r;
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) a4[i] = (up4 ? v[4 + i] : v[i]) + __shfl_xor_sync(0xffffffffu, up4 ? v[i] : v[4 + i], LPR / 2);
+                    for (int i = 0; i < 4; ++i) a4[i] = (up4 ? v[4 + i] : v[i]) + __shfl_xor_sync(0xffffffffu, up4 ? v[i] : v[4 + i], 4);
 #pragma unroll
-                    for (int i = 0; i < 2; ++i) a2[i] = (up2 ? a4[2 + i] : a4[i]) + __shfl_xor_sync(0xffffffffu, up2 ? a4[i] : a4[2 + i], LPR / 4);
-                    r = (up1 ? a2[1] : a2[0]) + __shfl_xor_sync(0xffffffffu, up1 ? a2[0] : a2[1], LPR / 8);
-                    if (LPR == 16) r += __shfl_xor_sync(0xffffffffu, r, 1);
+                    for (int i = 0; i < 2; ++i) a2[i] = (up2 ? a4[2 + i] : a4[i]) + __shfl_xor_sync(0xffffffffu, up2 ? a4[i] : a4[2 + i], 2);
+                    r = (up1 ? a2[1] : a2[0]) + __shfl_xor_sync(0xffffffffu, up1 ? a2[0] : a2[1], 1);
                     const int code = up4 ? t[u0 + 1].x : t[u0].x; // the entry of this lane's sum
-                    if (code >= 0 && !(code & 1) && (l & (LPR / 8 - 1)) == 0) partial[(size_t)(code >> 1) * 4] = r;
+                    if (code >= 0 && !(code & 1)) partial[(size_t)(code >> 1) * 4] = r;
                 }
             }
         }
