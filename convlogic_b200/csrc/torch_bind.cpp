@@ -1005,16 +1005,17 @@ public:
         check(clb_net_device_bytes(data.data(), data.size(), &need));
         c10::cuda::CUDAGuard guard(device_);
         params_ = at::empty({(int64_t)(need < 16 ? 16 : need)}, at::TensorOptions().dtype(at::kByte).device(device_));
-        check(clb_net_create(data.data(), data.size(), ptr(params_), cur_stream(), &net_));
-        if (const size_t bytes = clb_net_record_bytes(net_)) {
+        clb_net *made = nullptr;
+        check(clb_net_create(data.data(), data.size(), ptr(params_), cur_stream(), &made));
+        net_.reset(made); // released also when something below throws
+        if (const size_t bytes = clb_net_record_bytes(made)) {
             records_ = at::empty({(int64_t)bytes}, params_.options());
-            check(clb_net_records(net_, ptr(records_), cur_stream()));
+            check(clb_net_records(made, ptr(records_), cur_stream()));
         }
         c10::cuda::getCurrentCUDAStream().synchronize(); // the blob is pageable host memory: wait for the copy
-        check(clb_net_info(net_, &features, &classes, &layers));
+        check(clb_net_info(made, &features, &classes, &layers));
     }
     Net(const Net &) = delete;
-    ~Net() { clb_net_destroy(net_); }
     // bool / uint8 bits [B, ...] -> counts
     Tensor forward(const Tensor &x_in) const
     {
@@ -1034,10 +1035,10 @@ public:
     {
         need_input(x);
         Below below(params_);
-        const size_t bytes = clb_net_workspace_bytes(net_, batch);
+        const size_t bytes = clb_net_workspace_bytes(net_.get(), batch);
         Tensor workspace = scratch_bytes(bytes, params_);
         Tensor counts = alloc({batch, classes}, params_, at::kInt);
-        check(clb_net_forward(net_, kind, ptr(x), thresholds ? ptr<float>(*thresholds) : nullptr, thresholds ? (int)thresholds->numel() : 0, batch,
+        check(clb_net_forward(net_.get(), kind, ptr(x), thresholds ? ptr<float>(*thresholds) : nullptr, thresholds ? (int)thresholds->numel() : 0, batch,
                               ptr<int32_t>(counts), ptr(workspace), bytes, cur_stream()));
         return counts;
     }
@@ -1047,7 +1048,10 @@ public:
 private:
     c10::Device device_;
     Tensor params_, records_;
-    clb_net *net_ = nullptr;
+    struct Destroy {
+        void operator()(clb_net *n) const { clb_net_destroy(n); }
+    };
+    std::unique_ptr<clb_net, Destroy> net_;
 };
 
 // raw forward / backward of the fused block for callers that handle autograd themselves
