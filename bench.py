@@ -683,12 +683,13 @@ def run_c5(ctx, args):
     peak, kind = measured_peaks()
     row = width * batch * 4          # one activation [width, batch] fp32
     xin = 3072 * batch * 4
+    layers = lambda kernel: trace.get(kernel, (0, 0))[0]            # of a step that the kernel ran: the choice goes by size
     names = {
-        "logic_fwd_kernel": (xin + row) + (depth - 1) * 2 * row,    # layer 1: x + y; the others: x + y
-        "logic_bwd_w_kernel": (xin + row) + (depth - 1) * 2 * row,  # gy + x per layer
-        "logic_bwd_x_kernel": (depth - 1) * 3 * row,                # all but the first layer: gy + x + gx
-        "logic_fwd_cols_kernel": (depth - 1) * 2 * row,             # the layers that walk the batch in stretches: x + y
-        "logic_bwd_kernel": (depth - 1) * 3 * row,                  # both gradients of all but the first layer: gy + x + gx
+        "logic_fwd_kernel": (xin + row) + (layers("logic_fwd_kernel") - 1) * 2 * row,      # layer 1: x + y; others: x + y
+        "logic_bwd_w_kernel": (xin + row) + (layers("logic_bwd_w_kernel") - 1) * 2 * row,  # layer 1 and others: gy + x
+        "logic_bwd_x_kernel": layers("logic_bwd_x_kernel") * 3 * row,                      # gy + x + gx
+        "logic_fwd_cols_kernel": layers("logic_fwd_cols_kernel") * 2 * row,                # the layers that walk the batch in stretches
+        "logic_bwd_kernel": layers("logic_bwd_kernel") * 3 * row,                          # both gradients: gy + x + gx
         "group_sum_partial_kernel": row, "group_sum_bwd_kernel": row,
     }
     kernels = kernel_table(trace, names, peak, traffic=None)
