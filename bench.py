@@ -194,10 +194,10 @@ def traced(fn, steps):
 # chunk (c4) of the default workload sizes: dram__bytes.sum over one capture of the same bench command.  Other sizes, and
 # kernels without an entry, report null.
 NCU_TRAFFIC = {
-    "c3": {"convtree_bwd_plane_kernel": 1930.7e6, "plane_sum_kernel": 1526.9e6, "logic_tree_bwd_kernel": 954.8e6,
-           "row_segment_sum_kernel": 706.5e6, "convtree_fwd_plane_kernel": 420.8e6, "adam_step_kernel": 245.7e6,
-           "logic_tree_fwd_sum_kernel": 92.1e6, "convtree_bwd_w_plane32_kernel": 97.8e6},
-    "c4": {"packed_tree_kernel": 1639.4e6, "thermometer_pack_kernel": 65.1e6},
+    "c3": {"convtree_bwd_plane_kernel": 1881.2e6, "plane_sum_kernel": 1514.0e6, "logic_tree_bwd_kernel": 948.7e6,
+           "row_segment_sum_kernel": 703.1e6, "convtree_fwd_plane_kernel": 411.5e6, "adam_step_kernel": 240.4e6,
+           "logic_tree_fwd_sum_kernel": 89.3e6, "convtree_bwd_w_plane32_kernel": 94.5e6},
+    "c4": {"packed_convtree_slab3_kernel": 2667.6e6, "packed_tree_kernel": 1603.2e6, "group_popcount_kernel": 672.0e6, "thermometer_pack_kernel": 64.0e6},
 }
 
 
