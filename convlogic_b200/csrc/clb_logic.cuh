@@ -77,4 +77,93 @@ template <typename T, int V> __device__ __forceinline__ void vstore(T *p, const 
     *reinterpret_cast<VT *>(p) = v;
 }
 
+// a gate's 16 values as four vectors
+__device__ __forceinline__ void load16(const float *__restrict__ w, float (&v)[16])
+{
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(w) + q);
+        v[4 * q] = t.x, v[4 * q + 1] = t.y, v[4 * q + 2] = t.z, v[4 * q + 3] = t.w;
+    }
+}
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b)
+{
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ float sum2(f32x2 v)
+{
+    float a, b;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+    return a + b;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
+// R vectors of V floats at stride LPR * V, as R * V / 2 packed pairs; zeros beyond the row
+template <int LPR, int V, int R> struct Row {
+    static constexpr int P = R * V / 2;
+    f32x2 p[P];
+    __device__ __forceinline__ void zero()
+    {
+#pragma unroll
+        for (int i = 0; i < P; ++i) p[i] = 0ull;
+    }
+    __device__ __forceinline__ void load(const float *__restrict__ row, int left) // row: the lane's first element, left: how many follow
+    {
+        if constexpr (V == 4) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                ulonglong2 q = make_ulonglong2(0ull, 0ull);
+                if (r * LPR * 4 < left) q = __ldg(reinterpret_cast<const ulonglong2 *>(row + r * LPR * 4));
+                p[2 * r] = q.x, p[2 * r + 1] = q.y;
+            }
+        } else if constexpr (V == 2) {
+#pragma unroll
+            for (int r = 0; r < R; ++r) p[r] = r * LPR * 2 < left ? __ldg(reinterpret_cast<const f32x2 *>(row + r * LPR * 2)) : 0ull;
+        } else {
+            float t[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) t[r] = r * LPR < left ? __ldg(row + r * LPR) : 0.f;
+#pragma unroll
+            for (int r = 0; r < P; ++r) p[r] = pack2(t[2 * r], t[2 * r + 1]);
+        }
+    }
+    __device__ __forceinline__ void store(float *__restrict__ row, int left) const
+    {
+        if constexpr (V == 4) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (r * LPR * 4 < left) __stcs(reinterpret_cast<float4 *>(row + r * LPR * 4), *reinterpret_cast<const float4 *>(&p[2 * r]));
+        } else if constexpr (V == 2) {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (r * LPR * 2 < left) __stcs(reinterpret_cast<float2 *>(row + r * LPR * 2), *reinterpret_cast<const float2 *>(&p[r]));
+        } else {
+#pragma unroll
+            for (int r = 0; r < R; ++r)
+                if (r * LPR < left) row[r * LPR] = __uint_as_float((unsigned)(r & 1 ? p[r / 2] >> 32 : p[r / 2]));
+        }
+    }
+};
+
 } // namespace clb

@@ -45,16 +45,6 @@ __global__ void __launch_bounds__(256) logic_entries_kernel(const int64_t *__res
     }
 }
 
-// a gate's 16 values as four vectors
-__device__ __forceinline__ void load16(const float *__restrict__ w, float (&v)[16])
-{
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const float4 t = __ldg(reinterpret_cast<const float4 *>(w) + q);
-        v[4 * q] = t.x, v[4 * q + 1] = t.y, v[4 * q + 2] = t.z, v[4 * q + 3] = t.w;
-    }
-}
-
 // What the forward pass leaves for the backward where it does not run logic_fwd_kernel: a thread per neuron.
 __global__ void __launch_bounds__(256) logic_coef_kernel(const float *__restrict__ w, float4 *__restrict__ coef, long long out_dim, int wmode)
 {
@@ -88,89 +78,11 @@ __global__ void __launch_bounds__(256) logic_fwd_cols_kernel(const float *__rest
     }
 }
 
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2(float a, float b)
-{
-    f32x2 d;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-    return d;
-}
-__device__ __forceinline__ float sum2(f32x2 v)
-{
-    float a, b;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-    return a + b;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
-{
-    f32x2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
-{
-    f32x2 d;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-    return d;
-}
-
-// R vectors of V floats at stride LPR * V, as R * V / 2 packed pairs; zeros beyond the row
-template <int LPR, int V, int R> struct Row {
-    static constexpr int P = R * V / 2;
-    f32x2 p[P];
-    __device__ __forceinline__ void zero()
-    {
-#pragma unroll
-        for (int i = 0; i < P; ++i) p[i] = 0ull;
-    }
-    __device__ __forceinline__ void load(const float *__restrict__ row, int left) // row: the lane's first element, left: how many follow
-    {
-        if constexpr (V == 4) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) {
-                ulonglong2 q = make_ulonglong2(0ull, 0ull);
-                if (r * LPR * 4 < left) q = __ldg(reinterpret_cast<const ulonglong2 *>(row + r * LPR * 4));
-                p[2 * r] = q.x, p[2 * r + 1] = q.y;
-            }
-        } else if constexpr (V == 2) {
-#pragma unroll
-            for (int r = 0; r < R; ++r) p[r] = r * LPR * 2 < left ? __ldg(reinterpret_cast<const f32x2 *>(row + r * LPR * 2)) : 0ull;
-        } else {
-            float t[R];
-#pragma unroll
-            for (int r = 0; r < R; ++r) t[r] = r * LPR < left ? __ldg(row + r * LPR) : 0.f;
-#pragma unroll
-            for (int r = 0; r < P; ++r) p[r] = pack2(t[2 * r], t[2 * r + 1]);
-        }
-    }
-    __device__ __forceinline__ void store(float *__restrict__ row, int left) const
-    {
-        if constexpr (V == 4) {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (r * LPR * 4 < left) __stcs(reinterpret_cast<float4 *>(row + r * LPR * 4), *reinterpret_cast<const float4 *>(&p[2 * r]));
-        } else if constexpr (V == 2) {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (r * LPR * 2 < left) __stcs(reinterpret_cast<float2 *>(row + r * LPR * 2), *reinterpret_cast<const float2 *>(&p[r]));
-        } else {
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-                if (r * LPR < left) row[r * LPR] = __uint_as_float((unsigned)(r & 1 ? p[r / 2] >> 32 : p[r / 2]));
-        }
-    }
-};
-
 template <int LPR, int V, int R, int U, bool GW>
 __global__ void __launch_bounds__(256, 3) logic_bwd_kernel(const float *__restrict__ x, const float *__restrict__ gy, const float4 *__restrict__ coef,
                                                         const int32_t *__restrict__ start, const int2 *__restrict__ entry, float *__restrict__ gx,
-                                                        float *__restrict__ partial, int in_dim, int out_dim, int B)
+                                                        float *__restrict__ partial, int in_dim, int out_dim, int B,
+                                                        const int32_t *__restrict__ list /* !GW: the features, or null for all of them */)
 {
     using RowT = Row<LPR, V, R>;
     constexpr int GPW = 32 / LPR; // features a warp works on at a time
@@ -188,8 +100,9 @@ __global__ void __launch_bounds__(256, 3) logic_bwd_kernel(const float *__restri
             x += LPR * V * R, gy += LPR * V * R, gx += LPR * V * R, partial += (size_t)out_dim * 4;
         }
         if (left + l * V <= 0) return; // the whole warp
-        const int f = wf * GPW + grp;
+        int f = wf * GPW + grp;
         const bool mine = f < in_dim;
+        if (!GW && list != nullptr && mine) f = __ldg(list + f);
         int lo = 0, hi = 0;
         if (mine) lo = __ldg(start + f), hi = __ldg(start + f + 1);
         RowT xf, acc;
@@ -346,7 +259,7 @@ extern "C" int clb_logic_bwd(const float *x, const float *w, const float *coef, 
         const long long wave = (long long)sm_count() * 3; // resident at once; a second wave would walk all stretches again
         if (blocks > wave) blocks = wave;
         CLB_TRACED("logic_bwd_kernel", st,
-                   kern<<<(unsigned)blocks, 256, 0, st>>>(x, gy, (const float4 *)coef, start32, (const int2 *)entry, gx, (float *)scratch, (int)in_dim, (int)out_dim, (int)B));
+                   kern<<<(unsigned)blocks, 256, 0, st>>>(x, gy, (const float4 *)coef, start32, (const int2 *)entry, gx, (float *)scratch, (int)in_dim, (int)out_dim, (int)B, nullptr));
     };
     if (vec && cut.wide)
         gw ? go(logic_bwd_kernel<8, 4, 2, 2, true>, 8) : go(logic_bwd_kernel<8, 4, 2, 2, false>, 8);
@@ -364,6 +277,31 @@ extern "C" int clb_logic_bwd(const float *x, const float *w, const float *coef, 
     CLB_TRACED("logic_bwd_finish_kernel", st,
                logic_bwd_finish_kernel<<<(unsigned)((out_dim + 127) / 128), 128, 0, st>>>((const float4 *)scratch, w, gw, out_dim, cut.cols, wmode));
     return check_launch(2);
+}
+
+// Input gradient of the features in a list alone (logic_path.cu).  vec: floats per access.
+int clb_logic_bwd_open(const float *x, const float *gy, const float *coef, const int32_t *start32, const void *entry, const int32_t *open, int64_t n_open,
+                       float *gx, int64_t B, int vec, int wide, cudaStream_t st)
+{
+    const int64_t cols = wide ? (B + 63) / 64 : (B + 31) / 32;
+    long long blocks = (n_open * cols * 8 + 255) / 256;
+    if (blocks > (long long)sm_count() * 3) blocks = (long long)sm_count() * 3;
+    auto go = [&](auto kern) {
+        CLB_TRACED("logic_bwd_kernel", st,
+                   kern<<<(unsigned)blocks, 256, 0, st>>>(x, gy, (const float4 *)coef, start32, (const int2 *)entry, gx, nullptr, (int)n_open, 0, (int)B, open));
+    };
+    switch (vec) {
+    case 4: wide ? go(logic_bwd_kernel<8, 4, 2, 2, false>) : go(logic_bwd_kernel<8, 4, 1, 4, false>); break;
+    case 2: wide ? go(logic_bwd_kernel<8, 2, 4, 2, false>) : go(logic_bwd_kernel<8, 2, 2, 4, false>); break;
+    default: wide ? go(logic_bwd_kernel<8, 1, 8, 2, false>) : go(logic_bwd_kernel<8, 1, 4, 4, false>); break;
+    }
+    return check_launch();
+}
+
+int clb_logic_coef(const float *w, float *coef, int64_t out_dim, int wmode, cudaStream_t st)
+{
+    CLB_TRACED("logic_coef_kernel", st, logic_coef_kernel<<<(unsigned)((out_dim + 255) / 256), 256, 0, st>>>(w, (float4 *)coef, out_dim, wmode));
+    return check_launch();
 }
 
 // Forward of a layer too large for the L2 (V = 4 rows): the gates' coefficients, then the rows stretch by stretch.

@@ -535,6 +535,10 @@ struct LogicPlan {
     LogicKey key;
     int64_t in = 0, out = 0;
     Tensor start32, entry;
+    Tensor rec, open;    // neurons in the order of paths, features whose gradient a path does not complete; undefined: lists and connections disagree
+    int64_t n_open = 0;
+    bool path_fwd(int64_t batch) const { return rec.defined() && clb_logic_path_pays(in, out, batch, n_open, 0); }
+    bool path_bwd(int64_t batch) const { return rec.defined() && clb_logic_path_pays(in, out, batch, n_open, 1); }
 };
 using LogicPlanPtr = std::shared_ptr<LogicPlan>;
 
@@ -554,6 +558,16 @@ LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const 
     p->start32 = alloc({in + 1}, start, at::kInt), p->entry = alloc({2 * out, 2}, start, at::kInt);
     check(clb_logic_entries(ptr<int64_t>(a), ptr<int64_t>(b), ptr<int64_t>(start), ptr<int64_t>(cons), ptr<int32_t>(p->start32), ptr(p->entry), in, out,
                             cur_stream()));
+    if (out) {
+        const size_t bytes = clb_logic_path_scratch_bytes(in, out);
+        const Tensor scratch = scratch_bytes(bytes, start), count = alloc({2}, start, at::kInt);
+        p->rec = alloc({out, 4}, start, at::kInt), p->open = alloc({in}, start, at::kInt);
+        check(clb_logic_path(ptr<int64_t>(a), ptr<int64_t>(b), ptr<int32_t>(p->start32), ptr(p->entry), ptr(p->rec), ptr<int32_t>(p->open), ptr<int32_t>(count),
+                             ptr(scratch), bytes, in, out, cur_stream()));
+        const Tensor host = count.to(at::kCPU);
+        p->n_open = host.data_ptr<int32_t>()[1];
+        if (host.data_ptr<int32_t>()[0] != out) p->rec = p->open = Tensor();
+    }
     // the plan outlives this call: work of other streams may read it next
     c10::cuda::getCurrentCUDAStream().synchronize();
     start_obj.attr("_clb_plan") = p;
@@ -631,8 +645,17 @@ struct LogicNode : public Node {
             if (gx.defined()) gx.zero_();
         } else {
             int rc = CLB_ERR_SHAPE;
-            const size_t bytes = need_gx && need_gw && plan ? clb_logic_bwd_scratch_bytes(in, out, batch) : 0;
-            if (need_gx && plan && (bytes || !need_gw)) { // both gradients in one pass, where that is the faster way
+            if (need_gx && need_gw && plan && plan->path_bwd(batch)) {
+                const Tensor cc = coef.unpack();
+                const size_t bytes = clb_logic_path_bwd_scratch_bytes(out, batch);
+                Tensor scratch = scratch_bytes(bytes, xx);
+                rc = clb_logic_path_bwd(ptr<float>(xx), ptr<float>(ww), ptr<float>(cc), ptr<float>(gy), ptr<float>(gx), ptr<float>(gw),
+                                        ptr<int32_t>(plan->start32), ptr(plan->entry), ptr(plan->rec), ptr<int32_t>(plan->open), plan->n_open, ptr(scratch),
+                                        bytes, in, out, batch, wmode, cur_stream());
+                if (rc != CLB_ERR_SHAPE) check(rc);
+            }
+            const size_t bytes = rc == CLB_ERR_SHAPE && need_gx && need_gw && plan ? clb_logic_bwd_scratch_bytes(in, out, batch) : 0;
+            if (rc == CLB_ERR_SHAPE && need_gx && plan && (bytes || !need_gw)) { // both gradients in one pass, where that is the faster way
                 const Tensor cc = coef.unpack();
                 Tensor scratch;
                 if (need_gw) scratch = scratch_bytes(bytes, xx);
@@ -683,7 +706,12 @@ Tensor logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w_
             if (plan) coef = alloc({out, 4}, x);
         }
         if (!coef.defined() && clb_logic_fwd_scratch_bytes(in, out, batch, dt)) coef = alloc({out, 4}, x); // (then not kept)
-        if (batch && out)
+        int rc = CLB_ERR_SHAPE;
+        if (batch && out && plan && plan->path_fwd(batch)) {
+            rc = clb_logic_path_fwd(ptr<float>(x_fm), ptr(plan->rec), ptr<float>(w), ptr<float>(y), ptr<float>(coef), in, out, batch, wmode, cur_stream());
+            if (rc != CLB_ERR_SHAPE) check(rc);
+        }
+        if (batch && out && rc == CLB_ERR_SHAPE)
             check(clb_logic_fwd_coef(ptr(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(w), ptr(y), ptr(coef), in, out, batch, wmode, dt, cur_stream()));
     }
     if (graph) {

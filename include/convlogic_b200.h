@@ -262,6 +262,23 @@ size_t clb_logic_bwd_scratch_bytes(int64_t in_dim, int64_t out_dim, int64_t B);
 int clb_logic_bwd(const float *x, const float *w, const float *coef, const float *gy, float *gx, float *gw, const int32_t *start32,
                   const void *entry, void *scratch, size_t scratch_bytes, int64_t in_dim, int64_t out_dim, int64_t B, int wmode,
                   void *stream);
+/* The same layer walked as paths: features are vertices, neurons edges, and consecutive neurons share a feature, so that a pass
+ * reads one row of x per neuron (and one of gy), each about once.  clb_logic_path lays the walk out from the tables above: rec
+ * 16 bytes per neuron (16-byte aligned), open int32 [in], count int32 [2] on the device = (neurons laid out: anything but out_dim means
+ * that lists and connections disagree and rec must not be used; entries of open, the features whose input gradient the walk does
+ * not complete).  clb_logic_path_pays: is it the faster way (what: 0 forward, 1 backward)?  The passes themselves take every size.
+ * The forward writes coef as clb_logic_fwd_coef does; the backward takes both gradients, scratch
+ * clb_logic_path_bwd_scratch_bytes, 16-byte aligned.  CLB_ERR_SHAPE for w, coef or gw that are not 16-byte aligned. */
+size_t clb_logic_path_scratch_bytes(int64_t in_dim, int64_t out_dim);
+int clb_logic_path(const int64_t *a, const int64_t *b, const int32_t *start32, const void *entry, void *rec, int32_t *open, int32_t *count,
+                   void *scratch, size_t scratch_bytes, int64_t in_dim, int64_t out_dim, void *stream);
+int clb_logic_path_pays(int64_t in_dim, int64_t out_dim, int64_t B, int64_t n_open, int what);
+int clb_logic_path_fwd(const float *x, const void *rec, const float *w, float *y, float *coef, int64_t in_dim, int64_t out_dim, int64_t B,
+                       int wmode, void *stream);
+size_t clb_logic_path_bwd_scratch_bytes(int64_t out_dim, int64_t B);
+int clb_logic_path_bwd(const float *x, const float *w, const float *coef, const float *gy, float *gx, float *gw, const int32_t *start32,
+                       const void *entry, const void *rec, const int32_t *open, int64_t n_open, void *scratch, size_t scratch_bytes,
+                       int64_t in_dim, int64_t out_dim, int64_t B, int wmode, void *stream);
 int clb_logic_bwd_w(const void *x, const int64_t *a, const int64_t *b, const void *w, const void *gy, void *gw,
                     int64_t in_dim, int64_t out_dim, int64_t B, int wmode, int dtype, void *stream);
 int clb_logic_bwd_x(const void *x, const int64_t *a, const int64_t *b, const void *w, const void *gy, void *gx,

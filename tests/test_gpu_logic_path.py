@@ -1,0 +1,152 @@
+"""Flat layers walked as paths, against autograd through the gates in fp64: batches around the 32- and 64-sample stretches, rows of
+16-, 8- and 4-byte alignment, layers of a neuron to a few thousand, and connections whose graph is unlike the constructor's."""
+
+import ctypes as C
+
+import pytest
+import torch
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _ptr(t):
+    return C.c_void_p(t.data_ptr())
+
+
+def _stream():
+    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+
+def _plan(a, b, fin):
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    lib, fout = _lib.lib(), a.numel()
+    start, cons = (t.cuda() for t in cb.LogicLayer.build_consumer_lists(a, b, fin))
+    a, b = a.cuda(), b.cuda()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    p = dict(a=a, b=b, start=torch.empty(fin + 1, **i32), entry=torch.empty(2 * fout, 2, **i32), rec=torch.empty(fout, 4, **i32),
+             open=torch.empty(fin, **i32), count=torch.empty(2, **i32))
+    assert lib.clb_logic_entries(_ptr(a), _ptr(b), _ptr(start), _ptr(cons), _ptr(p["start"]), _ptr(p["entry"]), fin, fout, _stream()) == 0
+    n = lib.clb_logic_path_scratch_bytes(fin, fout)
+    scratch = torch.empty(n, dtype=torch.uint8, device="cuda")
+    assert lib.clb_logic_path(_ptr(a), _ptr(b), _ptr(p["start"]), _ptr(p["entry"]), _ptr(p["rec"]), _ptr(p["open"]), _ptr(p["count"]), _ptr(scratch), n,
+                              fin, fout, _stream()) == 0
+    return p
+
+
+def _connections(kind, fin, fout):
+    g = torch.Generator().manual_seed(fin + fout)
+    if kind == "twice":      # every feature read exactly twice (fin = fout): what the constructor draws
+        c = torch.randperm(2 * fout, generator=g) % fin
+        return c[:fout].clone(), c[fout:].clone()
+    if kind == "any":        # any number of readers, a neuron that reads one feature twice, features nobody reads
+        a, b = torch.randint(0, fin, (fout,), generator=g), torch.randint(0, max(1, fin - 1), (fout,), generator=g)
+        b[0] = a[0]
+        return a, b
+    if kind == "pairs":      # neurons 2i and 2i + 1 read the same two features: closed trails of two neurons
+        a = torch.arange(fout) // 2 * 2 % fin
+        return a, (a + 1) % fin
+    a = torch.arange(fout) % fin   # one long trail
+    return a, (a + 1) % fin
+
+
+def _check_plan(p, fin, fout):
+    laid, n_open = p["count"].tolist()
+    rec = p["rec"].cpu().long()
+    j, second = rec[:, 0] >> 1, (rec[:, 0] & 1).bool()
+    a, b = p["a"].cpu()[j], p["b"].cpu()[j]
+    assert laid == fout and torch.equal(j.sort().values, torch.arange(fout))
+    assert torch.equal(torch.where(second, b, a), rec[:, 1]) and torch.equal(torch.where(second, a, b), rec[:, 2])
+    linked, closes = (rec[:, 3] & 1).bool(), (rec[:, 3] & 2).bool()
+    assert not linked[0] and torch.equal(rec[1:, 1][linked[1:]], rec[:-1, 2][linked[1:]])
+    assert bool((linked | ~closes).all())
+    both = torch.cat([rec[:, 1][closes], p["open"][:n_open].cpu().long()])
+    assert torch.equal(both.sort().values, torch.arange(fin))
+    return n_open
+
+
+@pytest.mark.parametrize("kind,fin,fout,batch", [
+    ("twice", 1, 1, 1), ("twice", 2, 2, 4), ("twice", 40, 40, 33), ("twice", 300, 300, 64), ("twice", 300, 300, 66), ("twice", 1000, 1000, 31),
+    ("twice", 3000, 3000, 520), ("twice", 3000, 3000, 513), ("twice", 3001, 3001, 514), ("twice", 20000, 20000, 16), ("any", 7, 9, 5),
+    ("any", 500, 900, 100), ("any", 900, 500, 36), ("pairs", 600, 600, 96), ("trail", 5000, 5000, 40), ("trail", 3, 200, 12)])
+def test_path_passes_against_oracle(kind, fin, fout, batch):
+    from convlogic_b200 import _lib
+
+    lib = _lib.lib()
+    a, b = _connections(kind, fin, fout)
+    p = _plan(a, b, fin)
+    n_open = _check_plan(p, fin, fout)
+    g = torch.Generator().manual_seed(batch)
+    w = torch.randn(fout, 16, generator=g)
+    x, gy = torch.rand(fin, batch, generator=g), torch.randn(fout, batch, generator=g)
+    xd, gyd, wd = x.cuda(), gy.cuda(), w.cuda()
+    y, coef = torch.empty(fout, batch, device="cuda"), torch.empty(fout, 4, device="cuda")
+    assert lib.clb_logic_path_fwd(_ptr(xd), _ptr(p["rec"]), _ptr(wd), _ptr(y), _ptr(coef), fin, fout, batch, _lib.W_SOFTMAX, _stream()) == 0
+    n = lib.clb_logic_path_bwd_scratch_bytes(fout, batch)
+    scratch = torch.empty(n, dtype=torch.uint8, device="cuda")
+
+    def backward():
+        gx, gw = torch.full_like(xd, float("nan")), torch.full_like(wd, float("nan"))
+        assert lib.clb_logic_path_bwd(_ptr(xd), _ptr(wd), _ptr(coef), _ptr(gyd), _ptr(gx), _ptr(gw), _ptr(p["start"]), _ptr(p["entry"]), _ptr(p["rec"]),
+                                      _ptr(p["open"]), n_open, _ptr(scratch), n, fin, fout, batch, _lib.W_SOFTMAX, _stream()) == 0
+        return gx, gw
+
+    gx, gw = backward()
+    xo, wo = x.t().double().requires_grad_(True), w.double().requires_grad_(True)
+    yo = oracle.logic_layer(xo, a, b, oracle.gate_probabilities(wo, True))
+    yo.backward(gy.t().double())
+
+    def close(got, want):
+        # sums of up to 520 products of fp32 values: an error of a few roundings of the largest
+        return float((got.cpu().double() - want).abs().max()) <= 1e-5 * float(want.abs().max())
+
+    assert close(y, yo.detach().t()) and close(gx, xo.grad.t()) and close(gw, wo.grad)
+    p2 = _plan(a, b, fin)    # the trails may be laid out in another order, the sums stay as they are
+    p["rec"], p["open"], n_open = p2["rec"], p2["open"], _check_plan(p2, fin, fout)
+    again = backward()
+    assert torch.equal(gx, again[0]) and torch.equal(gw, again[1])
+
+
+def test_lists_that_contradict_the_connections_are_noticed():
+    fin = fout = 64
+    a, b = _connections("twice", fin, fout)
+    p = _plan(a, b, fin)
+    other = _plan(a.flip(0), b.flip(0), fin)
+    lib_args = [_ptr(p["a"]), _ptr(p["b"]), _ptr(other["start"]), _ptr(other["entry"])]
+    from convlogic_b200 import _lib
+
+    n = _lib.lib().clb_logic_path_scratch_bytes(fin, fout)
+    scratch = torch.empty(n, dtype=torch.uint8, device="cuda")
+    assert _lib.lib().clb_logic_path(*lib_args, _ptr(p["rec"]), _ptr(p["open"]), _ptr(p["count"]), _ptr(scratch), n, fin, fout, _stream()) == 0
+    rec = p["rec"].cpu().long()
+    if int(p["count"][0]) == fout:   # every neuron once all the same: then a linked neuron does read what the one before read
+        linked = (rec[1:, 3] & 1).bool()
+        assert torch.equal(rec[1:, 1][linked], rec[:-1, 2][linked])
+
+
+@pytest.mark.parametrize("width,batch,path", [(40000, 210, True), (40000, 200, False), (83400, 101, True), (83000, 101, False), (28000, 900, True)])
+def test_layers_take_the_path_by_size(width, batch, path):
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib, ops
+    from convlogic_b200._lib import W_SOFTMAX
+
+    torch.manual_seed(batch)
+    layer = cb.LogicLayer(width, width).cuda().train()
+    x, gy = torch.rand(width, batch, device="cuda"), torch.randn(width, batch, device="cuda")
+    tables = (layer.indices_0, layer.indices_1, layer.weights.detach())
+    xd = x.t().detach().requires_grad_(True)
+    _lib.trace(True)
+    y = layer(xd)
+    y.backward(gy.t())
+    torch.cuda.synchronize()
+    names = _lib.trace_report()
+    _lib.trace(False)
+    assert ("logic_path_bwd_kernel" in names) == path, names
+    # the same terms in another order
+    for got, want in ((y.detach().t(), ops.logic_fwd(x, *tables, W_SOFTMAX)),
+                      (xd.grad.t(), ops.logic_bwd_x(x, *tables, gy, layer.given_x_indices_of_y_start, layer.given_x_indices_of_y, W_SOFTMAX)),
+                      (layer.weights.grad, ops.logic_bwd_w(x, *tables, gy, W_SOFTMAX))):
+        assert (got - want).norm() <= 1e-5 * want.norm()
