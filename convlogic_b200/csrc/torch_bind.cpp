@@ -535,30 +535,39 @@ struct LogicPlan {
     LogicKey key;
     int64_t in = 0, out = 0;
     Tensor start32, entry;
-    Tensor rec, open;    // neurons in the order of paths, features whose gradient a path does not complete; undefined: lists and connections disagree
+    bool paths = false;
+    Tensor rec, open;    // (paths) neurons in the order of paths, features whose gradient a path does not complete; undefined: lists and connections disagree
     int64_t n_open = 0;
     bool path_fwd(int64_t batch) const { return rec.defined() && clb_logic_path_pays(in, out, batch, n_open, 0); }
     bool path_bwd(int64_t batch) const { return rec.defined() && clb_logic_path_pays(in, out, batch, n_open, 1); }
 };
 using LogicPlanPtr = std::shared_ptr<LogicPlan>;
 
-LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const Tensor &b, const Tensor &start, const Tensor &cons, int64_t in, int64_t out)
+// paths: with the neurons in the order of paths (a plan is never changed: one without is replaced by one that shares its lists)
+LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const Tensor &b, const Tensor &start, const Tensor &cons, int64_t in, int64_t out,
+                            bool paths)
 {
     const LogicKey key = logic_key(a, b, start, cons);
-    if (LogicPlanPtr p = kept<LogicPlan>(start_obj); p && p->key == key && p->in == in && p->out == out) return p;
+    LogicPlanPtr old = kept<LogicPlan>(start_obj);
+    if (old && !(old->key == key && old->in == in && old->out == out)) old = nullptr;
+    if (old && (old->paths || !paths)) return old;
     need_inputs(a, b, start, cons);
     TORCH_CHECK(start.scalar_type() == at::kLong && cons.scalar_type() == at::kLong && start.numel() == in + 1 && cons.numel() == 2 * out,
                 "convlogic_b200: consumer lists must be int64 [in_dim + 1] and [2 * out_dim]");
     if (in > 0x3fffffff || out > 0x3fffffff) return nullptr;
     // inside a stream capture nothing would be laid out before the replay: this call runs the two separate gradient kernels
-    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return nullptr;
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return old;
     auto p = std::make_shared<LogicPlan>();
-    p->key = key, p->in = in, p->out = out;
+    p->key = key, p->in = in, p->out = out, p->paths = paths;
     Below below(start);
-    p->start32 = alloc({in + 1}, start, at::kInt), p->entry = alloc({2 * out, 2}, start, at::kInt);
-    check(clb_logic_entries(ptr<int64_t>(a), ptr<int64_t>(b), ptr<int64_t>(start), ptr<int64_t>(cons), ptr<int32_t>(p->start32), ptr(p->entry), in, out,
-                            cur_stream()));
-    if (out) {
+    if (old) {
+        p->start32 = old->start32, p->entry = old->entry;
+    } else {
+        p->start32 = alloc({in + 1}, start, at::kInt), p->entry = alloc({2 * out, 2}, start, at::kInt);
+        check(clb_logic_entries(ptr<int64_t>(a), ptr<int64_t>(b), ptr<int64_t>(start), ptr<int64_t>(cons), ptr<int32_t>(p->start32), ptr(p->entry), in, out,
+                                cur_stream()));
+    }
+    if (paths && out) {
         const size_t bytes = clb_logic_path_scratch_bytes(in, out);
         const Tensor scratch = scratch_bytes(bytes, start), count = alloc({2}, start, at::kInt);
         p->rec = alloc({out, 4}, start, at::kInt), p->open = alloc({in}, start, at::kInt);
@@ -702,7 +711,7 @@ Tensor logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w_
         x_fm = fm ? x.contiguous() : feature_major_storage(x);
         y = fm ? alloc({out, batch}, x) : alloc_strided({batch, out}, {1, std::max<int64_t>(batch, 1)}, x);
         if (graph && x.requires_grad() && dt == CLB_F32 && out) { // the backward takes both gradients in one pass
-            plan = logic_plan_for(start_obj, a, b, start, cons, in, out);
+            plan = logic_plan_for(start_obj, a, b, start, cons, in, out, clb_logic_path_pays(in, out, batch, 0, 0) || clb_logic_path_pays(in, out, batch, 0, 1));
             if (plan) coef = alloc({out, 4}, x);
         }
         if (!coef.defined() && clb_logic_fwd_scratch_bytes(in, out, batch, dt)) coef = alloc({out, 4}, x); // (then not kept)
