@@ -349,6 +349,66 @@ __global__ void __launch_bounds__(256) packed_logic_kernel(const V *__restrict__
     }
 }
 
+constexpr int kPathBlocks = 6; // packed_path_kernel: resident per SM
+
+// The same layer walked as paths (logic_path.cu: the next neuron reads what the last one read second): one gathered row per neuron
+// instead of two.  A group of 2^LG lanes owns a range of positions and a stretch of R units per lane.  What bound it first was the issue
+// of integer instructions (171 per neuron and stretch of five words): offsets within a row are constants now, which lanes are inside
+// it is found once, and a gate's four masks come from a table; then the bytes in flight, for which many warps with one row each beat
+// fewer with two to four (us for one layer, x in the L2 as the layer before leaves it, two rows per neuron / this with four blocks and two
+// rows / with six and one: 3072 -> 64000 neurons, 1252 bytes 37 / 23 / 23, 64000 -> 64000 45 / 41 / 37, 128000 x 2500 171 / 141 / 128).
+template <typename V, int R, int LG>
+__global__ void __launch_bounds__(256, kPathBlocks) packed_path_kernel(const V *__restrict__ x, const int4 *__restrict__ rec, const uint8_t *__restrict__ ops,
+                                                             V *__restrict__ y, int n, int units, int cols, int ranges)
+{
+    constexpr int N = Words<V>::N, G = 1 << LG;
+    __shared__ uint4 masks[32]; // of gate op, and from 16 on of the gate with its inputs swapped
+    if (threadIdx.x < 32) {
+        const int op = threadIdx.x & 15, o = threadIdx.x < 16 ? op : (op & 9) | (op & 2) << 1 | (op & 4) >> 1;
+        masks[threadIdx.x] = make_uint4(o & 1 ? ~0u : 0u, o & 2 ? ~0u : 0u, o & 4 ? ~0u : 0u, o & 8 ? ~0u : 0u);
+    }
+    __syncthreads();
+    const int unit = (int)((blockIdx.x * 256u + threadIdx.x) >> LG), range = unit / cols, col = unit - range * cols;
+    const int turns = (n + ranges - 1) / ranges, p0 = range * turns, p1 = min(n, p0 + turns), u0 = col * G * R + (threadIdx.x & (G - 1));
+    if (p0 >= p1 || u0 >= units) return;
+    x += u0, y += u0;
+    bool in[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) in[r] = u0 + r * G < units;
+    Words<V> a[R];
+    auto load = [&](Words<V>(&row)[R], int f) {
+        const V *p = x + (size_t)f * units;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+            if (in[r]) row[r] = load_words(p + r * G);
+    };
+    int4 next = __ldg(rec + p0);
+    load(a, next.y);
+    next.w |= 1; // (linked: the row entered through is there)
+    for (int p = p0; p < p1; ++p) {
+        const int4 t = next;
+        Words<V> b[R];
+        load(b, t.z);
+        const int op = __ldg(ops + (t.x >> 1));
+        if (p + 1 < p1) next = __ldg(rec + p + 1);
+        if (!(t.w & 1)) load(a, t.y);
+        const uint4 m = masks[op & 15 | (t.x & 1) << 4];
+        V *row = y + (size_t)(t.x >> 1) * units;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            V v;
+            unsigned *w = reinterpret_cast<unsigned *>(&v);
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+                const unsigned va = a[r].w[i], vb = b[r].w[i], r1 = (vb & m.x) | (~vb & m.y), r0 = (vb & m.z) | (~vb & m.w);
+                w[i] = (va & r1) | (~va & r0);
+            }
+            if (in[r]) row[r * G] = v;
+            a[r] = b[r];
+        }
+    }
+}
+
 // bytes 4 w .. 4 w + 3 from p on, of which `valid` (more than 4: all) belong to the row: only words that hold one of those are read
 __device__ __forceinline__ unsigned word_at(const uint8_t *p, long long w, long long valid = 4)
 {
@@ -1117,6 +1177,63 @@ extern "C" int clb_packed_logic(const void *x, const int64_t *a, const int64_t *
                    packed_logic_bytes_kernel<<<blocks(lg), 256, 0, st>>>((const uint8_t *)x, a, b, ops, (uint8_t *)y, out_dim, (int)rowbytes, lg));
     }
     return check_launch();
+}
+
+// From 6 MB of output on, where no input is left unread (20000 x 500 bytes 11.9 / 9.8 us, 100000 x 68 22.9 / 9.5; below, the eight positions in
+// turn of a range take longer than the second row: 5000 x 400 8 / 13, 2000 x 40 7 / 11).
+extern "C" int clb_packed_path_pays(int64_t in_dim, int64_t out_dim, int64_t words, int bits)
+{
+    if (in_dim <= 0 || out_dim < in_dim || words <= 0 || !bits_ok(bits)) return 0;
+    const int64_t rowbytes = words * (bits / 8);
+    return rowbytes % 4 == 0 && out_dim * rowbytes >= (6LL << 20);
+}
+
+extern "C" int clb_packed_path(const void *x, const void *rec, const uint8_t *ops, void *y, int64_t in_dim, int64_t out_dim, int64_t words, int bits,
+                               void *stream)
+{
+    if (!x || !rec || !ops || !y || in_dim <= 0 || out_dim < 0 || words < 0 || !bits_ok(bits)) return CLB_ERR_ARG;
+    const long long rowbytes = words * (bits / 8);
+    if (out_dim == 0 || rowbytes == 0) return CLB_OK;
+    if (rowbytes % 4 || rowbytes > 0x7fffffffLL || in_dim > 0x3fffffff || out_dim > 0x3fffffff || !aligned_to(rec, 16) || !aligned_to(x, 4) || !aligned_to(y, 4))
+        return CLB_ERR_SHAPE;
+    cudaStream_t st = (cudaStream_t)stream;
+    auto go = [&](auto unit, auto per, auto lanes) {
+        using V = decltype(unit);
+        constexpr int R = decltype(per)::value, LG = decltype(lanes)::value;
+        const long long units = rowbytes / (long long)sizeof(V), cols = (units + (R << LG) - 1) / (R << LG), groups = (long long)sm_count() * kPathBlocks * 256 >> LG;
+        long long ranges = groups / cols; // one wave of resident blocks, eight positions per group at least
+        if (ranges > out_dim / 8) ranges = out_dim / 8;
+        if (ranges < 1) ranges = 1;
+        if (((ranges * cols) << LG) + 255 > 0x7fffffffLL) return (int)CLB_ERR_SHAPE;
+        CLB_TRACED("packed_path_kernel", st,
+                   packed_path_kernel<V, R, LG><<<(unsigned)(((ranges * cols << LG) + 255) / 256), 256, 0, st>>>((const V *)x, (const int4 *)rec, ops, (V *)y,
+                                                                                                              (int)out_dim, (int)units, (int)cols, (int)ranges));
+        return check_launch();
+    };
+    // a warp takes 2 to 5 (of 8 bytes 4, of 16 bytes 2) units per lane, whichever leaves the fewest lanes idle; short rows a quarter of a warp and two
+    auto rows = [&](auto unit) {
+        using V = decltype(unit);
+        const long long units = rowbytes / (long long)sizeof(V);
+        constexpr int most = sizeof(V) == 16 ? 2 : sizeof(V) == 8 ? 4 : 5;
+        if (units <= 32) return go(unit, std::integral_constant<int, 2>{}, std::integral_constant<int, 3>{});
+        int best = 2;
+        long long idle = -1;
+        for (int r = most; r >= 2; --r) {
+            const long long over = (units + 32 * r - 1) / (32 * r) * (32 * r);
+            if (idle < 0 || over < idle) best = r, idle = over;
+        }
+        const auto warp = std::integral_constant<int, 5>{};
+        if constexpr (most >= 5)
+            if (best == 5) return go(unit, std::integral_constant<int, 5>{}, warp);
+        if constexpr (most >= 4) {
+            if (best == 4) return go(unit, std::integral_constant<int, 4>{}, warp);
+            if (best == 3) return go(unit, std::integral_constant<int, 3>{}, warp);
+        }
+        return go(unit, std::integral_constant<int, 2>{}, warp);
+    };
+    if (rowbytes % 16 == 0 && aligned_to(x, 16) && aligned_to(y, 16)) return rows(uint4{});
+    if (rowbytes % 8 == 0 && aligned_to(x, 8) && aligned_to(y, 8)) return rows(uint2{});
+    return rows(0u);
 }
 
 extern "C" int clb_packed_tree(const void *x, const int32_t *leaf, const uint8_t *ops, void *y, int64_t in_dim, int64_t out_dim, int levels,

@@ -1006,12 +1006,28 @@ std::pair<Tensor, int64_t> pack_bits(const Tensor &t, int bits, bool sample_majo
     return {packed, (bits - b % bits) % bits};
 }
 
-Tensor packed_logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &ops)
+// start_obj, cons: the layer's consumer lists, or None: the neurons in their own order
+Tensor packed_logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &ops, const py::object &start_obj, const std::optional<Tensor> &cons)
 {
     need_inputs(x, a, b, ops);
     TORCH_CHECK(ops.scalar_type() == at::kByte, "convlogic_b200: gate ids must be uint8");
     Below below(x);
     Tensor y = alloc({ops.size(0), x.size(1)}, x);
+    const int bits = (int)x.element_size() * 8;
+    if (!start_obj.is_none() && cons && a.numel() == ops.size(0) && b.numel() == ops.size(0) &&
+        clb_packed_path_pays(x.size(0), ops.size(0), x.size(1), bits)) {
+        const Tensor start = start_obj.cast<Tensor>();
+        auto list = [&](const Tensor &t, int64_t n) { return t.scalar_type() == at::kLong && t.numel() == n && t.is_contiguous() && t.device() == x.device(); };
+        // (inference tensors carry no version to tell a change by)
+        if (!(a.is_inference() || b.is_inference() || start.is_inference() || cons->is_inference()) && list(start, x.size(0) + 1) && list(*cons, 2 * ops.size(0))) {
+            const LogicPlanPtr plan = logic_plan_for(start_obj, a, b, start, *cons, x.size(0), ops.size(0), true);
+            if (plan && plan->rec.defined()) {
+                const int rc = clb_packed_path(ptr(x), ptr(plan->rec), ptr<uint8_t>(ops), ptr(y), x.size(0), ops.size(0), x.size(1), bits, cur_stream());
+                if (rc == CLB_OK) return y;
+                if (rc != CLB_ERR_SHAPE) check(rc);
+            }
+        }
+    }
     check(clb_packed_logic(ptr(x), ptr<int64_t>(a), ptr<int64_t>(b), ptr<uint8_t>(ops), ptr(y), x.size(0), ops.size(0), x.size(1), (int)x.element_size() * 8,
                            cur_stream()));
     return y;
@@ -1143,7 +1159,8 @@ PYBIND11_MODULE(_clb_torch, m)
     m.def("adam_step", &adam_step);
     m.def("count_sinks", [](int64_t change) { g_sinks += change; });
     m.def("pack_bits", &pack_bits);
-    m.def("packed_logic", &packed_logic);
+    m.def("packed_logic", &packed_logic, py::arg("x"), py::arg("a"), py::arg("b"), py::arg("ops"), py::arg("start") = py::none(),
+          py::arg("consumers") = std::nullopt);
     m.def("group_popcount", &group_popcount);
     py::class_<Net>(m, "Net")
         .def(py::init([](const py::bytes &blob, const std::string &device) { return std::make_unique<Net>(blob, c10::Device(device)); }))

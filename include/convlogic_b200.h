@@ -299,6 +299,10 @@ int clb_pack_bits_nmajor(const uint8_t *t, void *packed, int64_t N, int64_t F, i
  * x [in,words], ops uint8 [out] gate ids 0..15 -> y [out,words]. */
 int clb_packed_logic(const void *x, const int64_t *a, const int64_t *b, const uint8_t *ops, void *y,
                      int64_t in_dim, int64_t out_dim, int64_t words, int bits, void *stream);
+/* The same on the paths of clb_logic_path (rec).  CLB_ERR_SHAPE for rows that are not whole 4-byte words.  _pays: is it the faster way? */
+int clb_packed_path_pays(int64_t in_dim, int64_t out_dim, int64_t words, int bits);
+int clb_packed_path(const void *x, const void *rec, const uint8_t *ops, void *y, int64_t in_dim, int64_t out_dim, int64_t words, int bits,
+                    void *stream);
 /* Replaces difflogic_cuda.groupbitsum (difflogic.cpp:22-33; difflogic_kernel.cu:418-482).
  * x [F,words] -> counts int32 [B,k], B = words*bits - pad_len; F must be divisible by k
  * (CLB_ERR_SHAPE otherwise, the reference's ValueError). */

@@ -76,3 +76,48 @@ def test_more_thermometer_levels_than_a_pass(n, side, levels, bytes_):
     bits = torch.cat([px.float() / 255 > t for t in th], dim=1)
     want, _ = ops.pack_bits(bits.reshape(n, -1), 64, sample_major=True)
     assert torch.equal(got.reshape(want.shape), want)
+
+
+@pytest.mark.parametrize("bits,words", [(8, 4), (8, 68), (16, 34), (32, 1), (32, 31), (32, 161), (64, 1), (64, 17), (64, 41), (64, 129), (32, 400)])
+@pytest.mark.parametrize("fin,fout", [(1, 1), (300, 300), (50, 1000), (700, 400)])
+def test_packed_layer_on_paths(bits, words, fin, fout):
+    """Rows of 4-, 8- and 16-byte alignment, around the widths at which lanes and stretches change, against the neurons' own order."""
+    import ctypes as C
+
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    g = torch.Generator().manual_seed(words + fin)
+    a, b = torch.randint(0, fin, (fout,), generator=g), torch.randint(0, fin, (fout,), generator=g)
+    if fin == fout:
+        c = torch.randperm(2 * fout, generator=g) % fin
+        a, b = c[:fout].contiguous(), c[fout:].contiguous()
+    start, cons = (t.cuda() for t in cb.LogicLayer.build_consumer_lists(a, b, fin))
+    a, b, ops = a.cuda(), b.cuda(), torch.randint(0, 16, (fout,), generator=g, dtype=torch.uint8).cuda()
+    x = torch.randint(0, 256, (fin, words * bits // 8), generator=g, dtype=torch.uint8).cuda().view({8: torch.int8, 16: torch.int16, 32: torch.int32, 64: torch.int64}[bits])
+    lib, ptr, stream = _lib.lib(), lambda t: C.c_void_p(t.data_ptr()), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    s32, entry, rec, open_, count = (torch.empty(n, **i32) for n in (fin + 1, 4 * fout, 4 * fout, fin, 2))
+    n = lib.clb_logic_path_scratch_bytes(fin, fout)
+    scratch, y = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.empty(fout, words, dtype=x.dtype, device="cuda")
+    assert lib.clb_logic_entries(ptr(a), ptr(b), ptr(start), ptr(cons), ptr(s32), ptr(entry), fin, fout, stream) == 0
+    assert lib.clb_logic_path(ptr(a), ptr(b), ptr(s32), ptr(entry), ptr(rec), ptr(open_), ptr(count), ptr(scratch), n, fin, fout, stream) == 0
+    assert lib.clb_packed_path(ptr(x), ptr(rec), ptr(ops), ptr(y), fin, fout, words, bits, stream) == 0
+    assert torch.equal(y, _lib.native().packed_logic(x, a, b, ops))
+
+
+def test_large_packed_layers_take_the_paths_by_themselves():
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    torch.manual_seed(0)
+    layer = cb.LogicLayer(30000, 30000).cuda().eval()
+    layer.weights.data.normal_()
+    x = cb.PackBitsTensor(torch.rand(2000, 30000, device="cuda") < 0.5, 32)
+    _lib.trace(True)
+    y = layer(x)
+    torch.cuda.synchronize()
+    names = _lib.trace_report()
+    _lib.trace(False)
+    assert "packed_path_kernel" in names, names
+    assert torch.equal(y.rows(), _lib.native().packed_logic(x.rows(), layer.indices_0, layer.indices_1, layer._gate_ids()))
