@@ -94,7 +94,7 @@ __device__ __forceinline__ void window_bwd(const float (&a)[8], const Gate<float
 int clb_plane_parts(int N, int C, int images_per_iteration, int groups, int resident);
 
 // Pass 1 of the backward of a block of square images of 32, 28, 16, 12 or 6 pixels (convtree_tile.cu): partial [parts][C][28] basis
-// sums, planes [N][C][2][side * side] gradients of the two input channels of every output channel.  gy, amax and x are those
+// sums, planes [C][2][N][side * side] gradients of the two input channels of every output channel.  gy, amax and x are those
 // of the first of the N images; fm: gy is [C][windows][n_stride].
 struct ClbTileBwd {
     const float *gy, *x, *w;

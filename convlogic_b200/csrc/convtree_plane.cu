@@ -604,9 +604,9 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const floa
         const int u = lane + 32 * q;
         constexpr int W4 = S / 4;
         const int col4 = u % W4, row = (u / W4) % S, slot = (u / (W4 * S)) & 1, img = u / (W4 * S * 2);
-        pdst[q] = planes + (((size_t)(n_lo + img) * s.C + c) * 2 + slot) * HW + row * S + col4 * 4;
+        pdst[q] = planes + (((size_t)c * 2 + slot) * s.N + n_lo + img) * HW + row * S + col4 * 4;
     }
-    const size_t pstep = (size_t)Cf::NIMG * s.C * 2 * HW;
+    constexpr int pstep = Cf::NIMG * HW;
     auto finish = [&]() {
         // write the interior of the gradient planes out and clear it for the next iteration
 #pragma unroll
@@ -797,7 +797,10 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_w_plane32_kernel(const 
 }
 
 // Pass 2: gx[n][ch] = sum of the gradient planes (c, slot) that belong to input channel ch, in list order.
-// `start` [Ci + 1], `entry` [..] = 2*c + slot.  One float4 per thread; grid-stride over N * Ci * HW / 4.
+// `start` [Ci + 1], `entry` [..] = 2*c + slot.  One float4 per thread, of one channel the images one after the other: planes are
+// stored [c][slot][image], so that a block streams through as many runs as the channel's list has entries, and read past the L2.  (Planes
+// of one image after the other, a channel's pieces of 64 bytes to 4 KB apart: 297 us for the three layers of the k = 256 stack at batch 256,
+// 94 for 9 -> 256 channels of 32x32; in runs 262 and 91, past the L2 as well 245 and 77: 5.6 and 7 TB/s.)
 // The first fin.blocks blocks of the same launch finish the gate gradient instead (one thread per gate: the per-part basis
 // sums added in part order, then the 16 gradients): one launch less per layer and step.
 struct GateFinish {
@@ -819,40 +822,31 @@ __device__ __forceinline__ void gate_finish_thread(const GateFinish &fin, long l
 
 template <typename IDX>
 __global__ void __launch_bounds__(256) plane_sum_kernel(const float *__restrict__ planes, const int32_t *__restrict__ start,
-                                                        const int32_t *__restrict__ entry, float *__restrict__ gx, int N, int Ci, int C, int HW4,
-                                                        GateFinish fin)
+                                                        const int32_t *__restrict__ entry, float *__restrict__ gx, int N, int Ci, int HW4, GateFinish fin)
 {
     if ((int)blockIdx.x < fin.blocks) {
         gate_finish_thread(fin, (long long)blockIdx.x * blockDim.x + threadIdx.x);
         return;
     }
-    // IDX: 32-bit when the output has fewer than 2^31 float4 units (the three index divisions per unit are then cheap)
+    // IDX: 32-bit when the output has fewer than 2^31 float4 units (the index divisions are then cheap)
     const IDX block = (IDX)blockIdx.x - (IDX)fin.blocks, nblocks = (IDX)gridDim.x - (IDX)fin.blocks;
-    // (Measured slower at batch 256: two units per thread a grid stride apart with eight streaming loads in flight,
-    // 0.32 -> 0.40 ms per step; walking the images last to first to catch what pass 1 left in L2, 0.32 -> 0.33 ms.)
-    const IDX total = (IDX)N * (IDX)Ci * (IDX)HW4;
+    const IDX run = (IDX)N * (IDX)HW4, total = run * (IDX)Ci;
     for (IDX i = block * (IDX)blockDim.x + (IDX)threadIdx.x; i < total; i += nblocks * (IDX)blockDim.x) {
-        const int e = (int)(i % (IDX)HW4);
-        const IDX r = i / (IDX)HW4;
-        const int ch = (int)(r % (IDX)Ci);
-        const IDX n = r / (IDX)Ci;
-        const int lo = start[ch], hi = start[ch + 1];
+        const int ch = (int)(i / run);
+        const IDX u = i - (IDX)ch * run, n = u / (IDX)HW4;
+        const int e = (int)(u - n * (IDX)HW4), lo = __ldg(start + ch), hi = __ldg(start + ch + 1);
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 *base = reinterpret_cast<const float4 *>(planes) + (size_t)n * C * 2 * HW4 + e;
-        int l = lo;
-        for (; l + 3 < hi; l += 4) { // four loads in flight
-            const float4 a = __ldg(base + (size_t)entry[l] * HW4), b = __ldg(base + (size_t)entry[l + 1] * HW4);
-            const float4 p = __ldg(base + (size_t)entry[l + 2] * HW4), q = __ldg(base + (size_t)entry[l + 3] * HW4);
-            acc.x += a.x, acc.y += a.y, acc.z += a.z, acc.w += a.w;
-            acc.x += b.x, acc.y += b.y, acc.z += b.z, acc.w += b.w;
-            acc.x += p.x, acc.y += p.y, acc.z += p.z, acc.w += p.w;
-            acc.x += q.x, acc.y += q.y, acc.z += q.z, acc.w += q.w;
+        const float4 *base = reinterpret_cast<const float4 *>(planes) + u;
+        for (int l = lo; l < hi; l += 4) { // (three or eight at a time: 2 and 14 % slower)
+            float4 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (l + k < hi) v[k] = __ldcs(base + (size_t)__ldg(entry + l + k) * run);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (l + k < hi) acc.x += v[k].x, acc.y += v[k].y, acc.z += v[k].z, acc.w += v[k].w;
         }
-        for (; l < hi; ++l) {
-            const float4 a = __ldg(base + (size_t)entry[l] * HW4);
-            acc.x += a.x, acc.y += a.y, acc.z += a.z, acc.w += a.w;
-        }
-        reinterpret_cast<float4 *>(gx)[i] = acc;
+        reinterpret_cast<float4 *>(gx)[((size_t)n * Ci + ch) * HW4 + e] = acc;
     }
 }
 
@@ -1096,7 +1090,7 @@ extern "C" int clb_convtree_bwd_plane(const void *gy, const void *x, const void 
         if (gw && i + 1 == slices) fin.blocks = (int)((fin.ngates + 255) / 256);
         auto sum = [&](auto kernel) {
             CLB_TRACED("plane_sum_kernel", st,
-                       kernel<<<(unsigned)(blocks + fin.blocks), 256, 0, st>>>(planes, ch_start, ch_entry, (float *)gx + pixels, n, Ci, C, HW4, fin));
+                       kernel<<<(unsigned)(blocks + fin.blocks), 256, 0, st>>>(planes, ch_start, ch_entry, (float *)gx + pixels, n, Ci, HW4, fin));
         };
         if (total + (blocks + fin.blocks) * 256 < 0x7fffffffLL)
             sum(plane_sum_kernel<unsigned>);

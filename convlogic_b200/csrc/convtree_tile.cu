@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kThreads, Tile<S>::BLOCKS) convtree_bwd_plane_
     }
     // the thread's units of the planes
     const float *xb = s.x + (size_t)n_lo * s.Ci * HW;
-    float *pb = s.planes + ((size_t)n_lo * s.C + c) * 2 * HW;
+    float *pb = s.planes + ((size_t)c * 2 * s.N + n_lo) * HW;
     constexpr int UR = T::REGULAR ? 1 : UPT; // places kept in registers; those of the others of a regular thread are constants away
     int xoff[UR], poff[UR], uimg[UR];
     uint32_t ucell[UR];
@@ -147,13 +147,13 @@ __global__ void __launch_bounds__(kThreads, Tile<S>::BLOCKS) convtree_bwd_plane_
         const int r = S == 16 ? (k % 4) * 2 + k / 4 : S == 32 ? (k % 2) * 8 + k / 2 : k; // rows of a half-warp's pairs in different banks
         const int y = 2 * r + even;                                                      // padded row y + 1
         xoff[q] = (img * s.Ci + (slot ? si.ch[1] : si.ch[0])) * HW + y * S + QUAD * col4;
-        poff[q] = (img * s.C * 2 + slot) * HW + y * S + QUAD * col4;
+        poff[q] = (slot * s.N + img) * HW + y * S + QUAD * col4;
         ucell[q] = tile + 4u * (uint32_t)(T::LEAD + slot * T::SLOT + (even ? 0 : 2 * T::PL) + img * T::IMG + (r + even) * T::P + QUAD / 2 * col4);
         uimg[q] = u < T::UNITS ? img : 1 << 20;
     }
-    const int second = T::REGULAR ? (si.ch[1] - si.ch[0]) * HW : 0;
+    const int second = T::REGULAR ? (si.ch[1] - si.ch[0]) * HW : 0, second_plane = T::REGULAR ? s.N * HW : 0;
     auto x_at = [&](int q) { return T::REGULAR ? xoff[0] + (q & 1) * S + (q >> 1) * second : xoff[q]; };
-    auto p_at = [&](int q) { return T::REGULAR ? poff[0] + (q & 1) * S + (q >> 1) * HW : poff[q]; };
+    auto p_at = [&](int q) { return T::REGULAR ? poff[0] + (q & 1) * S + (q >> 1) * second_plane : poff[q]; };
     auto cell_at = [&](int q) { return T::REGULAR ? ucell[0] + 4u * (uint32_t)((q & 1) * (T::P - 2 * T::PL) + (q >> 1) * T::SLOT) : ucell[q]; };
     auto img_at = [&](int q) { return uimg[T::REGULAR ? 0 : q]; };
 
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kThreads, Tile<S>::BLOCKS) convtree_bwd_plane_
                 if (img_at(q) < have) *reinterpret_cast<float2 *>(pb + p_at(q)) = make_float2(odd, even);
             }
         }
-        pb += (size_t)NIMG * s.C * 2 * HW;
+        pb += NIMG * HW;
     }
 
     const float sum = warp_sums28(acc, lane);
