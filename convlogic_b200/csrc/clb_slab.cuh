@@ -8,9 +8,12 @@ namespace clb {
 namespace slab {
 struct __align__(16) Rec {
     int4 off[4];               // tile offsets of taps 2i and 2i + 1, each for the left and the right conv column of a window
-    int code[8];               // gate ids folded to 0..7 (7 used) ...
-    unsigned inv[8];           // ... and their output inversion
-    int ch[2], nst, all_in_tile;
+    int code[7];               // gate ids folded to 0..7 ...
+    int c;                     // (output channel)
+    unsigned inv[7];           // ... and their output inversion
+    unsigned fresh;            // planes (bit 0: the first) that the record before does not leave in place
+    int ch[2];                 // input channels of the tile's planes
+    int planes, all_in_tile;   // planes to copy where no record came before
     int word[8];               // the raw selection words (global path)
 };
 } // namespace slab
@@ -30,7 +33,11 @@ __host__ __device__ __forceinline__ int split_position(int pixel, int side) // s
 // does the kernel take this block?  (U > 0 slabs of side * side units below 2^31 in all: 268 million samples of 32x32)
 bool clb_slab3_covers(int H, int W, int sh, int sw, int ph, int pw, int kh, int kw);
 size_t clb_slab3_record_bytes(int C);
-int clb_slab3_records(const uint8_t *ops, const int32_t *sel, void *recs, int Ci, int side, int C, cudaStream_t st);
+// An order of the output channels in which neighbours share input channels: 3 ints each {channel, first plane, second plane | fresh << 16}
+// (host; false: a selection that does not fit two planes, whose records keep the channels' own order)
+bool clb_slab3_order(const int32_t *sel, int Ci, int C, int32_t *order);
+// order: that table on the device, or null
+int clb_slab3_records(const uint8_t *ops, const int32_t *sel, const int32_t *order, void *recs, int Ci, int side, int C, cudaStream_t st);
 // in: kSlabs or kSplitSlabs; out: any order (kSplitSlabs: side >= 8)
 int clb_slab3_block(const void *x, const void *recs, void *y, int Ci, int side, int C, int64_t U, clb::Order in, clb::Order out, cudaStream_t st);
 

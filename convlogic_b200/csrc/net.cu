@@ -29,7 +29,7 @@ namespace {
 
 constexpr char kMagic[8] = {'C', 'L', 'B', 'N', 'E', 'T', '0', '1'};
 constexpr size_t kHeaderBytes = 64, kLayerBytes = 64;
-// The one-launch kernel (net_cluster.cu) against layer-by-layer launches, us per call on B200: mnist k=64 (cost 0.1 M) batch 1 25 / 52,
+// The one-launch kernel (net_cluster.cu, with slabs of 128 samples; smaller ones only lower the first figure) against layer-by-layer launches, us per call on B200: mnist k=64 (cost 0.1 M) batch 1 25 / 52,
 // batch 8192 103 / 148; cifar k=32 (0.13 M) batch 1 31 / 39, batch 2000 57 / 62, batch 8192 131 / 127; cifar k=64 (0.25 M) batch 1
 // 43 / 39, batch 500 43 / 49, batch 1000 66 / 59, batch 8192 233 / 190; cifar k=128 batch 1 66 / 45.  Beyond one slab per SM the
 // clusters come in waves and the layered kernels win from k=32 on.
@@ -55,7 +55,8 @@ struct Layer {
     int levels;
     size_t off_a, off_b, off_ops;
     bool slab3 = false;   // a 3x3 block of the stacks' geometry, which works from tap records ...
-    size_t off_recs = 0;  // ... in the records memory, where the caller gave some
+    size_t off_recs = 0;  // ... in the records memory, where the caller gave some, with the table of their order behind them
+    std::vector<int32_t> order; // (clb_slab3_order)
 };
 
 } // namespace
@@ -77,6 +78,8 @@ struct clb_net {
  // packed.cu
 int clb_net_cluster_launch(const clb::NetPlan &net, const void *input, const float *thresholds, const unsigned char *params, void *work,
                            int32_t *counts, int64_t batch, cudaStream_t st); // net_cluster.cu
+
+static size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 static bool parse(const void *blob, size_t bytes, clb_net &net)
 {
@@ -161,7 +164,7 @@ static bool parse(const void *blob, size_t bytes, clb_net &net)
         }
         if (L.kind == 1 && clb_slab3_covers(L.H, L.W, L.stride, L.stride, L.ph, L.pw, L.kh, L.kw)) {
             L.slab3 = true, L.off_recs = net.record_bytes;
-            net.record_bytes += (clb_slab3_record_bytes(L.C) + 255) / 256 * 256;
+            net.record_bytes += align256(clb_slab3_record_bytes(L.C)) + align256((size_t)L.C * 12);
         }
         net.layers.push_back(L);
     }
@@ -244,6 +247,11 @@ extern "C" int clb_net_create(const void *blob, size_t bytes, void *device_mem, 
         return check_launch(0);
     }
     net->dev = (const unsigned char *)device_mem;
+    for (Layer &L : net->layers) {
+        if (!L.slab3) continue;
+        L.order.resize((size_t)L.C * 3);
+        if (!clb_slab3_order((const int32_t *)((const unsigned char *)blob + L.off_a), L.Ci, L.C, L.order.data())) L.order.clear();
+    }
     plan_one_launch(*net);
     *out = net;
     return CLB_OK;
@@ -256,8 +264,11 @@ extern "C" int clb_net_records(clb_net *net, void *records, void *stream)
     if (!net || (net->record_bytes && (!records || (reinterpret_cast<uintptr_t>(records) & 15)))) return CLB_ERR_ARG;
     for (const Layer &L : net->layers) {
         if (!L.slab3) continue;
-        const int rc = clb_slab3_records(net->dev + L.off_ops, (const int32_t *)(net->dev + L.off_a), (unsigned char *)records + L.off_recs, L.Ci, L.H, L.C,
-                                         (cudaStream_t)stream);
+        unsigned char *recs = (unsigned char *)records + L.off_recs;
+        int32_t *order = L.order.empty() ? nullptr : (int32_t *)(recs + align256(clb_slab3_record_bytes(L.C)));
+        if (order && cudaMemcpyAsync(order, L.order.data(), L.order.size() * sizeof(int32_t), cudaMemcpyHostToDevice, (cudaStream_t)stream) != cudaSuccess)
+            return check_launch(0);
+        const int rc = clb_slab3_records(net->dev + L.off_ops, (const int32_t *)(net->dev + L.off_a), order, recs, L.Ci, L.H, L.C, (cudaStream_t)stream);
         if (rc != CLB_OK) return rc;
     }
     net->records = (const unsigned char *)records;
@@ -278,7 +289,6 @@ extern "C" int clb_net_info(const clb_net *net, int64_t *in_features, int *num_c
 // Activations ping-pong between two buffers sized for the widest layer; the batch is padded to 128 samples so
 // that every pixel row is a whole number of 16-byte units (slab layout, 128-bit kernels).
 static size_t row_bytes(int64_t batch) { return (size_t)((batch + 127) / 128) * 16; }
-static size_t align256(size_t v) { return (v + 255) / 256 * 256; }
 
 static size_t widest(const clb_net *net)
 {
@@ -363,7 +373,7 @@ extern "C" int clb_net_forward(const clb_net *net, int input_kind, const void *i
             if (L.slab3) { // takes either slab order and writes what the next layer reads
                 const void *recs = net->records ? (const void *)(net->records + L.off_recs) : scratch;
                 if (!net->records) {
-                    st = clb_slab3_records(P + L.off_ops, (const int32_t *)(P + L.off_a), scratch, L.Ci, L.H, L.C, cs);
+                    st = clb_slab3_records(P + L.off_ops, (const int32_t *)(P + L.off_a), nullptr, scratch, L.Ci, L.H, L.C, cs);
                     if (st != CLB_OK) return st;
                 }
                 st = clb_slab3_block(buf[cur], recs, buf[cur ^ 1], L.Ci, L.H, L.C, U, order, next, cs);

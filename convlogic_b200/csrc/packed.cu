@@ -1405,7 +1405,7 @@ extern "C" int clb_packed_convtree_slab(const void *x, const uint8_t *ops, const
     if ((long long)Ci * U * H * W >= (1LL << 31) || (long long)C * U * I >= (1LL << 31)) return CLB_ERR_SHAPE;
     if (C == 0 || U == 0) return CLB_OK;
     if (clb_slab3_covers(H, W, sh, sw, ph, pw, kh, kw)) { // the stacks' own geometry
-        const int rc = clb_slab3_records(ops, sel, scratch, Ci, H, C, (cudaStream_t)stream);
+        const int rc = clb_slab3_records(ops, sel, nullptr, scratch, Ci, H, C, (cudaStream_t)stream);
         return rc != CLB_OK ? rc : clb_slab3_block(x, scratch, y, Ci, H, C, U, kSlabs, kSlabs, (cudaStream_t)stream);
     }
     s.U = (int)U;

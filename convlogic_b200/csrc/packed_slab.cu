@@ -12,8 +12,12 @@
 //   * a gate is one lop3 per word whose third operand is the output inversion, so that the sixteen gates are EIGHT cases behind one
 //     indexed branch that a warp takes together;
 //   * eight warps per scheduler at 64 registers a thread, one buffer per block, the copies of one block
-//     running while the SM's others compute (two buffers and half the blocks measured 5 to 30 % slower);
-//   * the tap records (offsets, gate codes) are laid out once per network and arrive two items ahead.
+//     running while the SM's others compute (two buffers and half the blocks measured 5 to 30 % slower), and blocks as small as a
+//     slab or, for small images, a warp or two, so that few threads wait at an item's two barriers (k = 1024, 8192 samples, us with
+//     blocks of 256, 256, 128 threads / of 64, 64, 32: 16x16 images 448 / 378, 8x8 479 / 433, 4x4 252 / 240);
+//   * the tap records (offsets, gate codes) are laid out once per network and arrive two items ahead, in an order in which
+//     neighbours share an input channel (clb_slab3_order), whose plane then stays in the tile: half of the copies, 443, 464, 521, 275 us for
+//     the four blocks in the channels' own order, 411, 452, 483, 254 in that one.
 //
 // Tile of one slab and channel: (S + 1) rows of units of 16 bytes (128 samples of a pixel).  A padded row holds its odd columns,
 // one zero unit, and its even columns: the zero unit is the right halo of the odd columns and the left halo of the even ones,
@@ -23,13 +27,14 @@
 #include "clb_common.cuh"
 #include "clb_slab.cuh"
 
+#include <vector>
+
 namespace clb {
 namespace slab {
 
-// Blocks come in two sizes: the large one, and (but for 32x32 images) one for few slabs, where most of a large block's threads had none.
-template <int S, bool SMALL> struct Geo {
+template <int S> struct Geo {
     static constexpr int H2 = S / 2, I = H2 * H2;                // pooled side, outputs (threads) per slab
-    static constexpr int THREADS = SMALL ? (S == 16 ? 64 : 32) : S == 4 ? 128 : 256;
+    static constexpr int THREADS = S == 32 ? 256 : S == 4 ? 32 : 64;
     static constexpr int UB = THREADS / I;                       // slabs of a block
     static constexpr int PITCH = S == 8 ? 10 : S + 1;            // units of a padded row
     static constexpr int SLAB = S == 4 ? 28 : (S + 1) * PITCH;   // units from one slab to the next
@@ -86,7 +91,8 @@ __device__ __forceinline__ void taps(unsigned (&a)[8], unsigned (&b)[8], const R
 
 struct Shape {
     int Ci, C, U, n_ug;
-    int in, out; // Order
+    int in, out;               // Order
+    int runs, per_run, longer; // runs of items, items of a run, runs that have one more
 };
 
 // one pooled output straight from global memory, for selections the tile does not cover
@@ -118,11 +124,11 @@ template <int S> __device__ __noinline__ uint4 window_global(const uint4 *__rest
     return acc;
 }
 
-template <int S, bool SMALL>
-__global__ void __launch_bounds__(Geo<S, SMALL>::THREADS, 1024 / Geo<S, SMALL>::THREADS)
+template <int S>
+__global__ void __launch_bounds__(Geo<S>::THREADS, 1024 / Geo<S>::THREADS)
     packed_convtree_slab3_kernel(const uint4 *__restrict__ x, const Rec *__restrict__ recs, uint4 *__restrict__ y, Shape s)
 {
-    using G = Geo<S, SMALL>;
+    using G = Geo<S>;
     constexpr int NT = G::THREADS;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ __align__(16) Rec rec[3];
@@ -138,11 +144,13 @@ __global__ void __launch_bounds__(Geo<S, SMALL>::THREADS, 1024 / Geo<S, SMALL>::
     // destination is computed and the others are constants away
     const unsigned sdst = base + 16u * (unsigned)((tid / G::HW) * G::SLAB + (tid % G::HW / S + 1) * G::PITCH +
                                           (s.in == kSplitSlabs ? tid % S + (tid % S >= G::H2) : column<S>(tid % S + 1)));
-    auto stage = [&](int ug, const Rec &R) {
+    auto stage = [&](int ug, const Rec &R, bool fresh) {
         if (!R.all_in_tile) return;
         const int u0 = ug * G::UB, n = (s.U - u0) * G::HW - tid; // units from this thread's first to the end
+        const int which = fresh ? R.planes : (int)R.fresh;
 #pragma unroll 1
-        for (int slot = 0; slot < R.nst; ++slot) {
+        for (int slot = 0; slot < 2; ++slot) {
+            if (!(which >> slot & 1)) continue;
             const uint4 *src = x + ((size_t)R.ch[slot] * s.U + u0) * G::HW + tid;
             const unsigned d = sdst + slot * G::PLANE_BYTES;
             constexpr int D1 = unit_step<S, G>(1), D2 = unit_step<S, G>(2), D3 = unit_step<S, G>(3);
@@ -160,31 +168,52 @@ __global__ void __launch_bounds__(Geo<S, SMALL>::THREADS, 1024 / Geo<S, SMALL>::
     const int ub = tid / G::I, t = tid % G::I, py = t / G::H2, px = t % G::H2; // window (py, px) of slab ub
     const unsigned at0 = base + 16u * (unsigned)(ub * G::SLAB + 2 * py * G::PITCH + px);
 
-    // items are (slab group ug, output channel c), c fastest: the blocks that run together work on the same few slabs of all input
-    // channels (L2-resident); a block takes every gridDim.x-th item, keeping the (c, ug) of three items by carried additions
-    const int dug = gridDim.x / s.C, dc = gridDim.x - dug * s.C;
-    auto advance = [&](int &c, int &ug) {
-        c += dc, ug += dug;
-        if (c >= s.C) c -= s.C, ++ug;
+    // Items are (slab group ug, record), records fastest: the blocks that run together work on the same few slabs of all input
+    // channels (L2-resident).  A block takes every gridDim.x-th run of consecutive items, within which a record copies
+    // the planes only that the one before did not leave in the tile; the items of three are known ahead.
+    struct Item {
+        int i, end, run, ug, r; // item, end of its run, the run; its slab group and record
+        bool fresh;             // nothing in the tile
     };
-    int ug0 = blockIdx.x / s.C, c0 = blockIdx.x - ug0 * s.C, c1 = c0, ug1 = ug0;
-    advance(c1, ug1);
-    int c2 = c1, ug2 = ug1;
-    advance(c2, ug2);
-    if (ug0 < s.n_ug) fetch_rec(c0, rec[0]);
-    if (ug1 < s.n_ug) fetch_rec(c1, rec[1]);
+    auto begin = [&](Item &t) {
+        if (t.run < s.runs) {
+            t.i = t.run * s.per_run + min(t.run, s.longer), t.end = t.i + s.per_run + (t.run < s.longer);
+            t.ug = t.i / s.C, t.r = t.i - t.ug * s.C;
+        } else {
+            t.ug = s.n_ug;
+        }
+        t.fresh = true;
+    };
+    auto advance = [&](Item &t) {
+        if (++t.i < t.end) {
+            t.fresh = ++t.r == s.C;
+            if (t.fresh) t.r = 0, ++t.ug;
+        } else {
+            t.run += gridDim.x;
+            begin(t);
+        }
+    };
+    Item n0, n1, n2;
+    n0.run = blockIdx.x;
+    begin(n0);
+    n1 = n0;
+    advance(n1);
+    n2 = n1;
+    if (n2.ug < s.n_ug) advance(n2);
+    if (n0.ug < s.n_ug) fetch_rec(n0.r, rec[0]);
+    if (n1.ug < s.n_ug) fetch_rec(n1.r, rec[1]);
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads(); // records and halo zeros in place
-    if (ug0 < s.n_ug) stage(ug0, rec[0]);
+    if (n0.ug < s.n_ug) stage(n0.ug, rec[0], true);
     cp_async_commit();
-    for (int r0 = 0; ug0 < s.n_ug; r0 = r0 == 2 ? 0 : r0 + 1) {
+    for (int r0 = 0; n0.ug < s.n_ug; r0 = r0 == 2 ? 0 : r0 + 1) {
         const int r1 = r0 == 2 ? 0 : r0 + 1, r2 = r1 == 2 ? 0 : r1 + 1;
         cp_async_wait_all();
         __syncthreads(); // this item's planes and the next item's record have landed
-        if (ug2 < s.n_ug) fetch_rec(c2, rec[r2]);
+        if (n2.ug < s.n_ug) fetch_rec(n2.r, rec[r2]);
         const Rec &R = rec[r0];
-        const int u0 = ug0 * G::UB;
+        const int u0 = n0.ug * G::UB, c0 = R.c;
         const bool live = ub < s.U - u0;
         uint4 out = make_uint4(0u, 0u, 0u, 0u);
         if (live) {
@@ -212,29 +241,32 @@ __global__ void __launch_bounds__(Geo<S, SMALL>::THREADS, 1024 / Geo<S, SMALL>::
             }
         }
         __syncthreads(); // every thread is done with the tile: the next item's planes go there while the SM's other blocks compute
-        if (ug1 < s.n_ug) stage(ug1, rec[r1]);
+        if (n1.ug < s.n_ug) stage(n1.ug, rec[r1], n1.fresh);
         cp_async_commit();
         if (live) {
             if (s.out == kRows) y[((size_t)c0 * G::I + t) * s.U + u0 + ub] = out;
             else y[((size_t)c0 * s.U + u0 + ub) * G::I + (s.out == kSplitSlabs ? split_position(t, G::H2) : t)] = out;
         }
-        c0 = c1, ug0 = ug1, c1 = c2, ug1 = ug2;
-        advance(c2, ug2);
+        n0 = n1, n1 = n2;
+        if (n2.ug < s.n_ug) advance(n2);
     }
     cp_async_wait_all();
 }
 
-// The record of output channel c; offsets are bytes from a window's unit of the first plane.
-template <int S, bool SMALL> __device__ __forceinline__ void lay_out_record(const uint8_t *__restrict__ ops, const int32_t *__restrict__ sel, Rec *__restrict__ recs, int c, int Ci)
+// Record i: of output channel i, or as the order tells; offsets are bytes from a window's unit of the first plane.
+template <int S>
+__device__ __forceinline__ void lay_out_record(const uint8_t *__restrict__ ops, const int32_t *__restrict__ sel, const int32_t *__restrict__ order,
+                                               Rec *__restrict__ recs, int i, int Ci)
 {
-    using G = Geo<S, SMALL>;
+    using G = Geo<S>;
     Rec R;
-    int ch0 = 0, ch1 = -1;
+    int ch0 = -1, ch1 = -1, c = i;
+    if (order) c = order[3 * i], ch0 = order[3 * i + 1], ch1 = order[3 * i + 2] & 0xFFFF;
     bool all = true;
     for (int k = 0; k < 8; ++k) {
         const int w = sel[c * 8 + k];
         const int ch = min((w >> 16) & 0xFFFF, Ci - 1), r = (w >> 8) & 0xFF, sx = w & 0xFF;
-        if (k == 0) ch0 = ch;
+        if (ch0 < 0) ch0 = ch;
         if (ch1 < 0 && ch != ch0) ch1 = ch;
         all = all && (ch == ch0 || ch == ch1) && r < 3 && sx < 3;
         const int row = min(r, 2) * G::PITCH, col = min(sx, 2), second = ch == ch0 ? 0 : 1;
@@ -242,48 +274,43 @@ template <int S, bool SMALL> __device__ __forceinline__ void lay_out_record(cons
         if (k & 1) R.off[k / 2].z = l, R.off[k / 2].w = q;
         else R.off[k / 2].x = l, R.off[k / 2].y = q;
         R.word[k] = w;
-        const int op = k < 7 ? ops[c * 7 + k] & 15 : 0;
-        R.code[k] = op < 8 ? op : 15 - op, R.inv[k] = op < 8 ? 0u : ~0u;
+        if (k < 7) {
+            const int op = ops[c * 7 + k] & 15;
+            R.code[k] = op < 8 ? op : 15 - op, R.inv[k] = op < 8 ? 0u : ~0u;
+        }
     }
-    R.ch[0] = ch0, R.ch[1] = ch1 < 0 ? ch0 : ch1, R.nst = ch1 < 0 ? 1 : 2, R.all_in_tile = all;
-    recs[c] = R;
+    R.c = c, R.ch[0] = ch0, R.ch[1] = ch1 < 0 ? ch0 : ch1, R.planes = ch1 < 0 ? 1 : 3, R.all_in_tile = all;
+    R.fresh = order ? (unsigned)order[3 * i + 2] >> 16 : (unsigned)R.planes;
+    recs[i] = R;
 }
 
-// Those of the large blocks and behind them those of the small ones (but for 32x32 images), in one launch: a module's call lays them
-// out every time (two launches: 64 -> 256 channels of 16x16, 1000 samples 39 us, before 37).
-template <int S> __global__ void packed_slab3_records_kernel(const uint8_t *__restrict__ ops, const int32_t *__restrict__ sel, Rec *__restrict__ recs, int C, int Ci)
+template <int S> __global__ void packed_slab3_records_kernel(const uint8_t *__restrict__ ops, const int32_t *__restrict__ sel,
+                                                                    const int32_t *__restrict__ order, Rec *__restrict__ recs, int C, int Ci)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < C) {
-        lay_out_record<S, false>(ops, sel, recs, i, Ci);
-    } else if constexpr (S < 32) {
-        if (i < 2 * C) lay_out_record<S, true>(ops, sel, recs + C, i - C, Ci);
-    }
+    if (i < C) lay_out_record<S>(ops, sel, order, recs, i, Ci);
 }
 
-template <int S, bool SMALL> static int launch(const void *x, const void *recs, void *y, int Ci, int C, int64_t U, Order in, Order out, cudaStream_t st)
+template <int S> static int launch(const void *x, const void *recs, void *y, int Ci, int C, int64_t U, Order in, Order out, cudaStream_t st)
 {
-    using G = Geo<S, SMALL>;
+    using G = Geo<S>;
     using namespace clb_host;
-    Shape s{Ci, C, (int)U, (int)((U + G::UB - 1) / G::UB), in, out};
+    Shape s{Ci, C, (int)U, (int)((U + G::UB - 1) / G::UB), in, out, 0, 0, 0};
     constexpr int bytes = 2 * G::PLANE_BYTES;
-    auto k = packed_convtree_slab3_kernel<S, SMALL>;
+    auto k = packed_convtree_slab3_kernel<S>;
     if (ensure_dynamic_smem(k, bytes) != cudaSuccess) return check_launch(0);
     constexpr int by_smem = 227 * 1024 / (bytes + 2048), by_threads = 1024 / G::THREADS; // 64 registers a thread
     const long long items = (long long)C * s.n_ug, all = (long long)sm_count() * (by_smem < by_threads ? by_smem : by_threads);
+    // runs of about 16 items, as many for one block as for another (k = 1024, 8192 samples, four blocks: 1610 us with 4, 1590 with 16 and 32)
+    const long long grid = items < all ? items : all, rounds = (items + 8 * grid) / (16 * grid), runs = grid * (rounds > 0 ? rounds : 1);
+    s.runs = (int)runs, s.per_run = (int)(items / runs), s.longer = (int)(items % runs);
     CLB_TRACED("packed_convtree_slab3_kernel", st,
-               k<<<(unsigned)(items < all ? items : all), G::THREADS, bytes, st>>>((const uint4 *)x, (const Rec *)recs + (SMALL ? C : 0), (uint4 *)y, s));
+               k<<<(unsigned)grid, G::THREADS, bytes, st>>>((const uint4 *)x, (const Rec *)recs, (uint4 *)y, s));
     return check_launch();
 }
-// Small blocks where a large one would be at most half full (k = 1024, 100 samples: 8x8 images 52 -> 16 us, 4x4 61 -> 28).
-template <int S> static int launch_by_slabs(const void *x, const void *recs, void *y, int Ci, int C, int64_t U, Order in, Order out, cudaStream_t st)
+template <int S> static int records(const uint8_t *ops, const int32_t *sel, const int32_t *order, Rec *recs, int Ci, int C, cudaStream_t st)
 {
-    return 2 * U <= Geo<S, false>::UB ? launch<S, true>(x, recs, y, Ci, C, U, in, out, st) : launch<S, false>(x, recs, y, Ci, C, U, in, out, st);
-}
-template <int S> static int records(const uint8_t *ops, const int32_t *sel, Rec *recs, int Ci, int C, cudaStream_t st)
-{
-    const int n = S < 32 ? 2 * C : C;
-    packed_slab3_records_kernel<S><<<(n + 127) / 128, 128, 0, st>>>(ops, sel, recs, C, Ci);
+    packed_slab3_records_kernel<S><<<(C + 127) / 128, 128, 0, st>>>(ops, sel, order, recs, C, Ci);
     return clb_host::check_launch();
 }
 
@@ -297,21 +324,96 @@ bool clb_slab3_covers(int H, int W, int sh, int sw, int ph, int pw, int kh, int 
 {
     return H == W && (H == 32 || H == 16 || H == 8 || H == 4) && sh == 1 && sw == 1 && ph == 1 && pw == 1 && kh == 3 && kw == 3;
 }
-size_t clb_slab3_record_bytes(int C) { return 2 * (size_t)C * sizeof(slab::Rec); } // of the large and of the small blocks
+// Channels are vertices, output channels edges between the two that they read; the order follows trails: next comes an edge between
+// both channels in the tile, else one that shares the channel with more edges left, whose other plane is then replaced.
+bool clb_slab3_order(const int32_t *sel, int Ci, int C, int32_t *order)
+{
+    std::vector<int> a((size_t)C), b((size_t)C), start((size_t)Ci + 1, 0), edges;
+    for (int c = 0; c < C; ++c) {
+        int ch0 = -1, ch1 = -1;
+        for (int k = 0; k < 8; ++k) {
+            const int w = sel[c * 8 + k], ch = (w >> 16) & 0xFFFF;
+            if (w < 0 || ch >= Ci || ((w >> 8) & 0xFF) > 2 || (w & 0xFF) > 2) return false;
+            if (ch0 < 0) ch0 = ch;
+            else if (ch != ch0 && ch1 < 0) ch1 = ch;
+            else if (ch != ch0 && ch != ch1) return false;
+        }
+        a[c] = ch0, b[c] = ch1 < 0 ? ch0 : ch1;
+        ++start[a[c] + 1];
+        if (b[c] != a[c]) ++start[b[c] + 1];
+    }
+    for (int v = 0; v < Ci; ++v) start[v + 1] += start[v];
+    edges.resize((size_t)start[Ci]);
+    std::vector<int> end(start.begin(), start.end() - 1), left((size_t)Ci, 0);
+    for (int c = 0; c < C; ++c) {
+        edges[end[a[c]]++] = c, ++left[a[c]];
+        if (b[c] != a[c]) edges[end[b[c]]++] = c, ++left[b[c]];
+    }
+    std::vector<char> used((size_t)C, 0);
+    // an unused edge at v, one to `other` if there is one; used ones are dropped from the list's front
+    auto pick = [&](int v, int other, bool &both) {
+        int found = -1;
+        both = false;
+        for (int e = start[v], keep = e; e < end[v]; ++e) {
+            const int c = edges[e];
+            if (used[c]) {
+                if (e == keep) start[v] = ++keep;
+                continue;
+            }
+            if (found < 0) found = c;
+            if (a[c] + b[c] - v == other || a[c] == b[c]) {
+                both = true;
+                return c;
+            }
+            if (e - start[v] >= 64) break;
+        }
+        return found;
+    };
+    int slot[2] = {-1, -1}, next = 0;
+    for (int i = 0; i < C; ++i) {
+        int c = -1;
+        bool both = false;
+        if (slot[0] >= 0) {
+            const int k = left[slot[0]] >= left[slot[1]] ? 0 : 1;
+            c = pick(slot[k], slot[1 - k], both);
+            if (c < 0) c = pick(slot[1 - k], slot[k], both);
+        }
+        if (c < 0) {
+            while (used[next]) ++next;
+            c = next;
+        }
+        int fresh = 0;
+        if (slot[0] < 0 || (a[c] != slot[0] && a[c] != slot[1] && b[c] != slot[0] && b[c] != slot[1])) {
+            slot[0] = a[c], slot[1] = b[c], fresh = 3;
+        } else {
+            const bool has_a = a[c] == slot[0] || a[c] == slot[1], has_b = b[c] == slot[0] || b[c] == slot[1];
+            if (!has_a || !has_b) {
+                const int kept = has_a ? a[c] : b[c], k = kept == slot[0] ? 1 : 0; // the other plane goes
+                slot[k] = has_a ? b[c] : a[c], fresh = 1 << k;
+            }
+        }
+        used[c] = 1, --left[a[c]];
+        if (b[c] != a[c]) --left[b[c]];
+        order[3 * i] = c, order[3 * i + 1] = slot[0], order[3 * i + 2] = slot[1] | fresh << 16;
+    }
+    return true;
+}
 
-int clb_slab3_records(const uint8_t *ops, const int32_t *sel, void *recs, int Ci, int side, int C, cudaStream_t st)
+size_t clb_slab3_record_bytes(int C) { return (size_t)C * sizeof(slab::Rec); }
+
+int clb_slab3_records(const uint8_t *ops, const int32_t *sel, const int32_t *order, void *recs, int Ci, int side, int C, cudaStream_t st)
 {
     slab::Rec *r = (slab::Rec *)recs;
-    if (side == 32) return slab::records<32>(ops, sel, r, Ci, C, st);
-    if (side == 16) return slab::records<16>(ops, sel, r, Ci, C, st);
-    if (side == 8) return slab::records<8>(ops, sel, r, Ci, C, st);
-    return slab::records<4>(ops, sel, r, Ci, C, st);
+    if (side == 32) return slab::records<32>(ops, sel, order, r, Ci, C, st);
+    if (side == 16) return slab::records<16>(ops, sel, order, r, Ci, C, st);
+    if (side == 8) return slab::records<8>(ops, sel, order, r, Ci, C, st);
+    return slab::records<4>(ops, sel, order, r, Ci, C, st);
 }
 
 int clb_slab3_block(const void *x, const void *recs, void *y, int Ci, int side, int C, int64_t U, Order in, Order out, cudaStream_t st)
 {
-    if (side == 32) return slab::launch<32, false>(x, recs, y, Ci, C, U, in, out, st);
-    if (side == 16) return slab::launch_by_slabs<16>(x, recs, y, Ci, C, U, in, out, st);
-    if (side == 8) return slab::launch_by_slabs<8>(x, recs, y, Ci, C, U, in, out, st);
-    return slab::launch_by_slabs<4>(x, recs, y, Ci, C, U, in, out, st);
+    if (side == 32) return slab::launch<32>(x, recs, y, Ci, C, U, in, out, st);
+    if (side == 16) return slab::launch<16>(x, recs, y, Ci, C, U, in, out, st);
+    if (side == 8) return slab::launch<8>(x, recs, y, Ci, C, U, in, out, st);
+    return slab::launch<4>(x, recs, y, Ci, C, U, in, out, st);
 }
