@@ -19,10 +19,10 @@ struct FastDiv {
     __host__ __device__ __forceinline__ int div(int n) const { return d > 1 ? (int)(((unsigned long long)(unsigned)n * magic) >> 32) : n; }
 };
 
-// Where the units (16 bytes = 128 samples of one feature) of a layer's input live inside a slab's storage: channels of
+// Where the units (4, 8 or 16 bytes = 32, 64 or 128 samples of one feature) of a layer's input live inside a slab's storage: channels of
 // rows x pitch units, the feature's image inside a halo of `ph` rows and `pw` columns.  Flat features: one "channel".
 struct NetStorage {
-    int base;                // first unit (a multiple of 8: 128 bytes)
+    int base;                // first unit (a multiple of 8)
     int W, image;            // image width and size (rows * W), 1-D features: image = features
     int pitch, per_channel;  // units per stored row / channel
     int rows, ph, pw;        // image rows, halo

@@ -1,12 +1,16 @@
 // Compiled network, small calls: the whole stack in ONE launch.
 //
 // A small network on a small batch is bound by launches: run layer by layer, a mnist-sized stack at batch 1 to 256 was 12 to
-// 15 launches of 2 to 5 us (72-76 us per call, of which no kernel was busy for more than a few).  But a 128-sample slab of
+// 15 launches of 2 to 5 us (72-76 us per call, of which no kernel was busy for more than a few).  But a slab of samples of
 // packed activations goes through the network on its own -- no layer mixes samples -- so a slab can be given to one
 // thread-block cluster, which packs its input, runs layer after layer with a cluster barrier in between (about 0.5 us instead
-// of a launch) and counts the class sums.  Activations stay in global memory in units of 16 bytes (128 samples of one
-// feature): a few hundred KB, L2 and L1 resident.  Every storage is written once and read after a barrier, each slab has its
+// of a launch) and counts the class sums.  Activations stay in global memory in units of 4, 8 or 16 bytes (32, 64 or 128 samples of
+// one feature): a few hundred KB, L2 and L1 resident.  Every storage is written once and read after a barrier, each slab has its
 // own, and conv inputs are stored with their padding as a halo of zeros, so that a tap is one unconditional load.
+//
+// The size of a unit: what a thread waits for is the eight taps of a window on their way from the L2 and the barrier behind a layer, so that
+// small units pay twice, in bytes per tap and in slabs, hence SMs, per call (clb_net_cluster_launch; us with units of 4 / 8 / 16
+// bytes: mnist k = 16 batch 1 10.4 / 11.6 / 13.7, batch 256 13.5 / 12.9 / 15.2; cifar k = 32 batch 1000 40.0 / 39.1 / 42.2).
 //
 // Work split: a thread owns one unit of one feature.  Warps are dealt to the blocks of the cluster round robin (32
 // consecutive features per warp), so that a layer with few features still uses every SM of the cluster.  Gates are the
@@ -22,26 +26,57 @@ namespace {
 
 constexpr int kNetThreads = 512;
 
-__device__ __forceinline__ uint4 ld_unit(const uint4 *p)
+// 32 * N samples of one feature
+template <int N> struct __align__(4 * N) Unit {
+    unsigned w[N];
+    static __device__ __forceinline__ Unit zero()
+    {
+        Unit u;
+#pragma unroll
+        for (int i = 0; i < N; ++i) u.w[i] = 0u;
+        return u;
+    }
+    __device__ __forceinline__ void operator|=(const Unit &o)
+    {
+#pragma unroll
+        for (int i = 0; i < N; ++i) w[i] |= o.w[i];
+    }
+};
+
+// not the read-only path: the units were written earlier in this kernel by other blocks
+__device__ __forceinline__ Unit<4> ld_unit(const Unit<4> *p)
 {
-    // not the read-only path: the units were written earlier in this kernel by other blocks
-    uint4 v;
-    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    Unit<4> v;
+    asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ Unit<2> ld_unit(const Unit<2> *p)
+{
+    Unit<2> v;
+    asm volatile("ld.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.w[0]), "=r"(v.w[1]) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ Unit<1> ld_unit(const Unit<1> *p)
+{
+    Unit<1> v;
+    asm volatile("ld.global.u32 %0, [%1];" : "=r"(v.w[0]) : "l"(p) : "memory");
     return v;
 }
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
-// gate `op` (truth-table bits 3..0 = f(0,0), f(0,1), f(1,0), f(1,1)) on 128 samples
-__device__ __forceinline__ uint4 gate128(int op, const uint4 &a, const uint4 &b)
+// gate `op` (truth-table bits 3..0 = f(0,0), f(0,1), f(1,0), f(1,1)) on a unit
+template <int N> __device__ __forceinline__ Unit<N> gate(int op, const Unit<N> &a, const Unit<N> &b)
 {
     const unsigned m11 = (op & 1) ? ~0u : 0u, m10 = (op & 2) ? ~0u : 0u, m01 = (op & 4) ? ~0u : 0u, m00 = (op & 8) ? ~0u : 0u;
-    auto f = [&](unsigned x, unsigned y) {
-        const unsigned r1 = (y & m11) | (~y & m10), r0 = (y & m01) | (~y & m00);
-        return (x & r1) | (~x & r0);
-    };
-    return make_uint4(f(a.x, b.x), f(a.y, b.y), f(a.z, b.z), f(a.w, b.w));
+    Unit<N> r;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+        const unsigned x = a.w[i], y = b.w[i], r1 = (y & m11) | (~y & m10), r0 = (y & m01) | (~y & m00);
+        r.w[i] = (x & r1) | (~x & r0);
+    }
+    return r;
 }
 
 // lane s gets, in bit t, bit s of lane t's word
@@ -78,30 +113,32 @@ struct ConvWindow {
 #pragma unroll
         for (int k = 0; k < 8; ++k) tap[k] = first + ((word[k] >> 16) & 0xFFFF) * in.per_channel + ((word[k] >> 8) & 0xFF) * in.pitch + (word[k] & 0xFF);
     }
-    __device__ __forceinline__ uint4 position(const uint4 *x) const
+    template <int N> __device__ __forceinline__ Unit<N> position(const Unit<N> *x) const
     {
-        uint4 a[8];
+        Unit<N> a[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) a[k] = ld_unit(x + tap[k]);
-        const uint4 g0 = gate128(op[0], a[0], a[1]), g1 = gate128(op[1], a[2], a[3]);
-        const uint4 g2 = gate128(op[2], a[4], a[5]), g3 = gate128(op[3], a[6], a[7]);
-        return gate128(op[6], gate128(op[4], g0, g1), gate128(op[5], g2, g3));
+        const Unit<N> g0 = gate(op[0], a[0], a[1]), g1 = gate(op[1], a[2], a[3]);
+        const Unit<N> g2 = gate(op[2], a[4], a[5]), g3 = gate(op[3], a[6], a[7]);
+        return gate(op[6], gate(op[4], g0, g1), gate(op[5], g2, g3));
     }
 };
 
 } // namespace
 
+template <int N>
 __global__ void __launch_bounds__(kNetThreads, 1) net_cluster_kernel(const __grid_constant__ NetPlan net, const void *__restrict__ input,
                                                                      const float *__restrict__ thresholds, const unsigned char *__restrict__ params,
-                                                                     uint4 *work, int *counts, long long batch)
+                                                                     Unit<N> *work, int *counts, long long batch)
 {
+    using U = Unit<N>;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned rank, csize;
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(csize));
     const int slab = blockIdx.x / csize;
     const int gwarp = warp * (int)csize + (int)rank, nwarps = (kNetThreads / 32) * (int)csize;
-    uint4 *const base = work + (size_t)slab * net.slab_units;
+    U *const base = work + (size_t)slab * net.slab_units;
     __shared__ int cutoff[kNetMaxLevels]; // byte pixels: the first value above the threshold, by the comparison u / 255 > t itself
     if (net.input_kind == 2) {
         for (int i = threadIdx.x; i < net.levels; i += kNetThreads) {
@@ -118,8 +155,8 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_cluster_kernel(const __gri
         }
         __syncthreads();
     }
-    const long long s0 = (long long)slab * 128;
-    const int live = (int)min(128LL, batch - s0); // samples of this slab
+    const long long s0 = (long long)slab * (32 * N);
+    const int live = (int)min(32LL * N, batch - s0); // samples of this slab
 
     // ---- input: one 32-sample word of every feature per (feature group, word) task; class sums cleared
     for (int i = gwarp * 32 + lane; i < live * net.classes; i += nwarps * 32) counts[s0 * net.classes + i] = 0;
@@ -127,15 +164,15 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_cluster_kernel(const __gri
         const NetStorage st = net.store[0];
         unsigned *words = reinterpret_cast<unsigned *>(base + st.base);
         for (int i = gwarp * 32 + lane; i < st.halo_units; i += nwarps * 32) // zeros of the halo (the interior follows)
-            if (st.halo(i)) base[st.base + i] = make_uint4(0u, 0u, 0u, 0u);
+            if (st.halo(i)) base[st.base + i] = U::zero();
         if (net.input_kind == 0) { // bytes [batch][features]
             const unsigned char *x = static_cast<const unsigned char *>(input);
             const long long F = net.in_features;
             const bool quad = (F & 3) == 0 && (reinterpret_cast<uintptr_t>(x) & 3) == 0; // four features per lane and load
             const int per = quad ? 128 : 32, groups = (int)((F + per - 1) / per);
-            for (int task = gwarp; task < groups * 4; task += nwarps) {
-                const int w = task & 3;
-                const long long f = (long long)(task >> 2) * per + (quad ? 4 * lane : lane);
+            for (int task = gwarp; task < groups * N; task += nwarps) {
+                const int w = task % N;
+                const long long f = (long long)(task / N) * per + (quad ? 4 * lane : lane);
                 const int n0 = w * 32, n = min(32, live - n0);
                 if (f >= F) continue;
                 const unsigned char *src = x + (s0 + n0) * F + f;
@@ -152,20 +189,20 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_cluster_kernel(const __gri
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         const unsigned lo = __byte_perm(g[0], g[1], 0x40 + 0x11 * k), hi = __byte_perm(g[2], g[3], 0x40 + 0x11 * k);
-                        words[4 * st.unit((int)f + k) + w] = (lo & 0xffffu) | (hi << 16);
+                        words[N * st.unit((int)f + k) + w] = (lo & 0xffffu) | (hi << 16);
                     }
                 } else {
                     unsigned v = 0u;
                     for (int j = 0; j < n; ++j) v |= (__ldg(src + j * F) != 0 ? 1u : 0u) << j;
-                    words[4 * st.unit((int)f) + w] = v;
+                    words[N * st.unit((int)f) + w] = v;
                 }
             }
         } else { // pixels [batch][P], features threshold-major: feature i * P + p is pixel p > threshold i
             const int P = (int)(net.in_features / net.levels);
             const int level_step = st.halo_units ? P / st.image * st.per_channel : P; // units from a feature to its next threshold's
             const int groups = (P + 31) / 32;
-            for (int task = gwarp; task < groups * 4; task += nwarps) {
-                const int w = task & 3, p = (task >> 2) * 32 + lane;
+            for (int task = gwarp; task < groups * N; task += nwarps) {
+                const int w = task % N, p = task / N * 32 + lane;
                 const int n0 = w * 32, n = min(32, live - n0);
                 if (p >= P) continue;
                 const unsigned mask = n >= 32 ? ~0u : n > 0 ? (1u << n) - 1u : 0u; // a negative threshold must not set pad bits
@@ -174,8 +211,8 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_cluster_kernel(const __gri
                     float v[32];
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = j < n ? __ldg(src + (long long)j * P) : 0.f;
-                    unsigned *dst = words + 4 * st.unit(p) + w;
-                    for (int i = 0; i < net.levels; ++i, dst += 4 * level_step) {
+                    unsigned *dst = words + N * st.unit(p) + w;
+                    for (int i = 0; i < net.levels; ++i, dst += N * level_step) {
                         const float t = __ldg(thresholds + i);
                         unsigned m = 0u;
 #pragma unroll
@@ -188,8 +225,8 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_cluster_kernel(const __gri
                     int v[32];
 #pragma unroll
                     for (int j = 0; j < 32; ++j) v[j] = j < n ? (int)__ldg(src + (long long)j * P) : 0;
-                    unsigned *dst = words + 4 * st.unit(p) + w;
-                    for (int i = 0; i < net.levels; ++i, dst += 4 * level_step) {
+                    unsigned *dst = words + N * st.unit(p) + w;
+                    for (int i = 0; i < net.levels; ++i, dst += N * level_step) {
                         const int t = cutoff[i];
                         unsigned m = 0u;
 #pragma unroll
@@ -218,15 +255,15 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_cluster_kernel(const __gri
         // between arrive and wait: what does not depend on the other blocks' results
         if (conv) {
             for (int i = gwarp * 32 + lane; i < out.halo_units; i += nwarps * 32) // the next layer's padding
-                if (out.halo(i)) base[out.base + i] = make_uint4(0u, 0u, 0u, 0u);
+                if (out.halo(i)) base[out.base + i] = U::zero();
             if (item < items) cw.load(L, params, in, split ? item >> 2 : item);
         }
         cluster_wait();
         if (conv) {
-            const uint4 *x = base + in.base;
-            uint4 *y = base + out.base;
+            const U *x = base + in.base;
+            U *y = base + out.base;
             while (item < items) {
-                uint4 acc;
+                U acc;
                 if (split) {
                     const int d = item & 3;
                     acc = cw.position(x + (d >> 1) * L.stride * in.pitch + (d & 1) * L.stride);
@@ -234,16 +271,13 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_cluster_kernel(const __gri
                     const unsigned quad = 0xfu << (lane & 28);
 #pragma unroll
                     for (int o = 1; o <= 2; o <<= 1) {
-                        acc.x |= __shfl_xor_sync(quad, acc.x, o), acc.y |= __shfl_xor_sync(quad, acc.y, o);
-                        acc.z |= __shfl_xor_sync(quad, acc.z, o), acc.w |= __shfl_xor_sync(quad, acc.w, o);
+#pragma unroll
+                        for (int i = 0; i < N; ++i) acc.w[i] |= __shfl_xor_sync(quad, acc.w[i], o);
                     }
                 } else {
-                    acc = make_uint4(0u, 0u, 0u, 0u);
+                    acc = U::zero();
 #pragma unroll
-                    for (int d = 0; d < 4; ++d) {
-                        const uint4 z = cw.position(x + (d >> 1) * L.stride * in.pitch + (d & 1) * L.stride);
-                        acc.x |= z.x, acc.y |= z.y, acc.z |= z.z, acc.w |= z.w;
-                    }
+                    for (int d = 0; d < 4; ++d) acc |= cw.position(x + (d >> 1) * L.stride * in.pitch + (d & 1) * L.stride);
                 }
                 if (!split || (item & 3) == 0) y[cw.c * out.per_channel + (cw.py + out.ph) * out.pitch + cw.px + out.pw] = acc;
                 item += nwarps * 32;
@@ -255,51 +289,53 @@ __global__ void __launch_bounds__(kNetThreads, 1) net_cluster_kernel(const __gri
         const bool last = li + 1 == net.n_layers;
         const int S = last ? L.out_dim / net.classes : L.out_dim;  // features per class
         const int chunks = (S + 31) / 32, total = chunks * (last ? net.classes : 1);
-        const uint4 *x = base + in.base;
+        const U *x = base + in.base;
         // (flat) a warp takes consecutive chunks of 32 features, so that its class changes rarely
         const int lo = (int)((long long)total * gwarp / nwarps), hi = (int)((long long)total * (gwarp + 1) / nwarps);
-        int cls = -1, sum[4] = {0, 0, 0, 0};
+        int cls = -1, sum[N];
+#pragma unroll
+        for (int w = 0; w < N; ++w) sum[w] = 0;
         auto flush = [&]() {
             if (cls < 0) return;
 #pragma unroll
-            for (int w = 0; w < 4; ++w)
+            for (int w = 0; w < N; ++w)
                 if (w * 32 + lane < live && sum[w]) atomicAdd(counts + (s0 + w * 32 + lane) * net.classes + cls, sum[w]);
 #pragma unroll
-            for (int w = 0; w < 4; ++w) sum[w] = 0;
+            for (int w = 0; w < N; ++w) sum[w] = 0;
         };
         for (int ch = lo; ch < hi; ++ch) {
             const int c = ch / chunks, i = (ch - c * chunks) * 32 + lane; // feature i of class c
             const int t = c * S + i;
-            uint4 r = make_uint4(0u, 0u, 0u, 0u);
+            U r = U::zero();
             if (i < S) {
                 if (L.kind == 2) {
                     const long long a = __ldg(reinterpret_cast<const long long *>(params + L.off_a) + t), b = __ldg(reinterpret_cast<const long long *>(params + L.off_b) + t);
-                    r = gate128(__ldg(params + L.off_ops + t), ld_unit(x + a), ld_unit(x + b));
+                    r = gate(__ldg(params + L.off_ops + t), ld_unit(x + a), ld_unit(x + b));
                 } else if (L.levels == 3) {
                     const int4 *leaf = reinterpret_cast<const int4 *>(params + L.off_a) + 2 * t;
                     const int4 la = __ldg(leaf), lb = __ldg(leaf + 1);
                     int op[7];
 #pragma unroll
                     for (int g = 0; g < 7; ++g) op[g] = __ldg(params + L.off_ops + (long long)t * 7 + g);
-                    const uint4 v0 = ld_unit(x + la.x), v1 = ld_unit(x + la.y), v2 = ld_unit(x + la.z), v3 = ld_unit(x + la.w);
-                    const uint4 v4 = ld_unit(x + lb.x), v5 = ld_unit(x + lb.y), v6 = ld_unit(x + lb.z), v7 = ld_unit(x + lb.w);
-                    r = gate128(op[6], gate128(op[4], gate128(op[0], v0, v1), gate128(op[1], v2, v3)),
-                                gate128(op[5], gate128(op[2], v4, v5), gate128(op[3], v6, v7)));
+                    const U v0 = ld_unit(x + la.x), v1 = ld_unit(x + la.y), v2 = ld_unit(x + la.z), v3 = ld_unit(x + la.w);
+                    const U v4 = ld_unit(x + lb.x), v5 = ld_unit(x + lb.y), v6 = ld_unit(x + lb.z), v7 = ld_unit(x + lb.w);
+                    r = gate(op[6], gate(op[4], gate(op[0], v0, v1), gate(op[1], v2, v3)),
+                                gate(op[5], gate(op[2], v4, v5), gate(op[3], v6, v7)));
                 } else {
                     const int4 la = __ldg(reinterpret_cast<const int4 *>(params + L.off_a) + t);
                     int op[3];
 #pragma unroll
                     for (int g = 0; g < 3; ++g) op[g] = __ldg(params + L.off_ops + (long long)t * 3 + g);
-                    const uint4 v0 = ld_unit(x + la.x), v1 = ld_unit(x + la.y), v2 = ld_unit(x + la.z), v3 = ld_unit(x + la.w);
-                    r = gate128(op[2], gate128(op[0], v0, v1), gate128(op[1], v2, v3));
+                    const U v0 = ld_unit(x + la.x), v1 = ld_unit(x + la.y), v2 = ld_unit(x + la.z), v3 = ld_unit(x + la.w);
+                    r = gate(op[2], gate(op[0], v0, v1), gate(op[1], v2, v3));
                 }
                 if (!last) base[out.base + t] = r;
             }
             if (last) {
                 if (c != cls) flush();
                 cls = c;
-                sum[0] += __popc(transpose32(r.x, lane)), sum[1] += __popc(transpose32(r.y, lane));
-                sum[2] += __popc(transpose32(r.z, lane)), sum[3] += __popc(transpose32(r.w, lane));
+#pragma unroll
+                for (int w = 0; w < N; ++w) sum[w] += __popc(transpose32(r.w[w], lane));
             }
         }
         if (last) flush();
@@ -318,15 +354,16 @@ using namespace clb_host;
 static constexpr int kSizes[] = {16, 9, 6, 5, 4, 3, 2, 1};
 static constexpr int kNSizes = sizeof(kSizes) / sizeof(kSizes[0]);
 
-static bool cluster_size(int slabs, int &out)
+// The largest cluster of N-word units with which so many slabs are resident at once; 0: with none.
+template <int N> static int cluster_size(int slabs)
 {
     static std::atomic<int> resident[64][kNSizes]; // clusters resident at once + 1
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
     for (int i = 0; i < kNSizes; ++i) {
         int have = resident[dev][i].load(std::memory_order_relaxed);
         if (!have) {
-            if (i == 0 && cudaFuncSetAttribute(net_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return false;
+            if (i == 0 && cudaFuncSetAttribute(net_cluster_kernel<N>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return 0;
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim = dim3((unsigned)kSizes[i]), cfg.blockDim = dim3(kNetThreads);
             cudaLaunchAttribute attr[1];
@@ -334,22 +371,19 @@ static bool cluster_size(int slabs, int &out)
             attr[0].val.clusterDim.x = (unsigned)kSizes[i], attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
             cfg.attrs = attr, cfg.numAttrs = 1;
             int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, net_cluster_kernel, &cfg) != cudaSuccess) cudaGetLastError(), n = 0;
+            if (cudaOccupancyMaxActiveClusters(&n, net_cluster_kernel<N>, &cfg) != cudaSuccess) cudaGetLastError(), n = 0;
             have = n + 1;
             resident[dev][i].store(have, std::memory_order_relaxed);
         }
-        out = kSizes[i];
-        if (slabs <= have - 1) break; // the last shape takes whatever is left, in several waves
+        if (slabs <= have - 1) return kSizes[i];
     }
-    return true;
+    return 0;
 }
 
-int clb_net_cluster_launch(const NetPlan &net, const void *input, const float *thresholds, const unsigned char *params, void *work, int32_t *counts,
-                           int64_t batch, cudaStream_t st)
+template <int N>
+static int launch(const NetPlan &net, int slabs, int csize, const void *input, const float *thresholds, const unsigned char *params, void *work, int32_t *counts,
+                  int64_t batch, cudaStream_t st)
 {
-    const int slabs = (int)((batch + 127) / 128);
-    int csize;
-    if (!cluster_size(slabs, csize)) return check_launch(0);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(slabs * csize)), cfg.blockDim = dim3(kNetThreads), cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -357,6 +391,18 @@ int clb_net_cluster_launch(const NetPlan &net, const void *input, const float *t
     attr[0].val.clusterDim.x = (unsigned)csize, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr, cfg.numAttrs = 1;
     CLB_TRACED("net_cluster_kernel", st,
-               cudaLaunchKernelEx(&cfg, net_cluster_kernel, net, input, thresholds, params, static_cast<uint4 *>(work), counts, (long long)batch));
+               cudaLaunchKernelEx(&cfg, net_cluster_kernel<N>, net, input, thresholds, params, static_cast<Unit<N> *>(work), counts, (long long)batch));
     return check_launch();
+}
+
+int clb_net_cluster_launch(const NetPlan &net, const void *input, const float *thresholds, const unsigned char *params, void *work, int32_t *counts,
+                           int64_t batch, cudaStream_t st)
+{
+    const int s1 = (int)((batch + 31) / 32), s2 = (int)((batch + 63) / 64), s4 = (int)((batch + 127) / 128);
+    // a thread's time goes as 1.5 + the words of a unit, and with the features that the blocks of a cluster share
+    const int c1 = cluster_size<1>(s1), c2 = cluster_size<2>(s2), c4 = cluster_size<4>(s4);
+    const double t1 = c1 ? 2.5 / c1 : 1e9, t2 = c2 ? 3.5 / c2 : 1e9, t4 = 5.5 / (c4 ? c4 : 1);
+    if (t1 < t2 && t1 < t4) return launch<1>(net, s1, c1, input, thresholds, params, work, counts, batch, st);
+    if (t2 < t4) return launch<2>(net, s2, c2, input, thresholds, params, work, counts, batch, st);
+    return launch<4>(net, s4, c4 ? c4 : 1, input, thresholds, params, work, counts, batch, st); // (the last shape: in several waves)
 }
