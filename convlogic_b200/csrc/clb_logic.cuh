@@ -77,6 +77,26 @@ template <typename T, int V> __device__ __forceinline__ void vstore(T *p, const 
     *reinterpret_cast<VT *>(p) = v;
 }
 
+// the same for what does not fit the L2 until it is read again
+template <typename T, int V> __device__ __forceinline__ void vstore_once(T *p, const T (&r)[V])
+{
+    using VT = typename Vec<T, V>::type;
+    VT v;
+    T *e = reinterpret_cast<T *>(&v);
+#pragma unroll
+    for (int k = 0; k < V; ++k) e[k] = r[k];
+    __stcs(reinterpret_cast<VT *>(p), v);
+}
+
+template <typename T, int V> __device__ __forceinline__ void vload_once(const T *p, T (&r)[V])
+{
+    using VT = typename Vec<T, V>::type;
+    const VT v = __ldcs(reinterpret_cast<const VT *>(p));
+    const T *e = reinterpret_cast<const T *>(&v);
+#pragma unroll
+    for (int k = 0; k < V; ++k) r[k] = e[k];
+}
+
 // a gate's 16 values as four vectors
 __device__ __forceinline__ void load16(const float *__restrict__ w, float (&v)[16])
 {

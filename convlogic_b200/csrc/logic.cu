@@ -340,15 +340,15 @@ __global__ void __launch_bounds__(256) group_sum_ce_sample_kernel(float *__restr
     float sc = -3.0e38f;
     if (lane < k) {
         float t = 0.f;
-        int p = 0;
-        for (; p + 8 <= parts; p += 8) {
-            float v[8];
+        for (int p = 0; p < parts; p += 32) { // (a chain of loads eight at a time took 7.1 us for 59 parts of 256 samples)
+            float v[32];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = partial[((long long)(p + j) * k + lane) * B + b];
+            for (int j = 0; j < 32; ++j)
+                if (p + j < parts) v[j] = partial[((long long)(p + j) * k + lane) * B + b];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) t += v[j];
+            for (int j = 0; j < 32; ++j)
+                if (p + j < parts) t += v[j];
         }
-        for (; p < parts; ++p) t += partial[((long long)p * k + lane) * B + b];
         sc = t / tau;
     }
     float mx = sc;
@@ -508,11 +508,10 @@ __device__ __forceinline__ float quad_sum(float v)
     return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-// the lane's four entries of the mixture over the 16 gates (zeros on an idle lane); every lane of the warp calls this
-__device__ __forceinline__ void quad_mixture(const float *__restrict__ w16, int wmode, int q, bool active, float (&p)[4])
+// the lane's four entries of the mixture over the 16 gates from those of the values p (zeros on an idle lane); every lane of the warp
+// calls this
+__device__ __forceinline__ void quad_mixture(int wmode, int q, float (&p)[4])
 {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) p[i] = active ? __ldg(w16 + 4 * q + i) : 0.f;
     if (wmode == CLB_W_SOFTMAX) {
         float m = fmaxf(fmaxf(p[0], p[1]), fmaxf(p[2], p[3]));
         m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
@@ -559,23 +558,51 @@ __device__ __forceinline__ const float *tree_row(const TreeTables &tt, int lane,
     return tt.w[g < 4 ? 0 : (g < 6 ? 1 : 2)] + n * 16;
 }
 
-// every lane gets all seven gates; n: the lane's neuron (lanes >= 28: any value), p: the lane's four mixture entries
-__device__ __forceinline__ void tree_gates_of(const TreeTables &tt, long long n, int lane, int wmode, Gate<float> (&g)[7], float (&p)[4])
+// the lane's four of the values of its neuron n
+__device__ __forceinline__ void tree_values(const TreeTables &tt, long long n, int lane, float (&p)[4])
 {
     const bool active = lane < 28;
-    quad_mixture(tree_row(tt, active ? lane : 0, n), wmode, lane & 3, active, p);
-    const Gate<float> mine = quad_gate(p, lane & 3);
+    const float *w16 = tree_row(tt, active ? lane : 0, n);
 #pragma unroll
-    for (int i = 0; i < 7; ++i) {
-        g[i].k1 = __shfl_sync(0xffffffffu, mine.k1, 4 * i), g[i].ka = __shfl_sync(0xffffffffu, mine.ka, 4 * i);
-        g[i].kb = __shfl_sync(0xffffffffu, mine.kb, 4 * i), g[i].kab = __shfl_sync(0xffffffffu, mine.kab, 4 * i);
+    for (int i = 0; i < 4; ++i) p[i] = active ? __ldg(w16 + 4 * (lane & 3) + i) : 0.f;
+}
+
+// The seven gates of the warp's tree into sg (as k1, ka, kb, kab); p: the lane's four values, then its four mixture entries.
+__device__ __forceinline__ void tree_gates_to(float4 *sg, int lane, int wmode, float (&p)[4])
+{
+    quad_mixture(wmode, lane & 3, p);
+    const Gate<float> mine = quad_gate(p, lane & 3);
+    __syncwarp(); // the tree before is done with them
+    if (lane < 28 && (lane & 3) == 0) sg[lane >> 2] = make_float4(mine.k1, mine.ka, mine.kb, mine.kab);
+    __syncwarp();
+}
+__device__ __forceinline__ Gate<float> tree_gate(const float4 *sg, int i)
+{
+    const float4 v = sg[i];
+    return Gate<float>{v.x, v.y, v.z, v.w};
+}
+// the trees' output for the lane's V samples
+template <int V> __device__ __forceinline__ void tree_eval(const float4 *sg, const float (&a)[8][V], float (&r)[V])
+{
+    float t[2][V];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const Gate<float> g0 = tree_gate(sg, 2 * h), g1 = tree_gate(sg, 2 * h + 1), g2 = tree_gate(sg, 4 + h);
+#pragma unroll
+        for (int e = 0; e < V; ++e)
+            t[h][e] = gate_eval<float>(g2, gate_eval<float>(g0, a[4 * h][e], a[4 * h + 1][e]), gate_eval<float>(g1, a[4 * h + 2][e], a[4 * h + 3][e]));
     }
+    const Gate<float> g = tree_gate(sg, 6);
+#pragma unroll
+    for (int e = 0; e < V; ++e) r[e] = gate_eval<float>(g, t[0][e], t[1][e]);
 }
 
 template <int V>
 __global__ void __launch_bounds__(256, 3) logic_tree_fwd_kernel(const float *__restrict__ x, TreeTables tt, float *__restrict__ y, long long T,
                                                              long long B, int wmode)
 {
+    __shared__ float4 gates[8][7];
+    float4 *sg = gates[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
     // The tables of a tree (leaf rows on lanes 0..7, the gates' neurons on lanes 0..27) are fetched one tree ahead, so that
@@ -586,9 +613,9 @@ __global__ void __launch_bounds__(256, 3) logic_tree_fwd_kernel(const float *__r
         const long long tn = t + nwarps;
         const int nx_leaf = (tn < T && lane < 8) ? __ldg(tt.leaf + tn * 8 + lane) : 0;
         const int nx_node = (tn < T && lane < 28) ? __ldg(tt.node + tn * 7 + (lane >> 2)) : 0;
-        Gate<float> g[7];
         float pq[4];
-        tree_gates_of(tt, my_node, lane, wmode, g, pq);
+        tree_values(tt, my_node, lane, pq);
+        tree_gates_to(sg, lane, wmode, pq);
         const float *row[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) row[k] = x + (long long)__shfl_sync(0xffffffffu, my_leaf, k) * B;
@@ -597,12 +624,7 @@ __global__ void __launch_bounds__(256, 3) logic_tree_fwd_kernel(const float *__r
             float a[8][V], r[V];
 #pragma unroll
             for (int k = 0; k < 8; ++k) vload<float, V>(row[k] + b0, a[k]);
-#pragma unroll
-            for (int e = 0; e < V; ++e) {
-                const float g0 = gate_eval<float>(g[0], a[0][e], a[1][e]), g1 = gate_eval<float>(g[1], a[2][e], a[3][e]);
-                const float g2 = gate_eval<float>(g[2], a[4][e], a[5][e]), g3 = gate_eval<float>(g[3], a[6][e], a[7][e]);
-                r[e] = gate_eval<float>(g[6], gate_eval<float>(g[4], g0, g1), gate_eval<float>(g[5], g2, g3));
-            }
+            tree_eval<V>(sg, a, r);
             vstore<float, V>(y + t * B + b0, r);
         }
     }
@@ -612,54 +634,66 @@ __global__ void __launch_bounds__(256, 3) logic_tree_fwd_kernel(const float *__r
 // class sums reads it in a training step).  Block (part, class): its 8 warps share the trees of one part of one class
 // (tree i of the part goes to warp i % 8), a lane adds up the outputs of its samples over the warp's trees in tree order, the
 // 8 warps' sums are added in warp order: partial[(part * k + class) * B + b], the layout group_sum_ce_sample_kernel reads.
+// Gates and running sums in shared memory, four rows at a time and a gate's values a tree ahead: 64 registers, so that four blocks of an SM
+// take nearly all parts in one wave (k = 256, 256 samples 108 -> 104 us, k = 32, 100 samples 13.5 -> 11.7; it is a hundredth of
+// the blocks that are left for a second one, and fewer parts would add in another order).
 template <int TR>
-__global__ void __launch_bounds__(256, TR <= 2 ? 3 : 2) logic_tree_fwd_sum_kernel(const float *__restrict__ x, TreeTables tt, float *__restrict__ partial,
-                                                                 long long T, long long B, int k, int wmode)
+__global__ void __launch_bounds__(256, 4) logic_tree_fwd_sum_kernel(const float *__restrict__ x, TreeTables tt, float *__restrict__ partial,
+                                                                 long long T, long long batch, int k, int wmode)
 {
-    __shared__ float red[8][TR * 128];
+    __shared__ __align__(16) float red[8][TR * 128]; // a lane's running sums: in registers they would cost a resident block
+    __shared__ float4 gates[8][7];
     const int lane = threadIdx.x & 31, wv = threadIdx.x >> 5;
     const int cls = blockIdx.y, part = blockIdx.x, parts = gridDim.x;
     const long long S = T / k;
-    const long long t_lo = cls * S + S * part / parts, t_hi = cls * S + S * (part + 1) / parts;
-    float acc[TR][4];
+    const int t_lo = (int)(cls * S + S * part / parts), t_hi = (int)(cls * S + S * (part + 1) / parts), B = (int)batch;
+    float4 *sg = gates[wv];
+    float4 *const acc = reinterpret_cast<float4 *>(red[wv]) + lane;
 #pragma unroll
-    for (int tr = 0; tr < TR; ++tr)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[tr][e] = 0.f;
-    const long long t0 = t_lo + wv;
+    for (int tr = 0; tr < TR; ++tr) acc[tr * 32] = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int t0 = t_lo + wv;
     int my_leaf = (t0 < t_hi && lane < 8) ? __ldg(tt.leaf + t0 * 8 + lane) : 0;   // index tables one tree ahead
     int my_node = (t0 < t_hi && lane < 28) ? __ldg(tt.node + t0 * 7 + (lane >> 2)) : 0;
-    for (long long t = t0; t < t_hi; t += 8) {
-        const long long tn = t + 8;
+    int nx_node = (t0 + 8 < t_hi && lane < 28) ? __ldg(tt.node + (t0 + 8) * 7 + (lane >> 2)) : 0;
+    float raw[4]; // its values one tree ahead
+    tree_values(tt, my_node, lane, raw);
+    for (int t = t0; t < t_hi; t += 8) {
+        const int tn = t + 8, tnn = t + 16;
         const int nx_leaf = (tn < t_hi && lane < 8) ? __ldg(tt.leaf + tn * 8 + lane) : 0;
-        const int nx_node = (tn < t_hi && lane < 28) ? __ldg(tt.node + tn * 7 + (lane >> 2)) : 0;
-        Gate<float> g[7];
+        const int nn_node = (tnn < t_hi && lane < 28) ? __ldg(tt.node + tnn * 7 + (lane >> 2)) : 0;
         float pq[4];
-        tree_gates_of(tt, my_node, lane, wmode, g, pq);
-        const float *row[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) row[q] = x + (long long)__shfl_sync(0xffffffffu, my_leaf, q) * B;
-        my_leaf = nx_leaf, my_node = nx_node;
-#pragma unroll
+        for (int i = 0; i < 4; ++i) pq[i] = raw[i];
+        if (tn < t_hi) tree_values(tt, nx_node, lane, raw);
+        tree_gates_to(sg, lane, wmode, pq);
+#pragma unroll 1
         for (int tr = 0; tr < TR; ++tr) {
-            const long long b0 = ((long long)tr * 32 + lane) * 4;
-            if (b0 < B) {
-                float a[8][4];
+            const int b0 = (tr * 32 + lane) * 4;
+            float t[2][4];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) vload<float, 4>(row[q] + b0, a[q]);
+            for (int h = 0; h < 2; ++h) { // four rows at a time
+                float a[4][4];
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                    const float g0 = gate_eval<float>(g[0], a[0][e], a[1][e]), g1 = gate_eval<float>(g[1], a[2][e], a[3][e]);
-                    const float g2 = gate_eval<float>(g[2], a[4][e], a[5][e]), g3 = gate_eval<float>(g[3], a[6][e], a[7][e]);
-                    acc[tr][e] += gate_eval<float>(g[6], gate_eval<float>(g[4], g0, g1), gate_eval<float>(g[5], g2, g3));
+                for (int q = 0; q < 4; ++q) {
+                    const float *row = x + ((long long)__shfl_sync(0xffffffffu, my_leaf, 4 * h + q) * B + b0);
+                    if (b0 < B) vload<float, 4>(row, a[q]);
                 }
+                const Gate<float> g0 = tree_gate(sg, 2 * h), g1 = tree_gate(sg, 2 * h + 1), g2 = tree_gate(sg, 4 + h);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) t[h][e] = gate_eval<float>(g2, gate_eval<float>(g0, a[0][e], a[1][e]), gate_eval<float>(g1, a[2][e], a[3][e]));
+            }
+            if (b0 < B) {
+                float r[4];
+                const Gate<float> g = tree_gate(sg, 6);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) r[e] = gate_eval<float>(g, t[0][e], t[1][e]);
+                float4 sum = acc[tr * 32];
+                sum.x += r[0], sum.y += r[1], sum.z += r[2], sum.w += r[3];
+                acc[tr * 32] = sum;
             }
         }
+        my_leaf = nx_leaf, my_node = nx_node, nx_node = nn_node;
     }
-#pragma unroll
-    for (int tr = 0; tr < TR; ++tr)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) red[wv][(tr * 32 + lane) * 4 + e] = acc[tr][e];
     __syncthreads();
     for (int i = threadIdx.x; i < TR * 128; i += 256) {
         if (i < B) {
@@ -681,41 +715,108 @@ struct TreeHead {
     float tau;
 };
 
-template <int V, bool HEAD>
+// The head's upstream gradients as rows, a class each: up [k][B].  Read straight from dscore, a lane's four values lie four lines
+// apart (32 look-ups in the L1 per load instead of four) and are divided again for every tree.
+__global__ void __launch_bounds__(256) tree_head_rows_kernel(float *__restrict__ up, long long B, TreeHead head)
+{
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= B * head.k) return;
+    const long long c = i / B, b = i - c * B;
+    up[i] = __ldg(head.dscore + b * head.k + c) / (head.tau / __ldg(head.scale));
+}
+
+constexpr int kTreeStages = 2, // (k = 256, 256 samples: 202 us with two, 208 with three, 215 with four)
+              kTreeStageBytes = 8 * 512, kTreeSmem = 4 * kTreeStages * kTreeStageBytes;
+
+// !HEAD: tree t's upstream gradient is row t / head.S of gy
+template <int V, bool HEAD, bool ONCE>
 __global__ void __launch_bounds__(128, 3) logic_tree_bwd_kernel(const float *__restrict__ x, TreeTables tt, const float *__restrict__ gy,
                                                              float *__restrict__ tapgrad, float *__restrict__ gw0, float *__restrict__ gw1,
-                                                             float *__restrict__ gw2, long long T, long long B, int wmode, TreeHead head)
+                                                             float *__restrict__ gw2, int T, int B, int wmode, TreeHead head)
 {
+    extern __shared__ __align__(16) unsigned char tree_smem[];
+    __shared__ float4 gates[4][7];
     const int lane = threadIdx.x & 31;
-    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    const int warp = (int)((blockIdx.x * 128u + threadIdx.x) >> 5), nwarps = (int)(gridDim.x * 4u);
+    // V = 4: the leaf rows arrive kTreeStages - 1 trips of 128 samples ahead in shared memory, each lane's 16 bytes by its own copy (so that
+    // nothing has to be synchronised), in one wave of blocks that walk on from tree to tree; a gate's values come a tree ahead.  What was
+    // waited for before: the classes' upstream gradients (tree_head_rows_kernel), rows and values of a tree one after the other at
+    // 12 warps per SM (k = 256, 256 samples: 269 us, now 193; k = 32, 100 samples 23 and 18).  The tree and trip fetched next:
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(tree_smem) + (threadIdx.x >> 5) * (kTreeStages * kTreeStageBytes) + lane * 16;
+    int ft = warp, fb = 0, fslot = 0, f_leaf = 0, f_next = 0;
+    auto fetch = [&] {
+        if (ft < T) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const float *row = x + ((long long)__shfl_sync(0xffffffffu, f_leaf, k) * B + fb + lane * 4);
+                if (fb + lane * 4 < B) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ring + fslot * kTreeStageBytes + k * 512), "l"(row) : "memory");
+            }
+            fb += 128;
+            if (fb >= B) {
+                fb = 0, ft += nwarps, f_leaf = f_next;
+                f_next = (ft + nwarps < T && lane < 8) ? __ldg(tt.leaf + (ft + nwarps) * 8 + lane) : 0;
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        fslot = fslot + 1 == kTreeStages ? 0 : fslot + 1;
+    };
+    int slot = 0;
+    if (V == 4) {
+        f_leaf = (warp < T && lane < 8) ? __ldg(tt.leaf + warp * 8 + lane) : 0;
+        f_next = (warp + nwarps < T && lane < 8) ? __ldg(tt.leaf + (warp + nwarps) * 8 + lane) : 0;
+#pragma unroll
+        for (int i = 0; i < kTreeStages - 1; ++i) fetch();
+    }
     // 128-thread blocks, three per SM: 168 registers, nothing spilled (at 256 threads x 2 blocks the limit of 128 registers
     // spilled 144 bytes).  The index tables are fetched one tree ahead, as in the forward kernel.
-    int my_leaf = (warp < T && lane < 8) ? __ldg(tt.leaf + warp * 8 + lane) : 0;
+    int my_leaf = (V != 4 && warp < T && lane < 8) ? __ldg(tt.leaf + warp * 8 + lane) : 0;
     int my_node = (warp < T && lane < 28) ? __ldg(tt.node + warp * 7 + (lane >> 2)) : 0;
-    for (long long t = warp; t < T; t += nwarps) {
-        const long long tn = t + nwarps;
-        const int nx_leaf = (tn < T && lane < 8) ? __ldg(tt.leaf + tn * 8 + lane) : 0;
-        const int nx_node = (tn < T && lane < 28) ? __ldg(tt.node + tn * 7 + (lane >> 2)) : 0;
+    int nx_node = (warp + nwarps < T && lane < 28) ? __ldg(tt.node + (warp + nwarps) * 7 + (lane >> 2)) : 0;
+    float raw[4];
+    tree_values(tt, my_node, lane, raw);
+    for (int t = warp; t < T; t += nwarps) {
+        const int tn = t + nwarps, tnn = tn + nwarps;
+        const int nx_leaf = (V != 4 && tn < T && lane < 8) ? __ldg(tt.leaf + tn * 8 + lane) : 0;
+        const int nn_node = (tnn < T && lane < 28) ? __ldg(tt.node + tnn * 7 + (lane >> 2)) : 0;
         Gate<float> g[7];
         float pq[4]; // the lane's four mixture entries, kept for the soft-max Jacobian at the end
-        tree_gates_of(tt, my_node, lane, wmode, g, pq);
-        const float *row[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) row[k] = x + (long long)__shfl_sync(0xffffffffu, my_leaf, k) * B;
+        for (int i = 0; i < 4; ++i) pq[i] = raw[i];
+        if (tn < T) tree_values(tt, nx_node, lane, raw); // a tree ahead
+        tree_gates_to(gates[threadIdx.x >> 5], lane, wmode, pq);
+#pragma unroll
+        for (int i = 0; i < 7; ++i) g[i] = tree_gate(gates[threadIdx.x >> 5], i);
         float bs[28];
 #pragma unroll
         for (int i = 0; i < 28; ++i) bs[i] = 0.f;
-        for (long long b0 = (long long)lane * V; b0 < B; b0 += 32 * V) {
+        for (int bb = 0; bb < B; bb += 32 * V) { // uniform over the warp: the rows' numbers are handed round
+            const int b0 = bb + lane * V;
             float a[8][V], dz[V], dg[4][V];
+            if constexpr (V == 4) {
+                fetch();
+                asm volatile("cp.async.wait_group %0;" ::"n"(kTreeStages - 1) : "memory");
+                if (b0 < B) {
 #pragma unroll
-            for (int k = 0; k < 8; ++k) vload<float, V>(row[k] + b0, a[k]);
+                    for (int k = 0; k < 8; ++k)
+                        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(a[k][0]), "=f"(a[k][1]), "=f"(a[k][2]), "=f"(a[k][3])
+                                     : "r"(ring + slot * kTreeStageBytes + k * 512));
+                }
+                slot = slot + 1 == kTreeStages ? 0 : slot + 1;
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const float *row = x + (long long)__shfl_sync(0xffffffffu, my_leaf, k) * B;
+                    if (b0 < B) vload<float, V>(row + b0, a[k]);
+                }
+            }
+            if (b0 >= B) continue;
             if (HEAD) {
                 const float taus = head.tau / __ldg(head.scale);
-                const float *ds = head.dscore + b0 * head.k + (unsigned)t / head.S;
+                const float *ds = head.dscore + (long long)b0 * head.k + (unsigned)t / head.S;
 #pragma unroll
                 for (int e = 0; e < V; ++e) dz[e] = __ldg(ds + e * head.k) / taus;
             } else {
-                vload<float, V>(gy + t * B + b0, dz);
+                vload<float, V>(gy + (long long)((unsigned)t / head.S) * B + b0, dz);
             }
 #pragma unroll
             for (int e = 0; e < V; ++e) {
@@ -741,8 +842,11 @@ __global__ void __launch_bounds__(128, 3) logic_tree_bwd_kernel(const float *__r
                     bs[4 * p] = fmaf(d, x0 * x1, bs[4 * p]), bs[4 * p + 1] = fmaf(d, x0, bs[4 * p + 1]);
                     bs[4 * p + 2] = fmaf(d, x1, bs[4 * p + 2]), bs[4 * p + 3] += d;
                 }
-                vstore<float, V>(tapgrad + (t * 8 + 2 * p) * B + b0, ta);
-                vstore<float, V>(tapgrad + (t * 8 + 2 * p + 1) * B + b0, tb);
+                float *const to = tapgrad + ((long long)(t * 8 + 2 * p) * B + b0);
+                if (ONCE)
+                    vstore_once<float, V>(to, ta), vstore_once<float, V>(to + B, tb);
+                else
+                    vstore<float, V>(to, ta), vstore<float, V>(to + B, tb);
             }
         }
         // batch totals: a transposed butterfly leaves total i on lane i, i.e. basis sum k = lane & 3 of gate lane >> 2 on
@@ -765,7 +869,7 @@ __global__ void __launch_bounds__(128, 3) logic_tree_bwd_kernel(const float *__r
         for (int k = 0; k < 4; ++k) s4[k] = __shfl_sync(0xffffffffu, v[0], (lane & ~3) + k);
         const float(&p)[4] = pq;
         const long long n = my_node;
-        my_leaf = nx_leaf, my_node = nx_node;
+        my_leaf = nx_leaf, my_node = nx_node, nx_node = nn_node;
         const int q = lane & 3;
         const float q3 = (float)(q >> 1), q2 = (float)(q & 1);
         const float base = (q3 - q2) * s4[0] - q3 * s4[1] + (q2 - q3) * s4[2] + q3 * s4[3];
@@ -788,7 +892,7 @@ __global__ void __launch_bounds__(128, 3) logic_tree_bwd_kernel(const float *__r
 template <int V>
 __global__ void __launch_bounds__(256) row_segment_sum_kernel(const float *__restrict__ rows, const int64_t *__restrict__ start,
                                                               const int32_t *__restrict__ list, float *__restrict__ gx, long long F,
-                                                              long long B)
+                                                              long long B, bool once)
 {
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -809,7 +913,11 @@ __global__ void __launch_bounds__(256) row_segment_sum_kernel(const float *__res
                     for (int u = 0; u < 4; ++u) {
                         const int r = __shfl_sync(0xffffffffu, mine, min(i0 + u, n - 1));
                         if (in) {
-                            vload<float, V>(rows + (long long)r * B + b0, v[u]);
+                            const float *from = rows + (long long)r * B + b0;
+                            if (once)
+                                vload_once<float, V>(from, v[u]);
+                            else
+                                vload<float, V>(from, v[u]);
                         } else {
 #pragma unroll
                             for (int k = 0; k < V; ++k) v[u][k] = 0.f;
@@ -1169,30 +1277,48 @@ static int logic_tree_bwd_impl(const float *x, const int32_t *leaf, const int32_
 {
     if (!tree_args_ok(x, leaf, node, w0, w1, w2, T, B, wmode) || (!gy && !head) || !tapgrad || !gw0 || !gw1 || !gw2 || in_dim <= 0) return CLB_ERR_ARG;
     if (gx && (!start || !list)) return CLB_ERR_ARG;
-    if (T * 8 > 0x7fffffffLL) return CLB_ERR_SHAPE;
+    if (T * 8 > 0x7fffffffLL || B > 0x7fffff00LL) return CLB_ERR_SHAPE;
     if (B == 0) return CLB_OK;
     TreeTables tt{leaf, node, {w0, w1, w2}};
     cudaStream_t st = (cudaStream_t)stream;
     const bool vec = B % 4 == 0 && aligned16(x) && (head || aligned16(gy)) && aligned16(tapgrad) && (!gx || aligned16(gx));
     const TreeHead none{nullptr, nullptr, 1, 1u, 1.f};
+    // leaf gradients beyond half the L2 go past it, both ways: x stays there (k = 256, 256 samples, 671 MB: 202 -> 193 us, their sums 129 -> 121;
+    // at k = 32, 33 MB, the sums 7.3 -> 8.5)
+    const bool once = T * 8 * B * 4 > (64LL << 20);
     int launched = 0;
     if (T > 0) {
-        const int grid = 2 * logic_grid(T);
+        const long long resident = (long long)sm_count() * 3; // vec: one wave, whose warps fetch ahead from tree to tree
+        const int grid = vec && (T + 3) / 4 > resident ? (int)resident : 2 * logic_grid(T);
+        TreeHead rows = none;
+        if (head && vec && gx && in_dim >= head->k) { // the input gradient's memory holds the classes' rows until the sums are written to it
+            tree_head_rows_kernel<<<(unsigned)((B * head->k + 255) / 256), 256, 0, st>>>(gx, B, *head);
+            gy = gx, rows.S = head->S, head = nullptr;
+            ++launched;
+        }
+        bool ok = true;
+        auto go = [&](auto kern, int smem, const TreeHead &h) {
+            if (smem) ok = ensure_dynamic_smem(kern, smem) == cudaSuccess;
+            if (ok) CLB_TRACED("logic_tree_bwd_kernel", st, kern<<<grid, 128, smem, st>>>(x, tt, gy, tapgrad, gw0, gw1, gw2, (int)T, (int)B, wmode, h));
+        };
         if (head && vec)
-            CLB_TRACED("logic_tree_bwd_kernel", st, logic_tree_bwd_kernel<4, true><<<grid, 128, 0, st>>>(x, tt, gy, tapgrad, gw0, gw1, gw2, T, B, wmode, *head));
+            go(logic_tree_bwd_kernel<4, true, false>, kTreeSmem, *head);
         else if (head)
-            CLB_TRACED("logic_tree_bwd_kernel", st, logic_tree_bwd_kernel<1, true><<<grid, 128, 0, st>>>(x, tt, gy, tapgrad, gw0, gw1, gw2, T, B, wmode, *head));
+            go(logic_tree_bwd_kernel<1, true, false>, 0, *head);
+        else if (vec && once)
+            go(logic_tree_bwd_kernel<4, false, true>, kTreeSmem, rows);
         else if (vec)
-            CLB_TRACED("logic_tree_bwd_kernel", st, logic_tree_bwd_kernel<4, false><<<grid, 128, 0, st>>>(x, tt, gy, tapgrad, gw0, gw1, gw2, T, B, wmode, none));
+            go(logic_tree_bwd_kernel<4, false, false>, kTreeSmem, rows);
         else
-            CLB_TRACED("logic_tree_bwd_kernel", st, logic_tree_bwd_kernel<1, false><<<grid, 128, 0, st>>>(x, tt, gy, tapgrad, gw0, gw1, gw2, T, B, wmode, none));
+            go(logic_tree_bwd_kernel<1, false, false>, 0, rows);
+        if (!ok) return check_launch(0);
         ++launched;
     }
     if (gx) {
         if (vec)
-            CLB_TRACED("row_segment_sum_kernel", st, row_segment_sum_kernel<4><<<logic_grid(in_dim), 256, 0, st>>>(tapgrad, start, list, gx, in_dim, B));
+            CLB_TRACED("row_segment_sum_kernel", st, row_segment_sum_kernel<4><<<logic_grid(in_dim), 256, 0, st>>>(tapgrad, start, list, gx, in_dim, B, once));
         else
-            CLB_TRACED("row_segment_sum_kernel", st, row_segment_sum_kernel<1><<<logic_grid(in_dim), 256, 0, st>>>(tapgrad, start, list, gx, in_dim, B));
+            CLB_TRACED("row_segment_sum_kernel", st, row_segment_sum_kernel<1><<<logic_grid(in_dim), 256, 0, st>>>(tapgrad, start, list, gx, in_dim, B, once));
         ++launched;
     }
     return check_launch(launched);
