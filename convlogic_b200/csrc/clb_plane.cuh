@@ -15,27 +15,19 @@ struct SlotInfo {
     int nslot; // 3 = the selection does not fit two staged planes (more channels, or taps outside the 3x3 window)
 };
 
-// channel -> slot map of output channel c's taps (one thread fills it)
-__device__ __forceinline__ void fill_slots(SlotInfo &si, const int32_t *__restrict__ sel, int c, int Ci)
+// channel -> slot map of an output channel's taps: the first channel that they name has slot 0, another one slot 1.  word: tap lane & 7 of
+// the selection; the whole warp calls this.  (One thread that walked the taps took longer than the soft-max of the gates.  The map goes
+// through shared memory because in registers it cost the kernels a resident block.)
+__device__ __forceinline__ void fill_slots(SlotInfo &si, int word, int Ci, int lane)
 {
-    int n = 0, chs[8];
-    bool inside = true;
-    for (int k = 0; k < 8; ++k) {
-        const int word = sel[c * 8 + k];
-        const int ch = (word >> 16) & 0xFFFF;
-        inside = inside && word >= 0 && ch < Ci && ((word >> 8) & 0xFF) < 3 && (word & 0xFF) < 3;
-        int slot = -1;
-        for (int j = 0; j < n; ++j)
-            if (chs[j] == ch) slot = j;
-        if (slot < 0) {
-            slot = n;
-            chs[n++] = ch;
-        }
-        si.slot[k] = slot;
-    }
-    si.ch[0] = min(chs[0], Ci - 1);
-    si.ch[1] = min(chs[n > 1 ? 1 : 0], Ci - 1);
-    si.nslot = (inside && n <= 2) ? n : 3;
+    const int ch = (word >> 16) & 0xFFFF;
+    const bool inside = __all_sync(0xffffffffu, word >= 0 && ch < Ci && ((word >> 8) & 0xFF) < 3 && (word & 0xFF) < 3);
+    const int first = __shfl_sync(0xffffffffu, ch, 0);
+    const unsigned rest = __ballot_sync(0xffffffffu, ch != first) & 0xffu;
+    const int other = __shfl_sync(0xffffffffu, ch, rest ? __ffs((int)rest) - 1 : 0);
+    const unsigned more = __ballot_sync(0xffffffffu, ch != first && ch != other);
+    if (lane < 8) si.slot[lane] = (int)(rest >> lane & 1u);
+    if (lane == 0) si.ch[0] = min(first, Ci - 1), si.ch[1] = min(other, Ci - 1), si.nslot = !inside || more ? 3 : rest ? 2 : 1;
 }
 
 // 28 per-lane sums: lane i ends up with the warp's sum i (a transposed butterfly over the 32 lanes)

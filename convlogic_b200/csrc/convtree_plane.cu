@@ -169,10 +169,11 @@ template <int S> struct FwdCfg {
     static constexpr int LANES = S == 28 ? 32 : S, RPG = S == 6 ? GSIZE / LANES : GSIZE / 32 * (32 / LANES), ROWS = ROW_PAIRS ? HP / 2 : NIMG / 2 * HP, SUB = (ROWS + RPG - 1) / RPG;
     static constexpr bool FULL = 32 % S == 0 && ROWS % RPG == 0;  // else some threads have no position, or none in the last turn
     static_assert(IMG >= R * P && IMG % 4 == 0 && P % 4 == 0 && (!TMA || IMG == R * P) && (SUB == 1 || NIMG <= 2), "tile geometry");
-    static constexpr int STAGES = S == 16 ? 4 : 3;
+    static constexpr int STAGES = S == 16 ? 4 : S == 8 || S == 4 ? 2 : 3;
     static constexpr int SMEM = GROUPS * STAGES * STAGE_BYTES + (FULL ? 0 : 2 * 2 * P * 4); // rows that a last turn reads in vain
-    // resident per SM: by registers (16 and 6), else by shared memory
-    static constexpr int BLOCKS = S == 16 ? 7 : S >= 28 ? 6 : S == 8 || S == 6 ? 5 : S == 4 ? 4 : 3;
+    // resident per SM, by registers (16, 8, 6) or shared memory.  8: with three stages and 80 registers 133 us for 1024 -> 4096 channels, 256 images,
+    // now 125; four blocks and three stages 99 us for 4096 -> 8192 of 4x4, now 88.
+    static constexpr int BLOCKS = S == 16 ? 7 : S >= 28 || S == 4 ? 6 : S == 8 || S == 6 ? 5 : 3;
     // asynchronous copies of PIECE floats: per iteration, and per thread
     static constexpr int PIECE = S % 4 == 0 ? 4 : 2, UNITS = NIMG * 2 * S * (S / PIECE), CPQ = (UNITS + GSIZE - 1) / GSIZE;
 };
@@ -201,7 +202,7 @@ template <int S, int ST, int J> __device__ __forceinline__ void fwd_stage(const 
 }
 
 template <int S>
-__global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __grid_constant__ CUtensorMap xmap, const float *__restrict__ x,
+__global__ void __launch_bounds__(kThreads, FwdCfg<S>::BLOCKS) convtree_fwd_plane_kernel(const __grid_constant__ CUtensorMap xmap, const float *__restrict__ x,
                                                                       const float *__restrict__ w, const int32_t *__restrict__ sel,
                                                                       float *__restrict__ y, uint8_t *__restrict__ amax, Args s)
 {
@@ -233,8 +234,10 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
     Gate<float> *sg = sgs[gid];
     SlotInfo &si = sis[gid];
 
-    if (gt < 7) sg[gt] = gate_load<float>(w + ((size_t)c * 7 + gt) * 16, s.wmode);
-    if (gt == (Cf::WIDE ? 32 : 8)) fill_slots(si, sel, c, s.Ci);
+    const int taps = !Cf::WIDE || warp == 0 ? __ldg(sel + (size_t)c * 8 + (lane & 7)) : 0;
+    const int gate = Cf::WIDE ? tid - 32 : lane;
+    if (gate >= 0 && gate < 7) sg[gate] = gate_load<float>(w + ((size_t)c * 7 + gate) * 16, s.wmode);
+    if (!Cf::WIDE || warp == 0) fill_slots(si, taps, s.Ci, lane);
     if (gt == (Cf::WIDE ? 64 : 9)) {
         for (int st = 0; st < Cf::STAGES; ++st) clb_tma::mbar_init(&full[gid][st], 1);
         clb_tma::mbar_init_fence();
@@ -344,8 +347,10 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
         group_sync();
         CLB_FWD_ISSUE_CP(0, 0)
         CLB_FWD_ISSUE_CP(1, 1)
-        CLB_FWD_ISSUE_CP(2, 2)
-        static_assert(Cf::TMA || Cf::STAGES == 3, "prologue of the cp.async ring");
+        if constexpr (Cf::STAGES > 2) {
+            CLB_FWD_ISSUE_CP(2, 2)
+        }
+        static_assert(Cf::TMA || Cf::STAGES <= 3, "prologue of the cp.async ring");
     }
 
     // 2x2 pool: lanes ox and ox^1 hold the two columns of a window, each for both members of the pair.  The even lane
@@ -416,7 +421,9 @@ __global__ void __launch_bounds__(kThreads) convtree_fwd_plane_kernel(const __gr
     }
         CLB_FWD_STAGE(0)
         CLB_FWD_STAGE(1)
-        CLB_FWD_STAGE(2)
+        if constexpr (Cf::STAGES > 2) {
+            CLB_FWD_STAGE(2)
+        }
         if constexpr (Cf::STAGES > 3) {
             CLB_FWD_STAGE(3)
         }
@@ -443,7 +450,7 @@ template <int S> struct BwdCfg {
     static constexpr int IMG = R * P;
     static constexpr int SLOT = (NIMG * IMG + 31) / 32 * 32;
     static constexpr int STAGE_FLOATS = 2 * SLOT, STAGE_BYTES = STAGE_FLOATS * 4;
-    static constexpr int XST = 3;                       // stages of input planes
+    static constexpr int XST = S == 4 ? 2 : 3;          // stages of input planes
     static constexpr int GT_BYTES = XST * STAGE_BYTES;  // byte distance from stage 0 to the gradient tile: the same cell offsets
     static constexpr int WARP_BYTES = (XST + 1) * STAGE_BYTES;
     static constexpr int SMEM = (kThreads / 32) * WARP_BYTES;
@@ -506,8 +513,9 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const floa
     const int c = (int)(task % s.C), part = (int)(task / s.C);
     Gate<float> *sg = sgs[warp];
     SlotInfo &si = sis[warp];
+    const int taps = __ldg(sel + (size_t)c * 8 + (lane & 7));
     if (lane < 7) sg[lane] = gate_load<float>(w + ((size_t)c * 7 + lane) * 16, s.wmode);
-    if (lane == 8) fill_slots(si, sel, c, s.Ci);
+    fill_slots(si, taps, s.Ci, lane);
     __syncwarp();
     Gate<float> g[7];
 #pragma unroll
@@ -574,8 +582,10 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const floa
     __syncwarp();
     CLB_BWD_ISSUE_CP(0, 0)
     CLB_BWD_ISSUE_CP(1, 1)
-    CLB_BWD_ISSUE_CP(2, 2)
-    static_assert(XST == 3, "prologue of the cp.async ring");
+    if constexpr (XST > 2) {
+        CLB_BWD_ISSUE_CP(2, 2)
+    }
+    static_assert(XST == 2 || XST == 3, "prologue of the cp.async ring");
 
     // upstream gradient and arg-max: fetched one iteration ahead
     float dz_next[WPT];
@@ -637,7 +647,9 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const floa
     }
         CLB_BWD_STAGE(0)
         CLB_BWD_STAGE(1)
-        CLB_BWD_STAGE(2)
+        if constexpr (XST > 2) {
+            CLB_BWD_STAGE(2)
+        }
 #undef CLB_BWD_STAGE
 #undef CLB_BWD_ISSUE_CP
     }
@@ -685,7 +697,7 @@ template <int ST> __device__ __forceinline__ void bww_window(uint32_t base, cons
     }
 }
 
-__global__ void __launch_bounds__(kThreads) convtree_bwd_w_plane32_kernel(const __grid_constant__ CUtensorMap xmap, const float *__restrict__ gy,
+__global__ void __launch_bounds__(kThreads, 5) convtree_bwd_w_plane32_kernel(const __grid_constant__ CUtensorMap xmap, const float *__restrict__ gy,
                                                                           const float *__restrict__ w, const int32_t *__restrict__ sel,
                                                                           const uint8_t *__restrict__ amax, float *__restrict__ partial, Args s)
 {
@@ -699,8 +711,9 @@ __global__ void __launch_bounds__(kThreads) convtree_bwd_w_plane32_kernel(const 
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int c = blockIdx.x % s.C, part = blockIdx.x / s.C;
+    const int taps = warp == 1 ? __ldg(sel + (size_t)c * 8 + (lane & 7)) : 0;
     if (tid < 7) sg[tid] = gate_load<float>(w + ((size_t)c * 7 + tid) * 16, s.wmode);
-    if (tid == 32) fill_slots(si, sel, c, s.Ci);
+    if (warp == 1) fill_slots(si, taps, s.Ci, lane);
     if (tid == 64) {
         for (int st = 0; st < Cf::STAGES; ++st) clb_tma::mbar_init(&full[st], 1);
         clb_tma::mbar_init_fence();

@@ -96,8 +96,9 @@ __global__ void __launch_bounds__(kThreads, Tile<S>::BLOCKS) convtree_bwd_plane_
         else
             __syncthreads();
     };
+    const int taps = gwarp == 0 ? __ldg(s.sel + (size_t)c * 8 + (lane & 7)) : 0;
     if (gt < 7) sgs[gid][gt] = gate_load<float>(s.w + ((size_t)c * 7 + gt) * 16, s.wmode);
-    if (gt == 8) fill_slots(sis[gid], s.sel, c, s.Ci);
+    if (gwarp == 0) fill_slots(sis[gid], taps, s.Ci, lane);
     const uint32_t tile = clb_tma::smem_addr(smem_raw) + gid * 2 * T::GRAD;
     for (int i = gt; i < 2 * T::GRAD / 4; i += T::GSIZE) sts1<0>(tile + 4 * i, 0.f); // halos stay zero, the gradient tile starts as zeros
     group_sync();
