@@ -68,3 +68,20 @@ def test_one_channel_image_of_more_than_65536_pixels():
     got = cb.CompiledLogicNet(net.eval(), input_shape=(1, 260, 260)).compile()(x)
     with torch.no_grad():
         assert torch.equal(got, net.cuda()(cb.PackBitsTensor(x, 64)))
+
+
+@pytest.mark.parametrize("batch", [32, 33, 64, 65, 96, 127, 224, 225, 256, 257, 448, 449, 512, 1025])
+def test_slabs_of_every_size(one_launch, batch):
+    """Batches around the slabs of 32, 64 and 128 samples and around the points where the choice between them changes."""
+    import convlogic_b200 as cb
+
+    torch.manual_seed(batch)
+    net = cb.ConvLogicMnistModel(k_param=2).network
+    for p in net.parameters():
+        p.data.normal_()
+    compiled = cb.CompiledLogicNet(net.eval(), input_shape=(1, 28, 28)).compile()
+    x = torch.rand(batch, 1, 28, 28, device="cuda") < 0.4
+    one_launch(0)
+    want = compiled(x)
+    one_launch(2)
+    assert torch.equal(compiled(x), want)

@@ -75,3 +75,34 @@ def test_records_laid_out_on_every_call_equal_those_laid_out_once():
     finally:
         _lib.check(lib.clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 1))
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("batch", [100, 1100])
+@pytest.mark.parametrize("kind", ["one channel each", "one pair", "chain", "any pairs"])
+@pytest.mark.parametrize("side,c", [(32, 40), (16, 70), (8, 300), (4, 700)])
+def test_output_channels_in_an_order_that_shares_planes(side, c, kind, batch):
+    """Trails through the graph of input channels: several runs of items per block, records with no, one or two new planes, a run that begins in the
+    middle of a trail, output channels that read one input channel only."""
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    ci = 5
+    torch.manual_seed(side + c)
+    i = torch.arange(c)
+    first, second = {"one channel each": (i % ci, i % ci), "one pair": (i * 0 + 1, i * 0 + 3), "chain": (i % ci, (i + 1) % ci),
+                     "any pairs": tuple(torch.randint(0, ci, (2, c)))}[kind]
+    ch = torch.where(torch.rand(c, 8) < 0.5, first[:, None], second[:, None])
+    words = ((ch << 16) | (torch.randint(0, 3, (c, 8)) << 8) | torch.randint(0, 3, (c, 8))).int()
+    feat = c * (side // 2) ** 2
+    net = torch.nn.Sequential(cb.ConvLogicLayer(ci, c, padding=1, kernel=3, selection=words, complete=True), torch.nn.Flatten(),
+                              cb.LogicLayer(feat, feat // 2 * 2), cb.GroupSum(2)).cuda()
+    for p in net.parameters():
+        p.data.normal_()
+    bits = torch.rand(batch, ci, side, side, device="cuda") < 0.5
+    with torch.no_grad():
+        want = net.eval()(bits.float()).round().long()
+    _lib.check(_lib.lib().clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 0))
+    try:
+        assert torch.equal(cb.CompiledLogicNet(net, input_shape=(ci, side, side)).compile()(bits).long(), want)
+    finally:
+        _lib.check(_lib.lib().clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 1))
