@@ -13,8 +13,8 @@
 // A feature whose gradient the walk completes is `closed`; the others (cuts, features with other than two readers) are
 // in the `open` list, and their gradient is taken from the consumer lists (logic_bwd.cu).
 //
-// What bounds both passes is DRAM: 256000 -> 256000, 1024 samples, forward 2.1 GB in 344 us (436 as a walk of the neurons in their own
-// order, stretch by stretch), backward 3.3 GB with the sums in 512 + 23 us (951 + 20 for the walk of the features), open features 14.
+// What bounds both passes is DRAM: 256000 -> 256000, 1024 samples, forward 2.1 GB in 345 us (436 as a walk of the neurons in their own
+// order, stretch by stretch), backward 3.3 GB with the sums in 503 + 16 us (951 + 20 for the walk of the features), open features 14.
 // Eight lanes own a range of positions and a stretch of 64 samples, the stretches of a row lying side by side in a block. Two
 // neurons' rows in flight per group and four (forward) or two (backward: 100 registers) blocks per SM; with three blocks the backward
 // spills (564 -> 624 us), four neurons at two blocks wait longer for the first (650), stretches of 32 samples read pieces too
@@ -164,8 +164,9 @@ __global__ void __launch_bounds__(256, kFwdBlocks) logic_path_fwd_kernel(const f
     }
 }
 
-// Input gradient of the closed features and the four basis sums of every neuron, partial [stretch][position][4].
-template <int V, int R, int U>
+// Input gradient of the closed features and the four basis sums of every neuron, partial [stretch, or four of them][position][4].
+// MERGED: a warp's four groups are neighbouring stretches of the same neurons, and their sums are added (as a branch it cost the rest 7 to 19 %).
+template <int V, int R, int U, bool MERGED>
 __global__ void __launch_bounds__(256, kBwdBlocks) logic_path_bwd_kernel(const float *__restrict__ x, const float *__restrict__ gy, const int4 *__restrict__ rec,
                                                              const float4 *__restrict__ coef, float *__restrict__ gx, float *__restrict__ partial, int n,
                                                              int B, int cols, int ranges)
@@ -175,7 +176,8 @@ __global__ void __launch_bounds__(256, kBwdBlocks) logic_path_bwd_kernel(const f
     const PathUnit t(n, cols, ranges);
     const int s0 = t.col * 8 * V * R + t.l * V, left = B - s0;
     x += s0, gy += s0, gx += s0;
-    partial += ((size_t)t.col * n + t.p0) * 4 + t.l;
+    partial += ((size_t)(MERGED ? t.col >> 2 : t.col) * n + t.p0) * 4 + t.l;
+    const bool writes = !MERGED || (threadIdx.x & 24) == 0;
     const bool up4 = t.l & 4, up2 = t.l & 2, up1 = t.l & 1;
     const int4 none = make_int4(-1, 0, 0, kLinked);
     int4 r[U];
@@ -244,14 +246,15 @@ __global__ void __launch_bounds__(256, kBwdBlocks) logic_path_bwd_kernel(const f
 #pragma unroll
             for (int i = 0; i < 2; ++i) a2[i] = (up2 ? a4[2 + i] : a4[i]) + __shfl_xor_sync(0xffffffffu, up2 ? a4[i] : a4[2 + i], 2);
             s = (up1 ? a2[1] : a2[0]) + __shfl_xor_sync(0xffffffffu, up1 ? a2[0] : a2[1], 1);
-            if (t.p0 + d + u0 + (t.l >> 2) < t.p1) partial[(size_t)(d + u0) * 4] = s; // lane i: sum i & 3 of neuron i >> 2
+            if (MERGED) s += __shfl_xor_sync(0xffffffffu, s, 8), s += __shfl_xor_sync(0xffffffffu, s, 16);
+            if (writes && t.p0 + d + u0 + (t.l >> 2) < t.p1) partial[(size_t)(d + u0) * 4] = s; // lane i: sum i & 3 of neuron i >> 2
         }
     }
 }
 
 // Adds the stretches' basis sums of a neuron in stretch order and turns them into its 16 gradients: a thread per position.
 __global__ void __launch_bounds__(128) logic_path_finish_kernel(const float4 *__restrict__ partial, const int4 *__restrict__ rec, const float *__restrict__ w,
-                                                                float *__restrict__ gw, int n, int cols, int wmode)
+                                                                float *__restrict__ gw, int n, int parts, int wmode)
 {
     const int p = blockIdx.x * 128 + threadIdx.x;
     if (p >= n) return;
@@ -259,7 +262,7 @@ __global__ void __launch_bounds__(128) logic_path_finish_kernel(const float4 *__
     float v[16], s[4] = {0.f, 0.f, 0.f, 0.f}, out[16];
     load16(w + (size_t)j * 16, v);
 #pragma unroll 8
-    for (int c = 0; c < cols; ++c) {
+    for (int c = 0; c < parts; ++c) {
         const float4 q = __ldg(partial + (size_t)c * n + p);
         s[0] += q.x, s[1] += q.y, s[2] += q.z, s[3] += q.w;
     }
@@ -283,19 +286,21 @@ static size_t up16(size_t n) { return (n + 15) & ~(size_t)15; }
 int clb_logic_bwd_open(const float *x, const float *gy, const float *coef, const int32_t *start32, const void *entry, const int32_t *open, int64_t n_open,
                        float *gx, int64_t B, int vec, int wide, cudaStream_t st); // logic_bwd.cu
 
-// A group's stretch is 64 samples, or 32 where that leaves fewer lanes idle; as many ranges as the resident blocks have groups for, of
-// eight positions at least.
+// A group's stretch is 64 samples, or 32 where that leaves a quarter fewer lanes idle (equally full, stretches of 32 are a quarter slower);
+// as many ranges as the resident blocks have groups for, of eight positions at least.  Partial sums beyond 24 MB are added over four
+// stretches first (us of a backward without / with: 256000 x 1024 560 / 532, 250000 x 511 357 / 353; 64000 x 256 60 / 64, 24000 x 1020 83 / 91).
 struct PathCut {
     bool wide;
-    int cols, ranges;
+    int cols, ranges, sums; // sums: partial sums per neuron
     unsigned blocks;
 };
 static PathCut path_cut(int64_t n, int64_t B, int resident)
 {
     PathCut c;
     const int64_t c64 = (B + 63) / 64, c32 = (B + 31) / 32;
-    c.wide = 2 * c64 == c32 || B > 512;
+    c.wide = 3 * c64 < 2 * c32;
     c.cols = (int)(c.wide ? c64 : c32);
+    c.sums = c.cols % 4 || !c.wide || n * c.cols * 16 < (24LL << 20) ? c.cols : c.cols / 4;
     int64_t r = (int64_t)sm_count() * resident * 32 / c.cols;
     if (r > n / 8) r = n / 8;
     if (r < 1) r = 1;
@@ -312,15 +317,15 @@ static int path_vec(int64_t B, std::initializer_list<const void *> rows)
 }
 
 // Where each feature has two readers, so that nearly all gradients are completed on the way, from these sizes of x on (us without / with):
-// forward, beyond the L2's useful half: 128000 x 300 84 / 75, 250000 x 128 68 / 63, 64000 x 1000 120 / 116; 64000 x 256 35 / 36, 20000 x 500
-// 25 / 26; backward, where three launches have something to do: 16000 x 512 42 / 38, 40000 x 200 48 / 46, 100000 x 97 69 / 56, 250000 x 511
-// 790 / 357; 64000 x 64 28 / 32, 8000 x 100 19 / 24.  Elsewhere the input is in the L2, or is read once either way (4096 -> 40960 x 500
+// forward, beyond the L2's useful half: 128000 x 300 84 / 75, 250000 x 128 68 / 63, 64000 x 1000 120 / 116; 250000 x 101 66 / 69, 100000 x 250
+// 53 / 54, 64000 x 256 35 / 36; backward, where three launches have something to do: 65536 x 128 42 / 42, 16000 x 512 42 / 38, 20000 x 420
+// 46 / 42, 260000 x 32 71 / 60, 100000 x 97 69 / 56, 250000 x 66 138 / 96, 250000 x 511 790 / 353; 64000 x 64 28 / 32, 8000 x 100 19 / 24.  Elsewhere the input is in the L2, or is read once either way (4096 -> 40960 x 500
 // forward 29 / 32, backward 71 / 89; 300000 -> 200000 x 256 103 / 110, 265 / 267).
 extern "C" int clb_logic_path_pays(int64_t in_dim, int64_t out_dim, int64_t B, int64_t n_open, int what)
 {
     const int64_t bytes = in_dim * B * 4;
     if (in_dim != out_dim || 16 * n_open > in_dim) return 0;
-    return bytes >= (what == 0 ? 96LL << 20 : 32LL << 20);
+    return bytes >= (what == 0 ? 120LL << 20 : 32LL << 20);
 }
 
 extern "C" size_t clb_logic_path_scratch_bytes(int64_t in_dim, int64_t out_dim)
@@ -381,7 +386,7 @@ extern "C" int clb_logic_path_fwd(const float *x, const void *rec, const float *
 
 extern "C" size_t clb_logic_path_bwd_scratch_bytes(int64_t out_dim, int64_t B)
 {
-    return out_dim > 0 && B > 0 ? (size_t)path_cut(out_dim, B, kBwdBlocks).cols * (size_t)out_dim * 16 : 0;
+    return out_dim > 0 && B > 0 ? (size_t)path_cut(out_dim, B, kBwdBlocks).sums * (size_t)out_dim * 16 : 0;
 }
 
 extern "C" int clb_logic_path_bwd(const float *x, const float *w, const float *coef, const float *gy, float *gx, float *gw, const int32_t *start32,
@@ -402,16 +407,18 @@ extern "C" int clb_logic_path_bwd(const float *x, const float *w, const float *c
         CLB_TRACED("logic_path_bwd_kernel", st,
                    kern<<<c.blocks, 256, 0, st>>>(x, gy, (const int4 *)rec, (const float4 *)coef, gx, (float *)scratch, (int)out_dim, (int)B, c.cols, c.ranges));
     };
+    // (stretches of 32 samples are few: their sums are never merged)
+    const bool merged = c.sums != c.cols;
     switch (vec) {
-    case 4: c.wide ? go(logic_path_bwd_kernel<4, 2, 2>) : go(logic_path_bwd_kernel<4, 1, 4>); break;
-    case 2: c.wide ? go(logic_path_bwd_kernel<2, 4, 2>) : go(logic_path_bwd_kernel<2, 2, 4>); break;
-    default: c.wide ? go(logic_path_bwd_kernel<1, 8, 2>) : go(logic_path_bwd_kernel<1, 4, 4>); break;
+    case 4: merged ? go(logic_path_bwd_kernel<4, 2, 2, true>) : c.wide ? go(logic_path_bwd_kernel<4, 2, 2, false>) : go(logic_path_bwd_kernel<4, 1, 4, false>); break;
+    case 2: merged ? go(logic_path_bwd_kernel<2, 4, 2, true>) : c.wide ? go(logic_path_bwd_kernel<2, 4, 2, false>) : go(logic_path_bwd_kernel<2, 2, 4, false>); break;
+    default: merged ? go(logic_path_bwd_kernel<1, 8, 2, true>) : c.wide ? go(logic_path_bwd_kernel<1, 8, 2, false>) : go(logic_path_bwd_kernel<1, 4, 4, false>); break;
     }
     int rc = check_launch();
     if (rc == CLB_OK && n_open) rc = clb_logic_bwd_open(x, gy, coef, start32, entry, open, n_open, gx, B, vec, c.wide, st);
     if (rc != CLB_OK) return rc;
     CLB_TRACED("logic_path_finish_kernel", st,
                logic_path_finish_kernel<<<(unsigned)((out_dim + 127) / 128), 128, 0, st>>>((const float4 *)scratch, (const int4 *)rec, w, gw, (int)out_dim,
-                                                                                           c.cols, wmode));
+                                                                                           c.sums, wmode));
     return check_launch();
 }

@@ -127,7 +127,7 @@ def test_lists_that_contradict_the_connections_are_noticed():
         assert torch.equal(rec[1:, 1][linked], rec[:-1, 2][linked])
 
 
-@pytest.mark.parametrize("width,batch,path", [(40000, 210, True), (40000, 200, False), (83400, 101, True), (83000, 101, False), (28000, 900, True)])
+@pytest.mark.parametrize("width,batch,path", [(40000, 210, True), (40000, 200, False), (83400, 101, True), (83000, 101, False), (28000, 900, True), (100000, 1024, True), (100000, 1022, True), (99001, 1021, True)])
 def test_layers_take_the_path_by_size(width, batch, path):
     import convlogic_b200 as cb
     from convlogic_b200 import _lib, ops
