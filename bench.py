@@ -194,10 +194,10 @@ def traced(fn, steps):
 # chunk (c4) of the default workload sizes: dram__bytes.sum over one capture of the same bench command.  Other sizes, and
 # kernels without an entry, report null.
 NCU_TRAFFIC = {
-    "c3": {"convtree_bwd_plane_kernel": 1881.2e6, "plane_sum_kernel": 1514.0e6, "logic_tree_bwd_kernel": 948.7e6,
-           "row_segment_sum_kernel": 703.1e6, "convtree_fwd_plane_kernel": 411.5e6, "adam_step_kernel": 240.4e6,
-           "logic_tree_fwd_sum_kernel": 89.3e6, "convtree_bwd_w_plane32_kernel": 94.5e6},
-    "c4": {"packed_convtree_slab3_kernel": 2667.6e6, "packed_tree_kernel": 1603.2e6, "group_popcount_kernel": 672.0e6, "thermometer_pack_kernel": 64.0e6},
+    "c3": {"convtree_bwd_plane_kernel": 1847.5e6, "plane_sum_kernel": 1385.8e6, "logic_tree_bwd_kernel": 853.7e6,
+           "row_segment_sum_kernel": 680.3e6, "convtree_fwd_plane_kernel": 403.9e6, "adam_step_kernel": 240.2e6,
+           "logic_tree_fwd_sum_kernel": 83.2e6, "convtree_bwd_w_plane32_kernel": 93.9e6},
+    "c4": {"packed_convtree_slab3_kernel": 1932.8e6, "packed_tree_kernel": 1627.6e6, "group_popcount_kernel": 672.0e6, "thermometer_pack_kernel": 64.2e6},
 }
 
 
@@ -689,7 +689,10 @@ def run_c5(ctx, args):
         "logic_bwd_w_kernel": (xin + row) + (layers("logic_bwd_w_kernel") - 1) * 2 * row,  # layer 1 and others: gy + x
         "logic_bwd_x_kernel": layers("logic_bwd_x_kernel") * 3 * row,                      # gy + x + gx
         "logic_fwd_cols_kernel": layers("logic_fwd_cols_kernel") * 2 * row,                # the layers that walk the batch in stretches
-        "logic_bwd_kernel": layers("logic_bwd_kernel") * 3 * row,                          # both gradients: gy + x + gx
+        "logic_path_fwd_kernel": layers("logic_path_fwd_kernel") * 2 * row,                # the layers walked as paths
+        "logic_path_bwd_kernel": layers("logic_path_bwd_kernel") * 3 * row,                # both gradients: gy + x + gx
+        # the same for layers walked by feature (behind a path it takes the one gradient row in a hundred that the path leaves open)
+        "logic_bwd_kernel": (layers("logic_bwd_kernel") - layers("logic_path_bwd_kernel")) * 3 * row,
         "group_sum_partial_kernel": row, "group_sum_bwd_kernel": row,
     }
     kernels = kernel_table(trace, names, peak, traffic=None)

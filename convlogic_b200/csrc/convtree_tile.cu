@@ -15,7 +15,7 @@
 // columns sit one bank lower, so that four neighbouring pixels of an image row are two aligned pairs; without that it would
 // be 1.66, and the copies in and out would cost more than the difference).  The planes arrive through registers, one iteration
 // ahead, because no copy engine can split columns.
-// 256 images, 256 -> 1024 channels of 16x16: 298 us with row-major tiles fetched by TMA, 259 with these.  (8x8 and 4x4 images keep the
+// 256 images, 256 -> 1024 channels of 16x16: 298 us with row-major tiles fetched by TMA, 241 with these.  (8x8 and 4x4 images keep the
 // row-major tiles of convtree_plane.cu: the many small copies cost these kernels more than the passes they save, 291 against 279 us
 // for 1024 -> 4096 channels of 8x8, 220 against 186 for 4096 -> 8192 of 4x4.)
 #include "clb_plane.cuh"

@@ -10,7 +10,7 @@
 // rows are 16-byte aligned).  One wave of blocks walks the features stretch by stretch, so that all work on the same columns of x
 // and gy: with 64 samples (256 bytes of a row) the columns of a layer whose activation is ten times the L2 are about a cache's
 // worth, and a row fetched for one consumer is often still there for the next (256000 neurons, batch 1024: 3.8 GB read from DRAM
-// instead of 5.2).  Shorter stretches make DRAM pages short of work, longer ones fall out of the cache.
+// instead of 5.2; layers with as many neurons as features no longer come here at such sizes, logic_path.cu).  Shorter stretches make DRAM pages short of work, longer ones fall out of the cache.
 // What binds is the bytes in flight per SM (the rows of 24 warps; 61 % of the DRAM rate): eight lanes with two vectors each at
 // three blocks per SM beat 16 lanes with one vector (0.95 against 1.00 to 1.2 ms for 256000 x 1024), four entries at a time (1.57),
 // two blocks (1.23) and fetching the tables a feature ahead (1.03: it costs registers, hence rows).  No division anywhere, sums
