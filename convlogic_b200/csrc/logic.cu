@@ -1252,7 +1252,7 @@ extern "C" int clb_logic_tree_fwd_ce(const float *x, const int32_t *leaf, const 
                                      size_t scratch_bytes, int64_t T, int64_t B, int k, double tau, int wmode, void *stream)
 {
     if (!tree_args_ok(x, leaf, node, w0, w1, w2, T, B, wmode) || !labels || !dscore || !loss || k <= 0 || tau == 0.0) return CLB_ERR_ARG;
-    if (T <= 0 || B <= 0 || T % k || k > 32 || B % 4 || B > 512 || !aligned16(x) || T / k > 0x7fffffffLL) return CLB_ERR_SHAPE;
+    if (T <= 0 || B <= 0 || T % k || k > 32 || B % 4 || B > 512 || !aligned16(x) || T * 8 > 0x7fffffffLL) return CLB_ERR_SHAPE;
     if (!scratch || scratch_bytes < clb_logic_tree_fwd_ce_scratch_bytes(T, B, k)) return CLB_ERR_SCRATCH;
     TreeTables tt{leaf, node, {w0, w1, w2}};
     cudaStream_t st = (cudaStream_t)stream;
