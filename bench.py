@@ -197,7 +197,7 @@ NCU_TRAFFIC = {
     "c3": {"convtree_bwd_plane_kernel": 1847.5e6, "plane_sum_kernel": 1385.8e6, "logic_tree_bwd_kernel": 853.7e6,
            "row_segment_sum_kernel": 680.3e6, "convtree_fwd_plane_kernel": 403.9e6, "adam_step_kernel": 240.2e6,
            "logic_tree_fwd_sum_kernel": 83.2e6, "convtree_bwd_w_plane32_kernel": 93.9e6},
-    "c4": {"packed_convtree_slab3_kernel": 1932.8e6, "packed_tree_kernel": 1627.6e6, "group_popcount_kernel": 672.0e6, "thermometer_pack_kernel": 64.2e6},
+    "c4": {"packed_convtree_slab3_kernel": 1932.8e6, "packed_tree_count_kernel": 439.2e6, "thermometer_pack_kernel": 64.2e6},
 }
 
 
@@ -472,8 +472,8 @@ def run_c4(ctx, args):
     ms_e2e = ctx.timed(step_e2e, 1, 1)
     clocks = sampler.stop()
     peak, kind = measured_peaks()
-    per_image = {"packed_convtree_slab3_kernel": 44672 + 65536 + 65536 + 49152, "packed_tree_kernel": 16384 + 81920,
-                 "group_popcount_kernel": 81920 + 40, "thermometer_pack_kernel": 3072 + 11904}
+    per_image = {"packed_convtree_slab3_kernel": 44672 + 65536 + 65536 + 49152, "packed_tree_count_kernel": 16384 + 40,
+                 "thermometer_pack_kernel": 3072 + 11904}
     kernels = kernel_table(trace, {k: v * chunk for k, v in per_image.items()}, peak, traffic=NCU_TRAFFIC["c4"] if chunk == 8192 else None)
     top = kernels[0] if kernels else {}
     alg = 1388200.0 * (hi - lo)   # layer-by-layer algorithmic bytes of this rank's shard

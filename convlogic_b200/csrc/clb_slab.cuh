@@ -48,3 +48,6 @@ int clb_thermometer_pack_units(const void *pixels, int pixels_u8, const float *t
 int clb_packed_rows_to_slabs(const void *rows, void *slabs, int64_t C, int64_t HW, int64_t U, int side, clb::Order order, cudaStream_t st);
 // class sums over rows of U units, of whose samples the first B count
 int clb_group_popcount_units(const void *x, int32_t *counts, int64_t F, int64_t U, int64_t B, int k, cudaStream_t st);
+// the same over the trees of clb_packed_tree on rows of U units, without their outputs; CLB_ERR_SHAPE: run the two apart
+int clb_packed_tree_count(const void *x, const int32_t *leaf, const uint8_t *ops, int32_t *counts, int64_t in_dim, int64_t out_dim, int levels, int64_t U,
+                          int64_t B, int k, cudaStream_t st);

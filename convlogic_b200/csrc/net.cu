@@ -406,6 +406,11 @@ extern "C" int clb_net_forward(const clb_net *net, int input_kind, const void *i
             cur ^= 1;
             feat = L.out_dim;
         } else {
+            if (i + 1 == net->layers.size()) { // with their class sums
+                st = clb_packed_tree_count(buf[cur], (const int32_t *)(P + L.off_a), P + L.off_ops, counts, L.in_dim, L.out_dim, L.levels, U, batch,
+                                           net->num_classes, cs);
+                if (st != CLB_ERR_SHAPE) return st;
+            }
             st = clb_packed_tree(buf[cur], (const int32_t *)(P + L.off_a), P + L.off_ops, buf[cur ^ 1], L.in_dim, L.out_dim, L.levels, words,
                                  64, stream);
             if (st != CLB_OK) return st;

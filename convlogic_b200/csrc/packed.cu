@@ -13,6 +13,7 @@
 #include "clb_common.cuh"
 #include "clb_slab.cuh"
 
+#include <algorithm>
 #include <type_traits>
 
 namespace clb {
@@ -612,6 +613,130 @@ __global__ void __launch_bounds__(256, 3) group_popcount_kernel(const uint8_t *_
             counts[s * k + cls] = c;
         else if (c)
             atomicAdd(counts + s * k + cls, c);
+    }
+}
+
+constexpr int kTreeCountBlocks = 2; // per SM (655360 trees, 8192 samples: 481 us; three 500, four, which spill, 539)
+
+// The last fused layers and the class sums in one pass: the trees' outputs go into bit-sliced counters as they are produced and are
+// neither written nor read again.  Block (2^LG units, part of a class, class): 256 / 2^LG walkers of 2^LG lanes, a unit of 128
+// samples each, take every 256 / 2^LG-th tree of the part.  The lowest four planes are in registers and the rest, into which sixteen
+// trees carry at most once, in shared memory; then the walkers' counters are added plane by plane.
+// Bound by the L2, which the gathered rows come from: 655360 trees of eight rows, 8192 samples 481 us, where the trees alone took 503 and
+// the class sums another 117 for the 671 MB of outputs.  The next tree's row numbers are fetched a tree ahead; its rows as well: 564.
+template <int M, int LG>
+__global__ void __launch_bounds__(256, kTreeCountBlocks) packed_tree_count_kernel(const uint4 *__restrict__ x, const int32_t *__restrict__ leaf,
+                                                                                  const uint8_t *__restrict__ ops, int *__restrict__ counts, long long S,
+                                                                                  unsigned units, unsigned u_lo, unsigned u_n, long long B, int k, int planes)
+{
+    constexpr int L = 1 << M, G = L - 1, WALK = 256 >> LG;
+    extern __shared__ uint4 plane[]; // [planes][256]
+    const int lane = threadIdx.x & ((1 << LG) - 1), walker = threadIdx.x >> LG;
+    const int cls = blockIdx.z, part = blockIdx.y, parts = gridDim.y;
+    const int hi = (int)(cls * S + S * (part + 1) / parts);
+    int t = (int)(cls * S + S * part / parts) + walker;
+    const unsigned first = blockIdx.x << LG;
+    const uint4 *xu = x + (u_lo + min(first + lane, u_n - 1)); // lanes behind the last unit count it, too, and keep it to themselves
+    unsigned n[4][4] = {};
+    for (int p = 4; p < planes; ++p) plane[p * 256 + threadIdx.x] = make_uint4(0u, 0u, 0u, 0u);
+    int next[L]; // the rows of the next tree
+    auto fetch = [&](int j) {
+        if (j < hi)
+#pragma unroll
+            for (int q = 0; q < L / 4; ++q) {
+                const int4 r = __ldg(reinterpret_cast<const int4 *>(leaf) + (long long)j * (L / 4) + q);
+                next[4 * q] = r.x, next[4 * q + 1] = r.y, next[4 * q + 2] = r.z, next[4 * q + 3] = r.w;
+            }
+    };
+    fetch(t);
+    auto tree = [&](unsigned (&out)[4]) { // of tree t, none behind the last
+        unsigned v[L][4];
+        const int j = t;
+        t += WALK;
+        if (j < hi) {
+#pragma unroll
+            for (int q = 0; q < L; ++q) {
+                const uint4 r = __ldg(xu + (unsigned)next[q] * units);
+                v[q][0] = r.x, v[q][1] = r.y, v[q][2] = r.z, v[q][3] = r.w;
+            }
+            fetch(t);
+            int g = 0;
+#pragma unroll
+            for (int m = L / 2; m >= 1; m /= 2) {
+#pragma unroll
+                for (int p = 0; p < m; ++p) {
+                    const OpMasks<unsigned> o = op_masks<unsigned>(__ldg(ops + (long long)j * G + g + p));
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) v[p][w] = op_apply<unsigned>(o, v[2 * p][w], v[2 * p + 1][w]);
+                }
+                g += m;
+            }
+        }
+#pragma unroll
+        for (int w = 0; w < 4; ++w) out[w] = j < hi ? v[0][w] : 0u;
+    };
+    while (t < hi) {
+        unsigned carry[4] = {};
+#pragma unroll 1
+        for (int q = 0; q < 4 && t < hi; ++q) {
+            unsigned a[4], b[4], two[4];
+            tree(a), tree(b);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) csa(two[w], n[0][w], n[0][w], a[w], b[w]);
+            tree(a), tree(b);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                unsigned also, four;
+                csa(also, n[0][w], n[0][w], a[w], b[w]);
+                csa(four, n[1][w], n[1][w], two[w], also);
+                const unsigned eight = n[2][w] & four;
+                n[2][w] ^= four;
+                carry[w] |= n[3][w] & eight;
+                n[3][w] ^= eight;
+            }
+        }
+        for (int p = 4; p < planes && (carry[0] | carry[1] | carry[2] | carry[3]); ++p) {
+            const uint4 h = plane[p * 256 + threadIdx.x];
+            plane[p * 256 + threadIdx.x] = make_uint4(h.x ^ carry[0], h.y ^ carry[1], h.z ^ carry[2], h.w ^ carry[3]);
+            carry[0] &= h.x, carry[1] &= h.y, carry[2] &= h.z, carry[3] &= h.w;
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+        if (p < planes) plane[p * 256 + threadIdx.x] = make_uint4(n[p][0], n[p][1], n[p][2], n[p][3]);
+    __syncthreads();
+    // a thread per word of 32 samples and EACH of these: bit p of their sums is the parity of what plane p and the carries hold
+    constexpr int WORDS = 4 << LG, EACH = 32 * WORDS / 256, BITS = 9 - LG; // carries stay below WALK = 2^(BITS - 1)
+    const int word = threadIdx.x & (WORDS - 1), s0 = threadIdx.x / WORDS * EACH;
+    if (first + (word >> 2) >= u_n) return;
+    const unsigned *pw = reinterpret_cast<const unsigned *>(plane) + word;
+    int count[EACH] = {};
+    unsigned sum[BITS] = {};
+    for (int p = 0; p < planes + BITS - 1; ++p) {
+        if (p < planes)
+#pragma unroll 8
+            for (int w = 0; w < WALK; ++w) {
+                unsigned carry = pw[p * 1024 + w * WORDS];
+#pragma unroll
+                for (int i = 0; i < BITS; ++i) {
+                    const unsigned c = sum[i] & carry;
+                    sum[i] ^= carry, carry = c;
+                }
+            }
+#pragma unroll
+        for (int i = 0; i < EACH; ++i) count[i] += (int)(sum[0] >> (s0 + i) & 1u) << p;
+#pragma unroll
+        for (int i = 0; i + 1 < BITS; ++i) sum[i] = sum[i + 1];
+        sum[BITS - 1] = 0u;
+    }
+    const long long s = ((long long)(u_lo + first) * 4 + word) * 32 + s0;
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) {
+        if (s + i >= B) break;
+        if (parts == 1)
+            counts[(s + i) * k + cls] = count[i];
+        else if (count[i])
+            atomicAdd(counts + (s + i) * k + cls, count[i]);
     }
 }
 
@@ -1236,6 +1361,16 @@ extern "C" int clb_packed_path(const void *x, const void *rec, const uint8_t *op
     return rows(0u);
 }
 
+// The leaves are gathered from all over the input: when it is larger than about three quarters of the 126 MB L2, the
+// rows are walked in pieces (a range of 16-byte units = a range of samples at a time), so that the piece of the input in
+// use stays cached.  Measured on a 134 MB input: 0.64 ms in one piece, 0.50 in two or four, 0.56 in eight.
+static long long tree_pieces(long long in_dim, long long units)
+{
+    long long pieces = 1;
+    while (in_dim * units * 16 / pieces > (96LL << 20) && units % (pieces * 2) == 0 && units / (pieces * 2) >= 8) pieces *= 2;
+    return pieces;
+}
+
 extern "C" int clb_packed_tree(const void *x, const int32_t *leaf, const uint8_t *ops, void *y, int64_t in_dim, int64_t out_dim, int levels,
                                int64_t words, int bits, void *stream)
 {
@@ -1247,11 +1382,7 @@ extern "C" int clb_packed_tree(const void *x, const int32_t *leaf, const uint8_t
     cudaStream_t st = (cudaStream_t)stream;
     if (rowbytes % 16 == 0 && aligned_to(x, 16) && aligned_to(y, 16)) {
         const long long units = rowbytes / 16;
-        // The leaves are gathered from all over the input: when it is larger than about three quarters of the 126 MB L2, the
-        // rows are walked in pieces (a range of units = a range of samples at a time), so that the piece of the input in
-        // use stays cached.  Measured on a 134 MB input: 0.64 ms in one piece, 0.50 in two or four, 0.56 in eight.
-        long long pieces = 1;
-        while (in_dim * rowbytes / pieces > (96LL << 20) && units % (pieces * 2) == 0 && units / (pieces * 2) >= 8) pieces *= 2;
+        const long long pieces = tree_pieces(in_dim, units);
         const long long u_n = units / pieces;
         const int grid = flat_grid(out_dim * u_n, 256);
         for (long long pc = 0; pc < pieces; ++pc) {
@@ -1278,6 +1409,43 @@ extern "C" int clb_packed_tree(const void *x, const int32_t *leaf, const uint8_t
         return CLB_ERR_SHAPE; // rows of 64-bit words only
     }
     return check_launch();
+}
+
+int clb_packed_tree_count(const void *x, const int32_t *leaf, const uint8_t *ops, int32_t *counts, int64_t in_dim, int64_t out_dim, int levels, int64_t U,
+                          int64_t B, int k, cudaStream_t st)
+{
+    if (k <= 0 || k > 65535 || out_dim % k || out_dim > 0x7fffff00LL || out_dim <= 0 || B <= 0 || in_dim * U >= 0xffffffffLL) return CLB_ERR_SHAPE;
+    if ((levels != 2 && levels != 3) || !aligned_to(x, 16) || !aligned_to(leaf, 16)) return CLB_ERR_SHAPE;
+    const long long pieces = tree_pieces(in_dim, U), u_n = U / pieces, S = out_dim / k;
+    // lanes of a walker: as many as leave fewest idle, of two the more
+    int lg = 5;
+    for (int g = 4; g >= 3; --g)
+        if (((u_n + (1 << g) - 1) >> g << g) < ((u_n + (1 << lg) - 1) >> lg << lg)) lg = g;
+    const long long chunks = (u_n + (1 << lg) - 1) >> lg, walkers = 256 >> lg;
+    // Adding up the walkers' counters takes 10 us or so and idle lanes read rows, too; the outputs of small layers stay in the L2 anyway.
+    // us in one pass / apart: 10.5 MB of outputs 22 / 20, 21 MB 28 / 30 and 27 / 33, 42 MB 43 / 46, 84 MB 72 / 84, 671 MB 483 / 622;
+    // 34 units on 40 lanes 36 / 33, 11 on 16 (115 MB) 127 / 122.
+    if (out_dim * U * 16 < (20LL << 20) || 16 * u_n < 15 * (chunks << lg)) return CLB_ERR_SHAPE;
+    // one wave of blocks, of at least 16 trees per walker, and no more than 2^12 - 1
+    long long parts = (long long)kTreeCountBlocks * sm_count() / (chunks * k);
+    parts = std::min(parts, S / (16 * walkers));
+    parts = std::max(parts, S / (walkers * 4000) + 1);
+    if (parts > 65535 || chunks > 0x7fffffffLL) return CLB_ERR_SHAPE;
+    const long long most = (S / parts + 1 + walkers - 1) / walkers;
+    int planes = 4;
+    while (most >> planes) ++planes;
+    if (parts > 1 && cudaMemsetAsync(counts, 0, (size_t)B * k * sizeof(int32_t), st) != cudaSuccess) return check_launch(0);
+    const dim3 grid((unsigned)chunks, (unsigned)parts, (unsigned)k);
+    auto go = [&](auto kern) {
+        for (long long pc = 0; pc < pieces; ++pc)
+            CLB_TRACED("packed_tree_count_kernel", st,
+                       kern<<<grid, 256, planes * 4096, st>>>((const uint4 *)x, leaf, ops, counts, S, (unsigned)U, (unsigned)(pc * u_n), (unsigned)u_n, B, k, planes));
+    };
+    if (levels == 2)
+        lg == 5 ? go(packed_tree_count_kernel<2, 5>) : lg == 4 ? go(packed_tree_count_kernel<2, 4>) : go(packed_tree_count_kernel<2, 3>);
+    else
+        lg == 5 ? go(packed_tree_count_kernel<3, 5>) : lg == 4 ? go(packed_tree_count_kernel<3, 4>) : go(packed_tree_count_kernel<3, 3>);
+    return check_launch((int)pieces);
 }
 
 // Rows of rowbytes bytes of which B samples count (whatever the bits behind them).
