@@ -13,8 +13,9 @@
 //     indexed branch that a warp takes together;
 //   * eight warps per scheduler at 64 registers a thread, one buffer per block, the copies of one block
 //     running while the SM's others compute (two buffers and half the blocks measured 5 to 30 % slower), and blocks as small as a
-//     slab or, for small images, a warp or two, so that few threads wait at an item's two barriers (k = 1024, 8192 samples, us with
-//     blocks of 256, 256, 128 threads / of 64, 64, 32: 16x16 images 448 / 378, 8x8 479 / 433, 4x4 252 / 240);
+//     slab or, for small images, a warp, so that few threads wait at an item's two barriers (k = 1024, 8192 samples, us with
+//     blocks of 256, 256, 128 threads / of 64, 32, 32: 16x16 images 448 / 378, 8x8 479 / 430, 4x4 252 / 237; two warps for 8x8: 420, but
+//     with 100 samples, a block's only slab, 24 against 17);
 //   * the tap records (offsets, gate codes) are laid out once per network and arrive two items ahead, in an order in which
 //     neighbours share an input channel (clb_slab3_order), whose plane then stays in the tile: half of the copies, 443, 464, 521, 275 us for
 //     the four blocks in the channels' own order, 411, 452, 483, 254 in that one.
@@ -34,7 +35,7 @@ namespace slab {
 
 template <int S> struct Geo {
     static constexpr int H2 = S / 2, I = H2 * H2;                // pooled side, outputs (threads) per slab
-    static constexpr int THREADS = S == 32 ? 256 : S == 4 ? 32 : 64;
+    static constexpr int THREADS = S == 32 ? 256 : S == 16 ? 64 : 32;
     static constexpr int UB = THREADS / I;                       // slabs of a block
     static constexpr int PITCH = S == 8 ? 10 : S + 1;            // units of a padded row
     static constexpr int SLAB = S == 4 ? 28 : (S + 1) * PITCH;   // units from one slab to the next
@@ -148,7 +149,7 @@ __global__ void __launch_bounds__(Geo<S>::THREADS, 1024 / Geo<S>::THREADS)
         if (!R.all_in_tile) return;
         const int u0 = ug * G::UB, n = (s.U - u0) * G::HW - tid; // units from this thread's first to the end
         const int which = fresh ? R.planes : (int)R.fresh;
-#pragma unroll 1
+#pragma unroll
         for (int slot = 0; slot < 2; ++slot) {
             if (!(which >> slot & 1)) continue;
             const uint4 *src = x + ((size_t)R.ch[slot] * s.U + u0) * G::HW + tid;
