@@ -121,3 +121,22 @@ def test_large_packed_layers_take_the_paths_by_themselves():
     _lib.trace(False)
     assert "packed_path_kernel" in names, names
     assert torch.equal(y.rows(), _lib.native().packed_logic(x.rows(), layer.indices_0, layer.indices_1, layer._gate_ids()))
+
+
+@pytest.mark.parametrize("width,batch", [(300, 100), (30000, 2000)])
+def test_packed_layers_need_no_consumer_lists(width, batch):
+    """A deployed layer without the lists, which belong to the backward pass; with one of them; and with them."""
+    import convlogic_b200 as cb
+
+    torch.manual_seed(width)
+    layer = cb.LogicLayer(width, width).cuda().eval()
+    layer.weights.data.normal_()
+    x = cb.PackBitsTensor(torch.rand(batch, width, device="cuda") < 0.5, 32)
+    start, cons = layer.given_x_indices_of_y_start, layer.given_x_indices_of_y
+    del layer.given_x_indices_of_y_start
+    without_start = layer(x).rows()
+    del layer.given_x_indices_of_y
+    without = layer(x).rows()
+    layer.register_buffer("given_x_indices_of_y_start", start)
+    layer.register_buffer("given_x_indices_of_y", cons)
+    assert torch.equal(without, layer(x).rows()) and torch.equal(without, without_start)
