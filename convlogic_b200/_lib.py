@@ -83,6 +83,9 @@ _SIGNATURES = {
     "clb_packed_logic": ([_vp] * 5 + [_i64] * 3 + [_i, _vp], _i),
     "clb_packed_path_pays": ([_i64] * 3 + [_i], _i),
     "clb_packed_path": ([_vp] * 4 + [_i64] * 3 + [_i, _vp], _i),
+    "clb_packed_order_scratch_bytes": ([_i64] * 2, _sz),
+    "clb_packed_order": ([_vp] * 4 + [_sz] + [_i64] * 2 + [_vp], _i),
+    "clb_packed_walk": ([_vp] * 6 + [_i64] * 3 + [_i, _vp], _i),
     "clb_group_popcount": ([_vp, _vp, _i64, _i64, _i, _i, _i, _vp], _i),
     "clb_packed_convtree": ([_vp] * 4 + [_i] * 10 + [_i64, _i, _vp], _i),
     "clb_packed_tree": ([_vp, _vp, _vp, _vp, _i64, _i64, _i, _i64, _i, _vp], _i),

@@ -352,26 +352,77 @@ __global__ void __launch_bounds__(256) packed_logic_kernel(const V *__restrict__
 
 constexpr int kPathBlocks = 6; // packed_path_kernel: resident per SM
 
-// The same layer walked as paths (logic_path.cu: the next neuron reads what the last one read second): one gathered row per neuron
-// instead of two.  A group of 2^LG lanes owns a range of positions and a stretch of R units per lane.  What bound it first was the issue
+// An order of the neurons in which the next one reads what the last one read second.  The half-edges of a feature (2 * j + side of
+// neuron j) are paired up as they come, one waiting in `slot` for the next; one pair in 128 is left apart, so that trails stay short
+// enough to be walked by one thread.  Each half-edge has at most one partner, and that is mutual, so that every neuron is laid out once,
+// whatever the connections.  The order may differ between runs; the outputs are bits.
+__global__ void __launch_bounds__(256) packed_pair_kernel(const int64_t *__restrict__ ia, const int64_t *__restrict__ ib, int32_t *slot, int32_t *link,
+                                                          int in_dim, int out_dim)
+{
+    const int h = blockIdx.x * 256 + threadIdx.x;
+    if (h >= 2 * out_dim) return;
+    const int64_t f = (h & 1 ? ib : ia)[h >> 1];
+    if (f < 0 || f >= in_dim) return;
+    for (int tries = 0; tries < 256; ++tries) { // (one that never gets through stays alone)
+        const int waiting = atomicCAS(slot + f, -1, h);
+        if (waiting < 0) return;
+        if (atomicCAS(slot + f, waiting, -1) != waiting) continue;
+        unsigned e = (unsigned)min(h, waiting);
+        e *= 0x9E3779B1u, e ^= e >> 15, e *= 0x85EBCA77u, e ^= e >> 13;
+        if ((waiting >> 1) != (h >> 1) && e % 128 != 0) link[waiting] = h, link[h] = waiting; // (a neuron fed twice by f is no link)
+        return;
+    }
+}
+
+// A thread per half-edge that is the end of a trail; of a trail's two ends the one with the smaller number lays it out.
+__global__ void __launch_bounds__(128) packed_walk_kernel(const int32_t *__restrict__ link, int32_t *__restrict__ order, uint8_t *__restrict__ placed,
+                                                          int32_t *__restrict__ count, int out_dim)
+{
+    const int h = blockIdx.x * 128 + threadIdx.x;
+    if (h >= 2 * out_dim || link[h] >= 0) return;
+    int n = 1, cur = h;
+    for (int next; n < out_dim && (next = __ldg(link + (cur ^ 1))) >= 0; ++n) cur = next;
+    if (h > (cur ^ 1)) return;
+    const int p = atomicAdd(count, n);
+    cur = h;
+    for (int i = 0; i < n; ++i) {
+        order[p + i] = cur, placed[cur >> 1] = 1;
+        cur = __ldg(link + (cur ^ 1));
+    }
+}
+
+// neurons that no trail end reaches (closed trails) stand alone
+__global__ void __launch_bounds__(256) packed_rest_kernel(int32_t *__restrict__ order, const uint8_t *__restrict__ placed, int32_t *__restrict__ count, int out_dim)
+{
+    const int j = blockIdx.x * 256 + threadIdx.x;
+    if (j < out_dim && !placed[j]) order[atomicAdd(count, 1)] = 2 * j;
+}
+
+// The same layer walked in such an order (or in that of logic_path.cu's records): one gathered row per neuron instead of two.
+// A group of 2^LG lanes owns a range of positions and a stretch of R units per lane.  What bound it first was the issue
 // of integer instructions (171 per neuron and stretch of five words): offsets within a row are constants now, which lanes are inside
 // it is found once, and a gate's four masks come from a table; then the bytes in flight, for which many warps with one row each beat
 // fewer with two to four (us for one layer, x in the L2 as the layer before leaves it, two rows per neuron / this with four blocks and two
 // rows / with six and one: 3072 -> 64000 neurons, 1252 bytes 37 / 23 / 23, 64000 -> 64000 45 / 41 / 37, 128000 x 2500 171 / 141 / 128).
+// step 1: an order, the connections from ia and ib as they are now (a lane each for as many positions as there are lanes, fetched as many
+// positions ahead, then through shared memory); step 4: records, with their own.
 template <typename V, int R, int LG>
-__global__ void __launch_bounds__(256, kPathBlocks) packed_path_kernel(const V *__restrict__ x, const int4 *__restrict__ rec, const uint8_t *__restrict__ ops,
+__global__ void __launch_bounds__(256, kPathBlocks) packed_path_kernel(const V *__restrict__ x, const int32_t *__restrict__ order, int step,
+                                                             const int64_t *__restrict__ ia, const int64_t *__restrict__ ib, const uint8_t *__restrict__ ops,
                                                              V *__restrict__ y, int n, int units, int cols, int ranges)
 {
     constexpr int N = Words<V>::N, G = 1 << LG;
     __shared__ uint4 masks[32]; // of gate op, and from 16 on of the gate with its inputs swapped
+    __shared__ int4 table[256];
     if (threadIdx.x < 32) {
         const int op = threadIdx.x & 15, o = threadIdx.x < 16 ? op : (op & 9) | (op & 2) << 1 | (op & 4) >> 1;
         masks[threadIdx.x] = make_uint4(o & 1 ? ~0u : 0u, o & 2 ? ~0u : 0u, o & 4 ? ~0u : 0u, o & 8 ? ~0u : 0u);
     }
     __syncthreads();
-    const int unit = (int)((blockIdx.x * 256u + threadIdx.x) >> LG), range = unit / cols, col = unit - range * cols;
-    const int turns = (n + ranges - 1) / ranges, p0 = range * turns, p1 = min(n, p0 + turns), u0 = col * G * R + (threadIdx.x & (G - 1));
-    if (p0 >= p1 || u0 >= units) return;
+    const int unit = (int)((blockIdx.x * 256u + threadIdx.x) >> LG), range = unit / cols, col = unit - range * cols, lane = threadIdx.x & (G - 1);
+    const unsigned group = LG == 5 ? ~0u : ((1u << G % 32) - 1) << (threadIdx.x & 31 & ~(G - 1)); // its lanes make the same turns
+    const int turns = (n + ranges - 1) / ranges, p0 = range * turns, p1 = min(n, p0 + turns), u0 = col * G * R + lane;
+    if (p0 >= p1) return;
     x += u0, y += u0;
     bool in[R];
 #pragma unroll
@@ -383,29 +434,49 @@ __global__ void __launch_bounds__(256, kPathBlocks) packed_path_kernel(const V *
         for (int r = 0; r < R; ++r)
             if (in[r]) row[r] = load_words(p + r * G);
     };
-    int4 next = __ldg(rec + p0);
-    load(a, next.y);
-    next.w |= 1; // (linked: the row entered through is there)
-    for (int p = p0; p < p1; ++p) {
-        const int4 t = next;
-        Words<V> b[R];
-        load(b, t.z);
-        const int op = __ldg(ops + (t.x >> 1));
-        if (p + 1 < p1) next = __ldg(rec + p + 1);
-        if (!(t.w & 1)) load(a, t.y);
-        const uint4 m = masks[op & 15 | (t.x & 1) << 4];
-        V *row = y + (size_t)(t.x >> 1) * units;
+    auto code_at = [&](int p) { return p < p1 ? __ldg(order + (size_t)p * step) : -1; };
+    // features entered from and left through
+    auto features = [&](int code, int p, int &u, int &v) {
+        u = v = 0;
+        if (code < 0) return;
+        if (step == 1) {
+            const int fa = (int)__ldg(ia + (code >> 1)), fb = (int)__ldg(ib + (code >> 1));
+            u = code & 1 ? fb : fa, v = code & 1 ? fa : fb;
+        } else {
+            u = __ldg(order + (size_t)p * 4 + 1), v = __ldg(order + (size_t)p * 4 + 2);
+        }
+    };
+    int code = code_at(p0 + lane), next = code_at(p0 + G + lane), u, v;
+    features(code, p0 + lane, u, v);
+    for (int base = p0; base < p1; base += G) {
+        int before = __shfl_up_sync(group, v, 1, G);
+        if (lane == 0) before = base > p0 ? table[threadIdx.x + G - 1].z : -1;
+        __syncwarp(group); // the positions before are done with
+        table[threadIdx.x] = make_int4(code, u == before ? -1 : u, v, 0); // (-1: the row entered through is there)
+        __syncwarp(group);
+        code = next;
+        features(code, base + G + lane, u, v);
+        next = code_at(base + 2 * G + lane);
+        for (int i = 0; i < min(G, p1 - base); ++i) {
+            const int4 t = table[(threadIdx.x & ~(G - 1)) + i];
+            Words<V> b[R];
+            load(b, t.z);
+            const int op = __ldg(ops + (t.x >> 1)) & 15;
+            if (t.y >= 0) load(a, t.y);
+            const uint4 k = masks[op | (t.x & 1) << 4];
+            V *row = y + (size_t)(t.x >> 1) * units;
 #pragma unroll
-        for (int r = 0; r < R; ++r) {
-            V v;
-            unsigned *w = reinterpret_cast<unsigned *>(&v);
+            for (int r = 0; r < R; ++r) {
+                V o;
+                unsigned *w = reinterpret_cast<unsigned *>(&o);
 #pragma unroll
-            for (int i = 0; i < N; ++i) {
-                const unsigned va = a[r].w[i], vb = b[r].w[i], r1 = (vb & m.x) | (~vb & m.y), r0 = (vb & m.z) | (~vb & m.w);
-                w[i] = (va & r1) | (~va & r0);
+                for (int q = 0; q < N; ++q) {
+                    const unsigned va = a[r].w[q], vb = b[r].w[q], r1 = (vb & k.x) | (~vb & k.y), r0 = (vb & k.z) | (~vb & k.w);
+                    w[q] = (va & r1) | (~va & r0);
+                }
+                if (in[r]) row[r * G] = o;
+                a[r] = b[r];
             }
-            if (in[r]) row[r * G] = v;
-            a[r] = b[r];
         }
     }
 }
@@ -1313,13 +1384,39 @@ extern "C" int clb_packed_path_pays(int64_t in_dim, int64_t out_dim, int64_t wor
     return rowbytes % 4 == 0 && out_dim * rowbytes >= (6LL << 20);
 }
 
-extern "C" int clb_packed_path(const void *x, const void *rec, const uint8_t *ops, void *y, int64_t in_dim, int64_t out_dim, int64_t words, int bits,
-                               void *stream)
+extern "C" size_t clb_packed_order_scratch_bytes(int64_t in_dim, int64_t out_dim)
 {
-    if (!x || !rec || !ops || !y || in_dim <= 0 || out_dim < 0 || words < 0 || !bits_ok(bits)) return CLB_ERR_ARG;
+    if (in_dim <= 0 || out_dim <= 0 || in_dim > 0x3fffffff || out_dim > 0x3fffffff) return 0;
+    return 4 * (size_t)in_dim + 9 * (size_t)out_dim + 4;
+}
+
+extern "C" int clb_packed_order(const int64_t *a, const int64_t *b, int32_t *order, void *scratch, size_t scratch_bytes, int64_t in_dim, int64_t out_dim,
+                                void *stream)
+{
+    if (!a || !b || !order || !scratch || in_dim <= 0 || out_dim <= 0) return CLB_ERR_ARG;
+    if (in_dim > 0x3fffffff || out_dim > 0x3fffffff) return CLB_ERR_SHAPE;
+    if (scratch_bytes < clb_packed_order_scratch_bytes(in_dim, out_dim) || !aligned_to(scratch, 4)) return CLB_ERR_SCRATCH;
+    cudaStream_t st = (cudaStream_t)stream;
+    int32_t *slot = (int32_t *)scratch, *link = slot + in_dim, *count = link + 2 * out_dim;
+    uint8_t *placed = (uint8_t *)(count + 1);
+    const int in = (int)in_dim, out = (int)out_dim;
+    if (cudaMemsetAsync(slot, 0xff, 4 * (size_t)in_dim + 8 * (size_t)out_dim, st) != cudaSuccess ||
+        cudaMemsetAsync(count, 0, 4 + (size_t)out_dim, st) != cudaSuccess)
+        return check_launch(0);
+    packed_pair_kernel<<<(unsigned)((2 * out_dim + 255) / 256), 256, 0, st>>>(a, b, slot, link, in, out);
+    packed_walk_kernel<<<(unsigned)((2 * out_dim + 127) / 128), 128, 0, st>>>(link, order, placed, count, out);
+    packed_rest_kernel<<<(unsigned)((out_dim + 255) / 256), 256, 0, st>>>(order, placed, count, out);
+    return check_launch(3);
+}
+
+// order: step 1 an order (with a and b), 4 records
+static int packed_path(const void *x, const void *rec, int step, const int64_t *a, const int64_t *b, const uint8_t *ops, void *y, int64_t in_dim,
+                       int64_t out_dim, int64_t words, int bits, void *stream)
+{
+    if (!x || !rec || (step == 1 && (!a || !b)) || !ops || !y || in_dim <= 0 || out_dim < 0 || words < 0 || !bits_ok(bits)) return CLB_ERR_ARG;
     const long long rowbytes = words * (bits / 8);
     if (out_dim == 0 || rowbytes == 0) return CLB_OK;
-    if (rowbytes % 4 || rowbytes > 0x7fffffffLL || in_dim > 0x3fffffff || out_dim > 0x3fffffff || !aligned_to(rec, 16) || !aligned_to(x, 4) || !aligned_to(y, 4))
+    if (rowbytes % 4 || rowbytes > 0x7fffffffLL || in_dim > 0x3fffffff || out_dim > 0x3fffffff || !aligned_to(rec, 4 * (size_t)step) || !aligned_to(x, 4) || !aligned_to(y, 4))
         return CLB_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
     auto go = [&](auto unit, auto per, auto lanes) {
@@ -1331,7 +1428,7 @@ extern "C" int clb_packed_path(const void *x, const void *rec, const uint8_t *op
         if (ranges < 1) ranges = 1;
         if (((ranges * cols) << LG) + 255 > 0x7fffffffLL) return (int)CLB_ERR_SHAPE;
         CLB_TRACED("packed_path_kernel", st,
-                   packed_path_kernel<V, R, LG><<<(unsigned)(((ranges * cols << LG) + 255) / 256), 256, 0, st>>>((const V *)x, (const int4 *)rec, ops, (V *)y,
+                   packed_path_kernel<V, R, LG><<<(unsigned)(((ranges * cols << LG) + 255) / 256), 256, 0, st>>>((const V *)x, (const int32_t *)rec, step, a, b, ops, (V *)y,
                                                                                                               (int)out_dim, (int)units, (int)cols, (int)ranges));
         return check_launch();
     };
@@ -1359,6 +1456,18 @@ extern "C" int clb_packed_path(const void *x, const void *rec, const uint8_t *op
     if (rowbytes % 16 == 0 && aligned_to(x, 16) && aligned_to(y, 16)) return rows(uint4{});
     if (rowbytes % 8 == 0 && aligned_to(x, 8) && aligned_to(y, 8)) return rows(uint2{});
     return rows(0u);
+}
+
+extern "C" int clb_packed_path(const void *x, const void *rec, const uint8_t *ops, void *y, int64_t in_dim, int64_t out_dim, int64_t words, int bits,
+                               void *stream)
+{
+    return packed_path(x, rec, 4, nullptr, nullptr, ops, y, in_dim, out_dim, words, bits, stream);
+}
+
+extern "C" int clb_packed_walk(const void *x, const int64_t *a, const int64_t *b, const int32_t *order, const uint8_t *ops, void *y, int64_t in_dim,
+                               int64_t out_dim, int64_t words, int bits, void *stream)
+{
+    return packed_path(x, order, 1, a, b, ops, y, in_dim, out_dim, words, bits, stream);
 }
 
 // The leaves are gathered from all over the input: when it is larger than about three quarters of the 126 MB L2, the

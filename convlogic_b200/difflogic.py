@@ -104,8 +104,8 @@ class LogicLayer(torch.nn.Module):
         t = x.rows()
         t = t.reshape(-1, t.shape[-1])
         assert t.shape[0] == self.in_dim, (tuple(t.shape), self.in_dim)
-        buf = self._buffers   # (a deployed layer may have dropped its consumer lists: they belong to the backward pass)
-        y = native().packed_logic(t, buf["indices_0"], buf["indices_1"], self._gate_ids(), buf.get("given_x_indices_of_y_start"), buf.get("given_x_indices_of_y"))
+        a, b = self._buffers["indices_0"], self._buffers["indices_1"]
+        y = native().packed_logic(t, a, b, self._gate_ids(), a)   # (the order of a large layer is kept on `a`)
         return PackBitsTensor.from_packed(y, x.pad_len)
 
     def _gate_ids(self):

@@ -303,6 +303,14 @@ int clb_packed_logic(const void *x, const int64_t *a, const int64_t *b, const ui
 int clb_packed_path_pays(int64_t in_dim, int64_t out_dim, int64_t words, int bits);
 int clb_packed_path(const void *x, const void *rec, const uint8_t *ops, void *y, int64_t in_dim, int64_t out_dim, int64_t words, int bits,
                     void *stream);
+/* The same in an order of the neurons alone, laid out once from the connections (scratch: clb_packed_order_scratch_bytes, 4-byte aligned): order
+ * int32 [out], 2 * j + (1: entered through its second input), any permutation of the neurons.  clb_packed_walk reads the connections themselves on
+ * every call, so that an order of others makes it slower and never wrong. */
+size_t clb_packed_order_scratch_bytes(int64_t in_dim, int64_t out_dim);
+int clb_packed_order(const int64_t *a, const int64_t *b, int32_t *order, void *scratch, size_t scratch_bytes, int64_t in_dim, int64_t out_dim,
+                     void *stream);
+int clb_packed_walk(const void *x, const int64_t *a, const int64_t *b, const int32_t *order, const uint8_t *ops, void *y, int64_t in_dim,
+                    int64_t out_dim, int64_t words, int bits, void *stream);
 /* Replaces difflogic_cuda.groupbitsum (difflogic.cpp:22-33; difflogic_kernel.cu:418-482).
  * x [F,words] -> counts int32 [B,k], B = words*bits - pad_len; F must be divisible by k
  * (CLB_ERR_SHAPE otherwise, the reference's ValueError). */

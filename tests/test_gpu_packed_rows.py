@@ -140,3 +140,107 @@ def test_packed_layers_need_no_consumer_lists(width, batch):
     layer.register_buffer("given_x_indices_of_y_start", start)
     layer.register_buffer("given_x_indices_of_y", cons)
     assert torch.equal(without, layer(x).rows()) and torch.equal(without, without_start)
+
+
+def _walk(x, a, b, ops, order):
+    import ctypes as C
+
+    from convlogic_b200 import _lib
+
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    y = torch.empty(a.numel(), x.shape[1], dtype=x.dtype, device="cuda")
+    assert _lib.lib().clb_packed_walk(ptr(x), ptr(a), ptr(b), ptr(order), ptr(ops), ptr(y), x.shape[0], a.numel(), x.shape[1], x.element_size() * 8,
+                                      C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    return y
+
+
+def _order(a, b, fin):
+    import ctypes as C
+
+    from convlogic_b200 import _lib
+
+    ptr, lib = lambda t: C.c_void_p(t.data_ptr()), _lib.lib()
+    n = lib.clb_packed_order_scratch_bytes(fin, a.numel())
+    scratch, order = torch.empty(n, dtype=torch.uint8, device="cuda"), torch.full((a.numel(),), -1, dtype=torch.int32, device="cuda")
+    assert lib.clb_packed_order(ptr(a), ptr(b), ptr(order), ptr(scratch), n, fin, a.numel(), C.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0
+    return order
+
+
+@pytest.mark.parametrize("bits,words", [(8, 4), (16, 34), (32, 31), (32, 161), (64, 1), (64, 17), (64, 41), (64, 129), (32, 400)])
+@pytest.mark.parametrize("kind,fin,fout", [("twice", 1, 1), ("twice", 300, 300), ("twice", 20000, 20000), ("any", 50, 1000), ("any", 700, 400), ("pairs", 600, 600),
+                                           ("one", 3, 5000)])
+def test_packed_layer_in_any_order(kind, fin, fout, bits, words):
+    """The order of the layer's own connections, and one that has nothing to do with them: every neuron once, the same bits."""
+    from convlogic_b200 import _lib
+
+    g = torch.Generator().manual_seed(words + fin)
+    i = torch.arange(fout)
+    if kind == "twice":
+        c = torch.randperm(2 * fout, generator=g) % fin
+        a, b = c[:fout].contiguous(), c[fout:].contiguous()
+    elif kind == "any":
+        a, b = torch.randint(0, fin, (fout,), generator=g), torch.randint(0, fin, (fout,), generator=g)
+    else:   # closed trails of two neurons; one feature that every neuron reads, some of them twice
+        a, b = (i // 2 * 2 % fin, (i // 2 * 2 + 1) % fin) if kind == "pairs" else (i * 0 + 1, i % fin)
+    a, b, ops = a.cuda(), b.cuda(), torch.randint(0, 16, (fout,), generator=g, dtype=torch.uint8).cuda()
+    x = torch.randint(0, 256, (fin, words * bits // 8), generator=g, dtype=torch.uint8).cuda().view({8: torch.int8, 16: torch.int16, 32: torch.int32, 64: torch.int64}[bits])
+    want = _lib.native().packed_logic(x, a, b, ops)
+    own = _order(a, b, fin)
+    other = (2 * torch.randperm(fout, generator=g) + torch.randint(0, 2, (fout,), generator=g)).int().cuda()
+    for order in (own, other):
+        assert torch.equal((order >> 1).sort().values.cpu(), i.int())
+        assert torch.equal(_walk(x, a, b, ops, order), want)
+    if fout == 20000:   # pairs apart and closed trails aside, the next neuron reads what the last one read second
+        j, second = (own >> 1).long(), (own & 1).bool()
+        entered, left = torch.where(second, b[j], a[j]), torch.where(second, a[j], b[j])
+        assert (entered[1:] == left[:-1]).float().mean() > 0.9
+
+
+def _large(width=30000):
+    import convlogic_b200 as cb
+
+    torch.manual_seed(0)
+    layer = cb.LogicLayer(width, width).cuda().eval()
+    layer.weights.data.normal_()
+    x = cb.PackBitsTensor(torch.rand(2000, width, device="cuda") < 0.5, 32)
+    from convlogic_b200 import _lib
+
+    def want():
+        return _lib.native().packed_logic(x.rows(), layer.indices_0.clone(), layer.indices_1.clone(), layer._gate_ids())
+
+    return layer, x, want
+
+
+def test_large_packed_layers_read_their_connections_on_every_call():
+    """Connections written in ways that leave their version as it is, and in ways that do not."""
+    layer, x, want = _large()
+    assert torch.equal(layer(x).rows(), want())
+    layer.indices_0.data.copy_(layer.indices_0.flip(0))
+    assert torch.equal(layer(x).rows(), want())
+    layer.indices_1.copy_(torch.randint(0, 30000, (30000,), device="cuda"))
+    assert torch.equal(layer(x).rows(), want())
+    with torch.inference_mode():
+        layer.indices_0 = layer.indices_0.clone()
+        assert layer.indices_0.is_inference() and torch.equal(layer(x).rows(), want())
+
+
+def test_large_packed_layers_do_not_read_their_lists():
+    layer, x, want = _large()
+    layer.given_x_indices_of_y.fill_(1 << 40)
+    layer.given_x_indices_of_y_start.fill_(-(1 << 40))
+    assert torch.equal(layer(x).rows(), want())
+
+
+def test_a_captured_packed_layer_follows_its_connections():
+    layer, x, want = _large()
+    layer(x)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = layer(x).rows()
+    for _ in range(2):
+        layer.indices_0.copy_(torch.randint(0, 30000, (30000,), device="cuda"))
+        layer(x)
+        filler = [torch.full((30000,), 1 << 30, dtype=torch.int32, device="cuda") for _ in range(64)]   # (the order's memory is not among it)
+        graph.replay()
+        assert torch.equal(y, want())
+        del filler

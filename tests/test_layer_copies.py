@@ -8,7 +8,7 @@ import pytest
 import torch
 
 
-@pytest.mark.parametrize("kind", ["BlockPlan", "LogicPlan"])
+@pytest.mark.parametrize("kind", ["BlockPlan", "LogicPlan", "PackedOrder"])
 def test_a_buffer_with_a_plan_is_copied_without_it(kind):
     from convlogic_b200 import _lib
 
