@@ -74,6 +74,7 @@ _SIGNATURES = {
     "clb_logic_path": ([_vp] * 8 + [_sz] + [_i64] * 2 + [_vp], _i),
     "clb_logic_path_pays": ([_i64] * 4 + [_i], _i),
     "clb_logic_path_fwd": ([_vp] * 5 + [_i64] * 3 + [_i, _vp], _i),
+    "clb_logic_path_fwd_live": ([_vp] * 8 + [_i64] * 3 + [_i, _vp], _i),
     "clb_logic_path_bwd_scratch_bytes": ([_i64] * 2, _sz),
     "clb_logic_path_bwd": ([_vp] * 10 + [_i64, _vp, _sz] + [_i64] * 3 + [_i, _vp], _i),
     "clb_logic_bwd_w": ([_vp] * 6 + [_i64] * 3 + [_i, _i, _vp], _i),

@@ -106,6 +106,25 @@ __global__ void __launch_bounds__(256) path_open_kernel(const uint8_t *__restric
     if (f < in_dim && !closed[f]) open[atomicAdd(count, 1)] = f;
 }
 
+// What a forward pass walks: the plan's order of the neurons, with the connections as they are now (they may have been written since the
+// plan was laid out, in a way that nothing tells), and the coefficients of the gates.  A thread per position and neuron, in the launch that
+// the coefficients take anyway.
+__global__ void __launch_bounds__(256) logic_path_live_kernel(const int64_t *__restrict__ ia, const int64_t *__restrict__ ib, const int4 *__restrict__ rec,
+                                                              int4 *__restrict__ live, const float *__restrict__ w, float4 *__restrict__ coef, int out_dim, int wmode)
+{
+    const int p = blockIdx.x * 256 + threadIdx.x;
+    if (p >= out_dim) return;
+    const int code = __ldg(&rec[p].x), j = code >> 1, prev = p > 0 ? __ldg(&rec[p - 1].x) : -1;
+    const int a = (int)__ldg(ia + j), b = (int)__ldg(ib + j), u = code & 1 ? b : a;
+    const int before = prev < 0 ? -1 : (int)__ldg((prev & 1 ? ia : ib) + (prev >> 1));
+    live[p] = make_int4(code, u, code & 1 ? a : b, before == u ? kLinked : 0);
+    float v[16], mix[16];
+    load16(w + (size_t)p * 16, v);
+    gate_mixture<float>(v, wmode, mix);
+    const Gate<float> g = gate_from_mixture<float>(mix);
+    coef[p] = make_float4(g.k1, g.ka, g.kb, g.kab);
+}
+
 // Eight lanes own a range of positions and 8 * V * R samples; the ranges of neighbouring groups are the same one, a stretch of samples
 // further on, so that a block reads whole rows.  Every group makes the same number of turns: warps stay whole.
 struct PathUnit {
@@ -362,14 +381,25 @@ extern "C" int clb_logic_path(const int64_t *a, const int64_t *b, const int32_t 
 
 int clb_logic_coef(const float *w, float *coef, int64_t out_dim, int wmode, cudaStream_t st); // logic_bwd.cu
 
-extern "C" int clb_logic_path_fwd(const float *x, const void *rec, const float *w, float *y, float *coef, int64_t in_dim, int64_t out_dim, int64_t B, int wmode,
-                                  void *stream)
+// live: room for the records of this call, or null: those of the plan as they are
+static int path_fwd(const float *x, const int64_t *a, const int64_t *b, const void *rec, void *live, const float *w, float *y, float *coef, int64_t in_dim,
+                    int64_t out_dim, int64_t B, int wmode, void *stream)
 {
-    if (!x || !rec || !w || !y || !coef || in_dim <= 0 || out_dim < 0 || B < 0 || wmode < 0 || wmode > 2) return CLB_ERR_ARG;
+    if (!x || !rec || !w || !y || !coef || (live && (!a || !b)) || in_dim <= 0 || out_dim < 0 || B < 0 || wmode < 0 || wmode > 2) return CLB_ERR_ARG;
     if (out_dim == 0 || B == 0) return CLB_OK;
-    if (in_dim > 0x3fffffff || out_dim > 0x3fffffff || B > 0x3fffffff || !aligned16(coef) || !aligned16(w) || !aligned16(rec)) return CLB_ERR_SHAPE;
+    if (in_dim > 0x3fffffff || out_dim > 0x3fffffff || B > 0x3fffffff || !aligned16(coef) || !aligned16(w) || !aligned16(rec) || !aligned16(live))
+        return CLB_ERR_SHAPE;
     cudaStream_t st = (cudaStream_t)stream;
-    const int rc = clb_logic_coef(w, coef, out_dim, wmode, st);
+    int rc = CLB_OK;
+    if (live) {
+        CLB_TRACED("logic_path_live_kernel", st,
+                   logic_path_live_kernel<<<(unsigned)((out_dim + 255) / 256), 256, 0, st>>>(a, b, (const int4 *)rec, (int4 *)live, w, (float4 *)coef,
+                                                                                             (int)out_dim, wmode));
+        rc = check_launch();
+        rec = live;
+    } else {
+        rc = clb_logic_coef(w, coef, out_dim, wmode, st);
+    }
     if (rc != CLB_OK) return rc;
     const PathCut c = path_cut(out_dim, B, kFwdBlocks);
     auto go = [&](auto kern) {
@@ -382,6 +412,19 @@ extern "C" int clb_logic_path_fwd(const float *x, const void *rec, const float *
     default: c.wide ? go(logic_path_fwd_kernel<1, 8, 2>) : go(logic_path_fwd_kernel<1, 4, 2>); break;
     }
     return check_launch();
+}
+
+extern "C" int clb_logic_path_fwd(const float *x, const void *rec, const float *w, float *y, float *coef, int64_t in_dim, int64_t out_dim, int64_t B, int wmode,
+                                  void *stream)
+{
+    return path_fwd(x, nullptr, nullptr, rec, nullptr, w, y, coef, in_dim, out_dim, B, wmode, stream);
+}
+
+extern "C" int clb_logic_path_fwd_live(const float *x, const int64_t *a, const int64_t *b, const void *rec, void *live, const float *w, float *y, float *coef,
+                                       int64_t in_dim, int64_t out_dim, int64_t B, int wmode, void *stream)
+{
+    if (!live) return CLB_ERR_ARG;
+    return path_fwd(x, a, b, rec, live, w, y, coef, in_dim, out_dim, B, wmode, stream);
 }
 
 extern "C" size_t clb_logic_path_bwd_scratch_bytes(int64_t out_dim, int64_t B)

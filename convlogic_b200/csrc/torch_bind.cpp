@@ -721,7 +721,9 @@ Tensor logic(const Tensor &x, const Tensor &a, const Tensor &b, const Tensor &w_
         if (!coef.defined() && clb_logic_fwd_scratch_bytes(in, out, batch, dt)) coef = alloc({out, 4}, x); // (then not kept)
         int rc = CLB_ERR_SHAPE;
         if (batch && out && plan && plan->path_fwd(batch)) {
-            rc = clb_logic_path_fwd(ptr<float>(x_fm), ptr(plan->rec), ptr<float>(w), ptr<float>(y), ptr<float>(coef), in, out, batch, wmode, cur_stream());
+            const Tensor live = alloc({out, 4}, x, at::kInt); // the order is the plan's, the connections are those of this call
+            rc = clb_logic_path_fwd_live(ptr<float>(x_fm), ptr<int64_t>(a), ptr<int64_t>(b), ptr(plan->rec), ptr(live), ptr<float>(w), ptr<float>(y),
+                                         ptr<float>(coef), in, out, batch, wmode, cur_stream());
             if (rc != CLB_ERR_SHAPE) check(rc);
         }
         if (batch && out && rc == CLB_ERR_SHAPE)

@@ -275,6 +275,10 @@ int clb_logic_path(const int64_t *a, const int64_t *b, const int32_t *start32, c
 int clb_logic_path_pays(int64_t in_dim, int64_t out_dim, int64_t B, int64_t n_open, int what);
 int clb_logic_path_fwd(const float *x, const void *rec, const float *w, float *y, float *coef, int64_t in_dim, int64_t out_dim, int64_t B,
                        int wmode, void *stream);
+/* The same in the order of rec alone: the connections are read from a and b on every call, so that rec of others makes it slower and never wrong.
+ * live: 16 bytes per neuron, 16-byte aligned, needed until the call's work is done. */
+int clb_logic_path_fwd_live(const float *x, const int64_t *a, const int64_t *b, const void *rec, void *live, const float *w, float *y, float *coef,
+                            int64_t in_dim, int64_t out_dim, int64_t B, int wmode, void *stream);
 size_t clb_logic_path_bwd_scratch_bytes(int64_t out_dim, int64_t B);
 int clb_logic_path_bwd(const float *x, const float *w, const float *coef, const float *gy, float *gx, float *gw, const int32_t *start32,
                        const void *entry, const void *rec, const int32_t *open, int64_t n_open, void *scratch, size_t scratch_bytes,

@@ -150,3 +150,44 @@ def test_layers_take_the_path_by_size(width, batch, path):
                       (xd.grad.t(), ops.logic_bwd_x(x, *tables, gy, layer.given_x_indices_of_y_start, layer.given_x_indices_of_y, W_SOFTMAX)),
                       (layer.weights.grad, ops.logic_bwd_w(x, *tables, gy, W_SOFTMAX))):
         assert (got - want).norm() <= 1e-5 * want.norm()
+
+
+@pytest.mark.parametrize("kind,fin,fout,batch", [("twice", 1, 1, 1), ("twice", 300, 300, 66), ("any", 500, 900, 100), ("any", 900, 500, 33), ("pairs", 600, 600, 96),
+                                                 ("trail", 5000, 5000, 40), ("twice", 3001, 3001, 514)])
+def test_forward_in_the_order_of_other_connections(kind, fin, fout, batch):
+    """The order of a plan, its own connections or not, and the connections of the call."""
+    from convlogic_b200 import _lib
+
+    lib = _lib.lib()
+    g = torch.Generator().manual_seed(batch)
+    a, b = _connections(kind, fin, fout)
+    w, x = torch.randn(fout, 16, generator=g), torch.rand(fin, batch, generator=g)
+    want = oracle.logic_layer(x.t().double(), a, b, oracle.gate_probabilities(w.double(), True)).t()
+    other = torch.randint(0, fin, (2, fout), generator=g)
+    a, b, w, x = a.cuda(), b.cuda(), w.cuda(), x.cuda()
+    for p in (_plan(a.cpu(), b.cpu(), fin), _plan(other[0].contiguous(), other[1].contiguous(), fin)):
+        y, coef, live = torch.empty(fout, batch, device="cuda"), torch.empty(fout, 4, device="cuda"), torch.empty_like(p["rec"])
+        assert lib.clb_logic_path_fwd_live(_ptr(x), _ptr(a), _ptr(b), _ptr(p["rec"]), _ptr(live), _ptr(w), _ptr(y), _ptr(coef), fin, fout, batch,
+                                           _lib.W_SOFTMAX, _stream()) == 0
+        assert float((y.cpu().double() - want).abs().max()) <= 1e-5   # outputs in [0, 1], a dozen roundings
+
+
+def test_large_layers_read_their_connections_on_every_call():
+    import convlogic_b200 as cb
+    from convlogic_b200 import ops
+    from convlogic_b200._lib import W_SOFTMAX
+
+    torch.manual_seed(0)
+    layer = cb.LogicLayer(100000, 100000).cuda().train()
+    x = torch.rand(100000, 320, device="cuda")
+    xd = x.t().detach().requires_grad_(True)
+
+    def same():
+        want = ops.logic_fwd(x, layer.indices_0.clone(), layer.indices_1.clone(), layer.weights.detach(), W_SOFTMAX)
+        return float((layer(xd).detach().t() - want).abs().max()) <= 1e-5
+
+    assert same()
+    layer.indices_0.data.copy_(layer.indices_0.flip(0))   # no version tells of this write
+    assert same()
+    layer.indices_1.copy_(layer.indices_1.flip(0))
+    assert same()
