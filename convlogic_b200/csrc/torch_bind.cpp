@@ -542,6 +542,8 @@ struct LogicPlan {
     bool paths = false;
     Tensor rec, open;    // (paths) neurons in the order of paths, features whose gradient a path does not complete; undefined: lists and connections disagree
     int64_t n_open = 0;
+    bool captured = false; // a stream capture reads it: its tables stay with the plan that replaces it, for the graph holds their addresses
+    std::shared_ptr<LogicPlan> held;
     bool path_fwd(int64_t batch) const { return rec.defined() && clb_logic_path_pays(in, out, batch, n_open, 0); }
     bool path_bwd(int64_t batch) const { return rec.defined() && clb_logic_path_pays(in, out, batch, n_open, 1); }
 };
@@ -552,17 +554,21 @@ LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const 
                             bool paths)
 {
     const LogicKey key = logic_key(a, b, start, cons);
-    LogicPlanPtr old = kept<LogicPlan>(start_obj);
+    const LogicPlanPtr last = kept<LogicPlan>(start_obj);
+    const bool capture = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+    LogicPlanPtr old = last;
     if (old && !(old->key == key && old->in == in && old->out == out)) old = nullptr;
+    if (old && capture) old->captured = true;
     if (old && (old->paths || !paths)) return old;
     need_inputs(a, b, start, cons);
     TORCH_CHECK(start.scalar_type() == at::kLong && cons.scalar_type() == at::kLong && start.numel() == in + 1 && cons.numel() == 2 * out,
                 "convlogic_b200: consumer lists must be int64 [in_dim + 1] and [2 * out_dim]");
     if (in > 0x3fffffff || out > 0x3fffffff) return nullptr;
     // inside a stream capture nothing would be laid out before the replay: this call runs the two separate gradient kernels
-    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return old;
+    if (capture) return old;
     auto p = std::make_shared<LogicPlan>();
     p->key = key, p->in = in, p->out = out, p->paths = paths;
+    if (last) p->held = last->captured ? last : last->held;
     Below below(start);
     if (old) {
         p->start32 = old->start32, p->entry = old->entry;

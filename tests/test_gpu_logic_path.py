@@ -191,3 +191,38 @@ def test_large_layers_read_their_connections_on_every_call():
     assert same()
     layer.indices_1.copy_(layer.indices_1.flip(0))
     assert same()
+
+
+@pytest.mark.parametrize("width,batch", [(100000, 320), (3000, 64)])
+def test_a_captured_step_keeps_the_plan_it_reads(width, batch):
+    """Connections written after a capture, a plan of the new ones in the old one's place, its memory asked for by others."""
+    import convlogic_b200 as cb
+
+    torch.manual_seed(0)
+    layer = cb.LogicLayer(width, width).cuda().train()
+    x, gy = torch.rand(batch, width, device="cuda", requires_grad=True), torch.randn(batch, width, device="cuda")
+
+    def step():
+        y = layer(x)
+        return [y.detach(), *torch.autograd.grad(y, [x, layer.weights], gy)]
+
+    with torch.cuda.stream(torch.cuda.Stream()):
+        want = step()
+        step()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = step()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    connections = layer.indices_0.clone()
+    layer.indices_0.copy_(layer.indices_0.flip(0))
+    step()
+    layer.indices_0.copy_(connections)   # what the graph's plan was laid out for
+    step()
+    filler = [torch.full((width * 4,), 1 << 29, dtype=torch.int32, device="cuda") for _ in range(64)]
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(got, want))
+    del filler
