@@ -27,6 +27,7 @@
 namespace clb {
 
 constexpr unsigned kCut = 128; // pairs left apart: one in kCut
+constexpr int kLongest = 64 * kCut; // no trail is longer ((1 - 1 / kCut)^kLongest = 1e-28), unless lists contradict the connections
 constexpr int kFwdBlocks = 4, kBwdBlocks = 2; // resident per SM
 enum { kLinked = 1, kCloses = 2 };
 
@@ -36,34 +37,31 @@ __device__ __forceinline__ bool cut_here(unsigned e)
     return e % kCut == 0;
 }
 
-__global__ void __launch_bounds__(256) path_link_kernel(const int32_t *__restrict__ start, const int2 *__restrict__ entry, int32_t *__restrict__ link, int in_dim)
+// (lists of any values: what lies outside the tables is not followed, and what is listed twice gives a count that tells)
+__global__ void __launch_bounds__(256) path_link_kernel(const int32_t *__restrict__ start, const int2 *__restrict__ entry, int32_t *__restrict__ link, int in_dim,
+                                                        int out_dim)
 {
     const int f = blockIdx.x * 256 + threadIdx.x;
     if (f >= in_dim) return;
-    const int hi = start[f + 1];
-    for (int e = start[f]; e < hi; e += 2) {
-        const int h0 = entry[e].x;
-        if (e + 1 == hi) {
-            link[h0] = -1;
-            break;
-        }
-        const int h1 = entry[e + 1].x;
-        const bool apart = (h0 >> 1) == (h1 >> 1) || cut_here((unsigned)e); // a neuron fed twice by f is no link
-        link[h0] = apart ? -1 : h1, link[h1] = apart ? -1 : h0;
+    const int hi = min(start[f + 1], 2 * out_dim);
+    for (int e = max(start[f], 0); e + 1 < hi; e += 2) { // (the last of an odd number stays apart)
+        const int h0 = entry[e].x, h1 = entry[e + 1].x;
+        if ((unsigned)h0 >= 2u * (unsigned)out_dim || (unsigned)h1 >= 2u * (unsigned)out_dim) continue;
+        if ((h0 >> 1) != (h1 >> 1) && !cut_here((unsigned)e)) link[h0] = h1, link[h1] = h0; // a neuron fed twice by f is no link
     }
 }
 
 // A thread per half-edge that is the end of a trail; of a trail's two ends the one with the smaller number lays it out.
 __global__ void __launch_bounds__(128) path_walk_kernel(const int32_t *__restrict__ link, int32_t *__restrict__ order, uint8_t *__restrict__ placed,
-                                                        int32_t *__restrict__ count, int out_dim)
+                                                        unsigned long long *__restrict__ laid, int out_dim)
 {
     const int h = blockIdx.x * 128 + threadIdx.x;
     if (h >= 2 * out_dim || link[h] >= 0) return;
     int n = 1, cur = h;
-    for (int next; n <= out_dim && (next = __ldg(link + (cur ^ 1))) >= 0; ++n) cur = next;
-    if (h > (cur ^ 1)) return;
-    const int p = atomicAdd(count, n);
-    if (n > out_dim || p + n > out_dim || p < 0) return; // lists that contradict the connections: the count tells
+    for (int next; n <= kLongest && (next = __ldg(link + (cur ^ 1))) >= 0; ++n) cur = next;
+    if (n <= kLongest && h > (cur ^ 1)) return;
+    const unsigned long long p = atomicAdd(laid, n <= kLongest ? (unsigned long long)n : out_dim + 1ull);
+    if (p + n > (unsigned long long)out_dim) return; // a neuron is listed twice, or there is no end: the count tells
     cur = h;
     for (int i = 0; i < n; ++i) {
         order[p + i] = cur, placed[cur >> 1] = i > 0 ? 2 : 1;
@@ -72,12 +70,12 @@ __global__ void __launch_bounds__(128) path_walk_kernel(const int32_t *__restric
 }
 
 // neurons that no trail end reaches stand alone
-__global__ void __launch_bounds__(256) path_rest_kernel(int32_t *__restrict__ order, uint8_t *__restrict__ placed, int32_t *__restrict__ count, int out_dim)
+__global__ void __launch_bounds__(256) path_rest_kernel(int32_t *__restrict__ order, uint8_t *__restrict__ placed, unsigned long long *__restrict__ laid, int out_dim)
 {
     const int j = blockIdx.x * 256 + threadIdx.x;
     if (j >= out_dim || placed[j]) return;
-    const int p = atomicAdd(count, 1);
-    if (p < out_dim) order[p] = 2 * j;
+    const unsigned long long p = atomicAdd(laid, 1ull);
+    if (p < (unsigned long long)out_dim) order[p] = 2 * j;
     placed[j] = 1;
 }
 
@@ -100,10 +98,12 @@ __global__ void __launch_bounds__(256) path_record_kernel(const int64_t *__restr
     rec[p] = make_int4(code, u, v, (linked ? kLinked : 0) | (closes ? kCloses : 0));
 }
 
-__global__ void __launch_bounds__(256) path_open_kernel(const uint8_t *__restrict__ closed, int32_t *__restrict__ open, int32_t *__restrict__ count, int in_dim)
+__global__ void __launch_bounds__(256) path_open_kernel(const uint8_t *__restrict__ closed, int32_t *__restrict__ open, int32_t *__restrict__ count,
+                                                       const unsigned long long *__restrict__ laid, int in_dim)
 {
     const int f = blockIdx.x * 256 + threadIdx.x;
-    if (f < in_dim && !closed[f]) open[atomicAdd(count, 1)] = f;
+    if (f == 0) count[0] = (int)min(*laid, 0x7fffffffull);
+    if (f < in_dim && !closed[f]) open[atomicAdd(count + 1, 1)] = f;
 }
 
 // What a forward pass walks: the plan's order of the neurons, with the connections as they are now (they may have been written since the
@@ -350,7 +350,7 @@ extern "C" int clb_logic_path_pays(int64_t in_dim, int64_t out_dim, int64_t B, i
 extern "C" size_t clb_logic_path_scratch_bytes(int64_t in_dim, int64_t out_dim)
 {
     if (in_dim <= 0 || out_dim <= 0 || in_dim > 0x3fffffff || out_dim > 0x3fffffff) return 0;
-    return 12 * (size_t)out_dim + up16((size_t)out_dim) + (size_t)in_dim;
+    return 16 + 12 * (size_t)out_dim + up16((size_t)out_dim) + (size_t)in_dim;
 }
 
 extern "C" int clb_logic_path(const int64_t *a, const int64_t *b, const int32_t *start32, const void *entry, void *rec, int32_t *open, int32_t *count,
@@ -358,24 +358,26 @@ extern "C" int clb_logic_path(const int64_t *a, const int64_t *b, const int32_t 
 {
     if (!a || !b || !start32 || !entry || !rec || !open || !count || !scratch || in_dim <= 0 || out_dim <= 0) return CLB_ERR_ARG;
     if (in_dim > 0x3fffffff || out_dim > 0x3fffffff || !aligned16(rec)) return CLB_ERR_SHAPE;
-    if (scratch_bytes < clb_logic_path_scratch_bytes(in_dim, out_dim)) return CLB_ERR_SCRATCH;
+    if (scratch_bytes < clb_logic_path_scratch_bytes(in_dim, out_dim) || (reinterpret_cast<uintptr_t>(scratch) & 7)) return CLB_ERR_SCRATCH;
     cudaStream_t st = (cudaStream_t)stream;
-    int32_t *link = (int32_t *)scratch, *order = link + 2 * out_dim;
+    unsigned long long *laid = (unsigned long long *)scratch; // neurons laid out; more than there are where one is listed twice
+    int32_t *link = (int32_t *)scratch + 4, *order = link + 2 * out_dim;
     uint8_t *placed = (uint8_t *)(order + out_dim), *closed = placed + up16((size_t)out_dim);
     const int in = (int)in_dim, out = (int)out_dim;
     const unsigned fin = (unsigned)((in_dim + 255) / 256), fout = (unsigned)((out_dim + 255) / 256);
     cudaError_t e = cudaMemsetAsync(placed, 0, up16((size_t)out_dim) + (size_t)in_dim, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(count, 0, 8, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(laid, 0, 8, st);
     if (e == cudaSuccess) e = cudaMemsetAsync(link, 0xff, 12 * (size_t)out_dim, st); // order too: 2 * j + side of no neuron
     if (e != cudaSuccess) {
         set_last_cuda_error((int)e);
         return CLB_ERR_LAUNCH;
     }
-    path_link_kernel<<<fin, 256, 0, st>>>(start32, (const int2 *)entry, link, in);
-    path_walk_kernel<<<(unsigned)((2 * out_dim + 127) / 128), 128, 0, st>>>(link, order, placed, count, out);
-    path_rest_kernel<<<fout, 256, 0, st>>>(order, placed, count, out);
+    path_link_kernel<<<fin, 256, 0, st>>>(start32, (const int2 *)entry, link, in, out);
+    path_walk_kernel<<<(unsigned)((2 * out_dim + 127) / 128), 128, 0, st>>>(link, order, placed, laid, out);
+    path_rest_kernel<<<fout, 256, 0, st>>>(order, placed, laid, out);
     path_record_kernel<<<fout, 256, 0, st>>>(a, b, start32, order, placed, (int4 *)rec, closed, out);
-    path_open_kernel<<<fin, 256, 0, st>>>(closed, open, count + 1, in);
+    path_open_kernel<<<fin, 256, 0, st>>>(closed, open, count, laid, in);
     return check_launch(5);
 }
 

@@ -226,3 +226,44 @@ def test_a_captured_step_keeps_the_plan_it_reads(width, batch):
     torch.cuda.synchronize()
     assert all(torch.equal(a, b) for a, b in zip(got, want))
     del filler
+
+
+def _layout(a, b, start, entry, fin):
+    from convlogic_b200 import _lib
+
+    fout = a.numel()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    rec, open_, count = torch.empty(fout, 4, **i32), torch.empty(fin, **i32), torch.empty(2, **i32)
+    n = _lib.lib().clb_logic_path_scratch_bytes(fin, fout)
+    scratch = torch.empty(n + 256, dtype=torch.uint8, device="cuda").fill_(77)
+    assert _lib.lib().clb_logic_path(_ptr(a), _ptr(b), _ptr(start), _ptr(entry), _ptr(rec), _ptr(open_), _ptr(count), _ptr(scratch), n, fin, fout, _stream()) == 0
+    assert bool((scratch[n:] == 77).all())
+    return rec, count.tolist()
+
+
+@pytest.mark.parametrize("kind", ["a neuron listed twice", "an end that runs into another trail", "values outside the tables", "starts outside the tables"])
+def test_lists_of_other_connections_are_counted(kind):
+    """What is outside the tables is not followed.  Either every neuron is laid out once, linked only where it does read what the one before reads, or
+    the count is another than the number of neurons."""
+    fin = fout = 40000
+    a, b = _connections("trail", fin, fout)
+    p = _plan(a, b, fin)
+    start, entry = p["start"].clone(), p["entry"].clone()
+    if kind == "a neuron listed twice":
+        entry[2:20000:4, 0] = entry[0:19998:4, 0]
+    elif kind == "an end that runs into another trail":
+        entry[1001, 0] = entry[1003, 0]
+    elif kind == "values outside the tables":
+        entry[0::2, 0], entry[1::4, 0] = 1 << 30, -5
+    else:
+        start[1::2], start[0::2] = 1 << 30, -(1 << 30)
+        start[:2] = 0
+    rec, (laid, _) = _layout(p["a"], p["b"], start, entry, fin)
+    if kind == "an end that runs into another trail":
+        assert laid != fout
+    else:
+        code, linked = rec[:, 0].long(), (rec[1:, 3] & 1).bool()
+        assert laid == fout and torch.equal((code >> 1).sort().values.cpu(), torch.arange(fout))
+        a, b, second = p["a"][code >> 1], p["b"][code >> 1], (code & 1).bool()
+        entered, left = torch.where(second, b, a), torch.where(second, a, b)
+        assert torch.equal(entered[1:][linked], left[:-1][linked])
