@@ -15,6 +15,7 @@
 #include "clb_logic.cuh"
 
 #include <cmath>
+#include <type_traits>
 
 namespace clb {
 
@@ -789,8 +790,17 @@ __global__ void __launch_bounds__(128, 3) logic_tree_bwd_kernel(const float *__r
         float bs[28];
 #pragma unroll
         for (int i = 0; i < 28; ++i) bs[i] = 0.f;
-        for (int bb = 0; bb < B; bb += 32 * V) { // uniform over the warp: the rows' numbers are handed round
-            const int b0 = bb + lane * V;
+        // V = 1: rows found once per tree and numbers of 64 bits (at every trip of 32 samples, in 32 bits, 40960 trees of 131 samples took 142 us,
+        // 120 with the rows alone, now 117)
+        using Index = std::conditional_t<V == 4, int, long long>;
+        const Index samples = B;
+        const float *row[8];
+        if constexpr (V != 4) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) row[k] = x + (long long)__shfl_sync(0xffffffffu, my_leaf, k) * B;
+        }
+        for (Index bb = V == 4 ? 0 : lane; bb < B; bb += 32 * V) { // V = 4: uniform over the warp, the rows' numbers are handed round
+            const Index b0 = V == 4 ? bb + lane * V : bb;
             float a[8][V], dz[V], dg[4][V];
             if constexpr (V == 4) {
                 fetch();
@@ -804,10 +814,7 @@ __global__ void __launch_bounds__(128, 3) logic_tree_bwd_kernel(const float *__r
                 slot = slot + 1 == kTreeStages ? 0 : slot + 1;
             } else {
 #pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    const float *row = x + (long long)__shfl_sync(0xffffffffu, my_leaf, k) * B;
-                    if (b0 < B) vload<float, V>(row + b0, a[k]);
-                }
+                for (int k = 0; k < 8; ++k) vload<float, V>(row[k] + b0, a[k]);
             }
             if (b0 >= B) continue;
             if (HEAD) {
@@ -842,11 +849,11 @@ __global__ void __launch_bounds__(128, 3) logic_tree_bwd_kernel(const float *__r
                     bs[4 * p] = fmaf(d, x0 * x1, bs[4 * p]), bs[4 * p + 1] = fmaf(d, x0, bs[4 * p + 1]);
                     bs[4 * p + 2] = fmaf(d, x1, bs[4 * p + 2]), bs[4 * p + 3] += d;
                 }
-                float *const to = tapgrad + ((long long)(t * 8 + 2 * p) * B + b0);
+                float *const to = tapgrad + ((long long)(t * 8 + 2 * p) * samples + b0);
                 if (ONCE)
                     vstore_once<float, V>(to, ta), vstore_once<float, V>(to + B, tb);
                 else
-                    vstore<float, V>(to, ta), vstore<float, V>(to + B, tb);
+                    vstore<float, V>(to, ta), vstore<float, V>(to + samples, tb);
             }
         }
         // batch totals: a transposed butterfly leaves total i on lane i, i.e. basis sum k = lane & 3 of gate lane >> 2 on
