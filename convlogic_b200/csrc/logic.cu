@@ -896,7 +896,9 @@ __global__ void __launch_bounds__(128, 3) logic_tree_bwd_kernel(const float *__r
 }
 
 // gx[f][b] = sum over the entries e of feature f of rows[list[e]][b]  (rows = tapgrad, list = leaf slots t*8+k)
-template <int V>
+// ASK: read past the L2 where `once` tells; a branch at run time, which makes the better code of V = 4 (21.4 us for 84 MB of 64 samples, an
+// instance of its own 28.6), but spilled for V = 1 (10240 trees, 99 samples, 32 MB: 17.3 us, without it 15.7; 40960, 131 samples: 63.8 and 69).
+template <int V, bool ASK>
 __global__ void __launch_bounds__(256) row_segment_sum_kernel(const float *__restrict__ rows, const int64_t *__restrict__ start,
                                                               const int32_t *__restrict__ list, float *__restrict__ gx, long long F,
                                                               long long B, bool once)
@@ -921,7 +923,7 @@ __global__ void __launch_bounds__(256) row_segment_sum_kernel(const float *__res
                         const int r = __shfl_sync(0xffffffffu, mine, min(i0 + u, n - 1));
                         if (in) {
                             const float *from = rows + (long long)r * B + b0;
-                            if (once)
+                            if (ASK && once)
                                 vload_once<float, V>(from, v[u]);
                             else
                                 vload<float, V>(from, v[u]);
@@ -1323,9 +1325,11 @@ static int logic_tree_bwd_impl(const float *x, const int32_t *leaf, const int32_
     }
     if (gx) {
         if (vec)
-            CLB_TRACED("row_segment_sum_kernel", st, row_segment_sum_kernel<4><<<logic_grid(in_dim), 256, 0, st>>>(tapgrad, start, list, gx, in_dim, B, once));
+            CLB_TRACED("row_segment_sum_kernel", st, row_segment_sum_kernel<4, true><<<logic_grid(in_dim), 256, 0, st>>>(tapgrad, start, list, gx, in_dim, B, once));
+        else if (once)
+            CLB_TRACED("row_segment_sum_kernel", st, row_segment_sum_kernel<1, true><<<logic_grid(in_dim), 256, 0, st>>>(tapgrad, start, list, gx, in_dim, B, true));
         else
-            CLB_TRACED("row_segment_sum_kernel", st, row_segment_sum_kernel<1><<<logic_grid(in_dim), 256, 0, st>>>(tapgrad, start, list, gx, in_dim, B, once));
+            CLB_TRACED("row_segment_sum_kernel", st, row_segment_sum_kernel<1, false><<<logic_grid(in_dim), 256, 0, st>>>(tapgrad, start, list, gx, in_dim, B, false));
         ++launched;
     }
     return check_launch(launched);
