@@ -1301,7 +1301,7 @@ static int logic_tree_bwd_impl(const float *x, const int32_t *leaf, const int32_
         const int grid = vec && (T + 3) / 4 > resident ? (int)resident : 2 * logic_grid(T);
         TreeHead rows = none;
         if (head && vec && gx && in_dim >= head->k) { // the input gradient's memory holds the classes' rows until the sums are written to it
-            tree_head_rows_kernel<<<(unsigned)((B * head->k + 255) / 256), 256, 0, st>>>(gx, B, *head);
+            CLB_TRACED("tree_head_rows_kernel", st, tree_head_rows_kernel<<<(unsigned)((B * head->k + 255) / 256), 256, 0, st>>>(gx, B, *head));
             gy = gx, rows.S = head->S, head = nullptr;
             ++launched;
         }

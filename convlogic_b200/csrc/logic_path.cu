@@ -373,11 +373,11 @@ extern "C" int clb_logic_path(const int64_t *a, const int64_t *b, const int32_t 
         set_last_cuda_error((int)e);
         return CLB_ERR_LAUNCH;
     }
-    path_link_kernel<<<fin, 256, 0, st>>>(start32, (const int2 *)entry, link, in, out);
-    path_walk_kernel<<<(unsigned)((2 * out_dim + 127) / 128), 128, 0, st>>>(link, order, placed, laid, out);
-    path_rest_kernel<<<fout, 256, 0, st>>>(order, placed, laid, out);
-    path_record_kernel<<<fout, 256, 0, st>>>(a, b, start32, order, placed, (int4 *)rec, closed, out);
-    path_open_kernel<<<fin, 256, 0, st>>>(closed, open, count, laid, in);
+    CLB_TRACED("path_link_kernel", st, path_link_kernel<<<fin, 256, 0, st>>>(start32, (const int2 *)entry, link, in, out));
+    CLB_TRACED("path_walk_kernel", st, path_walk_kernel<<<(unsigned)((2 * out_dim + 127) / 128), 128, 0, st>>>(link, order, placed, laid, out));
+    CLB_TRACED("path_rest_kernel", st, path_rest_kernel<<<fout, 256, 0, st>>>(order, placed, laid, out));
+    CLB_TRACED("path_record_kernel", st, path_record_kernel<<<fout, 256, 0, st>>>(a, b, start32, order, placed, (int4 *)rec, closed, out));
+    CLB_TRACED("path_open_kernel", st, path_open_kernel<<<fin, 256, 0, st>>>(closed, open, count, laid, in));
     return check_launch(5);
 }
 

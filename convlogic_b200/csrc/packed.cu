@@ -1403,9 +1403,9 @@ extern "C" int clb_packed_order(const int64_t *a, const int64_t *b, int32_t *ord
     if (cudaMemsetAsync(slot, 0xff, 4 * (size_t)in_dim + 8 * (size_t)out_dim, st) != cudaSuccess ||
         cudaMemsetAsync(count, 0, 4 + (size_t)out_dim, st) != cudaSuccess)
         return check_launch(0);
-    packed_pair_kernel<<<(unsigned)((2 * out_dim + 255) / 256), 256, 0, st>>>(a, b, slot, link, in, out);
-    packed_walk_kernel<<<(unsigned)((2 * out_dim + 127) / 128), 128, 0, st>>>(link, order, placed, count, out);
-    packed_rest_kernel<<<(unsigned)((out_dim + 255) / 256), 256, 0, st>>>(order, placed, count, out);
+    CLB_TRACED("packed_pair_kernel", st, packed_pair_kernel<<<(unsigned)((2 * out_dim + 255) / 256), 256, 0, st>>>(a, b, slot, link, in, out));
+    CLB_TRACED("packed_walk_kernel", st, packed_walk_kernel<<<(unsigned)((2 * out_dim + 127) / 128), 128, 0, st>>>(link, order, placed, count, out));
+    CLB_TRACED("packed_rest_kernel", st, packed_rest_kernel<<<(unsigned)((out_dim + 255) / 256), 256, 0, st>>>(order, placed, count, out));
     return check_launch(3);
 }
 

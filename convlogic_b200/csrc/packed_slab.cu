@@ -311,7 +311,7 @@ template <int S> static int launch(const void *x, const void *recs, void *y, int
 }
 template <int S> static int records(const uint8_t *ops, const int32_t *sel, const int32_t *order, Rec *recs, int Ci, int C, cudaStream_t st)
 {
-    packed_slab3_records_kernel<S><<<(C + 127) / 128, 128, 0, st>>>(ops, sel, order, recs, C, Ci);
+    CLB_TRACED("packed_slab3_records_kernel", st, packed_slab3_records_kernel<S><<<(C + 127) / 128, 128, 0, st>>>(ops, sel, order, recs, C, Ci));
     return clb_host::check_launch();
 }
 
