@@ -716,6 +716,8 @@ struct TreeHead {
     float tau;
 };
 
+constexpr long long kTreeRows = 1LL << 19; // outputs of the trees from which on their upstream gradients are laid out as rows
+
 // The head's upstream gradients as rows, a class each: up [k][B].  Read straight from dscore, a lane's four values lie four lines
 // apart (32 look-ups in the L1 per load instead of four) and are divided again for every tree.
 __global__ void __launch_bounds__(256) tree_head_rows_kernel(float *__restrict__ up, long long B, TreeHead head)
@@ -1300,7 +1302,9 @@ static int logic_tree_bwd_impl(const float *x, const int32_t *leaf, const int32_
         const long long resident = (long long)sm_count() * 3; // vec: one wave, whose warps fetch ahead from tree to tree
         const int grid = vec && (T + 3) / 4 > resident ? (int)resident : 2 * logic_grid(T);
         TreeHead rows = none;
-        if (head && vec && gx && in_dim >= head->k) { // the input gradient's memory holds the classes' rows until the sums are written to it
+        // Classes' upstream gradients as rows: a launch of 1.8 us, and one more to wait for, which the trees make good from there on (us of their kernel,
+        // from dscore / from rows: 5120 trees, 128 samples 12.8 / 10.6, 10240, 16 19.2 / 17.1; 10240, 100 22.2 / 18.1, 2560, 256 13.3 / 9.8)
+        if (head && vec && gx && in_dim >= head->k && T * B >= kTreeRows) { // (in the input gradient's memory, until the sums are written to it)
             CLB_TRACED("tree_head_rows_kernel", st, tree_head_rows_kernel<<<(unsigned)((B * head->k + 255) / 256), 256, 0, st>>>(gx, B, *head));
             gy = gx, rows.S = head->S, head = nullptr;
             ++launched;

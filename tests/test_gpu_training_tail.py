@@ -239,3 +239,43 @@ def test_group_sum_on_both_sides_of_its_lines(rows, batch, k, launches):
     assert len(names) == launches, names
     want = y.double().reshape(batch, k, rows).sum(-1) / 3.0
     assert (got - want).abs().max() <= rows / 3.0 * 2.0 ** -24 * (rows / 8 + 24)   # chains of an eighth of the rows at most, 24 further additions
+
+
+@pytest.mark.parametrize("dims,batch,rows", [((300, 16000, 8000, 4000), 128, False), ((300, 16000, 8000, 4000), 132, True), ((300, 16000, 8000, 4000), 256, True),
+                                             ((300, 16000, 8000, 4000), 300, True), ((300, 16000, 8000, 4000), 131, False), ((300, 32000, 16000, 8000), 300, True),
+                                             ((300, 32000, 16000, 8000), 301, False), ((512, 80000, 40000, 20000), 100, True), ((512, 80040, 40020, 20010), 256, True)])
+def test_many_trees_with_the_loss_head_against_float64_layers(dims, batch, rows):
+    """Several trees per warp and several trips per tree, forward (up to 60 parts per class) and backward; upstream gradients from the scores and as
+    rows; leaf gradients up to and beyond 64 MB; with the loss head and without.  Against the layers one by one in float64."""
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    torch.manual_seed(batch)
+    k, tau = 10, 30.0
+    seq = torch.nn.Sequential(*[cb.LogicLayer(i, o) for i, o in zip(dims[:-1], dims[1:])], cb.GroupSum(k, tau)).cuda().train()
+    for p in seq.parameters():
+        p.data.normal_()
+    x, lab = torch.rand(batch, dims[0], device="cuda"), torch.randint(0, k, (batch,), device="cuda")
+    fused = cb.fuse_logic_layers(seq)[0].train()
+
+    def grads(loss_fn, params, xi):
+        return list(torch.autograd.grad(loss_fn(xi), [xi, *params]))
+
+    params = [layer.weights for layer in seq[:3]]
+    got_sum = grads(lambda xi: cb.GroupSumCrossEntropy(k, tau)(fused(xi), lab), params, x.clone().requires_grad_(True))
+    _lib.trace(True)
+    loss = fused.cross_entropy(xi := x.clone().requires_grad_(True), lab, k, tau)
+    got = list(torch.autograd.grad(loss, [xi, *params]))
+    torch.cuda.synchronize()
+    names = _lib.trace_report()
+    _lib.trace(False)
+    assert ("tree_head_rows_kernel" in names) == rows, names
+    seq.double()
+    xd = x.double().requires_grad_(True)
+    want_loss = torch.nn.functional.cross_entropy(seq(xd), lab)
+    want = torch.autograd.grad(want_loss, [xd, *(layer.weights for layer in seq[:3])])
+    # scores: sums of up to 2001 outputs in [0, 1] over tau; gradients: of the size of their largest entry, sums of at most 301 products
+    assert abs(float(loss) - float(want_loss)) <= 1e-5 * float(want_loss)
+    for u, v, w in zip(got, got_sum, want):
+        assert_close(u, w, 2e-5, "with the loss head")
+        assert_close(v, w, 2e-5, "without")
