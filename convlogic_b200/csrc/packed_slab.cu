@@ -125,7 +125,9 @@ template <int S> __device__ __noinline__ uint4 window_global(const uint4 *__rest
     return acc;
 }
 
-template <int S>
+// ONE: a block per item.  What lets a block go on from item to item (two more places of the fetches and copies, the items ahead) then only holds
+// up the first: one slab, us for 32x32, 16x16, 8x8 images with it / without, k = 128 4.9, 4.5, 5.6 / 4.5, 4.1, 4.9, k = 256 5.7, 5.2, 7.9 / 5.3, 4.6, 7.4.
+template <int S, bool ONE>
 __global__ void __launch_bounds__(Geo<S>::THREADS, 1024 / Geo<S>::THREADS)
     packed_convtree_slab3_kernel(const uint4 *__restrict__ x, const Rec *__restrict__ recs, uint4 *__restrict__ y, Shape s)
 {
@@ -173,48 +175,49 @@ __global__ void __launch_bounds__(Geo<S>::THREADS, 1024 / Geo<S>::THREADS)
     // channels (L2-resident).  A block takes every gridDim.x-th run of consecutive items, within which a record copies
     // the planes only that the one before did not leave in the tile; the items of three are known ahead.
     struct Item {
-        int i, end, run, ug, r; // item, end of its run, the run; its slab group and record
-        bool fresh;             // nothing in the tile
+        int left, run, ug, r; // items left of its run, the run; its slab group and record
+        bool fresh;           // nothing in the tile
     };
-    auto begin = [&](Item &t) {
-        if (t.run < s.runs) {
-            t.i = t.run * s.per_run + min(t.run, s.longer), t.end = t.i + s.per_run + (t.run < s.longer);
-            t.ug = t.i / s.C, t.r = t.i - t.ug * s.C;
+    auto advance = [&](Item &t) {
+        t.fresh = true;
+        if (t.left > 0) {
+            --t.left;
+            t.fresh = ++t.r == s.C;
+            if (t.fresh) t.r = 0, ++t.ug;
+        } else if ((t.run += gridDim.x) < s.runs) {
+            const int i = t.run * s.per_run + min(t.run, s.longer);
+            t.left = s.per_run - (t.run < s.longer ? 0 : 1), t.ug = i / s.C, t.r = i - t.ug * s.C;
         } else {
             t.ug = s.n_ug;
         }
-        t.fresh = true;
-    };
-    auto advance = [&](Item &t) {
-        if (++t.i < t.end) {
-            t.fresh = ++t.r == s.C;
-            if (t.fresh) t.r = 0, ++t.ug;
-        } else {
-            t.run += gridDim.x;
-            begin(t);
-        }
     };
     Item n0, n1, n2;
-    n0.run = blockIdx.x;
-    begin(n0);
-    n1 = n0;
-    advance(n1);
-    n2 = n1;
-    if (n2.ug < s.n_ug) advance(n2);
-    if (n0.ug < s.n_ug) fetch_rec(n0.r, rec[0]);
-    if (n1.ug < s.n_ug) fetch_rec(n1.r, rec[1]);
+    if constexpr (ONE) {
+        n0.ug = blockIdx.x / s.C, n0.r = blockIdx.x - n0.ug * s.C;
+        n1.ug = n2.ug = s.n_ug;
+        fetch_rec(n0.r, rec[0]);
+    } else {
+        n0.run = (int)blockIdx.x - (int)gridDim.x, n0.left = 0;
+        advance(n0);
+        n1 = n0;
+        advance(n1);
+        n2 = n1;
+        if (n2.ug < s.n_ug) advance(n2);
+        fetch_rec(n0.r, rec[0]);
+        if (n1.ug < s.n_ug) fetch_rec(n1.r, rec[1]);
+    }
     cp_async_commit();
     cp_async_wait_all();
     __syncthreads(); // records and halo zeros in place
-    if (n0.ug < s.n_ug) stage(n0.ug, rec[0], true);
+    stage(n0.ug, rec[0], true);
     cp_async_commit();
-    for (int r0 = 0; n0.ug < s.n_ug; r0 = r0 == 2 ? 0 : r0 + 1) {
+    for (int r0 = 0; ONE ? r0 == 0 : n0.ug < s.n_ug; r0 = r0 == 2 ? 0 : r0 + 1) {
         const int r1 = r0 == 2 ? 0 : r0 + 1, r2 = r1 == 2 ? 0 : r1 + 1;
         cp_async_wait_all();
         __syncthreads(); // this item's planes and the next item's record have landed
-        if (n2.ug < s.n_ug) fetch_rec(n2.r, rec[r2]);
+        if (!ONE && n2.ug < s.n_ug) fetch_rec(n2.r, rec[r2]);
         const Rec &R = rec[r0];
-        const int u0 = n0.ug * G::UB, c0 = R.c;
+        const int u0 = n0.ug * G::UB;
         const bool live = ub < s.U - u0;
         uint4 out = make_uint4(0u, 0u, 0u, 0u);
         if (live) {
@@ -241,15 +244,20 @@ __global__ void __launch_bounds__(Geo<S>::THREADS, 1024 / Geo<S>::THREADS)
                 out = window_global<S>(x + (size_t)(u0 + ub) * G::HW, R, s, py, px);
             }
         }
-        __syncthreads(); // every thread is done with the tile: the next item's planes go there while the SM's other blocks compute
-        if (n1.ug < s.n_ug) stage(n1.ug, rec[r1], n1.fresh);
-        cp_async_commit();
+        if constexpr (!ONE) {
+            __syncthreads(); // every thread is done with the tile: the next item's planes go there while the SM's other blocks compute
+            if (n1.ug < s.n_ug) stage(n1.ug, rec[r1], n1.fresh);
+            cp_async_commit();
+        }
         if (live) {
+            const int c0 = R.c;
             if (s.out == kRows) y[((size_t)c0 * G::I + t) * s.U + u0 + ub] = out;
             else y[((size_t)c0 * s.U + u0 + ub) * G::I + (s.out == kSplitSlabs ? split_position(t, G::H2) : t)] = out;
         }
-        n0 = n1, n1 = n2;
-        if (n2.ug < s.n_ug) advance(n2);
+        if constexpr (!ONE) {
+            n0 = n1, n1 = n2;
+            if (n2.ug < s.n_ug) advance(n2);
+        }
     }
     cp_async_wait_all();
 }
@@ -298,15 +306,18 @@ template <int S> static int launch(const void *x, const void *recs, void *y, int
     using namespace clb_host;
     Shape s{Ci, C, (int)U, (int)((U + G::UB - 1) / G::UB), in, out, 0, 0, 0};
     constexpr int bytes = 2 * G::PLANE_BYTES;
-    auto k = packed_convtree_slab3_kernel<S>;
-    if (ensure_dynamic_smem(k, bytes) != cudaSuccess) return check_launch(0);
     constexpr int by_smem = 227 * 1024 / (bytes + 2048), by_threads = 1024 / G::THREADS; // 64 registers a thread
     const long long items = (long long)C * s.n_ug, all = (long long)sm_count() * (by_smem < by_threads ? by_smem : by_threads);
     // runs of about 16 items, as many for one block as for another (k = 1024, 8192 samples, four blocks: 1610 us with 4, 1590 with 16 and 32)
     const long long grid = items < all ? items : all, rounds = (items + 8 * grid) / (16 * grid), runs = grid * (rounds > 0 ? rounds : 1);
     s.runs = (int)runs, s.per_run = (int)(items / runs), s.longer = (int)(items % runs);
+    // A block per item up to a quarter more than are resident at once (4x4 images, 4096 items on 3552 places: 7.9 us with blocks that go on, 7.5; 8192:
+    // 10.7 either way; 32x32, 1024 on 592: 11.2 / 12.3).
+    const bool one = 4 * items <= 5 * all;
+    auto k = one ? packed_convtree_slab3_kernel<S, true> : packed_convtree_slab3_kernel<S, false>;
+    if (ensure_dynamic_smem(k, bytes) != cudaSuccess) return check_launch(0);
     CLB_TRACED("packed_convtree_slab3_kernel", st,
-               k<<<(unsigned)grid, G::THREADS, bytes, st>>>((const uint4 *)x, (const Rec *)recs, (uint4 *)y, s));
+               k<<<(unsigned)(one ? items : grid), G::THREADS, bytes, st>>>((const uint4 *)x, (const Rec *)recs, (uint4 *)y, s));
     return check_launch();
 }
 template <int S> static int records(const uint8_t *ops, const int32_t *sel, const int32_t *order, Rec *recs, int Ci, int C, cudaStream_t st)

@@ -106,3 +106,33 @@ def test_output_channels_in_an_order_that_shares_planes(side, c, kind, batch):
         assert torch.equal(cb.CompiledLogicNet(net, input_shape=(ci, side, side)).compile()(bits).long(), want)
     finally:
         _lib.check(_lib.lib().clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 1))
+
+
+@pytest.mark.parametrize("kind", ["chain", "any pairs"])
+@pytest.mark.parametrize("side,c,batch", [(32, 40, 2300), (32, 40, 2450), (32, 40, 4900), (32, 40, 46000), (16, 70, 5300), (16, 70, 5500), (16, 70, 105000), (8, 300, 4700),
+                                          (8, 300, 4900), (8, 300, 91000), (4, 700, 6000), (4, 700, 7000), (4, 700, 126000)])
+def test_blocks_of_one_item_and_of_many(side, c, batch, kind):
+    """On both sides of the line between a block per item and blocks that go on from item to item (148 SMs), and with several runs of items per block."""
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    ci = 5
+    torch.manual_seed(side + c)
+    i = torch.arange(c)
+    first, second = (i % ci, (i + 1) % ci) if kind == "chain" else tuple(torch.randint(0, ci, (2, c)))
+    ch = torch.where(torch.rand(c, 8) < 0.5, first[:, None], second[:, None])
+    words = ((ch << 16) | (torch.randint(0, 3, (c, 8)) << 8) | torch.randint(0, 3, (c, 8))).int()
+    feat = c * (side // 2) ** 2
+    net = torch.nn.Sequential(cb.ConvLogicLayer(ci, c, padding=1, kernel=3, selection=words, complete=True), torch.nn.Flatten(),
+                              cb.LogicLayer(feat, feat // 2 * 2), cb.GroupSum(2)).cuda()
+    for p in net.parameters():
+        p.data.normal_()
+    bits = torch.rand(batch, ci, side, side, device="cuda") < 0.5
+    net.eval()
+    with torch.no_grad():
+        want = torch.cat([net(part.float()).round().long() for part in bits.split(10000)])
+    _lib.check(_lib.lib().clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 0))
+    try:
+        assert torch.equal(cb.CompiledLogicNet(net, input_shape=(ci, side, side)).compile()(bits).long(), want)
+    finally:
+        _lib.check(_lib.lib().clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 1))
