@@ -451,6 +451,9 @@ template <int S> struct BwdCfg {
     static constexpr int SLOT = (NIMG * IMG + 31) / 32 * 32;
     static constexpr int STAGE_FLOATS = 2 * SLOT, STAGE_BYTES = STAGE_FLOATS * 4;
     static constexpr int XST = S == 4 ? 2 : 3;          // stages of input planes
+    // resident per SM, by registers and shared memory: what parts of the batch are planned for (4x4 planned for three, as it was with three
+    // stages: 1600 -> 3200 channels, 500 images 170 us, now 136; 128 -> 1000, 333 images 36.0 / 31.1; 512 -> 1024, 100 images 13.5 / 14.2)
+    static constexpr int BLOCKS = 4;
     static constexpr int GT_BYTES = XST * STAGE_BYTES;  // byte distance from stage 0 to the gradient tile: the same cell offsets
     static constexpr int WARP_BYTES = (XST + 1) * STAGE_BYTES;
     static constexpr int SMEM = (kThreads / 32) * WARP_BYTES;
@@ -496,7 +499,7 @@ __device__ __forceinline__ void bwd_windows(const uint32_t (&base)[WPT], const u
 }
 
 template <int S, bool FM>
-__global__ void __launch_bounds__(kThreads) convtree_bwd_plane_kernel(const float *__restrict__ gy, const float *__restrict__ x,
+__global__ void __launch_bounds__(kThreads, BwdCfg<S>::BLOCKS) convtree_bwd_plane_kernel(const float *__restrict__ gy, const float *__restrict__ x,
                                                                       const float *__restrict__ w, const int32_t *__restrict__ sel,
                                                                       const uint8_t *__restrict__ amax, float *__restrict__ partial,
                                                                       float *__restrict__ planes, Args s)
@@ -954,7 +957,8 @@ int bwd_slice(int N, int C, int HW)
 }
 int bwd_parts(int side, int N, int C)
 {
-    return side == 8 ? clb_plane_parts(N, C, BwdCfg<8>::NIMG, 4, 4) : side == 4 ? clb_plane_parts(N, C, BwdCfg<4>::NIMG, 4, 3) : clb_tile_bwd_parts(side, N, C);
+    return side == 8 ? clb_plane_parts(N, C, BwdCfg<8>::NIMG, 4, BwdCfg<8>::BLOCKS)
+           : side == 4 ? clb_plane_parts(N, C, BwdCfg<4>::NIMG, 4, BwdCfg<4>::BLOCKS) : clb_tile_bwd_parts(side, N, C);
 }
 size_t bwd_partial_bytes(int side, int N, int C)
 {
