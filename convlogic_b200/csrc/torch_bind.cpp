@@ -544,6 +544,14 @@ struct LogicPlan {
     int64_t n_open = 0;
     bool captured = false; // a stream capture reads it: its tables stay with the plan that replaces it, for the graph holds their addresses
     std::shared_ptr<LogicPlan> held;
+    c10::Stream stream{c10::Stream::UNSAFE, c10::Device(c10::kCPU), 0}; // of the tables' memory
+    void used() const // on the current stream: the memory of a plan that goes waits for what that stream still reads
+    {
+        const c10::Stream now = c10::cuda::getCurrentCUDAStream().unwrap();
+        if (now == stream) return;
+        for (const Tensor &t : {start32, entry, rec, open})
+            if (t.defined()) t.record_stream(now);
+    }
     bool path_fwd(int64_t batch) const { return rec.defined() && clb_logic_path_pays(in, out, batch, n_open, 0); }
     bool path_bwd(int64_t batch) const { return rec.defined() && clb_logic_path_pays(in, out, batch, n_open, 1); }
 };
@@ -559,7 +567,10 @@ LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const 
     LogicPlanPtr old = last;
     if (old && !(old->key == key && old->in == in && old->out == out)) old = nullptr;
     if (old && capture) old->captured = true;
-    if (old && (old->paths || !paths)) return old;
+    if (old && (old->paths || !paths)) {
+        old->used();
+        return old;
+    }
     need_inputs(a, b, start, cons);
     TORCH_CHECK(start.scalar_type() == at::kLong && cons.scalar_type() == at::kLong && start.numel() == in + 1 && cons.numel() == 2 * out,
                 "convlogic_b200: consumer lists must be int64 [in_dim + 1] and [2 * out_dim]");
@@ -568,9 +579,11 @@ LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const 
     if (capture) return old;
     auto p = std::make_shared<LogicPlan>();
     p->key = key, p->in = in, p->out = out, p->paths = paths;
+    p->stream = c10::cuda::getCurrentCUDAStream().unwrap();
     if (last) p->held = last->captured ? last : last->held;
     Below below(start);
     if (old) {
+        old->used();
         p->start32 = old->start32, p->entry = old->entry;
     } else {
         p->start32 = alloc({in + 1}, start, at::kInt), p->entry = alloc({2 * out, 2}, start, at::kInt);

@@ -267,3 +267,32 @@ def test_lists_of_other_connections_are_counted(kind):
         a, b, second = p["a"][code >> 1], p["b"][code >> 1], (code & 1).bool()
         entered, left = torch.where(second, b, a), torch.where(second, a, b)
         assert torch.equal(entered[1:][linked], left[:-1][linked])
+
+
+@pytest.mark.parametrize("packed", [False, True])
+def test_a_plan_that_goes_while_another_stream_reads_it(packed):
+    """Laid out on one stream, read on another that is behind, given back and its memory asked for on the first."""
+    import convlogic_b200 as cb
+
+    torch.manual_seed(0)
+    n = 30000 if packed else 100000
+    layer, side = cb.LogicLayer(n, n).cuda(), torch.cuda.Stream()
+    layer.train(not packed)
+    holder = layer.indices_0 if packed else layer.given_x_indices_of_y_start
+    x = cb.PackBitsTensor(torch.rand(2000, n, device="cuda") < 0.5, 32) if packed else torch.rand(320, n, device="cuda", requires_grad=True)
+
+    def call():
+        return layer(x).rows() if packed else layer(x).detach()
+
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        want = call()
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)
+    got = call()
+    del holder._clb_plan
+    with torch.cuda.stream(side):
+        filler = [torch.full((size,), 1 << 29, dtype=torch.int32, device="cuda") for size in (n, n, n + 1, 2 * n, 4 * n, 4 * n) for _ in range(4)]
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
+    del filler
