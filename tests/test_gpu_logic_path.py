@@ -110,25 +110,48 @@ def test_path_passes_against_oracle(kind, fin, fout, batch):
     assert torch.equal(gx, again[0]) and torch.equal(gw, again[1])
 
 
-def test_lists_that_contradict_the_connections_are_noticed():
+def test_lists_of_a_layer_with_the_same_number_of_readers():
+    """Consistent tables of other connections: every neuron once all the same, linked only where it does read what the one before reads."""
     fin = fout = 64
     a, b = _connections("twice", fin, fout)
-    p = _plan(a, b, fin)
-    other = _plan(a.flip(0), b.flip(0), fin)
-    lib_args = [_ptr(p["a"]), _ptr(p["b"]), _ptr(other["start"]), _ptr(other["entry"])]
-    from convlogic_b200 import _lib
-
-    n = _lib.lib().clb_logic_path_scratch_bytes(fin, fout)
-    scratch = torch.empty(n, dtype=torch.uint8, device="cuda")
-    assert _lib.lib().clb_logic_path(*lib_args, _ptr(p["rec"]), _ptr(p["open"]), _ptr(p["count"]), _ptr(scratch), n, fin, fout, _stream()) == 0
-    rec = p["rec"].cpu().long()
-    if int(p["count"][0]) == fout:   # every neuron once all the same: then a linked neuron does read what the one before read
-        linked = (rec[1:, 3] & 1).bool()
-        assert torch.equal(rec[1:, 1][linked], rec[:-1, 2][linked])
+    p, other = _plan(a, b, fin), _plan(a.flip(0), b.flip(0), fin)
+    rec, (laid, _) = _layout(p["a"], p["b"], other["start"], other["entry"], fin)
+    rec = rec.cpu().long()
+    assert laid == fout and torch.equal((rec[:, 0] >> 1).sort().values, torch.arange(fout))
+    linked = (rec[1:, 3] & 1).bool()
+    assert torch.equal(rec[1:, 1][linked], rec[:-1, 2][linked])
 
 
-@pytest.mark.parametrize("width,batch,path", [(40000, 210, True), (40000, 200, False), (83400, 101, True), (83000, 101, False), (28000, 900, True), (100000, 1024, True), (100000, 1022, True), (99001, 1021, True)])
-def test_layers_take_the_path_by_size(width, batch, path):
+def test_a_layer_whose_lists_contradict_its_connections_does_not_walk():
+    """Neurons listed twice, others not at all: no plan of paths, and outputs of the connections."""
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib, ops
+    from convlogic_b200._lib import W_SOFTMAX
+
+    n, batch = 100000, 320
+    torch.manual_seed(0)
+    layer = cb.LogicLayer(n, n).cuda().train()
+    a, b = _connections("trail", n, n)
+    layer.indices_0.copy_(a), layer.indices_1.copy_(b)
+    start, cons = cb.LogicLayer.build_consumer_lists(a, b, n)
+    cons[129:150000:128] = cons[131:150002:128]
+    layer.given_x_indices_of_y_start.copy_(start), layer.given_x_indices_of_y.copy_(cons)
+    x = torch.rand(n, batch, device="cuda")
+    xd = x.t().detach().requires_grad_(True)
+    _lib.trace(True)
+    y = layer(xd)
+    y.sum().backward()
+    torch.cuda.synchronize()
+    names = _lib.trace_report()
+    _lib.trace(False)
+    assert "path_walk_kernel" in names and not {"logic_path_fwd_kernel", "logic_path_bwd_kernel"} & set(names), names
+    assert float((y.detach().t() - ops.logic_fwd(x, layer.indices_0, layer.indices_1, layer.weights.detach(), W_SOFTMAX)).abs().max()) <= 1e-5
+
+
+@pytest.mark.parametrize("width,batch,path,forward", [(40000, 210, True, False), (40000, 200, False, False), (83400, 101, True, False), (83000, 101, False, False),
+                                                      (28000, 900, True, False), (100000, 1024, True, True), (100000, 1022, True, True), (99001, 1021, True, True),
+                                                      (99000, 318, True, True), (98000, 318, True, False)])
+def test_layers_take_the_path_by_size(width, batch, path, forward):
     import convlogic_b200 as cb
     from convlogic_b200 import _lib, ops
     from convlogic_b200._lib import W_SOFTMAX
@@ -144,12 +167,32 @@ def test_layers_take_the_path_by_size(width, batch, path):
     torch.cuda.synchronize()
     names = _lib.trace_report()
     _lib.trace(False)
-    assert ("logic_path_bwd_kernel" in names) == path, names
+    assert ("logic_path_bwd_kernel" in names) == path and ("logic_path_fwd_kernel" in names) == forward, names
     # the same terms in another order
     for got, want in ((y.detach().t(), ops.logic_fwd(x, *tables, W_SOFTMAX)),
                       (xd.grad.t(), ops.logic_bwd_x(x, *tables, gy, layer.given_x_indices_of_y_start, layer.given_x_indices_of_y, W_SOFTMAX)),
                       (layer.weights.grad, ops.logic_bwd_w(x, *tables, gy, W_SOFTMAX))):
         assert (got - want).norm() <= 1e-5 * want.norm()
+    # and a range of neurons and of features against the gates in fp64
+    a, b = layer.indices_0, layer.indices_1
+    some = torch.arange(width // 3, width // 3 + 50, device="cuda")
+    xs = x.t().double()[:, torch.cat([a[some], b[some]])].cpu().requires_grad_(True)
+    ws = layer.weights.detach()[some].double().cpu().requires_grad_(True)
+    i = torch.arange(50)
+    ys = oracle.logic_layer(xs, i, i + 50, oracle.gate_probabilities(ws, True))
+    ys.backward(gy[some].t().double().cpu())
+    assert (y.detach()[:, some].double().cpu() - ys).abs().max() <= 1e-5
+    assert (layer.weights.grad[some].double().cpu() - ws.grad).abs().max() <= 1e-5 * ws.grad.abs().max()   # sums of 1024 products
+    readers = [((a == f) | (b == f)).nonzero().flatten() for f in some[:10]]
+    for f, js in zip(some[:10], readers):
+        xs = x.t().double()[:, torch.cat([a[js], b[js]])].cpu()
+        at = torch.cat([a[js], b[js]]).cpu() == int(f)
+        col = x[f].double().cpu().requires_grad_(True)
+        inputs = torch.where(at, col[:, None], xs)
+        k = torch.arange(len(js))
+        out = oracle.logic_layer(inputs, k, k + len(js), oracle.gate_probabilities(layer.weights.detach()[js].double().cpu(), True))
+        out.backward(gy[js].t().double().cpu())
+        assert (xd.grad[:, f].double().cpu() - col.grad).abs().max() <= 1e-5 * max(1.0, float(col.grad.abs().max()))
 
 
 @pytest.mark.parametrize("kind,fin,fout,batch", [("twice", 1, 1, 1), ("twice", 300, 300, 66), ("any", 500, 900, 100), ("any", 900, 500, 33), ("pairs", 600, 600, 96),
