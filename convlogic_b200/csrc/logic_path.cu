@@ -335,16 +335,19 @@ static int path_vec(int64_t B, std::initializer_list<const void *> rows)
     return bits % 16 == 0 ? 4 : bits % 8 == 0 ? 2 : 1;
 }
 
-// Where each feature has two readers, so that nearly all gradients are completed on the way, from these sizes of x on (us without / with):
-// forward, beyond the L2's useful half: 128000 x 300 84 / 75, 250000 x 128 68 / 63, 64000 x 1000 120 / 116; 250000 x 101 66 / 69, 100000 x 250
-// 53 / 54, 64000 x 256 35 / 36; backward, where three launches have something to do: 65536 x 128 42 / 42, 16000 x 512 42 / 38, 20000 x 420
-// 46 / 42, 260000 x 32 71 / 60, 100000 x 97 69 / 56, 250000 x 66 138 / 96, 250000 x 511 790 / 353; 64000 x 64 28 / 32, 8000 x 100 19 / 24.  Elsewhere the input is in the L2, or is read once either way (4096 -> 40960 x 500
-// forward 29 / 32, backward 71 / 89; 300000 -> 200000 x 256 103 / 110, 265 / 267).
+// Where each feature has two readers, so that nearly all gradients are completed on the way, from these sizes of x on (us of the whole pass, the
+// L2 flushed before it, without / with).  Forward, beyond the L2's useful half: 128000 x 300 84 / 75, 250000 x 128 68 / 64, 64000 x 1000 120 / 116; 250000 x
+// 101 66 / 69, 100000 x 250 53 / 54, 64000 x 256 35 / 38; not where a batch of more than 48 samples leaves much of its stretches empty: 458000 x 72 84 /
+// 87, 347000 x 95 84 / 102, 243000 x 136 76 / 85 (444000 x 136 134 / 154), but 687000 x 48 105 / 97, 344000 x 96 78 / 75, 206000 x 160 74 / 73, 187500 x 176 72 /
+// 73, 166000 x 360 140 / 110.  Backward, where three launches have something to do: 65536 x 128 42 / 42, 16000 x 512 42 / 38, 20000 x 420 46 / 40, 260000 x 32
+// 70 / 60, 100000 x 97 71 / 56, 250000 x 66 138 / 95, 250000 x 511 783 / 349; 64000 x 64 28 / 32, 8000 x 100 19 / 24.  Elsewhere the input is in the L2, or
+// is read once either way (4096 -> 40960 x 500 forward 29 / 32, backward 71 / 89; 300000 -> 200000 x 256 103 / 110, 265 / 267).
 extern "C" int clb_logic_path_pays(int64_t in_dim, int64_t out_dim, int64_t B, int64_t n_open, int what)
 {
     const int64_t bytes = in_dim * B * 4;
     if (in_dim != out_dim || 16 * n_open > in_dim) return 0;
-    return bytes >= (what == 0 ? 120LL << 20 : 32LL << 20);
+    if (what == 0) return bytes >= 120LL << 20 && (B >= 160 || B % 32 == 0 || B <= 48);
+    return bytes >= 32LL << 20;
 }
 
 extern "C" size_t clb_logic_path_scratch_bytes(int64_t in_dim, int64_t out_dim)

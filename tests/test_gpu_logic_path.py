@@ -150,7 +150,8 @@ def test_a_layer_whose_lists_contradict_its_connections_does_not_walk():
 
 @pytest.mark.parametrize("width,batch,path,forward", [(40000, 210, True, False), (40000, 200, False, False), (83400, 101, True, False), (83000, 101, False, False),
                                                       (28000, 900, True, False), (100000, 1024, True, True), (100000, 1022, True, True), (99001, 1021, True, True),
-                                                      (99000, 318, True, True), (98000, 318, True, False)])
+                                                      (99000, 318, True, True), (98000, 318, True, False),
+                                                      (331000, 96, True, True), (331000, 97, True, False), (198000, 159, True, False), (198000, 160, True, True)])
 def test_layers_take_the_path_by_size(width, batch, path, forward):
     import convlogic_b200 as cb
     from convlogic_b200 import _lib, ops
@@ -249,6 +250,7 @@ def test_a_captured_step_keeps_the_plan_it_reads(width, batch):
         y = layer(x)
         return [y.detach(), *torch.autograd.grad(y, [x, layer.weights], gy)]
 
+    torch.cuda.synchronize()
     with torch.cuda.stream(torch.cuda.Stream()):
         want = step()
         step()
