@@ -1375,13 +1375,23 @@ extern "C" int clb_packed_logic(const void *x, const int64_t *a, const int64_t *
     return check_launch();
 }
 
-// From 6 MB of output on, where no input is left unread (20000 x 500 bytes 11.9 / 9.8 us, 100000 x 68 22.9 / 9.5; below, the eight positions in
-// turn of a range take longer than the second row: 5000 x 400 8 / 13, 2000 x 40 7 / 11).
+// Where no input is left unread, by bytes of output and by how the plain kernel reads a row: in units of 16, 8 or 4 bytes, by as many lanes, up to
+// 32, as the power of two that covers it.  us per layer with it / on this walk, layer after layer in one graph:
+//   rows of four units or fewer: never (32 bytes, 8 MB 5.7 / 12.4, 40 MB 30 / 54; 64 bytes, 20 MB 10.4 / 14.2; 24 bytes, 12 MB 13.8 / 17.1)
+//   4-byte units, fewer than 64                     6 MB  36 bytes 18.1 / 8.6, 100 bytes 14.0 / 6.5, 252 bytes 7.5 / 6.1; at 4 MB 5.7 / 6.0
+//   longer rows                                     8.5   500 bytes, 8 MB 6.4 / 6.0, 1252 bytes 6.0 / 6.6; at 12 MB 8.7 / 6.5, 7.8 / 6.5
+//   8-byte units, fewer than 32                     6     40 bytes 9.3 / 7.3, 120 bytes 7.0 / 6.5, 248 bytes 6.9 / 7.2; at 4 MB 6.9 / 6.5, 5.2 / 7.0, 5.2 / 6.8
+//   longer rows                                     12    504 bytes, 12 MB 7.6 / 6.6, 1256 bytes 6.9 / 6.6, 2008 bytes 6.0 / 6.5; at 8 MB 5.3 / 6.3
+//   16-byte units, fewer than 32, no power of two   10    80 bytes, 8 MB 7.2 / 7.5, 12 MB 9.9 / 8.5, 400 bytes 6.3 / 6.7, 8.2 / 6.8
+//   other rows                                      18    256 bytes, 12 MB 7.1 / 8.0, 20 MB 10.1 / 8.2, 1024 bytes 5.4 / 6.6, 7.5 / 7.1
 extern "C" int clb_packed_path_pays(int64_t in_dim, int64_t out_dim, int64_t words, int bits)
 {
     if (in_dim <= 0 || out_dim < in_dim || words <= 0 || !bits_ok(bits)) return 0;
-    const int64_t rowbytes = words * (bits / 8);
-    return rowbytes % 4 == 0 && out_dim * rowbytes >= (6LL << 20);
+    const int64_t rowbytes = words * (bits / 8), unit = rowbytes % 16 == 0 ? 16 : rowbytes % 8 == 0 ? 8 : 4, units = rowbytes / unit;
+    if (rowbytes % 4 || units < 5) return 0;
+    const bool idle = unit == 4 ? units < 64 : units < 32 && (units & (units - 1)) != 0;
+    const int64_t line = unit == 4 ? (idle ? 6000000 : 8500000) : unit == 8 ? (idle ? 6000000 : 12000000) : (idle ? 10000000 : 18000000);
+    return out_dim * rowbytes >= line;
 }
 
 extern "C" size_t clb_packed_order_scratch_bytes(int64_t in_dim, int64_t out_dim)

@@ -188,3 +188,19 @@ def test_when_a_flat_forward_asks_for_memory(lib):
     assert not asks(1 << 17, 1 << 17, 500) and asks(1 << 16, 1 << 16, 1020) and not asks(1 << 16, 1 << 16, 1022)
     assert not asks(200000, 199999, 512) and asks(66000, 33001, 260) and not asks(80000, 40000, 260) and asks(200000, 200000, 512)
     assert not asks(1 << 17, 1 << 17, 512, 1) and not asks(0, 5, 512) and not asks(5, 0, 512)
+
+
+@pytest.mark.parametrize("rowbytes,bytes_", [(16, 0), (32, 0), (64, 0), (24, 0), (12, 0), (4, 0), (36, 6000000), (252, 6000000), (256 - 4, 6000000), (260, 8500000), (1252, 8500000),
+                                             (40, 6000000), (248, 6000000), (264, 12000000), (1256, 12000000), (80, 10000000), (400, 10000000), (128, 18000000),
+                                             (256, 18000000), (512, 18000000), (1248, 18000000), (250, 0), (1250, 0)])
+def test_packed_layers_walk_from_their_line_on(rowbytes, bytes_):
+    from convlogic_b200 import _lib
+
+    pays = _lib.lib().clb_packed_path_pays
+    for bits in (8, 16) if rowbytes % 4 else (8, 16, 32):
+        words = rowbytes * 8 // bits
+        if not bytes_:
+            assert not pays(100, 50000000 // rowbytes * 10, words, bits)
+            continue
+        least = -(-bytes_ // rowbytes)
+        assert pays(least, least, words, bits) and pays(10, least, words, bits) and not pays(least - 1, least - 1, words, bits) and not pays(least + 1, least, words, bits)
