@@ -563,7 +563,8 @@ LogicPlanPtr logic_plan_for(const py::handle &start_obj, const Tensor &a, const 
 {
     const LogicKey key = logic_key(a, b, start, cons);
     const LogicPlanPtr last = kept<LogicPlan>(start_obj);
-    const bool capture = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+    // (the default stream, which cannot be captured, is not asked: it would cost half a microsecond per layer and step)
+    const bool capture = c10::cuda::getCurrentCUDAStream().stream() && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
     LogicPlanPtr old = last;
     if (old && !(old->key == key && old->in == in && old->out == out)) old = nullptr;
     if (old && capture) old->captured = true;
