@@ -1545,10 +1545,22 @@ int clb_packed_tree_count(const void *x, const int32_t *leaf, const uint8_t *ops
     // us in one pass / apart: 10.5 MB of outputs 22 / 20, 21 MB 28 / 30 and 27 / 33, 42 MB 43 / 46, 84 MB 72 / 84, 671 MB 483 / 622;
     // 34 units on 40 lanes 36 / 33, 11 on 16 (115 MB) 127 / 122.
     if (out_dim * U * 16 < (20LL << 20) || 16 * u_n < 15 * (chunks << lg)) return CLB_ERR_SHAPE;
-    // one wave of blocks, of at least 16 trees per walker, and no more than 2^12 - 1
-    long long parts = (long long)kTreeCountBlocks * sm_count() / (chunks * k);
-    parts = std::min(parts, S / (16 * walkers));
-    parts = std::max(parts, S / (walkers * 4000) + 1);
+    // Parts of a class, of at least 16 trees per walker and no more than 2^12 - 1: those of the least time, in trees of a walker, when a wave of blocks
+    // takes a part's trees and the adding up, and one with a block per SM at most 0.6 of that; one wave more for a twentieth at least.  (As many as fit one wave:
+    // 150 classes of 2000 trees, 4096 samples have 150 blocks for 296 places, 147 us apart, 201 so, 138 in five parts; 10 of 2000, 30720 81 / 106 / 82.)
+    const long long slots = (long long)kTreeCountBlocks * sm_count();
+    const double adding = 3.0 + 0.4 * (double)walkers;
+    const long long least = S / (walkers * 4000) + 1, limit = std::max(least, std::min(S / (16 * walkers), 1024LL));
+    long long parts = least, full = -1;
+    double cost = -1.0;
+    for (long long p = least; p <= limit; ++p) {
+        const long long blocks = chunks * k * p, rest = blocks % slots, waves = (blocks + slots - 1) / slots;
+        const double c = ((double)(blocks / slots) + (rest == 0 ? 0.0 : 2 * rest <= slots ? 0.6 : 1.0)) * ((double)S / (double)(p * walkers) + adding);
+        if (cost < 0.0 || c < (waves == full ? 1.0 : 0.95) * cost) cost = c, parts = p, full = waves;
+    }
+    // Many classes leave no choice of parts: apart where more than a third of that time is idle (50 classes of 500 trees, 12288 samples 48 / 63 us, 200 of
+    // 500, 3000 samples 48 / 56; 100 of 500, 16384 samples, which fill it, 111 / 93).
+    if (k >= 32 && (double)(chunks * k) / (double)slots * (double)S / (double)walkers < 0.62 * cost) return CLB_ERR_SHAPE;
     if (parts > 65535 || chunks > 0x7fffffffLL) return CLB_ERR_SHAPE;
     const long long most = (S / parts + 1 + walkers - 1) / walkers;
     int planes = 4;

@@ -39,3 +39,31 @@ def test_counts_equal_layer_launches(levels, classes, size, batch, features):
         _lib.check(_lib.lib().clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 1))
     assert "packed_tree_count_kernel" in names and "group_popcount_kernel" not in names
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("classes, size, batch, fused_counts", [(50, 500, 12288, False), (200, 500, 3000, False), (100, 500, 16384, True), (150, 2000, 4096, True), (31, 500, 12288, True),
+                                                                (32, 500, 6000, False), (10, 2000, 30720, True), (100, 1000, 8192, True)])
+def test_many_classes_on_both_sides_of_their_line(classes, size, batch, fused_counts):
+    """One part and several, one wave of blocks and several (148 SMs); apart where too few blocks would be left."""
+    import convlogic_b200 as cb
+    from convlogic_b200 import _lib
+
+    torch.manual_seed(size)
+    net = torch.nn.Sequential(cb.LogicLayer(50, classes * size * 4), cb.LogicLayer(classes * size * 4, classes * size * 2),
+                              cb.LogicLayer(classes * size * 2, classes * size), cb.GroupSum(classes)).cuda().eval()
+    for p in net.parameters():
+        p.data.normal_()
+    x = torch.rand(batch, 50, device="cuda") < 0.4
+    want = cb.CompiledLogicNet(net, fuse=False).compile()(x)
+    fused = cb.CompiledLogicNet(net, fuse=True).compile()
+    _lib.check(_lib.lib().clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 0))
+    try:
+        _lib.trace(True)
+        got = fused(x)
+        torch.cuda.synchronize()
+        names = _lib.trace_report()
+    finally:
+        _lib.trace(False)
+        _lib.check(_lib.lib().clb_tune(_lib.TUNE_NET_ONE_LAUNCH, 1))
+    assert ("packed_tree_count_kernel" in names) == fused_counts, names
+    assert torch.equal(got, want)
