@@ -13,11 +13,12 @@
 // A feature whose gradient the walk completes is `closed`; the others (cuts, features with other than two readers) are
 // in the `open` list, and their gradient is taken from the consumer lists (logic_bwd.cu).
 //
-// What bounds both passes is DRAM: 256000 -> 256000, 1024 samples, forward 2.1 GB in 345 us (436 as a walk of the neurons in their own
-// order, stretch by stretch), backward 3.3 GB with the sums in 503 + 16 us (951 + 20 for the walk of the features), open features 14.
+// What bounds both passes is DRAM: 256000 -> 256000, 1024 samples, kernels alone (a profiler's times): forward 2.1 GB in 344 us and 9.5 for the records and
+// coefficients (436 and 6 as a walk of the neurons in their own order, stretch by stretch), backward 3.3 GB with the sums in 494 + 16 us (951 + 20 for
+// the walk of the features), open features 13.
 // Eight lanes own a range of positions and a stretch of 64 samples, the stretches of a row lying side by side in a block. Two
-// neurons' rows in flight per group and four (forward) or two (backward: 100 registers) blocks per SM; with three blocks the backward
-// spills (564 -> 624 us), four neurons at two blocks wait longer for the first (650), stretches of 32 samples read pieces too
+// neurons' rows in flight per group and four (forward) or two (backward: 100 registers) blocks per SM; of a backward that took 564 us,
+// its sums not merged yet, three blocks spill (624), four neurons at two blocks wait longer for the first (650), stretches of 32 samples read pieces too
 // small for a DRAM page (654); the forward with one neuron and six blocks 378, eight neurons and two blocks 620.
 #include "clb_common.cuh"
 #include "clb_logic.cuh"
@@ -307,7 +308,7 @@ int clb_logic_bwd_open(const float *x, const float *gy, const float *coef, const
 
 // A group's stretch is 64 samples, or 32 where that leaves a quarter fewer lanes idle (equally full, stretches of 32 are a quarter slower);
 // as many ranges as the resident blocks have groups for, of eight positions at least.  Partial sums beyond 24 MB are added over four
-// stretches first (us of a backward without / with: 256000 x 1024 560 / 532, 250000 x 511 357 / 353; 64000 x 256 60 / 64, 24000 x 1020 83 / 91).
+// stretches first (us of a whole backward without / with: 256000 x 1024 560 / 532, 250000 x 511 357 / 349; 64000 x 256 60 / 64, 24000 x 1020 83 / 91).
 struct PathCut {
     bool wide;
     int cols, ranges, sums; // sums: partial sums per neuron

@@ -29,10 +29,11 @@ namespace {
 
 constexpr char kMagic[8] = {'C', 'L', 'B', 'N', 'E', 'T', '0', '1'};
 constexpr size_t kHeaderBytes = 64, kLayerBytes = 64;
-// The one-launch kernel (net_cluster.cu, with slabs of 128 samples; smaller ones only lower the first figure) against layer-by-layer launches, us per call on B200: mnist k=64 (cost 0.1 M) batch 1 25 / 52,
-// batch 8192 103 / 148; cifar k=32 (0.13 M) batch 1 31 / 39, batch 2000 57 / 62, batch 8192 131 / 127; cifar k=64 (0.25 M) batch 1
-// 43 / 39, batch 500 43 / 49, batch 1000 66 / 59, batch 8192 233 / 190; cifar k=128 batch 1 66 / 45.  Beyond one slab per SM the
-// clusters come in waves and the layered kernels win from k=32 on.
+// The one-launch kernel (net_cluster.cu) against layer-by-layer launches, us per call on B200: mnist k=64 (cost 0.1 M) batch 1 16.5 / 51,
+// batch 8192 104 / 146; cifar k=32 (0.13 M) batch 1 21 / 40, batch 1000 41 / 41, batch 2000 52 / 58, batch 8192 133 / 124; cifar k=48 (0.19 M) batch 1 23 / 39,
+// batch 1000 50 / 51; cifar k=64 (0.25 M) batch 1 27 / 39, batch 500 43 / 43, batch 1000 64 / 56, batch 8192 236 / 178.  The line was drawn when slabs had 128
+// samples and k=64 took 43 / 39 at batch 1; calls of a slab or two beyond it would be faster in one launch now (cifar k=128 batch 1 39 / 47, mnist k=128
+// 25 / 55, k=256 37 / 63; batch 500 of cifar k=128 68 / 61).  Beyond one slab per SM the clusters come in waves and the layered kernels win from k=32 on.
 constexpr long long kOneLaunchCost = 200000;
 
 struct Header {

@@ -402,8 +402,8 @@ __global__ void __launch_bounds__(256) packed_rest_kernel(int32_t *__restrict__ 
 // A group of 2^LG lanes owns a range of positions and a stretch of R units per lane.  What bound it first was the issue
 // of integer instructions (171 per neuron and stretch of five words): offsets within a row are constants now, which lanes are inside
 // it is found once, and a gate's four masks come from a table; then the bytes in flight, for which many warps with one row each beat
-// fewer with two to four (us for one layer, x in the L2 as the layer before leaves it, two rows per neuron / this with four blocks and two
-// rows / with six and one: 3072 -> 64000 neurons, 1252 bytes 37 / 23 / 23, 64000 -> 64000 45 / 41 / 37, 128000 x 2500 171 / 141 / 128).
+// fewer with two to four (128000 neurons, rows of 2500 bytes: four blocks and two rows 141 us, six and one 128).  us for one layer, x in the L2 as the layer
+// before leaves it, two rows per neuron / this: 3072 -> 64000 neurons, 1252 bytes 37.6 / 22.9, 64000 -> 64000 45.3 / 34.3, 128000 x 2500 171 / 126.
 // step 1: an order, the connections from ia and ib as they are now (a lane each for as many positions as there are lanes, fetched as many
 // positions ahead, then through shared memory); step 4: records, with their own.
 template <typename V, int R, int LG>
